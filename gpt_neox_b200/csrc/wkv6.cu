@@ -7,201 +7,414 @@
 // kernel_backward_111 / _222), which walks the whole sequence in one thread per channel and needs
 // the sequence length as a compile-time constant for a per-thread array.
 //
-// Here the sequence is cut into chunks of 128 steps that run in parallel.  The recurrence is linear
-// in the state, so a chunk's end state is  P (.) S_start + S_local  with P[i] = prod_t d_t[i]:
-//   wkv_local : every chunk from a zero state -> S_local and sum_t(-exp(w_t)) per chunk
-//   wkv_fold  : sequential over the (few) chunks -> the state at the start of every chunk
-//   wkv_sweep : every chunk from its true start state -> outputs
-// The same three kernels run time-reversed for the gradient state G (dL/dS).  Two thread mappings:
-// "column" (a thread owns S[:, j], output indexed by j: y and gv) and "row" (a thread owns S[i, :],
-// output indexed by i: gr and gk).  The decay gradient needs no kernel of its own: with
-// Q_t[i] = sum_j G_t[i][j] S_t[i][j] one has Q_{t-1} - Q_t = r_t gr_t - k_t gk_t, so it follows from
-// gr and gk by a reverse cumulative sum (done by the caller).
+// One CTA of N threads walks one head's piece of the sequence with the N x N state in registers: warp w owns 32 columns
+// j, a lane N / 8 rows i by 8 columns.  Per step a lane reads N / 8 values of each row vector and 8 of each column
+// vector from shared memory (column vectors are stored twice side by side, so that the packed fp32 pairs, which run
+// over neighbouring rows, need no register moves) and does 3 packed operations per 2 state elements: one for the output
+// sum, two for the update.  The former one-column-per-thread mapping read every row vector whole in every thread, which
+// used the shared-memory port as fully as the FMA pipe.  The u term is taken out of the sums: it is a dot product per
+// step (formed while staging) times one value.  Sums over rows / columns leave a lane by transposing exchanges.
+//   forward  : one sweep: y (sum over i)
+//   backward : a forward sweep: gr (sum over j), then ONE reverse sweep of the gradient state G = dL/dS with both
+//              gk (sum over j) and gv (sum over i), which also forms the decay gradient: with
+//              Q_t[i] = sum_j G_t[i][j] S_t[i][j] one has Q_{t-1} - Q_t = r_t gr_t - k_t gk_t and
+//              dL/d(ew_t) = Q_t - k_t (gk_t - r_t u s_t),  s_t = <gy_t, v_t>,  ew = -exp(w)
+// Bound by the FMA pipe: 3 + 3 + 4 operations per state element and step.  Forward + backward of 32 x 512 tokens, 12 heads
+// of 64: 3.03 ms before, 0.91 ms now.
+//
+// The sequence is cut into chunks only when batch x heads leaves the chip idle (wkv_chunk_count): the recurrence is
+// linear, so a chunk's end state is  P (.) S_start + S_local  with P[i] = prod_t d_t[i]; local passes start every chunk
+// from zero, a fold gives the chunks' start states, and Q at a chunk's end is <G, S> there.
 #include "common.h"
 #include "ptx.cuh"
 
 namespace nx {
 
-constexpr int WK_CHUNK = 128;
-constexpr int WK_SUB = 16;
+constexpr int WK_SUB = 16;          // steps staged together
+constexpr int WK_MAX_CHUNKS = 32;
+
+enum WkvMode { WK_LOCAL_FWD = 0, WK_LOCAL_REV = 1, WK_Y = 2, WK_GR = 3, WK_G = 4 };
 
 struct WkvParams {
-  // "a/b/c" roles: column sweep out[j] = sum_i a[i] (u[i] b[i] c[j] + S[i][j]),  S += b[i] c[j]
-  //                row sweep    out[i] = sum_j a[j] (u[i] b[i] c[j] + S[i][j]),  S += b[i] c[j]
-  const h16 *a, *b, *c, *w;
-  long long sb, st;                 // batch / time strides (elements) shared by a, b, c, w
+  const h16 *r, *k, *v, *w, *gy;
+  long long sb, st;                 // batch / time strides (elements) shared by r, k, v, w, gy
   const float* u;                   // [H, N]
-  void* out;                        // [B, T, C] contiguous in (osb, ost); bf16 or fp32
+  h16 *y, *o_gr, *o_gk, *o_gv, *o_gw;   // (osb, ost)
+  float* gr32;                      // (osb, ost)
+  float* gu;                        // [H, N], zeroed by the caller
   long long osb, ost;
-  int out_f32;
   float* local;                     // [B, H, NC, N, N] chunk-local end states
-  float* start;                     // [B, H, NC, N, N] chunk start states
+  const float* start;               // [B, H, NC, N, N] start states of this sweep; null = zero (one chunk)
+  const float* fstart;              // reverse sweep with several chunks: the forward sweep's start states
   float* sumew;                     // [B, H, NC, N]
-  int B, T, H, NC;
+  int B, T, H, NC, clen;            // clen: steps per chunk, a multiple of WK_SUB
 };
 
-__device__ __forceinline__ float ldb(const h16* p) { return h16_to_float(*p); }
-
-template <int N>
-struct WkvStage {
-  float a[WK_SUB][N], b[WK_SUB][N], c[WK_SUB][N], d[WK_SUB][N], ew[WK_SUB][N];
-};
-
-template <int N>
-__device__ __forceinline__ void wkv_stage(const WkvParams& p, WkvStage<N>& s, int bi, int h, int t0, int t_lo,
-                                          int t_hi, bool need_a) {
-  for (int i = threadIdx.x; i < WK_SUB * N; i += N) {
-    const int t = i / N, n = i % N, tt = t0 + t;
-    float av = 0.f, bv = 0.f, cv = 0.f, ew = 0.f;
-    if (tt >= t_lo && tt < t_hi) {
-      const long long o = bi * p.sb + tt * p.st + h * N + n;
-      if (need_a) av = ldb(p.a + o);
-      bv = ldb(p.b + o);
-      cv = ldb(p.c + o);
-      ew = -__expf(ldb(p.w + o));
-    }
-    s.a[t][n] = av; s.b[t][n] = bv; s.c[t][n] = cv; s.ew[t][n] = ew; s.d[t][n] = __expf(ew);
+template <bool VEC>
+__device__ __forceinline__ void wk_load8(const h16* p, bool ok, float (&f)[8]) {
+  if (VEC) {
+    uint4 q = make_uint4(0u, 0u, 0u, 0u);
+    if (ok) q = *reinterpret_cast<const uint4*>(p);
+    const float2 a = unpack_h16x2(q.x), b = unpack_h16x2(q.y), c = unpack_h16x2(q.z), d = unpack_h16x2(q.w);
+    f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] = ok ? h16_to_float(p[j]) : 0.f;
   }
 }
 
-// Chunk-local end state from zero (column mapping) and the chunk's sum of ew.
-template <int N, bool REV>
-__global__ void __launch_bounds__(N) wkv_local_kernel(const WkvParams p) {
-  __shared__ WkvStage<N> s;
-  const int j = threadIdx.x, c = blockIdx.x, h = blockIdx.y, bi = blockIdx.z;
-  const int t_lo = c * WK_CHUNK, t_hi = min(t_lo + WK_CHUNK, p.T);
-  float S[N];
+template <int N, int MODE>
+struct WkvSmem {
+  static constexpr bool ROW = MODE == WK_GR || MODE == WK_G, COL = MODE == WK_Y || MODE == WK_G;
+  float b[WK_SUB][N], d[WK_SUB][N];             // state update: S = S * d[i] + b[i] * c[j]
+  float2 c[WK_SUB][N];                          // (c, c)
+  float a[COL ? WK_SUB : 1][N];                 // sum over i of a[i] S[i][j]
+  float2 e[ROW ? WK_SUB : 1][N];                // (e, e): sum over j of e[j] S[i][j]
+  float ew[WK_SUB][N];
+  float colsum[COL ? WK_SUB : 1][N];
+  float rowsum[ROW ? N / 32 : 1][ROW ? WK_SUB : 1][N];
+  float dot_col[WK_SUB], dot_row[WK_SUB];       // <a, u b> and <e, c>
+};
+
+template <int N, int MODE, bool VEC>
+__global__ void __launch_bounds__(N) wkv_kernel(const WkvParams p) {
+  using Sm = WkvSmem<N, MODE>;
+  constexpr bool REV = MODE == WK_LOCAL_REV || MODE == WK_G, ROW = Sm::ROW, COL = Sm::COL;
+  constexpr bool LOCAL = MODE == WK_LOCAL_FWD || MODE == WK_LOCAL_REV;
+  constexpr int QUADS = N / 32, PAIRS = QUADS * 2;     // a lane's rows: QUADS groups of 4 neighbours
+  constexpr int TPR = N / 8;                           // staging threads per step
+  constexpr int NPASS = WK_SUB * TPR / N;              // staging passes (2)
+  extern __shared__ __align__(16) unsigned char wk_raw[];
+  Sm& s = *reinterpret_cast<Sm*>(wk_raw);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int jg = lane & 3, ig = lane >> 2;
+  const int c = LOCAL && REV ? blockIdx.x + 1 : blockIdx.x, h = blockIdx.y, bi = blockIdx.z;
+  const int t_lo = c * p.clen, t_hi = min(t_lo + p.clen, p.T);
+  const long long base = ((long long)bi * p.H + h) * p.NC + c;
+
+  float2 S[PAIRS][8];
+  auto row_of = [&](int pr) { return (pr >> 1) * 32 + ig * 4 + (pr & 1) * 2; };      // first row of a pair
+  auto col_of = [&](int k) { return warp * 32 + (k >> 1) * 8 + jg * 2 + (k & 1); };
 #pragma unroll
-  for (int i = 0; i < N; ++i) S[i] = 0.f;
-  float sew = 0.f;
+  for (int pr = 0; pr < PAIRS; ++pr)
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      S[pr][k] = make_float2(0.f, 0.f);
+      if (!LOCAL && p.start != nullptr) {
+        const float* q = p.start + (base * N + row_of(pr)) * N + col_of(k);
+        S[pr][k] = make_float2(q[0], q[N]);
+      }
+    }
+  // ---- reverse sweep: thread i < N carries channel i's decay-gradient sum
+  float Q = 0.f, gu = 0.f;
+  const float u_me = p.u[h * N + threadIdx.x];
+  if (MODE == WK_G && p.fstart != nullptr && c + 1 < p.NC) {
+    const float* g = p.start + (base * N + threadIdx.x) * N;
+    const float* f = p.fstart + ((base + 1) * N + threadIdx.x) * N;
+    for (int j = 0; j < N; ++j) Q += g[j] * f[j];
+  }
+  // ---- staging role: step trow (+ N / TPR per pass), 8 channels from ch8
+  const int trow = threadIdx.x / TPR, ch8 = (threadIdx.x % TPR) * 8;
+  float u8[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) u8[j] = p.u[h * N + ch8 + j];
+  float sew = 0.f;                                     // LOCAL: thread i sums ew of channel i
+
   const int nsub = (t_hi - t_lo + WK_SUB - 1) / WK_SUB;
   for (int q = 0; q < nsub; ++q) {
-    const int sub = REV ? nsub - 1 - q : q;
-    const int t0 = t_lo + sub * WK_SUB;
-    __syncthreads();
-    wkv_stage<N>(p, s, bi, h, t0, t_lo, t_hi, false);
-    __syncthreads();
-#pragma unroll 1
-    for (int tq = 0; tq < WK_SUB; ++tq) {
-      const int t = REV ? WK_SUB - 1 - tq : tq;
-      if (t0 + t >= t_hi) continue;
-      const float cj = s.c[t][j];
-      sew += s.ew[t][j];
+    const int t0 = t_lo + (REV ? nsub - 1 - q : q) * WK_SUB;
+    const int steps = min(WK_SUB, t_hi - t0);
+    float gr[MODE == WK_G ? WK_SUB : 1];
+    if (MODE == WK_G) {
 #pragma unroll
-      for (int i = 0; i < N; ++i) S[i] = S[i] * s.d[t][i] + s.b[t][i] * cj;
+      for (int t = 0; t < WK_SUB; ++t)
+        gr[t] = t < steps ? p.gr32[bi * p.osb + (long long)(t0 + t) * p.ost + h * N + threadIdx.x] : 0.f;
     }
-  }
-  const long long base = (((long long)bi * p.H + h) * p.NC + c);
 #pragma unroll
-  for (int i = 0; i < N; ++i) p.local[(base * N + i) * N + j] = S[i];
-  p.sumew[base * N + j] = sew;
+    for (int ps = 0; ps < NPASS; ++ps) {
+      const int t = trow + ps * (N / TPR);
+      const bool ok = t < steps;
+      const long long o = bi * p.sb + (long long)(t0 + t) * p.st + h * N + ch8;
+      float x[8], y[8], wv[8];
+      wk_load8<VEC>(p.w + o, ok, wv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float ew = ok ? -__expf(wv[j]) : 0.f;
+        s.ew[t][ch8 + j] = ew;
+        s.d[t][ch8 + j] = __expf(ew);
+      }
+      wk_load8<VEC>((REV ? p.r : p.k) + o, ok, x);     // b
+      wk_load8<VEC>((REV ? p.gy : p.v) + o, ok, y);    // c
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        s.b[t][ch8 + j] = x[j];
+        s.c[t][ch8 + j] = make_float2(y[j], y[j]);
+      }
+      if (COL) {
+        float a[8], dt = 0.f;
+        wk_load8<VEC>((MODE == WK_Y ? p.r : p.k) + o, ok, a);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          s.a[t][ch8 + j] = a[j];
+          dt += a[j] * u8[j] * x[j];
+        }
+#pragma unroll
+        for (int m = TPR / 2; m > 0; m >>= 1) dt += __shfl_xor_sync(0xffffffffu, dt, m);
+        if (ch8 == 0) s.dot_col[t] = dt;
+      }
+      if (ROW) {
+        float e[8], dt = 0.f;
+        wk_load8<VEC>((MODE == WK_GR ? p.gy : p.v) + o, ok, e);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          s.e[t][ch8 + j] = make_float2(e[j], e[j]);
+          dt += e[j] * y[j];
+        }
+#pragma unroll
+        for (int m = TPR / 2; m > 0; m >>= 1) dt += __shfl_xor_sync(0xffffffffu, dt, m);
+        if (ch8 == 0) s.dot_row[t] = dt;
+      }
+    }
+    __syncthreads();
+#pragma unroll 2
+    for (int tq = 0; tq < steps; ++tq) {
+      const int t = REV ? steps - 1 - tq : tq;
+      float2 dv[PAIRS], bv[PAIRS], av[PAIRS], racc[PAIRS], cacc[8];
+#pragma unroll
+      for (int g = 0; g < QUADS; ++g) {
+        const float4 d4 = *reinterpret_cast<const float4*>(&s.d[t][g * 32 + ig * 4]);
+        const float4 b4 = *reinterpret_cast<const float4*>(&s.b[t][g * 32 + ig * 4]);
+        dv[2 * g] = make_float2(d4.x, d4.y); dv[2 * g + 1] = make_float2(d4.z, d4.w);
+        bv[2 * g] = make_float2(b4.x, b4.y); bv[2 * g + 1] = make_float2(b4.z, b4.w);
+        if (COL) {
+          const float4 a4 = *reinterpret_cast<const float4*>(&s.a[t][g * 32 + ig * 4]);
+          av[2 * g] = make_float2(a4.x, a4.y); av[2 * g + 1] = make_float2(a4.z, a4.w);
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const float4 c4 = *reinterpret_cast<const float4*>(&s.c[t][warp * 32 + m * 8 + jg * 2]);
+        float4 e4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ROW) e4 = *reinterpret_cast<const float4*>(&s.e[t][warp * 32 + m * 8 + jg * 2]);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const int k = 2 * m + x;
+          const float2 cc = x ? make_float2(c4.z, c4.w) : make_float2(c4.x, c4.y);
+          const float2 ee = x ? make_float2(e4.z, e4.w) : make_float2(e4.x, e4.y);
+#pragma unroll
+          for (int pr = 0; pr < PAIRS; ++pr) {
+            if (COL) cacc[k] = pr == 0 ? fmul2(av[0], S[0][k]) : ffma2(av[pr], S[pr][k], cacc[k]);
+            if (ROW) racc[pr] = k == 0 ? fmul2(ee, S[pr][0]) : ffma2(ee, S[pr][k], racc[pr]);
+            S[pr][k] = ffma2(S[pr][k], dv[pr], fmul2(bv[pr], cc));
+          }
+        }
+      }
+      if (COL) {      // 8 columns over the 8 row groups: lane ig ends up with its column ig
+        float v8[8], v4[4], v2[2];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v8[k] = cacc[k].x + cacc[k].y;
+        const bool h2 = ig & 4, h1 = ig & 2, h0 = ig & 1;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          v4[k] = (h2 ? v8[4 + k] : v8[k]) + __shfl_xor_sync(0xffffffffu, h2 ? v8[k] : v8[4 + k], 16);
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+          v2[k] = (h1 ? v4[2 + k] : v4[k]) + __shfl_xor_sync(0xffffffffu, h1 ? v4[k] : v4[2 + k], 8);
+        s.colsum[t][col_of(ig)] = (h0 ? v2[1] : v2[0]) + __shfl_xor_sync(0xffffffffu, h0 ? v2[0] : v2[1], 4);
+      }
+      if (ROW) {      // a lane's N / 8 rows over the 4 column groups
+        const bool h1 = jg & 2, h0 = jg & 1;
+        float2 w2[PAIRS / 2];
+#pragma unroll
+        for (int k = 0; k < PAIRS / 2; ++k) {
+          const float2 keep = h1 ? racc[PAIRS / 2 + k] : racc[k], give = h1 ? racc[k] : racc[PAIRS / 2 + k];
+          w2[k].x = keep.x + __shfl_xor_sync(0xffffffffu, give.x, 2);
+          w2[k].y = keep.y + __shfl_xor_sync(0xffffffffu, give.y, 2);
+        }
+        if (PAIRS == 4) {
+          const float2 keep = h0 ? w2[PAIRS / 2 - 1] : w2[0], give = h0 ? w2[0] : w2[PAIRS / 2 - 1];
+          const float2 o = make_float2(keep.x + __shfl_xor_sync(0xffffffffu, give.x, 1),
+                                       keep.y + __shfl_xor_sync(0xffffffffu, give.y, 1));
+          *reinterpret_cast<float2*>(&s.rowsum[warp][t][row_of((h1 ? 2 : 0) + (h0 ? 1 : 0))]) = o;
+        } else {
+          const float o = (h0 ? w2[0].y : w2[0].x) + __shfl_xor_sync(0xffffffffu, h0 ? w2[0].x : w2[0].y, 1);
+          s.rowsum[warp][t][row_of(h1 ? 1 : 0) + (h0 ? 1 : 0)] = o;
+        }
+      }
+    }
+    __syncthreads();
+    const int me = threadIdx.x;
+    const long long oo = bi * p.osb + (long long)t0 * p.ost + h * N + me;
+    if (LOCAL) {
+      for (int t = 0; t < steps; ++t) sew += s.ew[t][me];
+    } else {
+      // (thread me: channel me, step by step in the sweep's direction)
+#pragma unroll
+      for (int tq = 0; tq < WK_SUB; ++tq) {
+        const int t = REV ? WK_SUB - 1 - tq : tq;
+        if (t >= steps) continue;
+        float row = 0.f;
+        if (ROW) {
+#pragma unroll
+          for (int w = 0; w < QUADS; ++w) row += s.rowsum[w][t][me];
+        }
+        if (MODE == WK_Y) {
+          p.y[oo + t * p.ost] = float_to_h16(s.colsum[t][me] + s.c[t][me].x * s.dot_col[t]);
+        } else if (MODE == WK_GR) {
+          p.gr32[oo + t * p.ost] = row + u_me * s.b[t][me] * s.dot_row[t];
+        } else {
+          const float r_ = s.b[t][me], k_ = s.a[t][me], st = s.dot_row[t];
+          const float gk = row + u_me * r_ * st;
+          const float g = gr[MODE == WK_G ? t : 0];
+          p.o_gr[oo + t * p.ost] = float_to_h16(g);
+          p.o_gk[oo + t * p.ost] = float_to_h16(gk);
+          p.o_gv[oo + t * p.ost] = float_to_h16(s.colsum[t][me] + s.c[t][me].x * s.dot_col[t]);
+          p.o_gw[oo + t * p.ost] = float_to_h16((Q - k_ * row) * s.ew[t][me]);
+          Q += r_ * g - k_ * gk;
+          gu += r_ * k_ * st;
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (LOCAL) {
+#pragma unroll
+    for (int pr = 0; pr < PAIRS; ++pr)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        float* o = p.local + (base * N + row_of(pr)) * N + col_of(k);
+        o[0] = S[pr][k].x;
+        o[N] = S[pr][k].y;
+      }
+    p.sumew[base * N + threadIdx.x] = sew;
+  }
+  if (MODE == WK_G) atomicAdd(p.gu + h * N + threadIdx.x, gu);
 }
 
 // start[c] for every chunk: forward  start[0] = 0, start[c+1] = P_c start[c] + local[c];
 //                           reverse  start[NC-1] = 0, start[c-1] = P_c start[c] + local[c].
 template <int N, bool REV>
-__global__ void __launch_bounds__(N) wkv_fold_kernel(const WkvParams p) {
-  const int j = threadIdx.x, h = blockIdx.y, bi = blockIdx.z;
-  float S[N];
-#pragma unroll
-  for (int i = 0; i < N; ++i) S[i] = 0.f;
-  for (int q = 0; q < p.NC; ++q) {
-    const int c = REV ? p.NC - 1 - q : q;
-    const long long base = (((long long)bi * p.H + h) * p.NC + c);
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      p.start[(base * N + i) * N + j] = S[i];
-      S[i] = S[i] * __expf(p.sumew[base * N + i]) + p.local[(base * N + i) * N + j];
-    }
+__global__ void __launch_bounds__(N) wkv_fold_kernel(const float* local, const float* sumew, float* start, int NC) {
+  const int j = threadIdx.x, i = blockIdx.x;
+  const long long head = (long long)blockIdx.z * gridDim.y + blockIdx.y;
+  float S = 0.f;
+  for (int q = 0; q < NC; ++q) {
+    const int c = REV ? NC - 1 - q : q;
+    const long long o = ((head * NC + c) * N + i) * N + j;
+    start[o] = S;
+    if (q + 1 < NC) S = S * __expf(sumew[(head * NC + c) * N + i]) + local[o];
   }
 }
 
-template <int N>
-__device__ __forceinline__ void wkv_store(const WkvParams& p, long long o, float v) {
-  if (p.out_f32) reinterpret_cast<float*>(p.out)[o] = v;
-  else reinterpret_cast<h16*>(p.out)[o] = float_to_h16(v);
-}
-
-// ROW = false: thread j owns S[:, j]; ROW = true: thread i owns S[i, :].
-template <int N, bool REV, bool ROW>
-__global__ void __launch_bounds__(N) wkv_sweep_kernel(const WkvParams p) {
-  __shared__ WkvStage<N> s;
-  __shared__ float us[N];
-  const int me = threadIdx.x, c = blockIdx.x, h = blockIdx.y, bi = blockIdx.z;
-  const int t_lo = c * WK_CHUNK, t_hi = min(t_lo + WK_CHUNK, p.T);
-  us[me] = p.u[h * N + me];
-  float S[N];
-  const long long base = (((long long)bi * p.H + h) * p.NC + c);
-#pragma unroll
-  for (int x = 0; x < N; ++x) S[x] = ROW ? p.start[(base * N + me) * N + x] : p.start[(base * N + x) * N + me];
-  const int nsub = (t_hi - t_lo + WK_SUB - 1) / WK_SUB;
-  for (int q = 0; q < nsub; ++q) {
-    const int sub = REV ? nsub - 1 - q : q;
-    const int t0 = t_lo + sub * WK_SUB;
-    __syncthreads();
-    wkv_stage<N>(p, s, bi, h, t0, t_lo, t_hi, true);
-    __syncthreads();
-#pragma unroll 1
-    for (int tq = 0; tq < WK_SUB; ++tq) {
-      const int t = REV ? WK_SUB - 1 - tq : tq;
-      if (t0 + t >= t_hi) continue;
-      float acc = 0.f;
-      if (!ROW) {
-        const float cj = s.c[t][me];
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-          const float x = s.b[t][i] * cj;
-          acc += s.a[t][i] * (us[i] * x + S[i]);
-          S[i] = S[i] * s.d[t][i] + x;
-        }
-      } else {
-        const float bi_ = s.b[t][me], di = s.d[t][me], ui = us[me];
-#pragma unroll
-        for (int jx = 0; jx < N; ++jx) {
-          const float x = bi_ * s.c[t][jx];
-          acc += s.a[t][jx] * (ui * x + S[jx]);
-          S[jx] = S[jx] * di + x;
-        }
-      }
-      wkv_store<N>(p, bi * p.osb + (long long)(t0 + t) * p.ost + h * N + me, acc);
-    }
+template <int N, int MODE>
+static int wkv_launch(const WkvParams& p, bool vec, int chunks, cudaStream_t stream) {
+  const int smem = (int)sizeof(WkvSmem<N, MODE>);
+  static bool attr_set = false;
+  if (!attr_set) {
+    NX_CUDA_CHECK(cudaFuncSetAttribute(wkv_kernel<N, MODE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    NX_CUDA_CHECK(cudaFuncSetAttribute(wkv_kernel<N, MODE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    attr_set = true;
   }
-}
-
-template <int N>
-static int wkv_run(const WkvParams& p, int mode, cudaStream_t stream) {
-  dim3 grid(p.NC, p.H, p.B), gridf(1, p.H, p.B);
-  switch (mode) {
-    case 0: wkv_local_kernel<N, false><<<grid, N, 0, stream>>>(p); break;
-    case 1: wkv_local_kernel<N, true><<<grid, N, 0, stream>>>(p); break;
-    case 2: wkv_fold_kernel<N, false><<<gridf, N, 0, stream>>>(p); break;
-    case 3: wkv_fold_kernel<N, true><<<gridf, N, 0, stream>>>(p); break;
-    case 4: wkv_sweep_kernel<N, false, false><<<grid, N, 0, stream>>>(p); break;   // forward, column (y)
-    case 5: wkv_sweep_kernel<N, true, false><<<grid, N, 0, stream>>>(p); break;    // reverse, column (gv)
-    case 6: wkv_sweep_kernel<N, false, true><<<grid, N, 0, stream>>>(p); break;    // forward, row (gr)
-    case 7: wkv_sweep_kernel<N, true, true><<<grid, N, 0, stream>>>(p); break;     // reverse, row (gk)
-    default: return NX_ERR_ARG;
-  }
+  const dim3 grid(chunks, p.H, p.B);
+  if (vec) wkv_kernel<N, MODE, true><<<grid, N, smem, stream>>>(p);
+  else wkv_kernel<N, MODE, false><<<grid, N, smem, stream>>>(p);
   NX_LAUNCH_CHECK();
   return NX_OK;
 }
 
-NX_API int NX_SYM(nx_wkv6_chunks)(int T) { return (T + WK_CHUNK - 1) / WK_CHUNK; }
+// Chunks the sequence is cut into: time goes with the CTAs of the fullest SM times the chunk length; more than one
+// chunk adds the local pass (2 of the sweep's 3 operations) over all chunks but one.  Below four CTAs (two warps per
+// scheduler) an SM does not overlap its steps' exchanges and loads with arithmetic.
+static int wkv_chunk_count(int B, int T, int H) {
+  const int subs = (T + WK_SUB - 1) / WK_SUB, sms = sm_count();
+  int best = 1;
+  float best_cost = 1e30f;
+  for (int nc = 1; nc <= WK_MAX_CHUNKS && nc <= subs; ++nc) {
+    const int len = (subs + nc - 1) / nc;
+    if ((subs + len - 1) / len != nc) continue;
+    const long long per_sm = (static_cast<long long>(B) * H * nc + sms - 1) / sms;
+    const float cost = len * fmaxf(static_cast<float>(per_sm), 2.f) * (1.f + 0.67f * (nc - 1) / nc) + 0.05f * subs * (nc > 1);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = nc;
+    }
+  }
+  return best;
+}
+static int wkv_chunk_len(int T, int nc) { return ((T + WK_SUB - 1) / WK_SUB + nc - 1) / nc * WK_SUB; }
 
-// mode: 0/1 local state fwd/rev, 2/3 fold fwd/rev, 4 y, 5 gv, 6 gr, 7 gk (see wkv_run).
-// a, b, c, w: bf16 [B, T, H*N] addressed by (sb, st); u fp32 [H, N]; out bf16 or fp32 by (osb, ost).
-// local / start: fp32 [B, H, NC, N, N]; sumew fp32 [B, H, NC, N].
-NX_API int NX_SYM(nx_wkv6_pass)(int mode, const void* a, const void* b, const void* c, const void* w, long long sb,
-                        long long st, const void* u, void* out, long long osb, long long ost, int out_f32,
-                        void* local, void* start, void* sumew, int B, int T, int H, int N, cudaStream_t stream) {
+static bool wkv_vec_ok(const WkvParams& p) {
+  auto ok = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  return ok(p.r) && ok(p.k) && ok(p.v) && ok(p.w) && ok(p.gy) && p.sb % 8 == 0 && p.st % 8 == 0;
+}
+
+template <int N>
+static int wkv_forward(WkvParams p, float* start, cudaStream_t stream) {
+  const bool vec = wkv_vec_ok(p);
+  if (p.NC > 1) {
+    int rc = wkv_launch<N, WK_LOCAL_FWD>(p, vec, p.NC - 1, stream);
+    if (rc != NX_OK) return rc;
+    wkv_fold_kernel<N, false><<<dim3(N, p.H, p.B), N, 0, stream>>>(p.local, p.sumew, start, p.NC);
+    NX_LAUNCH_CHECK();
+    p.start = start;
+  }
+  return wkv_launch<N, WK_Y>(p, vec, p.NC, stream);
+}
+
+template <int N>
+static int wkv_backward(WkvParams p, const float* fstart, float* rstart, cudaStream_t stream) {
+  const bool vec = wkv_vec_ok(p);
+  p.start = p.NC > 1 ? fstart : nullptr;
+  int rc = wkv_launch<N, WK_GR>(p, vec, p.NC, stream);
+  if (rc != NX_OK) return rc;
+  p.start = nullptr;
+  if (p.NC > 1) {
+    rc = wkv_launch<N, WK_LOCAL_REV>(p, vec, p.NC - 1, stream);
+    if (rc != NX_OK) return rc;
+    wkv_fold_kernel<N, true><<<dim3(N, p.H, p.B), N, 0, stream>>>(p.local, p.sumew, rstart, p.NC);
+    NX_LAUNCH_CHECK();
+    p.start = rstart;
+    p.fstart = fstart;
+  }
+  return wkv_launch<N, WK_G>(p, vec, p.NC, stream);
+}
+
+NX_API int NX_SYM(nx_wkv6_chunks)(int B, int T, int H) { return wkv_chunk_count(B, T, H); }
+
+// r, k, v, w: bf16 [B, T, H*N] addressed by (sb, st); u fp32 [H, N]; y bf16 by (osb, ost).  With NC =
+// nx_wkv6_chunks(B, T, H) > 1: local / start fp32 [B, H, NC, N, N] and sumew fp32 [B, H, NC, N] are scratch, and
+// `start` is kept for the backward; they may be null for NC = 1.
+NX_API int NX_SYM(nx_wkv6_fwd)(const void* r, const void* k, const void* v, const void* w, long long sb, long long st,
+                       const void* u, void* y, long long osb, long long ost, void* local, void* start, void* sumew,
+                       int B, int T, int H, int N, cudaStream_t stream) {
   NX_REQUIRE(N == 64 || N == 32, "wkv6: head size %d not supported (32 or 64)", N);
+  if (B <= 0 || T <= 0 || H <= 0) return NX_OK;
   WkvParams p{};
-  p.a = (const h16*)a; p.b = (const h16*)b; p.c = (const h16*)c;
-  p.w = (const h16*)w; p.sb = sb; p.st = st; p.u = (const float*)u;
-  p.out = out; p.osb = osb; p.ost = ost; p.out_f32 = out_f32;
-  p.local = (float*)local; p.start = (float*)start; p.sumew = (float*)sumew;
-  p.B = B; p.T = T; p.H = H; p.NC = (T + WK_CHUNK - 1) / WK_CHUNK;
-  return N == 64 ? wkv_run<64>(p, mode, stream) : wkv_run<32>(p, mode, stream);
+  p.r = (const h16*)r; p.k = (const h16*)k; p.v = (const h16*)v; p.w = (const h16*)w;
+  p.sb = sb; p.st = st; p.u = (const float*)u;
+  p.y = (h16*)y; p.osb = osb; p.ost = ost;
+  p.local = (float*)local; p.sumew = (float*)sumew;
+  p.B = B; p.T = T; p.H = H; p.NC = wkv_chunk_count(B, T, H); p.clen = wkv_chunk_len(T, p.NC);
+  return N == 64 ? wkv_forward<64>(p, (float*)start, stream) : wkv_forward<32>(p, (float*)start, stream);
+}
+
+// gy like r.  gr / gk / gv / gw: bf16 by (osb, ost); gr32: fp32 scratch of the same shape and strides; gu fp32 [H, N],
+// zeroed by the caller.  fstart: the forward's start states; local, rstart, sumew: scratch (all null for NC = 1).
+NX_API int NX_SYM(nx_wkv6_bwd)(const void* r, const void* k, const void* v, const void* w, const void* gy, long long sb,
+                       long long st, const void* u, void* gr, void* gk, void* gv, void* gw, void* gr32, void* gu,
+                       long long osb, long long ost, void* local, const void* fstart, void* rstart, void* sumew,
+                       int B, int T, int H, int N, cudaStream_t stream) {
+  NX_REQUIRE(N == 64 || N == 32, "wkv6: head size %d not supported (32 or 64)", N);
+  if (B <= 0 || T <= 0 || H <= 0) return NX_OK;
+  WkvParams p{};
+  p.r = (const h16*)r; p.k = (const h16*)k; p.v = (const h16*)v; p.w = (const h16*)w; p.gy = (const h16*)gy;
+  p.sb = sb; p.st = st; p.u = (const float*)u;
+  p.o_gr = (h16*)gr; p.o_gk = (h16*)gk; p.o_gv = (h16*)gv; p.o_gw = (h16*)gw;
+  p.gr32 = (float*)gr32; p.gu = (float*)gu; p.osb = osb; p.ost = ost;
+  p.local = (float*)local; p.sumew = (float*)sumew;
+  p.B = B; p.T = T; p.H = H; p.NC = wkv_chunk_count(B, T, H); p.clen = wkv_chunk_len(T, p.NC);
+  return N == 64 ? wkv_backward<64>(p, (const float*)fstart, (float*)rstart, stream)
+                 : wkv_backward<32>(p, (const float*)fstart, (float*)rstart, stream);
 }
 
 }  // namespace nx

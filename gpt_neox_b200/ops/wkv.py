@@ -46,14 +46,6 @@ def decay_grad_from_gr_gk(r, k, v, w, u, gy, gr, gk):
     return gw, gu
 
 
-def _pass(mode, a, b, c, w, u, out, local, start, sumew, B, T, H, N):
-    LAUNCHES["n"] += 1
-    o = (out.stride(0), out.stride(1), int(out.dtype == torch.float32)) if out is not None else (0, 0, 0)
-    _lib.check(_lib.lib(b).nx_wkv6_pass(mode, _lib.ptr(a), _lib.ptr(b), _lib.ptr(c), _lib.ptr(w), b.stride(0),
-                                       b.stride(1), _lib.ptr(u), _lib.ptr(out), o[0], o[1], o[2], _lib.ptr(local),
-                                       _lib.ptr(start), _lib.ptr(sumew), B, T, H, N, _lib.stream()), "nx_wkv6_pass")
-
-
 def _same_layout(*ts):
     """Views sharing (batch, time) strides with contiguous channels; copies to time-major otherwise."""
     s0 = (ts[0].stride(0), ts[0].stride(1))
@@ -75,46 +67,46 @@ class _WkvFn(torch.autograd.Function):
         H, N = u.shape
         r, k, v, w = _same_layout(r, k, v, w)
         u32 = u.float().contiguous()
-        nc = _lib.lib().nx_wkv6_chunks(T)
+        lib = _lib.lib(r)
+        nc = lib.nx_wkv6_chunks(B, T, H)
         dev = r.device
-        local = torch.empty((B, H, nc, N, N), device=dev, dtype=torch.float32)
-        start = torch.empty_like(local)
-        sumew = torch.empty((B, H, nc, N), device=dev, dtype=torch.float32)
+        local = start = sumew = None
+        if nc > 1:
+            local = torch.empty((B, H, nc, N, N), device=dev, dtype=torch.float32)
+            start = torch.empty_like(local)
+            sumew = torch.empty((B, H, nc, N), device=dev, dtype=torch.float32)
         y = torch.empty((T, B, C), device=dev, dtype=r.dtype).transpose(0, 1)
-        _pass(0, None, k, v, w, u32, None, local, start, sumew, B, T, H, N)
-        _pass(2, None, k, v, w, u32, None, local, start, sumew, B, T, H, N)
-        _pass(4, r, k, v, w, u32, y, local, start, sumew, B, T, H, N)
-        ctx.save_for_backward(r, k, v, w, u32, start, sumew)
+        LAUNCHES["n"] += 1 if nc == 1 else 3
+        _lib.check(lib.nx_wkv6_fwd(_lib.ptr(r), _lib.ptr(k), _lib.ptr(v), _lib.ptr(w), r.stride(0), r.stride(1),
+                                   _lib.ptr(u32), _lib.ptr(y), y.stride(0), y.stride(1), _lib.ptr(local),
+                                   _lib.ptr(start), _lib.ptr(sumew), B, T, H, N, _lib.stream()), "nx_wkv6_fwd")
+        ctx.save_for_backward(r, k, v, w, u32, start)
         ctx.u_dtype = u.dtype
         return y
 
     @staticmethod
     def backward(ctx, gy):
-        r, k, v, w, u32, start, sumew = ctx.saved_tensors
+        r, k, v, w, u32, start = ctx.saved_tensors
         B, T, C = r.shape
         H, N = u32.shape
         if gy.stride(2) != 1 or (gy.stride(0), gy.stride(1)) != (r.stride(0), r.stride(1)):
-            buf = torch.empty((T, B, C), device=gy.device, dtype=gy.dtype).transpose(0, 1)
-            buf.copy_(gy)
-            if (buf.stride(0), buf.stride(1)) != (r.stride(0), r.stride(1)):
-                r, k, v, w = (x.contiguous() for x in (r, k, v, w))
-                buf = gy.contiguous()
-            gy = buf
+            gy = torch.empty((T, B, C), device=gy.device, dtype=gy.dtype).transpose(0, 1).copy_(gy)
+            r, k, v, w, gy = _same_layout(r, k, v, w, gy)      # (time-major already, as a rule: nothing to copy)
         dev = r.device
-        f32 = lambda: torch.empty((T, B, C), device=dev, dtype=torch.float32).transpose(0, 1)
-        gr, gk, gv = f32(), f32(), f32()
-        # forward-state sweep: gr (start states were kept from the forward)
-        _pass(6, gy, k, v, w, u32, gr, None, start, sumew, B, T, H, N)
-        # reverse state G: local, fold, then gk (rows) and gv (columns)
-        local = torch.empty_like(start)
-        rstart = torch.empty_like(start)
-        _pass(1, None, r, gy, w, u32, None, local, rstart, sumew, B, T, H, N)
-        _pass(3, None, r, gy, w, u32, None, local, rstart, sumew, B, T, H, N)
-        _pass(7, v, r, gy, w, u32, gk, None, rstart, sumew, B, T, H, N)
-        _pass(5, k, r, gy, w, u32, gv, None, rstart, sumew, B, T, H, N)
-        gw, gu = decay_grad_from_gr_gk(r, k, v, w, u32, gy, gr, gk)
-        dt = r.dtype
-        return gr.to(dt), gk.to(dt), gv.to(dt), gw.to(dt), gu.to(ctx.u_dtype)
+        gr, gk, gv, gw = (torch.empty((T, B, C), device=dev, dtype=r.dtype).transpose(0, 1) for _ in range(4))
+        gr32 = torch.empty((T, B, C), device=dev, dtype=torch.float32).transpose(0, 1)
+        gu = torch.zeros((H, N), device=dev, dtype=torch.float32)
+        local = rstart = sumew = None
+        if start is not None:
+            local, rstart = torch.empty_like(start), torch.empty_like(start)
+            sumew = torch.empty(start.shape[:4], device=dev, dtype=torch.float32)
+        LAUNCHES["n"] += 2 if start is None else 4
+        _lib.check(_lib.lib(r).nx_wkv6_bwd(
+            _lib.ptr(r), _lib.ptr(k), _lib.ptr(v), _lib.ptr(w), _lib.ptr(gy), r.stride(0), r.stride(1), _lib.ptr(u32),
+            _lib.ptr(gr), _lib.ptr(gk), _lib.ptr(gv), _lib.ptr(gw), _lib.ptr(gr32), _lib.ptr(gu), gr.stride(0),
+            gr.stride(1), _lib.ptr(local), _lib.ptr(start), _lib.ptr(rstart), _lib.ptr(sumew), B, T, H, N,
+            _lib.stream()), "nx_wkv6_bwd")
+        return gr, gk, gv, gw, gu.to(ctx.u_dtype)
 
 
 def wkv6(r, k, v, w, u):

@@ -84,3 +84,27 @@ def test_sparse_attention_types_train_on_cpu(kind):
     cfg = tiny_config(use_cpu_initialization=True, attention_config=[[[kind], 2]], sparsity_config={"block": 4})
     losses = run_distributed(_train, 1, cfg, 3)[0]
     assert all(l == l for l in losses)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,T,H,N,pad", [(1, 1, 1, 64, 0), (2, 17, 3, 32, 0), (1, 333, 2, 64, 0), (40, 48, 12, 64, 0),
+                                         (1, 130, 1, 32, 4), (3, 64, 2, 64, 8)])
+def test_wkv6_chunks_and_layouts(B, T, H, N, pad, dtype):
+    """Sub-block remainders, one chunk (many heads) and many (few heads), views whose rows are not 16-byte aligned."""
+    from gpt_neox_b200.ops.wkv import wkv6, wkv6_reference
+    torch.manual_seed(7)
+    C = H * N
+    mk = lambda m=0.0: (torch.randn(T, B, C + pad, device="cuda") * 0.5 + m).to(dtype)[..., pad:].transpose(0, 1)
+    leaves = [t.detach().requires_grad_(True) for t in (mk(), mk(), mk(), mk(-1.5))]
+    leaves.append((torch.randn(H, N, device="cuda") * 0.3).to(dtype).requires_grad_(True))
+    ref = [t.detach().float().clone().requires_grad_(True) for t in leaves]
+    gy = (torch.randn(B, T, C, device="cuda") * 0.5).to(dtype)
+    y = wkv6(*leaves)
+    got = torch.autograd.grad(y, leaves, gy)
+    yr = wkv6_reference(*ref)
+    want = torch.autograd.grad(yr, ref, gy.float(), allow_unused=True)       # (T = 1: nothing decays)
+    want = [torch.zeros_like(t) if r is None else r for t, r in zip(ref, want)]
+    eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -11
+    for a, r in zip((y,) + got, [yr] + want):                   # one rounding to 16 bits; fp32 sums on both sides
+        assert (a.float() - r).abs().max().item() <= 2 * eps * r.abs().max().item() + 1e-3
