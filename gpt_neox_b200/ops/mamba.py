@@ -98,52 +98,55 @@ class _ScanFn(torch.autograd.Function):
         L_ = _lib.lib(x)
         B, L, Dm = x.shape
         dev = x.device
-        nc = L_.nx_scan_chunks(L)
+        nc = L_.nx_scan_chunks(B, L, Dm, 0)
         out = torch.empty((L, B, Dm), device=dev, dtype=x.dtype).transpose(0, 1)   # time-major memory
-        state = torch.empty((B, nc, Dm, 16), device=dev, dtype=torch.float32)
-        h0 = torch.empty((B, nc, Dm, 16), device=dev, dtype=torch.float32)
-        sumdt = torch.empty((B, nc, Dm), device=dev, dtype=torch.float32)
+        state = sumdt = ckpt = None
+        if nc > 1:
+            state = torch.empty((B, nc, Dm, 16), device=dev, dtype=torch.float32)
+            sumdt = torch.empty((B, nc, Dm), device=dev, dtype=torch.float32)
+        if any(ctx.needs_input_grad):       # the state at the start of every 32-step block, for the backward
+            ckpt = torch.empty((B, L_.nx_scan_blocks(L), Dm, 16), device=dev, dtype=torch.float32)
         zs = (z.stride(0), z.stride(1)) if z is not None else (0, 0)
         LAUNCHES["n"] += 2 if nc > 1 else 1
         _lib.check(L_.nx_selective_scan_fwd(
             _lib.ptr(x), x.stride(0), x.stride(1), _lib.ptr(dt), dt.stride(0), dt.stride(1), _lib.ptr(z), zs[0],
             zs[1], _lib.ptr(Bm), Bm.stride(0), Bm.stride(1), _lib.ptr(Cm), Cm.stride(0), Cm.stride(1),
             _lib.ptr(A), _lib.ptr(D), _lib.ptr(dt_bias), _lib.ptr(out), out.stride(0), out.stride(1),
-            _lib.ptr(state), _lib.ptr(sumdt), _lib.ptr(h0), B, L, Dm, _lib.stream()), "nx_selective_scan_fwd")
-        ctx.save_for_backward(x, dt, A, Bm, Cm, D, z, dt_bias, sumdt, h0)
+            _lib.ptr(state), _lib.ptr(sumdt), _lib.ptr(ckpt), B, L, Dm, _lib.stream()), "nx_selective_scan_fwd")
+        ctx.save_for_backward(x, dt, A, Bm, Cm, D, z, dt_bias, ckpt)
         return out
 
     @staticmethod
     def backward(ctx, gout):
-        x, dt, A, Bm, Cm, D, z, dt_bias, sumdt, h0 = ctx.saved_tensors
+        x, dt, A, Bm, Cm, D, z, dt_bias, ckpt = ctx.saved_tensors
         L_ = _lib.lib(x)
         B, L, Dm = x.shape
         dev = x.device
         if gout.stride(2) != 1:
             gout = gout.contiguous()
-        nc = L_.nx_scan_chunks(L)
-        nb = L_.nx_scan_channel_blocks(Dm)
+        nc = L_.nx_scan_chunks(B, L, Dm, 1)
         dx = torch.empty((L, B, Dm), device=dev, dtype=x.dtype).transpose(0, 1)
         ddt = torch.empty((L, B, Dm), device=dev, dtype=x.dtype).transpose(0, 1)
         dz = torch.empty((L, B, Dm), device=dev, dtype=x.dtype).transpose(0, 1) if z is not None else None
-        part = torch.empty((nb, B, L, 32), device=dev, dtype=torch.float32)
-        dA = torch.zeros((Dm, 16), device=dev, dtype=torch.float32)
-        dD = torch.zeros(Dm, device=dev, dtype=torch.float32) if D is not None else None
-        dbias = torch.zeros(Dm, device=dev, dtype=torch.float32)
-        E = torch.empty((B, nc, Dm, 16), device=dev, dtype=torch.float32)
+        dB, dC = (torch.empty((B, L, 16), device=dev, dtype=x.dtype) for _ in range(2))
+        part = torch.empty((L_.nx_scan_channel_blocks(Dm), B, L, 32), device=dev, dtype=torch.float32)
+        sums = torch.zeros(Dm * 18, device=dev, dtype=torch.float32)           # dA [Dm, 16], dD [Dm], d dt_bias [Dm]
+        dA, dD, dbias = sums[:16 * Dm].view(Dm, 16), sums[16 * Dm:17 * Dm], sums[17 * Dm:]
+        dD = dD if D is not None else None
+        state = sumdt = None
+        if nc > 1:
+            state = torch.empty((B, nc, Dm, 16), device=dev, dtype=torch.float32)
+            sumdt = torch.empty((B, nc, Dm), device=dev, dtype=torch.float32)
         zs = (z.stride(0), z.stride(1)) if z is not None else (0, 0)
-        LAUNCHES["n"] += 2 if nc > 1 else 1
+        LAUNCHES["n"] += 3 if nc > 1 else 2
         _lib.check(L_.nx_selective_scan_bwd(
             _lib.ptr(x), x.stride(0), x.stride(1), _lib.ptr(dt), dt.stride(0), dt.stride(1), _lib.ptr(z), zs[0],
             zs[1], _lib.ptr(Bm), Bm.stride(0), Bm.stride(1), _lib.ptr(Cm), Cm.stride(0), Cm.stride(1),
             _lib.ptr(A), _lib.ptr(D), _lib.ptr(dt_bias), _lib.ptr(gout), gout.stride(0), gout.stride(1),
-            _lib.ptr(dx), _lib.ptr(ddt), _lib.ptr(dz), dx.stride(0), dx.stride(1), _lib.ptr(part), _lib.ptr(dA),
-            _lib.ptr(dD), _lib.ptr(dbias), _lib.ptr(sumdt), _lib.ptr(h0), _lib.ptr(E), B, L, Dm, _lib.stream()),
-            "nx_selective_scan_bwd")
-        bc = part.sum(0)
-        dB = bc[..., :16].to(Bm.dtype)
-        dC = bc[..., 16:].to(Cm.dtype)
-        return dx, ddt, dA, dB, dC, dD, dz, dbias
+            _lib.ptr(dx), _lib.ptr(ddt), _lib.ptr(dz), dx.stride(0), dx.stride(1), _lib.ptr(dB), _lib.ptr(dC),
+            _lib.ptr(part), _lib.ptr(dA), _lib.ptr(dD), _lib.ptr(dbias), _lib.ptr(ckpt), _lib.ptr(state),
+            _lib.ptr(sumdt), B, L, Dm, _lib.stream()), "nx_selective_scan_bwd")
+        return dx, ddt, dA, dB.to(Bm.dtype), dC.to(Cm.dtype), dD, dz, dbias
 
 
 def selective_scan(x, dt, A, Bm, Cm, D=None, z=None, dt_bias=None):
@@ -157,6 +160,9 @@ def selective_scan(x, dt, A, Bm, Cm, D=None, z=None, dt_bias=None):
             raise _lib.KernelError("selective_scan: CUDA path needs bf16 activations and d_state == 16")
         if dt_bias is None:
             dt_bias = torch.zeros(x.shape[2], device=x.device, dtype=torch.float32)
-        return _ScanFn.apply(x, dt, A.float().contiguous(), Bm, Cm, None if D is None else D.float().contiguous(),
+        A = A.float().contiguous()
+        if A.data_ptr() % 16:           # the kernels read a channel's states 16 bytes at a time
+            A = A.clone()
+        return _ScanFn.apply(x, dt, A, Bm, Cm, None if D is None else D.float().contiguous(),
                              z, dt_bias.float().contiguous())
     return selective_scan_reference(x, dt, A, Bm, Cm, D, z, dt_bias)

@@ -100,3 +100,54 @@ def test_selective_scan_kernel(L, D, use_z):
         scale = r.grad.abs().max().item() + 1e-6
         err = (a.grad.float() - r.grad).abs().max().item()
         assert err <= 0.03 * scale + 1e-3, f"grad {n}: err {err} vs scale {scale}"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("L,D,W,off", [(1, 8, 4, 0), (15, 64, 4, 0), (67, 264, 2, 0), (129, 40, 4, 4), (33, 36, 3, 0),
+                                       (130, 8, 1, 2)])
+def test_conv1d_silu_tiles_and_alignments(L, D, W, off, dtype):
+    """Time-tile remainders, and channel counts / offsets that the 8- and 4-channel forms take or leave to the
+    one-channel form."""
+    from gpt_neox_b200.ops.mamba import causal_conv1d_silu, causal_conv1d_silu_reference
+    torch.manual_seed(3)
+    x = torch.randn(L, 2, D + 8, device="cuda").to(dtype)[..., off:off + D].transpose(0, 1).detach().requires_grad_(True)
+    w = (torch.randn(D, W, device="cuda") * 0.5).to(dtype).requires_grad_(True)
+    b = torch.randn(D, device="cuda").to(dtype).requires_grad_(True)
+    g = torch.randn(2, L, D, device="cuda").to(dtype)
+    y = causal_conv1d_silu(x, w, b)
+    got = torch.autograd.grad(y, (x, w, b), g)
+    ref = [t.detach().float().requires_grad_(True) for t in (x, w, b)]
+    yr = causal_conv1d_silu_reference(*ref)
+    want = torch.autograd.grad(yr, ref, g.float())
+    eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -11
+    for a, r in zip((y,) + got, (yr,) + want):                  # one rounding to 16 bits; fp32 sums on both sides
+        assert (a.float() - r).abs().max().item() <= 2 * eps * r.abs().max().item() + 1e-4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,L,D", [(1, 1, 32), (2, 31, 40), (1, 33, 36), (1, 700, 64), (2, 257, 8), (40, 96, 136)])
+def test_selective_scan_blocks_and_chunks(B, L, D, dtype):
+    """Block and chunk remainders, one chunk (many channels) and many (few channels), channel counts that the 16-byte
+    staging takes or not; forward with and without the states for the backward."""
+    from gpt_neox_b200.ops.mamba import selective_scan, selective_scan_reference
+    torch.manual_seed(6)
+    mk = lambda *s: (torch.randn(*s, device="cuda") * 0.5).to(dtype)
+    xz, bc = mk(L, B, 2 * D), mk(L, B, 40)
+    x, z, dt = xz[..., :D].transpose(0, 1), xz[..., D:].transpose(0, 1), mk(L, B, D).transpose(0, 1)
+    Bm, Cm = bc[..., 3:19].transpose(0, 1), bc[..., 19:35].transpose(0, 1)
+    A, Dp = -(torch.rand(D, 16, device="cuda") * 4 + 0.5), torch.randn(D, device="cuda")
+    dtb = torch.randn(D, device="cuda") * 0.5 - 2.0
+    leaves = [t.detach().requires_grad_(True) for t in (x, dt, A, Bm, Cm, Dp, z, dtb)]
+    ref = [t.detach().float().clone().requires_grad_(True) for t in leaves]
+    g = mk(B, L, D)
+    y = selective_scan(*leaves)
+    got = torch.autograd.grad(y, leaves, g)
+    yr = selective_scan_reference(*ref)
+    want = torch.autograd.grad(yr, ref, g.float())
+    eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -11
+    for a, r in zip((y,) + got, (yr,) + want):
+        assert (a.float() - r).abs().max().item() <= 2 * eps * r.abs().max().item() + 1e-4
+    with torch.no_grad():
+        assert torch.equal(selective_scan(*leaves), y)
