@@ -1,0 +1,223 @@
+// C[M, N] = epilogue(A[M, K] * W[N, K]^T) for few rows M (generation steps, short prompts) on tcgen05.
+//
+// Bound by reading W once.  The 128 x 256 tiles of gemm_tcgen05.cu give such a product ceil(N / 256) CTAs, each walking
+// the whole reduction: 16 CTAs of 148 SMs for N = 4096.  Here the roles are swapped: W supplies the 128-row operand of
+// the MMA and the few rows of A its N operand (NX = M rounded up to 16 .. 256), so no MMA row is padding, and the
+// reduction is cut over the CTAs of a cluster until about two CTAs per SM stream W.  The partial tiles (fp32) meet in
+// distributed shared memory in rank order: one launch, no workspace, a result that does not depend on timing.
+//
+// 4 rows x (4096 -> 22016, 11008 -> 4096): 54 us for both, 5.0 TB/s of weights (164 us before, 1.6 TB/s).
+//
+// 192 threads: warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 epilogue.  A TMEM lane is a row of W, i.e. a column
+// of C, so a warp's store of one row of C is 32 consecutive elements.
+#include "gemm_skinny.h"
+
+#include <cooperative_groups.h>
+
+namespace cg = cooperative_groups;
+
+namespace nx {
+
+constexpr int SK_BW = 128;   // rows of W per tile
+constexpr int SK_BK = 64;
+constexpr int SK_THREADS = 192;
+constexpr int SK_MAX_SPLITS = 8;
+
+// the epilogue bits this kernel knows (same values as in gemm_tcgen05.cu)
+enum : int {
+  SK_BIAS = 1, SK_GELU_ERF = 2, SK_GELU_TANH = 4, SK_AUX_OUT = 8, SK_RESIDUAL = 64, SK_SCALE = 512, SK_AUX_DERIV = 1024
+};
+
+template <int NX, int STAGES>
+struct SkinnySmem {
+  static constexpr int W_BYTES = SK_BW * SK_BK * 2;
+  static constexpr int X_BYTES = NX * SK_BK * 2;
+  static constexpr int STAGE = W_BYTES + X_BYTES;
+  static constexpr int PART = NX * SK_BW * 4;               // the fp32 partial tile, over the drained ring
+  static constexpr int RING = STAGES * STAGE > PART ? STAGES * STAGE : PART;
+  static constexpr int BAR_OFF = RING;                      // full[STAGES], empty[STAGES], done, TMEM base
+  static constexpr int DYN = BAR_OFF + (2 * STAGES + 2) * 8 + 1024;
+};
+
+// One element of C (row m, column n) from its accumulator value.
+__device__ __forceinline__ void skinny_store(const SkinnyParams& p, int m, int n, float v, float bias) {
+  if (p.flags & SK_SCALE) v *= p.alpha;
+  v += bias;
+  if (p.flags & SK_AUX_OUT) {
+    float d = v;
+    if (p.flags & SK_AUX_DERIV) {       // derivative out, activation in place
+      const float x = v;
+      if (p.flags & SK_GELU_TANH) gelu_tanh_both(x, v, d);
+      else gelu_erf_both(x, v, d);
+    }
+    p.aux_out[m * p.ld_aux + n] = float_to_h16(d);
+  }
+  if (!(p.flags & SK_AUX_DERIV)) {
+    if (p.flags & SK_GELU_ERF) v = gelu_erf(v);
+    else if (p.flags & SK_GELU_TANH) v = gelu_tanh(v);
+  }
+  if (p.flags & SK_RESIDUAL) v += h16_to_float(p.residual[m * p.ld_aux + n]);
+  p.C[m * p.ldc + n] = float_to_h16(v);
+}
+
+template <int NX, int STAGES>
+__global__ void __launch_bounds__(SK_THREADS)
+gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const SkinnyParams p) {
+  using L = SkinnySmem<NX, STAGES>;
+  constexpr uint32_t TMEM_COLS = NX < 32 ? 32 : NX;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* sgen = smem_raw + (sbase - smem_u32(smem_raw));
+  auto full_bar = [&](int s) { return sbase + L::BAR_OFF + 8u * s; };
+  auto empty_bar = [&](int s) { return sbase + L::BAR_OFF + 8u * (STAGES + s); };
+  const uint32_t done_bar = sbase + L::BAR_OFF + 8u * (2 * STAGES);
+  const uint32_t tmem_slot = done_bar + 8u;
+  volatile uint32_t* tmem_slot_gen = reinterpret_cast<volatile uint32_t*>(sgen + L::BAR_OFF + 8 * (2 * STAGES + 1));
+  cg::cluster_group cluster = cg::this_cluster();
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nsplit = gridDim.x, split = blockIdx.x;         // the cluster spans the x dimension
+  const int n0 = blockIdx.y * SK_BW;
+  const int num_kb = (p.K + SK_BK - 1) / SK_BK;
+  const int kb0 = static_cast<int>(static_cast<long long>(num_kb) * split / nsplit);
+  const int kb1 = static_cast<int>(static_cast<long long>(num_kb) * (split + 1) / nsplit);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(empty_bar(s), 1);
+    }
+    mbar_init(done_bar, 1);
+    fence_barrier_init();
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = *tmem_slot_gen;
+  bool aborted = false;
+
+  if (warp == 0) {
+    if (elect_one()) {
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const int i = kb - kb0, st = i % STAGES;
+        if (!mbar_wait(empty_bar(st), ((i / STAGES) & 1) ^ 1, p.err, 70)) { aborted = true; break; }
+        mbar_expect_tx(full_bar(st), L::STAGE);
+        tma_load_2d(sbase + st * L::STAGE, &tmW, full_bar(st), kb * SK_BK, n0);
+        tma_load_2d(sbase + st * L::STAGE + L::W_BYTES, &tmX, full_bar(st), kb * SK_BK, 0);
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      constexpr uint32_t idesc = umma_idesc_bf16(SK_BW, NX, 0, 0);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const int i = kb - kb0, st = i % STAGES;
+        if (!mbar_wait(full_bar(st), (i / STAGES) & 1, p.err, 71)) { aborted = true; break; }
+        tc_fence_after_sync();
+        const uint32_t w = sbase + st * L::STAGE, x = w + L::W_BYTES;
+#pragma unroll
+        for (int k = 0; k < SK_BK / 16; ++k)
+          umma_bf16_ss(tmem, umma_smem_desc_sw128(w + k * 32, 0, 1024), umma_smem_desc_sw128(x + k * 32, 0, 1024), idesc,
+                       (i | k) != 0 ? 1u : 0u);
+        umma_commit(empty_bar(st));
+      }
+      if (!aborted) umma_commit(done_bar);
+    }
+  }
+  // ---- epilogue warps: the accumulator, then C or the partial tile
+  const int col = (warp & 3) * 32 + lane;                   // row of W in the tile == TMEM lane
+  const int n = n0 + col;
+  float* part = reinterpret_cast<float*>(sgen);             // [NX][SK_BW]
+  float bias = 0.f;
+  if (warp >= 2) {
+    aborted = !__all_sync(0xffffffffu, mbar_wait(done_bar, 0, p.err, 72));
+    tc_fence_after_sync();
+    if ((p.flags & SK_BIAS) && n < p.N) bias = h16_to_float(p.bias[n]);
+    if (!aborted) {
+#pragma unroll 1
+      for (int c = 0; c < NX && c < p.M; c += 16) {
+        uint32_t r[16];
+        tmem_ld_32x32b_x16(tmem + c + (static_cast<uint32_t>((warp & 3) * 32) << 16), r);
+        tmem_ld_wait();
+        if (nsplit == 1) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (c + j < p.M && n < p.N) skinny_store(p, c + j, n, __uint_as_float(r[j]), bias);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) part[(c + j) * SK_BW + col] = __uint_as_float(r[j]);
+        }
+      }
+    }
+  }
+  __syncwarp();
+  if (aborted) {
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);       // copies in flight land before the shared memory goes away
+  }
+  if (nsplit > 1) {
+    cluster.sync();
+    if (warp >= 2 && !aborted && n < p.N) {
+      for (int m = split; m < p.M; m += nsplit) {
+        float v = 0.f;
+        for (int r = 0; r < nsplit; ++r) v += cluster.map_shared_rank(part, r)[m * SK_BW + col];
+        skinny_store(p, m, n, v, bias);
+      }
+    }
+    cluster.sync();                                         // nobody leaves while its partial tile may still be read
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem, TMEM_COLS);
+  }
+}
+
+template <int NX, int STAGES>
+static int launch_skinny(const void* A, const void* B, long long lda, long long ldb, const SkinnyParams& p,
+                         cudaStream_t stream) {
+  using L = SkinnySmem<NX, STAGES>;
+  auto kern = gemm_skinny_kernel<NX, STAGES>;
+  static bool configured = false;
+  if (!configured) {
+    NX_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::DYN));
+    configured = true;
+  }
+  CUtensorMap tmW, tmX;
+  if (!make_tma_2d(&tmW, B, p.N, p.K, ldb * 2, SK_BW, SK_BK, 2)) return NX_ERR_ARG;
+  if (!make_tma_2d(&tmX, A, p.M, p.K, lda * 2, NX, SK_BK, 2)) return NX_ERR_ARG;
+  const int tiles = (p.N + SK_BW - 1) / SK_BW, num_kb = (p.K + SK_BK - 1) / SK_BK;
+  // splits: until two CTAs per SM are in flight, with at least four 64-wide steps each
+  int splits = 1;
+  while (splits < SK_MAX_SPLITS && tiles * splits * 2 <= 2 * sm_count() && num_kb >= splits * 2 * 4) splits *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(splits, tiles, 1);
+  cfg.blockDim = dim3(SK_THREADS);
+  cfg.dynamicSmemBytes = L::DYN;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = splits;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  NX_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tmW, tmX, p));
+  return NX_OK;
+}
+
+int gemm_skinny_launch(const void* A, const void* B, long long lda, long long ldb, const SkinnyParams& p,
+                       cudaStream_t stream) {
+  // ring depths: two CTAs fit an SM's shared memory up to NX = 128
+  if (p.M <= 16) return launch_skinny<16, 6>(A, B, lda, ldb, p, stream);
+  if (p.M <= 32) return launch_skinny<32, 5>(A, B, lda, ldb, p, stream);
+  if (p.M <= 64) return launch_skinny<64, 4>(A, B, lda, ldb, p, stream);
+  if (p.M <= 128) return launch_skinny<128, 3>(A, B, lda, ldb, p, stream);
+  return launch_skinny<256, 4>(A, B, lda, ldb, p, stream);
+}
+
+}  // namespace nx

@@ -22,6 +22,7 @@
 #include <string.h>
 
 #include "common.h"
+#include "gemm_skinny.h"
 #include "ptx.cuh"
 
 namespace nx {
@@ -688,7 +689,20 @@ struct CommArgs {
   const int* tile_expert = nullptr;
   const int* row_offsets = nullptr;
   long long c_stride = 0;
+  bool skinny = false;   // few rows: gemm_skinny_tcgen05.cu
 };
+
+// Whether a product goes to the few-rows kernel: its layouts and epilogues, and up to 64 rows always (a generation step;
+// 4 rows of the 7B gated MLP: 164 -> 54 us for its two GEMMs), up to 256 where the tiles here would leave half the SMs
+// without one.
+static bool skinny_better(int M, int N, int transA, int transB, int flags) {
+  using namespace nx;
+  constexpr int known = EPI_BIAS | EPI_GELU_ERF | EPI_GELU_TANH | EPI_AUX_OUT | EPI_AUX_DERIV | EPI_RESIDUAL | EPI_SCALE;
+  if (transA || transB || (flags & ~known) != 0 || M > SKINNY_MAX_M) return false;
+  const int BN = N <= 128 ? 128 : 256;
+  const long long tiles = static_cast<long long>((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+  return M <= 64 || 2 * tiles <= sm_count();
+}
 
 static int gemm_common(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                        long long ldc, int transA, int transB, const void* bias, const void* aux_in, void* aux_out,
@@ -707,6 +721,18 @@ static int gemm_common(const void* A, const void* B, void* C, int M, int N, int 
   if (flags & EPI_AUX_OUT) NX_REQUIRE(aux_out != nullptr && ld_aux % 8 == 0, "gemm: aux_out");
   if (flags & EPI_RESIDUAL) NX_REQUIRE(residual != nullptr && ld_aux % 8 == 0, "gemm: residual");
 
+  if (ca.skinny) {
+    SkinnyParams q;
+    q.M = M; q.N = N; q.K = K;
+    q.C = static_cast<h16*>(C); q.ldc = ldc;
+    q.bias = static_cast<const h16*>(bias);
+    q.aux_out = static_cast<h16*>(aux_out);
+    q.residual = static_cast<const h16*>(residual);
+    q.ld_aux = ld_aux;
+    q.flags = flags; q.alpha = alpha;
+    q.err = device_error_word();
+    return gemm_skinny_launch(A, B, lda, ldb, q, stream);
+  }
   const int BN = (N <= 128) ? 128 : 256;
   GemmParams p;
   memset(&p, 0, sizeof(p));
@@ -790,6 +816,7 @@ NX_API int NX_SYM(nx_gemm_bf16)(const void* A, const void* B, void* C, int M, in
                         const void* aux_in, void* aux_out, const void* residual, long long ld_aux,
                         int flags, float alpha, void* stream_) {
   CommArgs ca;
+  ca.skinny = skinny_better(M, N, transA, transB, flags);
   return gemm_common(A, B, C, M, N, K, lda, ldb, ldc, transA, transB, bias, aux_in, aux_out, residual, ld_aux,
                      flags, alpha, ca, static_cast<cudaStream_t>(stream_));
 }

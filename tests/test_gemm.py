@@ -93,3 +93,28 @@ def test_linear_autograd():
 def test_no_device_error():
     from gpt_neox_b200.ops import _lib
     assert _lib.read_device_error(clear=False) == 0
+
+
+@pytest.mark.parametrize("M", [1, 15, 16, 17, 33, 64, 65, 128, 129, 256])
+@pytest.mark.parametrize("N,K", [(8, 8), (136, 72), (1000, 520), (768, 3072), (4096, 4096)])
+def test_gemm_few_rows(M, N, K):
+    """The few-rows kernel: every width of its row operand, tile remainders in N and K, one to eight splits of K; the
+    epilogues a generation step and a short prompt use."""
+    from gpt_neox_b200.ops.gemm import gemm
+    torch.manual_seed(5)
+    base = torch.randn(M, K + 8, device="cuda", dtype=DT)
+    a, w = base[:, :K], torch.randn(N, K, device="cuda", dtype=DT) * K ** -0.5      # a: rows further apart than K
+    _check(gemm(a, w), _ref(a, w, False, False), K)
+    bias, res = torch.randn(N, device="cuda", dtype=DT), torch.randn(M, N, device="cuda", dtype=DT)
+    pre = a.float() @ w.float().t() * 0.5 + bias.float()
+    _check(gemm(a, w, bias=bias, residual=res, alpha=0.5), pre + res.float(), K)
+    pre = pre.requires_grad_(True)
+    for kind, approx in (("erf", "none"), ("tanh", "tanh")):
+        act = torch.nn.functional.gelu(pre, approximate=approx)
+        (d,) = torch.autograd.grad(act.sum(), pre)
+        aux = torch.empty(M, N, device="cuda", dtype=DT)
+        _check(gemm(a, w, bias=bias, gelu=kind, alpha=0.5, aux_out=aux, aux_deriv=True), act.detach(), K)
+        _check(aux, d, K)
+        _check(gemm(a, w, bias=bias, gelu=kind, alpha=0.5, aux_out=aux), act.detach(), K)
+        _check(aux, pre.detach(), K)
+        _check(gemm(a, w, bias=bias, gelu=kind, alpha=0.5), act.detach(), K)
