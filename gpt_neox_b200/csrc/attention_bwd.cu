@@ -156,13 +156,14 @@ __device__ __forceinline__ void mma_nt(uint32_t d_tmem, uint32_t a, uint32_t b) 
 }
 // D[128 x DP] (+)= A_tmem[128 x 128 (bf16, 64 columns)] * B[128 x DP] with B's head dim contiguous
 // (MN-major B operand).
-// KR: rows of B (the contraction length), 128 or 64; b points at the first of them.
-template <int DP, int KR = AB>
+// KR: rows of B (the contraction length), 128 or 64; b points at the first of them.  SPLIT: every 16 columns of A (32
+// rows of B) start 32 columns apart instead of lying back to back.
+template <int DP, int KR = AB, bool SPLIT = false>
 __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b, bool accumulate) {
   constexpr uint32_t idesc = umma_idesc_bf16(AB, DP, 0, 1);
 #pragma unroll
   for (int k = 0; k < KR / 16; ++k) {
-    umma_bf16_ts(d_tmem, a_tmem + k * 8, umma_smem_desc_sw128(b + k * 2048, AB * 128, 1024), idesc,
+    umma_bf16_ts(d_tmem, a_tmem + (SPLIT ? (k >> 1) * 32 + (k & 1) * 8 : k * 8), umma_smem_desc_sw128(b + k * 2048, AB * 128, 1024), idesc,
                  (accumulate || k != 0) ? 1u : 0u);
   }
 }
@@ -175,8 +176,11 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_
 // The MMA warp issues S / dP of half u + 1 before it waits for dS of half u, so the tensor core computes the next
 // half (and dQ += dS K of the previous one) while the element-wise warps work on the current one; without PIPE
 // the tensor core and the element-wise warps take turns.
+// GEN (this kernel and the next): ALiBi and block-sparse layouts; without them a block that needs a mask differs from one
+// that does not by one select per element (batch 4, 32 heads, 2048 x 128 causal: dQ 318 -> 288 us, dK / dV, with its
+// barriers gone, 334 -> 323 us).
 // ------------------------------------------------------------------------------------------------
-template <int DP, bool DROP, int HALVES, bool PIPE>
+template <int DP, bool DROP, int HALVES, bool PIPE, bool GEN>
 __global__ void __launch_bounds__(ab_threads(HALVES), 1)
     attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -208,7 +212,7 @@ __global__ void __launch_bounds__(ab_threads(HALVES), 1)
   const int nblk = max((kv_end + AB - 1) / AB - jb, 0);
   // block-sparse layouts: key tiles without a live block for this query tile are skipped by every role; ring
   // stages and barrier phases count the live tiles
-  auto tile_live = [&](int kt) { return p.blk_any == nullptr || p.blk_any[static_cast<long long>(qt) * p.blk_nkt + kt] != 0; };
+  auto tile_live = [&](int kt) { return !GEN || p.blk_any == nullptr || p.blk_any[static_cast<long long>(qt) * p.blk_nkt + kt] != 0; };
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < NUSED; ++i) {
@@ -319,7 +323,7 @@ __global__ void __launch_bounds__(ab_threads(HALVES), 1)
     const long long stat_idx = (static_cast<long long>(batch) * p.H + head) * p.Sq_pad + qi;
     const float lse2 = p.lse[stat_idx];     // +inf for rows past Sq -> P = 0
     const float delta = p.delta[stat_idx];
-    const float slope2 = p.alibi != nullptr ? p.alibi[head] * LOG2E : 0.f;
+    const float slope2 = GEN && p.alibi != nullptr ? p.alibi[head] * LOG2E : 0.f;
     int nlive = 0;
     for (int t = 0; t < nblk; ++t) {
       if (!tile_live(jb + t)) continue;
@@ -327,10 +331,10 @@ __global__ void __launch_bounds__(ab_threads(HALVES), 1)
       const int st = i & 1;
       const int k0 = (jb + t) * AB;
       uint32_t bits = 0xffffffffu;
-      if (p.blk_rows != nullptr)
+      if (GEN && p.blk_rows != nullptr)
         bits = row_ok ? p.blk_rows[static_cast<long long>(qi) * p.blk_nkt + (jb + t)] : 0u;
       const uint32_t full_bits = (1u << (AB >> p.blk_shift)) - 1u;
-      const bool blk_partial = p.blk_rows != nullptr && !__all_sync(0xffffffffu, (bits & full_bits) == full_bits);
+      const bool blk_partial = GEN && p.blk_rows != nullptr && !__all_sync(0xffffffffu, (bits & full_bits) == full_bits);
       if (!PIPE) {
         if (!mbar_wait(bar(SDP_FULL, 0), i & 1, p.err, 38)) { aborted = true; break; }
         if (i >= 2 && !mbar_wait(bar(DQ_DONE, st), ((i - 2) >> 1) & 1, p.err, 39)) { aborted = true; break; }
@@ -369,7 +373,14 @@ __global__ void __launch_bounds__(ab_threads(HALVES), 1)
           }
         }
         uint32_t pk[16];
-        if (!need_mask && p.alibi == nullptr) {
+        if (!GEN || (!need_mask && p.alibi == nullptr)) {
+          if (!GEN && need_mask) {      // masked scores: -inf, probability 0
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const int idx = c * 32 + j;
+              if (idx < lo || idx > hi) sv[j] = __float_as_uint(p.scale_log2 < 0.f ? INFINITY : -INFINITY);
+            }
+          }
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
             // the softmax scale of dS is applied once, to dQ, in the epilogue
@@ -470,9 +481,12 @@ __global__ void __launch_bounds__(ab_threads(HALVES), 1)
 // own S^T / dP^T buffers (S^T_h at [64 h, 64 h + 64), dP^T_h at [128 + 64 h, ...)) and their own barriers.  The MMA
 // warp issues S^T / dP^T of half u + 1 before it waits for P^T / dS^T of half u, so the tensor core works on the
 // next half (and on dV / dK of the previous one) while the element-wise warps are busy with the current one;
-// without PIPE the four phases of a step run one after the other.
+// without PIPE the four phases of a step run one after the other.  In the pipelined form a warp writes its 16-bit
+// results over the first half of the 32 columns it read itself (the MMA takes its A operand in pieces of 16 query rows,
+// each with its own column address), so the two warps of a quadrant never touch each other's columns and need no
+// barrier between reading and writing.
 // ------------------------------------------------------------------------------------------------
-template <int DP, bool DROP, int HALVES, bool PIPE>
+template <int DP, bool DROP, int HALVES, bool PIPE, bool GEN>
 __global__ void __launch_bounds__(ab_threads(HALVES), 1)
     attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                         const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -504,7 +518,7 @@ __global__ void __launch_bounds__(ab_threads(HALVES), 1)
   const int nsteps = nq * group;
   // block-sparse layouts: query tiles without a live block for this key tile are skipped by every role
   auto step_live = [&](int t) {
-    return p.blk_any == nullptr || p.blk_any[static_cast<long long>(ib + t % nq) * p.blk_nkt + kt] != 0;
+    return !GEN || p.blk_any == nullptr || p.blk_any[static_cast<long long>(ib + t % nq) * p.blk_nkt + kt] != 0;
   };
 
   if (threadIdx.x == 0) {
@@ -569,8 +583,8 @@ __global__ void __launch_bounds__(ab_threads(HALVES), 1)
           if (u + 1 < nsub && !issue_m1(u + 1)) { aborted = true; break; }
           if (!mbar_wait(bar(PT_FULL, h), t & 1, p.err, 54)) { aborted = true; break; }
           tc_fence_after_sync();
-          mma_ts<DP, 64>(T_DV, T_ST + h * 64, tile(4 + st) + h * (64 * 128), u != 0);    // dV += P^T_h dO_h
-          mma_ts<DP, 64>(T_DK, T_DPT + h * 64, tile(2 + st) + h * (64 * 128), u != 0);   // dK += dS^T_h Q_h
+          mma_ts<DP, 64, true>(T_DV, T_ST + h * 64, tile(4 + st) + h * (64 * 128), u != 0);    // dV += P^T_h dO_h
+          mma_ts<DP, 64, true>(T_DK, T_DPT + h * 64, tile(2 + st) + h * (64 * 128), u != 0);   // dK += dS^T_h Q_h
           if (h == 1) umma_commit(bar(Q_EMPTY, st));
         }
         n = nl;
@@ -605,7 +619,7 @@ __global__ void __launch_bounds__(ab_threads(HALVES), 1)
       const int t = nlive++;
       const int head = kv_head * group + tt / nq;
       const int q0 = (ib + tt % nq) * AB;
-      const float slope2 = p.alibi != nullptr ? p.alibi[head] * LOG2E : 0.f;
+      const float slope2 = GEN && p.alibi != nullptr ? p.alibi[head] * LOG2E : 0.f;
       const int st = t & 1;
       // lse / delta of this query block were bulk-copied next to the Q / dO tiles
       bool ok = mbar_wait(bar(Q_FULL, st), (t >> 1) & 1, p.err, 57);
@@ -623,10 +637,10 @@ __global__ void __launch_bounds__(ab_threads(HALVES), 1)
       int lo = p.causal ? rel0 : -(1 << 30);
       int hi = p.window >= 0 ? rel0 + p.window : (1 << 30);
       if (!key_ok) hi = -(1 << 30);
-      const bool need_mask = __any_sync(0xffffffffu, lo > 0 || hi < AB - 1) || p.blk_rows != nullptr;
+      const bool need_mask = __any_sync(0xffffffffu, lo > 0 || hi < AB - 1) || (GEN && p.blk_rows != nullptr);
       const float bias0 = slope2 * static_cast<float>(rel0);
       const uint32_t kbit = 1u << (r >> p.blk_shift);      // this key row's sub-block within the key tile
-      const bool plain = !need_mask && p.alibi == nullptr;   // warp-uniform: no per-element compares in the hot path
+      const bool plain = !GEN || (!need_mask && p.alibi == nullptr);   // warp-uniform: no per-element compares in the hot path
       // P^T and dS^T (16 bit) go over the columns S^T and dP^T were read from, and the partner warp of this
       // quadrant reads the other half of those columns: both chunks of this warp are kept in registers until the
       // two warps have finished reading (named barrier of the quadrant's 64 threads), then everything is stored.
@@ -641,10 +655,10 @@ __global__ void __launch_bounds__(ab_threads(HALVES), 1)
       const int cbase = PIPE ? grp * 2 + half : (half * (2 / HALVES) + grp) * 2;
       // where this pass's chunks sit in TMEM: columns of the S^T buffer read / of the 16-bit result written
       const uint32_t rd0 = PIPE ? grp * 64 + half * 32 : cbase * 32;
-      const uint32_t wr0 = PIPE ? grp * 64 + half * 16 : cbase * 16;
+      const uint32_t wr0 = PIPE ? rd0 : cbase * 16;
       if (PIPE) {
         if (ok) ok = mbar_wait(bar(ST_FULL, grp), t & 1, p.err, 55);
-        if (!pair_all(ok, 5 + quad)) { aborted = true; break; }
+        if (!__all_sync(0xffffffffu, ok)) { aborted = true; break; }
         tc_fence_after_sync();
       }
       uint32_t pp_all[NCC][16], pd_all[NCC][16];
@@ -669,6 +683,13 @@ __global__ void __launch_bounds__(ab_threads(HALVES), 1)
           }
         }
         if (plain) {
+          if (!GEN && need_mask) {      // masked scores: -inf, probability 0
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const int idx = c * 32 + j;
+              if (idx < lo || idx > hi) sv[j] = __float_as_uint(p.scale_log2 < 0.f ? INFINITY : -INFINITY);
+            }
+          }
 #pragma unroll
           for (int j = 0; j < 32; j += 4) {
             const float4 l4 = v_lse[(c * 32 + j) >> 2];
@@ -716,7 +737,7 @@ __global__ void __launch_bounds__(ab_threads(HALVES), 1)
           }
         }
       }
-      if (HALVES == 2) asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory");
+      if (HALVES == 2 && !PIPE) asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory");
 #pragma unroll
       for (int cc = 0; cc < NCC; ++cc) {
         tmem_st_32x32b_x16(T_ST + wr0 + cc * 16 + lane_off, pp_all[cc]);
@@ -797,42 +818,41 @@ static bool bwd_map(CUtensorMap* m, const void* base, int B, int Hh, int S, int 
   return make_tma_4d(m, base, dims, strides, box, 2, true);
 }
 
+template <int DP, bool DROP, int HALVES, bool PIPE_Q, bool PIPE_K, bool GEN>
+static int launch_bwd_as(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
+                         const AttnBwdParams& p, cudaStream_t s) {
+  auto dq = attn_bwd_dq_kernel<DP, DROP, HALVES, PIPE_Q, GEN>;
+  auto dkv = attn_bwd_dkv_kernel<DP, DROP, HALVES, PIPE_K, GEN>;
+  static bool cfg = false;
+  if (!cfg) {
+    NX_CUDA_CHECK(cudaFuncSetAttribute(dq, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<DP>::DYN));
+    NX_CUDA_CHECK(cudaFuncSetAttribute(dkv, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<DP>::DYN));
+    cfg = true;
+  }
+  dq<<<dim3((p.Sq + AB - 1) / AB, p.H, p.B), ab_threads(HALVES), BwdSmem<DP>::DYN, s>>>(tq, tk, tv, tdo, p);
+  NX_LAUNCH_CHECK();
+  dkv<<<dim3((p.Sk + AB - 1) / AB, p.Hk, p.B), ab_threads(HALVES), BwdSmem<DP>::DYN, s>>>(tq, tk, tv, tdo, p);
+  NX_LAUNCH_CHECK();
+  return NX_OK;
+}
+
 template <int DP, bool DROP, int HALVES>
 static int launch_bwd_h(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                       const CUtensorMap& tdo, const AttnBwdParams& p, cudaStream_t s) {
-  static bool cfg = false;
-  if (!cfg) {
-    NX_CUDA_CHECK(cudaFuncSetAttribute(attn_bwd_dq_kernel<DP, DROP, HALVES, false>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<DP>::DYN));
-    NX_CUDA_CHECK(cudaFuncSetAttribute(attn_bwd_dq_kernel<DP, DROP, HALVES, HALVES == 2>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<DP>::DYN));
-    NX_CUDA_CHECK(cudaFuncSetAttribute(attn_bwd_dkv_kernel<DP, DROP, HALVES, false>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<DP>::DYN));
-    NX_CUDA_CHECK(cudaFuncSetAttribute(attn_bwd_dkv_kernel<DP, DROP, HALVES, HALVES == 2>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<DP>::DYN));
-    cfg = true;
-  }
-  dim3 gq((p.Sq + AB - 1) / AB, p.H, p.B);
-  static const bool serial_q = [] {        // NEOX_ATTN_DQ_PIPE=0: the unpipelined form
-    const char* e = getenv("NEOX_ATTN_DQ_PIPE");
+  constexpr bool PIPE = HALVES == 2;
+  auto off = [](const char* name) {
+    const char* e = getenv(name);
     return e != nullptr && atoi(e) == 0;
-  }();
-  if (HALVES == 2 && !serial_q)
-    attn_bwd_dq_kernel<DP, DROP, HALVES, HALVES == 2><<<gq, ab_threads(HALVES), BwdSmem<DP>::DYN, s>>>(tq, tk, tv, tdo, p);
-  else
-    attn_bwd_dq_kernel<DP, DROP, HALVES, false><<<gq, ab_threads(HALVES), BwdSmem<DP>::DYN, s>>>(tq, tk, tv, tdo, p);
-  NX_LAUNCH_CHECK();
-  dim3 gk((p.Sk + AB - 1) / AB, p.Hk, p.B);
-  static const bool serial = [] {        // NEOX_ATTN_DKV_PIPE=0: the unpipelined form
-    const char* e = getenv("NEOX_ATTN_DKV_PIPE");
-    return e != nullptr && atoi(e) == 0;
-  }();
-  if (HALVES == 2 && !serial)
-    attn_bwd_dkv_kernel<DP, DROP, HALVES, HALVES == 2><<<gk, ab_threads(HALVES), BwdSmem<DP>::DYN, s>>>(tq, tk, tv, tdo, p);
-  else
-    attn_bwd_dkv_kernel<DP, DROP, HALVES, false><<<gk, ab_threads(HALVES), BwdSmem<DP>::DYN, s>>>(tq, tk, tv, tdo, p);
-  NX_LAUNCH_CHECK();
-  return NX_OK;
+  };
+  static const bool serial_q = off("NEOX_ATTN_DQ_PIPE"), serial_k = off("NEOX_ATTN_DKV_PIPE");   // =0: unpipelined
+  if (PIPE && serial_q && serial_k) return launch_bwd_as<DP, DROP, HALVES, false, false, true>(tq, tk, tv, tdo, p, s);
+  if (PIPE && serial_q) return launch_bwd_as<DP, DROP, HALVES, false, PIPE, true>(tq, tk, tv, tdo, p, s);
+  if (PIPE && serial_k) return launch_bwd_as<DP, DROP, HALVES, PIPE, false, true>(tq, tk, tv, tdo, p, s);
+  // (a row without a visible key, possible for Sq > Sk, has lse = -inf: there a masked score must not reach the exponent;
+  //  a zero scale would turn a masked score into NaN)
+  if (!PIPE || DROP || p.alibi != nullptr || p.blk_rows != nullptr || p.Sq > p.Sk || p.scale == 0.f)
+    return launch_bwd_as<DP, DROP, HALVES, PIPE, PIPE, true>(tq, tk, tv, tdo, p, s);
+  return launch_bwd_as<DP, DROP, HALVES, PIPE, PIPE, false>(tq, tk, tv, tdo, p, s);
 }
 
 template <int DP, bool DROP>

@@ -146,7 +146,12 @@ __device__ __forceinline__ uint32_t pack_h16x2_alu(float lo, float hi) {
 // save); 1 = MUFU + integer packing; 2 = every second exp2 as the polynomial + integer packing
 // (NEOX_ATTN_EXP selects).
 // DROP: dropout on the probabilities (the row sum stays that of the undropped softmax).
-template <int DP, int EXPV, bool DROP, int BN, int HALVES>
+// GEN: ALiBi and block-sparse layouts.  Without them (and for a positive scale) masked scores are set to -inf as they
+// are and every block goes through the same scale / exp2 code; the general form keeps scaled logits in one branch and
+// raw scores in the other.  (Issue and latency of the softmax warps bound the kernel, not a pipe: batch 4, 32 heads, 2048
+// x 128 causal 189 us in the general form, 167 us without it and without the two waits per block that the order of the
+// MMAs already covers.)
+template <int DP, int EXPV, bool DROP, int BN, int HALVES, bool GEN>
 __global__ void __launch_bounds__(att_threads(HALVES), BN == 64 ? 2 : 1)
     attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const AttnFwdParams p) {
@@ -186,7 +191,7 @@ __global__ void __launch_bounds__(att_threads(HALVES), BN == 64 ? 2 : 1)
   // (the layout tables are kept per 128-key tile; a 64-key block looks up the tile it lies in)
   constexpr int KT_SHIFT = BN == 64 ? 1 : 0;
   auto tile_live = [&](int kt) {
-    return p.blk_any == nullptr || p.blk_any[static_cast<long long>(qt) * p.blk_nkt + (kt >> KT_SHIFT)] != 0;
+    return !GEN || p.blk_any == nullptr || p.blk_any[static_cast<long long>(qt) * p.blk_nkt + (kt >> KT_SHIFT)] != 0;
   };
 
   if (threadIdx.x == 0) {
@@ -276,7 +281,8 @@ __global__ void __launch_bounds__(att_threads(HALVES), BN == 64 ? 2 : 1)
         const int st = i & 1;
         const uint32_t ph = (i >> 1) & 1;
         if (!mbar_wait(bar(K_FULL, st), ph, p.err, 16)) { aborted = true; break; }
-        if (!mbar_wait(bar(S_EMPTY, st), ph ^ 1, p.err, 17)) { aborted = true; break; }
+        // (64-key shape: P_i lies over S_i and PV_i is issued before S_{i+2}, so its P_FULL wait has covered this)
+        if (BN == 128 && !mbar_wait(bar(S_EMPTY, st), ph ^ 1, p.err, 17)) { aborted = true; break; }
         tc_fence_after_sync();
         const uint32_t qb = sbase + L::Q_OFF, kb = sbase + L::K_OFF + st * L::KV_TILE;
 #pragma unroll
@@ -329,12 +335,12 @@ __global__ void __launch_bounds__(att_threads(HALVES), BN == 64 ? 2 : 1)
       const int k0 = (jb + t) * ATT_BN;
       // block-sparse: which 16..128-key sub-blocks of this key tile the row attends to
       uint32_t bits = 0xffffffffu;
-      if (p.blk_rows != nullptr) {
+      if (GEN && p.blk_rows != nullptr) {
         bits = qi < p.Sq ? p.blk_rows[static_cast<long long>(qi) * p.blk_nkt + ((jb + t) >> KT_SHIFT)] : 0u;
         if (BN == 64) bits >>= ((jb + t) & 1) * (64 >> p.blk_shift);      // the 64-key half of the 128-key tile
       }
       const uint32_t full_bits = (1u << max(1, ATT_BN >> p.blk_shift)) - 1u;
-      const bool blk_partial = p.blk_rows != nullptr && !__all_sync(0xffffffffu, (bits & full_bits) == full_bits);
+      const bool blk_partial = GEN && p.blk_rows != nullptr && !__all_sync(0xffffffffu, (bits & full_bits) == full_bits);
       if (!mbar_wait(bar(S_FULL, st), ph, p.err, 18)) { aborted = true; break; }
       tc_fence_after_sync();
       // One read of the whole score row into registers.
@@ -345,9 +351,23 @@ __global__ void __launch_bounds__(att_threads(HALVES), BN == 64 ? 2 : 1)
       // Does this block need per-element masking?  (warp-uniform decision)
       const bool need_mask = (k0 + ATT_BN > p.Sk) || (p.causal && k0 + ATT_BN - 1 > q0 + quad * 32 + off) ||
                              (p.window >= 0 && k0 < q0 + quad * 32 + 31 + off - p.window) || blk_partial;
-      const bool plain = !need_mask && p.alibi == nullptr;
+      const bool plain = !GEN || (!need_mask && p.alibi == nullptr);
       float mx;
-      if (plain) {
+      if (!GEN) {
+        if (need_mask) {
+          int hi = p.Sk - k0 - 1;
+          if (p.causal) hi = min(hi, qpos - k0);
+          const int lo = p.window >= 0 ? qpos - k0 - p.window : -(1 << 30);
+#pragma unroll
+          for (int c = 0; c < NC; ++c)
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const int idx = col0 + c * 32 + j;
+              if (idx < lo || idx > hi) sv[c][j] = __float_as_uint(-INFINITY);
+            }
+        }
+        mx = row_max_plain<NC>(sv) * p.scale_log2;
+      } else if (plain) {
         mx = row_max_plain<NC>(sv) * p.scale_log2;
       } else {
         // columns idx (0..127) of this block are alive for lo <= idx <= hi
@@ -395,8 +415,9 @@ __global__ void __launch_bounds__(att_threads(HALVES), BN == 64 ? 2 : 1)
         }
         tmem_st_wait();
       }
-      // P buffer `st` was last read by PV_{i-2}.
-      if (i >= 2) {
+      // P buffer `st` was last read by PV_{i-2}.  (64-key shape: PV_{i-2} was issued before S_i, whose completion this
+      // warp has waited for.)
+      if (BN == 128 && i >= 2) {
         if (!mbar_wait(bar(PV_DONE, st), ((i - 2) >> 1) & 1, p.err, 20)) { aborted = true; break; }
       }
       // probabilities (base 2), packed to bf16 and written to TMEM as the A operand of P V
@@ -432,7 +453,7 @@ __global__ void __launch_bounds__(att_threads(HALVES), BN == 64 ? 2 : 1)
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(bar(S_EMPTY, st));
+        if (BN == 128) mbar_arrive(bar(S_EMPTY, st));
         mbar_arrive(bar(P_FULL, st));
       }
     }
@@ -477,9 +498,10 @@ __global__ void __launch_bounds__(att_threads(HALVES), BN == 64 ? 2 : 1)
           }
         }
       }
-      if (row_ok && half == 0) {
-        // base-2 log-sum-exp of the scaled scores; rows are padded to a multiple of 128
-        const float lse2 = l > 0.f ? m_used + log2f(l) : -INFINITY;
+      if (half == 0) {
+        // base-2 log-sum-exp of the scaled scores; rows are padded to a multiple of 128 with +inf (the backward reads
+        // whole 128-row blocks: +inf makes the padding contribute zero probability)
+        const float lse2 = !row_ok ? INFINITY : l > 0.f ? m_used + log2f(l) : -INFINITY;
         p.lse[(static_cast<long long>(batch) * p.H + head) * p.Sq_pad + qi] = lse2;
       }
     }
@@ -510,7 +532,7 @@ static bool attn_map(CUtensorMap* m, const void* base, int B, int Hh, int S, int
 
 // q [B,H,Sq,D], k/v [B,Hk,Sk,D], o [B,H,Sq,D] as strided views (element strides for batch, head,
 // sequence; head dim contiguous); lse: fp32 [B,H,Sq_pad] (Sq rounded up to 128), receives the
-// base-2 log-sum-exp of the scaled scores for rows < Sq (the caller pre-fills it with +inf).  alibi: fp32 [H] or null.
+// base-2 log-sum-exp of the scaled scores for rows < Sq and +inf for the padding rows.  alibi: fp32 [H] or null.
 // window < 0: no sliding window.  D % 8 == 0, D <= 128.  dropout_p > 0: dropout on the probabilities with
 // the mask of dropout_patch() under `seed` (the backward must be given the same p and seed).
 // blk_rows / blk_any (both or neither): block-sparse layout tables, uint8 [Sq, ceil(Sk / 128)] and
@@ -573,10 +595,10 @@ NX_API int NX_SYM(nx_flash_attn_fwd)(const void* q, const void* k, const void* v
     const int v = e ? atoi(e) : 0;
     return v < 0 || v > 2 ? 0 : v;
   }();
-#define NX_ATTN_LAUNCH(DPV, EV, DR, BNV, HV)                                                                 \
+#define NX_ATTN_LAUNCH(DPV, EV, DR, BNV, HV, GE)                                                             \
   do {                                                                                                       \
     static bool cfg = false;                                                                                 \
-    auto kern = attn_fwd_kernel<DPV, EV, DR, BNV, HV>;                                                       \
+    auto kern = attn_fwd_kernel<DPV, EV, DR, BNV, HV, GE>;                                                   \
     if (!cfg) {                                                                                              \
       NX_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,                  \
                                          AttnSmem<DPV, BNV>::DYN));                                          \
@@ -586,33 +608,36 @@ NX_API int NX_SYM(nx_flash_attn_fwd)(const void* q, const void* k, const void* v
   } while (0)
   if (shape == 3) {
     if (drop) {
-      if (D <= 64) NX_ATTN_LAUNCH(64, 0, true, 64, 2);
-      else NX_ATTN_LAUNCH(128, 0, true, 64, 2);
+      if (D <= 64) NX_ATTN_LAUNCH(64, 0, true, 64, 2, true);
+      else NX_ATTN_LAUNCH(128, 0, true, 64, 2, true);
     } else if (D <= 64) {
-      NX_ATTN_LAUNCH(64, 0, false, 64, 2);
+      NX_ATTN_LAUNCH(64, 0, false, 64, 2, true);
     } else {
-      NX_ATTN_LAUNCH(128, 0, false, 64, 2);
+      NX_ATTN_LAUNCH(128, 0, false, 64, 2, true);
     }
   } else if (shape == 2) {
+    const bool gen = alibi != nullptr || blk_rows != nullptr || !(scale > 0.f);
     if (drop) {
-      if (D <= 64) NX_ATTN_LAUNCH(64, 0, true, 64, 1);
-      else NX_ATTN_LAUNCH(128, 0, true, 64, 1);
+      if (D <= 64) NX_ATTN_LAUNCH(64, 0, true, 64, 1, true);
+      else NX_ATTN_LAUNCH(128, 0, true, 64, 1, true);
     } else if (D <= 64) {
-      NX_ATTN_LAUNCH(64, 0, false, 64, 1);
+      if (gen) NX_ATTN_LAUNCH(64, 0, false, 64, 1, true);
+      else NX_ATTN_LAUNCH(64, 0, false, 64, 1, false);
     } else {
-      NX_ATTN_LAUNCH(128, 0, false, 64, 1);
+      if (gen) NX_ATTN_LAUNCH(128, 0, false, 64, 1, true);
+      else NX_ATTN_LAUNCH(128, 0, false, 64, 1, false);
     }
   } else if (drop) {
-    if (D <= 64) NX_ATTN_LAUNCH(64, 0, true, 128, 2);
-    else NX_ATTN_LAUNCH(128, 0, true, 128, 2);
+    if (D <= 64) NX_ATTN_LAUNCH(64, 0, true, 128, 2, true);
+    else NX_ATTN_LAUNCH(128, 0, true, 128, 2, true);
   } else if (D <= 64) {
-    if (expv == 0) NX_ATTN_LAUNCH(64, 0, false, 128, 2);
-    else if (expv == 1) NX_ATTN_LAUNCH(64, 1, false, 128, 2);
-    else NX_ATTN_LAUNCH(64, 2, false, 128, 2);
+    if (expv == 0) NX_ATTN_LAUNCH(64, 0, false, 128, 2, true);
+    else if (expv == 1) NX_ATTN_LAUNCH(64, 1, false, 128, 2, true);
+    else NX_ATTN_LAUNCH(64, 2, false, 128, 2, true);
   } else {
-    if (expv == 0) NX_ATTN_LAUNCH(128, 0, false, 128, 2);
-    else if (expv == 1) NX_ATTN_LAUNCH(128, 1, false, 128, 2);
-    else NX_ATTN_LAUNCH(128, 2, false, 128, 2);
+    if (expv == 0) NX_ATTN_LAUNCH(128, 0, false, 128, 2, true);
+    else if (expv == 1) NX_ATTN_LAUNCH(128, 1, false, 128, 2, true);
+    else NX_ATTN_LAUNCH(128, 2, false, 128, 2, true);
   }
 #undef NX_ATTN_LAUNCH
   NX_LAUNCH_CHECK();

@@ -123,6 +123,7 @@ def _declare(lib):
     sig("nx_moe_weight_grad", [P, P, P, I, P, I, I, P])
     sig("nx_gemm_bf16_grouped", [I, P, P, P, I, I, I, L, L, L, I, I, P, P, L, P, P, L, I, P])
     sig("nx_rope", [P, P, P, P, I, I, I, I, I, L, L, L, L, L, L, I, I, P])
+    sig("nx_rope_qk", [P] * 7 + [I] * 6 + [C.POINTER(L), I, I, P])
     sig("nx_embedding_fwd", [P, P, P, L, I, L, L, P])
     sig("nx_embedding_bwd", [P, P, P, L, I, L, L, P])
     sig("nx_flash_attn_fwd", [P] * 6 + [I] * 6 + [L] * 12 + [F, I, I, F, U, P, P, I, P])

@@ -169,10 +169,10 @@ def _fwd(q, k, v, scale, causal, window, alibi, dropout_p=0.0, seed=0, layout=No
     b, sq, h, d = q.shape
     sk, hk = k.shape[1], k.shape[2]
     o = torch.empty((b, sq, h, d), device=q.device, dtype=q.dtype)
-    # base-2 log-sum-exp, rows padded to a multiple of 128 with +inf (the backward reads whole
+    # base-2 log-sum-exp, rows padded to a multiple of 128 (the kernel writes +inf there: the backward reads whole
     # 128-row blocks of it; +inf makes the padding contribute zero probability)
     sq_pad = (sq + 127) // 128 * 128
-    lse = torch.full((b, h, sq_pad), float("inf"), device=q.device, dtype=torch.float32)
+    lse = torch.empty((b, h, sq_pad), device=q.device, dtype=torch.float32)
     LAUNCHES["n"] += 1
     rows, anyt, blk, _keep = _layout_args(layout, sq, sk, q.device)
     _lib.check(_lib.lib(q).nx_flash_attn_fwd(

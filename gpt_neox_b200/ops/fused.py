@@ -23,8 +23,7 @@ from .attention import _fwd as _attn_fwd_launch
 from .attention import _strides_bhs, attention_reference
 from .elementwise import bias_grad, colsum
 from .gemm import LAUNCHES, gemm, wgrad
-from .rope import _launch as _rope_launch
-from .rope import apply_rotary
+from .rope import apply_rotary, rotate_qk_
 
 
 class _MLPGeluFn(torch.autograd.Function):
@@ -99,13 +98,12 @@ class _QKVAttentionFn(torch.autograd.Function):
         s, b = qkv.shape[0], qkv.shape[1]
         q, k, v = _qkv_views(qkv, np_, kvp, hn)
         if rot > 0:
-            _rope_launch(q, q, cos, sin, rot, pos0, False)
-            _rope_launch(k, k, cos, sin, rot, pos0, False)
+            rotate_qk_(q, k, cos, sin, rot, pos0, False)
         qb, kb, vb = (t.permute(1, 0, 2, 3) for t in (q, k, v))  # [b, s, heads, hn] views
         out = torch.empty((s, b, np_, hn), device=qkv.device, dtype=qkv.dtype)
         ob = out.permute(1, 0, 2, 3)
         sq_pad = (s + 127) // 128 * 128
-        lse = torch.full((b, np_, sq_pad), float("inf"), device=qkv.device, dtype=torch.float32)
+        lse = torch.empty((b, np_, sq_pad), device=qkv.device, dtype=torch.float32)
         LAUNCHES["n"] += 1
         _lib.check(_lib.lib(qkv).nx_flash_attn_fwd(
             _lib.ptr(qb), _lib.ptr(kb), _lib.ptr(vb), _lib.ptr(ob), _lib.ptr(lse), _lib.ptr(alibi),
@@ -142,8 +140,7 @@ class _QKVAttentionFn(torch.autograd.Function):
             float(scale), 1, int(window), ctx.dropout[0], ctx.dropout[1], None, None, 0, _lib.stream()),
             "nx_flash_attn_bwd")
         if rot > 0:
-            _rope_launch(dq, dq, cos, sin, rot, pos0, True)
-            _rope_launch(dk, dk, cos, sin, rot, pos0, True)
+            rotate_qk_(dq, dk, cos, sin, rot, pos0, True)
         return (dqkv,) + (None,) * 12
 
 

@@ -555,3 +555,24 @@ def test_bias_and_norm_gradients_accumulate_straight_into_main_grad():
     for k, p in params.items():
         assert p.grad is None, k
         assert rel(p.main_grad, 2 * ref[k].grad) < 2e-2, k
+
+
+@pytest.mark.parametrize("hn,rot,np_,kvp", [(64, 16, 12, 12), (128, 32, 4, 4), (128, 128, 8, 2), (64, 64, 3, 1)])
+def test_rotate_qk_matches_the_per_tensor_kernel_and_writes_the_cache(hn, rot, np_, kvp):
+    from gpt_neox_b200.ops.fused import _qkv_views
+    from gpt_neox_b200.ops.rope import _launch_qk, _qk_ok, apply_rotary, rotary_tables, rotate_qk_
+    torch.manual_seed(3)
+    s, b, pos0 = 5, 3, 7
+    cos, sin = rotary_tables(rot, 64, device=DEV)
+    qkv = bf(s, b, (np_ + 2 * kvp) * hn)
+    q, k, v = _qkv_views(qkv, np_, kvp, hn)
+    want_q, want_k, want_v = apply_rotary(q, cos, sin, rot, pos0), apply_rotary(k, cos, sin, rot, pos0), v.clone()
+    keep = qkv.clone()
+    cache = torch.zeros(2, 9, b, kvp, hn, device=DEV, dtype=DT)
+    assert _qk_ok(rot, hn, q, k, v, cache[0], cache[1])
+    _launch_qk(q, k, cos, sin, rot, pos0, False, v=v, k_out=cache[0, 4:], v_out=cache[1, 4:])
+    assert torch.equal(q, want_q) and torch.equal(cache[0, 4:], want_k) and torch.equal(cache[1, 4:], want_v)
+    assert torch.equal(k, _qkv_views(keep, np_, kvp, hn)[1]) and not cache[:, :4].any()      # k itself is left alone
+    q2, k2, v2 = _qkv_views(keep, np_, kvp, hn)
+    rotate_qk_(q2, k2, cos, sin, rot, pos0, False)
+    assert torch.equal(q2, want_q) and torch.equal(k2, want_k) and torch.equal(v2, want_v)
