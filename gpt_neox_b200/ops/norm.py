@@ -28,6 +28,36 @@ def _accum_param_grad(param: torch.Tensor, g_f32: torch.Tensor):
     return g_f32.to(param.dtype)
 
 
+def _forward(kind, x, gamma, beta, eps, gamma2, beta2):
+    """-> (x as contiguous rows, y1, y2 or None, mean or None, rstd)."""
+    H = x.shape[-1]
+    x2 = x.reshape(-1, H)
+    if not x2.is_contiguous():
+        x2 = x2.contiguous()
+    rows = x2.shape[0]
+    y1 = torch.empty_like(x2)
+    y2 = torch.empty_like(x2) if gamma2 is not None else None
+    mean = torch.empty(rows, device=x.device, dtype=torch.float32) if kind == LN else None
+    rstd = torch.empty(rows, device=x.device, dtype=torch.float32)
+    LAUNCHES["n"] += 1
+    _lib.check(_lib.lib(x2).nx_norm_fwd(
+        kind, _lib.ptr(x2), _lib.ptr(gamma), _lib.ptr(beta), _lib.ptr(y1), _lib.ptr(gamma2),
+        _lib.ptr(beta2), _lib.ptr(y2), _lib.ptr(mean), _lib.ptr(rstd), rows, H, float(eps),
+        _lib.stream()), "nx_norm_fwd")
+    return x2, y1, y2, mean, rstd
+
+
+def _outputs(x, x2, y1, y2, carry):
+    outs = (y1.view(x.shape),) + ((y2.view(x.shape),) if y2 is not None else ())
+    if carry:
+        return (x2.view(x.shape),) + outs
+    return outs if y2 is not None else outs[0]
+
+
+def _run(kind, x, gamma, beta, eps, gamma2=None, beta2=None, carry=False):
+    return _NormFn.apply(kind, x, gamma, beta, eps, gamma2, beta2, carry)
+
+
 class _NormFn(torch.autograd.Function):
     """One or two norms of ``x``.  ``carry``: also return ``x`` itself as the first output, so that the
     gradient of the residual stream flows through this node and is added inside the backward kernel
@@ -35,30 +65,11 @@ class _NormFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, kind, x, gamma, beta, eps, gamma2, beta2, carry):
-        H = x.shape[-1]
-        x2 = x.reshape(-1, H)
-        if not x2.is_contiguous():
-            x2 = x2.contiguous()
-        rows = x2.shape[0]
-        y1 = torch.empty_like(x2)
-        dual = gamma2 is not None
-        y2 = torch.empty_like(x2) if dual else None
-        mean = torch.empty(rows, device=x.device, dtype=torch.float32) if kind == LN else None
-        rstd = torch.empty(rows, device=x.device, dtype=torch.float32)
-        LAUNCHES["n"] += 1
-        _lib.check(_lib.lib(x2).nx_norm_fwd(
-            kind, _lib.ptr(x2), _lib.ptr(gamma), _lib.ptr(beta), _lib.ptr(y1), _lib.ptr(gamma2),
-            _lib.ptr(beta2), _lib.ptr(y2), _lib.ptr(mean), _lib.ptr(rstd), rows, H, float(eps),
-            _lib.stream()), "nx_norm_fwd")
-        ctx.kind, ctx.dual, ctx.shape, ctx.carry = kind, dual, x.shape, carry
-        ctx.has_beta = beta is not None
-        ctx.has_beta2 = beta2 is not None
-        ctx.params = tuple(getattr(t, "_nx_param", None) for t in (gamma, beta, gamma2, beta2))
+        x2, y1, y2, mean, rstd = _forward(kind, x, gamma, beta, eps, gamma2, beta2)
+        ctx.kind, ctx.dual, ctx.shape, ctx.carry = kind, gamma2 is not None, x.shape, carry
+        ctx.params = (gamma, beta, gamma2, beta2)       # the parameters themselves: their main_grad takes the gradients
         ctx.save_for_backward(x2, gamma, gamma2, mean, rstd)
-        outs = (y1.view(x.shape),) + ((y2.view(x.shape),) if dual else ())
-        if carry:
-            return (x2.view(x.shape),) + outs
-        return outs if dual else outs[0]
+        return _outputs(x, x2, y1, y2, carry)
 
     @staticmethod
     def backward(ctx, *gys):
@@ -76,73 +87,45 @@ class _NormFn(torch.autograd.Function):
         gys = gys[1:] if ctx.carry else gys
         g1 = flat(gys[0])
         g2 = flat(gys[1]) if ctx.dual else None
-        pairs = [(g, gm, hb) for g, gm, hb in ((g1, gamma, ctx.has_beta), (g2, gamma2, ctx.has_beta2))
-                 if g is not None]
-        new = lambda: torch.empty(H, device=x2.device, dtype=torch.float32)
-        grads = {}
+        grads = [None] * 4                              # gamma, beta, gamma2, beta2
         dx = gres
-        if pairs:
-            (ga, gma, hba), (gb, gmb, hbb) = pairs[0], (pairs[1] if len(pairs) == 2 else (None, None, False))
+        if g1 is not None or g2 is not None:
+            # one gradient stream (ga with gamma ia) or, for a dual norm with both, two
+            norms = [i for i, g in ((0, g1), (2, g2)) if g is not None]
+            ia, both = norms[0], len(norms) == 2
+            ga, gma, gmb = (g1, g2)[ia // 2], (gamma, gamma2)[ia // 2], (gamma2 if both else None)
             blocks = L.nx_norm_bwd_blocks(rows)
-            ws = torch.empty(blocks * (4 if gb is not None else 2) * H, device=x2.device, dtype=torch.float32)
+            ws = torch.empty(blocks * (4 if both else 2) * H, device=x2.device, dtype=torch.float32)
             dx = torch.empty_like(x2)
             # parameter gradients: straight into the fp32 main_grad buffers (added by the partial-sum reduction
-            # kernel) when every parameter of this call has one, else into fresh buffers that autograd routes
-            owners = {id(gamma): ctx.params[0:2], id(gamma2): ctx.params[2:4]} if ctx.dual else {id(gamma): ctx.params[0:2]}
-            want = [owners[id(gma)][0]] + ([owners[id(gma)][1]] if hba else [])
-            if gb is not None:
-                want += [owners[id(gmb)][0]] + ([owners[id(gmb)][1]] if hbb else [])
-            mgs = [getattr(p_, "main_grad", None) if p_ is not None else None for p_ in want]
+            # kernel) when every parameter of this call has one, else into fresh buffers: of the parameters' own type
+            # when autograd takes them as they are, fp32 when some main_grad of another kind has to be added to
+            need = ctx.needs_input_grad
+            want = [i + j for i in norms for j in (0, 1) if ctx.params[i + j] is not None and need[(2, 3, 5, 6)[i + j]]]
+            mgs = [getattr(ctx.params[i], "main_grad", None) for i in want]
             direct = all(m is not None and m.dtype == torch.float32 and m.is_contiguous() and m.numel() == H for m in mgs)
-            if direct:
-                it = iter(mgs)
-                dga, dba = next(it), (next(it) if hba else None)
-                dgb, dbb = (next(it) if gb is not None else None), (next(it) if (gb is not None and hbb) else None)
-            else:
-                dga, dba = new(), (new() if hba else None)
-                dgb, dbb = (new() if gb is not None else None), (new() if hbb else None)
+            out16 = not direct and all(m is None and ctx.params[i].dtype == x2.dtype for i, m in zip(want, mgs))
+            out = [None] * 4
+            for i, m in zip(want, mgs):
+                out[i] = m if direct else torch.empty(H, device=x2.device, dtype=x2.dtype if out16 else torch.float32)
             LAUNCHES["n"] += 2
             _lib.check(L.nx_norm_bwd(
-                ctx.kind, _lib.ptr(ga), _lib.ptr(gb), _lib.ptr(x2), _lib.ptr(mean), _lib.ptr(rstd),
-                _lib.ptr(gma), _lib.ptr(gmb), _lib.ptr(gres), _lib.ptr(dx), _lib.ptr(dga), _lib.ptr(dba),
-                _lib.ptr(dgb), _lib.ptr(dbb), _lib.ptr(ws), rows, H, 1 if direct else 0, _lib.stream()), "nx_norm_bwd")
+                ctx.kind, _lib.ptr(ga), _lib.ptr(g2 if both else None), _lib.ptr(x2), _lib.ptr(mean), _lib.ptr(rstd),
+                _lib.ptr(gma), _lib.ptr(gmb), _lib.ptr(gres), _lib.ptr(dx), _lib.ptr(out[ia]), _lib.ptr(out[ia + 1]),
+                _lib.ptr(out[2] if both else None), _lib.ptr(out[3] if both else None), _lib.ptr(ws), rows, H,
+                1 if direct else 0, 1 if out16 else 0, _lib.stream()), "nx_norm_bwd")
             if not direct:
-                grads[id(gma)] = (dga, dba)
-                if gb is not None:
-                    grads[id(gmb)] = (dgb, dbb)
-        d1 = grads.get(id(gamma), (None, None))
-        d2 = grads.get(id(gamma2), (None, None)) if ctx.dual else (None, None)
-        return (None, dx.view(ctx.shape) if dx is not None else None, d1[0], d1[1], None, d2[0], d2[1], None)
-
-
-class _ParamGrad(torch.autograd.Function):
-    """Identity on a parameter whose backward converts the fp32 kernel gradient to the
-    parameter's dtype (or accumulates it into ``param.main_grad``)."""
-
-    @staticmethod
-    def forward(ctx, p):
-        ctx.p = p
-        ctx.set_materialize_grads(False)      # no gradient arrives when the norm kernel wrote into main_grad itself
-        return p.detach()
-
-    @staticmethod
-    def backward(ctx, g):
-        return None if g is None else _accum_param_grad(ctx.p, g)
-
-
-def _wrap(p):
-    if p is None or not p.requires_grad:
-        return p
-    w = _ParamGrad.apply(p)
-    w._nx_param = p          # the norm's backward adds into p.main_grad itself when it can (see _NormFn.backward)
-    return w
+                for i in want:
+                    p = ctx.params[i]
+                    grads[i] = out[i].view_as(p) if out16 else _accum_param_grad(p, out[i])
+        return (None, dx.view(ctx.shape) if dx is not None else None, grads[0], grads[1], None, grads[2], grads[3], None)
 
 
 def layer_norm(x, weight, bias=None, eps: float = 1e-5, carry: bool = False):
     """``carry``: return ``(x, y)``; the gradient of that ``x`` (the residual stream) is added to the
     norm's input gradient inside the backward kernel."""
     if _cuda_ok(x):
-        return _NormFn.apply(LN, x, _wrap(weight), _wrap(bias), eps, None, None, carry)
+        return _run(LN, x, weight, bias, eps, carry=carry)
     if carry:
         return x, layer_norm(x, weight, bias, eps)
     if x.is_cuda:
@@ -156,14 +139,14 @@ def dual_layer_norm(x, w1, b1, w2, b2, eps: float = 1e-5, carry: bool = False):
     stands for the residual stream; its gradient is added to the norms' input gradient inside the
     backward kernel."""
     if _cuda_ok(x):
-        return _NormFn.apply(LN, x, _wrap(w1), _wrap(b1), eps, _wrap(w2), _wrap(b2), carry)
+        return _run(LN, x, w1, b1, eps, w2, b2, carry)
     y = layer_norm(x, w1, b1, eps), layer_norm(x, w2, b2, eps)
     return (x,) + y if carry else y
 
 
 def rms_norm(x, weight, eps: float = 1e-8, carry: bool = False):
     if _cuda_ok(x):
-        return _NormFn.apply(RMS, x, _wrap(weight), None, eps, None, None, carry)
+        return _run(RMS, x, weight, None, eps, carry=carry)
     if carry:
         return x, rms_norm(x, weight, eps)
     if x.is_cuda:
@@ -176,5 +159,5 @@ def rms_norm(x, weight, eps: float = 1e-8, carry: bool = False):
 
 def dual_rms_norm(x, w1, w2, eps: float = 1e-8):
     if _cuda_ok(x):
-        return _NormFn.apply(RMS, x, _wrap(w1), None, eps, _wrap(w2), None, False)
+        return _run(RMS, x, w1, None, eps, w2, None)
     return rms_norm(x, w1, eps), rms_norm(x, w2, eps)

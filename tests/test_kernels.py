@@ -576,3 +576,42 @@ def test_rotate_qk_matches_the_per_tensor_kernel_and_writes_the_cache(hn, rot, n
     q2, k2, v2 = _qkv_views(keep, np_, kvp, hn)
     rotate_qk_(q2, k2, cos, sin, rot, pos0, False)
     assert torch.equal(q2, want_q) and torch.equal(k2, want_k) and torch.equal(v2, want_v)
+
+
+@pytest.mark.parametrize("rows,H", [(1, 8), (9, 248), (17, 264), (1001, 1032), (8, 2048), (601, 2048), (3, 2056)])
+@pytest.mark.parametrize("form", ["dual", "layer", "rms"])
+def test_norm_row_sizes(rows, H, form):
+    """Row lengths around what a lane, a warp and the warp-per-row form take; every gradient in the parameters' type."""
+    from gpt_neox_b200.ops.norm import dual_layer_norm, layer_norm, rms_norm
+    torch.manual_seed(4)
+    x, ps = bf(rows, H, scale=2.0, grad=True), [bf(H, grad=True) for _ in range({"dual": 4, "layer": 2, "rms": 1}[form])]
+    xr, pr = x.detach().double().requires_grad_(True), [p.detach().double().requires_grad_(True) for p in ps]
+    if form == "dual":
+        ys, yr = dual_layer_norm(x, *ps), [F.layer_norm(xr, (H,), *pr[i:i + 2], 1e-5) for i in (0, 2)]
+    elif form == "layer":
+        ys, yr = [layer_norm(x, *ps)], [F.layer_norm(xr, (H,), *pr, 1e-5)]
+    else:
+        ys, yr = [rms_norm(x, *ps, eps=1e-5)], [pr[0] * xr * torch.rsqrt(xr.square().mean(-1, keepdim=True) + 1e-5)]
+    gs = [bf(rows, H) for _ in ys]
+    got = torch.autograd.grad(ys, [x] + ps, gs)
+    want = torch.autograd.grad(yr, [xr] + pr, [g.double() for g in gs])
+    tol = 2 ** -7 if DT == torch.bfloat16 else 2 ** -10          # one rounding to the output type
+    for a, r in zip(list(ys) + list(got), yr + list(want)):
+        assert a.dtype == DT and rel(a, r) < tol
+    with torch.no_grad():                                        # without autograd: the same kernel, the same bits
+        again = {"dual": lambda: dual_layer_norm(x, *ps), "layer": lambda: [layer_norm(x, *ps)],
+                 "rms": lambda: [rms_norm(x, *ps, eps=1e-5)]}[form]()
+    assert all(torch.equal(a, y) for a, y in zip(again, ys))
+
+
+def test_norm_parameter_shared_by_both_norms_and_frozen_parameters():
+    from gpt_neox_b200.ops.norm import dual_layer_norm
+    torch.manual_seed(5)
+    x, w, b = bf(40, 256, grad=True), bf(256, grad=True), bf(256)
+    y1, y2 = dual_layer_norm(x, w, b, w, b)
+    g1, g2 = bf(40, 256), bf(256 * 40).view(40, 256)
+    dx, dw = torch.autograd.grad([y1, y2], [x, w], [g1, g2])
+    xr, wr = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    yr = F.layer_norm(xr, (256,), wr, b.double(), 1e-5)
+    rx, rw = torch.autograd.grad([yr, yr], [xr, wr], [g1.double(), g2.double()])
+    assert rel(dx, rx) < 2e-2 and rel(dw, rw) < 2e-2
