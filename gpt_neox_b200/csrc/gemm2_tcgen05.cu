@@ -8,7 +8,7 @@
 //   both CTAs             : a TMA producer warp fills the CTA's own shared memory; the transaction
 //                           bytes of both CTAs are counted on the leader's "full" barrier (the
 //                           cta_group::2 form of the bulk tensor load may signal the peer's barrier);
-//                           four epilogue warps drain the CTA's own 128 TMEM lanes (its 128 rows of
+//                           eight epilogue warps drain the CTA's own 128 TMEM lanes (its 128 rows of
 //                           the tile, all 256 columns) and report to the leader's "tmem empty" barrier.
 //
 // Same contract as nx_gemm_bf16 (csrc/gemm_tcgen05.cu): C[M,N] = epilogue(op(A) * op(B)), layouts
@@ -30,7 +30,7 @@ constexpr int BN = 256;
 constexpr int BK = 64;
 constexpr int UK = 16;
 constexpr int STAGES = 6;
-constexpr int THREADS = 320;        // producer, MMA issuer, 4 epilogue warps, 4 all-gather push warps
+constexpr int THREADS = 320;        // producer, MMA issuer, 4 epilogue warps, 4 epilogue or all-gather push warps
 constexpr int RS_ROW_BYTES = 144;    // 64 bf16 columns + 16 B pad
 constexpr int RS_STAGE_BYTES = 4 * 32 * RS_ROW_BYTES;
 constexpr int A_BYTES = BM * BK * 2, B_BYTES = BNH * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
@@ -212,7 +212,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tmem_full_bar(a), 1);
-      mbar_init(tmem_empty_bar(a), 8);         // leader: four epilogue warps of each CTA
+      mbar_init(tmem_empty_bar(a), p.comm == COMM_NONE ? 16 : 8);    // leader: the epilogue warps of both CTAs
     }
     for (int k = 0; k < 8; ++k) mbar_init(ag_bar(k), 4);   // one arrival per push warp
     *ag_abort = 0;
@@ -342,9 +342,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         }
       }
     }
-  } else if (warp < 6) {
-    // ------------------------------------------------------------------ epilogue (warps 2..5, both CTAs)
+  } else if (warp < 6 || p.comm == COMM_NONE) {
+    // ------------------------------------------------------------------ epilogue (warps 2..5, both CTAs; without a
+    // collective warps 6..9 too, the two warps of a lane quadrant taking half of the tile's columns each)
     const int quad = warp & 3;
+    const int c_begin = p.comm == COMM_NONE && warp >= 6 ? BN / 64 : 0;
+    const int c_end = p.comm == COMM_NONE && warp < 6 ? BN / 64 : BN / 32;
     const int row_in_tile = quad * 32 + lane;
     int acc = 0;
     uint32_t acc_phase = 0;
@@ -376,7 +379,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         }
       }
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = c_begin; c < c_end; ++c) {
         const int col0 = n0 + c * 32;
         if (col0 >= p.N) break;
         uint32_t r[32];

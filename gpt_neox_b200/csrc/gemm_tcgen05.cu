@@ -7,10 +7,11 @@
 // (megatron/model/activations.py:78-112, megatron/model/fused_bias_dropout.py:44-55) into the
 // epilogue.
 //
-// Kernel shape: persistent, one CTA per SM, 192 threads:
+// Kernel shape: persistent, one CTA per SM, 320 threads:
 //   warp 0      TMA producer  (one elected lane)
 //   warp 1      TMEM allocator + tcgen05.mma issuer (one elected lane)
-//   warps 2..5  epilogue: tcgen05.ld from TMEM -> registers -> fused math -> global stores
+//   warps 2..9  epilogue: tcgen05.ld from TMEM -> registers -> fused math -> global stores (with a fused collective
+//               only warps 2..5; 6..9 push the all-gather)
 // Tile 128 x BN x 64 with a STAGES-deep operand ring and two TMEM accumulators, so the
 // epilogue of tile i overlaps the main loop of tile i+1.
 //
@@ -30,7 +31,7 @@ namespace nx {
 constexpr int BM = 128;
 constexpr int BK = 64;
 constexpr int UMMA_K = 16;
-constexpr int GEMM_THREADS = 320;   // producer, MMA issuer, 4 epilogue warps, 4 all-gather push warps
+constexpr int GEMM_THREADS = 320;   // producer, MMA issuer, 4 epilogue warps, 4 epilogue or all-gather push warps
 constexpr int RS_ROW_BYTES = 144;    // 64 bf16 columns + 16 B pad: conflict-free 16-byte rows in shared memory
 constexpr int RS_STAGE_BYTES = 4 * 32 * RS_ROW_BYTES;   // one 32-row x 64-column slab per epilogue warp
 
@@ -191,7 +192,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tmem_full_bar(a), 1);
-      mbar_init(tmem_empty_bar(a), 4);  // one arrival per epilogue warp
+      mbar_init(tmem_empty_bar(a), p.comm == COMM_NONE ? 8 : 4);  // one arrival per epilogue warp
     }
     for (int k = 0; k < 8; ++k) mbar_init(ag_bar(k), 4);  // one arrival per push warp
     *ag_abort = 0;
@@ -325,9 +326,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         }
       }
     }
-  } else if (warp < 6) {
-    // ------------------------------------------------------------------ epilogue (warps 2..5)
+  } else if (warp < 6 || p.comm == COMM_NONE) {
+    // ------------------------------------------------------------------ epilogue (warps 2..5; without a collective
+    // warps 6..9 too, each pair of warps of a lane quadrant taking half of the tile's columns: with four warps the
+    // GeLU and its derivative, or the loads of a stored derivative, took longer than the MMAs of a short reduction:
+    // dropless-MoE layer of 16384 tokens, 768 -> 3072, forward + backward 1454 -> 1341 us)
     const int quad = warp & 3;  // TMEM lane quadrant this warp may access
+    const int c_begin = p.comm == COMM_NONE && warp >= 6 ? BN / 64 : 0;
+    const int c_end = p.comm == COMM_NONE && warp < 6 ? BN / 64 : BN / 32;
     const int row_in_tile = quad * 32 + lane;
     int acc = 0;
     uint32_t acc_phase = 0;
@@ -358,7 +364,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         }
       }
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = c_begin; c < c_end; ++c) {
         const int col0 = n0 + c * 32;
         if (col0 >= p.N) break;  // warp-uniform
         uint32_t r[32];
