@@ -58,12 +58,15 @@ def combine(y, plan: Plan, weights=None):
     return out
 
 
-def weight_grad(g, y, plan: Plan):
+def combine_bwd(g, y, plan: Plan, weights):
+    """Backward of ``combine``: (gradient of y, padded permuted [max_rows, H]; gradient of the weights [C])."""
+    dy = torch.empty((plan.max_rows, g.shape[1]), device=g.device, dtype=g.dtype)
     dw = torch.empty(plan.C, device=g.device, dtype=g.dtype)
     LAUNCHES["n"] += 1
-    _lib.check(_lib.lib(g).nx_moe_weight_grad(_lib.ptr(g), _lib.ptr(y), _lib.ptr(plan.dest_row), plan.k,
-                                             _lib.ptr(dw), plan.C, g.shape[1], _lib.stream()), "nx_moe_weight_grad")
-    return dw
+    _lib.check(_lib.lib(g).nx_moe_combine_bwd(_lib.ptr(g), _lib.ptr(y), _lib.ptr(plan.src_copy), _lib.ptr(weights), plan.k,
+                                             _lib.ptr(dy), _lib.ptr(dw), plan.max_rows, g.shape[1], _lib.stream()),
+               "nx_moe_combine_bwd")
+    return dy, dw
 
 
 def grouped_gemm_rows(a, w, plan: Plan, n_out, *, trans_b, gelu=None, aux_out=None, dgelu_aux=None, dgelu=None,
@@ -132,8 +135,8 @@ class _ExpertsGeluFn(torch.autograd.Function):
         xp, pre, h, y, wf, w1, w2 = ctx.saved_tensors
         plan = ctx.plan
         g = g.contiguous()
-        d_w = weight_grad(g, y, plan).view(ctx.w_shape)
-        dy = gather_rows(g, plan, scale=wf)                               # [rows, hidden], zero padding
+        dy, d_w = combine_bwd(g, y, plan, wf)                             # [rows, hidden], zero padding
+        d_w = d_w.view(ctx.w_shape)
         dpre = grouped_gemm_rows(dy, w2, plan, w2.shape[0] // plan.E, trans_b=False, dgelu_aux=pre, dgelu="mul")
         dw2 = grouped_wgrad(h, dy, plan, w2)
         dxp = grouped_gemm_rows(dpre, w1, plan, w1.shape[1], trans_b=True)
