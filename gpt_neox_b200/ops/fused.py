@@ -129,8 +129,7 @@ class _QKVAttentionFn(torch.autograd.Function):
         qb, kb, vb, dqb, dkb, dvb = map(perm, (q, k, v, dq, dk, dv))
         ob = perm(out)
         dob = perm(gout.view(s, b, np_, hn))
-        # (rows beyond the sequence exist only when it is not a multiple of the 128-row tile: only then a fill)
-        delta = (torch.empty if lse.shape[-1] == s else torch.zeros)(lse.shape, device=qkv.device, dtype=torch.float32)
+        delta = torch.empty(lse.shape, device=qkv.device, dtype=torch.float32)
         LAUNCHES["n"] += 3
         _lib.check(_lib.lib(qkv).nx_flash_attn_bwd(
             _lib.ptr(qb), _lib.ptr(kb), _lib.ptr(vb), _lib.ptr(ob), _lib.ptr(dob), _lib.ptr(lse),
