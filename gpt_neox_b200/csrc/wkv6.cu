@@ -50,17 +50,22 @@ struct WkvParams {
   int B, T, H, NC, clen;            // clen: steps per chunk, a multiple of WK_SUB
 };
 
+// 8 consecutive 16-bit elements (zero where dead): one 16-byte load when VEC, single elements otherwise.
 template <bool VEC>
-__device__ __forceinline__ void wk_load8(const h16* p, bool ok, float (&f)[8]) {
-  if (VEC) {
-    uint4 q = make_uint4(0u, 0u, 0u, 0u);
-    if (ok) q = *reinterpret_cast<const uint4*>(p);
-    const float2 a = unpack_h16x2(q.x), b = unpack_h16x2(q.y), c = unpack_h16x2(q.z), d = unpack_h16x2(q.w);
-    f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
-  } else {
+__device__ __forceinline__ uint4 wk_load8(const h16* p, bool ok) {
+  uint4 u = make_uint4(0u, 0u, 0u, 0u);
+  if (!ok) return u;
+  if (VEC) return *reinterpret_cast<const uint4*>(p);
+  uint16_t e[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = ok ? h16_to_float(p[j]) : 0.f;
-  }
+  for (int j = 0; j < 8; ++j) e[j] = reinterpret_cast<const uint16_t*>(p)[j];
+  u.x = e[0] | (uint32_t)e[1] << 16; u.y = e[2] | (uint32_t)e[3] << 16;
+  u.z = e[4] | (uint32_t)e[5] << 16; u.w = e[6] | (uint32_t)e[7] << 16;
+  return u;
+}
+__device__ __forceinline__ void wk_unpack8(const uint4& u, float (&f)[8]) {
+  const float2 a = unpack_h16x2(u.x), b = unpack_h16x2(u.y), c = unpack_h16x2(u.z), d = unpack_h16x2(u.w);
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
 }
 
 template <int N, int MODE>
@@ -121,6 +126,23 @@ __global__ void __launch_bounds__(N) wkv_kernel(const WkvParams p) {
   float sew = 0.f;                                     // LOCAL: thread i sums ew of channel i
 
   const int nsub = (t_hi - t_lo + WK_SUB - 1) / WK_SUB;
+  // the next sub-block's inputs are fetched before the steps of this one
+  uint4 rw[NPASS], rb[NPASS], rc[NPASS], ra[COL ? NPASS : 1], re[ROW ? NPASS : 1];
+  auto fetch = [&](int q) {
+    const int t0 = t_lo + (REV ? nsub - 1 - q : q) * WK_SUB;
+#pragma unroll
+    for (int ps = 0; ps < NPASS; ++ps) {
+      const int t = t0 + trow + ps * (N / TPR);
+      const bool ok = t < t_hi;
+      const long long o = bi * p.sb + (long long)t * p.st + h * N + ch8;
+      rw[ps] = wk_load8<VEC>(p.w + o, ok);
+      rb[ps] = wk_load8<VEC>((REV ? p.r : p.k) + o, ok);
+      rc[ps] = wk_load8<VEC>((REV ? p.gy : p.v) + o, ok);
+      if (COL) ra[COL ? ps : 0] = wk_load8<VEC>((MODE == WK_Y ? p.r : p.k) + o, ok);
+      if (ROW) re[ROW ? ps : 0] = wk_load8<VEC>((MODE == WK_GR ? p.gy : p.v) + o, ok);
+    }
+  };
+  fetch(0);
   for (int q = 0; q < nsub; ++q) {
     const int t0 = t_lo + (REV ? nsub - 1 - q : q) * WK_SUB;
     const int steps = min(WK_SUB, t_hi - t0);
@@ -134,25 +156,21 @@ __global__ void __launch_bounds__(N) wkv_kernel(const WkvParams p) {
     for (int ps = 0; ps < NPASS; ++ps) {
       const int t = trow + ps * (N / TPR);
       const bool ok = t < steps;
-      const long long o = bi * p.sb + (long long)(t0 + t) * p.st + h * N + ch8;
       float x[8], y[8], wv[8];
-      wk_load8<VEC>(p.w + o, ok, wv);
+      wk_unpack8(rw[ps], wv);
+      wk_unpack8(rb[ps], x);
+      wk_unpack8(rc[ps], y);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float ew = ok ? -__expf(wv[j]) : 0.f;
         s.ew[t][ch8 + j] = ew;
         s.d[t][ch8 + j] = __expf(ew);
-      }
-      wk_load8<VEC>((REV ? p.r : p.k) + o, ok, x);     // b
-      wk_load8<VEC>((REV ? p.gy : p.v) + o, ok, y);    // c
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
         s.b[t][ch8 + j] = x[j];
         s.c[t][ch8 + j] = make_float2(y[j], y[j]);
       }
       if (COL) {
         float a[8], dt = 0.f;
-        wk_load8<VEC>((MODE == WK_Y ? p.r : p.k) + o, ok, a);
+        wk_unpack8(ra[COL ? ps : 0], a);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           s.a[t][ch8 + j] = a[j];
@@ -164,7 +182,7 @@ __global__ void __launch_bounds__(N) wkv_kernel(const WkvParams p) {
       }
       if (ROW) {
         float e[8], dt = 0.f;
-        wk_load8<VEC>((MODE == WK_GR ? p.gy : p.v) + o, ok, e);
+        wk_unpack8(re[ROW ? ps : 0], e);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           s.e[t][ch8 + j] = make_float2(e[j], e[j]);
@@ -175,6 +193,7 @@ __global__ void __launch_bounds__(N) wkv_kernel(const WkvParams p) {
         if (ch8 == 0) s.dot_row[t] = dt;
       }
     }
+    if (q + 1 < nsub) fetch(q + 1);
     __syncthreads();
 #pragma unroll 2
     for (int tq = 0; tq < steps; ++tq) {
