@@ -1,0 +1,58 @@
+"""Key / value caches that grow in place while generating.
+
+A layer's cache is the tensor it returns as ``present``: ``[2, n, b, heads, hn]``.  Here that tensor is the front of a
+buffer with room for more rows, so a step writes its own rows behind the ones that are there instead of copying the
+whole cache (concatenating k and v and stacking them moves every cached byte twice per step).
+
+Only the tensor that the layer returned last, unchanged in length and on the same stream, is extended in place; an older
+one (a second continuation of the same prefix), another layer's or a caller's own is copied into a buffer of its own, so
+no ``present`` ever sees rows that were appended to another.
+"""
+from __future__ import annotations
+
+import threading
+import weakref
+
+import torch
+
+_LOCK = threading.Lock()
+#: layer -> (weak reference to the cache it returned last, stream); the cache itself is held by whoever uses it
+_LAST: "weakref.WeakKeyDictionary" = weakref.WeakKeyDictionary()
+_MIN_ROOM = 256
+
+
+def _stream(t):
+    return torch.cuda.current_stream(t.device).cuda_stream if t.is_cuda else 0
+
+
+def _claim(layer, past, stream) -> bool:
+    """Whether ``past`` is the cache ``layer`` returned last; the answer is yes once per returned cache."""
+    with _LOCK:
+        ref, st = _LAST.get(layer, (None, None))
+        if ref is None or ref() is not past or st != stream:
+            return False
+        del _LAST[layer]
+        return True
+
+
+def extend(layer, past, rows: int, like: torch.Tensor) -> torch.Tensor:
+    """The cache ``[2, n + rows, b, heads, hn]`` whose first n rows are ``past``'s (None or empty: n = 0) and whose last
+    ``rows`` rows the caller fills.  ``like``: [*, b, heads, hn], the new keys (shape, dtype and device)."""
+    n = 0 if past is None else past[0].shape[0]
+    shape = tuple(like.shape[1:])
+    stream, total = _stream(like), n + rows
+    buf = None
+    if torch.is_tensor(past) and past.dtype == like.dtype and past.device == like.device \
+            and tuple(past.shape[2:]) == shape and _claim(layer, past, stream):
+        room = past.stride(0) // past.stride(1)
+        if total <= room:
+            buf = past.as_strided((2, room) + shape, past.stride())
+    if buf is None:
+        buf = torch.empty((2, total + max(_MIN_ROOM, total // 4)) + shape, device=like.device, dtype=like.dtype)
+        if n:
+            buf[0, :n].copy_(past[0])
+            buf[1, :n].copy_(past[1])
+    present = buf[:, :total]
+    with _LOCK:
+        _LAST[layer] = (weakref.ref(present), stream)
+    return present

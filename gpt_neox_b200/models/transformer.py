@@ -23,7 +23,10 @@ from ..ops.attention import flash_attention, next_dropout_seed
 from ..ops.elementwise import bias_dropout_add
 from ..ops.gemm import gemm as gemm_op
 from ..ops.gemm import linear as linear_op
+from ..ops.layer_infer import layer_infer, takes
 from ..ops.norm import dual_layer_norm
+from ..ops import _lib as kernel_lib
+from ..ops import rope as rope_ops
 from ..ops.rope import apply_rotary
 from ..ops.softmax import scaled_causal_softmax, scaled_masked_softmax
 from ..parallel.mappings import (copy_to_model_parallel_region, gather_from_sequence_parallel_region,
@@ -31,6 +34,7 @@ from ..parallel.mappings import (copy_to_model_parallel_region, gather_from_sequ
                                  reduce_scatter_to_sequence_parallel_region)
 from .activations import get_activation
 from .norms import LayerNorm, RMSNorm, get_norm
+from . import kv_cache
 from .positional_embeddings import AliBi, RotaryEmbedding
 
 
@@ -289,6 +293,22 @@ class ParallelSelfAttention(nn.Module):
         ctx = torch.bmm(probs.to(v2.dtype), v2)                          # [b*np, sq, hn]
         return ctx.view(b, np_, sq, hn).permute(2, 0, 1, 3).reshape(sq, b, np_ * hn)
 
+    def _rotate_into_cache(self, q, k, v, past, cos, sin):
+        """Generation without autograd: q rotated, and the cache with this step's (rotated) k and v behind ``past``;
+        one kernel does the rotation and the cache write.  -> (q, present)"""
+        n = past[0].shape[0] if past is not None else 0
+        present = kv_cache.extend(self, past, k.shape[0], k)
+        k_new, v_new = present[0, n:], present[1, n:]
+        if self.rotary_emb is not None and rope_ops._qk_ok(self.rotary_dim, q.shape[3], q, k, v, k_new, v_new):
+            rope_ops._launch_qk(q, k, cos, sin, self.rotary_dim, n, False, v=v, k_out=k_new, v_out=v_new)
+            return q, present
+        if self.rotary_emb is not None:
+            q = apply_rotary(q, cos, sin, self.rotary_dim, n)
+            k = apply_rotary(k, cos, sin, self.rotary_dim, n)
+        k_new.copy_(k)
+        v_new.copy_(v)
+        return q, present
+
     # -------------------------------------------------------------------- forward
     def forward(self, hidden_states, attention_mask=None, layer_past=None, residual=None):
         """hidden_states [sq, b, h] -> (output [sq, b, h] without dense bias, dense bias)
@@ -319,13 +339,17 @@ class ParallelSelfAttention(nn.Module):
                 q = self.qk_layernorm(q.contiguous())
                 k = self.qk_layernorm(k.contiguous()) if kvp == np_ else k
             offset = layer_past[0].shape[0] if has_past else 0
-            if self.rotary_emb is not None:
-                q = apply_rotary(q, cos, sin, self.rotary_dim, offset)
-                k = apply_rotary(k, cos, sin, self.rotary_dim, offset)
-            if has_past:
-                k = torch.cat((layer_past[0].type_as(k), k), dim=0)
-                v = torch.cat((layer_past[1].type_as(v), v), dim=0)
-            present = torch.stack((k, v)) if self.use_cache else None
+            if self.use_cache and q.is_cuda and q.dtype in kernel_lib.H16 and kernel_lib.untracked():
+                q, present = self._rotate_into_cache(q, k, v, layer_past if has_past else None, cos, sin)
+                k, v = present[0], present[1]
+            else:
+                if self.rotary_emb is not None:
+                    q = apply_rotary(q, cos, sin, self.rotary_dim, offset)
+                    k = apply_rotary(k, cos, sin, self.rotary_dim, offset)
+                if has_past:
+                    k = torch.cat((layer_past[0].type_as(k), k), dim=0)
+                    v = torch.cat((layer_past[1].type_as(v), v), dim=0)
+                present = torch.stack((k, v)) if self.use_cache else None
             sparse_kernel = (self.sparse and self.rpe is None and q.is_cuda and self.sparse_layout.kernel_ok
                              and q.dtype in (torch.bfloat16, torch.float16) and hn % 8 == 0 and hn <= 128)
             if (self.use_flash_attention and self.rpe is None) or sparse_kernel:
@@ -345,8 +369,14 @@ class ParallelSelfAttention(nn.Module):
         # output projection; bias (and the optional residual) are applied by the caller / epilogue
         if residual is not None and ctx.is_cuda and not self.dense.sequence_parallel and \
                 mpu.get_model_parallel_world_size() == 1:
-            out = _linear_residual(ctx, self.dense.weight, residual)
-            bias = self.dense.bias
+            if kernel_lib.untracked():
+                # the bias too goes into the GEMM's epilogue (a training step sums it with the MLP's instead, so that
+                # one column sum serves both gradients)
+                out = _linear_bias_residual(ctx, self.dense.weight, self.dense.bias, residual)
+                bias = None
+            else:
+                out = _linear_residual(ctx, self.dense.weight, residual)
+                bias = self.dense.bias
         else:
             out, bias = self.dense(ctx)
             if residual is not None:
@@ -379,6 +409,12 @@ class _LinearResidualFn(torch.autograd.Function):
         gx = gemm_op(gy2, w, trans_b=True).view(ctx.x_shape)
         gw = wgrad(gy2, x2, w)
         return gx, gw, gy2.view(gy.shape)
+
+
+def _linear_bias_residual(x, w, bias, residual):
+    """x @ w^T (+ bias) + residual without autograd."""
+    x2, r2 = x.reshape(-1, x.shape[-1]).contiguous(), residual.reshape(-1, residual.shape[-1]).contiguous()
+    return gemm_op(x2, w, bias=bias, residual=r2).view(*x.shape[:-1], w.shape[0])
 
 
 def _linear_residual(x, w, residual):
@@ -432,6 +468,48 @@ class ParallelTransformerLayer(nn.Module):
                                            output_layer_init_method=output_layer_init_method)
         self.layer_past = None
 
+    def _infer(self, x, layer_past):
+        """The whole layer in one native call, or None where it has to run op by op: generation without autograd, dense
+        parallel-residual layer with two LayerNorms, rotary flash attention and a GeLU MLP on one tensor-parallel rank,
+        plain modules that nobody hooks into."""
+        a, m = self.attention, self.mlp
+        if not (self.use_cache and x.is_cuda and x.is_contiguous() and x.shape[0] > 0 and x.shape[1] > 0
+                and kernel_lib.untracked() and self._dual_norm_ok(x)
+                and type(a) is ParallelSelfAttention and type(m) is ParallelMLP and a.use_cache and a.use_flash_attention
+                and not a.use_qk_layernorm and a.rpe is None and a.rotary_emb is not None
+                and not (self.training and (self.hidden_dropout > 0 or a.dropout_p > 0))
+                and mpu.get_model_parallel_world_size() == 1 and m._fusable(x)):
+            return None
+        hn = a.hidden_size_per_attention_head
+        linears = (a.query_key_value, a.dense, m.linear1, m.linear2)
+        mods = (self.input_layernorm, self.post_attention_layernorm, a, a.rotary_emb, m) + linears
+        if hn % 8 or hn > 128 or a.rotary_dim % 16 or any(
+                l.use_mup or getattr(l, "use_fp8", False) or getattr(l, "gather_output", False) for l in linears) \
+                or type(linears[0]) is not mpu.ColumnParallelLinear or type(linears[2]) is not mpu.ColumnParallelLinear \
+                or type(linears[1]) is not mpu.RowParallelLinear or type(linears[3]) is not mpu.RowParallelLinear \
+                or linears[0].skip_bias_add \
+                or torch.nn.modules.module._has_any_global_hook() or any(
+                    z._forward_hooks or z._forward_pre_hooks for z in mods):
+            return None
+        norms = (self.input_layernorm.weight, self.input_layernorm.bias, self.post_attention_layernorm.weight,
+                 self.post_attention_layernorm.bias)
+        weights = [(l.weight, l.bias) for l in linears]
+        has_past = layer_past is not None and (not torch.is_tensor(layer_past) or layer_past.numel() > 0)
+        past = layer_past[0].shape[0] if has_past else 0
+        cos, sin = a.rotary_emb(seq_len=x.shape[0] + past)
+        if not takes(x, *norms, *(t for wb in weights for t in wb)) or cos.data_ptr() % 16 or sin.data_ptr() % 16 \
+                or self.input_layernorm.eps != self.post_attention_layernorm.eps:
+            return None
+        kvp = a.num_kv_heads_per_partition
+        present = kv_cache.extend(a, layer_past if has_past else None, x.shape[0], x.new_empty((0, x.shape[1], kvp, hn)))
+        out = layer_infer(
+            x, norms, *weights, cos, sin, a.alibi_embed.slopes if a.pos_emb == "alibi" else None, present, past,
+            heads=a.num_attention_heads_per_partition, kv_heads=kvp, head_dim=hn, rot=a.rotary_dim,
+            window=a.sliding_window_width if a.sliding_window_width is not None else -1, scale=a.attn_scale,
+            eps=self.input_layernorm.eps, gelu="tanh" if m.bias_gelu_fusion else "erf")
+        self.layer_past = present
+        return out
+
     def _dual_norm_ok(self, x):
         return (isinstance(self.input_layernorm, LayerNorm) and not self.gpt_j_tied
                 and len(self.input_layernorm.normalized_shape) == 1)
@@ -441,6 +519,9 @@ class ParallelTransformerLayer(nn.Module):
         p = self.hidden_dropout if self.training else 0.0
         ws = mpu.get_model_parallel_world_size()
         if self.gpt_j_residual:
+            out = self._infer(x, layer_past) if self.use_cache else None
+            if out is not None:
+                return out
             residual = x
             if self.gpt_j_tied:
                 x1 = x2 = self.input_layernorm(x)
@@ -453,10 +534,10 @@ class ParallelTransformerLayer(nn.Module):
                                                    carry=True)
             else:
                 x1, x2 = self.input_layernorm(x), self.post_attention_layernorm(x)
-            fusable = (p == 0.0 and x.is_cuda and self.num_experts <= 1 and not self.use_cache
+            fusable = (p == 0.0 and x.is_cuda and self.num_experts <= 1
                        and isinstance(self.mlp, ParallelMLP) and self.mlp._fusable(x2))
-            fast = fusable and ws == 1
-            if fusable and self.sequence_parallel:
+            fast = fusable and ws == 1 and (not self.use_cache or kernel_lib.untracked())
+            if fusable and self.sequence_parallel and not self.use_cache:
                 from ..ops import fused_tp
                 be = fused_tp.backend(x, mpu.get_model_parallel_group())
                 m_full = x.shape[0] * x.shape[1] * ws
@@ -477,7 +558,9 @@ class ParallelTransformerLayer(nn.Module):
             if fast:
                 # x + attn + b_attn + mlp + b_mlp with both adds of matrices inside GEMM epilogues:
                 #   t = dense(ctx) + x ;  out = linear2(h) + t ; the two bias vectors are added once.
-                t, b_attn = self.attention(x1, attention_mask, layer_past=layer_past, residual=residual)
+                t, b_attn, *cache = self.attention(x1, attention_mask, layer_past=layer_past, residual=residual)
+                if cache:
+                    self.layer_past = cache[0]
                 out, _ = self.mlp(x2, residual=t, out_bias=_sum_bias(b_attn, self.mlp.linear2.bias))
                 return out
             att = self.attention(x1, attention_mask, layer_past=layer_past)

@@ -124,6 +124,9 @@ def _declare(lib):
     sig("nx_gemm_bf16_grouped", [I, P, P, P, I, I, I, L, L, L, I, I, P, P, L, P, P, L, I, P])
     sig("nx_rope", [P, P, P, P, I, I, I, I, I, L, L, L, L, L, L, I, I, P])
     sig("nx_rope_qk", [P] * 7 + [I] * 6 + [C.POINTER(L), I, I, P])
+    sig("nx_layer_infer_work", [P], L)
+    sig("nx_layer_infer_stats", [P], L)
+    sig("nx_layer_infer", [P, P])
     sig("nx_embedding_fwd", [P, P, P, L, I, L, L, P])
     sig("nx_embedding_bwd", [P, P, P, L, I, L, L, P])
     sig("nx_flash_attn_fwd", [P] * 6 + [I] * 6 + [L] * 12 + [F, I, I, F, U, P, P, I, P])
@@ -168,6 +171,13 @@ def ptr(t):
         # of letting the GPU fault on it
         raise KernelError(f"host tensor (shape {tuple(t.shape)}, {t.dtype}) passed to a CUDA kernel")
     return c_void_p(t.data_ptr())
+
+
+def untracked() -> bool:
+    """Nothing records what runs now (no gradient mode, no forward-mode level, no tracer): an op may launch its kernel
+    without an autograd node around it."""
+    return (not torch.is_grad_enabled() and torch.autograd.forward_ad._current_level < 0
+            and not torch.jit.is_tracing())
 
 
 def stream():

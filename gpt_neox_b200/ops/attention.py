@@ -236,6 +236,8 @@ def flash_attention(q, k, v, *, scale: float | None = None, causal: bool = True,
         if block_layout is not None and not block_layout.kernel_ok:
             raise _lib.KernelError(f"flash_attention: block-sparse layouts need blocks of 16, 32, 64 or 128 tokens "
                                    f"(got {block_layout.block})")
+        if _lib.untracked():
+            return _fwd(fix(q), fix(k), fix(v), scale, causal, window, alibi, float(dropout_p), seed, block_layout)[0]
         return _FlashAttnFn.apply(fix(q), fix(k), fix(v), scale, causal, window, alibi, float(dropout_p), seed,
                                   block_layout)
     return attention_reference(q, k, v, scale=scale, causal=causal, window=window, alibi=alibi, dropout_p=dropout_p,

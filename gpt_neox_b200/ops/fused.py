@@ -71,6 +71,11 @@ class _MLPGeluFn(torch.autograd.Function):
 def mlp_gelu(x, w1, b1, w2, b2=None, residual=None, kind: str = "erf", recompute_act: bool = False):
     """``gelu(x @ w1^T + b1) @ w2^T (+ b2) (+ residual)``; kind in {"erf", "tanh"}."""
     if x.is_cuda and x.dtype in _lib.H16:
+        if _lib.untracked():        # nothing will ask for the activation's derivative
+            x2 = x.reshape(-1, x.shape[-1]).contiguous()
+            r2 = residual.reshape(x2.shape[0], -1).contiguous() if residual is not None else None
+            y = gemm(gemm(x2, w1, bias=b1, gelu=kind), w2, bias=b2, residual=r2)
+            return y.view(*x.shape[:-1], w2.shape[0])
         return _MLPGeluFn.apply(x, w1, b1, w2, b2, residual, kind, recompute_act)
     if x.is_cuda:
         raise _lib.KernelError("mlp_gelu: CUDA path needs bf16")

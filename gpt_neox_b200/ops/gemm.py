@@ -167,6 +167,8 @@ def wgrad(gy2: torch.Tensor, x2: torch.Tensor, weight: torch.Tensor):
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
     """``F.linear`` on the tcgen05 GEMM for CUDA bf16 / fp16 tensors; PyTorch on CPU (oracle path)."""
     if x.is_cuda and x.dtype in _lib.H16:
+        if _lib.untracked():
+            return gemm(_as_2d(x), weight, bias=bias).view(*x.shape[:-1], weight.shape[0])
         return _LinearFn.apply(x, weight, bias)
     if x.is_cuda:
         raise _lib.KernelError(f"linear: the CUDA kernels take bf16 or fp16 activations, got {x.dtype}")

@@ -263,3 +263,110 @@ def test_eval_harness_runs_end_to_end_on_local_task_files(tmp_path):
             assert pp2["results"][task][metric] == pytest.approx(v, rel=1e-4), (task, metric)
     from gpt_neox_b200.eval_tasks import local_tasks
     assert local_tasks.resolve("hellaswag") is None
+
+
+def test_growing_cache_keeps_every_continuation_apart():
+    """The in-place growth of a layer's cache against plain concatenation: steps, a second continuation of an older
+    cache, another layer's cache, a caller's own tensor, and growth past the buffer's room."""
+    import torch
+    from gpt_neox_b200.models import kv_cache
+
+    class Layer:
+        pass
+
+    torch.manual_seed(0)
+    layer, other = Layer(), Layer()
+
+    def step(owner, past, rows):
+        new = torch.randn(2, rows, 2, 3, 4)
+        want = new if past is None else torch.cat((torch.stack((past[0], past[1])), new), dim=1)
+        got = kv_cache.extend(owner, past, rows, new[0])
+        got[:, got.shape[1] - rows:].copy_(new)
+        assert torch.equal(got, want)
+        return got, want.clone()
+
+    seen = [step(layer, None, 5)]
+    for rows in (1, 1, 3, 1):
+        seen.append(step(layer, seen[-1][0], rows))
+    assert seen[1][0].data_ptr() == seen[4][0].data_ptr()               # grown in place
+    fork = step(layer, seen[2][0], 2)                                   # an older cache: a copy
+    again = step(layer, seen[4][0], 1)                                  # no longer the last one returned: a copy
+    cross = step(other, again[0], 1)                                    # another layer's
+    own = step(layer, torch.randn(2, 7, 2, 3, 4), 1)                    # a caller's tensor
+    pair = step(layer, (own[0][0], own[0][1]), 1)                       # (k, v) instead of one tensor
+    big = step(layer, pair[0], 2000)                                    # more than the buffer has room for
+    last = step(layer, big[0], 1)
+    for got, want in seen + [fork, again, cross, own, pair, big, last]:
+        assert torch.equal(got, want)
+    empty = step(layer, torch.empty(2, 0, 2, 3, 4), 4)
+    assert empty[0].shape[1] == 4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("over", [dict(), dict(num_kv_heads=2, rotary_pct=1.0), dict(pos_emb="alibi"),
+                                  dict(gpt_j_residual=False, norm="rmsnorm", rotary_pct=0.5)])
+def test_cached_steps_match_the_whole_prefix_on_the_gpu(over):
+    """Prompt + single-token steps through the growing cache (in place, no autograd, fused rotary write) against one
+    uncached pass over the whole sequence."""
+    import torch
+    from common import tiny_config
+    from test_model_gpu import _build
+    base = dict(num_layers=2, hidden_size=256, num_attention_heads=4, seq_length=512, max_position_embeddings=512,
+                synthetic_vocab_size=1000, attention_config=[[["flash"], 2]], distributed_backend="nccl",
+                precision="bfloat16", pipe_parallel_size=0)
+    base.update(over)
+    _, model = _build(tiny_config(**base))
+    model.eval()
+    tokens = torch.randint(0, 1000, (2, 300), device="cuda")
+    pos = torch.arange(300, device="cuda")[None].expand(2, -1)
+    with torch.no_grad():
+        full = model((tokens, pos, None)).float()
+        model.inference_mode(use_cache=True)
+        model.clear_cache()
+        got, at = [], 0
+        for n in [20, 1, 1, 7] + [1] * 5 + [256, 1, 1]:          # the 256-row step outgrows the first buffer
+            got.append(model((tokens[:, at:at + n].contiguous(), pos[:, at:at + n].contiguous(), None)).float())
+            at += n
+    got = torch.cat(got, dim=1)
+    err = (got - full[:, :at]).norm() / full[:, :at].norm()
+    assert err < 2e-2, err.item()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["bfloat16", "fp16"])
+@pytest.mark.parametrize("over", [dict(), dict(num_kv_heads=2, rotary_pct=1.0), dict(bias_gelu_fusion=True),
+                                  dict(sliding_window_width=16), dict(use_bias_in_attn_linear=False,
+                                                                      use_bias_in_mlp=False)])
+def test_a_layer_in_one_call_gives_the_bits_of_the_op_by_op_path(over, precision):
+    """A hook on a submodule sends the layer down the op-by-op path; without it one native call launches the same
+    kernels."""
+    from test_model_gpu import _build
+    base = dict(num_layers=2, hidden_size=256, num_attention_heads=4, seq_length=512, max_position_embeddings=512,
+                synthetic_vocab_size=1000, attention_config=[[["flash"], 2]], distributed_backend="nccl",
+                precision=precision, pipe_parallel_size=0)
+    base.update(over)
+    _, model = _build(tiny_config(**base))
+    model.eval()
+    model.inference_mode(use_cache=True)
+    tokens = torch.randint(0, 1000, (3, 330), device="cuda")
+    pos = torch.arange(330, device="cuda")[None].expand(3, -1)
+
+    def steps():
+        model.clear_cache()
+        out, at = [], 0
+        with torch.no_grad():
+            for n in (40, 1, 1, 5, 1, 270, 1):
+                out.append(model((tokens[:, at:at + n].contiguous(), pos[:, at:at + n].contiguous(), None)))
+                at += n
+        layers = [m for m in model.modules() if type(m).__name__.startswith("ParallelTransformerLayer")]
+        return out + [l.layer_past.clone() for l in layers]
+
+    one = steps()
+    mlps = [m for m in model.modules() if type(m).__name__ == "ParallelMLP"]
+    calls = []
+    handles = [m.register_forward_hook(lambda *a: calls.append(1)) for m in mlps]
+    ops = steps()
+    for h in handles:
+        h.remove()
+    assert len(calls) == 14 and len(one) == len(ops)
+    assert all(torch.equal(a, b) for a, b in zip(one, ops))
