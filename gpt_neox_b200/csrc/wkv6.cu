@@ -7,8 +7,8 @@
 // kernel_backward_111 / _222), which walks the whole sequence in one thread per channel and needs
 // the sequence length as a compile-time constant for a per-thread array.
 //
-// One CTA of N threads walks one head's piece of the sequence with the N x N state in registers: warp w owns 32 columns
-// j, a lane N / 8 rows i by 8 columns.  Per step a lane reads N / 8 values of each row vector and 8 of each column
+// One CTA of 2 N threads walks one head's piece of the sequence with the N x N state in registers: warp w owns 16 columns
+// j, a lane N / 8 rows i by 4 columns.  Per step a lane reads N / 8 values of each row vector and 4 of each column
 // vector from shared memory (column vectors are stored twice side by side, so that the packed fp32 pairs, which run
 // over neighbouring rows, need no register moves) and does 3 packed operations per 2 state elements: one for the output
 // sum, two for the update.  The former one-column-per-thread mapping read every row vector whole in every thread, which
@@ -19,8 +19,10 @@
 //              gk (sum over j) and gv (sum over i), which also forms the decay gradient: with
 //              Q_t[i] = sum_j G_t[i][j] S_t[i][j] one has Q_{t-1} - Q_t = r_t gr_t - k_t gk_t and
 //              dL/d(ew_t) = Q_t - k_t (gk_t - r_t u s_t),  s_t = <gy_t, v_t>,  ew = -exp(w)
-// Bound by the FMA pipe: 3 + 3 + 4 operations per state element and step.  Forward + backward of 32 x 512 tokens, 12 heads
-// of 64: 3.03 ms before, 0.91 ms now.
+// 3 + 3 + 4 operations per state element and step; at 32 x 512 tokens, 12 heads of 64, the schedulers have 2.6 warps each and
+// are bound by the latency of the steps' shared-memory loads and exchanges (issue slots about half used).  Forward +
+// backward of that size: 3.03 ms with one column per thread in seven passes, 0.87 ms with 8 columns per lane and half the
+// warps, 0.79 ms now.
 //
 // The sequence is cut into chunks only when batch x heads leaves the chip idle (wkv_chunk_count): the recurrence is
 // linear, so a chunk's end state is  P (.) S_start + S_local  with P[i] = prod_t d_t[i]; local passes start every chunk
@@ -77,18 +79,18 @@ struct WkvSmem {
   float2 e[ROW ? WK_SUB : 1][N];                // (e, e): sum over j of e[j] S[i][j]
   float ew[WK_SUB][N];
   float colsum[COL ? WK_SUB : 1][N];
-  float rowsum[ROW ? N / 32 : 1][ROW ? WK_SUB : 1][N];
+  float rowsum[ROW ? N / 16 : 1][ROW ? WK_SUB : 1][N];
   float dot_col[WK_SUB], dot_row[WK_SUB];       // <a, u b> and <e, c>
 };
 
 template <int N, int MODE, bool VEC>
-__global__ void __launch_bounds__(N) wkv_kernel(const WkvParams p) {
+__global__ void __launch_bounds__(2 * N) wkv_kernel(const WkvParams p) {
   using Sm = WkvSmem<N, MODE>;
   constexpr bool REV = MODE == WK_LOCAL_REV || MODE == WK_G, ROW = Sm::ROW, COL = Sm::COL;
   constexpr bool LOCAL = MODE == WK_LOCAL_FWD || MODE == WK_LOCAL_REV;
   constexpr int QUADS = N / 32, PAIRS = QUADS * 2;     // a lane's rows: QUADS groups of 4 neighbours
-  constexpr int TPR = N / 8;                           // staging threads per step
-  constexpr int NPASS = WK_SUB * TPR / N;              // staging passes (2)
+  constexpr int TPR = N / 8;                           // staging threads per step: 2 N threads stage 16 steps
+  static_assert(WK_SUB * TPR == 2 * N, "one staging pass");
   extern __shared__ __align__(16) unsigned char wk_raw[];
   Sm& s = *reinterpret_cast<Sm*>(wk_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -97,28 +99,29 @@ __global__ void __launch_bounds__(N) wkv_kernel(const WkvParams p) {
   const int t_lo = c * p.clen, t_hi = min(t_lo + p.clen, p.T);
   const long long base = ((long long)bi * p.H + h) * p.NC + c;
 
-  float2 S[PAIRS][8];
+  float2 S[PAIRS][4];
   auto row_of = [&](int pr) { return (pr >> 1) * 32 + ig * 4 + (pr & 1) * 2; };      // first row of a pair
-  auto col_of = [&](int k) { return warp * 32 + (k >> 1) * 8 + jg * 2 + (k & 1); };
+  auto col_of = [&](int k) { return warp * 16 + (k >> 1) * 8 + jg * 2 + (k & 1); };
 #pragma unroll
   for (int pr = 0; pr < PAIRS; ++pr)
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 0; k < 4; ++k) {
       S[pr][k] = make_float2(0.f, 0.f);
       if (!LOCAL && p.start != nullptr) {
         const float* q = p.start + (base * N + row_of(pr)) * N + col_of(k);
         S[pr][k] = make_float2(q[0], q[N]);
       }
     }
-  // ---- reverse sweep: thread i < N carries channel i's decay-gradient sum
+  // ---- output role: channel me; of the two threads of a channel the first carries the decay-gradient sum (reverse sweep)
+  const int me = threadIdx.x % N, second = threadIdx.x / N;
   float Q = 0.f, gu = 0.f;
-  const float u_me = p.u[h * N + threadIdx.x];
-  if (MODE == WK_G && p.fstart != nullptr && c + 1 < p.NC) {
-    const float* g = p.start + (base * N + threadIdx.x) * N;
-    const float* f = p.fstart + ((base + 1) * N + threadIdx.x) * N;
+  const float u_me = p.u[h * N + me];
+  if (MODE == WK_G && !second && p.fstart != nullptr && c + 1 < p.NC) {
+    const float* g = p.start + (base * N + me) * N;
+    const float* f = p.fstart + ((base + 1) * N + me) * N;
     for (int j = 0; j < N; ++j) Q += g[j] * f[j];
   }
-  // ---- staging role: step trow (+ N / TPR per pass), 8 channels from ch8
+  // ---- staging role: step trow, 8 channels from ch8
   const int trow = threadIdx.x / TPR, ch8 = (threadIdx.x % TPR) * 8;
   float u8[8];
 #pragma unroll
@@ -127,39 +130,34 @@ __global__ void __launch_bounds__(N) wkv_kernel(const WkvParams p) {
 
   const int nsub = (t_hi - t_lo + WK_SUB - 1) / WK_SUB;
   // the next sub-block's inputs are fetched before the steps of this one
-  uint4 rw[NPASS], rb[NPASS], rc[NPASS], ra[COL ? NPASS : 1], re[ROW ? NPASS : 1];
+  uint4 rw, rb, rc, ra, re;
   auto fetch = [&](int q) {
-    const int t0 = t_lo + (REV ? nsub - 1 - q : q) * WK_SUB;
-#pragma unroll
-    for (int ps = 0; ps < NPASS; ++ps) {
-      const int t = t0 + trow + ps * (N / TPR);
-      const bool ok = t < t_hi;
-      const long long o = bi * p.sb + (long long)t * p.st + h * N + ch8;
-      rw[ps] = wk_load8<VEC>(p.w + o, ok);
-      rb[ps] = wk_load8<VEC>((REV ? p.r : p.k) + o, ok);
-      rc[ps] = wk_load8<VEC>((REV ? p.gy : p.v) + o, ok);
-      if (COL) ra[COL ? ps : 0] = wk_load8<VEC>((MODE == WK_Y ? p.r : p.k) + o, ok);
-      if (ROW) re[ROW ? ps : 0] = wk_load8<VEC>((MODE == WK_GR ? p.gy : p.v) + o, ok);
-    }
+    const int t = t_lo + (REV ? nsub - 1 - q : q) * WK_SUB + trow;
+    const bool ok = t < t_hi;
+    const long long o = bi * p.sb + (long long)t * p.st + h * N + ch8;
+    rw = wk_load8<VEC>(p.w + o, ok);
+    rb = wk_load8<VEC>((REV ? p.r : p.k) + o, ok);
+    rc = wk_load8<VEC>((REV ? p.gy : p.v) + o, ok);
+    if (COL) ra = wk_load8<VEC>((MODE == WK_Y ? p.r : p.k) + o, ok);
+    if (ROW) re = wk_load8<VEC>((MODE == WK_GR ? p.gy : p.v) + o, ok);
   };
   fetch(0);
   for (int q = 0; q < nsub; ++q) {
     const int t0 = t_lo + (REV ? nsub - 1 - q : q) * WK_SUB;
     const int steps = min(WK_SUB, t_hi - t0);
+    const long long oo = bi * p.osb + (long long)t0 * p.ost + h * N + me;
     float gr[MODE == WK_G ? WK_SUB : 1];
     if (MODE == WK_G) {
 #pragma unroll
-      for (int t = 0; t < WK_SUB; ++t)
-        gr[t] = t < steps ? p.gr32[bi * p.osb + (long long)(t0 + t) * p.ost + h * N + threadIdx.x] : 0.f;
+      for (int t = 0; t < WK_SUB; ++t) gr[t] = t < steps ? p.gr32[oo + t * p.ost] : 0.f;
     }
-#pragma unroll
-    for (int ps = 0; ps < NPASS; ++ps) {
-      const int t = trow + ps * (N / TPR);
+    {
+      const int t = trow;
       const bool ok = t < steps;
       float x[8], y[8], wv[8];
-      wk_unpack8(rw[ps], wv);
-      wk_unpack8(rb[ps], x);
-      wk_unpack8(rc[ps], y);
+      wk_unpack8(rw, wv);
+      wk_unpack8(rb, x);
+      wk_unpack8(rc, y);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float ew = ok ? -__expf(wv[j]) : 0.f;
@@ -170,7 +168,7 @@ __global__ void __launch_bounds__(N) wkv_kernel(const WkvParams p) {
       }
       if (COL) {
         float a[8], dt = 0.f;
-        wk_unpack8(ra[COL ? ps : 0], a);
+        wk_unpack8(ra, a);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           s.a[t][ch8 + j] = a[j];
@@ -182,7 +180,7 @@ __global__ void __launch_bounds__(N) wkv_kernel(const WkvParams p) {
       }
       if (ROW) {
         float e[8], dt = 0.f;
-        wk_unpack8(re[ROW ? ps : 0], e);
+        wk_unpack8(re, e);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           s.e[t][ch8 + j] = make_float2(e[j], e[j]);
@@ -198,7 +196,7 @@ __global__ void __launch_bounds__(N) wkv_kernel(const WkvParams p) {
 #pragma unroll 2
     for (int tq = 0; tq < steps; ++tq) {
       const int t = REV ? steps - 1 - tq : tq;
-      float2 dv[PAIRS], bv[PAIRS], av[PAIRS], racc[PAIRS], cacc[8];
+      float2 dv[PAIRS], bv[PAIRS], av[PAIRS], racc[PAIRS], cacc[4];
 #pragma unroll
       for (int g = 0; g < QUADS; ++g) {
         const float4 d4 = *reinterpret_cast<const float4*>(&s.d[t][g * 32 + ig * 4]);
@@ -211,10 +209,10 @@ __global__ void __launch_bounds__(N) wkv_kernel(const WkvParams p) {
         }
       }
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        const float4 c4 = *reinterpret_cast<const float4*>(&s.c[t][warp * 32 + m * 8 + jg * 2]);
+      for (int m = 0; m < 2; ++m) {
+        const float4 c4 = *reinterpret_cast<const float4*>(&s.c[t][warp * 16 + m * 8 + jg * 2]);
         float4 e4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (ROW) e4 = *reinterpret_cast<const float4*>(&s.e[t][warp * 32 + m * 8 + jg * 2]);
+        if (ROW) e4 = *reinterpret_cast<const float4*>(&s.e[t][warp * 16 + m * 8 + jg * 2]);
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
           const int k = 2 * m + x;
@@ -228,18 +226,17 @@ __global__ void __launch_bounds__(N) wkv_kernel(const WkvParams p) {
           }
         }
       }
-      if (COL) {      // 8 columns over the 8 row groups: lane ig ends up with its column ig
-        float v8[8], v4[4], v2[2];
+      if (COL) {      // 4 columns over the 8 row groups: lanes ig = 2 k, 2 k + 1 end up with column k
+        float v4[4], v2[2];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v8[k] = cacc[k].x + cacc[k].y;
-        const bool h2 = ig & 4, h1 = ig & 2, h0 = ig & 1;
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          v4[k] = (h2 ? v8[4 + k] : v8[k]) + __shfl_xor_sync(0xffffffffu, h2 ? v8[k] : v8[4 + k], 16);
+        for (int k = 0; k < 4; ++k) v4[k] = cacc[k].x + cacc[k].y;
+        const bool h2 = ig & 4, h1 = ig & 2;
 #pragma unroll
         for (int k = 0; k < 2; ++k)
-          v2[k] = (h1 ? v4[2 + k] : v4[k]) + __shfl_xor_sync(0xffffffffu, h1 ? v4[k] : v4[2 + k], 8);
-        s.colsum[t][col_of(ig)] = (h0 ? v2[1] : v2[0]) + __shfl_xor_sync(0xffffffffu, h0 ? v2[0] : v2[1], 4);
+          v2[k] = (h2 ? v4[2 + k] : v4[k]) + __shfl_xor_sync(0xffffffffu, h2 ? v4[k] : v4[2 + k], 16);
+        float v = (h1 ? v2[1] : v2[0]) + __shfl_xor_sync(0xffffffffu, h1 ? v2[0] : v2[1], 8);
+        v += __shfl_xor_sync(0xffffffffu, v, 4);
+        if (!(ig & 1)) s.colsum[t][col_of(ig >> 1)] = v;
       }
       if (ROW) {      // a lane's N / 8 rows over the 4 column groups
         const bool h1 = jg & 2, h0 = jg & 1;
@@ -262,36 +259,45 @@ __global__ void __launch_bounds__(N) wkv_kernel(const WkvParams p) {
       }
     }
     __syncthreads();
-    const int me = threadIdx.x;
-    const long long oo = bi * p.osb + (long long)t0 * p.ost + h * N + me;
     if (LOCAL) {
-      for (int t = 0; t < steps; ++t) sew += s.ew[t][me];
-    } else {
-      // (thread me: channel me, step by step in the sweep's direction)
+      if (!second)
+        for (int t = 0; t < steps; ++t) sew += s.ew[t][me];
+    } else if (MODE != WK_G) {
+      // the two threads of a channel take half of the steps each
 #pragma unroll
-      for (int tq = 0; tq < WK_SUB; ++tq) {
-        const int t = REV ? WK_SUB - 1 - tq : tq;
+      for (int tq = 0; tq < WK_SUB / 2; ++tq) {
+        const int t = second * (WK_SUB / 2) + tq;
         if (t >= steps) continue;
-        float row = 0.f;
-        if (ROW) {
-#pragma unroll
-          for (int w = 0; w < QUADS; ++w) row += s.rowsum[w][t][me];
-        }
         if (MODE == WK_Y) {
           p.y[oo + t * p.ost] = float_to_h16(s.colsum[t][me] + s.c[t][me].x * s.dot_col[t]);
-        } else if (MODE == WK_GR) {
-          p.gr32[oo + t * p.ost] = row + u_me * s.b[t][me] * s.dot_row[t];
         } else {
-          const float r_ = s.b[t][me], k_ = s.a[t][me], st = s.dot_row[t];
-          const float gk = row + u_me * r_ * st;
-          const float g = gr[MODE == WK_G ? t : 0];
-          p.o_gr[oo + t * p.ost] = float_to_h16(g);
-          p.o_gk[oo + t * p.ost] = float_to_h16(gk);
-          p.o_gv[oo + t * p.ost] = float_to_h16(s.colsum[t][me] + s.c[t][me].x * s.dot_col[t]);
-          p.o_gw[oo + t * p.ost] = float_to_h16((Q - k_ * row) * s.ew[t][me]);
-          Q += r_ * g - k_ * gk;
-          gu += r_ * k_ * st;
+          float row = 0.f;
+#pragma unroll
+          for (int w = 0; w < N / 16; ++w) row += s.rowsum[ROW ? w : 0][ROW ? t : 0][me];
+          p.gr32[oo + t * p.ost] = row + u_me * s.b[t][me] * s.dot_row[t];
         }
+      }
+    } else if (second) {
+#pragma unroll
+      for (int t = 0; t < WK_SUB; ++t) {
+        if (t >= steps) continue;
+        p.o_gr[oo + t * p.ost] = float_to_h16(gr[MODE == WK_G ? t : 0]);
+        p.o_gv[oo + t * p.ost] = float_to_h16(s.colsum[COL ? t : 0][me] + s.c[t][me].x * s.dot_col[t]);
+      }
+    } else {
+#pragma unroll
+      for (int tq = 0; tq < WK_SUB; ++tq) {      // in the sweep's direction
+        const int t = WK_SUB - 1 - tq;
+        if (t >= steps) continue;
+        float row = 0.f;
+#pragma unroll
+        for (int w = 0; w < N / 16; ++w) row += s.rowsum[ROW ? w : 0][ROW ? t : 0][me];
+        const float r_ = s.b[t][me], k_ = s.a[COL ? t : 0][me], st = s.dot_row[t];
+        const float gk = row + u_me * r_ * st;
+        p.o_gk[oo + t * p.ost] = float_to_h16(gk);
+        p.o_gw[oo + t * p.ost] = float_to_h16((Q - k_ * row) * s.ew[t][me]);
+        Q += r_ * gr[MODE == WK_G ? t : 0] - k_ * gk;
+        gu += r_ * k_ * st;
       }
     }
     __syncthreads();
@@ -300,14 +306,14 @@ __global__ void __launch_bounds__(N) wkv_kernel(const WkvParams p) {
 #pragma unroll
     for (int pr = 0; pr < PAIRS; ++pr)
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
+      for (int k = 0; k < 4; ++k) {
         float* o = p.local + (base * N + row_of(pr)) * N + col_of(k);
         o[0] = S[pr][k].x;
         o[N] = S[pr][k].y;
       }
-    p.sumew[base * N + threadIdx.x] = sew;
+    if (!second) p.sumew[base * N + me] = sew;
   }
-  if (MODE == WK_G) atomicAdd(p.gu + h * N + threadIdx.x, gu);
+  if (MODE == WK_G && !second) atomicAdd(p.gu + h * N + me, gu);
 }
 
 // start[c] for every chunk: forward  start[0] = 0, start[c+1] = P_c start[c] + local[c];
@@ -335,24 +341,25 @@ static int wkv_launch(const WkvParams& p, bool vec, int chunks, cudaStream_t str
     attr_set = true;
   }
   const dim3 grid(chunks, p.H, p.B);
-  if (vec) wkv_kernel<N, MODE, true><<<grid, N, smem, stream>>>(p);
-  else wkv_kernel<N, MODE, false><<<grid, N, smem, stream>>>(p);
+  if (vec) wkv_kernel<N, MODE, true><<<grid, 2 * N, smem, stream>>>(p);
+  else wkv_kernel<N, MODE, false><<<grid, 2 * N, smem, stream>>>(p);
   NX_LAUNCH_CHECK();
   return NX_OK;
 }
 
-// Chunks the sequence is cut into: time goes with the CTAs of the fullest SM times the chunk length; more than one
-// chunk adds the local pass (2 of the sweep's 3 operations) over all chunks but one.  Below four CTAs (two warps per
-// scheduler) an SM does not overlap its steps' exchanges and loads with arithmetic.
+// Chunks the sequence is cut into.  The sweeps are bound by latency until an SM holds WK_CTAS CTAs, so time goes with the
+// chunk length times the number of rounds the CTAs take; more than one chunk adds the local pass (2 of the sweep's 3
+// operations) over all chunks but one, and the fold.
+constexpr int WK_CTAS = 3;
 static int wkv_chunk_count(int B, int T, int H) {
-  const int subs = (T + WK_SUB - 1) / WK_SUB, sms = sm_count();
+  const int subs = (T + WK_SUB - 1) / WK_SUB, slots = WK_CTAS * sm_count();
   int best = 1;
   float best_cost = 1e30f;
   for (int nc = 1; nc <= WK_MAX_CHUNKS && nc <= subs; ++nc) {
     const int len = (subs + nc - 1) / nc;
     if ((subs + len - 1) / len != nc) continue;
-    const long long per_sm = (static_cast<long long>(B) * H * nc + sms - 1) / sms;
-    const float cost = len * fmaxf(static_cast<float>(per_sm), 2.f) * (1.f + 0.67f * (nc - 1) / nc) + 0.05f * subs * (nc > 1);
+    const long long rounds = (static_cast<long long>(B) * H * nc + slots - 1) / slots;
+    const float cost = len * rounds * (1.f + 0.67f * (nc - 1) / nc) + (nc > 1 ? 0.5f + 0.1f * nc : 0.f);
     if (cost < best_cost) {
       best_cost = cost;
       best = nc;
