@@ -11,12 +11,12 @@
 // chip busy (scan_chunk_count): one chunk needs one pass; with more, a light pass first runs every chunk from a zero
 // state and records its end state and its sum of delta (the chunk's decay is exp(A * sum delta)), and the main pass
 // folds the earlier chunks into its start state.  The reverse recurrence of dL/dh is cut the same way.
-// The forward keeps the state at the start of every 32-step block for the backward, which recomputes 16 steps at a
+// The forward keeps the state at the start of every 32-step block for the backward, which recomputes 8 steps at a
 // time into registers and walks them in reverse.
 // Bound by the exponentials exp(delta A), one per (step, channel, state) on the 16-lane special-function pipe, and
 // in the backward by instruction issue; memory traffic is a tenth of either.  Convolution + scan, forward + backward, 4 x
-// 2048 steps of 1536 channels: 1.78 ms before (all chunks of 128 steps in two passes each way, the states recomputed in
-// three of them, scalar staging), 0.98 ms now.
+// 2048 steps of 1536 channels: 1.78 ms with chunks of 128 steps in two passes each way, the states recomputed in three of
+// them and scalar staging; 0.98 ms with two (forward three) CTAs an SM; 0.86 ms now.
 #include "common.h"
 #include "ptx.cuh"
 
@@ -329,10 +329,12 @@ NX_API int NX_SYM(nx_conv1d_silu_bwd)(const void* x, long long xsb, long long xs
 // ---------------------------------------------------------------------------------------------
 constexpr int SC_CH = 32;       // channels per CTA
 constexpr int SC_T = 32;        // timesteps per block (staged together; the forward keeps a state per block)
-constexpr int SC_HALF = 16;     // steps whose states the backward holds in registers
+constexpr int SC_REG = 8;       // steps whose states the backward holds in registers
 constexpr int SC_THREADS = SC_CH * 4;
 constexpr int SC_LD = 40;       // row length of the [step][channel] result arrays: four steps land on distinct banks
 constexpr int SC_MAX_CHUNKS = 32;
+constexpr int SC_FWD_CTAS = 5, SC_BWD_CTAS = 3;   // CTAs per SM: latency (exponentials, shared memory, exchanges) is hidden
+                                                  // by other warps, so registers are bounded for more of them
 constexpr float LOG2E = 1.44269504088896340736f, LN2 = 0.69314718055994530942f;
 
 struct ScanParams {
@@ -431,7 +433,7 @@ __device__ __forceinline__ float4 f4(const float2 (&h)[2]) { return make_float4(
 
 // FINAL = false: chunks 0 .. NC - 2 from a zero state -> end state and sum of delta.
 template <bool FINAL, bool VEC>
-__global__ void __launch_bounds__(SC_THREADS)
+__global__ void __launch_bounds__(SC_THREADS, SC_FWD_CTAS)
 scan_fwd_kernel(const ScanParams p) {
   __shared__ __align__(16) float2 dd[SC_T][SC_CH];        // (delta, delta * x)
   __shared__ __align__(16) float Bs[SC_T][16], Cs[FINAL ? SC_T : 1][16];
@@ -491,7 +493,7 @@ scan_fwd_kernel(const ScanParams p) {
       *reinterpret_cast<float4*>(p.ckpt + (((long long)b * ((p.L + SC_T - 1) / SC_T) + t0 / SC_T) * p.D + d) * 16 + q * 4) =
           f4(h);
     __syncthreads();
-#pragma unroll
+#pragma unroll 2
     for (int g = 0; g < SC_T; g += 4) {
       float yp[4];
 #pragma unroll
@@ -596,12 +598,13 @@ struct ScanBwdSmem {
   float Bs[SC_T][16], Cs[SC_T][16];
   float dzf[SC_T][SC_LD];                     // d out / d z without the scan value
   float s_gb[SC_T][SC_LD], s_da[SC_T][SC_LD], s_hc[SC_T][SC_LD];   // sums over the 16 states
+  float4 ck[SC_T / SC_REG][SC_THREADS];       // states at the starts of the block's quarters
   float acc[SC_THREADS][17];                  // dD and dbias of a staging thread's 8 channels
   float bc[SC_THREADS / 32][SC_T][32];
 };
 
 template <bool VEC>
-__global__ void __launch_bounds__(SC_THREADS, 2)
+__global__ void __launch_bounds__(SC_THREADS, SC_BWD_CTAS)
 scan_bwd_kernel(const ScanParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   ScanBwdSmem& s = *reinterpret_cast<ScanBwdSmem*>(smem_raw);
@@ -673,29 +676,37 @@ scan_bwd_kernel(const ScanParams p) {
     }
     put_bc(s.Bs, bv);
     put_bc(s.Cs, cv);
-    const float2 h0[2] = {{hc.x, hc.y}, {hc.z, hc.w}};
-    if (t0 - SC_T >= tc0) fetch(t0 - SC_T);       // in flight during this block
     __syncthreads();
-    // the state at the middle of the block
-    float2 hm[2] = {h0[0], h0[1]};
-#pragma unroll 4
-    for (int t = 0; t < SC_HALF; ++t) {
-      const float4 v = s.dd[t][ch];
-      const float4 B4 = *reinterpret_cast<const float4*>(&s.Bs[t][q * 4]);
-      const float2 dx2 = make_float2(v.y, v.y);
-      float2 a[2];
-      exp4(A01, A23, v.x, a);
-      hm[0] = ffma2(a[0], hm[0], fmul2(dx2, make_float2(B4.x, B4.y)));
-      hm[1] = ffma2(a[1], hm[1], fmul2(dx2, make_float2(B4.z, B4.w)));
-    }
+    // the states at the starts of the quarters (read back by the thread that wrote them)
+    {
+      float2 h[2] = {{hc.x, hc.y}, {hc.z, hc.w}};
+      s.ck[0][threadIdx.x] = f4(h);
 #pragma unroll 1
-    for (int half = 1; half >= 0; --half) {
-      const int tb = half * SC_HALF;
-      float2 hs[SC_HALF + 1][2], as[SC_HALF][2];  // hs[t + 1]: state after step t
-      hs[0][0] = half ? hm[0] : h0[0];
-      hs[0][1] = half ? hm[1] : h0[1];
+      for (int quarter = 1; quarter < SC_T / SC_REG; ++quarter) {
 #pragma unroll
-      for (int t = 0; t < SC_HALF; ++t) {
+        for (int k = 0; k < SC_REG; ++k) {
+          const int t = (quarter - 1) * SC_REG + k;
+          const float4 v = s.dd[t][ch];
+          const float4 B4 = *reinterpret_cast<const float4*>(&s.Bs[t][q * 4]);
+          const float2 dx2 = make_float2(v.y, v.y);
+          float2 a[2];
+          exp4(A01, A23, v.x, a);
+          h[0] = ffma2(a[0], h[0], fmul2(dx2, make_float2(B4.x, B4.y)));
+          h[1] = ffma2(a[1], h[1], fmul2(dx2, make_float2(B4.z, B4.w)));
+        }
+        s.ck[quarter][threadIdx.x] = f4(h);
+      }
+    }
+    if (t0 - SC_T >= tc0) fetch(t0 - SC_T);       // in flight during this block
+#pragma unroll 1
+    for (int quarter = SC_T / SC_REG - 1; quarter >= 0; --quarter) {
+      const int tb = quarter * SC_REG;
+      float2 hs[SC_REG + 1][2], as[SC_REG][2];    // hs[t + 1]: state after step t
+      const float4 h0 = s.ck[quarter][threadIdx.x];
+      hs[0][0] = make_float2(h0.x, h0.y);
+      hs[0][1] = make_float2(h0.z, h0.w);
+#pragma unroll
+      for (int t = 0; t < SC_REG; ++t) {
         const float4 v = s.dd[tb + t][ch];
         const float4 B4 = *reinterpret_cast<const float4*>(&s.Bs[tb + t][q * 4]);
         const float2 dx2 = make_float2(v.y, v.y);
@@ -704,7 +715,7 @@ scan_bwd_kernel(const ScanParams p) {
         hs[t + 1][1] = ffma2(as[t][1], hs[t][1], fmul2(dx2, make_float2(B4.z, B4.w)));
       }
 #pragma unroll
-      for (int g = SC_HALF - 4; g >= 0; g -= 4) {
+      for (int g = SC_REG - 4; g >= 0; g -= 4) {
         float v_gb[4], v_da[4], v_hc[4];
 #pragma unroll
         for (int u = 3; u >= 0; --u) {
@@ -812,18 +823,18 @@ scan_bc_reduce_kernel(const float* __restrict__ part, int ntiles, long long rows
   *reinterpret_cast<uint2*>(o) = make_uint2(pack_h16x2(a.x, a.y), pack_h16x2(a.z, a.w));
 }
 
-// Chunks the sequence is cut into.  Time goes with the largest number of CTAs an SM gets times the chunk length; more
-// than one chunk adds the light pass over all chunks but one (about `light` of the main pass).
-static int scan_chunk_count(int B, int L, int D, float light) {
-  const int tiles = (D + SC_CH - 1) / SC_CH * B, blocks = (L + SC_T - 1) / SC_T, sms = sm_count();
+// Chunks the sequence is cut into.  The kernels are bound by latency until an SM holds its `ctas` CTAs, so time goes with
+// the chunk length times the number of rounds the CTAs take; more than one chunk adds the light pass over all chunks but
+// one (about `light` of the main pass).
+static int scan_chunk_count(int B, int L, int D, int ctas, float light) {
+  const int tiles = (D + SC_CH - 1) / SC_CH * B, blocks = (L + SC_T - 1) / SC_T, slots = ctas * sm_count();
   int best = 1;
   float best_cost = 1e30f;
   for (int nc = 1; nc <= SC_MAX_CHUNKS && nc <= blocks; ++nc) {
     const int len = (blocks + nc - 1) / nc, real = (blocks + len - 1) / len;
     if (real != nc) continue;
-    const int per_sm = static_cast<int>((static_cast<long long>(tiles) * nc + sms - 1) / sms);
-    // below four CTAs (one warp per scheduler each) an SM does not overlap enough to reach its full rate
-    const float cost = len * fmaxf(static_cast<float>(per_sm), 1.5f) * (1.f + light * (nc - 1) / nc) + 0.02f * blocks * (nc > 1);
+    const int rounds = static_cast<int>((static_cast<long long>(tiles) * nc + slots - 1) / slots);
+    const float cost = len * rounds * (1.f + light * (nc - 1) / nc) + 0.02f * blocks * (nc > 1);
     if (cost < best_cost) {
       best_cost = cost;
       best = nc;
@@ -834,14 +845,14 @@ static int scan_chunk_count(int B, int L, int D, float light) {
 constexpr float LIGHT_FWD = 0.6f, LIGHT_BWD = 0.25f;
 
 NX_API int NX_SYM(nx_scan_chunks)(int B, int L, int D, int backward) {
-  return scan_chunk_count(B, L, D, backward ? LIGHT_BWD : LIGHT_FWD);
+  return scan_chunk_count(B, L, D, backward ? SC_BWD_CTAS : SC_FWD_CTAS, backward ? LIGHT_BWD : LIGHT_FWD);
 }
 NX_API int NX_SYM(nx_scan_channel_blocks)(int D) { return (D + SC_CH - 1) / SC_CH; }
 NX_API int NX_SYM(nx_scan_blocks)(int L) { return (L + SC_T - 1) / SC_T; }
 
-static void scan_common(ScanParams& p, int B, int L, int D, float light) {
+static void scan_common(ScanParams& p, int B, int L, int D, int ctas, float light) {
   p.B = B; p.L = L; p.D = D;
-  p.NC = scan_chunk_count(B, L, D, light);
+  p.NC = scan_chunk_count(B, L, D, ctas, light);
   p.clen = ((L + SC_T - 1) / SC_T + p.NC - 1) / p.NC * SC_T;
 }
 
@@ -865,7 +876,7 @@ NX_API int NX_SYM(nx_selective_scan_fwd)(const void* x, long long xsb, long long
   p.out = (h16*)out; p.osb = osb; p.ost = ost;
   p.chunk_state = (float*)chunk_state; p.chunk_sumdt = (float*)chunk_sumdt; p.ckpt = (float*)ckpt;
   if (B <= 0 || L <= 0 || D <= 0) return NX_OK;
-  scan_common(p, B, L, D, LIGHT_FWD);
+  scan_common(p, B, L, D, SC_FWD_CTAS, LIGHT_FWD);
   const bool vec = D % 8 == 0 && vec_ok(x, xsb, xst, 8) && vec_ok(dt, dsb, dst, 8) && vec_ok(z, zsb, zst, 8) &&
                    vec_ok(out, osb, ost, 8);
   const dim3 grid((D + SC_CH - 1) / SC_CH, p.NC, B);
@@ -904,7 +915,7 @@ NX_API int NX_SYM(nx_selective_scan_bwd)(const void* x, long long xsb, long long
   p.partBC = (float*)partBC; p.dA = (float*)dA; p.dD = (float*)dD; p.dbias = (float*)dbias;
   p.ckpt = (float*)ckpt; p.chunk_state = (float*)chunk_state; p.chunk_sumdt = (float*)chunk_sumdt;
   if (B <= 0 || L <= 0 || D <= 0) return NX_OK;
-  scan_common(p, B, L, D, LIGHT_BWD);
+  scan_common(p, B, L, D, SC_BWD_CTAS, LIGHT_BWD);
   const bool vec = D % 8 == 0 && vec_ok(x, xsb, xst, 8) && vec_ok(dt, dsb, dst, 8) && vec_ok(z, zsb, zst, 8) &&
                    vec_ok(dout, gsb, gst, 8) && vec_ok(dx, osb, ost, 8) && vec_ok(ddt, osb, ost, 8) &&
                    vec_ok(dz, osb, ost, 8);

@@ -92,27 +92,33 @@ def selective_scan_reference(x, dt, A, Bm, Cm, D=None, z=None, dt_bias=None):
     return y.to(dtype)
 
 
+def _scan_forward(x, dt, A, Bm, Cm, D, z, dt_bias, keep):
+    """-> (output, ``keep``: the state at the start of every 32-step block, for the backward, else None)."""
+    L_ = _lib.lib(x)
+    B, L, Dm = x.shape
+    dev = x.device
+    nc = L_.nx_scan_chunks(B, L, Dm, 0)
+    out = torch.empty((L, B, Dm), device=dev, dtype=x.dtype).transpose(0, 1)   # time-major memory
+    state = sumdt = ckpt = None
+    if nc > 1:
+        state = torch.empty((B, nc, Dm, 16), device=dev, dtype=torch.float32)
+        sumdt = torch.empty((B, nc, Dm), device=dev, dtype=torch.float32)
+    if keep:
+        ckpt = torch.empty((B, L_.nx_scan_blocks(L), Dm, 16), device=dev, dtype=torch.float32)
+    zs = (z.stride(0), z.stride(1)) if z is not None else (0, 0)
+    LAUNCHES["n"] += 2 if nc > 1 else 1
+    _lib.check(L_.nx_selective_scan_fwd(
+        _lib.ptr(x), x.stride(0), x.stride(1), _lib.ptr(dt), dt.stride(0), dt.stride(1), _lib.ptr(z), zs[0],
+        zs[1], _lib.ptr(Bm), Bm.stride(0), Bm.stride(1), _lib.ptr(Cm), Cm.stride(0), Cm.stride(1),
+        _lib.ptr(A), _lib.ptr(D), _lib.ptr(dt_bias), _lib.ptr(out), out.stride(0), out.stride(1),
+        _lib.ptr(state), _lib.ptr(sumdt), _lib.ptr(ckpt), B, L, Dm, _lib.stream()), "nx_selective_scan_fwd")
+    return out, ckpt
+
+
 class _ScanFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, dt, A, Bm, Cm, D, z, dt_bias):
-        L_ = _lib.lib(x)
-        B, L, Dm = x.shape
-        dev = x.device
-        nc = L_.nx_scan_chunks(B, L, Dm, 0)
-        out = torch.empty((L, B, Dm), device=dev, dtype=x.dtype).transpose(0, 1)   # time-major memory
-        state = sumdt = ckpt = None
-        if nc > 1:
-            state = torch.empty((B, nc, Dm, 16), device=dev, dtype=torch.float32)
-            sumdt = torch.empty((B, nc, Dm), device=dev, dtype=torch.float32)
-        if any(ctx.needs_input_grad):       # the state at the start of every 32-step block, for the backward
-            ckpt = torch.empty((B, L_.nx_scan_blocks(L), Dm, 16), device=dev, dtype=torch.float32)
-        zs = (z.stride(0), z.stride(1)) if z is not None else (0, 0)
-        LAUNCHES["n"] += 2 if nc > 1 else 1
-        _lib.check(L_.nx_selective_scan_fwd(
-            _lib.ptr(x), x.stride(0), x.stride(1), _lib.ptr(dt), dt.stride(0), dt.stride(1), _lib.ptr(z), zs[0],
-            zs[1], _lib.ptr(Bm), Bm.stride(0), Bm.stride(1), _lib.ptr(Cm), Cm.stride(0), Cm.stride(1),
-            _lib.ptr(A), _lib.ptr(D), _lib.ptr(dt_bias), _lib.ptr(out), out.stride(0), out.stride(1),
-            _lib.ptr(state), _lib.ptr(sumdt), _lib.ptr(ckpt), B, L, Dm, _lib.stream()), "nx_selective_scan_fwd")
+        out, ckpt = _scan_forward(x, dt, A, Bm, Cm, D, z, dt_bias, any(ctx.needs_input_grad))
         ctx.save_for_backward(x, dt, A, Bm, Cm, D, z, dt_bias, ckpt)
         return out
 
@@ -163,6 +169,8 @@ def selective_scan(x, dt, A, Bm, Cm, D=None, z=None, dt_bias=None):
         A = A.float().contiguous()
         if A.data_ptr() % 16:           # the kernels read a channel's states 16 bytes at a time
             A = A.clone()
-        return _ScanFn.apply(x, dt, A, Bm, Cm, None if D is None else D.float().contiguous(),
-                             z, dt_bias.float().contiguous())
+        D, dt_bias = None if D is None else D.float().contiguous(), dt_bias.float().contiguous()
+        if _lib.untracked():
+            return _scan_forward(x, dt, A, Bm, Cm, D, z, dt_bias, False)[0]
+        return _ScanFn.apply(x, dt, A, Bm, Cm, D, z, dt_bias)
     return selective_scan_reference(x, dt, A, Bm, Cm, D, z, dt_bias)
