@@ -5,7 +5,7 @@
 
 namespace nx {
 
-constexpr int SKINNY_MAX_M = 256;
+constexpr int SKINNY_MAX_M = 128;
 
 struct SkinnyParams {
   int M, N, K;

@@ -2,14 +2,14 @@
 //
 // Bound by reading W once.  The 128 x 256 tiles of gemm_tcgen05.cu give such a product ceil(N / 256) CTAs, each walking
 // the whole reduction: 16 CTAs of 148 SMs for N = 4096.  Here the roles are swapped: W supplies the 128-row operand of
-// the MMA and the few rows of A its N operand (NX = M rounded up to 16 .. 256), so no MMA row is padding, and the
+// the MMA and the few rows of A its N operand (NX = M rounded up to 16 .. 128), so no MMA row is padding, and the
 // reduction is cut over the CTAs of a cluster until about two CTAs per SM stream W.  The partial tiles (fp32) meet in
 // distributed shared memory in rank order: one launch, no workspace, a result that does not depend on timing.
 //
 // 4 rows x (4096 -> 22016, 11008 -> 4096): 54 us for both, 5.0 TB/s of weights (164 us before, 1.6 TB/s).
 //
 // 192 threads: warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 epilogue.  A TMEM lane is a row of W, i.e. a column
-// of C, so a warp's store of one row of C is 32 consecutive elements.
+// of C: the accumulator goes through shared memory and leaves as 4 columns per thread.
 #include "gemm_skinny.h"
 
 #include <cooperative_groups.h>
@@ -39,25 +39,41 @@ struct SkinnySmem {
   static constexpr int DYN = BAR_OFF + (2 * STAGES + 2) * 8 + 1024;
 };
 
-// One element of C (row m, column n) from its accumulator value.
-__device__ __forceinline__ void skinny_store(const SkinnyParams& p, int m, int n, float v, float bias) {
-  if (p.flags & SK_SCALE) v *= p.alpha;
-  v += bias;
+// Four elements of C (row m, columns n .. n + 3) from their accumulator values.
+__device__ __forceinline__ void skinny_store4(const SkinnyParams& p, int m, int n, float4 acc, const float (&bias)[4]) {
+  float v[4] = {acc.x, acc.y, acc.z, acc.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (p.flags & SK_SCALE) v[j] *= p.alpha;
+    v[j] += bias[j];
+  }
+  const long long aux = m * p.ld_aux + n;
   if (p.flags & SK_AUX_OUT) {
-    float d = v;
+    float d[4] = {v[0], v[1], v[2], v[3]};
     if (p.flags & SK_AUX_DERIV) {       // derivative out, activation in place
-      const float x = v;
-      if (p.flags & SK_GELU_TANH) gelu_tanh_both(x, v, d);
-      else gelu_erf_both(x, v, d);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (p.flags & SK_GELU_TANH) gelu_tanh_both(v[j], v[j], d[j]);
+        else gelu_erf_both(v[j], v[j], d[j]);
+      }
     }
-    p.aux_out[m * p.ld_aux + n] = float_to_h16(d);
+    *reinterpret_cast<uint2*>(p.aux_out + aux) = make_uint2(pack_h16x2(d[0], d[1]), pack_h16x2(d[2], d[3]));
   }
   if (!(p.flags & SK_AUX_DERIV)) {
-    if (p.flags & SK_GELU_ERF) v = gelu_erf(v);
-    else if (p.flags & SK_GELU_TANH) v = gelu_tanh(v);
+    if (p.flags & SK_GELU_ERF) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = gelu_erf(v[j]);
+    } else if (p.flags & SK_GELU_TANH) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = gelu_tanh(v[j]);
+    }
   }
-  if (p.flags & SK_RESIDUAL) v += h16_to_float(p.residual[m * p.ld_aux + n]);
-  p.C[m * p.ldc + n] = float_to_h16(v);
+  if (p.flags & SK_RESIDUAL) {
+    const uint2 r = *reinterpret_cast<const uint2*>(p.residual + aux);
+    const float2 a = unpack_h16x2(r.x), b = unpack_h16x2(r.y);
+    v[0] += a.x; v[1] += a.y; v[2] += b.x; v[3] += b.y;
+  }
+  *reinterpret_cast<uint2*>(p.C + m * p.ldc + n) = make_uint2(pack_h16x2(v[0], v[1]), pack_h16x2(v[2], v[3]));
 }
 
 template <int NX, int STAGES>
@@ -129,29 +145,20 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       if (!aborted) umma_commit(done_bar);
     }
   }
-  // ---- epilogue warps: the accumulator, then C or the partial tile
-  const int col = (warp & 3) * 32 + lane;                   // row of W in the tile == TMEM lane
-  const int n = n0 + col;
-  float* part = reinterpret_cast<float*>(sgen);             // [NX][SK_BW]
-  float bias = 0.f;
+  // ---- epilogue warps: the accumulator to shared memory as [row of A][row of W], then 4 columns of C per thread
+  float* part = reinterpret_cast<float*>(sgen);             // [NX][SK_BW], over the drained ring
   if (warp >= 2) {
+    const int col = (warp & 3) * 32 + lane;                 // row of W in the tile == TMEM lane
     aborted = !__all_sync(0xffffffffu, mbar_wait(done_bar, 0, p.err, 72));
     tc_fence_after_sync();
-    if ((p.flags & SK_BIAS) && n < p.N) bias = h16_to_float(p.bias[n]);
     if (!aborted) {
 #pragma unroll 1
       for (int c = 0; c < NX && c < p.M; c += 16) {
         uint32_t r[16];
         tmem_ld_32x32b_x16(tmem + c + (static_cast<uint32_t>((warp & 3) * 32) << 16), r);
         tmem_ld_wait();
-        if (nsplit == 1) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (c + j < p.M && n < p.N) skinny_store(p, c + j, n, __uint_as_float(r[j]), bias);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) part[(c + j) * SK_BW + col] = __uint_as_float(r[j]);
-        }
+        for (int j = 0; j < 16; ++j) part[(c + j) * SK_BW + col] = __uint_as_float(r[j]);
       }
     }
   }
@@ -159,17 +166,39 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   if (aborted) {
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);       // copies in flight land before the shared memory goes away
   }
-  if (nsplit > 1) {
-    cluster.sync();
-    if (warp >= 2 && !aborted && n < p.N) {
-      for (int m = split; m < p.M; m += nsplit) {
-        float v = 0.f;
-        for (int r = 0; r < nsplit; ++r) v += cluster.map_shared_rank(part, r)[m * SK_BW + col];
-        skinny_store(p, m, n, v, bias);
+  if (nsplit > 1) cluster.sync();
+  else __syncthreads();
+  if (warp >= 2 && !aborted) {
+    const int t = threadIdx.x - 64, n = n0 + (t & 31) * 4;
+    if (n < p.N) {
+      float bias[4] = {0.f, 0.f, 0.f, 0.f};
+      if (p.flags & SK_BIAS) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) bias[j] = h16_to_float(p.bias[n + j]);
+      }
+      // the cluster's CTAs take 4 rows each in turn; the partial tiles are added in rank order, their loads issued together
+      for (int m = split * 4 + (t >> 5); m < p.M; m += nsplit * 4) {
+        const int at = m * SK_BW + (t & 31) * 4;
+        float4 v;
+        if (nsplit == 1) {
+          v = *reinterpret_cast<const float4*>(part + at);
+        } else {
+          float4 x[SK_MAX_SPLITS];
+#pragma unroll
+          for (int r = 0; r < SK_MAX_SPLITS; ++r)
+            if (r < nsplit) x[r] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(part, r) + at);
+          v = x[0];
+#pragma unroll
+          for (int r = 1; r < SK_MAX_SPLITS; ++r)
+            if (r < nsplit) {
+              v.x += x[r].x; v.y += x[r].y; v.z += x[r].z; v.w += x[r].w;
+            }
+        }
+        skinny_store4(p, m, n, v, bias);
       }
     }
-    cluster.sync();                                         // nobody leaves while its partial tile may still be read
   }
+  if (nsplit > 1) cluster.sync();                           // nobody leaves while its partial tile may still be read
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) {
@@ -212,12 +241,11 @@ static int launch_skinny(const void* A, const void* B, long long lda, long long 
 
 int gemm_skinny_launch(const void* A, const void* B, long long lda, long long ldb, const SkinnyParams& p,
                        cudaStream_t stream) {
-  // ring depths: two CTAs fit an SM's shared memory up to NX = 128
+  // ring depths: two CTAs fit an SM's shared memory
   if (p.M <= 16) return launch_skinny<16, 6>(A, B, lda, ldb, p, stream);
   if (p.M <= 32) return launch_skinny<32, 5>(A, B, lda, ldb, p, stream);
   if (p.M <= 64) return launch_skinny<64, 4>(A, B, lda, ldb, p, stream);
-  if (p.M <= 128) return launch_skinny<128, 3>(A, B, lda, ldb, p, stream);
-  return launch_skinny<256, 4>(A, B, lda, ldb, p, stream);
+  return launch_skinny<128, 3>(A, B, lda, ldb, p, stream);
 }
 
 }  // namespace nx
