@@ -28,6 +28,7 @@
 // P_j = the first 32 columns of S_j.  NEOX_ATTN_FWD_SHAPE=1 selects the first shape.
 #include <cstdlib>
 
+#include "attention_decode.h"
 #include "common.h"
 #include "ptx.cuh"
 
@@ -558,6 +559,23 @@ NX_API int NX_SYM(nx_flash_attn_fwd)(const void* q, const void* k, const void* v
   NX_REQUIRE((o_ss % 8) == 0 && (o_sh % 8) == 0 && (o_sb % 8) == 0 &&
                  (reinterpret_cast<uintptr_t>(o) & 15) == 0,
              "flash_attn: output view must be 16-byte aligned");
+  if (Sq == 1 && dropout_p * 256.f + 0.5f < 1.f && blk_rows == nullptr) {
+    // one query row: the split-key kernel of attention_decode.cu
+    auto aligned = [](const void* t, long long sb, long long sh, long long ss) {
+      return (reinterpret_cast<uintptr_t>(t) & 15) == 0 && sb % 8 == 0 && sh % 8 == 0 && ss % 8 == 0;
+    };
+    NX_REQUIRE(aligned(q, q_sb, q_sh, q_ss) && aligned(k, k_sb, k_sh, k_ss) && aligned(v, v_sb, v_sh, v_ss),
+               "flash_attn: q / k / v views must be 16-byte aligned");
+    AttnDecodeParams d;
+    d.q = (const h16*)q; d.k = (const h16*)k; d.v = (const h16*)v; d.o = (h16*)o; d.lse = (float*)lse;
+    d.alibi = (const float*)alibi;
+    d.B = B; d.H = H; d.Hk = Hk; d.Sk = Sk; d.D = D;
+    d.q_sb = q_sb; d.q_sh = q_sh; d.k_sb = k_sb; d.k_sh = k_sh; d.k_ss = k_ss;
+    d.v_sb = v_sb; d.v_sh = v_sh; d.v_ss = v_ss; d.o_sb = o_sb; d.o_sh = o_sh;
+    d.scale_log2 = scale * 1.4426950408889634f;
+    d.key_lo = window >= 0 && Sk - 1 > window ? Sk - 1 - window : 0;
+    return attn_decode_launch(d, (cudaStream_t)stream_);
+  }
   CUtensorMap tq, tk, tv;
   // 2 (default): 64-key blocks, four softmax warps, two CTAs per SM; 1: 128-key blocks, eight softmax warps, one CTA per
   // SM; 3: 64-key blocks, eight softmax warps on 32-column half rows, two CTAs per SM

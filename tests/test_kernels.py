@@ -615,3 +615,23 @@ def test_norm_parameter_shared_by_both_norms_and_frozen_parameters():
     yr = F.layer_norm(xr, (256,), wr, b.double(), 1e-5)
     rx, rw = torch.autograd.grad([yr, yr], [xr, wr], [g1.double(), g2.double()])
     assert rel(dx, rx) < 2e-2 and rel(dw, rw) < 2e-2
+
+
+@pytest.mark.parametrize("b,h,hk,sk,d,window,alibi", [
+    (1, 1, 1, 1, 128, -1, False), (2, 4, 4, 127, 64, -1, False), (3, 12, 3, 129, 64, -1, True),
+    (1, 32, 4, 2049, 128, -1, False), (2, 6, 2, 1000, 40, 700, False), (8, 32, 32, 777, 128, -1, False),
+    (1, 16, 1, 4097, 72, 1023, True), (20, 32, 32, 300, 128, -1, False), (1, 3, 1, 511, 96, 0, False)])
+def test_one_query_attention(b, h, hk, sk, d, window, alibi):
+    """One query row per head against a cache in [seq, batch, head, dim] memory: every cluster size, group size and
+    remainder of the split-key kernel.  Only the output is rounded to 16 bits (2^-9 / 2^-12 of its size)."""
+    from gpt_neox_b200.ops.attention import _fwd, alibi_slopes, attention_reference
+    torch.manual_seed(21)
+    al = alibi_slopes(h).to(DEV) if alibi else None
+    q = bf(1, b, h, d).permute(1, 0, 2, 3)
+    cache = bf(2, sk + 3, b, hk, d)                              # a longer buffer: the keys are a view of its front
+    k, v = (t[:sk].permute(1, 0, 2, 3) for t in cache)
+    o, lse = _fwd(q, k, v, 1.0 / math.sqrt(d), True, window, al)
+    ref, rl = attention_reference(q.double(), k.double(), v.double(), window=window, alibi=al)
+    assert o.dtype == DT and rel(o, ref) < (2 ** -7 if DT == torch.bfloat16 else 2 ** -10)
+    torch.testing.assert_close(lse[:, :, 0], (rl[:, :, 0] / math.log(2.0)).float(), rtol=1e-4, atol=1e-4)
+    assert torch.isinf(lse[:, :, 1:]).all() and (lse[:, :, 1:] > 0).all()
