@@ -30,22 +30,14 @@ extern "C" {
 // rows [past, past + s) written here.
 struct nx_layer_infer_args {
   const void *x, *ln1_w, *ln1_b, *ln2_w, *ln2_b, *w_qkv, *b_qkv, *w_dense, *b_dense, *w1, *b1, *w2, *b2;
-  const void *cos, *sin, *alibi;
-  void *cache, *work, *stats, *out;     // work: 16-bit scratch, nx_layer_infer_work() elements; stats: fp32 scratch
+  const void *cos, *sin;
+  // scratch: work, 16-bit: x1, x2, the attention branch with the residual (rows x h each), qkv, context, the MLP's hidden
+  // layer; stats, fp32: mean and rstd of every row, the log-sum-exp of the attention [b, np, s rounded up to 128]
+  void *cache, *work, *stats, *out;
   long long cache_kv_stride;            // elements between the key and the value part of the cache
   int s, b, h, np, kvp, hn, ffn, past, rot, window, gelu_tanh, pair_gemm;
   float eps, scale;
 };
-}
-
-// 16-bit scratch elements: x1, x2, qkv, context, the attention branch with the residual, the MLP's hidden layer.
-NX_API long long NX_SYM(nx_layer_infer_work)(const nx_layer_infer_args* a) {
-  const long long rows = static_cast<long long>(a->s) * a->b, ctx = static_cast<long long>(a->np) * a->hn;
-  return rows * (3ll * a->h + (a->np + 2ll * a->kvp) * a->hn + ctx + a->ffn);
-}
-// fp32 scratch elements: mean and rstd of every row, the log-sum-exp of the attention.
-NX_API long long NX_SYM(nx_layer_infer_stats)(const nx_layer_infer_args* a) {
-  return 2ll * a->s * a->b + static_cast<long long>(a->b) * a->np * ((a->s + 127) / 128 * 128);
 }
 
 NX_API int NX_SYM(nx_layer_infer)(const nx_layer_infer_args* a, void* stream) {
@@ -85,7 +77,7 @@ NX_API int NX_SYM(nx_layer_infer)(const nx_layer_infer_args* a, void* stream) {
   NX_TRY(NX_SYM(nx_rope_qk)(q, k, v, kc + a->past * cs, vc + a->past * cs, a->cos, a->sin, a->s, a->b, a->np, a->kvp, hn,
                             a->rot, strides, a->past, 0, stream));
   // the context as [b, s, heads, hn] memory is what the op-by-op path writes; here it goes straight to [s, b, heads, hn]
-  NX_TRY(NX_SYM(nx_flash_attn_fwd)(q, kc, vc, ctx, lse, a->alibi, a->b, a->np, a->kvp, a->s, a->past + a->s, hn, sb, sh, ss,
+  NX_TRY(NX_SYM(nx_flash_attn_fwd)(q, kc, vc, ctx, lse, nullptr, a->b, a->np, a->kvp, a->s, a->past + a->s, hn, sb, sh, ss,
                                    cb, hn, cs, cb, hn, cs, ctx_n, hn, static_cast<long long>(a->b) * ctx_n, a->scale, 1,
                                    a->window, 0.f, 0, nullptr, nullptr, 0, stream));
   NX_TRY(gemm(ctx, a->w_dense, t, a->h, ctx_n, a->b_dense, a->x, 0));

@@ -35,11 +35,12 @@ def _claim(layer, past, stream) -> bool:
         return True
 
 
-def extend(layer, past, rows: int, like: torch.Tensor) -> torch.Tensor:
+def extend(layer, past, rows: int, like: torch.Tensor, shape=None) -> torch.Tensor:
     """The cache ``[2, n + rows, b, heads, hn]`` whose first n rows are ``past``'s (None or empty: n = 0) and whose last
-    ``rows`` rows the caller fills.  ``like``: [*, b, heads, hn], the new keys (shape, dtype and device)."""
-    n = 0 if past is None else past[0].shape[0]
-    shape = tuple(like.shape[1:])
+    ``rows`` rows the caller fills.  ``like``: a tensor of the cache's dtype and device, [*, b, heads, hn] unless ``shape``
+    gives (b, heads, hn)."""
+    n = 0 if past is None else past.shape[1] if torch.is_tensor(past) else past[0].shape[0]
+    shape = tuple(like.shape[1:]) if shape is None else shape
     stream, total = _stream(like), n + rows
     buf = None
     if torch.is_tensor(past) and past.dtype == like.dtype and past.device == like.device \

@@ -23,7 +23,7 @@ from ..ops.attention import flash_attention, next_dropout_seed
 from ..ops.elementwise import bias_dropout_add
 from ..ops.gemm import gemm as gemm_op
 from ..ops.gemm import linear as linear_op
-from ..ops.layer_infer import layer_infer, takes
+from ..ops.layer_infer import layer_infer, pointers
 from ..ops.norm import dual_layer_norm
 from ..ops import _lib as kernel_lib
 from ..ops import rope as rope_ops
@@ -491,22 +491,22 @@ class ParallelTransformerLayer(nn.Module):
                 or torch.nn.modules.module._has_any_global_hook() or any(
                     z._forward_hooks or z._forward_pre_hooks for z in mods):
             return None
-        norms = (self.input_layernorm.weight, self.input_layernorm.bias, self.post_attention_layernorm.weight,
-                 self.post_attention_layernorm.bias)
-        weights = [(l.weight, l.bias) for l in linears]
+        n1, n2, up = self.input_layernorm, self.post_attention_layernorm, m.linear1.weight
+        ptrs = pointers(x, n1.weight, n1.bias, n2.weight, n2.bias, *(t for l in linears for t in (l.weight, l.bias)))
+        if ptrs is None or n1.eps != n2.eps:
+            return None
         has_past = layer_past is not None and (not torch.is_tensor(layer_past) or layer_past.numel() > 0)
         past = layer_past[0].shape[0] if has_past else 0
         cos, sin = a.rotary_emb(seq_len=x.shape[0] + past)
-        if not takes(x, *norms, *(t for wb in weights for t in wb)) or cos.data_ptr() % 16 or sin.data_ptr() % 16 \
-                or self.input_layernorm.eps != self.post_attention_layernorm.eps:
+        if (cos.data_ptr() | sin.data_ptr()) & 15:
             return None
         kvp = a.num_kv_heads_per_partition
-        present = kv_cache.extend(a, layer_past if has_past else None, x.shape[0], x.new_empty((0, x.shape[1], kvp, hn)))
+        present = kv_cache.extend(a, layer_past if has_past else None, x.shape[0], x, (x.shape[1], kvp, hn))
         out = layer_infer(
-            x, norms, *weights, cos, sin, a.alibi_embed.slopes if a.pos_emb == "alibi" else None, present, past,
-            heads=a.num_attention_heads_per_partition, kv_heads=kvp, head_dim=hn, rot=a.rotary_dim,
-            window=a.sliding_window_width if a.sliding_window_width is not None else -1, scale=a.attn_scale,
-            eps=self.input_layernorm.eps, gelu="tanh" if m.bias_gelu_fusion else "erf")
+            x, ptrs, cos, sin, present, past,
+            heads=a.num_attention_heads_per_partition, kv_heads=kvp, head_dim=hn, ffn=up.shape[0], rot=a.rotary_dim,
+            window=a.sliding_window_width if a.sliding_window_width is not None else -1, scale=a.attn_scale, eps=n1.eps,
+            gelu="tanh" if m.bias_gelu_fusion else "erf")
         self.layer_past = present
         return out
 

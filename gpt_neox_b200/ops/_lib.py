@@ -124,8 +124,6 @@ def _declare(lib):
     sig("nx_gemm_bf16_grouped", [I, P, P, P, I, I, I, L, L, L, I, I, P, P, L, P, P, L, I, P])
     sig("nx_rope", [P, P, P, P, I, I, I, I, I, L, L, L, L, L, L, I, I, P])
     sig("nx_rope_qk", [P] * 7 + [I] * 6 + [C.POINTER(L), I, I, P])
-    sig("nx_layer_infer_work", [P], L)
-    sig("nx_layer_infer_stats", [P], L)
     sig("nx_layer_infer", [P, P])
     sig("nx_embedding_fwd", [P, P, P, L, I, L, L, P])
     sig("nx_embedding_bwd", [P, P, P, L, I, L, L, P])
