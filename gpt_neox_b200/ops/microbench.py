@@ -118,7 +118,7 @@ def build(op, a):
         dg = [torch.empty(a.n, device=dev) for _ in range(4)]
         P = _lib.ptr
         fn = lambda: _lib.check(L.nx_norm_bwd(0, P(g1), P(g2), P(x), P(mean), P(rstd), P(w1), P(w2), P(g0), P(dx),
-                                              P(dg[0]), P(dg[1]), P(dg[2]), P(dg[3]), P(ws), a.m, a.n, 0,
+                                              P(dg[0]), P(dg[1]), P(dg[2]), P(dg[3]), P(ws), a.m, a.n, 0, 0,
                                               _lib.stream()), "nx_norm_bwd")
         return fn, 0.0, 2.0 * 5 * a.m * a.n
     if op in ("scan_fwd", "scan_bwd", "conv1d"):
