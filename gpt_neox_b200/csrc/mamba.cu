@@ -13,8 +13,8 @@
 // folds the earlier chunks into its start state.  The reverse recurrence of dL/dh is cut the same way.
 // The forward keeps the state at the start of every 32-step block for the backward, which recomputes 8 steps at a
 // time into registers and walks them in reverse.
-// Bound by the exponentials exp(delta A), one per (step, channel, state) on the 16-lane special-function pipe, and
-// in the backward by instruction issue; memory traffic is a tenth of either.  Convolution + scan, forward + backward, 4 x
+// Bound by the shared-memory pipe (78-80 % busy in the main passes: a step's inputs, and the exchanges that sum dB, dC and
+// the channel sums over lanes); issue slots 42-50 %, DRAM 6-9 %.  Convolution + scan, forward + backward, 4 x
 // 2048 steps of 1536 channels: 1.78 ms with chunks of 128 steps in two passes each way, the states recomputed in three of
 // them and scalar staging; 0.98 ms with two (forward three) CTAs an SM; 0.86 ms with the exchanges of dB / dC step by
 // step; 0.82 ms now (backward sweep 418 us, 466 before).
