@@ -6,10 +6,10 @@
 // Here the keys of a head are cut over the CTAs of a cluster and, inside a CTA, over groups of DP / 8 lanes: a lane
 // owns 8 head dims (one 16-byte load of a K row, one of a V row) and a group takes UNROLL keys at a time.  The next keys'
 // K rows are loaded as soon as the scores of these have been taken, the next V rows after the sums, into the registers
-// just freed: loads are in flight throughout.  GT query heads that share a K / V head are done from the same loads.  Every group keeps
-// its own running maximum / sum / output in fp32 registers; groups meet through shuffles and shared memory, CTAs of a
-// cluster through distributed shared memory in rank order, so there is one launch, no workspace, and the result does
-// not depend on timing.  8 sequences, 32 heads of 128, 1543 keys: 35.9 us, 5.6 TB/s (39.7 us with the tiled kernel and its
+// just freed: loads are in flight throughout.  GT query heads that share a K / V head are done from the same loads.  Every
+// group keeps its own running maximum / sum / output in fp32 registers; groups meet through shuffles and shared memory,
+// CTAs of a cluster through distributed shared memory in rank order, so there is one launch, no workspace, and the result
+// does not depend on timing.  8 sequences, 32 heads of 128, 1543 keys: 35.9 us, 5.6 TB/s (39.7 us with the tiled kernel and its
 // fill; 52.6 us with loads only at the head of the loop).
 #include "attention_decode.h"
 

@@ -699,15 +699,16 @@ struct CommArgs {
 };
 
 // Whether a product goes to the few-rows kernel: its layouts and epilogues, and up to 64 rows always (a generation step;
-// 4 rows of the 7B gated MLP: 164 -> 54 us for its two GEMMs), up to 256 where the tiles here would leave half the SMs
-// without one.
-static bool skinny_better(int M, int N, int transA, int transB, int flags) {
+// 4 rows of the 7B gated MLP: 164 -> 54 us for its two GEMMs), up to 128 where the tiles here would leave half the SMs
+// without one and the reduction is long enough to be split (128 rows, there / here: 4096 x 4096 36.9 / 21.5 us, 4096 x
+// 16384 110.7 / 42.0 us; 2304 x 768 16.4 / 17.3 us, at 96 rows 16.4 / 15.3 us).
+static bool skinny_better(int M, int N, int K, int transA, int transB, int flags) {
   using namespace nx;
   constexpr int known = EPI_BIAS | EPI_GELU_ERF | EPI_GELU_TANH | EPI_AUX_OUT | EPI_AUX_DERIV | EPI_RESIDUAL | EPI_SCALE;
   if (transA || transB || (flags & ~known) != 0 || M > SKINNY_MAX_M) return false;
   const int BN = N <= 128 ? 128 : 256;
   const long long tiles = static_cast<long long>((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  return M <= 64 || 2 * tiles <= sm_count();
+  return M <= 64 || (2 * tiles <= sm_count() && (M <= 96 || K >= 1024));
 }
 
 static int gemm_common(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
@@ -822,7 +823,7 @@ NX_API int NX_SYM(nx_gemm_bf16)(const void* A, const void* B, void* C, int M, in
                         const void* aux_in, void* aux_out, const void* residual, long long ld_aux,
                         int flags, float alpha, void* stream_) {
   CommArgs ca;
-  ca.skinny = skinny_better(M, N, transA, transB, flags);
+  ca.skinny = skinny_better(M, N, K, transA, transB, flags);
   return gemm_common(A, B, C, M, N, K, lda, ldb, ldc, transA, transB, bias, aux_in, aux_out, residual, ld_aux,
                      flags, alpha, ca, static_cast<cudaStream_t>(stream_));
 }
