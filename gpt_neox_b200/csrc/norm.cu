@@ -300,7 +300,9 @@ norm_bwd_kernel(const h16* __restrict__ dy1, const h16* __restrict__ dy2,
 // the ring (up to ~200 KB), not by how many 16-byte loads the resident threads can hold in registers, and
 // the loads of the next rows run during the row reductions and the stores of the current one.  One thread
 // refills a stage as soon as every thread has taken its part of the row into registers (the barrier inside
-// the first block reduction).  Rows up to 8192 elements; wider rows use the kernels above.
+// the first block reduction).  Rows up to 8192 elements; wider rows use the kernels above.  One barrier per row, with the
+// warps' sums read back by every thread, was slower than the three here: its registers spill (two norms with the residual
+// gradient: 0.169 against 0.156 ms for 16384 x 4096, 0.166 against 0.146 ms for 8192 x 6144).
 // ---------------------------------------------------------------------------------------------
 constexpr int RING_MAX_STAGES = 8;
 
@@ -425,12 +427,10 @@ norm_bwd_ring_kernel(const h16* __restrict__ dy1, const h16* __restrict__ dy2, c
                      const h16* __restrict__ dx_in, h16* __restrict__ dx, float* __restrict__ ws, long long rows,
                      int H, int nst, int* err) {
   extern __shared__ __align__(128) unsigned char ring[];
-  // per-warp partial row sums, alternating between rows: one barrier per row, not three (two norms of 8192 x 2048 with the
-  // residual gradient: 68.7 -> 62.5 us)
-  __shared__ float2 sums[2][32];
+  __shared__ float sh[64];
   __shared__ __align__(8) unsigned long long bars[RING_MAX_STAGES];
   constexpr int NOUT = DUAL ? 4 : 2;
-  const int nv = H >> 3, nwarps = blockDim.x >> 5;
+  const int nv = H >> 3;
   const int idx = threadIdx.x;
   const bool live = idx < nv;
   const uint32_t row_bytes = static_cast<uint32_t>(H) * 2u;
@@ -465,7 +465,6 @@ norm_bwd_ring_kernel(const h16* __restrict__ dy1, const h16* __restrict__ dy2, c
     rstd_n = rstd_in[blockIdx.x];
   }
   int it = 0;
-  bool ok = true;      // a wait that ran out: no further waits or refills, the row loop still runs its barriers
   for (long long row = blockIdx.x; row < rows; row += gridDim.x, ++it) {
     const int st = it % nst;
     const float mean = mean_n, rstd = rstd_n;
@@ -473,9 +472,10 @@ norm_bwd_ring_kernel(const h16* __restrict__ dy1, const h16* __restrict__ dy2, c
       mean_n = RMS ? 0.f : mean_in[row + gridDim.x];
       rstd_n = rstd_in[row + gridDim.x];
     }
-    if (ok && !mbar_wait(bar0 + 8 * st, (it / nst) & 1, err, 61)) {
-      ok = false;
+    const bool ok = mbar_wait(bar0 + 8 * st, (it / nst) & 1, err, 61);
+    if (!__syncthreads_and(ok ? 1 : 0)) {
       ring_drain(bar0, nst, it, row, rows);
+      break;
     }
     const unsigned char* stage = ring + static_cast<size_t>(st) * stage_bytes;
     float xh[8], w[8];
@@ -510,13 +510,8 @@ norm_bwd_ring_kernel(const h16* __restrict__ dy1, const h16* __restrict__ dy2, c
         s2 += w[j];
       }
     }
-    s1 = warp_sum(s1);
-    s2 = warp_sum(s2);
-    if ((threadIdx.x & 31) == 0) sums[it & 1][threadIdx.x >> 5] = make_float2(s1, s2);
-    __syncthreads();                           // every thread has read its part of the stage, too
-    float2 r = make_float2(0.f, 0.f);
-    for (int w = 0; w < nwarps; ++w) r = fadd2(r, sums[it & 1][w]);
-    if (threadIdx.x == 0 && ok) {
+    const float2 r = block_sum2(s1, s2, sh);   // every thread has read its part of the stage once this returns
+    if (threadIdx.x == 0) {
       const long long nr = row + static_cast<long long>(nst) * gridDim.x;
       if (nr < rows) fill(st, nr);
     }
