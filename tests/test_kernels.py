@@ -635,3 +635,24 @@ def test_one_query_attention(b, h, hk, sk, d, window, alibi):
     assert o.dtype == DT and rel(o, ref) < (2 ** -7 if DT == torch.bfloat16 else 2 ** -10)
     torch.testing.assert_close(lse[:, :, 0], (rl[:, :, 0] / math.log(2.0)).float(), rtol=1e-4, atol=1e-4)
     assert torch.isinf(lse[:, :, 1:]).all() and (lse[:, :, 1:] > 0).all()
+
+
+@pytest.mark.parametrize("sk,h,hk", [(5, 4, 4), (300, 4, 4), (3000, 4, 4), (300, 16, 2), (3000, 32, 4)])
+def test_one_query_attention_passes_nan_and_inf_on(sk, h, hk):
+    """Non-finite scores and values in the split-key kernel, in the first, a middle and the last split: the outputs that are
+    NaN or infinite are those of the same query in a call of two rows (the tile kernel), in the other heads nothing is."""
+    from gpt_neox_b200.ops.attention import _fwd
+    torch.manual_seed(22)
+    base = [bf(1, n, m, 128) for n, m in ((1, h), (sk, hk), (sk, hk))]
+    run = lambda q, k, v: _fwd(q, k, v, 128 ** -0.5, False, -1, None)[0][0, -1]
+    for which, value in ((0, math.nan), (0, math.inf), (1, math.nan), (1, math.inf), (1, -math.inf), (2, math.nan),
+                         (2, -math.inf)):
+        for at in (0, sk // 2, sk - 1):
+            q, k, v = ts = [t.clone() for t in base]
+            ts[which][0, min(at, ts[which].shape[1] - 1), 1, 7] = value
+            one, two = run(q, k, v), run(torch.cat([q, q], 1), k, v)
+            assert torch.equal(one.isnan(), two.isnan()) and torch.equal(one.isinf(), two.isinf()), (which, value, at)
+            hit = slice(1, 2) if which == 0 else slice(h // hk, 2 * (h // hk))
+            assert not math.isnan(value) or one[hit].isnan().any(-1).all()
+            one[hit] = 0
+            assert one.isfinite().all()
