@@ -90,16 +90,20 @@ class ParallelMLP(nn.Module):
             return False        # fp8 GEMMs run through the per-module path
         return (not self.is_gated) and self.activation_type == "gelu" and x.is_cuda and x.dtype in (torch.bfloat16, torch.float16)
 
-    def forward(self, hidden_states, residual=None, out_bias=None):
+    def forward(self, hidden_states, residual=None, out_bias=None, infer=False):
         """-> (output without linear2's bias, that bias). ``residual`` (optional, fused path only)
         is added inside the second GEMM's epilogue; so is ``out_bias`` (a bias vector that already
-        includes linear2's: the returned bias is then None)."""
+        includes linear2's: the returned bias is then None).  ``infer`` (with a residual, one tensor-parallel
+        rank): a generation step without autograd."""
         if self._fusable(hidden_states):
             if self.sequence_parallel:
                 x = gather_from_sequence_parallel_region(hidden_states, seq_dim=0)
             else:
                 x = copy_to_model_parallel_region(hidden_states)
             kind = "tanh" if self.bias_gelu_fusion else "erf"
+            if infer:
+                return fused_ops.mlp_gelu_infer(x, self.linear1.weight, self.linear1.bias, self.linear2.weight, out_bias,
+                                                residual, kind), None
             out = fused_ops.mlp_gelu(x, self.linear1.weight, self.linear1.bias, self.linear2.weight, out_bias,
                                      residual=residual, kind=kind, recompute_act=self.recompute_act)
             if not self.parallel_output:
@@ -369,9 +373,10 @@ class ParallelSelfAttention(nn.Module):
         # output projection; bias (and the optional residual) are applied by the caller / epilogue
         if residual is not None and ctx.is_cuda and not self.dense.sequence_parallel and \
                 mpu.get_model_parallel_world_size() == 1:
-            if kernel_lib.untracked():
-                # the bias too goes into the GEMM's epilogue (a training step sums it with the MLP's instead, so that
-                # one column sum serves both gradients)
+            if self.use_cache and kernel_lib.untracked():
+                # generation: the bias too goes into the GEMM's epilogue (a training step sums it with the MLP's instead,
+                # so that one column sum serves both gradients; a checkpointed region runs without gradients first and
+                # has to round as its recompute does)
                 out = _linear_bias_residual(ctx, self.dense.weight, self.dense.bias, residual)
                 bias = None
             else:
@@ -561,7 +566,7 @@ class ParallelTransformerLayer(nn.Module):
                 t, b_attn, *cache = self.attention(x1, attention_mask, layer_past=layer_past, residual=residual)
                 if cache:
                     self.layer_past = cache[0]
-                out, _ = self.mlp(x2, residual=t, out_bias=_sum_bias(b_attn, self.mlp.linear2.bias))
+                out, _ = self.mlp(x2, residual=t, out_bias=_sum_bias(b_attn, self.mlp.linear2.bias), infer=self.use_cache)
                 return out
             att = self.attention(x1, attention_mask, layer_past=layer_past)
             if self.use_cache:

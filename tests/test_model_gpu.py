@@ -109,3 +109,35 @@ def test_other_model_families_match_fp32_oracle_loss(family, variant, precision)
     # the router of a top-k MoE is discontinuous (a 16-bit rounding can move a token to another expert), so its
     # stack gets a wider band than the smooth mixers
     assert worst < (0.25 if family == "dmoe" else 0.12), f"worst relative gradient error {worst} at {where}"
+
+
+@pytest.mark.parametrize("over", [dict(), dict(bias_gelu_fusion=True), dict(gpt_j_residual=False),
+                                  dict(norm="rmsnorm", activation="swiglu", mlp_multiple_of=64)])
+@pytest.mark.parametrize("precision", ["bfloat16", "fp16"])
+def test_a_layer_rounds_the_same_with_and_without_gradients(over, precision):
+    """Activation checkpointing runs a region without gradients first and again with them in the backward: the loss and
+    the gradients belong to one function only if both give the same bits (every bias non-zero here)."""
+    from gpt_neox_b200.models.transformer import ParallelTransformerLayer
+    from gpt_neox_b200.parallel.random import checkpoint
+    base = dict(num_layers=2, hidden_size=256, num_attention_heads=4, seq_length=256, max_position_embeddings=256,
+                synthetic_vocab_size=1000, attention_config=[[["flash"], 2]], distributed_backend="nccl",
+                precision=precision)
+    _, model = _build(tiny_config(**{**base, **over}))
+    layer = next(m for m in model.modules() if isinstance(m, ParallelTransformerLayer))
+    for p in layer.parameters():
+        if p.dim() == 1:
+            torch.nn.init.normal_(p, std=0.3)
+    run = lambda t: ParallelTransformerLayer.forward(layer, t)
+    for rows in (3, 250):                       # the few-rows GEMMs and the tiled ones
+        x = torch.randn(rows, 2, 256, device="cuda", dtype=next(layer.parameters()).dtype, requires_grad=True)
+        y = run(x)
+        with torch.no_grad():
+            assert torch.equal(run(x), y)
+        z = checkpoint(run, x)
+        assert torch.equal(z, y)
+        g = torch.randn_like(y)
+        grads = torch.autograd.grad(y, [x] + list(layer.parameters()), g)
+        z.backward(g)
+        for a, b in zip(grads, [x] + list(layer.parameters())):
+            assert (a.float() - b.grad.float()).abs().max() <= 1e-2 * a.float().abs().max()
+            b.grad = None
