@@ -3,7 +3,9 @@
 //
 // A step of a few tokens keeps the GPU busy for 30 - 40 us per layer; issued op by op the eight launches cost several
 // times that on the host.  The kernels, their order and their arguments are those of the op-by-op path
-// (models/transformer.py, ParallelTransformerLayer.forward with `use_cache`), so both give the same bits.
+// (models/transformer.py, ParallelTransformerLayer.forward with `use_cache`), so both give the same bits.  The attention
+// branch is rounded at its own size; it, the MLP and the residual stream meet in fp32 in the last GEMM's epilogue, so the
+// stream is rounded once per layer.
 #include "common.h"
 
 NX_API int NX_SYM(nx_norm_fwd)(int kind, const void* x, const void* g1, const void* b1, void* y1, const void* g2,
@@ -31,7 +33,7 @@ extern "C" {
 struct nx_layer_infer_args {
   const void *x, *ln1_w, *ln1_b, *ln2_w, *ln2_b, *w_qkv, *b_qkv, *w_dense, *b_dense, *w1, *b1, *w2, *b2;
   const void *cos, *sin;
-  // scratch: work, 16-bit: x1, x2, the attention branch with the residual (rows x h each), qkv, context, the MLP's hidden
+  // scratch: work, 16-bit: x1, x2, the attention branch (rows x h each), qkv, context, the MLP's hidden
   // layer; stats, fp32: mean and rstd of every row, the log-sum-exp of the attention [b, np, s rounded up to 128]
   void *cache, *work, *stats, *out;
   long long cache_kv_stride;            // elements between the key and the value part of the cache
@@ -42,7 +44,7 @@ struct nx_layer_infer_args {
 
 NX_API int NX_SYM(nx_layer_infer)(const nx_layer_infer_args* a, void* stream) {
   using namespace nx;
-  enum { BIAS = 1, GELU_ERF = 2, GELU_TANH = 4, RESIDUAL = 64 };
+  enum { BIAS = 1, GELU_ERF = 2, GELU_TANH = 4, RESIDUAL = 64, ADD_AUX = 4096 };
   const long long rows = static_cast<long long>(a->s) * a->b;
   if (rows == 0) return NX_OK;
   NX_REQUIRE(rows < (1ll << 31), "layer_infer: too many rows");
@@ -53,10 +55,11 @@ NX_API int NX_SYM(nx_layer_infer)(const nx_layer_infer_args* a, void* stream) {
   uint16_t *x1 = w, *x2 = x1 + rows * a->h, *t = x2 + rows * a->h, *qkv = t + rows * a->h, *ctx = qkv + rows * qkv_n,
            *mid = ctx + rows * ctx_n;
   float *mean = static_cast<float*>(a->stats), *rstd = mean + rows, *lse = rstd + rows;
-  auto gemm = [&](const void* A, const void* W, void* C, int N, int K, const void* bias, const void* residual, int act) {
-    const int flags = act | (bias != nullptr ? BIAS : 0) | (residual != nullptr ? RESIDUAL : 0);
+  auto gemm = [&](const void* A, const void* W, void* C, int N, int K, const void* bias, int act,
+                  const void* residual = nullptr, const void* residual2 = nullptr) {
+    const int flags = act | (bias != nullptr ? BIAS : 0) | (residual != nullptr ? RESIDUAL | ADD_AUX : 0);
     auto fn = a->pair_gemm && M >= 256 && N >= 256 ? NX_SYM(nx_gemm2_bf16) : NX_SYM(nx_gemm_bf16);
-    return fn(A, W, C, M, N, K, K, K, N, 0, 0, bias, nullptr, nullptr, residual, residual != nullptr ? N : 0, flags, 1.f,
+    return fn(A, W, C, M, N, K, K, K, N, 0, 0, bias, residual2, nullptr, residual, residual != nullptr ? N : 0, flags, 1.f,
               stream);
   };
 #define NX_TRY(expr)                  \
@@ -66,7 +69,7 @@ NX_API int NX_SYM(nx_layer_infer)(const nx_layer_infer_args* a, void* stream) {
   } while (0)
   NX_TRY(NX_SYM(nx_norm_fwd)(0, a->x, a->ln1_w, a->ln1_b, x1, a->ln2_w, a->ln2_b, x2, mean, rstd, rows, a->h, a->eps,
                              stream));
-  NX_TRY(gemm(x1, a->w_qkv, qkv, qkv_n, a->h, a->b_qkv, nullptr, 0));
+  NX_TRY(gemm(x1, a->w_qkv, qkv, qkv_n, a->h, a->b_qkv, 0));
   // q, k and v inside the projection's rows
   const bool mha = a->np == a->kvp;
   const long long ss = static_cast<long long>(a->b) * qkv_n, sb = qkv_n, sh = mha ? 3 * hn : hn;
@@ -80,9 +83,9 @@ NX_API int NX_SYM(nx_layer_infer)(const nx_layer_infer_args* a, void* stream) {
   NX_TRY(NX_SYM(nx_flash_attn_fwd)(q, kc, vc, ctx, lse, nullptr, a->b, a->np, a->kvp, a->s, a->past + a->s, hn, sb, sh, ss,
                                    cb, hn, cs, cb, hn, cs, ctx_n, hn, static_cast<long long>(a->b) * ctx_n, a->scale, 1,
                                    a->window, 0.f, 0, nullptr, nullptr, 0, stream));
-  NX_TRY(gemm(ctx, a->w_dense, t, a->h, ctx_n, a->b_dense, a->x, 0));
-  NX_TRY(gemm(x2, a->w1, mid, a->ffn, a->h, a->b1, nullptr, a->gelu_tanh ? GELU_TANH : GELU_ERF));
-  NX_TRY(gemm(mid, a->w2, a->out, a->h, a->ffn, a->b2, t, 0));
+  NX_TRY(gemm(ctx, a->w_dense, t, a->h, ctx_n, a->b_dense, 0));
+  NX_TRY(gemm(x2, a->w1, mid, a->ffn, a->h, a->b1, a->gelu_tanh ? GELU_TANH : GELU_ERF));
+  NX_TRY(gemm(mid, a->w2, a->out, a->h, a->ffn, a->b2, 0, t, a->x));
 #undef NX_TRY
   return NX_OK;
 }

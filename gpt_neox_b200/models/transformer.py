@@ -90,20 +90,20 @@ class ParallelMLP(nn.Module):
             return False        # fp8 GEMMs run through the per-module path
         return (not self.is_gated) and self.activation_type == "gelu" and x.is_cuda and x.dtype in (torch.bfloat16, torch.float16)
 
-    def forward(self, hidden_states, residual=None, out_bias=None, infer=False):
+    def forward(self, hidden_states, residual=None, out_bias=None, residual2=None):
         """-> (output without linear2's bias, that bias). ``residual`` (optional, fused path only)
         is added inside the second GEMM's epilogue; so is ``out_bias`` (a bias vector that already
-        includes linear2's: the returned bias is then None).  ``infer`` (with a residual, one tensor-parallel
-        rank): a generation step without autograd."""
+        includes linear2's: the returned bias is then None).  ``residual2``: a second residual, for a generation
+        step without autograd on one tensor-parallel rank."""
         if self._fusable(hidden_states):
             if self.sequence_parallel:
                 x = gather_from_sequence_parallel_region(hidden_states, seq_dim=0)
             else:
                 x = copy_to_model_parallel_region(hidden_states)
             kind = "tanh" if self.bias_gelu_fusion else "erf"
-            if infer:
+            if residual2 is not None:
                 return fused_ops.mlp_gelu_infer(x, self.linear1.weight, self.linear1.bias, self.linear2.weight, out_bias,
-                                                residual, kind), None
+                                                residual, residual2, kind), None
             out = fused_ops.mlp_gelu(x, self.linear1.weight, self.linear1.bias, self.linear2.weight, out_bias,
                                      residual=residual, kind=kind, recompute_act=self.recompute_act)
             if not self.parallel_output:
@@ -314,9 +314,10 @@ class ParallelSelfAttention(nn.Module):
         return q, present
 
     # -------------------------------------------------------------------- forward
-    def forward(self, hidden_states, attention_mask=None, layer_past=None, residual=None):
+    def forward(self, hidden_states, attention_mask=None, layer_past=None, residual=None, add_bias=False):
         """hidden_states [sq, b, h] -> (output [sq, b, h] without dense bias, dense bias)
-        (+ the updated KV cache when ``use_cache``)."""
+        (+ the updated KV cache when ``use_cache``).  ``add_bias``: the bias is added by the projection's GEMM (a
+        generation step without autograd on one tensor-parallel rank); None is returned for it."""
         mixed, _ = self.query_key_value(hidden_states)
         np_, kvp, hn = self.num_attention_heads_per_partition, self.num_kv_heads_per_partition, \
             self.hidden_size_per_attention_head
@@ -371,17 +372,12 @@ class ParallelSelfAttention(nn.Module):
                     mask = self.sparse_mask[..., sk_ - q.shape[0]:sk_, :sk_]
                 ctx = self._global_attention(q, k, v, mask)
         # output projection; bias (and the optional residual) are applied by the caller / epilogue
-        if residual is not None and ctx.is_cuda and not self.dense.sequence_parallel and \
+        if add_bias:
+            out, bias = linear_op(ctx, self.dense.weight, self.dense.bias), None
+        elif residual is not None and ctx.is_cuda and not self.dense.sequence_parallel and \
                 mpu.get_model_parallel_world_size() == 1:
-            if self.use_cache and kernel_lib.untracked():
-                # generation: the bias too goes into the GEMM's epilogue (a training step sums it with the MLP's instead,
-                # so that one column sum serves both gradients; a checkpointed region runs without gradients first and
-                # has to round as its recompute does)
-                out = _linear_bias_residual(ctx, self.dense.weight, self.dense.bias, residual)
-                bias = None
-            else:
-                out = _linear_residual(ctx, self.dense.weight, residual)
-                bias = self.dense.bias
+            out = _linear_residual(ctx, self.dense.weight, residual)
+            bias = self.dense.bias
         else:
             out, bias = self.dense(ctx)
             if residual is not None:
@@ -414,12 +410,6 @@ class _LinearResidualFn(torch.autograd.Function):
         gx = gemm_op(gy2, w, trans_b=True).view(ctx.x_shape)
         gw = wgrad(gy2, x2, w)
         return gx, gw, gy2.view(gy.shape)
-
-
-def _linear_bias_residual(x, w, bias, residual):
-    """x @ w^T (+ bias) + residual without autograd."""
-    x2, r2 = x.reshape(-1, x.shape[-1]).contiguous(), residual.reshape(-1, residual.shape[-1]).contiguous()
-    return gemm_op(x2, w, bias=bias, residual=r2).view(*x.shape[:-1], w.shape[0])
 
 
 def _linear_residual(x, w, residual):
@@ -541,7 +531,7 @@ class ParallelTransformerLayer(nn.Module):
                 x1, x2 = self.input_layernorm(x), self.post_attention_layernorm(x)
             fusable = (p == 0.0 and x.is_cuda and self.num_experts <= 1
                        and isinstance(self.mlp, ParallelMLP) and self.mlp._fusable(x2))
-            fast = fusable and ws == 1 and (not self.use_cache or kernel_lib.untracked())
+            fast = fusable and ws == 1
             if fusable and self.sequence_parallel and not self.use_cache:
                 from ..ops import fused_tp
                 be = fused_tp.backend(x, mpu.get_model_parallel_group())
@@ -560,13 +550,15 @@ class ParallelTransformerLayer(nn.Module):
                     kind = "tanh" if self.mlp.bias_gelu_fusion else "erf"
                     return fused_tp.mlp_gelu_sp(x2, self.mlp.linear1.weight, self.mlp.linear1.bias,
                                                 self.mlp.linear2.weight, attn_partial, bias_total, residual, kind, be)
-            if fast:
+            if fast and self.use_cache and kernel_lib.untracked():
+                # generation: the branches at their own size, then x + attn + mlp in one epilogue and one rounding
+                t, _, self.layer_past = self.attention(x1, attention_mask, layer_past=layer_past, add_bias=True)
+                return self.mlp(x2, residual=t, out_bias=self.mlp.linear2.bias, residual2=residual)[0]
+            if fast and not self.use_cache:
                 # x + attn + b_attn + mlp + b_mlp with both adds of matrices inside GEMM epilogues:
                 #   t = dense(ctx) + x ;  out = linear2(h) + t ; the two bias vectors are added once.
-                t, b_attn, *cache = self.attention(x1, attention_mask, layer_past=layer_past, residual=residual)
-                if cache:
-                    self.layer_past = cache[0]
-                out, _ = self.mlp(x2, residual=t, out_bias=_sum_bias(b_attn, self.mlp.linear2.bias), infer=self.use_cache)
+                t, b_attn = self.attention(x1, attention_mask, layer_past=layer_past, residual=residual)
+                out, _ = self.mlp(x2, residual=t, out_bias=_sum_bias(b_attn, self.mlp.linear2.bias))
                 return out
             att = self.attention(x1, attention_mask, layer_past=layer_past)
             if self.use_cache:

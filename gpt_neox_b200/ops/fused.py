@@ -79,11 +79,13 @@ def mlp_gelu(x, w1, b1, w2, b2=None, residual=None, kind: str = "erf", recompute
     return y if residual is None else y + residual
 
 
-def mlp_gelu_infer(x, w1, b1, w2, b2, residual, kind):
-    """``mlp_gelu`` of a generation step: no autograd node and no stored derivative.  Its GeLU is rounded differently from
-    the one that is evaluated together with the derivative, so nothing that a recompute repeats may call it."""
+def mlp_gelu_infer(x, w1, b1, w2, b2, residual, residual2, kind):
+    """``mlp_gelu`` of a generation step with two residuals: no autograd node and no stored derivative.  Its GeLU is rounded
+    differently from the one that is evaluated together with the derivative, so nothing that a recompute repeats may call
+    it."""
     x2 = x.reshape(-1, x.shape[-1]).contiguous()
-    y = gemm(gemm(x2, w1, bias=b1, gelu=kind), w2, bias=b2, residual=residual.reshape(x2.shape[0], -1).contiguous())
+    r, r2 = (t.reshape(x2.shape[0], -1).contiguous() for t in (residual, residual2))
+    y = gemm(gemm(x2, w1, bias=b1, gelu=kind), w2, bias=b2, residual=r, residual2=r2)
     return y.view(*x.shape[:-1], w2.shape[0])
 
 

@@ -370,3 +370,29 @@ def test_a_layer_in_one_call_gives_the_bits_of_the_op_by_op_path(over, precision
         h.remove()
     assert len(calls) == 14 and len(one) == len(ops)
     assert all(torch.equal(a, b) for a, b in zip(one, ops))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,x,branch,want", [("bfloat16", 1024.0, 3.0, 1032.0), ("fp16", 16384.0, 6.0, 16400.0)])
+@pytest.mark.parametrize("hook", [False, True])
+@pytest.mark.parametrize("rows", [1, 130, 300])
+def test_a_generation_step_rounds_the_residual_stream_once(precision, x, branch, want, hook, rows):
+    """Attention and MLP add less than half a unit in the last place of the residual stream each, and more than half
+    together (all matrices zero, so that the branches are their last biases): with the sum rounded once the stream moves,
+    with a rounding after each branch it does not.  One native call and op by op; the three GEMM kernels."""
+    import torch
+    from gpt_neox_b200.models.transformer import ParallelTransformerLayer
+    from test_model_gpu import _build
+    _, model = _build(tiny_config(num_layers=2, hidden_size=256, num_attention_heads=4, seq_length=512,
+                                  max_position_embeddings=512, synthetic_vocab_size=1000, pipe_parallel_size=0,
+                                  attention_config=[[["flash"], 2]], distributed_backend="nccl", precision=precision))
+    model.inference_mode(use_cache=True)
+    layer = next(m for m in model.modules() if isinstance(m, ParallelTransformerLayer))
+    for n, p in layer.named_parameters():
+        torch.nn.init.constant_(p, branch if n in ("attention.dense.bias", "mlp.linear2.bias") else 0.0)
+    if hook:
+        layer.mlp.register_forward_hook(lambda *a: None)
+    t = torch.full((rows, 1, 256), x, device="cuda", dtype=next(layer.parameters()).dtype)
+    with torch.no_grad():
+        out = ParallelTransformerLayer.forward(layer, t)
+    assert (out == want).all()
