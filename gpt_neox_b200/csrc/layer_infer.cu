@@ -16,9 +16,9 @@ NX_API int NX_SYM(nx_gemm_bf16)(const void* A, const void* B, void* C, int M, in
 NX_API int NX_SYM(nx_gemm2_bf16)(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                          long long ldc, int transA, int transB, const void* bias, const void* aux_in, void* aux_out,
                          const void* residual, long long ld_aux, int flags, float alpha, void* stream_);
-NX_API int NX_SYM(nx_rope_qk)(void* q, const void* k, const void* v, void* kd, void* vd, const void* cos, const void* sin,
-                      int S, int B, int NQ, int NK, int D, int R, const long long* strides, int pos0, int inverse,
-                      void* stream_);
+NX_API int NX_SYM(nx_rope_qk)(const void* q, const void* k, const void* v, void* qd, void* kd, void* vd, const void* cos,
+                      const void* sin, int S, int B, int NQ, int NK, int D, int R, const long long* strides, int pos0,
+                      int inverse, void* stream_);
 NX_API int NX_SYM(nx_flash_attn_fwd)(const void* q, const void* k, const void* v, void* o, void* lse, const void* alibi,
                              int B, int H, int Hk, int Sq, int Sk, int D, long long q_sb, long long q_sh,
                              long long q_ss, long long k_sb, long long k_sh, long long k_ss, long long v_sb,
@@ -76,8 +76,8 @@ NX_API int NX_SYM(nx_layer_infer)(const nx_layer_infer_args* a, void* stream) {
   uint16_t *q = qkv, *k = qkv + (mha ? hn : ctx_n), *v = qkv + (mha ? 2 * hn : ctx_n + a->kvp * hn);
   const long long cs = static_cast<long long>(a->b) * a->kvp * hn, cb = static_cast<long long>(a->kvp) * hn;
   uint16_t *kc = static_cast<uint16_t*>(a->cache), *vc = kc + a->cache_kv_stride;
-  const long long strides[15] = {ss, sb, sh, ss, sb, sh, ss, sb, sh, cs, cb, hn, cs, cb, hn};
-  NX_TRY(NX_SYM(nx_rope_qk)(q, k, v, kc + a->past * cs, vc + a->past * cs, a->cos, a->sin, a->s, a->b, a->np, a->kvp, hn,
+  const long long strides[18] = {ss, sb, sh, ss, sb, sh, ss, sb, sh, ss, sb, sh, cs, cb, hn, cs, cb, hn};
+  NX_TRY(NX_SYM(nx_rope_qk)(q, k, v, q, kc + a->past * cs, vc + a->past * cs, a->cos, a->sin, a->s, a->b, a->np, a->kvp, hn,
                             a->rot, strides, a->past, 0, stream));
   // the context as [b, s, heads, hn] memory is what the op-by-op path writes; here it goes straight to [s, b, heads, hn]
   NX_TRY(NX_SYM(nx_flash_attn_fwd)(q, kc, vc, ctx, lse, nullptr, a->b, a->np, a->kvp, a->s, a->past + a->s, hn, sb, sh, ss,

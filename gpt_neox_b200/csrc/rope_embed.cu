@@ -96,15 +96,16 @@ __global__ void rope_vec8_kernel(const RopeArgs a) {
 
 // q and k of one projection output together, in place or with k (and v) going to a cache: one launch where the
 // per-tensor form takes two, and, when generating, where two rotary copies, two concatenations and a stack would move
-// the whole cache (4 x 2048 tokens, 64 q and k heads, 32 rotary dims: 25 us in two launches, 21 us in one).  Work items of a token, 8 elements (of each half) per thread: the rotated pairs of the q heads, those
-// of the k heads, and with a cache the unrotated rest of the k heads and the v heads.
+// the whole cache (4 x 2048 tokens, 64 q and k heads, 32 rotary dims: 25 us in two launches, 21 us in one).  Work items of
+// a token, 8 elements (of each half) per thread: the rotated pairs of the q heads, those of the k heads, out of place the
+// unrotated rest of the q heads, and with a cache the unrotated rest of the k heads and the v heads.
 struct RopeQKArgs {
-  h16 *q, *kd, *vd;       // q is rotated in place; kd may be k itself; vd null: v is not touched
-  const h16 *k, *v;
+  h16 *qd, *kd, *vd;      // qd / kd may be q / k themselves; vd null: v is not touched
+  const h16 *q, *k, *v;
   const float *cos, *sin;
-  unsigned tokens, B, NQ, NK, G, KT, VT;   // G: 8-wide groups per half; KT / VT: 8-wide groups of a k rest / a v head
+  unsigned tokens, B, NQ, NK, G, QT, KT, VT;   // 8-wide groups: G of a half, QT / KT of the rest of a q / k head, VT of a v head
   int R;
-  long long qs, qb, qh, ks, kb, kh, vs, vb, vh, kds, kdb, kdh, vds, vdb, vdh;
+  long long qs, qb, qh, ks, kb, kh, vs, vb, vh, qds, qdb, qdh, kds, kdb, kdh, vds, vdb, vdh;
   int pos0;
   float sin_sign;
 };
@@ -130,7 +131,8 @@ __device__ __forceinline__ void rotate8(const h16* in, h16* out, const float* co
 
 __global__ void __launch_bounds__(256) rope_qk_kernel(const RopeQKArgs a) {
   const int half = a.R >> 1;
-  const unsigned n_q = a.NQ * a.G, n_k = a.NK * a.G, n_t = a.NK * a.KT, per = n_q + n_k + n_t + a.NK * a.VT;
+  const unsigned n_q = a.NQ * a.G, n_k = a.NK * a.G, n_u = a.NQ * a.QT, n_t = a.NK * a.KT,
+                 per = n_q + n_k + n_u + n_t + a.NK * a.VT;
   const unsigned i = blockIdx.x * 256u + threadIdx.x, tok = i / per;
   if (tok >= a.tokens) return;
   unsigned r = i - tok * per;
@@ -138,8 +140,8 @@ __global__ void __launch_bounds__(256) rope_qk_kernel(const RopeQKArgs a) {
   const long long trow = static_cast<long long>(a.pos0 + static_cast<int>(s)) * half;
   if (r < n_q) {
     const unsigned h = r / a.G, j = (r - h * a.G) * 8;
-    h16* p = a.q + s * a.qs + b * a.qb + h * a.qh + j;
-    rotate8(p, p, a.cos + trow + j, a.sin + trow + j, half, a.sin_sign);
+    rotate8(a.q + s * a.qs + b * a.qb + h * a.qh + j, a.qd + s * a.qds + b * a.qdb + h * a.qdh + j, a.cos + trow + j,
+            a.sin + trow + j, half, a.sin_sign);
     return;
   }
   r -= n_q;
@@ -150,6 +152,13 @@ __global__ void __launch_bounds__(256) rope_qk_kernel(const RopeQKArgs a) {
     return;
   }
   r -= n_k;
+  if (r < n_u) {
+    const unsigned h = r / a.QT, j = a.R + (r - h * a.QT) * 8;
+    *reinterpret_cast<uint4*>(a.qd + s * a.qds + b * a.qdb + h * a.qdh + j) =
+        *reinterpret_cast<const uint4*>(a.q + s * a.qs + b * a.qb + h * a.qh + j);
+    return;
+  }
+  r -= n_u;
   if (r < n_t) {
     const unsigned h = r / a.KT, j = a.R + (r - h * a.KT) * 8;
     *reinterpret_cast<uint4*>(a.kd + s * a.kds + b * a.kdb + h * a.kdh + j) =
@@ -228,30 +237,33 @@ NX_API int NX_SYM(nx_rope)(const void* in, void* out, const void* cos, const voi
   NX_LAUNCH_CHECK();
   return NX_OK;
 }
-// Rotates q [S, B, NQ, D] in place and k [S, B, NK, D] into kd (which may be k); vd non-null: copies v and the unrotated
-// dims of k too (the cache write of a generation step).  strides: element strides (s, b, head) of q, k, v, kd, vd.
-// Everything 16-byte aligned, D and R / 2 multiples of 8.
-NX_API int NX_SYM(nx_rope_qk)(void* q, const void* k, const void* v, void* kd, void* vd, const void* cos, const void* sin,
-                      int S, int B, int NQ, int NK, int D, int R, const long long* strides, int pos0, int inverse,
-                      void* stream_) {
+// Rotates q [S, B, NQ, D] into qd and k [S, B, NK, D] into kd; qd may be q, kd may be k.  qd other than q: the unrotated
+// dims of q are copied too; vd non-null: v and the unrotated dims of k are (the cache write of a generation step).
+// strides: element strides (s, b, head) of q, k, v, qd, kd, vd.  Everything 16-byte aligned, D and R / 2 multiples of 8.
+NX_API int NX_SYM(nx_rope_qk)(const void* q, const void* k, const void* v, void* qd, void* kd, void* vd, const void* cos,
+                      const void* sin, int S, int B, int NQ, int NK, int D, int R, const long long* strides, int pos0,
+                      int inverse, void* stream_) {
   using namespace nx;
   NX_REQUIRE(R % 16 == 0 && R <= D && D % 8 == 0, "rope_qk: rotary dims %d of head dim %d", R, D);
   if (S == 0 || B == 0) return NX_OK;
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-  bool ok = al(q) && al(k) && al(v) && al(kd) && al(vd) && al(cos) && al(sin);
-  for (int i = 0; i < (vd != nullptr ? 15 : 12); ++i) ok = ok && strides[i] % 8 == 0;
+  bool ok = al(q) && al(k) && al(v) && al(qd) && al(kd) && al(vd) && al(cos) && al(sin);
+  for (int i = 0; i < (vd != nullptr ? 18 : 15); ++i) ok = ok && strides[i] % 8 == 0;
   NX_REQUIRE(ok, "rope_qk: views must be 16-byte aligned");
   RopeQKArgs a;
-  a.q = (h16*)q; a.k = (const h16*)k; a.v = (const h16*)v; a.kd = (h16*)kd; a.vd = (h16*)vd;
+  a.q = (const h16*)q; a.k = (const h16*)k; a.v = (const h16*)v; a.qd = (h16*)qd; a.kd = (h16*)kd; a.vd = (h16*)vd;
   a.cos = (const float*)cos; a.sin = (const float*)sin;
   a.tokens = (unsigned)S * (unsigned)B; a.B = B; a.NQ = NQ; a.NK = NK; a.R = R; a.G = R / 16;
+  a.QT = qd != q ? (D - R) / 8 : 0;
   a.KT = vd != nullptr ? (D - R) / 8 : 0;
   a.VT = vd != nullptr ? D / 8 : 0;
   const long long* t = strides;
   a.qs = t[0]; a.qb = t[1]; a.qh = t[2]; a.ks = t[3]; a.kb = t[4]; a.kh = t[5]; a.vs = t[6]; a.vb = t[7]; a.vh = t[8];
-  a.kds = t[9]; a.kdb = t[10]; a.kdh = t[11]; a.vds = t[12]; a.vdb = t[13]; a.vdh = t[14];
+  a.qds = t[9]; a.qdb = t[10]; a.qdh = t[11]; a.kds = t[12]; a.kdb = t[13]; a.kdh = t[14];
+  a.vds = t[15]; a.vdb = t[16]; a.vdh = t[17];
   a.pos0 = pos0; a.sin_sign = inverse ? -1.f : 1.f;
-  const long long per = static_cast<long long>(NQ + NK) * a.G + static_cast<long long>(NK) * (a.KT + a.VT);
+  const long long per = static_cast<long long>(NQ + NK) * a.G + static_cast<long long>(NQ) * a.QT +
+                        static_cast<long long>(NK) * (a.KT + a.VT);
   const long long total = static_cast<long long>(S) * B * per;
   if (total == 0) return NX_OK;
   NX_REQUIRE(total < (1ll << 31), "rope_qk: too many elements");

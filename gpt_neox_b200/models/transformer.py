@@ -298,14 +298,17 @@ class ParallelSelfAttention(nn.Module):
         return ctx.view(b, np_, sq, hn).permute(2, 0, 1, 3).reshape(sq, b, np_ * hn)
 
     def _rotate_into_cache(self, q, k, v, past, cos, sin):
-        """Generation without autograd: q rotated, and the cache with this step's (rotated) k and v behind ``past``;
-        one kernel does the rotation and the cache write.  -> (q, present)"""
+        """Generation without autograd: q rotated (a tensor of its own: whoever kept the projection's output finds it as it
+        was), and the cache with this step's (rotated) k and v behind ``past``; one kernel does the rotation and the cache
+        write.  -> (q, present)"""
         n = past[0].shape[0] if past is not None else 0
         present = kv_cache.extend(self, past, k.shape[0], k)
         k_new, v_new = present[0, n:], present[1, n:]
-        if self.rotary_emb is not None and rope_ops._qk_ok(self.rotary_dim, q.shape[3], q, k, v, k_new, v_new):
-            rope_ops._launch_qk(q, k, cos, sin, self.rotary_dim, n, False, v=v, k_out=k_new, v_out=v_new)
-            return q, present
+        if self.rotary_emb is not None and rope_ops._qk_ok(self.rotary_dim, q.shape[3], q, k, v, k_new, v_new,
+                                                           tables=(cos, sin)):
+            q_out = torch.empty(q.shape, device=q.device, dtype=q.dtype)
+            rope_ops._launch_qk(q, k, cos, sin, self.rotary_dim, n, False, v=v, q_out=q_out, k_out=k_new, v_out=v_new)
+            return q_out, present
         if self.rotary_emb is not None:
             q = apply_rotary(q, cos, sin, self.rotary_dim, n)
             k = apply_rotary(k, cos, sin, self.rotary_dim, n)

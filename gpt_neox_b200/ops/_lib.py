@@ -123,7 +123,7 @@ def _declare(lib):
     sig("nx_moe_combine_bwd", [P, P, P, P, I, P, P, I, I, P])
     sig("nx_gemm_bf16_grouped", [I, P, P, P, I, I, I, L, L, L, I, I, P, P, L, P, P, L, I, P])
     sig("nx_rope", [P, P, P, P, I, I, I, I, I, L, L, L, L, L, L, I, I, P])
-    sig("nx_rope_qk", [P] * 7 + [I] * 6 + [C.POINTER(L), I, I, P])
+    sig("nx_rope_qk", [P] * 8 + [I] * 6 + [C.POINTER(L), I, I, P])
     sig("nx_layer_infer", [P, P])
     sig("nx_embedding_fwd", [P, P, P, L, I, L, L, P])
     sig("nx_embedding_bwd", [P, P, P, L, I, L, L, P])

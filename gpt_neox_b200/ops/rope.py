@@ -29,30 +29,31 @@ def _launch(x, out, cos, sin, rot, pos0, inverse):
                                   out.stride(2), int(pos0), int(inverse), _lib.stream()), "nx_rope")
 
 
-def _qk_ok(rot, hn, *views):
-    """Whether ``nx_rope_qk`` takes these [s, b, heads, hn] views (16-byte accesses on every row, 32-bit indices)."""
-    return (rot % 16 == 0 and hn % 8 == 0 and all(
+def _qk_ok(rot, hn, *views, tables=()):
+    """Whether ``nx_rope_qk`` takes these [s, b, heads, hn] views and tables (16-byte accesses on every row, 32-bit
+    indices)."""
+    return (rot % 16 == 0 and hn % 8 == 0 and all(t.data_ptr() % 16 == 0 for t in tables) and all(
         t.stride(3) == 1 and t.data_ptr() % 16 == 0 and not any(s % 8 for s in t.stride()[:3])
         and t.numel() < 2 ** 31 for t in views))
 
 
-def _launch_qk(q, k, cos, sin, rot, pos0, inverse, v=None, k_out=None, v_out=None):
-    """Rotate q and k in one launch: q in place, k in place or into ``k_out`` (then v and the unrotated dims of k are
-    copied to ``v_out`` / ``k_out`` as well)."""
+def _launch_qk(q, k, cos, sin, rot, pos0, inverse, v=None, q_out=None, k_out=None, v_out=None):
+    """Rotate q and k in one launch: q in place or into ``q_out``, k in place or into ``k_out`` (then v and the unrotated
+    dims of k are copied to ``v_out`` / ``k_out`` as well)."""
     S, B, NQ, D = q.shape
-    kd = k if k_out is None else k_out
+    qd, kd = q if q_out is None else q_out, k if k_out is None else k_out
     st = []
-    for t in (q, k, v, kd, v_out):
+    for t in (q, k, v, qd, kd, v_out):
         st += list(t.stride()[:3]) if t is not None else [0, 0, 0]
     LAUNCHES["n"] += 1
-    _lib.check(_lib.lib(q).nx_rope_qk(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(kd), _lib.ptr(v_out),
+    _lib.check(_lib.lib(q).nx_rope_qk(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(qd), _lib.ptr(kd), _lib.ptr(v_out),
                                      _lib.ptr(cos), _lib.ptr(sin), S, B, NQ, k.shape[2], D, rot,
-                                     (_lib.c_ll * 15)(*st), int(pos0), int(inverse), _lib.stream()), "nx_rope_qk")
+                                     (_lib.c_ll * 18)(*st), int(pos0), int(inverse), _lib.stream()), "nx_rope_qk")
 
 
 def rotate_qk_(q, k, cos, sin, rot, pos0, inverse):
     """q and k rotated in place: one launch where their layout allows 16-byte accesses, one each otherwise."""
-    if _qk_ok(rot, q.shape[3], q, k) and cos.data_ptr() % 16 == 0 and sin.data_ptr() % 16 == 0:
+    if _qk_ok(rot, q.shape[3], q, k, tables=(cos, sin)):
         _launch_qk(q, k, cos, sin, rot, pos0, inverse)
     else:
         _launch(q, q, cos, sin, rot, pos0, inverse)

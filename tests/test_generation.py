@@ -396,3 +396,23 @@ def test_a_generation_step_rounds_the_residual_stream_once(precision, x, branch,
     with torch.no_grad():
         out = ParallelTransformerLayer.forward(layer, t)
     assert (out == want).all()
+
+
+@pytest.mark.gpu
+def test_a_generation_step_leaves_the_projection_output_as_a_hook_saw_it():
+    import torch
+    from test_model_gpu import _build
+    _, model = _build(tiny_config(num_layers=2, hidden_size=256, num_attention_heads=4, seq_length=512,
+                                  max_position_embeddings=512, synthetic_vocab_size=1000, pipe_parallel_size=0,
+                                  attention_config=[[["flash"], 2]], distributed_backend="nccl", precision="bfloat16"))
+    model.inference_mode(use_cache=True)
+    kept = []
+    for m in model.modules():
+        if type(m).__name__ == "ParallelSelfAttention":
+            m.query_key_value.register_forward_hook(lambda m, i, o: kept.append((o[0], o[0].clone())))
+    tokens = torch.randint(0, 1000, (2, 20), device="cuda")
+    pos = torch.arange(20, device="cuda")[None].expand(2, -1)
+    with torch.no_grad():
+        for at in (slice(0, 19), slice(19, 20)):
+            model((tokens[:, at].contiguous(), pos[:, at].contiguous(), None))
+    assert len(kept) == 4 and all(torch.equal(a, b) for a, b in kept)

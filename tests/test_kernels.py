@@ -578,6 +578,21 @@ def test_rotate_qk_matches_the_per_tensor_kernel_and_writes_the_cache(hn, rot, n
     assert torch.equal(q2, want_q) and torch.equal(k2, want_k) and torch.equal(v2, want_v)
 
 
+@pytest.mark.parametrize("hn,rot,np_,kvp", [(64, 16, 12, 12), (128, 128, 8, 2), (64, 48, 3, 1)])
+def test_rotate_qk_out_of_place_leaves_the_projection_alone(hn, rot, np_, kvp):
+    from gpt_neox_b200.ops.fused import _qkv_views
+    from gpt_neox_b200.ops.rope import _launch_qk, apply_rotary, rotary_tables
+    torch.manual_seed(4)
+    cos, sin = rotary_tables(rot, 64, device=DEV)
+    qkv = bf(5, 3, (np_ + 2 * kvp) * hn)
+    keep = qkv.clone()
+    q, k, v = _qkv_views(qkv, np_, kvp, hn)
+    out, cache = torch.empty(q.shape, device=DEV, dtype=DT), torch.empty(2, 5, 3, kvp, hn, device=DEV, dtype=DT)
+    _launch_qk(q, k, cos, sin, rot, 7, False, v=v, q_out=out, k_out=cache[0], v_out=cache[1])
+    assert torch.equal(qkv, keep) and torch.equal(out, apply_rotary(q, cos, sin, rot, 7))
+    assert torch.equal(cache[0], apply_rotary(k, cos, sin, rot, 7)) and torch.equal(cache[1], v)
+
+
 @pytest.mark.parametrize("rows,H", [(1, 8), (9, 248), (17, 264), (1001, 1032), (8, 2048), (601, 2048), (3, 2056)])
 @pytest.mark.parametrize("form", ["dual", "layer", "rms"])
 def test_norm_row_sizes(rows, H, form):
