@@ -74,6 +74,32 @@ __global__ void bias_act_fwd_kernel(const h16* __restrict__ x,
   }
 }
 
+// out[r, c] = x[r, c] + (a[r, c] + ba[c]) + (m[r, c] + bm[c]): a parallel-residual layer's stream and its two branches, in
+// fp32 with one rounding.  out may be any of the inputs.  Bound by its launch for the few rows of a generation step.
+__global__ void branch_sum_kernel(const h16* x, const h16* a, const h16* ba, const h16* m, const h16* bm, h16* out,
+                                  long long nvec, int ncols8) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
+    const int c = static_cast<int>(i % ncols8) * 8;
+    float s[8], p[8], q[8], b[8];
+    ld8(x + i * 8, s);
+    ld8(a + i * 8, p);
+    ld8(m + i * 8, q);
+    if (ba != nullptr) {
+      ld8(ba + c, b);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) p[j] += b[j];
+    }
+    if (bm != nullptr) {
+      ld8(bm + c, b);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) q[j] += b[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s[j] = s[j] + p[j] + q[j];
+    st8(out + i * 8, s);
+  }
+}
+
 // dx[r, c] = dy[r, c] * act'(x[r, c] + bias[c])
 __global__ void bias_act_bwd_kernel(const h16* __restrict__ dy,
                                     const h16* __restrict__ x,
@@ -279,6 +305,22 @@ NX_API int NX_SYM(nx_bias_act_fwd)(const void* x, const void* bias, void* y, lon
   if (nvec == 0) return NX_OK;
   bias_act_fwd_kernel<<<grid_for(nvec, 256), 256, 0, (cudaStream_t)stream_>>>(
       (const bf*)x, (const bf*)bias, (bf*)y, nvec, cols / 8, act);
+  NX_LAUNCH_CHECK();
+  return NX_OK;
+}
+// x, a, m, out [rows, cols], out may be x, a or m; ba / bm [cols] or null.  Everything 16-byte aligned.
+NX_API int NX_SYM(nx_branch_sum)(const void* x, const void* a, const void* ba, const void* m, const void* bm, void* out,
+                         long long rows, int cols, void* stream_) {
+  using namespace nx;
+  NX_REQUIRE(cols % 8 == 0, "branch_sum: cols %% 8 != 0");
+  NX_REQUIRE(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(ba) |
+               reinterpret_cast<uintptr_t>(m) | reinterpret_cast<uintptr_t>(bm) | reinterpret_cast<uintptr_t>(out)) & 15) == 0,
+             "branch_sum: operands must be 16-byte aligned");
+  const long long nvec = rows * (cols / 8);
+  if (nvec == 0) return NX_OK;
+  branch_sum_kernel<<<grid_for(nvec, 256), 256, 0, (cudaStream_t)stream_>>>((const bf*)x, (const bf*)a, (const bf*)ba,
+                                                                           (const bf*)m, (const bf*)bm, (bf*)out, nvec,
+                                                                           cols / 8);
   NX_LAUNCH_CHECK();
   return NX_OK;
 }

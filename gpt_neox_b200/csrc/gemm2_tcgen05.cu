@@ -41,9 +41,8 @@ enum Comm : int { COMM_NONE = 0, COMM_RS = 1, COMM_AG = 2, COMM_AR = 3 };
 
 enum Epi : int { BIAS = 1, GELU_ERF = 2, GELU_TANH = 4, AUX_OUT = 8, DGELU_ERF = 16, DGELU_TANH = 32, RESIDUAL = 64,
                  ACCUM = 128, OUT_F32 = 256, SCALE = 512,
-                 AUX_DERIV = 1024,   // aux_out receives gelu'(pre-activation) instead of the pre-activation
-                 MUL_AUX = 2048,     // multiply by aux_in (the stored derivative): no erf / exp in the backward epilogue
-                 ADD_AUX = 4096 };   // + aux_in: a second residual, added before the one rounding (no GeLU then)
+                 AUX_DERIV = 1024,   // aux_out receives gelu'(pre-activation) instead of the pre-activation (none: see EPI_AUX_DERIV)
+                 MUL_AUX = 2048 };   // multiply by aux_in (the stored derivative): no erf / exp in the backward epilogue
 
 struct Params {
   int M, N, K;
@@ -406,7 +405,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
           }
         }
         if (row_ok) {
-          if (flags & AUX_OUT) {
+          if (flags & (AUX_OUT | AUX_DERIV)) {
             h16* ap = p.aux_out + row * p.ld_aux + col0;
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
@@ -423,7 +422,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                 uint4 o;
                 o.x = pack_h16x2(d[0], d[1]); o.y = pack_h16x2(d[2], d[3]);
                 o.z = pack_h16x2(d[4], d[5]); o.w = pack_h16x2(d[6], d[7]);
-                *reinterpret_cast<uint4*>(ap + j) = o;
+                if (flags & AUX_OUT) *reinterpret_cast<uint4*>(ap + j) = o;
               }
             }
           }
@@ -462,19 +461,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
           }
           if (flags & RESIDUAL) {
             const h16* rp = p.residual + row * p.ld_aux + col0;
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              if (col0 + j < p.N) {
-                const uint4 a = *reinterpret_cast<const uint4*>(rp + j);
-                const float2 x0 = unpack_h16x2(a.x), x1 = unpack_h16x2(a.y), x2 = unpack_h16x2(a.z),
-                             x3 = unpack_h16x2(a.w);
-                v[j + 0] += x0.x; v[j + 1] += x0.y; v[j + 2] += x1.x; v[j + 3] += x1.y;
-                v[j + 4] += x2.x; v[j + 5] += x2.y; v[j + 6] += x3.x; v[j + 7] += x3.y;
-              }
-            }
-          }
-          if (flags & ADD_AUX) {
-            const h16* rp = p.aux_in + row * p.ld_aux + col0;
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
               if (col0 + j < p.N) {
@@ -752,11 +738,8 @@ static int gemm2_common(const void* A, const void* B, void* C, int M, int N, int
   NX_REQUIRE(N % 8 == 0 && lda % 8 == 0 && ldb % 8 == 0, "gemm2: N / lda / ldb must be multiples of 8");
   NX_REQUIRE(ldc % ((flags & OUT_F32) ? 4 : 8) == 0, "gemm2: ldc alignment");
   NX_REQUIRE((reinterpret_cast<uintptr_t>(C) & 15) == 0, "gemm2: C must be 16-byte aligned");
-  if (flags & (DGELU_ERF | DGELU_TANH | MUL_AUX | ADD_AUX))
+  if (flags & (DGELU_ERF | DGELU_TANH | MUL_AUX))
     NX_REQUIRE(aux_in != nullptr && ld_aux % 8 == 0, "gemm2: aux_in is required by the epilogue flags");
-  if (flags & ADD_AUX)
-    NX_REQUIRE(!(flags & (GELU_ERF | GELU_TANH | DGELU_ERF | DGELU_TANH | MUL_AUX)) && ca.mode == COMM_NONE,
-               "gemm2: a second residual goes with neither GeLU, a derivative nor a collective");
   if (flags & AUX_OUT) NX_REQUIRE(aux_out != nullptr && ld_aux % 8 == 0, "gemm2: aux_out is required by the flags");
   if (flags & RESIDUAL) NX_REQUIRE(residual != nullptr && ld_aux % 8 == 0, "gemm2: residual is required by the flags");
   if (flags & BIAS) NX_REQUIRE(bias != nullptr, "gemm2: bias is required by the flags");

@@ -12,7 +12,6 @@ struct SkinnyParams {
   h16* C;
   long long ldc;
   const h16* bias;
-  const h16* aux_in;   // second residual
   h16* aux_out;
   const h16* residual;
   long long ld_aux;

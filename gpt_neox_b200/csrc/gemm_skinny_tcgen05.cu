@@ -25,8 +25,7 @@ constexpr int SK_MAX_SPLITS = 8;
 
 // the epilogue bits this kernel knows (same values as in gemm_tcgen05.cu)
 enum : int {
-  SK_BIAS = 1, SK_GELU_ERF = 2, SK_GELU_TANH = 4, SK_AUX_OUT = 8, SK_RESIDUAL = 64, SK_SCALE = 512, SK_AUX_DERIV = 1024,
-  SK_ADD_AUX = 4096
+  SK_BIAS = 1, SK_GELU_ERF = 2, SK_GELU_TANH = 4, SK_AUX_OUT = 8, SK_RESIDUAL = 64, SK_SCALE = 512, SK_AUX_DERIV = 1024
 };
 
 template <int NX, int STAGES>
@@ -60,7 +59,16 @@ __device__ __forceinline__ void skinny_store4(const SkinnyParams& p, int m, int 
     }
     *reinterpret_cast<uint2*>(p.aux_out + aux) = make_uint2(pack_h16x2(d[0], d[1]), pack_h16x2(d[2], d[3]));
   }
-  if (!(p.flags & SK_AUX_DERIV)) {
+  if (p.flags & SK_AUX_DERIV) {
+    if (!(p.flags & SK_AUX_OUT)) {        // the same activation without a place for its derivative
+      float unused;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (p.flags & SK_GELU_TANH) gelu_tanh_both(v[j], v[j], unused);
+        else gelu_erf_both(v[j], v[j], unused);
+      }
+    }
+  } else {
     if (p.flags & SK_GELU_ERF) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) v[j] = gelu_erf(v[j]);
@@ -69,13 +77,11 @@ __device__ __forceinline__ void skinny_store4(const SkinnyParams& p, int m, int 
       for (int j = 0; j < 4; ++j) v[j] = gelu_tanh(v[j]);
     }
   }
-  auto add = [&](const h16* t) {
-    const uint2 r = *reinterpret_cast<const uint2*>(t + aux);
+  if (p.flags & SK_RESIDUAL) {
+    const uint2 r = *reinterpret_cast<const uint2*>(p.residual + aux);
     const float2 a = unpack_h16x2(r.x), b = unpack_h16x2(r.y);
     v[0] += a.x; v[1] += a.y; v[2] += b.x; v[3] += b.y;
-  };
-  if (p.flags & SK_RESIDUAL) add(p.residual);
-  if (p.flags & SK_ADD_AUX) add(p.aux_in);
+  }
   *reinterpret_cast<uint2*>(p.C + m * p.ldc + n) = make_uint2(pack_h16x2(v[0], v[1]), pack_h16x2(v[2], v[3]));
 }
 

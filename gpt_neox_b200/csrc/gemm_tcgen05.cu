@@ -47,9 +47,9 @@ enum EpiFlags : int {
   EPI_OUT_F32 = 256,    // C is fp32 instead of bf16
   EPI_SCALE = 512,      // result *= alpha (applied first)
   EPI_AUX_DERIV = 1024, // with AUX_OUT + a GeLU flag: aux_out receives gelu'(pre-activation) instead of it, so
-                        // that the backward GEMM's epilogue is one multiply (EPI_MUL_AUX) with no erf / exp
+                        // that the backward GEMM's epilogue is one multiply (EPI_MUL_AUX) with no erf / exp;
+                        // without AUX_OUT: the activation as it is rounded there (a pass that nothing records)
   EPI_MUL_AUX = 2048,   // multiply by aux_in
-  EPI_ADD_AUX = 4096,   // + aux_in: a second residual, so that both are added before the one rounding (no GeLU then)
 };
 
 struct GemmParams {
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
           }
         }
         if (row_ok) {
-          if (flags & EPI_AUX_OUT) {
+          if (flags & (EPI_AUX_OUT | EPI_AUX_DERIV)) {
             h16* ap = p.aux_out + row * p.ld_aux + col0;
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                 o.y = pack_h16x2(d[2], d[3]);
                 o.z = pack_h16x2(d[4], d[5]);
                 o.w = pack_h16x2(d[6], d[7]);
-                *reinterpret_cast<uint4*>(ap + j) = o;
+                if (flags & EPI_AUX_OUT) *reinterpret_cast<uint4*>(ap + j) = o;
               }
             }
           }
@@ -449,19 +449,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
           }
           if (flags & EPI_RESIDUAL) {
             const h16* rp = p.residual + row * p.ld_aux + col0;
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              if (col0 + j < p.N) {
-                const uint4 a = *reinterpret_cast<const uint4*>(rp + j);
-                const float2 x0 = unpack_h16x2(a.x), x1 = unpack_h16x2(a.y),
-                             x2 = unpack_h16x2(a.z), x3 = unpack_h16x2(a.w);
-                v[j + 0] += x0.x; v[j + 1] += x0.y; v[j + 2] += x1.x; v[j + 3] += x1.y;
-                v[j + 4] += x2.x; v[j + 5] += x2.y; v[j + 6] += x3.x; v[j + 7] += x3.y;
-              }
-            }
-          }
-          if (flags & EPI_ADD_AUX) {
-            const h16* rp = p.aux_in + row * p.ld_aux + col0;
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
               if (col0 + j < p.N) {
@@ -718,8 +705,7 @@ struct CommArgs {
 // 16384 110.7 / 42.0 us; 2304 x 768 16.4 / 17.3 us, at 96 rows 16.4 / 15.3 us).
 static bool skinny_better(int M, int N, int K, int transA, int transB, int flags) {
   using namespace nx;
-  constexpr int known = EPI_BIAS | EPI_GELU_ERF | EPI_GELU_TANH | EPI_AUX_OUT | EPI_AUX_DERIV | EPI_RESIDUAL | EPI_SCALE |
-                        EPI_ADD_AUX;
+  constexpr int known = EPI_BIAS | EPI_GELU_ERF | EPI_GELU_TANH | EPI_AUX_OUT | EPI_AUX_DERIV | EPI_RESIDUAL | EPI_SCALE;
   if (transA || transB || (flags & ~known) != 0 || M > SKINNY_MAX_M) return false;
   const int BN = N <= 128 ? 128 : 256;
   const long long tiles = static_cast<long long>((M + BM - 1) / BM) * ((N + BN - 1) / BN);
@@ -738,11 +724,8 @@ static int gemm_common(const void* A, const void* B, void* C, int M, int N, int 
   NX_REQUIRE(ldc % ((flags & EPI_OUT_F32) ? 4 : 8) == 0, "gemm: ldc alignment");
   NX_REQUIRE((reinterpret_cast<uintptr_t>(C) & 15) == 0, "gemm: C must be 16-byte aligned");
   if (flags & EPI_BIAS) NX_REQUIRE(bias != nullptr && (reinterpret_cast<uintptr_t>(bias) & 15) == 0, "gemm: bias null/unaligned");
-  if (flags & (EPI_DGELU_ERF | EPI_DGELU_TANH | EPI_MUL_AUX | EPI_ADD_AUX))
+  if (flags & (EPI_DGELU_ERF | EPI_DGELU_TANH | EPI_MUL_AUX))
     NX_REQUIRE(aux_in != nullptr && ld_aux % 8 == 0, "gemm: aux_in");
-  if (flags & EPI_ADD_AUX)
-    NX_REQUIRE(!(flags & (EPI_GELU_ERF | EPI_GELU_TANH | EPI_DGELU_ERF | EPI_DGELU_TANH | EPI_MUL_AUX)) && ca.mode == COMM_NONE,
-               "gemm: a second residual goes with neither GeLU, a derivative nor a collective");
   if (flags & EPI_AUX_OUT) NX_REQUIRE(aux_out != nullptr && ld_aux % 8 == 0, "gemm: aux_out");
   if (flags & EPI_RESIDUAL) NX_REQUIRE(residual != nullptr && ld_aux % 8 == 0, "gemm: residual");
 
@@ -751,7 +734,6 @@ static int gemm_common(const void* A, const void* B, void* C, int M, int N, int 
     q.M = M; q.N = N; q.K = K;
     q.C = static_cast<h16*>(C); q.ldc = ldc;
     q.bias = static_cast<const h16*>(bias);
-    q.aux_in = static_cast<const h16*>(aux_in);
     q.aux_out = static_cast<h16*>(aux_out);
     q.residual = static_cast<const h16*>(residual);
     q.ld_aux = ld_aux;

@@ -3,9 +3,8 @@
 //
 // A step of a few tokens keeps the GPU busy for 30 - 40 us per layer; issued op by op the eight launches cost several
 // times that on the host.  The kernels, their order and their arguments are those of the op-by-op path
-// (models/transformer.py, ParallelTransformerLayer.forward with `use_cache`), so both give the same bits.  The attention
-// branch is rounded at its own size; it, the MLP and the residual stream meet in fp32 in the last GEMM's epilogue, so the
-// stream is rounded once per layer.
+// (models/transformer.py, ParallelTransformerLayer.forward with `use_cache`), so both give the same bits: the branches
+// are what the two modules return, rounded at their own size, and meet the residual stream in fp32 in the last kernel.
 #include "common.h"
 
 NX_API int NX_SYM(nx_norm_fwd)(int kind, const void* x, const void* g1, const void* b1, void* y1, const void* g2,
@@ -16,6 +15,8 @@ NX_API int NX_SYM(nx_gemm_bf16)(const void* A, const void* B, void* C, int M, in
 NX_API int NX_SYM(nx_gemm2_bf16)(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                          long long ldc, int transA, int transB, const void* bias, const void* aux_in, void* aux_out,
                          const void* residual, long long ld_aux, int flags, float alpha, void* stream_);
+NX_API int NX_SYM(nx_branch_sum)(const void* x, const void* a, const void* ba, const void* m, const void* bm, void* out,
+                         long long rows, int cols, void* stream_);
 NX_API int NX_SYM(nx_rope_qk)(const void* q, const void* k, const void* v, void* qd, void* kd, void* vd, const void* cos,
                       const void* sin, int S, int B, int NQ, int NK, int D, int R, const long long* strides, int pos0,
                       int inverse, void* stream_);
@@ -37,14 +38,14 @@ struct nx_layer_infer_args {
   // layer; stats, fp32: mean and rstd of every row, the log-sum-exp of the attention [b, np, s rounded up to 128]
   void *cache, *work, *stats, *out;
   long long cache_kv_stride;            // elements between the key and the value part of the cache
-  int s, b, h, np, kvp, hn, ffn, past, rot, window, gelu_tanh, pair_gemm;
+  int s, b, h, np, kvp, hn, ffn, past, rot, window, act, pair_gemm;     // act: the GeLU's EPI_* bits (gemm_tcgen05.cu)
   float eps, scale;
 };
 }
 
 NX_API int NX_SYM(nx_layer_infer)(const nx_layer_infer_args* a, void* stream) {
   using namespace nx;
-  enum { BIAS = 1, GELU_ERF = 2, GELU_TANH = 4, RESIDUAL = 64, ADD_AUX = 4096 };
+  enum { BIAS = 1 };
   const long long rows = static_cast<long long>(a->s) * a->b;
   if (rows == 0) return NX_OK;
   NX_REQUIRE(rows < (1ll << 31), "layer_infer: too many rows");
@@ -55,11 +56,9 @@ NX_API int NX_SYM(nx_layer_infer)(const nx_layer_infer_args* a, void* stream) {
   uint16_t *x1 = w, *x2 = x1 + rows * a->h, *t = x2 + rows * a->h, *qkv = t + rows * a->h, *ctx = qkv + rows * qkv_n,
            *mid = ctx + rows * ctx_n;
   float *mean = static_cast<float*>(a->stats), *rstd = mean + rows, *lse = rstd + rows;
-  auto gemm = [&](const void* A, const void* W, void* C, int N, int K, const void* bias, int act,
-                  const void* residual = nullptr, const void* residual2 = nullptr) {
-    const int flags = act | (bias != nullptr ? BIAS : 0) | (residual != nullptr ? RESIDUAL | ADD_AUX : 0);
+  auto gemm = [&](const void* A, const void* W, void* C, int N, int K, const void* bias, int act) {
     auto fn = a->pair_gemm && M >= 256 && N >= 256 ? NX_SYM(nx_gemm2_bf16) : NX_SYM(nx_gemm_bf16);
-    return fn(A, W, C, M, N, K, K, K, N, 0, 0, bias, residual2, nullptr, residual, residual != nullptr ? N : 0, flags, 1.f,
+    return fn(A, W, C, M, N, K, K, K, N, 0, 0, bias, nullptr, nullptr, nullptr, 0, act | (bias != nullptr ? BIAS : 0), 1.f,
               stream);
   };
 #define NX_TRY(expr)                  \
@@ -83,9 +82,10 @@ NX_API int NX_SYM(nx_layer_infer)(const nx_layer_infer_args* a, void* stream) {
   NX_TRY(NX_SYM(nx_flash_attn_fwd)(q, kc, vc, ctx, lse, nullptr, a->b, a->np, a->kvp, a->s, a->past + a->s, hn, sb, sh, ss,
                                    cb, hn, cs, cb, hn, cs, ctx_n, hn, static_cast<long long>(a->b) * ctx_n, a->scale, 1,
                                    a->window, 0.f, 0, nullptr, nullptr, 0, stream));
-  NX_TRY(gemm(ctx, a->w_dense, t, a->h, ctx_n, a->b_dense, 0));
-  NX_TRY(gemm(x2, a->w1, mid, a->ffn, a->h, a->b1, a->gelu_tanh ? GELU_TANH : GELU_ERF));
-  NX_TRY(gemm(mid, a->w2, a->out, a->h, a->ffn, a->b2, 0, t, a->x));
+  NX_TRY(gemm(ctx, a->w_dense, t, a->h, ctx_n, nullptr, 0));
+  NX_TRY(gemm(x2, a->w1, mid, a->ffn, a->h, a->b1, a->act));
+  NX_TRY(gemm(mid, a->w2, a->out, a->h, a->ffn, nullptr, 0));
+  NX_TRY(NX_SYM(nx_branch_sum)(a->x, t, a->b_dense, a->out, a->b2, a->out, rows, a->h, stream));
 #undef NX_TRY
   return NX_OK;
 }

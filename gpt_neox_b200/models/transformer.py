@@ -20,7 +20,7 @@ import torch.nn.functional as F
 from .. import parallel as mpu
 from ..ops import fused as fused_ops
 from ..ops.attention import flash_attention, next_dropout_seed
-from ..ops.elementwise import bias_dropout_add
+from ..ops.elementwise import bias_dropout_add, branch_sum
 from ..ops.gemm import gemm as gemm_op
 from ..ops.gemm import linear as linear_op
 from ..ops.layer_infer import layer_infer, pointers
@@ -90,20 +90,16 @@ class ParallelMLP(nn.Module):
             return False        # fp8 GEMMs run through the per-module path
         return (not self.is_gated) and self.activation_type == "gelu" and x.is_cuda and x.dtype in (torch.bfloat16, torch.float16)
 
-    def forward(self, hidden_states, residual=None, out_bias=None, residual2=None):
+    def forward(self, hidden_states, residual=None, out_bias=None):
         """-> (output without linear2's bias, that bias). ``residual`` (optional, fused path only)
         is added inside the second GEMM's epilogue; so is ``out_bias`` (a bias vector that already
-        includes linear2's: the returned bias is then None).  ``residual2``: a second residual, for a generation
-        step without autograd on one tensor-parallel rank."""
+        includes linear2's: the returned bias is then None)."""
         if self._fusable(hidden_states):
             if self.sequence_parallel:
                 x = gather_from_sequence_parallel_region(hidden_states, seq_dim=0)
             else:
                 x = copy_to_model_parallel_region(hidden_states)
             kind = "tanh" if self.bias_gelu_fusion else "erf"
-            if residual2 is not None:
-                return fused_ops.mlp_gelu_infer(x, self.linear1.weight, self.linear1.bias, self.linear2.weight, out_bias,
-                                                residual, residual2, kind), None
             out = fused_ops.mlp_gelu(x, self.linear1.weight, self.linear1.bias, self.linear2.weight, out_bias,
                                      residual=residual, kind=kind, recompute_act=self.recompute_act)
             if not self.parallel_output:
@@ -317,10 +313,9 @@ class ParallelSelfAttention(nn.Module):
         return q, present
 
     # -------------------------------------------------------------------- forward
-    def forward(self, hidden_states, attention_mask=None, layer_past=None, residual=None, add_bias=False):
+    def forward(self, hidden_states, attention_mask=None, layer_past=None, residual=None):
         """hidden_states [sq, b, h] -> (output [sq, b, h] without dense bias, dense bias)
-        (+ the updated KV cache when ``use_cache``).  ``add_bias``: the bias is added by the projection's GEMM (a
-        generation step without autograd on one tensor-parallel rank); None is returned for it."""
+        (+ the updated KV cache when ``use_cache``)."""
         mixed, _ = self.query_key_value(hidden_states)
         np_, kvp, hn = self.num_attention_heads_per_partition, self.num_kv_heads_per_partition, \
             self.hidden_size_per_attention_head
@@ -375,9 +370,7 @@ class ParallelSelfAttention(nn.Module):
                     mask = self.sparse_mask[..., sk_ - q.shape[0]:sk_, :sk_]
                 ctx = self._global_attention(q, k, v, mask)
         # output projection; bias (and the optional residual) are applied by the caller / epilogue
-        if add_bias:
-            out, bias = linear_op(ctx, self.dense.weight, self.dense.bias), None
-        elif residual is not None and ctx.is_cuda and not self.dense.sequence_parallel and \
+        if residual is not None and ctx.is_cuda and not self.dense.sequence_parallel and \
                 mpu.get_model_parallel_world_size() == 1:
             out = _linear_residual(ctx, self.dense.weight, residual)
             bias = self.dense.bias
@@ -504,7 +497,7 @@ class ParallelTransformerLayer(nn.Module):
             x, ptrs, cos, sin, present, past,
             heads=a.num_attention_heads_per_partition, kv_heads=kvp, head_dim=hn, ffn=up.shape[0], rot=a.rotary_dim,
             window=a.sliding_window_width if a.sliding_window_width is not None else -1, scale=a.attn_scale, eps=n1.eps,
-            gelu="tanh" if m.bias_gelu_fusion else "erf")
+            act=("tanh" if m.bias_gelu_fusion else "erf", not m.recompute_act))
         self.layer_past = present
         return out
 
@@ -554,9 +547,11 @@ class ParallelTransformerLayer(nn.Module):
                     return fused_tp.mlp_gelu_sp(x2, self.mlp.linear1.weight, self.mlp.linear1.bias,
                                                 self.mlp.linear2.weight, attn_partial, bias_total, residual, kind, be)
             if fast and self.use_cache and kernel_lib.untracked():
-                # generation: the branches at their own size, then x + attn + mlp in one epilogue and one rounding
-                t, _, self.layer_past = self.attention(x1, attention_mask, layer_past=layer_past, add_bias=True)
-                return self.mlp(x2, residual=t, out_bias=self.mlp.linear2.bias, residual2=residual)[0]
+                # generation: both modules give their plain output (a hook on them sees that), and stream, branches and
+                # biases meet in one kernel and one rounding
+                attn, b_attn, self.layer_past = self.attention(x1, attention_mask, layer_past=layer_past)
+                mlp, b_mlp = self.mlp(x2)
+                return branch_sum(residual, attn, b_attn, mlp, b_mlp)
             if fast and not self.use_cache:
                 # x + attn + b_attn + mlp + b_mlp with both adds of matrices inside GEMM epilogues:
                 #   t = dense(ctx) + x ;  out = linear2(h) + t ; the two bias vectors are added once.

@@ -81,6 +81,7 @@ def _declare(lib):
     sig("nx_norm_bwd_blocks", [L])
     sig("nx_norm_bwd", [I, P, P, P, P, P, P, P, P, P, P, P, P, P, P, L, I, I, I, P])
     sig("nx_bias_act_fwd", [P, P, P, L, I, I, P])
+    sig("nx_branch_sum", [P, P, P, P, P, P, L, I, P])
     sig("nx_bias_act_bwd", [P, P, P, P, L, I, I, P])
     sig("nx_gated_act_fwd", [P, P, L, I, I, P])
     sig("nx_gated_act_bwd", [P, P, P, L, I, I, P])

@@ -199,3 +199,15 @@ def bias_dropout_add(x, bias, residual, p: float, training: bool):
     out = x if bias is None else x + bias
     out = F.dropout(out, p=p, training=training)
     return out if residual is None else residual + out
+
+
+def branch_sum(x, a, a_bias, m, m_bias):
+    """``x + (a + a_bias) + (m + m_bias)`` (biases may be None) with one rounding, without autograd: CUDA 16-bit tensors of
+    one shape."""
+    x, a, m = (t.contiguous() for t in (x, a, m))
+    out = torch.empty_like(x)
+    LAUNCHES["n"] += 1
+    _lib.check(_lib.lib(x).nx_branch_sum(_lib.ptr(x), _lib.ptr(a), _lib.ptr(a_bias), _lib.ptr(m), _lib.ptr(m_bias),
+                                         _lib.ptr(out), x.numel() // x.shape[-1], x.shape[-1], _lib.stream()),
+               "nx_branch_sum")
+    return out

@@ -71,22 +71,19 @@ class _MLPGeluFn(torch.autograd.Function):
 def mlp_gelu(x, w1, b1, w2, b2=None, residual=None, kind: str = "erf", recompute_act: bool = False):
     """``gelu(x @ w1^T + b1) @ w2^T (+ b2) (+ residual)``; kind in {"erf", "tanh"}."""
     if x.is_cuda and x.dtype in _lib.H16:
+        if _lib.untracked():
+            # nothing asks for the activation's derivative, but the bits are those of the recorded pass: a checkpointed
+            # region runs like this first and with gradients in the backward
+            x2 = x.reshape(-1, x.shape[-1]).contiguous()
+            r2 = residual.reshape(x2.shape[0], -1).contiguous() if residual is not None else None
+            y = gemm(gemm(x2, w1, bias=b1, gelu=kind, aux_deriv=not recompute_act), w2, bias=b2, residual=r2)
+            return y.view(*x.shape[:-1], w2.shape[0])
         return _MLPGeluFn.apply(x, w1, b1, w2, b2, residual, kind, recompute_act)
     if x.is_cuda:
         raise _lib.KernelError("mlp_gelu: CUDA path needs bf16")
     h = F.gelu(F.linear(x, w1, b1), approximate="tanh" if kind == "tanh" else "none")
     y = F.linear(h, w2, b2)
     return y if residual is None else y + residual
-
-
-def mlp_gelu_infer(x, w1, b1, w2, b2, residual, residual2, kind):
-    """``mlp_gelu`` of a generation step with two residuals: no autograd node and no stored derivative.  Its GeLU is rounded
-    differently from the one that is evaluated together with the derivative, so nothing that a recompute repeats may call
-    it."""
-    x2 = x.reshape(-1, x.shape[-1]).contiguous()
-    r, r2 = (t.reshape(x2.shape[0], -1).contiguous() for t in (residual, residual2))
-    y = gemm(gemm(x2, w1, bias=b1, gelu=kind), w2, bias=b2, residual=r, residual2=r2)
-    return y.view(*x.shape[:-1], w2.shape[0])
 
 
 def _qkv_views(qkv, np_, kvp, hn):

@@ -27,7 +27,6 @@ EPI_OUT_F32 = 256
 EPI_SCALE = 512
 EPI_AUX_DERIV = 1024       # aux_out receives gelu'(pre-activation) instead of the pre-activation
 EPI_MUL_AUX = 2048         # multiply by dgelu_aux as it is (a stored derivative)
-EPI_ADD_AUX = 4096         # + a second residual
 
 #: counts launches of this library's kernels (read by bench.py for its ``gpu_launches`` claim)
 LAUNCHES = {"n": 0}
@@ -45,13 +44,14 @@ def _as_2d(x: torch.Tensor) -> torch.Tensor:
 def aux_flags(gelu, aux_out, aux_deriv, dgelu_aux, dgelu) -> int:
     """Epilogue flags of the auxiliary operands.  ``aux_deriv``: ``aux_out`` receives gelu'(pre-activation)
     instead of the pre-activation; the matching backward GEMM passes it as ``dgelu_aux`` with ``dgelu="mul"``,
-    so its epilogue is one multiply instead of an erf / exp evaluation per element."""
+    so its epilogue is one multiply instead of an erf / exp evaluation per element.  Without ``aux_out`` nothing is stored,
+    but the activation has the bits it has beside its derivative."""
     flags = 0
     if aux_out is not None:
         flags |= EPI_AUX_OUT
-        if aux_deriv:
-            assert gelu is not None, "aux_deriv needs a GeLU epilogue"
-            flags |= EPI_AUX_DERIV
+    if aux_deriv:
+        assert gelu is not None, "aux_deriv needs a GeLU epilogue"
+        flags |= EPI_AUX_DERIV
     if dgelu_aux is not None:
         flags |= {"tanh": EPI_DGELU_TANH, "mul": EPI_MUL_AUX}.get(dgelu, EPI_DGELU_ERF)
     return flags
@@ -63,14 +63,14 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
          dgelu: str | None = None, residual: torch.Tensor | None = None,
          out: torch.Tensor | None = None, accumulate: bool = False,
          out_dtype: torch.dtype | None = None, alpha: float | None = None,
-         aux_deriv: bool = False, residual2: torch.Tensor | None = None) -> torch.Tensor:
+         aux_deriv: bool = False) -> torch.Tensor:
     """``C = epilogue(op(a) @ op(b))`` with 2-D row-major 16-bit operands (bf16 or fp16, both the same dtype).
 
     ``trans_a=False``: a is [M,K]; ``True``: a is [K,M].
     ``trans_b=False``: b is [N,K] (weight layout); ``True``: b is [K,N].
     Epilogue order: scale, +bias, store ``aux_out`` (the pre-activation, or its GeLU derivative with
-    ``aux_deriv``), ×gelu'(``dgelu_aux``) (``dgelu="mul"``: × ``dgelu_aux`` itself), GeLU, +residual, +residual2,
-    (+= out if ``accumulate``).  ``residual2`` goes with neither ``gelu`` nor ``dgelu_aux``.
+    ``aux_deriv``), ×gelu'(``dgelu_aux``) (``dgelu="mul"``: × ``dgelu_aux`` itself), GeLU, +residual,
+    (+= out if ``accumulate``).
     """
     assert a.is_cuda and a.dtype in _lib.H16 and b.dtype == a.dtype, (a.dtype, b.dtype)
     if trans_a:
@@ -99,7 +99,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
     if gelu is not None:
         flags |= EPI_GELU_TANH if gelu == "tanh" else EPI_GELU_ERF
     ld_aux = 0
-    for t in (aux_out, dgelu_aux, residual, residual2):
+    for t in (aux_out, dgelu_aux, residual):
         if t is not None:
             assert t.shape == (M, N) and t.stride(1) == 1 and t.dtype == a.dtype
             assert ld_aux in (0, t.stride(0)), "aux tensors must share one leading dimension"
@@ -107,9 +107,6 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
     flags |= aux_flags(gelu, aux_out, aux_deriv, dgelu_aux, dgelu)
     if residual is not None:
         flags |= EPI_RESIDUAL
-    if residual2 is not None:
-        assert dgelu_aux is None and gelu is None
-        flags |= EPI_ADD_AUX
     if accumulate:
         flags |= EPI_ACCUM
     if alpha is not None:
@@ -121,7 +118,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         fn, name = L.nx_gemm2_bf16, "nx_gemm2_bf16"      # CTA-pair kernel (cta_group::2, 256 x 256 tiles)
     _lib.check(fn(
         _lib.ptr(a), _lib.ptr(b), _lib.ptr(out), M, N, K, a.stride(0), b.stride(0), out.stride(0),
-        int(trans_a), int(trans_b), _lib.ptr(bias), _lib.ptr(dgelu_aux if residual2 is None else residual2), _lib.ptr(aux_out),
+        int(trans_a), int(trans_b), _lib.ptr(bias), _lib.ptr(dgelu_aux), _lib.ptr(aux_out),
         _lib.ptr(residual), ld_aux, flags, float(alpha if alpha is not None else 1.0),
         _lib.stream()), name)
     return out

@@ -379,7 +379,7 @@ def test_a_layer_in_one_call_gives_the_bits_of_the_op_by_op_path(over, precision
 def test_a_generation_step_rounds_the_residual_stream_once(precision, x, branch, want, hook, rows):
     """Attention and MLP add less than half a unit in the last place of the residual stream each, and more than half
     together (all matrices zero, so that the branches are their last biases): with the sum rounded once the stream moves,
-    with a rounding after each branch it does not.  One native call and op by op; the three GEMM kernels."""
+    with a rounding after each branch it does not.  One native call and op by op."""
     import torch
     from gpt_neox_b200.models.transformer import ParallelTransformerLayer
     from test_model_gpu import _build
@@ -416,3 +416,39 @@ def test_a_generation_step_leaves_the_projection_output_as_a_hook_saw_it():
         for at in (slice(0, 19), slice(19, 20)):
             model((tokens[:, at].contiguous(), pos[:, at].contiguous(), None))
     assert len(kept) == 4 and all(torch.equal(a, b) for a, b in kept)
+
+
+@pytest.mark.gpu
+def test_hooks_see_the_modules_own_outputs_while_generating():
+    """Hooks on the attention, its output projection and the MLP fire, and see what the modules return when called alone:
+    the branch without the residual stream, and the bias beside it."""
+    import torch
+    from test_model_gpu import _build
+    _, model = _build(tiny_config(num_layers=2, hidden_size=256, num_attention_heads=4, seq_length=512,
+                                  max_position_embeddings=512, synthetic_vocab_size=1000, pipe_parallel_size=0,
+                                  attention_config=[[["flash"], 2]], distributed_backend="nccl", precision="bfloat16"))
+    for n, p in model.named_parameters():
+        if n.endswith("bias"):
+            torch.nn.init.normal_(p, std=0.3)
+    model.inference_mode(use_cache=True)
+    tokens = torch.randint(0, 1000, (2, 20), device="cuda")
+    pos = torch.arange(20, device="cuda")[None].expand(2, -1)
+    run = lambda: [model((tokens[:, a].contiguous(), pos[:, a].contiguous(), None)) for a in (slice(0, 19), slice(19, 20))]
+    with torch.no_grad():
+        plain = run()
+        seen = []
+        layers = [m for m in model.modules() if type(m).__name__.startswith("ParallelTransformerLayer")]
+        handles = [m.register_forward_hook(lambda m, i, o: seen.append((m, i, o)))
+                   for l in layers for m in (l.attention, l.attention.dense, l.mlp)]
+        model.clear_cache()
+        hooked = run()
+        for h in handles:
+            h.remove()
+        assert len(seen) == 2 * 2 * 3
+        for m, i, o in seen:
+            name = type(m).__name__
+            assert o[1] is {"ParallelSelfAttention": lambda: m.dense.bias, "RowParallelLinear": lambda: m.bias,
+                            "ParallelMLP": lambda: m.linear2.bias}[name]()
+            if name != "ParallelSelfAttention":
+                assert len(i) == 1 and torch.equal(m(i[0])[0], o[0])
+    assert all(torch.equal(a, b) for a, b in zip(plain, hooked))

@@ -671,3 +671,15 @@ def test_one_query_attention_passes_nan_and_inf_on(sk, h, hk):
             assert not math.isnan(value) or one[hit].isnan().any(-1).all()
             one[hit] = 0
             assert one.isfinite().all()
+
+
+@pytest.mark.parametrize("rows,H", [(1, 8), (3, 2056), (600, 768)])
+@pytest.mark.parametrize("ba,bm", [(True, True), (False, True), (False, False)])
+def test_branch_sum_rounds_once(rows, H, ba, bm):
+    from gpt_neox_b200.ops.elementwise import branch_sum
+    torch.manual_seed(23)
+    x, a, m = bf(rows, H, scale=100.0), bf(rows, H), bf(rows, H)
+    b1, b2 = bf(H) if ba else None, bf(H) if bm else None
+    got = branch_sum(x, a, b1, m, b2)
+    p, q = (t.float() if b is None else t.float() + b.float() for t, b in ((a, b1), (m, b2)))
+    assert torch.equal(got, (x.float() + p + q).to(DT))
