@@ -462,25 +462,24 @@ class ParallelTransformerLayer(nn.Module):
     def _infer(self, x, layer_past):
         """The whole layer in one native call, or None where it has to run op by op: generation without autograd, dense
         parallel-residual layer with two LayerNorms, rotary flash attention and a GeLU MLP on one tensor-parallel rank,
-        plain modules that nobody hooks into."""
+        plain modules whose calls nobody hooks into or replaces."""
         a, m = self.attention, self.mlp
         if not (self.use_cache and x.is_cuda and x.is_contiguous() and x.shape[0] > 0 and x.shape[1] > 0
                 and kernel_lib.untracked() and self._dual_norm_ok(x)
-                and type(a) is ParallelSelfAttention and type(m) is ParallelMLP and a.use_cache and a.use_flash_attention
+                and _plain(a, ParallelSelfAttention) and _plain(m, ParallelMLP) and a.use_cache and a.use_flash_attention
                 and not a.use_qk_layernorm and a.rpe is None and a.rotary_emb is not None
                 and not (self.training and (self.hidden_dropout > 0 or a.dropout_p > 0))
                 and mpu.get_model_parallel_world_size() == 1 and m._fusable(x)):
             return None
         hn = a.hidden_size_per_attention_head
         linears = (a.query_key_value, a.dense, m.linear1, m.linear2)
-        mods = (self.input_layernorm, self.post_attention_layernorm, a, a.rotary_emb, m) + linears
         if hn % 8 or hn > 128 or a.rotary_dim % 16 or any(
                 l.use_mup or getattr(l, "use_fp8", False) or getattr(l, "gather_output", False) for l in linears) \
-                or type(linears[0]) is not mpu.ColumnParallelLinear or type(linears[2]) is not mpu.ColumnParallelLinear \
-                or type(linears[1]) is not mpu.RowParallelLinear or type(linears[3]) is not mpu.RowParallelLinear \
-                or linears[0].skip_bias_add \
-                or torch.nn.modules.module._has_any_global_hook() or any(
-                    z._forward_hooks or z._forward_pre_hooks for z in mods):
+                or not (_plain(linears[0], mpu.ColumnParallelLinear) and _plain(linears[2], mpu.ColumnParallelLinear)
+                        and _plain(linears[1], mpu.RowParallelLinear) and _plain(linears[3], mpu.RowParallelLinear)
+                        and _plain(a.rotary_emb, RotaryEmbedding) and _plain(self.input_layernorm, LayerNorm)
+                        and _plain(self.post_attention_layernorm, LayerNorm)) \
+                or linears[0].skip_bias_add or torch.nn.modules.module._has_any_global_hook():
             return None
         n1, n2, up = self.input_layernorm, self.post_attention_layernorm, m.linear1.weight
         ptrs = pointers(x, n1.weight, n1.bias, n2.weight, n2.bias, *(t for l in linears for t in (l.weight, l.bias)))
@@ -597,6 +596,19 @@ class ParallelTransformerLayer(nn.Module):
         if mlp_bias is None and (self.num_experts > 1 or p == 0.0):
             return mlp_output + attention_output
         return bias_dropout_add(mlp_output, mlp_bias, attention_output, p, self.training)
+
+
+#: the forwards whose work the native layer call does itself
+_FORWARD = {c: c.forward for c in (ParallelSelfAttention, ParallelMLP, LayerNorm, RotaryEmbedding, mpu.ColumnParallelLinear,
+                                   mpu.RowParallelLinear)}
+
+
+def _plain(m, cls):
+    """Whether calling ``m`` runs ``cls.forward`` as it was defined and nothing else: no subclass (a parametrized module is
+    one), no hook, no forward replaced on the instance or on the class."""
+    d = m.__dict__
+    return type(m) is cls and cls.forward is _FORWARD[cls] and "forward" not in d and not d["_forward_hooks"] \
+        and not d["_forward_pre_hooks"]
 
 
 def _sum_bias(a, b):

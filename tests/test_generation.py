@@ -452,3 +452,41 @@ def test_hooks_see_the_modules_own_outputs_while_generating():
             if name != "ParallelSelfAttention":
                 assert len(i) == 1 and torch.equal(m(i[0])[0], o[0])
     assert all(torch.equal(a, b) for a, b in zip(plain, hooked))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,where", [(n, w) for n in ("attention", "attention.query_key_value", "attention.dense", "mlp")
+                                        for w in ("instance", "class")]
+                         + [(n, "parametrized") for n in ("input_layernorm", "attention.dense", "mlp.linear1")])
+def test_a_replaced_forward_is_called_while_generating(name, where, monkeypatch):
+    """Modules that generation calls: a forward replaced on one instance or on the class runs, and a weight that is computed
+    on access (a parametrization, whose value lives as long as the access) is used."""
+    import torch
+    from torch.nn.utils import parametrize
+    from test_model_gpu import _build
+    _, model = _build(tiny_config(num_layers=2, hidden_size=256, num_attention_heads=4, seq_length=512,
+                                  max_position_embeddings=512, synthetic_vocab_size=1000, pipe_parallel_size=0,
+                                  attention_config=[[["flash"], 2]], distributed_backend="nccl", precision="bfloat16"))
+    model.inference_mode(use_cache=True)
+    layers = [m for m in model.modules() if type(m).__name__.startswith("ParallelTransformerLayer")]
+    target = layers[0].get_submodule(name)
+    tokens = torch.randint(0, 1000, (2, 20), device="cuda")
+    pos = torch.arange(20, device="cuda")[None].expand(2, -1)
+    calls = []
+    with torch.no_grad():
+        want = model((tokens, pos, None))
+        if where == "parametrized":
+            class Count(torch.nn.Module):
+                def forward(self, w):
+                    calls.append(target)
+                    return w * 1
+            parametrize.register_parametrization(target, "weight", Count())
+            calls.clear()
+        else:
+            owner = target if where == "instance" else type(target)
+            old = owner.forward
+            monkeypatch.setattr(owner, "forward", lambda *a, **k: (calls.append(a[0] if where == "class" else target), old(*a, **k))[1],
+                                raising=False)
+        model.clear_cache()
+        got = model((tokens, pos, None))
+    assert any(c is target for c in calls) and torch.equal(got, want)
