@@ -848,9 +848,8 @@ static int launch_bwd_h(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
   if (PIPE && serial_q && serial_k) return launch_bwd_as<DP, DROP, HALVES, false, false, true>(tq, tk, tv, tdo, p, s);
   if (PIPE && serial_q) return launch_bwd_as<DP, DROP, HALVES, false, PIPE, true>(tq, tk, tv, tdo, p, s);
   if (PIPE && serial_k) return launch_bwd_as<DP, DROP, HALVES, PIPE, false, true>(tq, tk, tv, tdo, p, s);
-  // (a row without a visible key, possible for Sq > Sk, has lse = -inf: there a masked score must not reach the exponent;
-  //  a zero scale would turn a masked score into NaN)
-  if (!PIPE || DROP || p.alibi != nullptr || p.blk_rows != nullptr || p.Sq > p.Sk || p.scale == 0.f)
+  // (a zero scale would turn a masked score into NaN)
+  if (!PIPE || DROP || p.alibi != nullptr || p.blk_rows != nullptr || p.scale == 0.f)
     return launch_bwd_as<DP, DROP, HALVES, PIPE, PIPE, true>(tq, tk, tv, tdo, p, s);
   return launch_bwd_as<DP, DROP, HALVES, PIPE, PIPE, false>(tq, tk, tv, tdo, p, s);
 }

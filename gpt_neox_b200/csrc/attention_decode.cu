@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(DEC_THREADS, dec_ctas(GT)) attn_decode_kernel(
     }
     // (a NaN sum, from a NaN or +inf score, has to reach the output: only a sum of exactly 0 means a row without keys)
     if (d < p.D) p.o[b * p.o_sb + (head0 + g) * p.o_sh + d] = float_to_h16(ls == 0.f ? 0.f : acc / ls);
-    if (d == 0) p.lse[(static_cast<long long>(b) * p.H + head0 + g) * 128] = ls > 0.f ? mn + log2f(ls) : -INFINITY;
+    if (d == 0) p.lse[(static_cast<long long>(b) * p.H + head0 + g) * 128] = ls > 0.f ? mn + log2f(ls) : LSE_NONE;
   }
   for (int i = split * DEC_THREADS + threadIdx.x; i < GT * 128; i += nsplit * DEC_THREADS)
     if (i % 128 != 0) p.lse[(static_cast<long long>(b) * p.H + head0 + i / 128) * 128 + i % 128] = INFINITY;

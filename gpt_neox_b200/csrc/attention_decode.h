@@ -5,6 +5,11 @@
 
 namespace nx {
 
+// The log-sum-exp of a row without a usable sum (no visible key, or a NaN among its scores).  Finite and below every
+// score: the backward forms exp2(score - lse) with masked scores of -inf, which -inf here would turn into NaN, so that a NaN
+// row would reach the gradients of keys it does not see; an unmasked score still gives +inf or NaN.
+constexpr float LSE_NONE = -3.0e38f;
+
 struct AttnDecodeParams {
   const h16 *q, *k, *v;
   h16* o;

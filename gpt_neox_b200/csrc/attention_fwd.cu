@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(att_threads(HALVES), BN == 64 ? 2 : 1)
       if (half == 0) {
         // base-2 log-sum-exp of the scaled scores; rows are padded to a multiple of 128 with +inf (the backward reads
         // whole 128-row blocks: +inf makes the padding contribute zero probability)
-        const float lse2 = !row_ok ? INFINITY : l > 0.f ? m_used + log2f(l) : -INFINITY;
+        const float lse2 = !row_ok ? INFINITY : l > 0.f ? m_used + log2f(l) : LSE_NONE;
         p.lse[(static_cast<long long>(batch) * p.H + head) * p.Sq_pad + qi] = lse2;
       }
     }

@@ -683,3 +683,32 @@ def test_branch_sum_rounds_once(rows, H, ba, bm):
     got = branch_sum(x, a, b1, m, b2)
     p, q = (t.float() if b is None else t.float() + b.float() for t, b in ((a, b1), (m, b2)))
     assert torch.equal(got, (x.float() + p + q).to(DT))
+
+
+@pytest.mark.parametrize("s,at,d,window", [(256, 40, 128, -1), (200, 130, 64, -1), (300, 290, 128, 100), (130, 0, 64, -1)])
+def test_a_nan_row_leaves_the_values_it_does_not_see_alone(s, at, d, window):
+    """A query row of NaN: the gradients of the values it attends to are NaN, those of the keys that the causal mask, the
+    window or the end of the sequence hides from it are what they are without that row (its probabilities there are 0)."""
+    from gpt_neox_b200.ops.attention import flash_attention
+    torch.manual_seed(24)
+    q, k, v, g = bf(1, s, 2, d), bf(1, s, 2, d, grad=True), bf(1, s, 2, d, grad=True), bf(1, s, 2, d)
+    q[0, at, 1] = math.nan
+    (dv,) = torch.autograd.grad(flash_attention(q, k, v, window=window), [v], g)
+    pos = torch.arange(s, device=DEV)
+    seen = (pos <= at) & (pos >= (at - window if window >= 0 else 0))
+    assert dv[0, seen, 1].isnan().all() and dv[0, ~seen, 1].isfinite().all() and dv[0, :, 0].isfinite().all()
+
+
+@pytest.mark.parametrize("sq,sk,scale", [(200, 70, None), (129, 1, None), (140, 140, 0.0), (130, 200, -0.02)])
+def test_attention_gradients_of_rows_without_keys_and_odd_scales(sq, sk, scale):
+    """More queries than keys (the first rows see none), scale 0 and a negative one."""
+    from gpt_neox_b200.ops.attention import attention_reference, flash_attention
+    torch.manual_seed(25)
+    ts = [bf(2, n, 3, 64, grad=True) for n in (sq, sk, sk)]
+    ref = [t.detach().double().requires_grad_(True) for t in ts]
+    g = bf(2, sq, 3, 64)
+    live = slice(max(0, sq - sk), sq)
+    y, r = flash_attention(*ts, scale=scale), attention_reference(ref[0][:, live], *ref[1:], scale=scale)[0]
+    assert not y[:, :live.start].any() and rel(y[:, live], r) < 2e-2
+    for a, b in zip(torch.autograd.grad(y, ts, g), torch.autograd.grad(r, ref, g[:, live].to(r.dtype))):
+        assert (a.float() - b.float()).abs().max() <= 2e-2 * b.float().abs().max() + 1e-6
