@@ -43,7 +43,7 @@ struct WkvParams {
   const float* u;                   // [H, N]
   h16 *y, *o_gr, *o_gk, *o_gv, *o_gw;   // (osb, ost)
   float* gr32;                      // (osb, ost)
-  float* gu;                        // [H, N], zeroed by the caller
+  float* gu_part;                   // [B, NC, H, N]: the gradient of u by sequence and chunk
   long long osb, ost;
   float* local;                     // [B, H, NC, N, N] chunk-local end states
   const float* start;               // [B, H, NC, N, N] start states of this sweep; null = zero (one chunk)
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(2 * N) wkv_kernel(const WkvParams p) {
       }
     if (!second) p.sumew[base * N + me] = sew;
   }
-  if (MODE == WK_G && !second) atomicAdd(p.gu + h * N + me, gu);
+  if (MODE == WK_G && !second) p.gu_part[(((long long)bi * p.NC + c) * p.H + h) * N + me] = gu;
 }
 
 // start[c] for every chunk: forward  start[0] = 0, start[c+1] = P_c start[c] + local[c];
@@ -328,6 +328,25 @@ __global__ void __launch_bounds__(N) wkv_fold_kernel(const float* local, const f
     const long long o = ((head * NC + c) * N + i) * N + j;
     start[o] = S;
     if (q + 1 < NC) S = S * __expf(sumew[(head * NC + c) * N + i]) + local[o];
+  }
+}
+
+// gu[i] = sum of the parts, in an order of its own (no atomics: a backward repeats bit for bit).
+constexpr int WK_SUM_X = 32, WK_SUM_Y = 16;
+__global__ void __launch_bounds__(WK_SUM_X * WK_SUM_Y) wkv_sum_kernel(const float* part, float* gu, int parts, int n) {
+  __shared__ float s[WK_SUM_Y][WK_SUM_X];
+  const int i = blockIdx.x * WK_SUM_X + threadIdx.x;
+  float a = 0.f;
+  if (i < n) {
+#pragma unroll 4
+    for (int r = threadIdx.y; r < parts; r += WK_SUM_Y) a += part[(long long)r * n + i];
+  }
+  s[threadIdx.y][threadIdx.x] = a;
+  __syncthreads();
+  if (threadIdx.y == 0 && i < n) {
+#pragma unroll
+    for (int y = 1; y < WK_SUM_Y; ++y) a += s[y][threadIdx.x];
+    gu[i] = a;
   }
 }
 
@@ -388,7 +407,7 @@ static int wkv_forward(WkvParams p, float* start, cudaStream_t stream) {
 }
 
 template <int N>
-static int wkv_backward(WkvParams p, const float* fstart, float* rstart, cudaStream_t stream) {
+static int wkv_backward(WkvParams p, const float* fstart, float* rstart, float* gu, cudaStream_t stream) {
   const bool vec = wkv_vec_ok(p);
   p.start = p.NC > 1 ? fstart : nullptr;
   int rc = wkv_launch<N, WK_GR>(p, vec, p.NC, stream);
@@ -402,7 +421,12 @@ static int wkv_backward(WkvParams p, const float* fstart, float* rstart, cudaStr
     p.start = rstart;
     p.fstart = fstart;
   }
-  return wkv_launch<N, WK_G>(p, vec, p.NC, stream);
+  rc = wkv_launch<N, WK_G>(p, vec, p.NC, stream);
+  if (rc != NX_OK) return rc;
+  wkv_sum_kernel<<<(p.H * N + WK_SUM_X - 1) / WK_SUM_X, dim3(WK_SUM_X, WK_SUM_Y), 0, stream>>>(p.gu_part, gu, p.B * p.NC,
+                                                                                          p.H * N);
+  NX_LAUNCH_CHECK();
+  return NX_OK;
 }
 
 NX_API int NX_SYM(nx_wkv6_chunks)(int B, int T, int H) { return wkv_chunk_count(B, T, H); }
@@ -424,11 +448,12 @@ NX_API int NX_SYM(nx_wkv6_fwd)(const void* r, const void* k, const void* v, cons
   return N == 64 ? wkv_forward<64>(p, (float*)start, stream) : wkv_forward<32>(p, (float*)start, stream);
 }
 
-// gy like r.  gr / gk / gv / gw: bf16 by (osb, ost); gr32: fp32 scratch of the same shape and strides; gu fp32 [H, N],
-// zeroed by the caller.  fstart: the forward's start states; local, rstart, sumew: scratch (all null for NC = 1).
+// gy like r.  gr / gk / gv / gw: bf16 by (osb, ost); gr32: fp32 scratch of the same shape and strides; gu fp32 [H, N];
+// gu_part: fp32 scratch [B, NC, H, N].  fstart: the forward's start states; local, rstart, sumew: scratch (all null for
+// NC = 1).
 NX_API int NX_SYM(nx_wkv6_bwd)(const void* r, const void* k, const void* v, const void* w, const void* gy, long long sb,
                        long long st, const void* u, void* gr, void* gk, void* gv, void* gw, void* gr32, void* gu,
-                       long long osb, long long ost, void* local, const void* fstart, void* rstart, void* sumew,
+                       void* gu_part, long long osb, long long ost, void* local, const void* fstart, void* rstart, void* sumew,
                        int B, int T, int H, int N, cudaStream_t stream) {
   NX_REQUIRE(N == 64 || N == 32, "wkv6: head size %d not supported (32 or 64)", N);
   if (B <= 0 || T <= 0 || H <= 0) return NX_OK;
@@ -436,11 +461,11 @@ NX_API int NX_SYM(nx_wkv6_bwd)(const void* r, const void* k, const void* v, cons
   p.r = (const h16*)r; p.k = (const h16*)k; p.v = (const h16*)v; p.w = (const h16*)w; p.gy = (const h16*)gy;
   p.sb = sb; p.st = st; p.u = (const float*)u;
   p.o_gr = (h16*)gr; p.o_gk = (h16*)gk; p.o_gv = (h16*)gv; p.o_gw = (h16*)gw;
-  p.gr32 = (float*)gr32; p.gu = (float*)gu; p.osb = osb; p.ost = ost;
+  p.gr32 = (float*)gr32; p.gu_part = (float*)gu_part; p.osb = osb; p.ost = ost;
   p.local = (float*)local; p.sumew = (float*)sumew;
   p.B = B; p.T = T; p.H = H; p.NC = wkv_chunk_count(B, T, H); p.clen = wkv_chunk_len(T, p.NC);
-  return N == 64 ? wkv_backward<64>(p, (const float*)fstart, (float*)rstart, stream)
-                 : wkv_backward<32>(p, (const float*)fstart, (float*)rstart, stream);
+  return N == 64 ? wkv_backward<64>(p, (const float*)fstart, (float*)rstart, (float*)gu, stream)
+                 : wkv_backward<32>(p, (const float*)fstart, (float*)rstart, (float*)gu, stream);
 }
 
 }  // namespace nx

@@ -110,7 +110,7 @@ def _declare(lib):
                                   P, P, P, P, P, P, P, I, I, I, P])
     sig("nx_wkv6_chunks", [I, I, I])
     sig("nx_wkv6_fwd", [P, P, P, P, L, L, P, P, L, L, P, P, P, I, I, I, I, P])
-    sig("nx_wkv6_bwd", [P, P, P, P, P, L, L, P, P, P, P, P, P, P, L, L, P, P, P, P, I, I, I, I, P])
+    sig("nx_wkv6_bwd", [P, P, P, P, P, L, L, P, P, P, P, P, P, P, P, L, L, P, P, P, P, I, I, I, I, P])
     sig("nx_gemm_fp8", [P, P, P, I, I, I, L, L, L, I, I, P, P, I, I, P])
     sig("nx_fp8_quantize", [P, L, P, P, L, P, L, P, I, I, I, P])
     sig("nx_gemm_mxfp8", [P, P, P, I, I, I, L, L, L, P, P, L, L, I, I, P, P, I, I, I, P])

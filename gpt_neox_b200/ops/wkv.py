@@ -95,16 +95,19 @@ class _WkvFn(torch.autograd.Function):
         dev = r.device
         gr, gk, gv, gw = (torch.empty((T, B, C), device=dev, dtype=r.dtype).transpose(0, 1) for _ in range(4))
         gr32 = torch.empty((T, B, C), device=dev, dtype=torch.float32).transpose(0, 1)
-        gu = torch.zeros((H, N), device=dev, dtype=torch.float32)
+        if B * T == 0:
+            return gr, gk, gv, gw, torch.zeros((H, N), device=dev, dtype=ctx.u_dtype)
+        gu = torch.empty((H, N), device=dev, dtype=torch.float32)
+        gu_part = torch.empty((B, 1 if start is None else start.shape[2], H, N), device=dev, dtype=torch.float32)
         local = rstart = sumew = None
         if start is not None:
             local, rstart = torch.empty_like(start), torch.empty_like(start)
             sumew = torch.empty(start.shape[:4], device=dev, dtype=torch.float32)
-        LAUNCHES["n"] += 2 if start is None else 4
+        LAUNCHES["n"] += 3 if start is None else 5
         _lib.check(_lib.lib(r).nx_wkv6_bwd(
             _lib.ptr(r), _lib.ptr(k), _lib.ptr(v), _lib.ptr(w), _lib.ptr(gy), r.stride(0), r.stride(1), _lib.ptr(u32),
-            _lib.ptr(gr), _lib.ptr(gk), _lib.ptr(gv), _lib.ptr(gw), _lib.ptr(gr32), _lib.ptr(gu), gr.stride(0),
-            gr.stride(1), _lib.ptr(local), _lib.ptr(start), _lib.ptr(rstart), _lib.ptr(sumew), B, T, H, N,
+            _lib.ptr(gr), _lib.ptr(gk), _lib.ptr(gv), _lib.ptr(gw), _lib.ptr(gr32), _lib.ptr(gu), _lib.ptr(gu_part),
+            gr.stride(0), gr.stride(1), _lib.ptr(local), _lib.ptr(start), _lib.ptr(rstart), _lib.ptr(sumew), B, T, H, N,
             _lib.stream()), "nx_wkv6_bwd")
         return gr, gk, gv, gw, gu.to(ctx.u_dtype)
 

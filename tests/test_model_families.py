@@ -108,3 +108,23 @@ def test_wkv6_chunks_and_layouts(B, T, H, N, pad, dtype):
     eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -11
     for a, r in zip((y,) + got, [yr] + want):                   # one rounding to 16 bits; fp32 sums on both sides
         assert (a.float() - r).abs().max().item() <= 2 * eps * r.abs().max().item() + 1e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,T,H,N", [(96, 40, 2, 64), (1, 900, 2, 64), (3, 400, 1, 32)])
+def test_wkv6_gradients_repeat_bit_for_bit(B, T, H, N):
+    """Many sequences, and one cut into many chunks: the gradient of u is a sum over both, in a fixed order."""
+    from gpt_neox_b200.ops.wkv import wkv6, wkv6_reference
+    torch.manual_seed(9)
+    mk = lambda m=0.0: (torch.randn(B, T, H * N, device="cuda") * 0.5 + m).bfloat16().requires_grad_(True)
+    leaves = [mk(), mk(), mk(), mk(-1.5), (torch.randn(H, N, device="cuda") * 0.3).requires_grad_(True)]
+    g = torch.randn(B, T, H * N, device="cuda").bfloat16()
+    runs = [torch.autograd.grad(wkv6(*leaves), leaves, g) for _ in range(8)]
+    for r in runs[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(runs[0], r))
+    ref = [t.detach().double().requires_grad_(True) for t in leaves]
+    r, k, v, w, u = ref
+    s = (g.double() * v).view(B, T, H, N).sum(-1, keepdim=True)
+    want = ((r * k).view(B, T, H, N) * s).sum((0, 1))
+    err = (runs[0][4].double() - want).norm() / want.norm()
+    assert err < 1e-5, err.item()                  # fp32 sums of B * T products of 16-bit inputs
