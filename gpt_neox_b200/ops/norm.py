@@ -101,12 +101,14 @@ class _NormFn(torch.autograd.Function):
             ws = torch.empty(blocks * (4 if both else 2) * H, device=x2.device, dtype=torch.float32)
             dx = torch.empty_like(x2)
             # parameter gradients: straight into the fp32 main_grad buffers (added by the partial-sum reduction
-            # kernel) when every parameter of this call has one, else into fresh buffers: of the parameters' own type
-            # when autograd takes them as they are, fp32 when some main_grad of another kind has to be added to
+            # kernel) when every parameter of this call has one of its own (the kernel's blocks add to them without
+            # atomics: a parameter that both norms use must not be added to twice at once), else into fresh buffers: of
+            # the parameters' own type when autograd takes them as they are, fp32 when some main_grad has to be added to
             need = ctx.needs_input_grad
             want = [i + j for i in norms for j in (0, 1) if ctx.params[i + j] is not None and need[(2, 3, 5, 6)[i + j]]]
             mgs = [getattr(ctx.params[i], "main_grad", None) for i in want]
-            direct = all(m is not None and m.dtype == torch.float32 and m.is_contiguous() and m.numel() == H for m in mgs)
+            direct = all(m is not None and m.dtype == torch.float32 and m.is_contiguous() and m.numel() == H for m in mgs) \
+                and len({m.data_ptr() for m in mgs}) == len(mgs)
             out16 = not direct and all(m is None and ctx.params[i].dtype == x2.dtype for i, m in zip(want, mgs))
             out = [None] * 4
             for i, m in zip(want, mgs):

@@ -632,6 +632,25 @@ def test_norm_parameter_shared_by_both_norms_and_frozen_parameters():
     assert rel(dx, rx) < 2e-2 and rel(dw, rw) < 2e-2
 
 
+def test_norm_parameter_shared_by_both_norms_adds_to_its_main_grad_twice():
+    """Both norms' sums have to arrive in one fp32 buffer, for the weight and for the bias."""
+    from gpt_neox_b200.ops.norm import dual_layer_norm
+    torch.manual_seed(6)
+    H = 2048
+    x, w, b = bf(300, H, grad=True), bf(H, grad=True), bf(H, grad=True)
+    for p in (w, b):
+        p.main_grad = torch.zeros(H, device=DEV)
+    g1, g2 = bf(300, H), bf(300, H)
+    xr, wr, br = (t.detach().double().requires_grad_(True) for t in (x, w, b))
+    yr = F.layer_norm(xr, (H,), wr, br, 1e-5)
+    want = torch.autograd.grad([yr, yr], [wr, br], [g1.double(), g2.double()])
+    for n in range(1, 4):
+        torch.autograd.backward(dual_layer_norm(x, w, b, w, b), [g1, g2])
+        assert w.grad is None and b.grad is None
+        for p, r in zip((w, b), want):
+            assert ((p.main_grad - n * r).abs().max() / (n * r).abs().max()).item() < 1e-4
+
+
 @pytest.mark.parametrize("b,h,hk,sk,d,window,alibi", [
     (1, 1, 1, 1, 128, -1, False), (2, 4, 4, 127, 64, -1, False), (3, 12, 3, 129, 64, -1, True),
     (1, 32, 4, 2049, 128, -1, False), (2, 6, 2, 1000, 40, 700, False), (8, 32, 32, 777, 128, -1, False),
