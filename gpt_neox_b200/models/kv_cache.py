@@ -41,10 +41,14 @@ def extend(layer, past, rows: int, like: torch.Tensor, shape=None) -> torch.Tens
     gives (b, heads, hn)."""
     n = 0 if past is None else past.shape[1] if torch.is_tensor(past) else past[0].shape[0]
     shape = tuple(like.shape[1:]) if shape is None else shape
+    if n and any(tuple(t.shape) != (n,) + shape for t in (past[0], past[1])):
+        # (a copy would broadcast the cache of another batch or head count)
+        raise RuntimeError("kv_cache: the cache holds keys %s and values %s, this step appends rows of %s"
+                           % (tuple(past[0].shape), tuple(past[1].shape), shape))
     stream, total = _stream(like), n + rows
     buf = None
     if torch.is_tensor(past) and past.dtype == like.dtype and past.device == like.device \
-            and tuple(past.shape[2:]) == shape and _claim(layer, past, stream):
+            and _claim(layer, past, stream):
         room = past.stride(0) // past.stride(1)
         if total <= room:
             buf = past.as_strided((2, room) + shape, past.stride())

@@ -490,3 +490,23 @@ def test_a_replaced_forward_is_called_while_generating(name, where, monkeypatch)
         model.clear_cache()
         got = model((tokens, pos, None))
     assert any(c is target for c in calls) and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("past,shape", [((2, 3, 1, 2, 4), (4, 2, 4)), ((2, 3, 4, 1, 4), (4, 2, 4)), ((2, 3, 4, 2, 1), (4, 2, 4)),
+                                        ((2, 3, 4, 2, 8), (4, 2, 4)), ((2, 3, 2, 4), (4, 2, 4))])
+def test_a_cache_of_another_shape_is_refused(past, shape):
+    """As concatenating it was: no broadcast of a stale cache over this step's batch or heads."""
+    import torch
+    from gpt_neox_b200.models import kv_cache
+
+    class Layer:
+        pass
+    for p in (torch.zeros(past), tuple(torch.zeros(past))):
+        with pytest.raises(RuntimeError):
+            kv_cache.extend(Layer(), p, 1, torch.zeros((1,) + shape))
+    with pytest.raises(RuntimeError):                       # keys and values of different lengths
+        kv_cache.extend(Layer(), (torch.zeros((3,) + shape), torch.zeros((2,) + shape)), 1, torch.zeros((1,) + shape))
+    layer = Layer()                                         # and the layer's own last cache, after the batch has changed
+    last = kv_cache.extend(layer, None, 2, torch.zeros((1,) + shape))
+    with pytest.raises(RuntimeError):
+        kv_cache.extend(layer, last, 1, torch.zeros((1, 1) + shape[1:]))
