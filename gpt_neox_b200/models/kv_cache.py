@@ -6,7 +6,8 @@ whole cache (concatenating k and v and stacking them moves every cached byte twi
 
 Only the tensor that the layer returned last, unchanged in length and on the same stream, is extended in place; an older
 one (a second continuation of the same prefix), another layer's or a caller's own is copied into a buffer of its own, so
-no ``present`` ever sees rows that were appended to another.
+no ``present`` ever sees rows that were appended to another.  So is one that was returned in inference mode once that
+mode has ended: its memory may not be written any more.
 """
 from __future__ import annotations
 
@@ -31,6 +32,8 @@ def _claim(layer, past, stream) -> bool:
         ref, st = _LAST.get(layer, (None, None))
         if ref is None or ref() is not past or st != stream:
             return False
+        if past.is_inference() and not torch.is_inference_mode_enabled():
+            return False                # its buffer may not be written outside inference mode
         del _LAST[layer]
         return True
 

@@ -510,3 +510,27 @@ def test_a_cache_of_another_shape_is_refused(past, shape):
     last = kv_cache.extend(layer, None, 2, torch.zeros((1,) + shape))
     with pytest.raises(RuntimeError):
         kv_cache.extend(layer, last, 1, torch.zeros((1, 1) + shape[1:]))
+
+
+def test_a_cache_of_inference_mode_is_continued_outside_it():
+    import torch
+    from gpt_neox_b200.models import kv_cache
+
+    class Layer:
+        pass
+    torch.manual_seed(1)
+    layer, rows = Layer(), [torch.randn(2, n, 2, 3, 4) for n in (3, 1, 1, 1)]
+
+    def step(past, new):
+        got = kv_cache.extend(layer, past, new.shape[1], new[0])
+        got[:, got.shape[1] - new.shape[1]:].copy_(new)
+        return got
+    with torch.inference_mode():
+        first = step(None, rows[0])
+    with torch.no_grad():
+        second = step(first, rows[1])
+    with torch.inference_mode():
+        third = step(second, rows[2])
+    with torch.no_grad():
+        last = step(third, rows[3])
+    assert torch.equal(last, torch.cat(rows, 1)) and torch.equal(first, rows[0]) and torch.equal(third, torch.cat(rows[:3], 1))
