@@ -7,7 +7,12 @@ whole cache (concatenating k and v and stacking them moves every cached byte twi
 Only the tensor that the layer returned last, unchanged in length and on the same stream, is extended in place; an older
 one (a second continuation of the same prefix), another layer's or a caller's own is copied into a buffer of its own, so
 no ``present`` ever sees rows that were appended to another.  So is one that was returned in inference mode once that
-mode has ended: its memory may not be written any more.
+mode has ended: its memory may not be written any more.  Nothing is grown in place while a graph is captured, and
+nothing that a captured step returned is (on the stream of the steps around it, where the stream would not tell them
+apart): every replay writes that step's rows again.
+
+A grown cache shares its front with the shorter one it came from, and its storage holds room for more rows: clone a cache
+to change or to save it by itself.
 """
 from __future__ import annotations
 
@@ -23,7 +28,7 @@ _MIN_ROOM = 256
 
 
 def _stream(t):
-    return torch.cuda.current_stream(t.device).cuda_stream if t.is_cuda else 0
+    return torch._C._cuda_getCurrentRawStream(t.get_device()) if t.is_cuda else 0
 
 
 def _claim(layer, past, stream) -> bool:
@@ -44,23 +49,25 @@ def extend(layer, past, rows: int, like: torch.Tensor, shape=None) -> torch.Tens
     gives (b, heads, hn)."""
     n = 0 if past is None else past.shape[1] if torch.is_tensor(past) else past[0].shape[0]
     shape = tuple(like.shape[1:]) if shape is None else shape
-    if n and any(tuple(t.shape) != (n,) + shape for t in (past[0], past[1])):
-        # (a copy would broadcast the cache of another batch or head count)
-        raise RuntimeError("kv_cache: the cache holds keys %s and values %s, this step appends rows of %s"
-                           % (tuple(past[0].shape), tuple(past[1].shape), shape))
     stream, total = _stream(like), n + rows
     buf = None
-    if torch.is_tensor(past) and past.dtype == like.dtype and past.device == like.device \
-            and _claim(layer, past, stream):
+    capturing = like.is_cuda and torch.cuda.is_current_stream_capturing()
+    if torch.is_tensor(past) and past.dtype == like.dtype and past.device == like.device and not capturing \
+            and past.shape[2:] == shape and _claim(layer, past, stream):
         room = past.stride(0) // past.stride(1)
         if total <= room:
             buf = past.as_strided((2, room) + shape, past.stride())
     if buf is None:
+        if n and not (past[0].shape == past[1].shape == (n,) + shape):
+            # (the copies would broadcast the cache of another batch or head count)
+            raise RuntimeError("kv_cache: the cache holds keys %s and values %s, this step appends rows of %s"
+                               % (tuple(past[0].shape), tuple(past[1].shape), shape))
         buf = torch.empty((2, total + max(_MIN_ROOM, total // 4)) + shape, device=like.device, dtype=like.dtype)
         if n:
             buf[0, :n].copy_(past[0])
             buf[1, :n].copy_(past[1])
     present = buf[:, :total]
-    with _LOCK:
-        _LAST[layer] = (weakref.ref(present), stream)
+    if not capturing:
+        with _LOCK:
+            _LAST[layer] = (weakref.ref(present), stream)
     return present

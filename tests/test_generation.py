@@ -534,3 +534,36 @@ def test_a_cache_of_inference_mode_is_continued_outside_it():
     with torch.no_grad():
         last = step(third, rows[3])
     assert torch.equal(last, torch.cat(rows, 1)) and torch.equal(first, rows[0]) and torch.equal(third, torch.cat(rows[:3], 1))
+
+
+@pytest.mark.gpu
+def test_a_captured_step_does_not_share_its_cache_with_what_follows():
+    """A step captured in a graph on the stream of the eager ones: an eager continuation of its cache, and the cache it started from, keep their rows when
+    the graph is replayed on other inputs."""
+    import torch
+    from gpt_neox_b200.models import kv_cache
+
+    class Layer:
+        pass
+    layer, like = Layer(), torch.zeros(1, 2, 3, 8, device="cuda")
+
+    def step(past, value):
+        got = kv_cache.extend(layer, past, 1, like)
+        got[:, got.shape[1] - 1:].copy_(value)
+        return got
+    value = torch.full((), 2.0, device="cuda")
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        first = step(None, torch.ones((), device="cuda"))
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            captured = step(first, value)
+        graph.replay()
+        after = step(captured, torch.full((), 3.0, device="cuda"))
+        branch = step(first, torch.full((), 4.0, device="cuda"))
+        value.fill_(9.0)
+        graph.replay()
+    torch.cuda.synchronize()
+    for got, want in ((first, [1]), (captured, [1, 9]), (after, [1, 2, 3]), (branch, [1, 4])):
+        assert got[0, :, 0, 0, 0].tolist() == want and got.shape[1] == len(want)
