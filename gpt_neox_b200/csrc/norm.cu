@@ -113,17 +113,19 @@ __global__ void norm_fwd_kernel(const h16* __restrict__ x,
   }
 }
 
-// One warp per row, the row held as 16-byte vectors in registers (NV per lane, H <= 256 NV): no block barrier, and 48
-// to 64 rows in flight per SM where the block-per-row form waits at four barriers for each.  One norm of 8192 x 2048 from
-// DRAM, with its launch: 56.2 us with a block per row, 52.7 us; two norms of rows that are in L2: 22.7 and 23.9 us.
-constexpr int WARP_ROW_MAX_NV = 8;
+// One warp per row, the row held as 16-byte vectors in registers (NV per lane, H <= 256 NV): no block barrier, and 32
+// rows in flight per SM (48 - 63 registers, four blocks of eight) where the block-per-row form waits at four barriers for
+// each.  Bound by the latency of one row's chain for few rows, by DRAM for many.  us with a block / with a warp per row,
+// from DRAM: two norms of 8192 x 512 10.2 / 7.0, 8192 x 768 13.1 / 9.1, one RMS norm of 8192 x 768 8.8 / 6.8; of 16 x 768
+// 2.17 / 2.12.
+constexpr int WARP_ROW_MAX_NV = 3;
 template <bool RMS, int NV>
-__global__ void __launch_bounds__(256, NV <= 4 ? 4 : 3)
+__global__ void __launch_bounds__(256, 4)
 norm_fwd_warp_kernel(const h16* __restrict__ x, const h16* __restrict__ g1, const h16* __restrict__ b1,
                      h16* __restrict__ y1, const h16* __restrict__ g2, const h16* __restrict__ b2,
                      h16* __restrict__ y2, float* __restrict__ mean_out, float* __restrict__ rstd_out, long long rows,
                      int H, float eps) {
-  const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  const long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31, nv = H >> 3;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * H);
@@ -608,19 +610,22 @@ NX_API int NX_SYM(nx_norm_fwd)(int kind, const void* x, const void* g1, const vo
   auto s = static_cast<cudaStream_t>(stream_);
   const int t = threads_for(H);
   using bf = h16;
-  // one warp per row up to H = 2048; beyond that a lane's share of the row costs so many registers that fewer rows are in
-  // flight than with a block per row
+  // One warp per row up to H = 768: at every number of rows it is the faster one or within 0.1 us (an RMS norm of 160 x 512:
+  // 1.99 us with a block, 2.09 with a warp).  Wider rows lose it where few rows leave nothing but one lane's longer chain:
+  // two norms, block / warp, 16 x 1024 2.66 / 3.11, 16 x 2048 3.39 / 5.01, 8192 x 2048 20.1 / 21.5 us (8192 x 1024 would
+  // gain, 13.6 / 11.0, but a rule on the number of rows would make a row's bits depend on the batch).  Blocks of fewer
+  // warps while they still find an SM each: 16 x 768 2.40 us with eight rows in a block, 2.12 with one.
   if (H <= 256 * WARP_ROW_MAX_NV) {
     const int nvl = (H / 8 + 31) / 32;
-    const unsigned grid = static_cast<unsigned>((rows + 7) / 8);
+    const int wpb = rows >= 8ll * sm_count() ? 8 : rows >= 2ll * sm_count() ? 2 : 1;
+    const unsigned grid = static_cast<unsigned>((rows + wpb - 1) / wpb);
 #define NX_NORM_WARP(R, NV)                                                                                        \
-  norm_fwd_warp_kernel<R, NV><<<grid, 256, 0, s>>>((const bf*)x, (const bf*)g1, (const bf*)b1, (bf*)y1, (const bf*)g2, \
+  norm_fwd_warp_kernel<R, NV><<<grid, wpb * 32, 0, s>>>((const bf*)x, (const bf*)g1, (const bf*)b1, (bf*)y1, (const bf*)g2, \
                                                   (const bf*)b2, (bf*)y2, (float*)mean, (float*)rstd, rows, H, eps)
 #define NX_NORM_WARP_NV(R)                \
   do {                                    \
     if (nvl <= 2) NX_NORM_WARP(R, 2);     \
-    else if (nvl <= 4) NX_NORM_WARP(R, 4); \
-    else NX_NORM_WARP(R, 8);              \
+    else NX_NORM_WARP(R, 3);              \
   } while (0)
     if (kind == 0) NX_NORM_WARP_NV(false);
     else NX_NORM_WARP_NV(true);

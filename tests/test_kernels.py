@@ -593,7 +593,8 @@ def test_rotate_qk_out_of_place_leaves_the_projection_alone(hn, rot, np_, kvp):
     assert torch.equal(cache[0], apply_rotary(k, cos, sin, rot, 7)) and torch.equal(cache[1], v)
 
 
-@pytest.mark.parametrize("rows,H", [(1, 8), (9, 248), (17, 264), (1001, 1032), (8, 2048), (601, 2048), (3, 2056)])
+@pytest.mark.parametrize("rows,H", [(1, 8), (9, 248), (17, 264), (1001, 1032), (8, 2048), (601, 2048), (3, 2056), (33, 512),
+                                    (1001, 520), (300, 768), (5, 776)])
 @pytest.mark.parametrize("form", ["dual", "layer", "rms"])
 def test_norm_row_sizes(rows, H, form):
     """Row lengths around what a lane, a warp and the warp-per-row form take; every gradient in the parameters' type."""
