@@ -201,15 +201,62 @@ __global__ void __launch_bounds__(DEC_THREADS, dec_ctas(GT)) attn_decode_kernel(
   cluster.sync();     // nobody leaves while its shared memory may still be read
 }
 
+static int ceil_div(int a, int b) { return (a + b - 1) / b; }
+// splits that leave at least 64 keys to each, below which the merge costs more than the shorter loop saves
+static int max_splits(int keys) {
+  const int n = ceil_div(keys, 64);
+  return n < DEC_MAX_SPLITS ? n : DEC_MAX_SPLITS;
+}
+
+// Clusters of 1 .. 8 CTAs that are resident at once.  Fewer than CTAs / size: a cluster lies within one group of SMs.
+template <int DP, int GT>
+struct ClusterSlots {
+  int n[DEC_MAX_SPLITS + 1];
+  ClusterSlots() {
+    for (int s = 1; s <= DEC_MAX_SPLITS; ++s) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(s);
+      cfg.blockDim = dim3(DEC_THREADS);
+      cudaLaunchAttribute attr;
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = s;
+      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&n[s], attn_decode_kernel<DP, GT>, &cfg) != cudaSuccess || n[s] < 1) {
+        (void)cudaGetLastError();
+        n[s] = dec_ctas(GT) * sm_count() / s;
+      }
+    }
+  }
+};
+
 template <int DP, int GT>
 static int launch(const AttnDecodeParams& p, cudaStream_t stream) {
   const int G = p.H / p.Hk, rows = p.Hk * (G / GT);
   const int keys = p.Sk - p.key_lo;
-  // splits: as many CTAs as are resident at once, with at least 64 keys each, below which the merge costs more than the
-  // shorter loop saves
-  const long long slots = static_cast<long long>(dec_ctas(GT)) * sm_count() / (static_cast<long long>(rows) * p.B);
-  int splits = static_cast<int>(slots < 1 ? 1 : slots > DEC_MAX_SPLITS ? DEC_MAX_SPLITS : slots);
-  if (splits > (keys + 63) / 64) splits = (keys + 63) / 64;
+  // Splits: the most whose clusters are resident at once (16 sequences, 24 heads on 3, 4096 keys in eights: 96 us with the 6
+  // splits that fit by the number of CTAs, 74 with 4).  Otherwise, where every K / V row is read once (so that DRAM is the
+  // bound) and the parts stay long, what wastes least of the last wave: two rounds of thirds instead of one round that
+  // fills half of the places (14 x 32 heads of 128, 2048 keys: 89 / 82 us; quarters up to two thirds of the places, 18 x
+  // 32, 8192 keys: 395 / 366), halves where a second wave would be nearly empty (32 x 32, 1543 keys: 154 / 137).  The number depends on the batch, and with it the order of the sums: a
+  // sequence's last bits are not those it has in another batch.
+  static const ClusterSlots<DP, GT> slots;
+  const long long clusters = static_cast<long long>(rows) * p.B;
+  auto rounds = [&](int s) { return static_cast<int>((clusters + slots.n[s] - 1) / slots.n[s]); };
+  int splits = 1;
+  for (int s = max_splits(keys); s > 1 && splits == 1; --s)
+    if (rounds(s) == 1) splits = s;
+  if (splits == 1 && GT == G) {
+    const int row = keys / (128 / DP);          // in rows of 128
+    if (rounds(1) > 1) {
+      if (5 * rounds(2) <= 8 * rounds(1) && row >= 2 * 256) splits = 2;
+    } else if (rounds(3) <= 2 && row >= 3 * 256) {
+      splits = 3;
+    } else if (3 * clusters <= 2 * slots.n[1] && row >= 4 * 1024) {
+      splits = 4;
+    }
+  }
   const int per = (keys + splits - 1) / splits;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(splits, rows, p.B);
@@ -228,9 +275,17 @@ static int launch(const AttnDecodeParams& p, cudaStream_t stream) {
 template <int DP>
 static int launch_group(const AttnDecodeParams& p, cudaStream_t stream) {
   const int G = p.H / p.Hk;
-  if (G % 8 == 0) return launch<DP, 8>(p, stream);
-  if (G % 4 == 0) return launch<DP, 4>(p, stream);
-  if (G % 2 == 0) return launch<DP, 2>(p, stream);
+  // Heads per CTA: the most whose CTAs, with all the splits that the keys allow, still fill about half of their places (a
+  // sweep of 1 - 32 sequences, 1 - 16384 keys, 1 - 32 heads on a K / V head; pairs from a quarter on).  A CTA of
+  // eight heads does eight heads' exchanges for every key, so it needs the bytes it saves to be what counts: 1 sequence, 32
+  // heads on 4, 64 keys 9.2 us with eight, 3.9 with one (5.4 with the tile kernel); 8 sequences, 16384 keys 140 us with
+  // eight, 286 with one.
+  auto fits = [&](int gt, float share) {
+    return G % gt == 0 && 1.f * p.Hk * (G / gt) * p.B * max_splits(p.Sk - p.key_lo) >= share * dec_ctas(gt) * sm_count();
+  };
+  if (fits(8, 0.5f)) return launch<DP, 8>(p, stream);
+  if (fits(4, 0.5f)) return launch<DP, 4>(p, stream);
+  if (fits(2, 0.25f)) return launch<DP, 2>(p, stream);
   return launch<DP, 1>(p, stream);
 }
 

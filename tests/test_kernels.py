@@ -732,3 +732,18 @@ def test_attention_gradients_of_rows_without_keys_and_odd_scales(sq, sk, scale):
     assert not y[:, :live.start].any() and rel(y[:, live], r) < 2e-2
     for a, b in zip(torch.autograd.grad(y, ts, g), torch.autograd.grad(r, ref, g[:, live].to(r.dtype))):
         assert (a.float() - b.float()).abs().max() <= 2e-2 * b.float().abs().max() + 1e-6
+
+
+@pytest.mark.parametrize("b,h,hk,sk,d", [(14, 32, 32, 781, 128), (18, 32, 32, 4100, 128), (33, 32, 32, 523, 128),
+                                         (1, 16, 2, 65, 128), (3, 16, 2, 129, 64), (40, 16, 2, 40, 64), (5, 24, 3, 700, 128)])
+def test_one_query_attention_splits_and_head_groups(b, h, hk, sk, d):
+    """Thirds, quarters and halves of the keys where one round of CTAs would leave places empty, and one, two, four and
+    eight heads per CTA: against the tile kernel, which computes the same row as the last of two."""
+    from gpt_neox_b200.ops.attention import _fwd
+    torch.manual_seed(26)
+    q, k, v = bf(b, 1, h, d), bf(b, sk, hk, d), bf(b, sk, hk, d)
+    one, lse = _fwd(q, k, v, d ** -0.5, False, -1, None)
+    two, lse2 = _fwd(torch.cat([q, q], 1), k, v, d ** -0.5, False, -1, None)
+    # the tile kernel rounds its probabilities to 16 bits: each output within one unit of their weighted sum
+    assert rel(one[:, 0], two[:, 1]) < (2 ** -6 if DT == torch.bfloat16 else 2 ** -9)
+    torch.testing.assert_close(lse[:, :, 0], lse2[:, :, 1], rtol=1e-4, atol=1e-4)
