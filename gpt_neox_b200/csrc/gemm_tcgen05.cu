@@ -699,17 +699,27 @@ struct CommArgs {
   bool skinny = false;   // few rows: gemm_skinny_tcgen05.cu
 };
 
-// Whether a product goes to the few-rows kernel: its layouts and epilogues, and up to 64 rows always (a generation step;
-// 4 rows of the 7B gated MLP: 164 -> 54 us for its two GEMMs), up to 128 where the tiles here would leave half the SMs
-// without one and the reduction is long enough to be split (128 rows, there / here: 4096 x 4096 36.9 / 21.5 us, 4096 x
-// 16384 110.7 / 42.0 us; 2304 x 768 16.4 / 17.3 us, at 96 rows 16.4 / 15.3 us).
+// Whether a product goes to the few-rows kernel: its layouts and epilogues, and up to 64 rows (a generation step; 4 rows of
+// the 7B gated MLP: 164 -> 54 us for its two GEMMs), up to 128 where the tiles here would leave half the SMs without one
+// and the reduction is long enough to be split in four (us, here / there, 128 rows: 4096 x 4096 30.9 / 15.2, 4096 x 16384
+// 101 / 31, 768 x 1024 12.9 / 8.3; shorter ones gain nothing from 97 rows on: 2304 x 768 12.8 / 12.6, at 96 rows 11.9 /
+// 10.1).  Except (measured over 1 - 128 rows, 8 - 65536 columns, K of 64 - 16384):
+// - one tile of a short reduction has nothing to split or to spread (128 x 512, 32 rows 6.4 / 5.3, 64 rows 6.4 / 6.7, 96 rows
+//   6.4 / 8.3; 136 x 64, 96 rows 6.4 / 7.0; 64 x 1024, 128 rows 7.0 / 7.5);
+// - with more tiles than SMs the chip is full here too, and the rows of a short reduction cost the few-rows kernel's
+//   epilogue more (50304 x 768, 48 rows 22.2 / 21.9, 64 rows 22.2 / 23.1; 65536 x 640, 64 rows 0.92 of the rate).
 static bool skinny_better(int M, int N, int K, int transA, int transB, int flags) {
   using namespace nx;
   constexpr int known = EPI_BIAS | EPI_GELU_ERF | EPI_GELU_TANH | EPI_AUX_OUT | EPI_AUX_DERIV | EPI_RESIDUAL | EPI_SCALE;
   if (transA || transB || (flags & ~known) != 0 || M > SKINNY_MAX_M) return false;
   const int BN = N <= 128 ? 128 : 256;
   const long long tiles = static_cast<long long>((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  return M <= 64 || (2 * tiles <= sm_count() && (M <= 96 || K >= 1024));
+  const bool deep = K > 960;       // sixteen 64-wide steps: four splits
+  if (N <= 128 && !deep && M > 32) return false;
+  if (N <= 64 && K < 1536 && M > 112) return false;
+  if (N <= 256 && K <= 256 && M > 80) return false;
+  if (tiles > sm_count() && K > 256 && K <= 1024 && M > 48) return false;
+  return M <= 64 || (2 * tiles <= sm_count() && (M <= 96 || deep));
 }
 
 static int gemm_common(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,

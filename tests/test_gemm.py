@@ -95,8 +95,8 @@ def test_no_device_error():
     assert _lib.read_device_error(clear=False) == 0
 
 
-@pytest.mark.parametrize("M", [1, 15, 16, 17, 33, 64, 65, 128, 129, 256])
-@pytest.mark.parametrize("N,K", [(8, 8), (136, 72), (1000, 520), (768, 3072), (4096, 4096)])
+@pytest.mark.parametrize("M", [1, 15, 16, 17, 33, 48, 49, 64, 65, 128, 129, 256])
+@pytest.mark.parametrize("N,K", [(8, 8), (128, 1016), (128, 1024), (136, 72), (1000, 520), (768, 3072), (4096, 4096)])
 def test_gemm_few_rows(M, N, K):
     """The few-rows kernel: every width of its row operand, tile remainders in N and K, one to eight splits of K; the
     epilogues a generation step and a short prompt use."""
