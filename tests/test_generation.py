@@ -337,7 +337,7 @@ def test_cached_steps_match_the_whole_prefix_on_the_gpu(over):
 @pytest.mark.parametrize("over", [dict(), dict(num_kv_heads=2, rotary_pct=1.0), dict(bias_gelu_fusion=True),
                                   dict(sliding_window_width=16), dict(use_bias_in_attn_linear=False,
                                                                       use_bias_in_mlp=False)])
-def test_a_layer_in_one_call_gives_the_bits_of_the_op_by_op_path(over, precision):
+def test_a_layer_in_one_call_gives_the_bits_of_the_op_by_op_path(over, precision, monkeypatch):
     """A hook on a submodule sends the layer down the op-by-op path; without it one native call launches the same
     kernels."""
     from test_model_gpu import _build
@@ -350,6 +350,9 @@ def test_a_layer_in_one_call_gives_the_bits_of_the_op_by_op_path(over, precision
     model.inference_mode(use_cache=True)
     tokens = torch.randint(0, 1000, (3, 330), device="cuda")
     pos = torch.arange(330, device="cuda")[None].expand(3, -1)
+    from gpt_neox_b200.models import transformer
+    native, call = [], transformer.layer_infer
+    monkeypatch.setattr(transformer, "layer_infer", lambda *a, **k: (native.append(1), call(*a, **k))[1])
 
     def steps():
         model.clear_cache()
@@ -362,13 +365,14 @@ def test_a_layer_in_one_call_gives_the_bits_of_the_op_by_op_path(over, precision
         return out + [l.layer_past.clone() for l in layers]
 
     one = steps()
+    assert len(native) == 14                            # 2 layers x 7 steps
     mlps = [m for m in model.modules() if type(m).__name__ == "ParallelMLP"]
     calls = []
     handles = [m.register_forward_hook(lambda *a: calls.append(1)) for m in mlps]
     ops = steps()
     for h in handles:
         h.remove()
-    assert len(calls) == 14 and len(one) == len(ops)
+    assert len(native) == 14 and len(calls) == 14 and len(one) == len(ops)
     assert all(torch.equal(a, b) for a, b in zip(one, ops))
 
 

@@ -747,3 +747,19 @@ def test_one_query_attention_splits_and_head_groups(b, h, hk, sk, d):
     # the tile kernel rounds its probabilities to 16 bits: each output within one unit of their weighted sum
     assert rel(one[:, 0], two[:, 1]) < (2 ** -6 if DT == torch.bfloat16 else 2 ** -9)
     torch.testing.assert_close(lse[:, :, 0], lse2[:, :, 1], rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.parametrize("H", [64, 520, 768, 2048])
+@pytest.mark.parametrize("form", ["dual", "rms"])
+def test_a_nan_stays_in_its_row_of_a_norm(H, form):
+    from gpt_neox_b200.ops.norm import dual_layer_norm, rms_norm
+    torch.manual_seed(27)
+    x, w = bf(40, H), bf(H)
+    x[7, H - 1], x[19, 0], x[20, 3] = math.nan, math.inf, -math.inf
+    ys = dual_layer_norm(x, w, w, w, w) if form == "dual" else [rms_norm(x, w, eps=1e-5)]
+    bad = torch.zeros(40, dtype=torch.bool, device=DEV)
+    bad[[7, 19, 20]] = True
+    for y in ys:
+        assert y[~bad].isfinite().all() and y[7].isnan().all()
+        # an infinite element: the mean of a LayerNorm is infinite; an RMS norm divides by infinity (0, and inf * 0 = NaN)
+        assert y[19].isnan().all() if form == "dual" else (y[19, 0].isnan() and not y[19, 1:].any())

@@ -151,3 +151,22 @@ def test_selective_scan_blocks_and_chunks(B, L, D, dtype):
         assert (a.float() - r).abs().max().item() <= 2 * eps * r.abs().max().item() + 1e-4
     with torch.no_grad():
         assert torch.equal(selective_scan(*leaves), y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what,value", [("x", float("nan")), ("dt", float("nan")), ("B", float("nan")), ("C", float("inf")),
+                                        ("z", float("nan")), ("x", float("inf"))])
+@pytest.mark.parametrize("at", [0, 37, 255, 299])
+def test_selective_scan_passes_nan_and_inf_on(what, value, at):
+    """A non-finite input in the first, a middle and the last chunk of a sequence: the outputs that are not finite are those
+    of the sequential statement (its own channel and the steps after it)."""
+    from gpt_neox_b200.ops.mamba import selective_scan, selective_scan_reference
+    torch.manual_seed(12)
+    L, D = 300, 40
+    mk = lambda *s: (torch.randn(*s, device="cuda") * 0.5).bfloat16()
+    t = dict(x=mk(2, L, D), dt=mk(2, L, D), B=mk(2, L, 16), C=mk(2, L, 16), z=mk(2, L, D))
+    t[what][1, at, 3] = value
+    A, Dp, bias = -(torch.rand(D, 16, device="cuda") + 0.5), torch.randn(D, device="cuda"), torch.zeros(D, device="cuda") - 3
+    args = lambda c: (c(t["x"]), c(t["dt"]), A, c(t["B"]), c(t["C"]), Dp, c(t["z"]), bias)
+    got, want = selective_scan(*args(lambda u: u)), selective_scan_reference(*args(lambda u: u.float()))
+    assert torch.equal(got.isfinite(), want.isfinite()) and not got.isfinite().all()

@@ -128,3 +128,20 @@ def test_wkv6_gradients_repeat_bit_for_bit(B, T, H, N):
     want = ((r * k).view(B, T, H, N) * s).sum((0, 1))
     err = (runs[0][4].double() - want).norm() / want.norm()
     assert err < 1e-5, err.item()                  # fp32 sums of B * T products of 16-bit inputs
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what,value", [(0, float("nan")), (1, float("nan")), (2, float("inf")), (3, float("nan"))])
+@pytest.mark.parametrize("at", [0, 40, 331])
+def test_wkv6_passes_nan_and_inf_on(what, value, at):
+    """A non-finite r, k, v or w in the first, a middle and the last chunk of a sequence: the outputs that are not finite are
+    those of the sequential statement."""
+    from gpt_neox_b200.ops.wkv import wkv6, wkv6_reference
+    torch.manual_seed(10)
+    T, H, N = 333, 2, 64
+    ts = [(torch.randn(2, T, H * N, device="cuda") * 0.5 - (3.0 if i == 3 else 0.0)).bfloat16() for i in range(4)]
+    ts[what][1, at, 70] = value
+    u = (torch.randn(H, N, device="cuda") * 0.3).bfloat16()
+    got, want = wkv6(*ts, u), wkv6_reference(*(t.float() for t in ts), u.float())
+    assert torch.equal(got.isfinite(), want.isfinite())
+    assert got.isfinite().all() == want.isfinite().all()
