@@ -494,8 +494,9 @@ scan_fwd_kernel(const ScanParams p) {
       *reinterpret_cast<float4*>(p.ckpt + (((long long)b * ((p.L + SC_T - 1) / SC_T) + t0 / SC_T) * p.D + d) * 16 + q * 4) =
           f4(h);
     __syncthreads();
+    const int live = t_end - t0;                  // (padded steps of the last group of four leave the state as it is)
 #pragma unroll 2
-    for (int g = 0; g < SC_T; g += 4) {
+    for (int g = 0; g < SC_T && g < live; g += 4) {
       float yp[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -680,11 +681,12 @@ scan_bwd_kernel(const ScanParams p) {
     put_bc(s.Cs, cv);
     __syncthreads();
     // the states at the starts of the quarters (read back by the thread that wrote them)
+    const int quarters = min(SC_T / SC_REG, (t_end - t0 + SC_REG - 1) / SC_REG);
     {
       float2 h[2] = {{hc.x, hc.y}, {hc.z, hc.w}};
       s.ck[0][threadIdx.x] = f4(h);
 #pragma unroll 1
-      for (int quarter = 1; quarter < SC_T / SC_REG; ++quarter) {
+      for (int quarter = 1; quarter < quarters; ++quarter) {
 #pragma unroll
         for (int k = 0; k < SC_REG; ++k) {
           const int t = (quarter - 1) * SC_REG + k;
@@ -701,7 +703,7 @@ scan_bwd_kernel(const ScanParams p) {
     }
     if (t0 - SC_T >= tc0) fetch(t0 - SC_T);       // in flight during this block
 #pragma unroll 1
-    for (int quarter = SC_T / SC_REG - 1; quarter >= 0; --quarter) {
+    for (int quarter = quarters - 1; quarter >= 0; --quarter) {
       const int tb = quarter * SC_REG;
       float2 hs[SC_REG + 1][2], as[SC_REG][2];    // hs[t + 1]: state after step t
       const float4 h0 = s.ck[quarter][threadIdx.x];
