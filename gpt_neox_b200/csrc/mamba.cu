@@ -12,7 +12,9 @@
 // state and records its end state and its sum of delta (the chunk's decay is exp(A * sum delta)), and the main pass
 // folds the earlier chunks into its start state.  The reverse recurrence of dL/dh is cut the same way.
 // The forward keeps the state at the start of every 32-step block for the backward, which recomputes 8 steps at a
-// time into registers and walks them in reverse.
+// time into registers and walks them in reverse.  Those states take 2 bytes per token and channel from the forward to the
+// backward (25 MB for 4 x 2048 x 1536, as much as one more 16-bit activation; 6 MB when a state per 128 steps was kept),
+// and the tiles' partial sums of dB and dC 4 bytes during the backward.
 // Bound by the shared-memory pipe (78-80 % busy in the main passes: a step's inputs, and the exchanges that sum dB, dC and
 // the channel sums over lanes); issue slots 42-50 %, DRAM 6-9 %.  Convolution + scan, forward + backward, 4 x
 // 2048 steps of 1536 channels: 1.78 ms with chunks of 128 steps in two passes each way, the states recomputed in three of
@@ -838,7 +840,8 @@ scan_bc_reduce_kernel(const float* __restrict__ part, int ntiles, long long rows
 
 // Chunks the sequence is cut into.  The kernels are bound by latency until an SM holds its `ctas` CTAs, so time goes with
 // the chunk length times the number of rounds the CTAs take; more than one chunk adds the light pass over all chunks but
-// one (about `light` of the main pass).
+// one (about `light` of the main pass).  The count depends on the batch and the channels, and the chunks' states are folded
+// in fp32: a sequence's last bits are not those it has in another batch.
 static int scan_chunk_count(int B, int L, int D, int ctas, float light) {
   const int tiles = (D + SC_CH - 1) / SC_CH * B, blocks = (L + SC_T - 1) / SC_T, slots = ctas * sm_count();
   int best = 1;

@@ -368,7 +368,8 @@ static int wkv_launch(const WkvParams& p, bool vec, int chunks, cudaStream_t str
 
 // Chunks the sequence is cut into.  The sweeps are bound by latency until an SM holds WK_CTAS CTAs, so time goes with the
 // chunk length times the number of rounds the CTAs take; more than one chunk adds the local pass (2 of the sweep's 3
-// operations) over all chunks but one, and the fold.
+// operations) over all chunks but one, and the fold.  The count depends on the batch, and the chunks' states are folded in
+// fp32: a sequence's last bits are not those it has in another batch.
 constexpr int WK_CTAS = 3;
 static int wkv_chunk_count(int B, int T, int H) {
   const int subs = (T + WK_SUB - 1) / WK_SUB, slots = WK_CTAS * sm_count();
