@@ -202,9 +202,17 @@ def bias_dropout_add(x, bias, residual, p: float, training: bool):
 
 
 def branch_sum(x, a, a_bias, m, m_bias):
-    """``x + (a + a_bias) + (m + m_bias)`` (biases may be None) with one rounding, without autograd: CUDA 16-bit tensors of
-    one shape."""
-    x, a, m = (t.contiguous() for t in (x, a, m))
+    """``x + (a + a_bias) + (m + m_bias)`` (biases may be None) with one rounding, without autograd.  The kernel takes CUDA
+    16-bit tensors of one type and shape; anything else (what a hook puts in a module's place) is added by PyTorch."""
+    H, mats, vecs = x.shape[-1], (x, a, m), [b for b in (a_bias, m_bias) if b is not None]
+    if not (x.is_cuda and x.dtype in _lib.H16 and H % 8 == 0 and all(t.shape == x.shape for t in mats)
+            and all(b.shape == (H,) and b.is_contiguous() for b in vecs)
+            and all(t.dtype == x.dtype and t.device == x.device for t in (a, m, *vecs))):
+        a, m = a if a_bias is None else a + a_bias, m if m_bias is None else m + m_bias
+        return x + (a + m)
+    x, a, m = (t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
+               for t in mats)
+    a_bias, m_bias = (b if b is None or b.data_ptr() % 16 == 0 else b.clone() for b in (a_bias, m_bias))
     out = torch.empty_like(x)
     LAUNCHES["n"] += 1
     _lib.check(_lib.lib(x).nx_branch_sum(_lib.ptr(x), _lib.ptr(a), _lib.ptr(a_bias), _lib.ptr(m), _lib.ptr(m_bias),

@@ -763,3 +763,20 @@ def test_a_nan_stays_in_its_row_of_a_norm(H, form):
         assert y[~bad].isfinite().all() and y[7].isnan().all()
         # an infinite element: the mean of a LayerNorm is infinite; an RMS norm divides by infinity (0, and inf * 0 = NaN)
         assert y[19].isnan().all() if form == "dual" else (y[19, 0].isnan() and not y[19, 1:].any())
+
+
+def test_branch_sum_of_other_types_shapes_and_alignments():
+    """What the kernel does not take goes to PyTorch: a branch of another type, one that broadcasts, one on an odd address."""
+    from gpt_neox_b200.ops.elementwise import branch_sum
+    torch.manual_seed(28)
+    x, a, m, b = bf(3, 2, 64), bf(3, 2, 64), bf(3, 2, 64), bf(64)
+    want = (x.float() + (a.float() + b.float()) + m.float())
+    odd = torch.empty(3 * 2 * 64 + 1, device=DEV, dtype=DT)[1:].view(3, 2, 64).copy_(a)
+    oddb = torch.empty(65, device=DEV, dtype=DT)[1:].copy_(b)
+    assert torch.equal(branch_sum(x, odd, oddb, m.transpose(0, 1).contiguous().transpose(0, 1), None), want.to(DT))
+    wide = branch_sum(x, a.float(), b, m, None)
+    assert wide.dtype == torch.float32 and rel(wide, want) < 1e-2
+    none = torch.zeros((), device=DEV, dtype=DT)
+    assert rel(branch_sum(x, a, b, none, None), want - m.float()) < 1e-2
+    cpu = branch_sum(*(t.cpu() for t in (x, a, b, m)), None)
+    assert rel(cpu.to(DEV), want) < 2e-2
