@@ -473,12 +473,12 @@ class ParallelTransformerLayer(nn.Module):
             return None
         hn = a.hidden_size_per_attention_head
         linears = (a.query_key_value, a.dense, m.linear1, m.linear2)
-        if hn % 8 or hn > 128 or a.rotary_dim % 16 or any(
-                l.use_mup or getattr(l, "use_fp8", False) or getattr(l, "gather_output", False) for l in linears) \
+        if hn % 8 or hn > 128 or a.rotary_dim % 16 \
                 or not (_plain(linears[0], mpu.ColumnParallelLinear) and _plain(linears[2], mpu.ColumnParallelLinear)
                         and _plain(linears[1], mpu.RowParallelLinear) and _plain(linears[3], mpu.RowParallelLinear)
                         and _plain(a.rotary_emb, RotaryEmbedding) and _plain(self.input_layernorm, LayerNorm)
                         and _plain(self.post_attention_layernorm, LayerNorm)) \
+                or any(l.use_mup or l.use_fp8 or getattr(l, "gather_output", False) for l in linears) \
                 or linears[0].skip_bias_add or torch.nn.modules.module._has_any_global_hook():
             return None
         n1, n2, up = self.input_layernorm, self.post_attention_layernorm, m.linear1.weight

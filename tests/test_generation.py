@@ -571,3 +571,34 @@ def test_a_captured_step_does_not_share_its_cache_with_what_follows():
     torch.cuda.synchronize()
     for got, want in ((first, [1]), (captured, [1, 9]), (after, [1, 2, 3]), (branch, [1, 4])):
         assert got[0, :, 0, 0, 0].tolist() == want and got.shape[1] == len(want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["query_key_value", "dense"])
+def test_a_module_in_place_of_a_linear_is_called_while_generating(name):
+    """An adapter that wraps a projection has none of the parallel linears' attributes."""
+    import torch
+    from test_model_gpu import _build
+    _, model = _build(tiny_config(num_layers=2, hidden_size=256, num_attention_heads=4, seq_length=512,
+                                  max_position_embeddings=512, synthetic_vocab_size=1000, pipe_parallel_size=0,
+                                  attention_config=[[["flash"], 2]], distributed_backend="nccl", precision="bfloat16"))
+    model.inference_mode(use_cache=True)
+
+    class Adapter(torch.nn.Module):
+        def __init__(self, inner):
+            super().__init__()
+            self.inner = inner
+
+        def forward(self, x):
+            calls.append(1)
+            return self.inner(x)
+    calls = []
+    tokens = torch.randint(0, 1000, (2, 20), device="cuda")
+    pos = torch.arange(20, device="cuda")[None].expand(2, -1)
+    layer = next(m for m in model.modules() if type(m).__name__.startswith("ParallelTransformerLayer"))
+    with torch.no_grad():
+        want = model((tokens, pos, None))
+        setattr(layer.attention, name, Adapter(getattr(layer.attention, name)))
+        model.clear_cache()
+        got = model((tokens, pos, None))
+    assert calls == [1] and torch.equal(got, want)
