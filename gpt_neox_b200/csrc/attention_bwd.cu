@@ -2,32 +2,41 @@
 //
 // Three launches, no atomics, no fp32 scratch for dQ, deterministic:
 //   1. attn_delta_kernel    delta[b,h,q] = sum_d O * dO
-//   2. attn_bwd_dq_kernel   one CTA per 128 query rows: loops over key blocks, recomputes
-//                           S = Q K^T and dP = dO V^T on the tensor cores, forms
-//                           dS = P o (dP - delta) * scale per row (thread == query row), writes it
-//                           as bf16 into TMEM and accumulates dQ += dS K  (A operand from TMEM).
-//   3. attn_bwd_dkv_kernel  one CTA per 128 keys (per kv head; loops over the query heads of the
-//                           GQA group and over query blocks): computes the transposed tiles
-//                           S^T = K Q^T and dP^T = V dO^T so that thread == key row, writes P^T and
-//                           dS^T (bf16) over the same TMEM columns and accumulates
-//                           dV += P^T dO,  dK += dS^T Q.
-// Recomputing S and dP in both kernels costs 7 tile GEMMs instead of 5 but keeps every
-// accumulator in TMEM from first to last block.  Counterpart of the flash-attn 2 backward the
-// reference calls through autograd (megatron/model/transformer.py:573-690).
-#include <cstdlib>
-
+//   2. attn_bwd_dq_kernel   items of 128 query rows: loops over 128-key blocks, recomputes S = Q K^T and dP = dO V^T on
+//                           the tensor cores, forms dS = P o (dP - delta) * scale per row (thread == query row), writes
+//                           it as 16-bit values into TMEM and accumulates dQ += dS K  (A operand from TMEM).
+//   3. attn_bwd_dkv_kernel  items of 128 keys (per kv head; loops over the query heads of the GQA group and over blocks of
+//                           64 query rows): the transposed tiles S^T = K Q^T and dP^T = V dO^T, so that thread == key row,
+//                           P^T and dS^T as 16-bit values into TMEM, dV += P^T dO and dK += dS^T Q.
+// Recomputing S and dP in both kernels costs 7 tile GEMMs instead of 5 but keeps every accumulator in TMEM from first to
+// last block.  Counterpart of the flash-attn 2 backward the reference calls through autograd
+// (megatron/model/transformer.py:573-690).
+//
+// Both kernels are persistent, one CTA per SM that walks its share of the items:
+//   warp 0      TMA producer: streamed tiles in rings, the next item's resident tiles as soon as the last scores are issued
+//   warps 1, 2  tcgen05.mma issuers, one for the scores (which runs ahead, across items), one for the products
+//   warps 4 ..  element-wise: dQ eight warps, 64 of a block's key columns each; dK / dV two sets of eight warps (32 query
+//               columns each) that take the blocks in turn, so that one set's waits lie under the other's arithmetic.  They also
+//               store a finished item's accumulators, after the next item's first block.
+// What bounds them (cycle counts of the roles): neither the tensor cores nor the exponentials but the chain scores -> registers
+// -> 16-bit results -> products, with about 500 cycles from a commit or an arrival to the warp that waits for it, so a block
+// costs dQ 2,300 cycles (MMAs 1,536, exponentials 1,024) and dK / dV 1,750 per 64 queries (MMAs 1,024: one pair of result
+// buffers is all that the accumulators leave).  Hence everything that lets blocks overlap: issuers apart from each other (one
+// thread issuing all was the bound at 1,700 cycles per 64 rows), scores two blocks ahead, score buffers given back as soon as
+// they are in registers, the next item's tiles and stores in the shadow of the running one.
+// Batch 4, 32 heads, 2048 x 128 causal: dQ 293 -> 197 us, dK / dV 330 -> 290 us; 5003 tokens, 32 heads on 8, window of 4096:
+// 331 -> 232 us and 438 -> 322 us (before: a CTA per item, one issuing thread, all eight element-wise warps on the same 64
+// columns).  What was slower: two groups of four warps that write their results over their scores (260 / 333 us), dQ by 16
+// warps with 32 columns each (215 us), dQ with two K stages (258 us), one V stage (212 us).
 #include "common.h"
 #include "ptx.cuh"
 #include "reduce.cuh"
 
 namespace nx {
 
-constexpr int AB = 128;  // rows per tile in every role
-// Threads per CTA: producer warp, MMA warp and 4 * HALVES element-wise warps.  HALVES = 2 (default) puts two warps
-// on every TMEM lane quadrant, each taking half of the 128 columns of a block (one warp per scheduler leaves the
-// exponential / convert pipes idle during the serial S -> P -> dS chain); HALVES = 1 is the four-warp form
-// (NEOX_ATTN_BWD_WARPS=4 selects it).
-constexpr int ab_threads(int halves) { return 64 + 128 * halves; }
+constexpr int AB = 128;  // rows per resident tile and per key block of the dQ kernel
+constexpr int ABS = 64;  // query rows per block of the dK / dV kernel
+constexpr int DQ_THREADS = 32 * 12, DKV_THREADS = 32 * 20;
 constexpr float LOG2E = 1.4426950408889634f;
 
 struct AttnBwdParams {
@@ -110,117 +119,250 @@ attn_delta_any_kernel(const h16* __restrict__ o, const h16* __restrict__ dO, flo
   if (lane == 0) delta[(static_cast<long long>(b) * H + h) * Sq_pad + q] = s;
 }
 
-// AND of a predicate over the 64 threads (two warps) that meet at named barrier `id`.
-__device__ __forceinline__ bool pair_all(bool ok, int id) {
-  uint32_t out;
-  asm volatile(
-      "{\n"
-      ".reg .pred pi, po;\n"
-      "setp.ne.u32 pi, %1, 0;\n"
-      "bar.red.and.pred po, %2, 64, pi;\n"
-      "selp.u32 %0, 1, 0, po;\n"
-      "}\n"
-      : "=r"(out)
-      : "r"(ok ? 1u : 0u), "r"(id)
-      : "memory");
-  return out != 0;
-}
-
+// Shared memory, in tiles of 64 rows: the resident pair (128 rows each; dQ: Q, dO; dK / dV: K, V), ten tiles of rings (dQ: K in
+// three 128-row stages, V in two; dK / dV: Q and dO in four 64-row stages), the streamed rows' lse / delta (dK / dV), barriers.
 template <int DP>
 struct BwdSmem {
-  static constexpr int TILE = AB * DP * 2;
-  static constexpr int BAR_OFF = 6 * TILE;  // two resident tiles + 2 x 2 streamed tiles
-  static constexpr int NBAR = 24;
-  static constexpr int VEC_OFF = BAR_OFF + NBAR * 8;  // lse / delta staging: 2 stages x 2 x 128 floats
-  static constexpr int TOTAL = VEC_OFF + 4 * AB * 4 + 16;
+  static constexpr int T64 = 64 * DP * 2;
+  static constexpr int STR_OFF = 4 * T64;
+  static constexpr int V_OFF = STR_OFF + 6 * T64;              // dQ
+  static constexpr int VEC_OFF = STR_OFF + 8 * T64;            // dK / dV: [BWD_STAGES][lse, delta][64]
+  static constexpr int BAR_OFF = STR_OFF + 10 * T64;
+  static constexpr int TOTAL = BAR_OFF + 28 * 8;               // 27 barriers and the TMEM base word
   static constexpr int DYN = TOTAL + 1024;
 };
+constexpr int BWD_STAGES = 4;
+static_assert(BwdSmem<128>::DYN <= 232448, "shared memory of one SM");
+static_assert(BWD_STAGES * 2 * 64 * 4 <= 2 * BwdSmem<64>::T64, "lse / delta fit behind the ring");
 
-// Loads one [128 x DP] tile (rows contiguous in d) as DP/64 swizzled boxes.
-template <int DP>
-__device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap* m, uint32_t bar, int row0,
-                                          int head, int batch) {
-#pragma unroll
-  for (int c = 0; c < DP / 64; ++c) tma_load_4d(dst + c * (AB * 128), m, bar, c * 64, row0, head, batch);
+// Barriers.  RES: the two resident tiles; STR / STR2: rings of streamed tiles (STR2: V of the dQ kernel); S: scores of block n
+// in buffer n & 1 written by the tensor core (FULL), in the element-wise warps' registers (EMPTY: dK / dV); DP: the same of the
+// one dP buffer (dK / dV: FULL per set); P_FULL: the 16-bit results of block n written.  That these are consumed STR_EMPTY
+// tells: the products of a block are its stage's last readers.  ACC: an item's accumulators complete / read.
+enum { RES_FULL = 0, RES_EMPTY = 2, STR_FULL = 4, STR_EMPTY = 8, STR2_FULL = 12, STR2_EMPTY = 14, S_FULL = 16, S_EMPTY = 18,
+       DP_FULL = 20, DP_EMPTY = 22, P_FULL = 23, ACC_FULL = 25, ACC_EMPTY = 26, BWD_NBAR = 27 };
+__device__ __forceinline__ void bwd_init_barriers(uint32_t bar0) {
+  for (int i = 0; i < BWD_NBAR; ++i) {
+    const bool by_warps = i == S_EMPTY || i == S_EMPTY + 1 || i == DP_EMPTY || i == P_FULL || i == P_FULL + 1 || i == ACC_EMPTY;
+    mbar_init(bar0 + 8u * i, by_warps ? 8 : 1);     // one arrival per element-wise warp that shares a block
+  }
+  fence_barrier_init();
 }
-// D[128 x N] = A[128 x DP] * B[N x DP]^T, both K-major (head dim contiguous); b points at the first of the N rows.
-template <int DP, int N = AB>
-__device__ __forceinline__ void mma_nt(uint32_t d_tmem, uint32_t a, uint32_t b) {
+
+// Loads ROWS rows (contiguous in d) of one tensor as boxes of 64 rows x 64 columns, swizzled; 64-column panels are ROWS *
+// 128 bytes apart.
+template <int DP, int ROWS>
+__device__ __forceinline__ void load_rows(uint32_t dst, const CUtensorMap* m, uint32_t bar, int row0, int head, int batch) {
+#pragma unroll
+  for (int c = 0; c < DP / 64; ++c)
+#pragma unroll
+    for (int r = 0; r < ROWS; r += 64) tma_load_4d(dst + c * (ROWS * 128) + r * 128, m, bar, c * 64, row0 + r, head, batch);
+}
+// The two issuing warps run converged and only the instructions themselves are predicated on one lane: the descriptors then
+// live in uniform registers, where a single diverged lane pays moves for every operand.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, int* err, int where) {
+  const bool ok = mbar_wait(bar, parity, err, where);
+  return __all_sync(0xffffffffu, ok);
+}
+// D[128 x N] = A[128 x DP] * B[N x DP]^T, both K-major (head dim contiguous).
+template <int DP, int N>
+__device__ __forceinline__ void mma_nt(uint32_t leader, uint32_t d_tmem, uint32_t a, uint32_t b) {
   constexpr uint32_t idesc = umma_idesc_bf16(AB, N, 0, 0);
+  const uint32_t al = umma_desc_lo(a, 0), bl = umma_desc_lo(b, 0);
 #pragma unroll
-  for (int k = 0; k < DP / 16; ++k) {
-    const uint32_t o = (k >> 2) * (AB * 128) + (k & 3) * 32;
-    umma_bf16_ss(d_tmem, umma_smem_desc_sw128(a + o, 0, 1024), umma_smem_desc_sw128(b + o, 0, 1024),
-                 idesc, k != 0 ? 1u : 0u);
-  }
+  for (int k = 0; k < DP / 16; ++k)
+    umma_bf16_ss_by(leader, d_tmem, al + ((k >> 2) * (AB * 128) + (k & 3) * 32) / 16,
+                    bl + ((k >> 2) * (N * 128) + (k & 3) * 32) / 16, idesc, k != 0 ? 1u : 0u);
 }
-// D[128 x DP] (+)= A_tmem[128 x 128 (bf16, 64 columns)] * B[128 x DP] with B's head dim contiguous
-// (MN-major B operand).
-// KR: rows of B (the contraction length), 128 or 64; b points at the first of them.  SPLIT: every 16 columns of A (32
-// rows of B) start 32 columns apart instead of lying back to back.
-template <int DP, int KR = AB, bool SPLIT = false>
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b, bool accumulate) {
+// D[128 x DP] (+)= A_tmem[128 x KR (16 bit)] * B[KR x DP] with B's head dim contiguous (MN-major B operand).  The KR / 2
+// columns of A lie in two halves, `gap` columns from the first of one to the first of the other.
+template <int DP, int KR>
+__device__ __forceinline__ void mma_ts(uint32_t leader, uint32_t d_tmem, uint32_t a_tmem, int gap, uint32_t b, bool accumulate) {
   constexpr uint32_t idesc = umma_idesc_bf16(AB, DP, 0, 1);
+  const uint32_t bl = umma_desc_lo(b, KR * 128);
 #pragma unroll
-  for (int k = 0; k < KR / 16; ++k) {
-    umma_bf16_ts(d_tmem, a_tmem + (SPLIT ? (k >> 1) * 32 + (k & 1) * 8 : k * 8), umma_smem_desc_sw128(b + k * 2048, AB * 128, 1024), idesc,
-                 (accumulate || k != 0) ? 1u : 0u);
-  }
+  for (int k = 0; k < KR / 16; ++k)
+    umma_bf16_ts_by(leader, d_tmem, a_tmem + (k >= KR / 32 ? gap + (k - KR / 32) * 8 : k * 8), bl + k * (2048 / 16), idesc,
+                    (accumulate || k != 0) ? 1u : 0u);
 }
 
+// One piece of work: 128 rows of one head and its streamed blocks [j0, j1).
+struct BwdItem {
+  int tile, head, batch, j0, j1;
+  int n_i;      // dK / dV: query blocks per head (block j: query head j / n_i of the group)
+  int i0;       // dK / dV: first of them
+};
+
+// Which items a CTA takes: the longest first (causal), dealt out forwards and backwards in turn, so that a CTA which got a
+// longer item in one round gets a shorter one in the next.
+struct BwdOrder {
+  int total;
+  __device__ __forceinline__ bool next(int& r, int& w) const {
+    const int G = gridDim.x, c = blockIdx.x;
+    do {
+      ++r;
+      if (r * G >= total) return false;
+      w = r * G + ((r & 1) ? G - 1 - c : c);
+    } while (w >= total);
+    return true;
+  }
+};
+
+// GEN: block-sparse layouts skip the 128 x 128 tiles without a live block, in every role alike.
+template <bool GEN>
+struct DqWork {
+  const AttnBwdParams& p;
+  BwdOrder order;
+  int nt;
+  __device__ __forceinline__ explicit DqWork(const AttnBwdParams& p_) : p(p_) {
+    nt = (p.Sq + AB - 1) / AB;
+    order.total = nt * p.H * p.B;
+  }
+  __device__ __forceinline__ bool next(int& r, BwdItem& it) const {
+    int w;
+    if (!order.next(r, w)) return false;
+    const int hb = p.H * p.B, q = w / hb;
+    w -= q * hb;
+    it.tile = nt - 1 - q;
+    it.batch = w / p.H;
+    it.head = w - it.batch * p.H;
+    const int q0 = it.tile * AB, off = p.Sk - p.Sq;
+    const int kv_end = p.causal ? min(p.Sk, q0 + AB + off) : p.Sk;
+    const int kv_begin = p.window >= 0 ? max(0, q0 + off - p.window) : 0;
+    it.j0 = kv_begin / AB;
+    it.j1 = max((kv_end + AB - 1) / AB, it.j0);
+    return true;
+  }
+  __device__ __forceinline__ bool live(const BwdItem& it, int j) const {
+    return !GEN || p.blk_any == nullptr || p.blk_any[static_cast<long long>(it.tile) * p.blk_nkt + j] != 0;
+  }
+};
+template <bool GEN>
+struct DkvWork {
+  const AttnBwdParams& p;
+  BwdOrder order;
+  int group;
+  __device__ __forceinline__ explicit DkvWork(const AttnBwdParams& p_) : p(p_) {
+    group = p.H / p.Hk;
+    order.total = (p.Sk + AB - 1) / AB * p.Hk * p.B;
+  }
+  __device__ __forceinline__ bool next(int& r, BwdItem& it) const {
+    int w;
+    if (!order.next(r, w)) return false;
+    const int hb = p.Hk * p.B;
+    it.tile = w / hb;
+    w -= it.tile * hb;
+    it.batch = w / p.Hk;
+    it.head = w - it.batch * p.Hk;
+    const int k0 = it.tile * AB, off = p.Sk - p.Sq;
+    // query rows that can see this key tile: qpos >= k0 (causal), qpos <= k_last + window
+    const int q_begin = p.causal ? max(0, k0 - off) : 0;
+    const int q_end = p.window >= 0 ? min(p.Sq, k0 + AB + p.window - off) : p.Sq;
+    it.i0 = q_begin / ABS;
+    it.n_i = max((q_end + ABS - 1) / ABS - it.i0, 0);
+    it.j0 = 0;
+    it.j1 = it.n_i * group;
+    return true;
+  }
+  __device__ __forceinline__ bool live(const BwdItem& it, int j) const {
+    return !GEN || p.blk_any == nullptr ||
+           p.blk_any[static_cast<long long>((it.i0 + j % it.n_i) >> 1) * p.blk_nkt + it.tile] != 0;
+  }
+};
+
+// Waits for this warp's TMEM loads; their registers pass through it, so that no use can move in front of it.
+__device__ __forceinline__ void tmem_ld_wait_for(uint32_t (&r)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                 "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]),
+                 "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]),
+                 "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29])
+               :
+               : "memory");
+  asm volatile("" : "+r"(r[30]), "+r"(r[31]));
+}
+
+// A warp's 32 rows x 64 columns of a finished accumulator (zeros where the item had no block): scaled, rounded, transposed in
+// pieces of 16 bytes within groups of eight lanes and stored, a group a whole row of 128 bytes.  Written by each lane to its own
+// row, every store touched 32 lines, and an item's held up the element-wise warps for 3,800 cycles.
+__device__ __forceinline__ void bwd_acc_load(uint32_t tmem_cols, uint32_t (&lo)[32], uint32_t (&hi)[32]) {
+  tmem_ld_32x32b_x32(tmem_cols, lo);
+  tmem_ld_32x32b_x32(tmem_cols + 32, hi);
+  tmem_ld_wait_for(lo);
+  tmem_ld_wait_for(hi);
+}
+__device__ __forceinline__ void bwd_store(h16* base, long long row_stride, const uint32_t (&lo)[32], const uint32_t (&hi)[32],
+                                          float sc, int col, int row, int rows, int D) {
+  const int lane = threadIdx.x & 31;
+  uint32_t w[8][4];
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int e = (c & 3) * 8 + 2 * k;
+      const uint32_t x = c < 4 ? lo[e] : hi[e], y = c < 4 ? lo[e + 1] : hi[e + 1];
+      w[c][k] = pack_h16x2(__uint_as_float(x) * sc, __uint_as_float(y) * sc);
+    }
+#pragma unroll
+  for (int m = 4; m > 0; m >>= 1) {
+    const bool up = lane & m;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      if (c & m) continue;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? w[c][k] : w[c | m][k], m);
+        if (up) w[c][k] = got;
+        else w[c | m][k] = got;
+      }
+    }
+  }
+  // w[k]: piece lane % 8 of row (lane / 8) * 8 + k
+  const int c8 = col + (lane & 7) * 8, r0 = row + (lane & ~7);
+  if (c8 < D) {
+    h16* o = base + r0 * row_stride + c8;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (r0 + k < rows) *reinterpret_cast<uint4*>(o + k * row_stride) = make_uint4(w[k][0], w[k][1], w[k][2], w[k][3]);
+  }
+  __syncwarp();
+}
+
+// The first live block from j on (j1: none).
+template <class Work>
+__device__ __forceinline__ int next_live(const Work& work, const BwdItem& it, int j) {
+  while (j < it.j1 && !work.live(it, j)) ++j;
+  return j;
+}
 // ------------------------------------------------------------------------------------------------
-// dQ kernel.  smem tiles: 0 = Q, 1 = dO, 2..3 = K ring, 4..5 = V ring.
-// TMEM: S [0,128) dP [128,256) dQ [256,256+DP) dS0 [384,448) dS1 [448,512)
-// PIPE (default, eight element-wise warps): the 128 keys of a block are handled as two halves of 64 with their own
-// S / dP columns (S_h at [64 h, ...), dP_h at [128 + 64 h, ...)), dS_h at [384 + 32 h, ...) and their own barriers.
-// The MMA warp issues S / dP of half u + 1 before it waits for dS of half u, so the tensor core computes the next
-// half (and dQ += dS K of the previous one) while the element-wise warps work on the current one; without PIPE
-// the tensor core and the element-wise warps take turns.
+// dQ kernel.  Resident: Q, dO (128 rows).  Streamed: K, V (128 rows).  An element-wise warp has 64 of a block's key columns, in
+// two chunks of 32; dS goes over the first half of the score columns the warp itself has read.
+// TMEM: S of block n at [128 (n & 1), ...), dP [256, 384), dQ [384, 384 + DP).
 // GEN (this kernel and the next): ALiBi and block-sparse layouts; without them a block that needs a mask differs from one
-// that does not by one select per element (batch 4, 32 heads, 2048 x 128 causal: dQ 318 -> 288 us, dK / dV, with its
-// barriers gone, 334 -> 323 us).
+// that does not by one select per element.
 // ------------------------------------------------------------------------------------------------
-template <int DP, bool DROP, int HALVES, bool PIPE, bool GEN>
-__global__ void __launch_bounds__(ab_threads(HALVES), 1)
+template <int DP, bool DROP, bool GEN>
+__global__ void __launch_bounds__(DQ_THREADS, 1)
     attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                       const AttnBwdParams p) {
+                       const __grid_constant__ AttnBwdParams p) {
   using L = BwdSmem<DP>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sgen = smem_raw + (sbase - smem_u32(smem_raw));
   const uint32_t bar0 = sbase + L::BAR_OFF;
-  static_assert(!PIPE || HALVES == 2, "the pipelined form gives each of a half's 64 columns' halves to one warp");
-  enum { QDO_FULL = 0, K_FULL = 1, K_EMPTY = 3, V_FULL = 5, V_EMPTY = 7, SDP_FULL = 9, DS_FULL = 11, DQ_DONE = 13,
-         SDP_EMPTY = 15, NUSED = 16 };
   auto bar = [&](int which, int idx) { return bar0 + 8u * (which + idx); };
-  const uint32_t tmem_slot = bar0 + 8u * 23;
-  volatile uint32_t* tmem_slot_gen = reinterpret_cast<volatile uint32_t*>(sgen + L::BAR_OFF + 8 * 23);
-  auto tile = [&](int i) { return sbase + i * L::TILE; };
+  const uint32_t tmem_slot = bar0 + 8u * BWD_NBAR;
+  volatile uint32_t* tmem_slot_gen = reinterpret_cast<volatile uint32_t*>(sgen + L::BAR_OFF + 8 * BWD_NBAR);
+  auto res = [&](int which) { return sbase + which * (2 * L::T64); };
+  auto kst = [&](int stage) { return sbase + L::STR_OFF + stage * (2 * L::T64); };
+  auto vst = [&](int stage) { return sbase + L::V_OFF + stage * (2 * L::T64); };
+  constexpr uint32_t T_DP = 256, T_DQ = 384;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qt = gridDim.x - 1 - blockIdx.x;
-  const int head = blockIdx.y, batch = blockIdx.z;
-  const int kv_head = head / (p.H / p.Hk);
-  const int q0 = qt * AB;
   const int off = p.Sk - p.Sq;
-  int kv_end = p.Sk;
-  if (p.causal) kv_end = min(p.Sk, q0 + AB + off);
-  int kv_begin = 0;
-  if (p.window >= 0) kv_begin = max(0, q0 + off - p.window);
-  const int jb = kv_begin / AB;
-  const int nblk = max((kv_end + AB - 1) / AB - jb, 0);
-  // block-sparse layouts: key tiles without a live block for this query tile are skipped by every role; ring
-  // stages and barrier phases count the live tiles
-  auto tile_live = [&](int kt) { return !GEN || p.blk_any == nullptr || p.blk_any[static_cast<long long>(qt) * p.blk_nkt + kt] != 0; };
-
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < NUSED; ++i) {
-      const bool by_softmax = (i == SDP_EMPTY) || (i >= DS_FULL && i < DS_FULL + 2);
-      mbar_init(bar0 + 8u * i, by_softmax ? 4 * HALVES : 1);
-    }
-    fence_barrier_init();
-  }
+  const DqWork<GEN> work(p);
+  if (threadIdx.x == 0) bwd_init_barriers(bar0);
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
@@ -229,237 +371,278 @@ __global__ void __launch_bounds__(ab_threads(HALVES), 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot_gen;
-  const uint32_t T_S = tmem, T_DP = tmem + 128, T_DQ = tmem + 256, T_DS = tmem + 384;
   bool aborted = false;
 
   if (warp == 0) {
-    if (elect_one() && nblk > 0) {
-      mbar_expect_tx(bar(QDO_FULL, 0), 2 * L::TILE);
-      load_tile<DP>(tile(0), &tmQ, bar(QDO_FULL, 0), q0, head, batch);
-      load_tile<DP>(tile(1), &tmDO, bar(QDO_FULL, 0), q0, head, batch);
-      for (int t = 0, n = 0; t < nblk; ++t) {
-        if (!tile_live(jb + t)) continue;
-        const int i = n++;
-        const int st = i & 1;
-        const uint32_t ph = (i >> 1) & 1;
-        const int k0 = (jb + t) * AB;
-        if (!mbar_wait(bar(K_EMPTY, st), ph ^ 1, p.err, 31)) { aborted = true; break; }
-        mbar_expect_tx(bar(K_FULL, st), L::TILE);
-        load_tile<DP>(tile(2 + st), &tmK, bar(K_FULL, st), k0, kv_head, batch);
-        if (!mbar_wait(bar(V_EMPTY, st), ph ^ 1, p.err, 32)) { aborted = true; break; }
-        mbar_expect_tx(bar(V_FULL, st), L::TILE);
-        load_tile<DP>(tile(4 + st), &tmV, bar(V_FULL, st), k0, kv_head, batch);
+    if (elect_one()) {
+      int n = 0, t = 0, round = -1, ks = 0;
+      uint32_t kph = 0;
+      BwdItem it;
+      while (!aborted && work.next(round, it)) {
+        const int kv_head = it.head / (p.H / p.Hk);
+        bool any = false;
+        for (int j = it.j0; j < it.j1; ++j) {
+          if (!work.live(it, j)) continue;
+          const int vs = n & 1;
+          if (!mbar_wait(bar(STR_EMPTY, ks), kph ^ 1, p.err, 32)) { aborted = true; break; }
+          mbar_expect_tx(bar(STR_FULL, ks), 2 * L::T64);
+          load_rows<DP, AB>(kst(ks), &tmK, bar(STR_FULL, ks), j * AB, kv_head, it.batch);
+          if (!any) {
+            for (int w = 0; w < 2 && !aborted; ++w) {
+              if (!mbar_wait(bar(RES_EMPTY, w), (t & 1) ^ 1, p.err, 31)) { aborted = true; break; }
+              mbar_expect_tx(bar(RES_FULL, w), 2 * L::T64);
+              load_rows<DP, AB>(res(w), w == 0 ? &tmQ : &tmDO, bar(RES_FULL, w), it.tile * AB, it.head, it.batch);
+            }
+            any = true;
+            ++t;
+          }
+          if (aborted || !mbar_wait(bar(STR2_EMPTY, vs), ((n >> 1) & 1) ^ 1, p.err, 37)) { aborted = true; break; }
+          mbar_expect_tx(bar(STR2_FULL, vs), 2 * L::T64);
+          load_rows<DP, AB>(vst(vs), &tmV, bar(STR2_FULL, vs), j * AB, kv_head, it.batch);
+          ++n;
+          if (++ks == 3) {
+            ks = 0;
+            kph ^= 1;
+          }
+        }
       }
     }
   } else if (warp == 1) {
-    if (elect_one() && nblk > 0) {
-      auto issue_dq = [&](int i) -> bool {
-        const int st = i & 1;
-        if (!mbar_wait(bar(DS_FULL, st), (i >> 1) & 1, p.err, 33)) return false;
-        tc_fence_after_sync();
-        mma_ts<DP>(T_DQ, T_DS + st * 64, tile(2 + st), i != 0);
-        umma_commit(bar(DQ_DONE, st));
-        umma_commit(bar(K_EMPTY, st));
-        return true;
-      };
-      if (!mbar_wait(bar(QDO_FULL, 0), 0, p.err, 34)) aborted = true;
-      int n = 0;
-      if (PIPE) {
-        // sub-step u = 2 i + h of live block i: S_h = Q K_h^T, dP_h = dO V_h^T (64 keys), later dQ += dS_h K_h
-        int nl = 0;
-        for (int t = 0; t < nblk; ++t) nl += tile_live(jb + t) ? 1 : 0;
-        auto issue_m1 = [&](int u) -> bool {
-          const int i = u >> 1, h = u & 1, st = i & 1;
-          if (h == 0) {
-            if (!mbar_wait(bar(K_FULL, st), (i >> 1) & 1, p.err, 35)) return false;
-            if (!mbar_wait(bar(V_FULL, st), (i >> 1) & 1, p.err, 36)) return false;
-          }
-          tc_fence_after_sync();
-          mma_nt<DP, 64>(T_S + h * 64, tile(0), tile(2 + st) + h * (64 * 128));
-          mma_nt<DP, 64>(T_DP + h * 64, tile(1), tile(4 + st) + h * (64 * 128));
-          umma_commit(bar(SDP_FULL, h));
-          if (h == 1) umma_commit(bar(V_EMPTY, st));
-          return true;
-        };
-        const int nsub = 2 * nl;
-        if (!aborted && nsub > 0 && !issue_m1(0)) aborted = true;
-        for (int u = 0; u < nsub && !aborted; ++u) {
-          const int i = u >> 1, h = u & 1, st = i & 1;
-          if (u + 1 < nsub && !issue_m1(u + 1)) { aborted = true; break; }
-          if (!mbar_wait(bar(DS_FULL, h), i & 1, p.err, 33)) { aborted = true; break; }
-          tc_fence_after_sync();
-          mma_ts<DP, 64>(T_DQ, T_DS + h * 32, tile(2 + st) + h * (64 * 128), u != 0);    // dQ += dS_h K_h
-          if (h == 1) umma_commit(bar(K_EMPTY, st));
+    // S = Q K^T, dP = dO V^T
+    const uint32_t leader = elect_one() ? 1u : 0u;
+    int n = 0, t = 0, round = -1, ks = 0;
+    uint32_t kph = 0;
+    BwdItem it;
+    while (!aborted && work.next(round, it)) {
+      bool any = false;
+      for (int j = it.j0; j < it.j1; ++j) {
+        if (!work.live(it, j)) continue;
+        const bool last = next_live(work, it, j + 1) >= it.j1;
+        const int st = n & 1;
+        const uint32_t ph = (n >> 1) & 1;
+        // (S buffer n & 1 is free when dQ has taken dS of block n - 2: its stage is two back in the ring of three)
+        if ((!any && !warp_wait(bar(RES_FULL, 0), t & 1, p.err, 34)) || !warp_wait(bar(STR_FULL, ks), kph, p.err, 35) ||
+            (n >= 2 && !warp_wait(bar(STR_EMPTY, ks < 2 ? ks + 1 : 0), ks < 2 ? kph ^ 1 : kph, p.err, 39))) {
+          aborted = true;
+          break;
         }
-        if (!aborted && nsub > 0) umma_commit(bar(DQ_DONE, 0));
-        n = 0;      // (the loop below is the unpipelined form)
-      }
-      for (int t = 0; !PIPE && t < nblk && !aborted; ++t) {
-        if (!tile_live(jb + t)) continue;
-        const int i = n++;
-        const int st = i & 1;
-        const uint32_t ph = (i >> 1) & 1;
-        if (!mbar_wait(bar(K_FULL, st), ph, p.err, 35)) { aborted = true; break; }
-        if (!mbar_wait(bar(V_FULL, st), ph, p.err, 36)) { aborted = true; break; }
-        if (!mbar_wait(bar(SDP_EMPTY, 0), (i & 1) ^ 1, p.err, 37)) { aborted = true; break; }
         tc_fence_after_sync();
-        mma_nt<DP>(T_S, tile(0), tile(2 + st));
-        mma_nt<DP>(T_DP, tile(1), tile(4 + st));
-        umma_commit(bar(SDP_FULL, 0));
-        umma_commit(bar(V_EMPTY, st));
-        if (i > 0 && !issue_dq(i - 1)) { aborted = true; break; }
+        mma_nt<DP, AB>(leader, tmem + st * AB, res(0), kst(ks));
+        umma_commit_by(leader, bar(S_FULL, st));
+        if (last) umma_commit_by(leader, bar(RES_EMPTY, 0));
+        if ((!any && !warp_wait(bar(RES_FULL, 1), t & 1, p.err, 45)) || !warp_wait(bar(STR2_FULL, st), ph, p.err, 36) ||
+            !warp_wait(bar(DP_EMPTY, 0), (n & 1) ^ 1, p.err, 43)) {
+          aborted = true;
+          break;
+        }
+        tc_fence_after_sync();
+        mma_nt<DP, AB>(leader, tmem + T_DP, res(1), vst(st));
+        umma_commit_by(leader, bar(DP_FULL, 0));
+        umma_commit_by(leader, bar(STR2_EMPTY, st));
+        if (last) umma_commit_by(leader, bar(RES_EMPTY, 1));
+        any = true;
+        ++n;
+        if (++ks == 3) {
+          ks = 0;
+          kph ^= 1;
+        }
       }
-      if (!PIPE && !aborted && n > 0 && !issue_dq(n - 1)) aborted = true;
+      t += any;
     }
-  } else {
-    const int quad = warp & 3;
-    const int half = (warp - 2) >> 2;    // HALVES = 2: which 64 of the 128 key columns of a block (and half of dQ's columns)
-    constexpr int CPW = (AB / 32) / HALVES;   // 32-column chunks per warp and block
+  } else if (warp == 2) {
+    // dQ += dS K
+    const uint32_t leader = elect_one() ? 1u : 0u;
+    int n = 0, t = 0, round = -1, ks = 0;
+    BwdItem it;
+    while (!aborted && work.next(round, it)) {
+      bool any = false;
+      for (int j = it.j0; j < it.j1; ++j) {
+        if (!work.live(it, j)) continue;
+        if ((!any && !warp_wait(bar(ACC_EMPTY, 0), (t & 1) ^ 1, p.err, 33)) ||
+            !warp_wait(bar(P_FULL, n & 1), (n >> 1) & 1, p.err, 41)) {
+          aborted = true;
+          break;
+        }
+        tc_fence_after_sync();
+        mma_ts<DP, AB>(leader, tmem + T_DQ, tmem + (n & 1) * AB, 64, kst(ks), any);
+        umma_commit_by(leader, bar(STR_EMPTY, ks));
+        any = true;
+        ++n;
+        if (++ks == 3) ks = 0;
+      }
+      if (any) {
+        umma_commit_by(leader, bar(ACC_FULL, 0));
+        ++t;
+      }
+    }
+  } else if (warp >= 4) {
+    // ------------------------------------------------------------------ element-wise warps
+    const int quad = warp & 3, c0 = ((warp - 4) >> 2) * 64;      // first of this warp's 64 key columns of a block
     const int r = quad * 32 + lane;
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-    const int qi = q0 + r;
-    const int qpos = qi + off;
-    const bool row_ok = qi < p.Sq;
-    const long long stat_idx = (static_cast<long long>(batch) * p.H + head) * p.Sq_pad + qi;
-    const float lse2 = p.lse[stat_idx];     // +inf for rows past Sq -> P = 0
-    const float delta = p.delta[stat_idx];
-    const float slope2 = GEN && p.alibi != nullptr ? p.alibi[head] * LOG2E : 0.f;
-    int nlive = 0;
-    for (int t = 0; t < nblk; ++t) {
-      if (!tile_live(jb + t)) continue;
-      const int i = nlive++;
-      const int st = i & 1;
-      const int k0 = (jb + t) * AB;
-      uint32_t bits = 0xffffffffu;
-      if (GEN && p.blk_rows != nullptr)
-        bits = row_ok ? p.blk_rows[static_cast<long long>(qi) * p.blk_nkt + (jb + t)] : 0u;
-      const uint32_t full_bits = (1u << (AB >> p.blk_shift)) - 1u;
-      const bool blk_partial = GEN && p.blk_rows != nullptr && !__all_sync(0xffffffffu, (bits & full_bits) == full_bits);
-      if (!PIPE) {
-        if (!mbar_wait(bar(SDP_FULL, 0), i & 1, p.err, 38)) { aborted = true; break; }
-        if (i >= 2 && !mbar_wait(bar(DQ_DONE, st), ((i - 2) >> 1) & 1, p.err, 39)) { aborted = true; break; }
+    const uint32_t t_s = tmem + c0 + lane_off, t_dp = t_s + T_DP;
+    int n = 0, round = -1, t = 0;
+    BwdItem it;
+    bool pending = false;      // `done`: an item whose dQ this warp has still to store
+    BwdItem done;
+    const bool stores = c0 < DP;      // (64 columns of dQ per warp)
+    auto finish = [&](const BwdItem& i, bool live) -> bool {
+      uint32_t lo[32], hi[32];
+#pragma unroll
+      for (int e = 0; e < 32; ++e) lo[e] = hi[e] = 0u;
+      if (live) {
+        const bool ok = mbar_wait(bar(ACC_FULL, 0), t & 1, p.err, 40);
+        if (!__all_sync(0xffffffffu, ok)) return false;
         tc_fence_after_sync();
+        if (stores) bwd_acc_load(tmem + T_DQ + c0 + lane_off, lo, hi);
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(ACC_EMPTY, 0));
+        ++t;
       }
-      const bool need_mask = (k0 + AB > p.Sk) || (p.causal && k0 + AB - 1 > q0 + quad * 32 + off) ||
-                             (p.window >= 0 && k0 < q0 + quad * 32 + 31 + off - p.window) || blk_partial;
-      const int rel0 = k0 - qpos;
-      int hi = p.Sk - k0 - 1;
-      if (p.causal) hi = min(hi, -rel0);
-      const int lo = p.window >= 0 ? -rel0 - p.window : -(1 << 30);
-      const float bias0 = slope2 * static_cast<float>(rel0) - lse2;  // folded into the exponent
-      // PIPE: pass h = 0, 1 over the block's halves, this warp's chunk in each is c = 2 h + half (block columns
-      // 32 c ..), read from the half's own S / dP columns after its own barrier; otherwise CPW chunks of the one buffer.
-#pragma unroll 1
-      for (int cc = 0; cc < (PIPE ? 2 : CPW); ++cc) {
-        const int c = PIPE ? cc * 2 + half : half * CPW + cc;
-        if (PIPE) {
-          if (!mbar_wait(bar(SDP_FULL, cc), i & 1, p.err, 38)) { aborted = true; break; }
-          tc_fence_after_sync();
+      const int row = i.tile * AB + quad * 32;
+      if (stores)
+        bwd_store(p.dq + i.batch * p.dq_sb + i.head * p.dq_sh, p.dq_ss, lo, hi, p.scale, c0, row, p.Sq, p.D);
+      return true;
+    };
+    auto stat_of = [&](const BwdItem& i) {
+      return (static_cast<long long>(i.batch) * p.H + i.head) * p.Sq_pad + i.tile * AB + r;
+    };
+    auto wait = [&](int which, int idx, uint32_t parity, int where) -> bool {
+      const bool ok = mbar_wait(bar(which, idx), parity, p.err, where);
+      const bool all = __all_sync(0xffffffffu, ok);
+      tc_fence_after_sync();
+      return all;
+    };
+    bool have = work.next(round, it);
+    float lse2 = 0.f, delta = 0.f;     // lse: +inf for rows past Sq -> P = 0
+    if (have) {
+      lse2 = p.lse[stat_of(it)];
+      delta = p.delta[stat_of(it)];
+    }
+    while (have && !aborted) {
+      BwdItem nx;
+      const bool have_nx = work.next(round, nx);
+      float lse2_nx = 0.f, delta_nx = 0.f;
+      if (have_nx) {      // in flight during this item
+        lse2_nx = p.lse[stat_of(nx)];
+        delta_nx = p.delta[stat_of(nx)];
+      }
+      const int q0 = it.tile * AB, qi = q0 + r, qpos = qi + off;
+      const float slope2 = GEN && p.alibi != nullptr ? p.alibi[it.head] * LOG2E : 0.f;
+      // scores of the 32 keys from k0 on -> probabilities, in place
+      auto probs = [&](uint32_t (&sv)[32], int k0, uint32_t bits) {
+        const bool need_mask = (k0 + 32 > p.Sk) || (p.causal && k0 + 31 > q0 + quad * 32 + off) ||
+                               (p.window >= 0 && k0 < q0 + quad * 32 + 31 + off - p.window);
+        // columns e (0..31) are alive for lo <= e <= hi
+        const int rel0 = k0 - qpos;
+        int hi = p.Sk - k0 - 1;
+        if (p.causal) hi = min(hi, -rel0);
+        const int lo = p.window >= 0 ? -rel0 - p.window : -(1 << 30);
+        if (!GEN) {
+          if (need_mask) {      // masked scores: -inf, probability 0
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+              if (e < lo || e > hi) sv[e] = __float_as_uint(p.scale_log2 < 0.f ? INFINITY : -INFINITY);
+          }
+          const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), nl2 = make_float2(-lse2, -lse2);
+#pragma unroll
+          for (int e = 0; e < 32; e += 2) {
+            const float2 x = ffma2(u2f2(sv[e], sv[e + 1]), sc2, nl2);
+            sv[e] = __float_as_uint(exp2f(x.x));
+            sv[e + 1] = __float_as_uint(exp2f(x.y));
+          }
+        } else {
+          const float bias0 = slope2 * static_cast<float>(rel0) - lse2;  // folded into the exponent
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            const float x = fmaf(__uint_as_float(sv[e]), p.scale_log2, fmaf(slope2, static_cast<float>(e), bias0));
+            float pr = exp2f(x);
+            if (e < lo || e > hi || !((bits >> ((k0 % AB + e) >> p.blk_shift)) & 1u)) pr = 0.f;
+            sv[e] = __float_as_uint(pr);
+          }
         }
-        uint32_t sv[32], dv[32];
-        tmem_ld_32x32b_x32(T_S + c * 32 + lane_off, sv);
-        tmem_ld_32x32b_x32(T_DP + c * 32 + lane_off, dv);
-        tmem_ld_wait();
+      };
+      // probabilities, dP -> dS (16 bit); the softmax scale is applied once, to dQ, when it is stored
+      auto grads = [&](const uint32_t (&pr)[32], uint32_t (&dv)[32], int k0, uint32_t (&pk)[16]) {
         if (DROP) {
           // dP of a dropped probability is zero, of a kept one it carries the 1 / (1 - p) factor
 #pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const int kk = k0 + c * 32 + j;
-            const uint32_t patch = dropout_patch(p.seed_lo, p.seed_hi, static_cast<uint32_t>(batch * p.H + head),
+          for (int e = 0; e < 32; e += 2) {
+            const int kk = k0 + e;
+            const uint32_t patch = dropout_patch(p.seed_lo, p.seed_hi, static_cast<uint32_t>(it.batch * p.H + it.head),
                                                  static_cast<uint32_t>(qi) >> 1, static_cast<uint32_t>(kk) >> 1);
-            dv[j] = dropout_keep(patch, qi, kk, p.drop_thr) ? __float_as_uint(__uint_as_float(dv[j]) * p.drop_rp) : 0u;
-            dv[j + 1] = dropout_keep(patch, qi, kk + 1, p.drop_thr)
-                            ? __float_as_uint(__uint_as_float(dv[j + 1]) * p.drop_rp) : 0u;
+            dv[e] = dropout_keep(patch, qi, kk, p.drop_thr) ? __float_as_uint(__uint_as_float(dv[e]) * p.drop_rp) : 0u;
+            dv[e + 1] = dropout_keep(patch, qi, kk + 1, p.drop_thr)
+                            ? __float_as_uint(__uint_as_float(dv[e + 1]) * p.drop_rp) : 0u;
           }
         }
-        uint32_t pk[16];
-        if (!GEN || (!need_mask && p.alibi == nullptr)) {
-          if (!GEN && need_mask) {      // masked scores: -inf, probability 0
+        const float2 nd2 = make_float2(-delta, -delta);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const int idx = c * 32 + j;
-              if (idx < lo || idx > hi) sv[j] = __float_as_uint(p.scale_log2 < 0.f ? INFINITY : -INFINITY);
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            // the softmax scale of dS is applied once, to dQ, in the epilogue
-            const float p0 = exp2f(fmaf(__uint_as_float(sv[j]), p.scale_log2, -lse2));
-            const float p1 = exp2f(fmaf(__uint_as_float(sv[j + 1]), p.scale_log2, -lse2));
-            pk[j >> 1] = pack_h16x2(p0 * (__uint_as_float(dv[j]) - delta),
-                                     p1 * (__uint_as_float(dv[j + 1]) - delta));
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            float ds[2];
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int idx = c * 32 + j + e;
-              float x = fmaf(__uint_as_float(sv[j + e]), p.scale_log2,
-                             fmaf(slope2, static_cast<float>(idx), bias0));
-              float pr = exp2f(x);
-              if (idx < lo || idx > hi || !((bits >> (idx >> p.blk_shift)) & 1u)) pr = 0.f;
-              ds[e] = pr * (__uint_as_float(dv[j + e]) - delta);
-            }
-            pk[j >> 1] = pack_h16x2(ds[0], ds[1]);
-          }
+        for (int e = 0; e < 32; e += 2) {
+          const float2 d = fmul2(u2f2(pr[e], pr[e + 1]), fadd2(u2f2(dv[e], dv[e + 1]), nd2));
+          pk[e >> 1] = pack_h16x2(d.x, d.y);
         }
-        if (PIPE) {
-          // dS_h sits at [384 + 32 h, ...): the chunk's 16 columns at 16 c (c = 2 h + half)
-          tmem_st_32x32b_x16(T_DS + c * 16 + lane_off, pk);
-          tmem_st_wait();
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar(DS_FULL, cc));
-        } else {
-          tmem_st_32x32b_x16(T_DS + st * 64 + c * 16 + lane_off, pk);
-        }
+      };
+      uint32_t sa[32], sb[32], dv[32], pk[16];
+      int j = next_live(work, it, it.j0);
+      const bool live = j < it.j1;
+      if (live) {
+        if (!wait(S_FULL, n & 1, (n >> 1) & 1, 38)) { aborted = true; break; }
+        tmem_ld_32x32b_x32(t_s + (n & 1) * AB, sa);
+        tmem_ld_wait_for(sa);
       }
-      if (aborted) break;
-      if (!PIPE) {
+      bool first = true;
+      while (j < it.j1) {
+        const int jn = next_live(work, it, j + 1), k0 = j * AB + c0;
+        const uint32_t t_sn = t_s + (n & 1) * AB;
+        uint32_t bits = 0xffffffffu;
+        if (GEN && p.blk_rows != nullptr) bits = qi < p.Sq ? p.blk_rows[static_cast<long long>(qi) * p.blk_nkt + j] : 0u;
+        tmem_ld_32x32b_x32(t_sn + 32, sb);      // in flight during the first chunk's exponentials
+        probs(sa, k0, bits);
+        tmem_ld_wait_for(sb);
+        if (!wait(DP_FULL, 0, n & 1, 44)) { aborted = true; break; }
+        tmem_ld_32x32b_x32(t_dp, dv);           // ... the second chunk's
+        probs(sb, k0 + 32, bits);
+        tmem_ld_wait_for(dv);
+        grads(sa, dv, k0, pk);
+        tmem_ld_32x32b_x32(t_dp + 32, dv);
+        tmem_st_32x32b_x16(t_sn, pk);
+        tmem_ld_wait_for(dv);
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(DP_EMPTY, 0));
+        if (jn < it.j1) {                       // the next block's first chunk
+          if (!wait(S_FULL, (n + 1) & 1, ((n + 1) >> 1) & 1, 38)) { aborted = true; break; }
+          tmem_ld_32x32b_x32(t_s + ((n + 1) & 1) * AB, sa);
+        }
+        grads(sb, dv, k0 + 32, pk);
+        tmem_st_32x32b_x16(t_sn + 16, pk);
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(bar(SDP_EMPTY, 0));
-          mbar_arrive(bar(DS_FULL, st));
-        }
+        if (lane == 0) mbar_arrive(bar(P_FULL, n & 1));
+        tmem_ld_wait_for(sa);
+        ++n;
+        j = jn;
+        // the former item's dQ
+        if (first && pending && !finish(done, true)) { aborted = true; break; }
+        first = false;
       }
-    }
-    if (!aborted && nlive > 0) {
-      if (PIPE ? !mbar_wait(bar(DQ_DONE, 0), 0, p.err, 40)
-               : !mbar_wait(bar(DQ_DONE, (nlive - 1) & 1), ((nlive - 1) >> 1) & 1, p.err, 40)) aborted = true;
-      tc_fence_after_sync();
-    }
-    if (!aborted) {
-      h16* orow = p.dq + batch * p.dq_sb + head * p.dq_sh + static_cast<long long>(qi) * p.dq_ss;
-#pragma unroll 1
-      for (int c = half * (DP / 32 / HALVES); c < (half + 1) * (DP / 32 / HALVES); ++c) {   // this warp's dQ columns
-        uint32_t ov[32];
-        if (nlive > 0) {  // warp-uniform: every lane takes part in the collective TMEM load
-          tmem_ld_32x32b_x32(T_DQ + c * 32 + lane_off, ov);
-          tmem_ld_wait();
+      if (!aborted) {
+        if (live) {
+          done = it;
+          pending = true;
         } else {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) ov[j] = 0u;
-        }
-        if (row_ok) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 8) {
-            if (c * 32 + j < p.D) {
-              const float sc = p.scale;
-              uint4 o4;
-              o4.x = pack_h16x2(__uint_as_float(ov[j]) * sc, __uint_as_float(ov[j + 1]) * sc);
-              o4.y = pack_h16x2(__uint_as_float(ov[j + 2]) * sc, __uint_as_float(ov[j + 3]) * sc);
-              o4.z = pack_h16x2(__uint_as_float(ov[j + 4]) * sc, __uint_as_float(ov[j + 5]) * sc);
-              o4.w = pack_h16x2(__uint_as_float(ov[j + 6]) * sc, __uint_as_float(ov[j + 7]) * sc);
-              *reinterpret_cast<uint4*>(orow + c * 32 + j) = o4;
-            }
-          }
+          finish(it, false);
         }
       }
+      it = nx;
+      have = have_nx;
+      lse2 = lse2_nx;
+      delta = delta_nx;
     }
+    if (!aborted && pending && !finish(done, true)) aborted = true;
   }
   __syncwarp();
   if (aborted) {
@@ -474,57 +657,32 @@ __global__ void __launch_bounds__(ab_threads(HALVES), 1)
 }
 
 // ------------------------------------------------------------------------------------------------
-// dK / dV kernel.  smem tiles: 0 = K, 1 = V, 2..3 = Q ring, 4..5 = dO ring.
-// TMEM: S^T [0,128) (P^T bf16 overwrites cols [0,64)), dP^T [128,256) (dS^T bf16 over [128,192)),
-//       dK [256,256+DP), dV [384,384+DP)
-// PIPE (default, eight element-wise warps): a step's 128 query columns are handled as two halves of 64 with their
-// own S^T / dP^T buffers (S^T_h at [64 h, 64 h + 64), dP^T_h at [128 + 64 h, ...)) and their own barriers.  The MMA
-// warp issues S^T / dP^T of half u + 1 before it waits for P^T / dS^T of half u, so the tensor core works on the
-// next half (and on dV / dK of the previous one) while the element-wise warps are busy with the current one;
-// without PIPE the four phases of a step run one after the other.  In the pipelined form a warp writes its 16-bit
-// results over the first half of the 32 columns it read itself (the MMA takes its A operand in pieces of 16 query rows,
-// each with its own column address), so the two warps of a quadrant never touch each other's columns and need no
-// barrier between reading and writing.
+// dK / dV kernel.  Resident: K, V (128 rows).  Streamed: Q, dO (64 rows) with their lse / delta.  Two sets of eight element-wise
+// warps (32 query columns each) take the blocks in turn, so that one set's waits lie under the other's arithmetic.
+// TMEM: S^T of block n at [64 (n & 1), ...), dP^T [128, 192), P^T [192, 224), dS^T [224, 256), dK [256, 256 + DP), dV [384, 384 +
+// DP).
 // ------------------------------------------------------------------------------------------------
-template <int DP, bool DROP, int HALVES, bool PIPE, bool GEN>
-__global__ void __launch_bounds__(ab_threads(HALVES), 1)
+template <int DP, bool DROP, bool GEN>
+__global__ void __launch_bounds__(DKV_THREADS, 1)
     attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                         const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                        const AttnBwdParams p) {
+                        const __grid_constant__ AttnBwdParams p) {
   using L = BwdSmem<DP>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sgen = smem_raw + (sbase - smem_u32(smem_raw));
   const uint32_t bar0 = sbase + L::BAR_OFF;
-  static_assert(!PIPE || HALVES == 2, "the pipelined form splits a half's 64 columns over two warps per quadrant");
-  enum { KV_FULL = 0, Q_FULL = 1, Q_EMPTY = 3, ST_FULL = 5, PT_FULL = 7, ACC_DONE = 9, NUSED = 10 };
   auto bar = [&](int which, int idx) { return bar0 + 8u * (which + idx); };
-  const uint32_t tmem_slot = bar0 + 8u * 23;
-  volatile uint32_t* tmem_slot_gen = reinterpret_cast<volatile uint32_t*>(sgen + L::BAR_OFF + 8 * 23);
-  auto tile = [&](int i) { return sbase + i * L::TILE; };
+  const uint32_t tmem_slot = bar0 + 8u * BWD_NBAR;
+  volatile uint32_t* tmem_slot_gen = reinterpret_cast<volatile uint32_t*>(sgen + L::BAR_OFF + 8 * BWD_NBAR);
+  auto res = [&](int which) { return sbase + which * (2 * L::T64); };
+  auto str = [&](int stage, int which) { return sbase + L::STR_OFF + (stage * 2 + which) * L::T64; };
+  constexpr uint32_t T_DP = 128, T_P = 192, T_DS = 224, T_DK = 256, T_DV = 384;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kt = blockIdx.x;
-  const int kv_head = blockIdx.y, batch = blockIdx.z;
-  const int group = p.H / p.Hk;
-  const int k0 = kt * AB;
   const int off = p.Sk - p.Sq;
-  // query rows that can see this key block: qpos >= k0 (causal), qpos <= k_last + window
-  int q_begin = 0, q_end = p.Sq;
-  if (p.causal) q_begin = max(0, k0 - off);
-  if (p.window >= 0) q_end = min(p.Sq, k0 + AB - 1 + p.window - off + 1);
-  const int ib = q_begin / AB;
-  const int nq = max((q_end + AB - 1) / AB - ib, 0);
-  const int nsteps = nq * group;
-  // block-sparse layouts: query tiles without a live block for this key tile are skipped by every role
-  auto step_live = [&](int t) {
-    return !GEN || p.blk_any == nullptr || p.blk_any[static_cast<long long>(ib + t % nq) * p.blk_nkt + kt] != 0;
-  };
-
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < NUSED; ++i) mbar_init(bar0 + 8u * i, (i == PT_FULL || i == PT_FULL + 1) ? 4 * HALVES : 1);
-    fence_barrier_init();
-  }
+  const DkvWork<GEN> work(p);
+  if (threadIdx.x == 0) bwd_init_barriers(bar0);
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
@@ -533,270 +691,304 @@ __global__ void __launch_bounds__(ab_threads(HALVES), 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot_gen;
-  const uint32_t T_ST = tmem, T_DPT = tmem + 128, T_DK = tmem + 256, T_DV = tmem + 384;
   bool aborted = false;
 
   if (warp == 0) {
-    if (elect_one() && nsteps > 0) {
-      mbar_expect_tx(bar(KV_FULL, 0), 2 * L::TILE);
-      load_tile<DP>(tile(0), &tmK, bar(KV_FULL, 0), k0, kv_head, batch);
-      load_tile<DP>(tile(1), &tmV, bar(KV_FULL, 0), k0, kv_head, batch);
-      for (int t = 0, n = 0; t < nsteps; ++t) {
-        if (!step_live(t)) continue;
-        const int st = n & 1;
-        const uint32_t ph = (n >> 1) & 1;
-        ++n;
-        const int head = kv_head * group + t / nq;
-        const int q0 = (ib + t % nq) * AB;
-        if (!mbar_wait(bar(Q_EMPTY, st), ph ^ 1, p.err, 51)) { aborted = true; break; }
-        mbar_expect_tx(bar(Q_FULL, st), 2 * L::TILE + 2 * AB * 4);
-        load_tile<DP>(tile(2 + st), &tmQ, bar(Q_FULL, st), q0, head, batch);
-        load_tile<DP>(tile(4 + st), &tmDO, bar(Q_FULL, st), q0, head, batch);
-        const long long stat0 = (static_cast<long long>(batch) * p.H + head) * p.Sq_pad + q0;
-        bulk_load_1d(sbase + L::VEC_OFF + st * (2 * AB * 4), p.lse + stat0, AB * 4, bar(Q_FULL, st));
-        bulk_load_1d(sbase + L::VEC_OFF + st * (2 * AB * 4) + AB * 4, p.delta + stat0, AB * 4,
-                     bar(Q_FULL, st));
+    if (elect_one()) {
+      int st = 0, t = 0, round = -1;
+      uint32_t ph = 0;
+      BwdItem it;
+      while (!aborted && work.next(round, it)) {
+        bool any = false;
+        int g = 0, ib = it.i0 - 1;
+        for (int j = 0; j < it.j1; ++j) {
+          if (++ib == it.i0 + it.n_i) {
+            ib = it.i0;
+            ++g;
+          }
+          if (!work.live(it, j)) continue;
+          const int q0 = ib * ABS, head = it.head * work.group + g;
+          if (!mbar_wait(bar(STR_EMPTY, st), ph ^ 1, p.err, 52)) { aborted = true; break; }
+          mbar_expect_tx(bar(STR_FULL, st), 2 * L::T64 + 2 * ABS * 4);
+          load_rows<DP, ABS>(str(st, 0), &tmQ, bar(STR_FULL, st), q0, head, it.batch);
+          load_rows<DP, ABS>(str(st, 1), &tmDO, bar(STR_FULL, st), q0, head, it.batch);
+          const long long stat0 = (static_cast<long long>(it.batch) * p.H + head) * p.Sq_pad + q0;
+          const uint32_t vec = sbase + L::VEC_OFF + st * (2 * ABS * 4);
+          bulk_load_1d(vec, p.lse + stat0, ABS * 4, bar(STR_FULL, st));
+          bulk_load_1d(vec + ABS * 4, p.delta + stat0, ABS * 4, bar(STR_FULL, st));
+          if (!any) {
+            for (int w = 0; w < 2; ++w) {
+              if (!mbar_wait(bar(RES_EMPTY, w), (t & 1) ^ 1, p.err, 51)) { aborted = true; break; }
+              mbar_expect_tx(bar(RES_FULL, w), 2 * L::T64);
+              load_rows<DP, AB>(res(w), w == 0 ? &tmK : &tmV, bar(RES_FULL, w), it.tile * AB, it.head, it.batch);
+            }
+            if (aborted) break;
+            any = true;
+            ++t;
+          }
+          if (++st == BWD_STAGES) {
+            st = 0;
+            ph ^= 1;
+          }
+        }
       }
     }
   } else if (warp == 1) {
-    if (elect_one() && nsteps > 0) {
-      if (!mbar_wait(bar(KV_FULL, 0), 0, p.err, 52)) aborted = true;
-      int n = 0;
-      if (PIPE) {
-        // sub-step u = 2 t + h of live step t: S^T_h = K Q_h^T, dP^T_h = V dO_h^T (64 query rows), later
-        // dV += P^T_h dO_h, dK += dS^T_h Q_h
-        int nl = 0;
-        for (int tt = 0; tt < nsteps; ++tt) nl += step_live(tt) ? 1 : 0;
-        auto issue_m1 = [&](int u) -> bool {
-          const int t = u >> 1, h = u & 1, st = t & 1;
-          if (h == 0 && !mbar_wait(bar(Q_FULL, st), (t >> 1) & 1, p.err, 53)) return false;
-          tc_fence_after_sync();
-          mma_nt<DP, 64>(T_ST + h * 64, tile(0), tile(2 + st) + h * (64 * 128));
-          mma_nt<DP, 64>(T_DPT + h * 64, tile(1), tile(4 + st) + h * (64 * 128));
-          umma_commit(bar(ST_FULL, h));
-          return true;
-        };
-        const int nsub = 2 * nl;
-        if (!aborted && nsub > 0 && !issue_m1(0)) aborted = true;
-        for (int u = 0; u < nsub && !aborted; ++u) {
-          const int t = u >> 1, h = u & 1, st = t & 1;
-          if (u + 1 < nsub && !issue_m1(u + 1)) { aborted = true; break; }
-          if (!mbar_wait(bar(PT_FULL, h), t & 1, p.err, 54)) { aborted = true; break; }
-          tc_fence_after_sync();
-          mma_ts<DP, 64, true>(T_DV, T_ST + h * 64, tile(4 + st) + h * (64 * 128), u != 0);    // dV += P^T_h dO_h
-          mma_ts<DP, 64, true>(T_DK, T_DPT + h * 64, tile(2 + st) + h * (64 * 128), u != 0);   // dK += dS^T_h Q_h
-          if (h == 1) umma_commit(bar(Q_EMPTY, st));
+    // S^T = K Q^T, dP^T = V dO^T
+    const uint32_t leader = elect_one() ? 1u : 0u;
+    int n = 0, t = 0, round = -1, st = 0;
+    uint32_t ph = 0;
+    BwdItem it;
+    while (!aborted && work.next(round, it)) {
+      bool any = false;
+      for (int j = 0; j < it.j1; ++j) {
+        if (!work.live(it, j)) continue;
+        const bool last = next_live(work, it, j + 1) >= it.j1;
+        if ((!any && !warp_wait(bar(RES_FULL, 0), t & 1, p.err, 53)) || !warp_wait(bar(STR_FULL, st), ph, p.err, 54) ||
+            !warp_wait(bar(S_EMPTY, n & 1), ((n >> 1) & 1) ^ 1, p.err, 60)) {
+          aborted = true;
+          break;
         }
-        n = nl;
-      }
-      for (int tt = 0; !PIPE && tt < nsteps && !aborted; ++tt) {
-        if (!step_live(tt)) continue;
-        const int t = n++;          // live steps: ring stages, barrier phases and the accumulate flags count these
-        const int st = t & 1;
-        if (!mbar_wait(bar(Q_FULL, st), (t >> 1) & 1, p.err, 53)) { aborted = true; break; }
         tc_fence_after_sync();
-        mma_nt<DP>(T_ST, tile(0), tile(2 + st));   // S^T  = K Q^T
-        mma_nt<DP>(T_DPT, tile(1), tile(4 + st));  // dP^T = V dO^T
-        umma_commit(bar(ST_FULL, 0));
-        if (!mbar_wait(bar(PT_FULL, 0), t & 1, p.err, 54)) { aborted = true; break; }
+        mma_nt<DP, ABS>(leader, tmem + (n & 1) * ABS, res(0), str(st, 0));
+        umma_commit_by(leader, bar(S_FULL, n & 1));
+        if (last) umma_commit_by(leader, bar(RES_EMPTY, 0));
+        if ((!any && !warp_wait(bar(RES_FULL, 1), t & 1, p.err, 64)) ||
+            !warp_wait(bar(DP_EMPTY, 0), (n & 1) ^ 1, p.err, 62)) {
+          aborted = true;
+          break;
+        }
         tc_fence_after_sync();
-        mma_ts<DP>(T_DV, T_ST, tile(4 + st), t != 0);   // dV += P^T dO
-        mma_ts<DP>(T_DK, T_DPT, tile(2 + st), t != 0);  // dK += dS^T Q
-        umma_commit(bar(Q_EMPTY, st));
+        mma_nt<DP, ABS>(leader, tmem + T_DP, res(1), str(st, 1));
+        umma_commit_by(leader, bar(DP_FULL, n & 1));
+        if (last) umma_commit_by(leader, bar(RES_EMPTY, 1));
+        any = true;
+        ++n;
+        if (++st == BWD_STAGES) {
+          st = 0;
+          ph ^= 1;
+        }
       }
-      if (!aborted && n > 0) umma_commit(bar(ACC_DONE, 0));
+      t += any;
     }
-  } else {
-    const int quad = warp & 3;
-    const int half = (warp - 2) >> 2;   // which 64 of the 128 query columns of a step (and which half of dK / dV)
-    const int r = quad * 32 + lane;  // key row in tile
+  } else if (warp == 2) {
+    // dV += P^T dO, dK += dS^T Q
+    const uint32_t leader = elect_one() ? 1u : 0u;
+    int n = 0, t = 0, round = -1, st = 0;
+    BwdItem it;
+    while (!aborted && work.next(round, it)) {
+      bool any = false;
+      for (int j = 0; j < it.j1; ++j) {
+        if (!work.live(it, j)) continue;
+        const int h = n & 1;
+        if ((!any && !warp_wait(bar(ACC_EMPTY, 0), (t & 1) ^ 1, p.err, 55)) ||
+            !warp_wait(bar(P_FULL, h), (n >> 1) & 1, p.err, 56)) {
+          aborted = true;
+          break;
+        }
+        tc_fence_after_sync();
+        mma_ts<DP, ABS>(leader, tmem + T_DV, tmem + T_P, 16, str(st, 1), any);
+        mma_ts<DP, ABS>(leader, tmem + T_DK, tmem + T_DS, 16, str(st, 0), any);
+        umma_commit_by(leader, bar(STR_EMPTY, st));
+        any = true;
+        ++n;
+        if (++st == BWD_STAGES) st = 0;
+      }
+      if (any) {
+        umma_commit_by(leader, bar(ACC_FULL, 0));
+        ++t;
+      }
+    }
+  } else if (warp >= 4) {
+    // ------------------------------------------------------------------ element-wise sets
+    const int quad = warp & 3, h = (warp - 4) >> 3, half = (warp >> 2) & 1;
+    const int r = quad * 32 + lane, c0 = half * 32;      // key row in tile; first of this warp's 32 query columns of a block
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-    const int kcol = k0 + r;
-    const bool key_ok = kcol < p.Sk;
-    int nlive = 0;
-    for (int tt = 0; tt < nsteps; ++tt) {
-      if (!step_live(tt)) continue;
-      const int t = nlive++;
-      const int head = kv_head * group + tt / nq;
-      const int q0 = (ib + tt % nq) * AB;
-      const float slope2 = GEN && p.alibi != nullptr ? p.alibi[head] * LOG2E : 0.f;
-      const int st = t & 1;
-      // lse / delta of this query block were bulk-copied next to the Q / dO tiles
-      bool ok = mbar_wait(bar(Q_FULL, st), (t >> 1) & 1, p.err, 57);
-      const float4* v_lse = reinterpret_cast<const float4*>(sgen + L::VEC_OFF + st * (2 * AB * 4));
-      const float4* v_del = v_lse + AB / 4;
-      if (!PIPE) {
-        if (ok) ok = mbar_wait(bar(ST_FULL, 0), t & 1, p.err, 55);
-        // the two warps of a quadrant meet at a named barrier further down: they must take the same decision here
-        // (a wait that ran out on one of them ends the loop for both)
-        if (HALVES == 2 ? !pair_all(ok, 5 + quad) : !ok) { aborted = true; break; }
-        tc_fence_after_sync();
-      }
-      // query columns qq (0..127) of this block are alive for lo <= qq <= hi
-      const int rel0 = kcol - q0 - off;  // key position minus position of query column 0
-      int lo = p.causal ? rel0 : -(1 << 30);
-      int hi = p.window >= 0 ? rel0 + p.window : (1 << 30);
-      if (!key_ok) hi = -(1 << 30);
-      const bool need_mask = __any_sync(0xffffffffu, lo > 0 || hi < AB - 1) || (GEN && p.blk_rows != nullptr);
-      const float bias0 = slope2 * static_cast<float>(rel0);
-      const uint32_t kbit = 1u << (r >> p.blk_shift);      // this key row's sub-block within the key tile
-      const bool plain = !GEN || (!need_mask && p.alibi == nullptr);   // warp-uniform: no per-element compares in the hot path
-      // P^T and dS^T (16 bit) go over the columns S^T and dP^T were read from, and the partner warp of this
-      // quadrant reads the other half of those columns: both chunks of this warp are kept in registers until the
-      // two warps have finished reading (named barrier of the quadrant's 64 threads), then everything is stored.
-      // (With four warps a thread takes all four chunks, two at a time; its own earlier stores never reach columns
-      //  it has yet to read.)
-      // PIPE: two passes (the halves of the step), one 32-column chunk per warp and pass, each pass with its own
-      // S^T / dP^T buffer and barriers; otherwise 2 / HALVES passes over two chunks each in the one buffer.
-      constexpr int NGRP = PIPE ? 2 : 2 / HALVES;
-      constexpr int NCC = PIPE ? 1 : 2;
-#pragma unroll 1
-      for (int grp = 0; grp < NGRP; ++grp) {
-      const int cbase = PIPE ? grp * 2 + half : (half * (2 / HALVES) + grp) * 2;
-      // where this pass's chunks sit in TMEM: columns of the S^T buffer read / of the 16-bit result written
-      const uint32_t rd0 = PIPE ? grp * 64 + half * 32 : cbase * 32;
-      const uint32_t wr0 = PIPE ? rd0 : cbase * 16;
-      if (PIPE) {
-        if (ok) ok = mbar_wait(bar(ST_FULL, grp), t & 1, p.err, 55);
-        if (!__all_sync(0xffffffffu, ok)) { aborted = true; break; }
-        tc_fence_after_sync();
-      }
-      uint32_t pp_all[NCC][16], pd_all[NCC][16];
+    const uint32_t t_s = tmem + h * ABS + c0 + lane_off, t_dp = tmem + T_DP + c0 + lane_off,
+                   t_p = tmem + T_P + c0 / 2 + lane_off, t_ds = t_p + (T_DS - T_P);
+    int n = 0, round = -1, t = 0, st = 0;
+    uint32_t ph = 0;
+    BwdItem it;
+    bool pending = false;      // `done`: an item whose gradients this warp has still to store (set 0 stores)
+    BwdItem done;
+    const bool stores = half * 64 < DP;      // (64 columns of dK and of dV per warp; dK carries the softmax scale of dS)
+    auto finish = [&](const BwdItem& i, bool live) -> bool {
+      uint32_t lo[32], hi[32];
 #pragma unroll
-      for (int cc = 0; cc < NCC; ++cc) {
-        const int c = cbase + cc;
-        uint32_t (&pp)[16] = pp_all[cc];
-        uint32_t (&pd)[16] = pd_all[cc];
-        uint32_t sv[32], dv[32];
-        tmem_ld_32x32b_x32(T_ST + rd0 + cc * 32 + lane_off, sv);
-        tmem_ld_32x32b_x32(T_DPT + rd0 + cc * 32 + lane_off, dv);
-        tmem_ld_wait();
-        float keepf[32];      // DROP: 0 or 1 / (1 - p) per query column of this chunk (unused otherwise)
+      for (int e = 0; e < 32; ++e) lo[e] = hi[e] = 0u;
+      if (live) {
+        const bool ok = mbar_wait(bar(ACC_FULL, 0), t & 1, p.err, 59);
+        if (!__all_sync(0xffffffffu, ok)) return false;
+        tc_fence_after_sync();
+        if (stores) bwd_acc_load(tmem + T_DK + half * 64 + lane_off, lo, hi);
+      }
+      const int row = i.tile * AB + quad * 32;
+      if (stores)
+        bwd_store(p.dk + i.batch * p.dk_sb + i.head * p.dk_sh, p.dk_ss, lo, hi, p.scale, half * 64, row, p.Sk, p.D);
+      if (live) {
+        if (stores) bwd_acc_load(tmem + T_DV + half * 64 + lane_off, lo, hi);
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(ACC_EMPTY, 0));
+        ++t;
+      }
+      if (stores)
+        bwd_store(p.dv + i.batch * p.dv_sb + i.head * p.dv_sh, p.dv_ss, lo, hi, 1.f, half * 64, row, p.Sk, p.D);
+      return true;
+    };
+    auto wait = [&](int which, int idx, uint32_t parity, int where) -> bool {
+      const bool ok = mbar_wait(bar(which, idx), parity, p.err, where);
+      const bool all = __all_sync(0xffffffffu, ok);
+      tc_fence_after_sync();
+      return all;
+    };
+    while (!aborted && work.next(round, it)) {
+      const int kcol = it.tile * AB + r;
+      const bool key_ok = kcol < p.Sk;
+      const uint32_t kbit = 1u << (r >> p.blk_shift);      // this key row's sub-block within the key tile
+      bool first = true;
+      int g = 0, ib = it.i0 - 1;
+      for (int j = 0; j < it.j1; ++j) {
+        if (++ib == it.i0 + it.n_i) {
+          ib = it.i0;
+          ++g;
+        }
+        if (!work.live(it, j)) continue;
+        const int i = n++, cur = st;
+        const uint32_t cur_ph = ph;
+        if (++st == BWD_STAGES) {
+          st = 0;
+          ph ^= 1;
+        }
+        // the former item's gradients: before this item's first block where the other set has it, else after it
+        const bool store_former = first && pending;
+        first = false;
+        if ((i & 1) != h) {
+          if (store_former && !finish(done, true)) { aborted = true; break; }
+          continue;
+        }
+        const int q0 = ib * ABS + c0, head = it.head * work.group + g;      // this warp's first query row
+        const float slope2 = GEN && p.alibi != nullptr ? p.alibi[head] * LOG2E : 0.f;
+        // this warp's query columns e (0..31) are alive for lo <= e <= hi
+        const int rel0 = kcol - q0 - off;  // key position minus position of query column 0
+        const int lo = p.causal ? rel0 : -(1 << 30);
+        int hi = p.window >= 0 ? rel0 + p.window : (1 << 30);
+        if (!key_ok) hi = -(1 << 30);
+        const bool need_mask = __any_sync(0xffffffffu, lo > 0 || hi < 31) || (GEN && p.blk_rows != nullptr);
+        const uint32_t par = (i >> 1) & 1;
+        // (lse / delta of a query block were bulk-copied next to the Q / dO tiles)
+        const float4* v_lse = reinterpret_cast<const float4*>(sgen + L::VEC_OFF + cur * (2 * ABS * 4)) + c0 / 4;
+        const float4* v_del = v_lse + ABS / 4;
+        uint32_t sv[32], dv[32], pk[16];
+        if (!wait(STR_FULL, cur, cur_ph, 57) || !wait(S_FULL, h, par, 58)) { aborted = true; break; }
+        tmem_ld_32x32b_x32(t_s, sv);
+        tmem_ld_wait_for(sv);
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(S_EMPTY, h));
+        // probabilities, in place; dV takes them rounded (and dropped)
+        if (!GEN && need_mask) {      // masked scores: -inf, probability 0
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (e < lo || e > hi) sv[e] = __float_as_uint(p.scale_log2 < 0.f ? INFINITY : -INFINITY);
+        }
+        auto probs = [&](int first_e) {
+          if (!GEN) {
+            const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
+#pragma unroll
+            for (int z = 0; z < 16; z += 4) {
+              const int e = first_e + z;
+              const float4 l4 = v_lse[e >> 2];
+              const float2 x0 = ffma2(u2f2(sv[e], sv[e + 1]), sc2, make_float2(-l4.x, -l4.y));
+              const float2 x1 = ffma2(u2f2(sv[e + 2], sv[e + 3]), sc2, make_float2(-l4.z, -l4.w));
+              const float p0 = exp2f(x0.x), p1 = exp2f(x0.y), p2 = exp2f(x1.x), p3 = exp2f(x1.y);
+              pk[e >> 1] = pack_h16x2(p0, p1);
+              pk[(e >> 1) + 1] = pack_h16x2(p2, p3);
+              sv[e] = __float_as_uint(p0); sv[e + 1] = __float_as_uint(p1);
+              sv[e + 2] = __float_as_uint(p2); sv[e + 3] = __float_as_uint(p3);
+            }
+          } else {
+            const float bias0 = slope2 * static_cast<float>(rel0);
+#pragma unroll
+            for (int z = 0; z < 16; z += 4) {
+              const int e0 = first_e + z;
+              const float4 l4 = v_lse[e0 >> 2];
+              const float lq[4] = {l4.x, l4.y, l4.z, l4.w};
+              float kept[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const int idx = e0 + e, qq = q0 + idx;
+                float x = fmaf(__uint_as_float(sv[idx]), p.scale_log2, -lq[e]);
+                if (p.alibi != nullptr) x += fmaf(-slope2, static_cast<float>(idx), bias0);
+                float pr = exp2f(x);
+                if (need_mask) {
+                  if (idx < lo || idx > hi) pr = 0.f;
+                  if (p.blk_rows != nullptr &&       // the layout byte of query row qq (the same for the whole warp)
+                      !(p.blk_rows[static_cast<long long>(min(qq, p.Sq - 1)) * p.blk_nkt + it.tile] & kbit)) pr = 0.f;
+                }
+                sv[idx] = __float_as_uint(pr);
+                kept[e] = pr;
+                if (DROP) {
+                  const uint32_t patch = dropout_patch(p.seed_lo, p.seed_hi, static_cast<uint32_t>(it.batch * p.H + head),
+                                                       static_cast<uint32_t>(qq) >> 1, static_cast<uint32_t>(kcol) >> 1);
+                  kept[e] *= dropout_keep(patch, qq, kcol, p.drop_thr) ? p.drop_rp : 0.f;
+                }
+              }
+              pk[e0 >> 1] = pack_h16x2(kept[0], kept[1]);
+              pk[(e0 >> 1) + 1] = pack_h16x2(kept[2], kept[3]);
+            }
+          }
+        };
+        probs(0);
+        if (!wait(DP_FULL, h, par, 63)) { aborted = true; break; }
+        tmem_ld_32x32b_x32(t_dp, dv);           // in flight during the second half's exponentials
+        probs(16);
+        tmem_ld_wait_for(dv);
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(DP_EMPTY, 0));
         if (DROP) {
 #pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const int qq = q0 + c * 32 + j;
-            const uint32_t patch = dropout_patch(p.seed_lo, p.seed_hi, static_cast<uint32_t>(batch * p.H + head),
+          for (int e = 0; e < 32; ++e) {
+            const int qq = q0 + e;
+            const uint32_t patch = dropout_patch(p.seed_lo, p.seed_hi, static_cast<uint32_t>(it.batch * p.H + head),
                                                  static_cast<uint32_t>(qq) >> 1, static_cast<uint32_t>(kcol) >> 1);
-            keepf[j] = dropout_keep(patch, qq, kcol, p.drop_thr) ? p.drop_rp : 0.f;
-            keepf[j + 1] = dropout_keep(patch, qq + 1, kcol, p.drop_thr) ? p.drop_rp : 0.f;
+            dv[e] = __float_as_uint(__uint_as_float(dv[e]) * (dropout_keep(patch, qq, kcol, p.drop_thr) ? p.drop_rp : 0.f));
           }
         }
-        if (plain) {
-          if (!GEN && need_mask) {      // masked scores: -inf, probability 0
+        uint32_t pd[16];
+        const float2 m1 = make_float2(-1.f, -1.f);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const int idx = c * 32 + j;
-              if (idx < lo || idx > hi) sv[j] = __float_as_uint(p.scale_log2 < 0.f ? INFINITY : -INFINITY);
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            const float4 l4 = v_lse[(c * 32 + j) >> 2];
-            const float4 d4 = v_del[(c * 32 + j) >> 2];
-            const float lq[4] = {l4.x, l4.y, l4.z, l4.w}, dq_[4] = {d4.x, d4.y, d4.z, d4.w};
-            float pr[4], ds[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              pr[e] = exp2f(fmaf(__uint_as_float(sv[j + e]), p.scale_log2, -lq[e]));
-              const float dpe = DROP ? __uint_as_float(dv[j + e]) * keepf[j + e] : __uint_as_float(dv[j + e]);
-              ds[e] = pr[e] * (dpe - dq_[e]);     // softmax scale: once, on dK, in the epilogue
-              if (DROP) pr[e] *= keepf[j + e];    // dV takes the dropped probabilities
-            }
-            pp[j >> 1] = pack_h16x2(pr[0], pr[1]);
-            pp[(j >> 1) + 1] = pack_h16x2(pr[2], pr[3]);
-            pd[j >> 1] = pack_h16x2(ds[0], ds[1]);
-            pd[(j >> 1) + 1] = pack_h16x2(ds[2], ds[3]);
-          }
+        for (int e = 0; e < 32; e += 4) {      // softmax scale: once, on dK, when it is stored
+          const float4 d4 = v_del[e >> 2];
+          const float2 s0 = fmul2(u2f2(sv[e], sv[e + 1]), ffma2(make_float2(d4.x, d4.y), m1, u2f2(dv[e], dv[e + 1])));
+          const float2 s1 = fmul2(u2f2(sv[e + 2], sv[e + 3]), ffma2(make_float2(d4.z, d4.w), m1, u2f2(dv[e + 2], dv[e + 3])));
+          pd[e >> 1] = pack_h16x2(s0.x, s0.y);
+          pd[(e >> 1) + 1] = pack_h16x2(s1.x, s1.y);
+        }
+        // the products have taken block i - 1's results (its stage, one back in the ring, and the phase of that use)
+        if (i > 0 && !wait(STR_EMPTY, cur == 0 ? BWD_STAGES - 1 : cur - 1, cur == 0 ? cur_ph ^ 1 : cur_ph, 61)) {
+          aborted = true;
+          break;
+        }
+        tmem_st_32x32b_x16(t_p, pk);
+        tmem_st_32x32b_x16(t_ds, pd);
+        tmem_st_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(P_FULL, h));
+        if (store_former && !finish(done, true)) { aborted = true; break; }
+      }
+      if (!aborted && h == 0) {
+        if (!first) {
+          done = it;
+          pending = true;
         } else {
-#pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            const float4 l4 = v_lse[(c * 32 + j) >> 2];
-            const float4 d4 = v_del[(c * 32 + j) >> 2];
-            const float lq[4] = {l4.x, l4.y, l4.z, l4.w}, dq_[4] = {d4.x, d4.y, d4.z, d4.w};
-            float pr[4], ds[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const int idx = c * 32 + j + e;
-              float x = fmaf(__uint_as_float(sv[j + e]), p.scale_log2, -lq[e]);
-              if (p.alibi != nullptr) x += fmaf(-slope2, static_cast<float>(idx), bias0);
-              pr[e] = exp2f(x);
-              if (idx < lo || idx > hi) pr[e] = 0.f;
-              if (p.blk_rows != nullptr) {   // the layout byte of query row q0 + idx (the same for the whole warp)
-                const int qq = min(q0 + idx, p.Sq - 1);
-                if (!(p.blk_rows[static_cast<long long>(qq) * p.blk_nkt + kt] & kbit)) pr[e] = 0.f;
-              }
-              const float dpe = DROP ? __uint_as_float(dv[j + e]) * keepf[j + e] : __uint_as_float(dv[j + e]);
-              ds[e] = pr[e] * (dpe - dq_[e]);
-              if (DROP) pr[e] *= keepf[j + e];
-            }
-            pp[j >> 1] = pack_h16x2(pr[0], pr[1]);
-            pp[(j >> 1) + 1] = pack_h16x2(pr[2], pr[3]);
-            pd[j >> 1] = pack_h16x2(ds[0], ds[1]);
-            pd[(j >> 1) + 1] = pack_h16x2(ds[2], ds[3]);
-          }
-        }
-      }
-      if (HALVES == 2 && !PIPE) asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory");
-#pragma unroll
-      for (int cc = 0; cc < NCC; ++cc) {
-        tmem_st_32x32b_x16(T_ST + wr0 + cc * 16 + lane_off, pp_all[cc]);
-        tmem_st_32x32b_x16(T_DPT + wr0 + cc * 16 + lane_off, pd_all[cc]);
-      }
-      if (PIPE) {
-        tmem_st_wait();
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(PT_FULL, grp));
-      }
-      }
-      if (aborted) break;
-      if (!PIPE) {
-        tmem_st_wait();
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(PT_FULL, 0));
-      }
-    }
-    if (!aborted && nlive > 0) {
-      if (!mbar_wait(bar(ACC_DONE, 0), 0, p.err, 56)) aborted = true;
-      tc_fence_after_sync();
-    }
-    if (!aborted) {
-#pragma unroll 1
-      for (int which = 0; which < 2; ++which) {
-        const uint32_t T = which == 0 ? T_DK : T_DV;
-        h16* base = which == 0 ? p.dk : p.dv;
-        const long long sb = which == 0 ? p.dk_sb : p.dv_sb, sh = which == 0 ? p.dk_sh : p.dv_sh,
-                        ss = which == 0 ? p.dk_ss : p.dv_ss;
-        h16* orow = base + batch * sb + kv_head * sh + static_cast<long long>(kcol) * ss;
-#pragma unroll 1
-        for (int c = half * (DP / 32 / HALVES); c < (half + 1) * (DP / 32 / HALVES); ++c) {   // this warp's columns
-          uint32_t ov[32];
-          if (nlive > 0) {
-            tmem_ld_32x32b_x32(T + c * 32 + lane_off, ov);
-            tmem_ld_wait();
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) ov[j] = 0u;
-          }
-          if (key_ok) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              if (c * 32 + j < p.D) {
-                const float sc = which == 0 ? p.scale : 1.f;     // dK carries the softmax scale of dS
-                uint4 o4;
-                o4.x = pack_h16x2(__uint_as_float(ov[j]) * sc, __uint_as_float(ov[j + 1]) * sc);
-                o4.y = pack_h16x2(__uint_as_float(ov[j + 2]) * sc, __uint_as_float(ov[j + 3]) * sc);
-                o4.z = pack_h16x2(__uint_as_float(ov[j + 4]) * sc, __uint_as_float(ov[j + 5]) * sc);
-                o4.w = pack_h16x2(__uint_as_float(ov[j + 6]) * sc, __uint_as_float(ov[j + 7]) * sc);
-                *reinterpret_cast<uint4*>(orow + c * 32 + j) = o4;
-              }
-            }
-          }
+          finish(it, false);
         }
       }
     }
+    if (!aborted && pending && !finish(done, true)) aborted = true;
   }
   __syncwarp();
   if (aborted) {
@@ -814,54 +1006,42 @@ static bool bwd_map(CUtensorMap* m, const void* base, int B, int Hh, int S, int 
                     long long sh, long long ss) {
   const uint64_t dims[4] = {(uint64_t)D, (uint64_t)S, (uint64_t)Hh, (uint64_t)B};
   const uint64_t strides[3] = {(uint64_t)ss * 2, (uint64_t)sh * 2, (uint64_t)sb * 2};
-  const uint32_t box[4] = {64, AB, 1, 1};
+  const uint32_t box[4] = {64, ABS, 1, 1};
   return make_tma_4d(m, base, dims, strides, box, 2, true);
 }
 
-template <int DP, bool DROP, int HALVES, bool PIPE_Q, bool PIPE_K, bool GEN>
-static int launch_bwd_as(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-                         const AttnBwdParams& p, cudaStream_t s) {
-  auto dq = attn_bwd_dq_kernel<DP, DROP, HALVES, PIPE_Q, GEN>;
-  auto dkv = attn_bwd_dkv_kernel<DP, DROP, HALVES, PIPE_K, GEN>;
+struct BwdMaps {
+  CUtensorMap q, k, v, d_o;
+};
+
+template <int DP, bool DROP, bool GEN>
+static int launch_bwd_as(const BwdMaps& m, const AttnBwdParams& p, cudaStream_t s) {
+  auto dq = attn_bwd_dq_kernel<DP, DROP, GEN>;
+  auto dkv = attn_bwd_dkv_kernel<DP, DROP, GEN>;
   static bool cfg = false;
   if (!cfg) {
     NX_CUDA_CHECK(cudaFuncSetAttribute(dq, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<DP>::DYN));
     NX_CUDA_CHECK(cudaFuncSetAttribute(dkv, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<DP>::DYN));
     cfg = true;
   }
-  dq<<<dim3((p.Sq + AB - 1) / AB, p.H, p.B), ab_threads(HALVES), BwdSmem<DP>::DYN, s>>>(tq, tk, tv, tdo, p);
+  const long long nq = static_cast<long long>((p.Sq + AB - 1) / AB) * p.H * p.B;
+  const long long nk = static_cast<long long>((p.Sk + AB - 1) / AB) * p.Hk * p.B;
+  NX_REQUIRE(nq < (1ll << 30) && nk < (1ll << 30), "flash_attn_bwd: too many tiles");
+  dq<<<static_cast<unsigned>(min(nq, static_cast<long long>(sm_count()))), DQ_THREADS, BwdSmem<DP>::DYN, s>>>(m.q, m.k, m.v, m.d_o, p);
   NX_LAUNCH_CHECK();
-  dkv<<<dim3((p.Sk + AB - 1) / AB, p.Hk, p.B), ab_threads(HALVES), BwdSmem<DP>::DYN, s>>>(tq, tk, tv, tdo, p);
+  dkv<<<static_cast<unsigned>(min(nk, static_cast<long long>(sm_count()))), DKV_THREADS, BwdSmem<DP>::DYN, s>>>(m.q, m.k, m.v, m.d_o, p);
   NX_LAUNCH_CHECK();
   return NX_OK;
 }
 
-template <int DP, bool DROP, int HALVES>
-static int launch_bwd_h(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                      const CUtensorMap& tdo, const AttnBwdParams& p, cudaStream_t s) {
-  constexpr bool PIPE = HALVES == 2;
-  auto off = [](const char* name) {
-    const char* e = getenv(name);
-    return e != nullptr && atoi(e) == 0;
-  };
-  static const bool serial_q = off("NEOX_ATTN_DQ_PIPE"), serial_k = off("NEOX_ATTN_DKV_PIPE");   // =0: unpipelined
-  if (PIPE && serial_q && serial_k) return launch_bwd_as<DP, DROP, HALVES, false, false, true>(tq, tk, tv, tdo, p, s);
-  if (PIPE && serial_q) return launch_bwd_as<DP, DROP, HALVES, false, PIPE, true>(tq, tk, tv, tdo, p, s);
-  if (PIPE && serial_k) return launch_bwd_as<DP, DROP, HALVES, PIPE, false, true>(tq, tk, tv, tdo, p, s);
-  // (a zero scale would turn a masked score into NaN)
-  if (!PIPE || DROP || p.alibi != nullptr || p.blk_rows != nullptr || p.scale == 0.f)
-    return launch_bwd_as<DP, DROP, HALVES, PIPE, PIPE, true>(tq, tk, tv, tdo, p, s);
-  return launch_bwd_as<DP, DROP, HALVES, PIPE, PIPE, false>(tq, tk, tv, tdo, p, s);
-}
-
 template <int DP, bool DROP>
-static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-                      const CUtensorMap& tdo, const AttnBwdParams& p, cudaStream_t s) {
-  static const bool four = [] {
-    const char* e = getenv("NEOX_ATTN_BWD_WARPS");
-    return e != nullptr && atoi(e) == 4;
-  }();
-  return four ? launch_bwd_h<DP, DROP, 1>(tq, tk, tv, tdo, p, s) : launch_bwd_h<DP, DROP, 2>(tq, tk, tv, tdo, p, s);
+static int launch_bwd(const BwdMaps& m, const AttnBwdParams& p, cudaStream_t s) {
+  // (a zero scale would turn a masked score into NaN)
+  if constexpr (!DROP) {
+    if (p.alibi == nullptr && p.blk_rows == nullptr && p.scale != 0.f)
+      return launch_bwd_as<DP, false, false>(m, p, s);
+  }
+  return launch_bwd_as<DP, DROP, true>(m, p, s);
 }
 
 }  // namespace nx
@@ -909,11 +1089,10 @@ NX_API int NX_SYM(nx_flash_attn_bwd)(const void* q, const void* k, const void* v
     else run(attn_delta_kernel<16>, 16 * DELTA_ROWS);
     NX_LAUNCH_CHECK();
   }
-  CUtensorMap tq, tk, tv, tdo;
-  if (!bwd_map(&tq, q, B, H, Sq, D, q_sb, q_sh, q_ss)) return NX_ERR_ARG;
-  if (!bwd_map(&tk, k, B, Hk, Sk, D, k_sb, k_sh, k_ss)) return NX_ERR_ARG;
-  if (!bwd_map(&tv, v, B, Hk, Sk, D, v_sb, v_sh, v_ss)) return NX_ERR_ARG;
-  if (!bwd_map(&tdo, dO, B, H, Sq, D, do_sb, do_sh, do_ss)) return NX_ERR_ARG;
+  BwdMaps m;
+  if (!bwd_map(&m.q, q, B, H, Sq, D, q_sb, q_sh, q_ss) || !bwd_map(&m.k, k, B, Hk, Sk, D, k_sb, k_sh, k_ss) ||
+      !bwd_map(&m.v, v, B, Hk, Sk, D, v_sb, v_sh, v_ss) || !bwd_map(&m.d_o, dO, B, H, Sq, D, do_sb, do_sh, do_ss))
+    return NX_ERR_ARG;
   AttnBwdParams p;
   p.lse = (const float*)lse; p.delta = (const float*)delta; p.alibi = (const float*)alibi;
   p.dq = (h16*)dq; p.dk = (h16*)dk; p.dv = (h16*)dv;
@@ -934,7 +1113,7 @@ NX_API int NX_SYM(nx_flash_attn_bwd)(const void* q, const void* k, const void* v
   p.blk_any = static_cast<const uint8_t*>(blk_any);
   p.blk_nkt = (Sk + AB - 1) / AB;
   p.blk_shift = blk_size == 16 ? 4 : blk_size == 32 ? 5 : blk_size == 64 ? 6 : 7;
-  if (p.drop_thr > 0u) return D <= 64 ? launch_bwd<64, true>(tq, tk, tv, tdo, p, s) : launch_bwd<128, true>(tq, tk, tv, tdo, p, s);
-  if (D <= 64) return launch_bwd<64, false>(tq, tk, tv, tdo, p, s);
-  return launch_bwd<128, false>(tq, tk, tv, tdo, p, s);
+  if (p.drop_thr > 0u) return D <= 64 ? launch_bwd<64, true>(m, p, s) : launch_bwd<128, true>(m, p, s);
+  if (D <= 64) return launch_bwd<64, false>(m, p, s);
+  return launch_bwd<128, false>(m, p, s);
 }

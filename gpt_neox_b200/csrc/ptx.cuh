@@ -350,6 +350,53 @@ __device__ __forceinline__ uint64_t umma_smem_desc_sw128(uint32_t smem_addr, uin
   return d;
 }
 
+// Low word of such a descriptor (address and leading byte offset; shared memory addresses stay below 2^18) and the high word
+// of every one with a stride of 1024 bytes: a warp that issues many steps its operands through the low words.
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
+  return (smem_addr >> 4) | ((lbo_bytes >> 4) << 16);
+}
+constexpr uint32_t UMMA_DESC_HI_1024 = (1024u >> 4) | (1u << 14) | (2u << 29);
+// The MMAs and the commit above for a converged warp: issued by the lane whose `leader` is not zero.
+__device__ __forceinline__ void umma_bf16_ss_by(uint32_t leader, uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
+                                                uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      ".reg .b64 da, db;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "setp.ne.b32 q, %5, 0;\n"
+      "mov.b64 da, {%1, %6};\n"
+      "mov.b64 db, {%2, %6};\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n"
+      "}\n" ::"r"(tmem_d),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(leader), "n"(UMMA_DESC_HI_1024)
+      : "memory");
+}
+__device__ __forceinline__ void umma_bf16_ts_by(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo,
+                                                uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      ".reg .b64 db;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "setp.ne.b32 q, %5, 0;\n"
+      "mov.b64 db, {%2, %6};\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n"
+      "}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(leader), "n"(UMMA_DESC_HI_1024)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_by(uint32_t leader, uint32_t bar) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %1, 0;\n"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+      "}\n" ::"r"(bar),
+      "r"(leader)
+      : "memory");
+}
+
 // Instruction descriptor for kind::f16 with 16-bit inputs (bf16, or fp16 in the NX_HALF build) and
 // fp32 accumulation.  c_format (F32=1) at bit 4, a/b format (F16=0, BF16=1) at bits 7/10, a/b major
 // (1 = MN-major) at bits 15/16, N>>3 at bit 17, M>>4 at bit 24.

@@ -415,6 +415,42 @@ def test_flash_attention(cfg):
     assert rel(q.grad, qr.grad) < 3e-2 and rel(k.grad, kr.grad) < 3e-2 and rel(v.grad, vr.grad) < 3e-2
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("b,sq,sk,h,hk,causal,window", [
+    (1, 1, 1, 1, 1, True, -1), (2, 63, 65, 2, 1, True, -1), (1, 129, 127, 2, 2, True, -1), (1, 128, 64, 1, 1, False, -1),
+    (1, 700, 190, 2, 1, True, -1),            # query rows and whole tiles that see no key
+    (1, 190, 700, 2, 2, True, 60),            # keys that no query row sees
+    (3, 257, 257, 40, 40, True, -1),          # several items per CTA, single-block ones among them
+    (2, 640, 640, 32, 4, True, 200)])         # grouped keys: a CTA's items run over several query heads
+def test_flash_attention_backward_tiles(b, sq, sk, h, hk, causal, window, d):
+    """The persistent backward kernels at the edges of their tiles, items and blocks, against the fp32 oracle.  A gradient is a
+    sum of products of values rounded to 16 bits (P or dS, relative 2^-9 or 2^-12 each, and O inside delta), rounded itself:
+    three roundings of unit eps."""
+    from gpt_neox_b200.ops.attention import attention_reference, flash_attention
+    torch.manual_seed(29)
+    q, k, v = bf(b, sq, h, d, grad=True), bf(b, sk, hk, d, grad=True), bf(b, sk, hk, d, grad=True)
+    g = bf(b, sq, h, d)
+    got = torch.autograd.grad(flash_attention(q, k, v, causal=causal, window=window), (q, k, v), g)
+    # (written out: autograd through the oracle's softmax has NaN for rows that see no key)
+    qd, kd, vd, gd = (t.detach().double() for t in (q, k, v, g))
+    _, lse = attention_reference(qd, kd, vd, causal=causal, window=window)
+    heads = lambda t: t.repeat_interleave(h // hk, 2)
+    pos = torch.arange(sq, device=DEV)[:, None] + sk - sq - torch.arange(sk, device=DEV)[None]
+    seen = ((pos >= 0) if causal else torch.ones_like(pos, dtype=torch.bool)) & ((pos <= window) | (window < 0))
+    scores = torch.einsum("bqhd,bkhd->bhqk", qd, heads(kd)) / d ** 0.5
+    p = torch.where(seen, (scores - lse[..., None]).exp(), 0.0)
+    dp = torch.einsum("bqhd,bkhd->bhqk", gd, heads(vd))
+    ds = p * (dp - (p * dp).sum(-1, keepdim=True)) / d ** 0.5
+    per_kv = lambda t: t.unflatten(2, (hk, h // hk)).sum(3)
+    want = (torch.einsum("bhqk,bkhd->bqhd", ds, heads(kd)), per_kv(torch.einsum("bhqk,bqhd->bkhd", ds, qd)),
+            per_kv(torch.einsum("bhqk,bqhd->bkhd", p, gd)))
+    eps = 2 ** -8 if DT == torch.bfloat16 else 2 ** -11
+    for x, y in zip(got, want):
+        assert x.isfinite().all()
+        # (one key: the true gradients of q and k are zero and what is left is the rounding of O against dP, of size |dO| |v|)
+        assert (x.double() - y).norm() <= 3 * eps * (y.norm() + d ** 0.5 * x.numel() ** 0.5 * (sk == 1))
+
+
 @pytest.mark.parametrize("env", [{"NEOX_ATTN_FWD_SHAPE": "1"}, {"NEOX_ATTN_FWD_SHAPE": "3"},
                                  {"NEOX_ATTN_BWD_WARPS": "4"}, {"NEOX_ATTN_DKV_PIPE": "0", "NEOX_ATTN_DQ_PIPE": "0"}],
                          ids=["fwd_shape1", "fwd_shape3", "bwd_4warps", "bwd_unpipelined"])
