@@ -103,9 +103,13 @@ struct SmemLayout {
   static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
   // full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2], tmem base word
   static constexpr int RS_OFFSET = BAR_OFFSET + (2 * STAGES + 4) * 8 + 16 + 8 * 8;   // + 8 chunk-ready barriers
-  static constexpr int TOTAL = RS_OFFSET + RS_STAGE_BYTES;
-  static constexpr int DYN_BYTES = TOTAL + 1024;  // slack for manual 1024-byte alignment
+  // the epilogue that stores by TMA: a barrier per epilogue warp, then 2 x 2 KB per warp
+  static constexpr int AUX_BAR_OFFSET = RS_OFFSET;
+  static constexpr int EPI_OFFSET = (AUX_BAR_OFFSET + 8 * 8 + 1023) / 1024 * 1024;
+  static constexpr int TOTAL = RS_OFFSET + RS_STAGE_BYTES, TMA_EPI_TOTAL = EPI_OFFSET + 8 * 4096;
+  static constexpr int dyn_bytes(bool tma_epi) { return (tma_epi ? TMA_EPI_TOTAL : TOTAL) + 1024; }  // slack for manual 1024-byte alignment
 };
+static_assert(SmemLayout<256, 4>::dyn_bytes(true) <= 232448, "shared memory of one SM");
 
 __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int& tm, int& tn) {
   // Group 8 row-tiles together so that concurrently running CTAs share B panels in L2.
@@ -161,10 +165,31 @@ __device__ __forceinline__ bool group_tile(int tile, const GemmParams& p, int nu
   return true;
 }
 
-template <int BN, int STAGES, bool A_MN, bool B_MN>
+// The tensor maps of the epilogue that stores by TMA: the result, aux_out, aux_in (32 x 32 boxes, rows of 64 bytes).
+struct EpiMaps {
+  CUtensorMap out, aux_out, aux_in;
+};
+// Chunk c (16 bytes) of row r of such a box (a swizzle, which would take the bank conflicts away, measured the same).
+__device__ __forceinline__ uint32_t epi_chunk(int r, int c) { return r * 64 + c * 16; }
+__device__ __forceinline__ void epi_put(uint8_t* box, int lane, const float (&v)[32]) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    *reinterpret_cast<uint4*>(box + epi_chunk(lane, c)) =
+        make_uint4(pack_h16x2(v[8 * c], v[8 * c + 1]), pack_h16x2(v[8 * c + 2], v[8 * c + 3]),
+                   pack_h16x2(v[8 * c + 4], v[8 * c + 5]), pack_h16x2(v[8 * c + 6], v[8 * c + 7]));
+}
+
+// TMA_EPI (grouped rows with more than 128 columns): a warp's 32 x 32 pieces of the result and of the stored derivative
+// leave through shared memory as TMA boxes, and a stored derivative comes in the same way, one piece ahead.  The GEMMs of a
+// short reduction are bound by their epilogue warps, which are bound by latency: what counts is that the 32 values of a lane
+// go through GeLU and derivative side by side, so the activation is chosen once per piece (chosen per value, the values' chains ran
+// one after the other: 3,400 cycles per piece).  Dropless MoE, 32,768 rows, 768 -> 3072: the GEMM with GeLU and derivative
+// 275 -> 179 us, the one that multiplies by the derivative 275 -> 151 us; with the chains one after the other 216 / 203, with
+// pieces transposed in registers instead of boxes 184 / 168; without any epilogue work 110.
+template <int BN, int STAGES, bool A_MN, bool B_MN, bool TMA_EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                     const __grid_constant__ CUtensorMap tmA2, const GemmParams p) {
+                     const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ EpiMaps em, const GemmParams p) {
   using L = SmemLayout<BN, STAGES>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -196,6 +221,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       mbar_init(tmem_empty_bar(a), p.comm == COMM_NONE ? 8 : 4);  // one arrival per epilogue warp
     }
     for (int k = 0; k < 8; ++k) mbar_init(ag_bar(k), 4);  // one arrival per push warp
+    if (TMA_EPI)
+      for (int k = 0; k < 8; ++k) mbar_init(smem_base + L::AUX_BAR_OFFSET + 8 * k, 1);
     *ag_abort = 0;
     fence_barrier_init();
   }
@@ -327,6 +354,148 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         }
       }
     }
+  } else if constexpr (TMA_EPI) {
+    const int w = warp - 2, quad = warp & 3;
+    const int c_begin = w < 4 ? 0 : BN / 64, c_end = w < 4 ? BN / 64 : BN / 32;
+    const uint32_t aux_bar = smem_base + L::AUX_BAR_OFFSET + 8 * w;
+    uint8_t* out_box = smem_gen + L::EPI_OFFSET + w * 4096;
+    uint8_t* aux_box = out_box + 2048;
+    const int flags = p.flags;
+    const bool aux_in = flags & (EPI_DGELU_ERF | EPI_DGELU_TANH | EPI_MUL_AUX);
+    int acc = 0, tm = 0, tn = 0, chunk, ge, kb0_, kb1_;
+    uint32_t acc_phase = 0, aux_phase = 0;
+    int tile = static_cast<int>(blockIdx.x) - static_cast<int>(gridDim.x);
+    auto next_tile = [&](int t, int& m, int& n) {      // the next tile with work after t
+      do {
+        t += gridDim.x;
+      } while (t < num_tiles && !group_tile(t, p, num_kb, m, n, chunk, ge, kb0_, kb1_));
+      return t;
+    };
+    auto fetch_aux = [&](int m, int n, int c) {
+      if (lane == 0) {
+        mbar_expect_tx(aux_bar, 2048);
+        tma_load_2d(smem_u32(aux_box), &em.aux_in, aux_bar, n * BN + c * 32, m * BM + quad * 32);
+      }
+    };
+    tile = next_tile(tile, tm, tn);
+    bool fetched = false;      // the piece that comes next is on its way
+    while (tile < num_tiles && !aborted) {
+      const int m0 = tm * BM, n0 = tn * BN;
+      int tm_nx = 0, tn_nx = 0;
+      const int tile_nx = next_tile(tile, tm_nx, tn_nx);
+      bool ok = mbar_wait(tmem_full_bar(acc), acc_phase, p.err, 4);
+      if (!__all_sync(0xffffffffu, ok)) {
+        aborted = true;
+        break;
+      }
+      tc_fence_after_sync();
+#pragma unroll 1
+      for (int c = c_begin; c < c_end; ++c) {
+        const int col0 = n0 + c * 32;
+        if (col0 >= p.N) break;  // warp-uniform
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(tmem_base + acc * BN + c * 32 + (static_cast<uint32_t>(quad * 32) << 16), r);
+        tmem_ld_wait();
+        float v[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+        if (aux_in) {
+          if (!fetched) fetch_aux(tm, tn, c);
+          ok = mbar_wait(aux_bar, aux_phase, p.err, 9);
+          if (!__all_sync(0xffffffffu, ok)) {
+            aborted = true;
+            break;
+          }
+          aux_phase ^= 1;
+          uint32_t x[16];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const uint4 u = *reinterpret_cast<const uint4*>(aux_box + epi_chunk(lane, k));
+            x[4 * k] = u.x; x[4 * k + 1] = u.y; x[4 * k + 2] = u.z; x[4 * k + 3] = u.w;
+          }
+          // Every lane has its values before the next piece comes in: this vote needs one word of each of their loads (never
+          // true, since M is positive).  A barrier alone lets the copy overtake loads that are still queued: 1 % of a
+          // gradient was wrong.
+          if (__any_sync(0xffffffffu, (x[3] ^ x[7] ^ x[11] ^ x[15]) == 0u && p.M < 0)) aborted = true;
+          // the next piece: of this tile, or the first of the next
+          const bool here = c + 1 < c_end && col0 + 32 < p.N;
+          fetched = here || (tile_nx < num_tiles && tn_nx * BN + c_begin * 32 < p.N);
+          if (fetched) fetch_aux(here ? tm : tm_nx, here ? tn : tn_nx, here ? c + 1 : c_begin);
+          auto times = [&](auto f) {
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+              const float2 a = unpack_h16x2(x[k]);
+              v[2 * k] *= f(a.x);
+              v[2 * k + 1] *= f(a.y);
+            }
+          };
+          if (flags & EPI_MUL_AUX) times([](float a) { return a; });
+          else if (flags & EPI_DGELU_ERF) times([](float a) { return gelu_erf_grad(a); });
+          else times([](float a) { return gelu_tanh_grad(a); });
+        }
+        const bool aux_out = flags & EPI_AUX_OUT;
+        if (flags & EPI_AUX_DERIV) {
+          float d[32];
+          if (flags & EPI_GELU_TANH) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) gelu_tanh_both(v[j], v[j], d[j]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) gelu_erf_both2(v[j], v[j + 1], d[j], d[j + 1]);
+          }
+          if (aux_out) {
+            if (lane == 0) tma_store_wait_read<1>();      // (all but the last store have left their boxes)
+            __syncwarp();
+            epi_put(aux_box, lane, d);
+          }
+        } else if (aux_out) {
+          if (lane == 0) tma_store_wait_read<1>();
+          __syncwarp();
+          epi_put(aux_box, lane, v);
+        }
+        if (aux_out) {
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_2d(&em.aux_out, smem_u32(aux_box), col0, m0 + quad * 32);
+            tma_store_commit();
+          }
+        }
+        if (!(flags & EPI_AUX_DERIV)) {
+          if (flags & EPI_GELU_ERF) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = gelu_erf(v[j]);
+          } else if (flags & EPI_GELU_TANH) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = gelu_tanh(v[j]);
+          }
+        }
+        if (lane == 0) {
+          if (aux_out) tma_store_wait_read<1>();
+          else tma_store_wait_read<0>();
+        }
+        __syncwarp();
+        epi_put(out_box, lane, v);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_2d(&em.out, smem_u32(out_box), col0, m0 + quad * 32);
+          tma_store_commit();
+        }
+      }
+      // This warp is done reading the accumulator: hand it back to the MMA issuer.
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(tmem_empty_bar(acc));
+      if (++acc == 2) {
+        acc = 0;
+        acc_phase ^= 1;
+      }
+      tile = tile_nx;
+      tm = tm_nx;
+      tn = tn_nx;
+    }
+    if (lane == 0) tma_store_wait_read<0>();      // shared memory outlives its last reader
   } else if (warp < 6 || p.comm == COMM_NONE) {
     // ------------------------------------------------------------------ epilogue (warps 2..5; without a collective
     // warps 6..9 too, each pair of warps of a lane quadrant taking half of the tile's columns: with four warps the
@@ -653,31 +822,38 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   }
 }
 
-template <int BN, int STAGES, bool A_MN, bool B_MN>
-static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmA2,
+template <int BN, int STAGES, bool A_MN, bool B_MN, bool TMA_EPI = false>
+static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmA2, const EpiMaps& em,
                        const GemmParams& p, cudaStream_t stream) {
   using L = SmemLayout<BN, STAGES>;
-  auto kern = gemm_bf16_kernel<BN, STAGES, A_MN, B_MN>;
+  auto kern = gemm_bf16_kernel<BN, STAGES, A_MN, B_MN, TMA_EPI>;
   static bool configured = false;
   if (!configured) {
     NX_CUDA_CHECK(
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::DYN_BYTES));
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::dyn_bytes(TMA_EPI)));
     configured = true;
   }
   const int tiles = p.total_tiles;
   const int grid = tiles < sm_count() ? tiles : sm_count();
-  kern<<<grid, GEMM_THREADS, L::DYN_BYTES, stream>>>(tmA, tmB, tmA2, p);
+  kern<<<grid, GEMM_THREADS, L::dyn_bytes(TMA_EPI), stream>>>(tmA, tmB, tmA2, em, p);
   NX_LAUNCH_CHECK();
   return NX_OK;
 }
 
 template <int BN, int STAGES>
 static int dispatch_layout(int transA, int transB, const CUtensorMap& tmA, const CUtensorMap& tmB,
-                           const CUtensorMap& tmA2, const GemmParams& p, cudaStream_t stream) {
-  if (!transA && !transB) return launch_gemm<BN, STAGES, false, false>(tmA, tmB, tmA2, p, stream);
-  if (!transA && transB) return launch_gemm<BN, STAGES, false, true>(tmA, tmB, tmA2, p, stream);
-  if (transA && !transB) return launch_gemm<BN, STAGES, true, false>(tmA, tmB, tmA2, p, stream);
-  return launch_gemm<BN, STAGES, true, true>(tmA, tmB, tmA2, p, stream);
+                           const CUtensorMap& tmA2, const EpiMaps& em, bool tma_epi, const GemmParams& p,
+                           cudaStream_t stream) {
+  if constexpr (BN == 256) {
+    if (tma_epi) {
+      if (!transB) return launch_gemm<BN, STAGES, false, false, true>(tmA, tmB, tmA2, em, p, stream);
+      return launch_gemm<BN, STAGES, false, true, true>(tmA, tmB, tmA2, em, p, stream);
+    }
+  }
+  if (!transA && !transB) return launch_gemm<BN, STAGES, false, false>(tmA, tmB, tmA2, em, p, stream);
+  if (!transA && transB) return launch_gemm<BN, STAGES, false, true>(tmA, tmB, tmA2, em, p, stream);
+  if (transA && !transB) return launch_gemm<BN, STAGES, true, false>(tmA, tmB, tmA2, em, p, stream);
+  return launch_gemm<BN, STAGES, true, true>(tmA, tmB, tmA2, em, p, stream);
 }
 
 }  // namespace nx
@@ -822,8 +998,21 @@ static int gemm_common(const void* A, const void* B, void* C, int M, int N, int 
     p.total_tiles = p.tiles_m * p.tiles_n * ca.experts;
   }
   p.err = device_error_word();
-  if (BN == 128) return dispatch_layout<128, 6>(transA, transB, tmA, tmB, tmA2, p, stream);
-  return dispatch_layout<256, 4>(transA, transB, tmA, tmB, tmA2, p, stream);
+  // (the other epilogues of grouped rows, which nothing here asks for, stay with the general kernel)
+  constexpr int aux_in_flags = EPI_DGELU_ERF | EPI_DGELU_TANH | EPI_MUL_AUX;
+  constexpr int tma_flags = EPI_GELU_ERF | EPI_GELU_TANH | EPI_AUX_OUT | EPI_AUX_DERIV | aux_in_flags;
+  const bool tma_epi = BN == 256 && ca.group_mode == GROUP_ROWS && (flags & ~tma_flags) == 0 &&
+                       !((flags & EPI_AUX_OUT) && (flags & aux_in_flags));
+  EpiMaps em;
+  memset(&em, 0, sizeof(em));
+  if (tma_epi) {
+    ok = make_tma_2d(&em.out, C, M, N, ldc * 2, 32, 32, 2, false);
+    if (flags & EPI_AUX_OUT) ok = ok && make_tma_2d(&em.aux_out, aux_out, M, N, ld_aux * 2, 32, 32, 2, false);
+    if (flags & aux_in_flags) ok = ok && make_tma_2d(&em.aux_in, aux_in, M, N, ld_aux * 2, 32, 32, 2, false);
+    if (!ok) return NX_ERR_ARG;
+  }
+  if (BN == 128) return dispatch_layout<128, 6>(transA, transB, tmA, tmB, tmA2, em, tma_epi, p, stream);
+  return dispatch_layout<256, 4>(transA, transB, tmA, tmB, tmA2, em, tma_epi, p, stream);
 }
 
 // C[M,N] = epilogue(op(A) * op(B)).  Leading dimensions in elements.  bias/aux/residual may be

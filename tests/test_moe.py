@@ -155,3 +155,36 @@ def test_expert_parallel_peer_memory_path_matches_fp32_oracle(ws, T, k, E, h, ff
     assert rel(torch.cat([d[0] for d in dws]), w1r.grad) < 3e-2
     assert rel(torch.cat([d[1] for d in dws]), w2r.grad) < 3e-2
     assert _lib.read_device_error() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("kind", ["erf", "tanh"])
+@pytest.mark.parametrize("T,n,K", [(150, 136, 64), (150, 256, 200), (150, 264, 64), (150, 392, 136), (150, 776, 768),
+                                   (12000, 1160, 64)])       # the last: several tiles per CTA, pieces prefetched across them
+def test_grouped_rows_epilogues(T, n, K, kind, dtype):
+    """GeLU with its derivative stored, and the product with a stored derivative, at ragged column counts (tiles of 256, a warp's
+    half of 128, pieces of 32) against 64 bits: results are rounded once, the sums behind them are fp32."""
+    from gpt_neox_b200.ops import moe as M
+    torch.manual_seed(3)
+    E = 3
+    idx = torch.randint(0, E, (T, 2), device="cuda")
+    plan = M.Plan(idx, E)
+    src, rows = plan.src_copy, (plan.src_copy >= 0).nonzero().flatten()
+    mk = lambda *s, scale=1.0: (torch.randn(*s, device="cuda") * scale).to(dtype)
+    xp = M.gather_rows(mk(T, K), plan)
+    w = mk(E * n, K, scale=K ** -0.5)
+    deriv = torch.empty((plan.max_rows, n), device="cuda", dtype=dtype)
+    act = M.grouped_gemm_rows(xp, w, plan, n, trans_b=False, gelu=kind, aux_out=deriv, aux_deriv=True)
+    prod = M.grouped_gemm_rows(xp, w, plan, n, trans_b=False, dgelu_aux=deriv, dgelu="mul")
+    expert = plan.tile_expert.long()[rows // 128]
+    z = torch.einsum("rk,rnk->rn", xp[rows].double(), w.view(E, n, K).double()[expert]).requires_grad_()
+    want = torch.nn.functional.gelu(z, approximate="tanh" if kind == "tanh" else "none")
+    (wd,) = torch.autograd.grad(want.sum(), z)
+    eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -11
+    # (tanh.approx has an absolute error of 2^-11, the erf series 1e-7; |z| < 8)
+    slack = 8 * 2 ** -11 if kind == "tanh" else 2 ** -18
+    assert (act[rows] - want).abs().sub(eps * want.abs()).max() <= slack
+    assert (deriv[rows] - wd).abs().sub(eps * wd.abs()).max() <= slack
+    ref = z.detach() * deriv[rows].double()
+    assert (prod[rows] - ref).abs().sub(eps * ref.abs()).max() <= 2 ** -18
