@@ -7,22 +7,21 @@
 // kernel_backward_111 / _222), which walks the whole sequence in one thread per channel and needs
 // the sequence length as a compile-time constant for a per-thread array.
 //
-// One CTA of 2 N threads walks one head's piece of the sequence with the N x N state in registers: warp w owns 16 columns
-// j, a lane N / 8 rows i by 4 columns.  Per step a lane reads N / 8 values of each row vector and 4 of each column
+// Heads of 64 (every configuration here) go in blocks of 16 steps as matrix products (second half of this file).  Heads of 32
+// go step by step: one CTA of 2 N threads walks one head's piece of the sequence with the N x N state in registers: warp w owns
+// 16 columns j, a lane N / 8 rows i by 4 columns.  Per step a lane reads N / 8 values of each row vector and 4 of each column
 // vector from shared memory (column vectors are stored twice side by side, so that the packed fp32 pairs, which run
 // over neighbouring rows, need no register moves) and does 3 packed operations per 2 state elements: one for the output
-// sum, two for the update.  The former one-column-per-thread mapping read every row vector whole in every thread, which
-// used the shared-memory port as fully as the FMA pipe.  The u term is taken out of the sums: it is a dot product per
-// step (formed while staging) times one value.  Sums over rows / columns leave a lane by transposing exchanges.
+// sum, two for the update.  The u term is taken out of the sums: it is a dot product per step (formed while staging) times
+// one value.  Sums over rows / columns leave a lane by transposing exchanges.
 //   forward  : one sweep: y (sum over i)
-//   backward : a forward sweep: gr (sum over j), then ONE reverse sweep of the gradient state G = dL/dS with both
-//              gk (sum over j) and gv (sum over i), which also forms the decay gradient: with
+//   backward : a forward sweep: gr (sum over j), then a reverse sweep of the gradient state G = dL/dS with gk (sum over j)
+//              and gv (sum over i; a sweep of its own for heads of 64), which also forms the decay gradient: with
 //              Q_t[i] = sum_j G_t[i][j] S_t[i][j] one has Q_{t-1} - Q_t = r_t gr_t - k_t gk_t and
 //              dL/d(ew_t) = Q_t - k_t (gk_t - r_t u s_t),  s_t = <gy_t, v_t>,  ew = -exp(w)
-// 3 + 3 + 4 operations per state element and step; at 32 x 512 tokens, 12 heads of 64, the schedulers have 2.6 warps each and
-// are bound by the steps' shared-memory loads and exchanges (that pipe 64-74 % busy, issue slots 38-45 %).  Forward +
-// backward of that size: 3.03 ms with one column per thread in seven passes, 0.87 ms with 8 columns per lane and half the
-// warps, 0.79 ms now.
+// Step by step the shared-memory loads and exchanges of the steps are the bound (32 x 512 tokens, 12 heads of 64, forward +
+// backward 788 us); 581 us with the products of
+// a block in their place (125 us for each sweep, 190 for gk with the decay gradient).
 //
 // The sequence is cut into chunks only when batch x heads leaves the chip idle (wkv_chunk_count): the recurrence is
 // linear, so a chunk's end state is  P (.) S_start + S_local  with P[i] = prod_t d_t[i]; local passes start every chunk
@@ -316,6 +315,608 @@ __global__ void __launch_bounds__(2 * N) wkv_kernel(const WkvParams p) {
   if (MODE == WK_G && !second) p.gu_part[(((long long)bi * p.NC + c) * p.H + h) * N + me] = gu;
 }
 
+// ------------------------------------------------------------------------------------------------
+// Heads of 64: the same sweeps in blocks of 16 steps, as matrix products.  In the order of a sweep (reverse sweeps run
+// backwards in time) let S be the state before a block, d_m the decays, a_t, b_t, c_t, e_t the step's vectors (S += b c^T):
+//   column sums   y_t[j]   = sum_i a_t[i] Pre_t[i] S[i][j] + sum_{s < t} A[t][s] c_s[j] + A[t][t] c_t[j]
+//   row sums      row_t[i] = Pre_t[i] sum_j e_t[j] S[i][j] + sum_{s < t} (prod_{s < m < t} d_m[i]) b_s[i] M[t][s]
+//   state         S[i][j] <- Tot[i] S[i][j] + sum_s Suf_s[i] b_s[i] c_s[j]
+// with Pre_t / Suf_t / Tot the products of the decays before / after t / of the block, M[t][s] = <e_t, c_s> and
+// A[t][s] = sum_i a_t[i] b_s[i] prod_{s < m < t} d_m[i] (A[t][t]: with u).  Only products of decays between two steps appear,
+// never a quotient, so no decay is too strong.  y = column sums forward with (r, k, v); gv the same backwards with (k, r, gy);
+// gr = row sums forward with (k, v | gy); gk backwards with (r, gy | v), which also forms the decay gradient.
+//
+// Four warps; the state is the accumulators of mma.m16n8k16 (warp w: 16 of its rows, a thread 32 values), fp32 throughout.
+// What is not a 16-bit input is split into three bf16 parts (24 bits: the products of parts of weight 2^-16 and above are
+// all formed; the rest is below fp32's last bit), fp16 inputs into two, which is exact: the sums are those of fp32
+// arithmetic in another order.  These products are far too small for tcgen05 (M = 16 rows of steps, operands made in
+// registers between every two of them), hence mma.sync.
+// Infinite states or inputs give NaN where step-by-step arithmetic may give infinities (a part of zero times infinity); a
+// product over a block's steps is formed value by value where an input of the block is not finite, so that what is not finite
+// does not reach earlier steps.
+// ------------------------------------------------------------------------------------------------
+constexpr int WM = 16;              // steps per block
+constexpr int WN = 64;              // head size
+constexpr int WP = WN + 8;          // row pitch of the 16-bit arrays: ldmatrix without bank conflicts
+constexpr int WM_THREADS = 128;
+#ifdef NX_HALF
+constexpr int WM_IN = 2;            // bf16 parts of an input
+#else
+constexpr int WM_IN = 1;
+#endif
+
+__device__ __forceinline__ uint32_t wm_bf16x2(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+__device__ __forceinline__ float2 wm_floats(uint32_t v) {
+  return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+}
+__device__ __forceinline__ void wm_split(float2 x, uint32_t (&p)[3]) {
+  const float2 m1 = make_float2(-1.f, -1.f);
+  p[0] = wm_bf16x2(x.x, x.y);
+  x = ffma2(wm_floats(p[0]), m1, x);
+  p[1] = wm_bf16x2(x.x, x.y);
+  x = ffma2(wm_floats(p[1]), m1, x);
+  p[2] = wm_bf16x2(x.x, x.y);
+}
+__device__ __forceinline__ void wm_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Four 8 x 8 matrices: (rows r0 .. r0 + 7 | r0 + 8 ..) x (columns c0 .. | c0 + 8 ..) of a 16-bit array.  Plain: registers 0, 1 =
+// the first rows' two column groups, 2, 3 = the second rows'; TRANS: each matrix transposed.
+template <bool TRANS>
+__device__ __forceinline__ void wm_ld4(uint32_t (&r)[4], const uint16_t* base, int r0, int c0, int pitch, bool rows_first) {
+  const int lane = threadIdx.x & 31, m = lane >> 3, i = lane & 7;
+  // rows_first: matrices in the order (0, 0), (1, 0), (0, 1), (1, 1) of (row group, column group), else (0, 0), (0, 1), ...
+  const int rg = rows_first ? m & 1 : m >> 1, cg = rows_first ? m >> 1 : m & 1;
+  const uint32_t addr = smem_u32(base + (r0 + rg * 8 + i) * pitch + c0 + cg * 8);
+  if (TRANS)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+
+// An input block: as it lies in memory (for the scalar uses), and as bf16 parts (for the products).
+struct WmIn {
+  uint16_t raw[WM][WP];
+#ifdef NX_HALF
+  uint16_t part[WM_IN][WM][WP];
+  __device__ __forceinline__ const uint16_t* parts(int p) const { return &part[p][0][0]; }
+#else
+  __device__ __forceinline__ const uint16_t* parts(int) const { return &raw[0][0]; }
+#endif
+  __device__ __forceinline__ void put(int t, int c8, const uint4& u) {
+    *reinterpret_cast<uint4*>(&raw[t][c8]) = u;
+#ifdef NX_HALF
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 x = unpack_h16x2(w[k]), m1 = make_float2(-1.f, -1.f);
+      hi[k] = wm_bf16x2(x.x, x.y);
+      const float2 rest = ffma2(wm_floats(hi[k]), m1, x);
+      lo[k] = wm_bf16x2(rest.x, rest.y);
+    }
+    *reinterpret_cast<uint4*>(&part[0][t][c8]) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<uint4*>(&part[1][t][c8]) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+#endif
+  }
+  __device__ __forceinline__ float at(int t, int c) const {
+    return h16_to_float(reinterpret_cast<const h16&>(raw[t][c]));
+  }
+  __device__ __forceinline__ float2 pair(int t, int c) const {
+    return unpack_h16x2(*reinterpret_cast<const uint32_t*>(&raw[t][c]));
+  }
+};
+
+__device__ __forceinline__ bool wm_all_finite(const uint4& u) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#ifdef NX_HALF
+  constexpr uint32_t E = 0x7c00u;
+#else
+  constexpr uint32_t E = 0x7f80u;
+#endif
+  bool ok = true;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) ok = ok && (w[k] & E) != E && ((w[k] >> 16) & E) != E;
+  return ok;
+}
+
+// Step s of block q in a sweep's order -> time.  Blocks start at the sweep's first step, so that a short one is the last.
+template <bool REV>
+__device__ __forceinline__ int wm_time(int t_lo, int t_hi, int q, int s) {
+  return REV ? t_hi - 1 - (q * WM + s) : t_lo + q * WM + s;
+}
+
+struct WmColSmem {
+  WmIn a, b, c;
+  float d[WM][WN];
+  uint16_t ap[3][WM][WP], bp[3][WM][WP];     // parts of a Pre, b Suf
+  uint16_t A[3][WM][24];
+  float tot[WN];
+  uint16_t out[WM][WP];
+};
+
+// Column sums (y, or gv in reverse), or (LOCAL) only the end state of a chunk from a zero state and the sums of ew.
+template <bool REV, bool LOCAL, bool VEC>
+__global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams p) {
+  extern __shared__ __align__(16) unsigned char wk_raw[];
+  WmColSmem& s = *reinterpret_cast<WmColSmem*>(wk_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ch = LOCAL && REV ? blockIdx.x + 1 : blockIdx.x, h = blockIdx.y, bi = blockIdx.z;
+  const int t_lo = ch * p.clen, t_hi = min(t_lo + p.clen, p.T);
+  const long long base = ((long long)bi * p.H + h) * p.NC + ch;
+  const h16 *ga = REV ? p.k : p.r, *gb = REV ? p.r : p.k, *gc = REV ? p.gy : p.v;
+  // S^T: rows j = 16 warp + lane / 4 (+ 8), columns i = 8 n + 2 (lane % 4) (+ 1)
+  float S[8][4];
+  const int j0 = warp * 16 + (lane >> 2), i0 = (lane & 3) * 2;
+#pragma unroll
+  for (int n = 0; n < 8; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      S[n][e] = 0.f;
+      if (!LOCAL && p.start != nullptr) S[n][e] = p.start[(base * WN + 8 * n + i0 + (e & 1)) * WN + j0 + (e >> 1) * 8];
+    }
+  // the zeros of A (its upper triangle is never written)
+  for (int x = tid; x < 3 * WM * 24; x += WM_THREADS) (&s.A[0][0][0])[x] = 0;
+  const int trow = tid >> 3, ch8 = (tid & 7) * 8;
+  float sew[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  const int nblk = (t_hi - t_lo + WM - 1) / WM;
+  uint4 ra, rb, rc, rw;
+  bool live;
+  auto fetch = [&](int q) {
+    const int t = wm_time<REV>(t_lo, t_hi, q, trow);
+    live = t >= t_lo && t < t_hi;
+    const long long o = bi * p.sb + (long long)t * p.st + h * WN + ch8;
+    if (!LOCAL) ra = wk_load8<VEC>(ga + o, live);
+    rb = wk_load8<VEC>(gb + o, live);
+    rc = wk_load8<VEC>(gc + o, live);
+    rw = wk_load8<VEC>(p.w + o, live);
+  };
+  fetch(0);
+  for (int q = 0; q < nblk; ++q) {
+    if (!LOCAL) s.a.put(trow, ch8, ra);
+    s.b.put(trow, ch8, rb);
+    s.c.put(trow, ch8, rc);
+    {
+      float w8[8], d8[8];
+      wk_unpack8(rw, w8);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float ew = live ? -__expf(w8[e]) : 0.f;
+        d8[e] = __expf(ew);
+        if (LOCAL) sew[e] += ew;
+      }
+      *reinterpret_cast<float4*>(&s.d[trow][ch8]) = make_float4(d8[0], d8[1], d8[2], d8[3]);
+      *reinterpret_cast<float4*>(&s.d[trow][ch8 + 4]) = make_float4(d8[4], d8[5], d8[6], d8[7]);
+    }
+    const bool finite = !__syncthreads_or(!LOCAL && !wm_all_finite(rc));
+    if (q + 1 < nblk) fetch(q + 1);      // in flight during this block
+    if (warp == 0) {
+      // a Pre, and Tot; two channels per thread
+      const int c = lane * 2;
+      float2 pre = make_float2(1.f, 1.f);
+#pragma unroll 4
+      for (int t = 0; t < WM; ++t) {
+        const float2 d = *reinterpret_cast<const float2*>(&s.d[t][c]);
+        if (!LOCAL) {
+          uint32_t x[3];
+          wm_split(fmul2(s.a.pair(t, c), pre), x);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&s.ap[k][t][c]) = x[k];
+        }
+        pre = fmul2(pre, d);
+      }
+      *reinterpret_cast<float2*>(&s.tot[c]) = pre;
+    } else if (warp == 1) {
+      const int c = lane * 2;
+      float2 suf = make_float2(1.f, 1.f);
+#pragma unroll 4
+      for (int t = WM - 1; t >= 0; --t) {
+        const float2 d = *reinterpret_cast<const float2*>(&s.d[t][c]);
+        uint32_t x[3];
+        wm_split(fmul2(s.b.pair(t, c), suf), x);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&s.bp[k][t][c]) = x[k];
+        suf = fmul2(suf, d);
+      }
+    } else if (!LOCAL) {
+      // A: eight groups of eight lanes (8 channels each); group g takes columns s = g and s = 15 - g, 15 entries together
+      const int g = (tid - 64) >> 3, c = (tid & 7) * 8, turn = WM - 1 - g;
+      float2 qv[4];
+      auto load_b = [&](int t) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) qv[k] = s.b.pair(t, c + 2 * k);
+      };
+      load_b(g);
+      float val[16], diag = 0.f;
+#pragma unroll
+      for (int it = 0; it < 15; ++it) {
+        if (it == turn) load_b(turn);
+        const int t = it < turn ? g + 1 + it : turn + 1 + (it - turn);
+        float2 acc = make_float2(0.f, 0.f);
+        const float4 d0 = *reinterpret_cast<const float4*>(&s.d[t][c]), d1 = *reinterpret_cast<const float4*>(&s.d[t][c + 4]);
+        const float2 dd[4] = {{d0.x, d0.y}, {d0.z, d0.w}, {d1.x, d1.y}, {d1.z, d1.w}};
+        const uint4 u = *reinterpret_cast<const uint4*>(&s.a.raw[t][c]);
+        const uint32_t aw[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          acc = ffma2(unpack_h16x2(aw[k]), qv[k], acc);
+          qv[k] = fmul2(qv[k], dd[k]);
+        }
+        val[it] = acc.x + acc.y;
+      }
+      // the diagonal entries g (slot 15) and 15 - g
+      float dg[2] = {0.f, 0.f};
+#pragma unroll
+      for (int z = 0; z < 2; ++z)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int t = z == 0 ? g : turn;
+          const float2 x = s.a.pair(t, c + 2 * k), y = s.b.pair(t, c + 2 * k);
+          dg[z] += x.x * p.u[h * WN + c + 2 * k] * y.x + x.y * p.u[h * WN + c + 2 * k + 1] * y.y;
+        }
+      val[15] = dg[0];
+      diag = dg[1];
+#pragma unroll
+      for (int m = 4; m > 0; m >>= 1) diag += __shfl_xor_sync(0xffffffffu, diag, m);
+      // 16 values over 8 lanes: lane l ends with values 2 l' , 2 l' + 1 of its own order
+      const bool h4 = lane & 4, h2 = lane & 2, h1 = lane & 1;
+      float v8[8], v4[4], v2[2];
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        v8[k] = (h4 ? val[8 + k] : val[k]) + __shfl_xor_sync(0xffffffffu, h4 ? val[k] : val[8 + k], 4);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        v4[k] = (h2 ? v8[4 + k] : v8[k]) + __shfl_xor_sync(0xffffffffu, h2 ? v8[k] : v8[4 + k], 2);
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        v2[k] = (h1 ? v4[2 + k] : v4[k]) + __shfl_xor_sync(0xffffffffu, h1 ? v4[k] : v4[2 + k], 1);
+      auto put_A = [&](int t, int col, float x) {
+        uint32_t y[3];
+        wm_split(make_float2(x, 0.f), y);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s.A[k][t][col] = static_cast<uint16_t>(y[k]);
+      };
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int it = (h4 ? 8 : 0) + (h2 ? 4 : 0) + (h1 ? 2 : 0) + k;
+        if (it == 15) put_A(g, g, v2[k]);
+        else if (it < turn) put_A(g + 1 + it, g, v2[k]);
+        else put_A(turn + 1 + (it - turn), turn, v2[k]);
+      }
+      if ((lane & 7) == 0) put_A(turn, turn, diag);
+    }
+    __syncthreads();
+    // ---- products
+    uint32_t cv[WM_IN][4];               // c^T: 16 rows j of this warp x 16 steps
+#pragma unroll
+    for (int k = 0; k < WM_IN; ++k) wm_ld4<true>(cv[k], s.c.parts(k), 0, warp * 16, WP, false);
+    if (!LOCAL) {
+      float y[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) {
+        uint32_t sp[3][4];               // S^T[16 j][16 i]
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          uint32_t x[3];
+          const float* src = S[2 * ks + (e >> 1)] + (e & 1) * 2;
+          wm_split(make_float2(src[0], src[1]), x);
+          sp[0][e] = x[0]; sp[1][e] = x[1]; sp[2][e] = x[2];
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          uint32_t b[4];
+          wm_ld4<false>(b, &s.ap[k][0][0], 0, 16 * ks, WP, false);
+#pragma unroll
+          for (int m = 2 - k; m >= 0; --m) {
+            wm_mma(y[0], sp[m], b[0], b[1]);
+            wm_mma(y[1], sp[m], b[2], b[3]);
+          }
+        }
+      }
+      if (finite) {
+#pragma unroll
+        for (int k = 2; k >= 0; --k) {
+          uint32_t b[4];
+          wm_ld4<false>(b, &s.A[k][0][0], 0, 0, 24, false);
+#pragma unroll
+          for (int m = 0; m < WM_IN; ++m) {
+            wm_mma(y[0], cv[m], b[0], b[1]);
+            wm_mma(y[1], cv[m], b[2], b[3]);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int t = 8 * n + i0 + (e & 1), j = j0 + (e >> 1) * 8;
+            for (int x = 0; x <= t; ++x) {
+              float a = 0.f;
+              for (int k = 2; k >= 0; --k) a += __uint_as_float(static_cast<uint32_t>(s.A[k][t][x]) << 16);
+              y[n][e] += a * s.c.at(x, j);
+            }
+          }
+      }
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const h16 o = float_to_h16(y[n][e]);
+          s.out[8 * n + i0 + (e & 1)][j0 + (e >> 1) * 8] = reinterpret_cast<const uint16_t&>(o);
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      const float2 d = *reinterpret_cast<const float2*>(&s.tot[8 * n + i0]);
+      S[n][0] *= d.x; S[n][1] *= d.y; S[n][2] *= d.x; S[n][3] *= d.y;
+    }
+#pragma unroll
+    for (int n = 0; n < 8; n += 2)
+#pragma unroll
+      for (int k = 2; k >= 0; --k) {
+        uint32_t b[4];
+        wm_ld4<true>(b, &s.bp[k][0][0], 0, 8 * n, WP, true);
+#pragma unroll
+        for (int m = 0; m < WM_IN; ++m) {
+          wm_mma(S[n], cv[m], b[0], b[1]);
+          wm_mma(S[n + 1], cv[m], b[2], b[3]);
+        }
+      }
+    __syncthreads();
+    if (!LOCAL) {
+      const int t = wm_time<REV>(t_lo, t_hi, q, trow);
+      if (t >= t_lo && t < t_hi)
+        *reinterpret_cast<uint4*>((REV ? p.o_gv : p.y) + bi * p.osb + (long long)t * p.ost + h * WN + ch8) =
+            *reinterpret_cast<const uint4*>(&s.out[trow][ch8]);
+      // (`out` is written again after the next block's two barriers)
+    }
+  }
+  if (LOCAL) {
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) p.local[(base * WN + 8 * n + i0 + (e & 1)) * WN + j0 + (e >> 1) * 8] = S[n][e];
+    // sums of ew over the 16 staging rows
+    float* r = &s.d[0][0];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) r[trow * WN + ch8 + e] = sew[e];
+    __syncthreads();
+    if (tid < WN) {
+      float a = 0.f;
+      for (int t = 0; t < WM; ++t) a += r[t * WN + tid];
+      p.sumew[base * WN + tid] = a;
+    }
+  }
+}
+
+struct WmRowSmem {
+  WmIn b, c, e;
+  uint16_t k[WM][WP];                        // gk: the other factor of the decay gradient
+  float d[WM][WN], ew[WM][WN];
+  uint16_t bp[3][WM][WP];
+  float M[2][WM][8];                         // <e_t, c_s>: s even | odd
+  float st[WM];
+  float part[2][WM][WN];                     // what a block's own steps add, by the parity of s
+  float pre[WM][WN], tot[WN];
+  float inter[WM][WN + 4];
+};
+
+// Row sums: gr (fp32 and rounded), or in reverse gk with the decay gradient and the sums for the gradient of u.
+template <bool REV, bool VEC>
+__global__ void __launch_bounds__(WM_THREADS, 4) wkv_row_kernel(const WkvParams p) {
+  extern __shared__ __align__(16) unsigned char wk_raw[];
+  WmRowSmem& s = *reinterpret_cast<WmRowSmem*>(wk_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ch = blockIdx.x, h = blockIdx.y, bi = blockIdx.z;
+  const int t_lo = ch * p.clen, t_hi = min(t_lo + p.clen, p.T);
+  const long long base = ((long long)bi * p.H + h) * p.NC + ch;
+  const h16 *gb = REV ? p.r : p.k, *gc = REV ? p.gy : p.v, *ge = REV ? p.v : p.gy;
+  // S: rows i = 16 warp + lane / 4 (+ 8), columns j = 8 n + 2 (lane % 4) (+ 1)
+  float S[8][4];
+  const int r0 = warp * 16 + (lane >> 2), n0 = (lane & 3) * 2;
+#pragma unroll
+  for (int n = 0; n < 8; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      S[n][e] = p.start != nullptr ? p.start[(base * WN + r0 + (e >> 1) * 8) * WN + 8 * n + n0 + (e & 1)] : 0.f;
+  const int me = tid & (WN - 1), half = tid >> 6;
+  const float u_me = p.u[h * WN + me];
+  float Q = 0.f, gu = 0.f;
+  if (REV && half == 0 && p.fstart != nullptr && ch + 1 < p.NC) {
+    const float* g = p.start + (base * WN + me) * WN;
+    const float* f = p.fstart + ((base + 1) * WN + me) * WN;
+    for (int j = 0; j < WN; ++j) Q += g[j] * f[j];
+  }
+  const int trow = tid >> 3, ch8 = (tid & 7) * 8;
+  const int nblk = (t_hi - t_lo + WM - 1) / WM;
+  uint4 rb, rc, re, rw, rk;
+  bool live;
+  auto fetch = [&](int q) {
+    const int t = wm_time<REV>(t_lo, t_hi, q, trow);
+    live = t >= t_lo && t < t_hi;
+    const long long o = bi * p.sb + (long long)t * p.st + h * WN + ch8;
+    rb = wk_load8<VEC>(gb + o, live);
+    rc = wk_load8<VEC>(gc + o, live);
+    re = wk_load8<VEC>(ge + o, live);
+    rw = wk_load8<VEC>(p.w + o, live);
+    if (REV) rk = wk_load8<VEC>(p.k + o, live);
+  };
+  fetch(0);
+  for (int q = 0; q < nblk; ++q) {
+    const int steps = min(WM, t_hi - t_lo - q * WM);
+    s.b.put(trow, ch8, rb);
+    s.c.put(trow, ch8, rc);
+    s.e.put(trow, ch8, re);
+    if (REV) *reinterpret_cast<uint4*>(&s.k[trow][ch8]) = rk;
+    {
+      float w8[8];
+      wk_unpack8(rw, w8);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float ew = live ? -__expf(w8[e]) : 0.f;
+        s.ew[trow][ch8 + e] = ew;
+        s.d[trow][ch8 + e] = __expf(ew);
+      }
+    }
+    __syncthreads();
+    if (q + 1 < nblk) fetch(q + 1);      // in flight during this block
+    const long long oo = bi * p.osb + h * WN + me;
+    float gr[REV ? WM : 1];
+    if (REV && half == 0) {
+#pragma unroll
+      for (int t = 0; t < WM; ++t) gr[REV ? t : 0] = t < steps ? p.gr32[oo + (long long)(t_hi - 1 - q * WM - t) * p.ost] : 0.f;
+    }
+    // ---- M: warp 0 the first eight s, warp 1 the others
+    if (warp < 2) {
+      float m4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+        for (int x = 0; x < WM_IN; ++x) {
+          uint32_t a[4];
+          wm_ld4<false>(a, s.e.parts(x), 0, 16 * ks, WP, true);
+#pragma unroll
+          for (int z = 0; z < WM_IN; ++z) {
+            uint32_t b[4];
+            wm_ld4<false>(b, s.c.parts(z), 0, 16 * ks, WP, false);
+            wm_mma(m4, a, warp == 0 ? b[0] : b[2], warp == 0 ? b[1] : b[3]);
+          }
+        }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int t = (lane >> 2) + (e >> 1) * 8, x = warp * 8 + n0 + (e & 1);
+        s.M[x & 1][t][x >> 1] = m4[e];
+        if (t == x) s.st[t] = m4[e];
+      }
+    }
+    __syncthreads();
+    // ---- a block's own steps, for one channel and every second s
+    {
+      float qv[8], pre = 1.f;
+#pragma unroll
+      for (int t = 0; t < WM; ++t) {
+        const float d = s.d[t][me];
+        float acc = 0.f;
+        const float4 m0 = *reinterpret_cast<const float4*>(&s.M[half][t][0]), m1 = *reinterpret_cast<const float4*>(&s.M[half][t][4]);
+        const float m[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+        // own s: 2 x + half < t; the last of them exists for half 1 only from t on that is even
+#pragma unroll
+        for (int x = 0; x < 8; ++x) {
+          if (2 * x + 1 < t) {
+            acc += qv[x] * m[x];
+            qv[x] *= d;
+          } else if (2 * x < t && half == 0) {
+            acc += qv[x] * m[x];
+            qv[x] *= d;
+          }
+        }
+        if ((t & 1) == half) qv[t >> 1] = s.b.at(t, me);
+        s.part[half][t][me] = acc;
+        if (half == 0) {
+          s.pre[t][me] = pre;
+          pre *= d;
+        }
+      }
+      if (half == 0) s.tot[me] = pre;
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        uint32_t y[3];
+        wm_split(make_float2(qv[x], 0.f), y);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s.bp[k][2 * x + half][me] = static_cast<uint16_t>(y[k]);
+      }
+    }
+    __syncthreads();
+    // ---- products
+    {
+      float y[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) {
+        uint32_t sp[3][4];               // S[16 i][16 j]
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          uint32_t x[3];
+          const float* src = S[2 * ks + (e >> 1)] + (e & 1) * 2;
+          wm_split(make_float2(src[0], src[1]), x);
+          sp[0][e] = x[0]; sp[1][e] = x[1]; sp[2][e] = x[2];
+        }
+#pragma unroll
+        for (int z = 0; z < WM_IN; ++z) {
+          uint32_t b[4];
+          wm_ld4<false>(b, s.e.parts(z), 0, 16 * ks, WP, false);
+#pragma unroll
+          for (int m = 2; m >= 0; --m) {
+            wm_mma(y[0], sp[m], b[0], b[1]);
+            wm_mma(y[1], sp[m], b[2], b[3]);
+          }
+        }
+      }
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s.inter[8 * n + n0 + (e & 1)][r0 + (e >> 1) * 8] = y[n][e];
+      const float t0 = s.tot[r0], t1 = s.tot[r0 + 8];
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        S[n][0] *= t0; S[n][1] *= t0; S[n][2] *= t1; S[n][3] *= t1;
+      }
+      uint32_t bt[3][4];                 // (b Suf)^T: 16 rows i x 16 steps
+#pragma unroll
+      for (int k = 0; k < 3; ++k) wm_ld4<true>(bt[k], &s.bp[k][0][0], 0, warp * 16, WP, false);
+#pragma unroll
+      for (int n = 0; n < 8; n += 2)
+#pragma unroll
+        for (int z = 0; z < WM_IN; ++z) {
+          uint32_t b[4];
+          wm_ld4<true>(b, s.c.parts(z), 0, 8 * n, WP, true);
+#pragma unroll
+          for (int k = 2; k >= 0; --k) {
+            wm_mma(S[n], bt[k], b[0], b[1]);
+            wm_mma(S[n + 1], bt[k], b[2], b[3]);
+          }
+        }
+    }
+    __syncthreads();
+    // ---- results
+    if (!REV) {
+#pragma unroll
+      for (int x = 0; x < WM / 2; ++x) {
+        const int t = half * (WM / 2) + x;
+        if (t >= steps) continue;
+        const float row = s.pre[t][me] * s.inter[t][me] + (s.part[0][t][me] + s.part[1][t][me]);
+        const float gr = row + u_me * s.b.at(t, me) * s.st[t];
+        const long long o = oo + (long long)(t_lo + q * WM + t) * p.ost;
+        p.gr32[o] = gr;
+        p.o_gr[o] = float_to_h16(gr);
+      }
+    } else if (half == 0) {
+#pragma unroll
+      for (int t = 0; t < WM; ++t) {
+        if (t >= steps) continue;
+        const float row = s.pre[t][me] * s.inter[t][me] + (s.part[0][t][me] + s.part[1][t][me]);
+        const float r_ = s.b.at(t, me), k_ = h16_to_float(reinterpret_cast<const h16&>(s.k[t][me])), st = s.st[t];
+        const float gk = row + u_me * r_ * st;
+        const long long o = oo + (long long)(t_hi - 1 - q * WM - t) * p.ost;
+        p.o_gk[o] = float_to_h16(gk);
+        p.o_gw[o] = float_to_h16((Q - k_ * row) * s.ew[t][me]);
+        Q += r_ * gr[REV ? t : 0] - k_ * gk;
+        gu += r_ * k_ * st;
+      }
+    }
+    __syncthreads();
+  }
+  if (REV && half == 0) p.gu_part[(((long long)bi * p.NC + ch) * p.H + h) * WN + me] = gu;
+}
+
 // start[c] for every chunk: forward  start[0] = 0, start[c+1] = P_c start[c] + local[c];
 //                           reverse  start[NC-1] = 0, start[c-1] = P_c start[c] + local[c].
 template <int N, bool REV>
@@ -394,35 +995,63 @@ static bool wkv_vec_ok(const WkvParams& p) {
   return ok(p.r) && ok(p.k) && ok(p.v) && ok(p.w) && ok(p.gy) && p.sb % 8 == 0 && p.st % 8 == 0;
 }
 
+template <typename Smem, typename K>
+static int wkv64_launch(K with_vec, K without, const WkvParams& p, bool vec, int chunks, cudaStream_t stream) {
+  const K kern = vec ? with_vec : without;
+  NX_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
+  kern<<<dim3(chunks, p.H, p.B), WM_THREADS, sizeof(Smem), stream>>>(p);
+  NX_LAUNCH_CHECK();
+  return NX_OK;
+}
+template <bool REV, bool LOCAL>
+static int wkv_col(const WkvParams& p, bool vec, int chunks, cudaStream_t stream) {
+  return wkv64_launch<WmColSmem>(wkv_col_kernel<REV, LOCAL, true>, wkv_col_kernel<REV, LOCAL, false>, p, vec, chunks, stream);
+}
+template <bool REV>
+static int wkv_row(const WkvParams& p, bool vec, cudaStream_t stream) {
+  return wkv64_launch<WmRowSmem>(wkv_row_kernel<REV, true>, wkv_row_kernel<REV, false>, p, vec, p.NC, stream);
+}
+
 template <int N>
 static int wkv_forward(WkvParams p, float* start, cudaStream_t stream) {
   const bool vec = wkv_vec_ok(p);
   if (p.NC > 1) {
-    int rc = wkv_launch<N, WK_LOCAL_FWD>(p, vec, p.NC - 1, stream);
+    int rc;
+    if constexpr (N == WN) rc = wkv_col<false, true>(p, vec, p.NC - 1, stream);
+    else rc = wkv_launch<N, WK_LOCAL_FWD>(p, vec, p.NC - 1, stream);
     if (rc != NX_OK) return rc;
     wkv_fold_kernel<N, false><<<dim3(N, p.H, p.B), N, 0, stream>>>(p.local, p.sumew, start, p.NC);
     NX_LAUNCH_CHECK();
     p.start = start;
   }
-  return wkv_launch<N, WK_Y>(p, vec, p.NC, stream);
+  if constexpr (N == WN) return wkv_col<false, false>(p, vec, p.NC, stream);
+  else return wkv_launch<N, WK_Y>(p, vec, p.NC, stream);
 }
 
 template <int N>
 static int wkv_backward(WkvParams p, const float* fstart, float* rstart, float* gu, cudaStream_t stream) {
   const bool vec = wkv_vec_ok(p);
   p.start = p.NC > 1 ? fstart : nullptr;
-  int rc = wkv_launch<N, WK_GR>(p, vec, p.NC, stream);
+  int rc;
+  if constexpr (N == WN) rc = wkv_row<false>(p, vec, stream);
+  else rc = wkv_launch<N, WK_GR>(p, vec, p.NC, stream);
   if (rc != NX_OK) return rc;
   p.start = nullptr;
   if (p.NC > 1) {
-    rc = wkv_launch<N, WK_LOCAL_REV>(p, vec, p.NC - 1, stream);
+    if constexpr (N == WN) rc = wkv_col<true, true>(p, vec, p.NC - 1, stream);
+    else rc = wkv_launch<N, WK_LOCAL_REV>(p, vec, p.NC - 1, stream);
     if (rc != NX_OK) return rc;
     wkv_fold_kernel<N, true><<<dim3(N, p.H, p.B), N, 0, stream>>>(p.local, p.sumew, rstart, p.NC);
     NX_LAUNCH_CHECK();
     p.start = rstart;
     p.fstart = fstart;
   }
-  rc = wkv_launch<N, WK_G>(p, vec, p.NC, stream);
+  if constexpr (N == WN) {
+    rc = wkv_row<true>(p, vec, stream);
+    if (rc == NX_OK) rc = wkv_col<true, false>(p, vec, p.NC, stream);
+  } else {
+    rc = wkv_launch<N, WK_G>(p, vec, p.NC, stream);
+  }
   if (rc != NX_OK) return rc;
   wkv_sum_kernel<<<(p.H * N + WK_SUM_X - 1) / WK_SUM_X, dim3(WK_SUM_X, WK_SUM_Y), 0, stream>>>(p.gu_part, gu, p.B * p.NC,
                                                                                           p.H * N);

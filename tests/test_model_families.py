@@ -131,6 +131,41 @@ def test_wkv6_gradients_repeat_bit_for_bit(B, T, H, N):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,T,H", [(1, 15, 1), (2, 16, 3), (1, 33, 2), (45, 50, 10), (1, 600, 2)])
+@pytest.mark.parametrize("w", [-12.0, -1.0, 2.0, 6.0])
+def test_wkv6_blocks_of_steps(B, T, H, w, dtype):
+    """Heads of 64 in blocks of 16 steps: short blocks, one chunk and many, decays from 1 - 6e-6 to an underflowing one, against
+    64 bits.  One rounding to 16 bits; inside, the sums are of fp32 precision: as many terms as steps and channels."""
+    from gpt_neox_b200.ops.wkv import wkv6
+    torch.manual_seed(11)
+    N = 64
+    mk = lambda m=0.0: (torch.randn(B, T, H * N, device="cuda") * 0.5 + m).to(dtype)
+    leaves = [t.requires_grad_(True) for t in (mk(), mk(), mk(), mk(w))]
+    leaves.append((torch.randn(H, N, device="cuda") * 0.3).to(dtype).requires_grad_(True))
+    gy = mk()
+    y = wkv6(*leaves)
+    got = (y,) + torch.autograd.grad(y, leaves, gy)
+    ref = [t.detach().double().requires_grad_(True) for t in leaves]
+    r, k, v, e = (t.view(B, T, H, N) for t in ref[:4])
+    S, ys = torch.zeros(B, H, N, N, device="cuda", dtype=torch.float64), []
+    for t in range(T):
+        kv = k[:, t, :, :, None] * v[:, t, :, None, :]
+        ys.append((r[:, t, :, :, None] * (ref[4][None, :, :, None] * kv + S)).sum(-2))
+        S = torch.exp(-torch.exp(e[:, t]))[..., None] * S + kv
+    yr = torch.stack(ys, 1).view(B, T, H * N)
+    want = (yr,) + torch.autograd.grad(yr, ref, gy.double())
+    eps = 2 ** -9 if dtype == torch.bfloat16 else 2 ** -12
+    for n, (a, b) in enumerate(zip(got, want)):
+        # (fp16: results below 2^-14 are subnormal, rounded to 2^-25)
+        lim = eps * b.norm() + (2 ** -20 * b.abs().max() + 2 ** -25) * b.numel() ** 0.5
+        if n == 4:
+            # the decay gradient is ew times a running difference of r gr and k gk: T terms of fp32 precision, which cancel
+            lim += T * 2 ** -20 * (ref[0].abs().max() * want[1].abs().max()) * ref[3].exp().max() * b.numel() ** 0.5
+        assert (a.double() - b).norm() <= lim, n
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("what,value", [(0, float("nan")), (1, float("nan")), (2, float("inf")), (3, float("nan"))])
 @pytest.mark.parametrize("at", [0, 40, 331])
 def test_wkv6_passes_nan_and_inf_on(what, value, at):
