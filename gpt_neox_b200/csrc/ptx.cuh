@@ -528,11 +528,12 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
 __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 fadd2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 fmul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-// gelu_erf_both of two values, in packed pairs: x0 / x1 become the activations, d0 / d1 the derivatives.
+// gelu_erf_both of two values, in packed pairs (the same roundings): x0 / x1 become the activations, d0 / d1 the derivatives.
 __device__ __forceinline__ void gelu_erf_both2(float& x0, float& x1, float& d0, float& d1) {
   auto c2 = [](float c) { return make_float2(c, c); };
   const float2 x = make_float2(x0, x1);
-  const float2 den = ffma2(make_float2(fabsf(x0), fabsf(x1)), c2(0.3275911f * 0.70710678118654752440f), c2(1.0f));
+  const float2 ay = fmul2(make_float2(fabsf(x0), fabsf(x1)), c2(0.70710678118654752440f));
+  const float2 den = ffma2(c2(0.3275911f), ay, c2(1.0f));
   const float2 t = make_float2(__fdividef(1.0f, den.x), __fdividef(1.0f, den.y));
   const float2 ex = fmul2(fmul2(x, x), c2(-0.72134752044448170368f));
   const float2 e = make_float2(exp2f(ex.x), exp2f(ex.y));      // exp(-x^2 / 2)
@@ -540,9 +541,8 @@ __device__ __forceinline__ void gelu_erf_both2(float& x0, float& x1, float& d0, 
   poly = ffma2(poly, t, c2(1.421413741f));
   poly = ffma2(poly, t, c2(-0.284496736f));
   poly = ffma2(poly, t, c2(0.254829592f));
-  const float2 q = fmul2(fmul2(fmul2(c2(0.5f), poly), t), e);
-  const float2 up = ffma2(q, c2(-1.0f), c2(1.0f));
-  const float2 cdf = make_float2(x0 < 0.0f ? q.x : up.x, x1 < 0.0f ? q.y : up.y);
+  const float2 nq = fmul2(fmul2(c2(-0.5f), poly), t), q = fmul2(nq, e), up = ffma2(nq, e, c2(1.0f));
+  const float2 cdf = make_float2(x0 < 0.0f ? -q.x : up.x, x1 < 0.0f ? -q.y : up.y);
   const float2 g = fmul2(x, cdf), dg = ffma2(fmul2(x, c2(0.39894228040143267794f)), e, cdf);
   x0 = g.x; x1 = g.y;
   d0 = dg.x; d1 = dg.y;
