@@ -23,9 +23,10 @@ constexpr int DEC_THREADS = 128;
 constexpr int DEC_WARPS = DEC_THREADS / 32;
 constexpr int DEC_MAX_SPLITS = 8;   // portable cluster size
 
+// (not ld.global.nc: this step's key and value row may still be written when the kernel begins)
 __device__ __forceinline__ uint4 ld_stream(const h16* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p));
   return v;
@@ -54,6 +55,8 @@ __global__ void __launch_bounds__(DEC_THREADS, dec_ctas(GT)) attn_decode_kernel(
   const int G = p.H / p.Hk, per_kv = G / GT;
   const int kvh = blockIdx.y / per_kv, head0 = kvh * G + (blockIdx.y % per_kv) * GT, b = blockIdx.z;
   const bool live = dl < p.D;                 // D below DP: the last lanes of a group hold zeros
+  allow_dependents();
+  grid_dependency_wait();
 
   constexpr bool Q16 = GT >= 4;               // many heads: q stays packed, 4 registers a head
   uint32_t qp[Q16 ? GT : 1][4];
@@ -258,17 +261,8 @@ static int launch(const AttnDecodeParams& p, cudaStream_t stream) {
     }
   }
   const int per = (keys + splits - 1) / splits;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(splits, rows, p.B);
-  cfg.blockDim = dim3(DEC_THREADS);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = splits;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  NX_CUDA_CHECK(cudaLaunchKernelEx(&cfg, attn_decode_kernel<DP, GT>, p, per));
+  NX_CUDA_CHECK(launch_dependent(attn_decode_kernel<DP, GT>, dim3(splits, rows, p.B), dim3(DEC_THREADS), 0, stream, splits, p,
+                                 per));
   return NX_OK;
 }
 

@@ -39,6 +39,28 @@ bool make_tma_4d(CUtensorMap* map, const void* base, const uint64_t dims[4],
                  const uint64_t strides_bytes[3], const uint32_t box[4], int elem_bytes,
                  bool swizzle128 = true);
 
+// Launches a kernel that may begin while the one before it in the stream is still running (ptx.cuh,
+// grid_dependency_wait): the launch itself and the kernel's set-up then lie under that one's end.  cluster: blocks per cluster
+// along x.
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, int smem, cudaStream_t stream, int cluster,
+                                    A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 0 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 }  // namespace nx
 
 // The kernels that work on 16-bit floating-point tensors are compiled twice from the same sources:

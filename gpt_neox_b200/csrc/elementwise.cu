@@ -78,6 +78,8 @@ __global__ void bias_act_fwd_kernel(const h16* __restrict__ x,
 // fp32 with one rounding.  out may be any of the inputs.  Bound by its launch for the few rows of a generation step.
 __global__ void branch_sum_kernel(const h16* x, const h16* a, const h16* ba, const h16* m, const h16* bm, h16* out,
                                   long long nvec, int ncols8) {
+  allow_dependents();
+  grid_dependency_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
     const int c = static_cast<int>(i % ncols8) * 8;
     float s[8], p[8], q[8], b[8];
@@ -123,10 +125,11 @@ __global__ void bias_act_bwd_kernel(const h16* __restrict__ dy,
 }
 
 // x: [rows, 2F] = [value | gate];  y[r, f] = value * act(gate)
-__global__ void gated_act_fwd_kernel(const h16* __restrict__ x,
-                                     h16* __restrict__ y, long long rows, int F, int act) {
+__global__ void gated_act_fwd_kernel(const h16* x, h16* y, long long rows, int F, int act) {
   const int f8 = F >> 3;
   const long long nvec = rows * f8;
+  allow_dependents();
+  grid_dependency_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvec;
        i += (long long)gridDim.x * blockDim.x) {
     const long long r = i / f8;
@@ -318,10 +321,9 @@ NX_API int NX_SYM(nx_branch_sum)(const void* x, const void* a, const void* ba, c
              "branch_sum: operands must be 16-byte aligned");
   const long long nvec = rows * (cols / 8);
   if (nvec == 0) return NX_OK;
-  branch_sum_kernel<<<grid_for(nvec, 256), 256, 0, (cudaStream_t)stream_>>>((const bf*)x, (const bf*)a, (const bf*)ba,
-                                                                           (const bf*)m, (const bf*)bm, (bf*)out, nvec,
-                                                                           cols / 8);
-  NX_LAUNCH_CHECK();
+  NX_CUDA_CHECK(launch_dependent(branch_sum_kernel, dim3(grid_for(nvec, 256)), dim3(256), 0, (cudaStream_t)stream_, 0,
+                                 (const bf*)x, (const bf*)a, (const bf*)ba, (const bf*)m, (const bf*)bm, (bf*)out, nvec,
+                                 cols / 8));
   return NX_OK;
 }
 NX_API int NX_SYM(nx_bias_act_bwd)(const void* dy, const void* x, const void* bias, void* dx, long long rows,
@@ -340,9 +342,8 @@ NX_API int NX_SYM(nx_gated_act_fwd)(const void* x, void* y, long long rows, int 
   NX_REQUIRE(F % 8 == 0, "gated_act: F %% 8 != 0");
   const long long nvec = rows * (F / 8);
   if (nvec == 0) return NX_OK;
-  gated_act_fwd_kernel<<<grid_for(nvec, 256), 256, 0, (cudaStream_t)stream_>>>((const bf*)x, (bf*)y,
-                                                                              rows, F, act);
-  NX_LAUNCH_CHECK();
+  NX_CUDA_CHECK(launch_dependent(gated_act_fwd_kernel, dim3(grid_for(nvec, 256)), dim3(256), 0, (cudaStream_t)stream_, 0,
+                                 (const bf*)x, (bf*)y, rows, F, act));
   return NX_OK;
 }
 NX_API int NX_SYM(nx_gated_act_bwd)(const void* dy, const void* x, void* dx, long long rows, int F, int act,

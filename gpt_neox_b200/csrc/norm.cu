@@ -121,11 +121,11 @@ __global__ void norm_fwd_kernel(const h16* __restrict__ x,
 constexpr int WARP_ROW_MAX_NV = 3;
 template <bool RMS, int NV>
 __global__ void __launch_bounds__(256, 4)
-norm_fwd_warp_kernel(const h16* __restrict__ x, const h16* __restrict__ g1, const h16* __restrict__ b1,
-                     h16* __restrict__ y1, const h16* __restrict__ g2, const h16* __restrict__ b2,
-                     h16* __restrict__ y2, float* __restrict__ mean_out, float* __restrict__ rstd_out, long long rows,
-                     int H, float eps) {
+norm_fwd_warp_kernel(const h16* x, const h16* g1, const h16* b1, h16* y1, const h16* g2, const h16* b2, h16* y2,
+                     float* mean_out, float* rstd_out, long long rows, int H, float eps) {
   const long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  allow_dependents();
+  grid_dependency_wait();
   if (row >= rows) return;
   const int lane = threadIdx.x & 31, nv = H >> 3;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * H);
@@ -620,8 +620,9 @@ NX_API int NX_SYM(nx_norm_fwd)(int kind, const void* x, const void* g1, const vo
     const int wpb = rows >= 8ll * sm_count() ? 8 : rows >= 2ll * sm_count() ? 2 : 1;
     const unsigned grid = static_cast<unsigned>((rows + wpb - 1) / wpb);
 #define NX_NORM_WARP(R, NV)                                                                                        \
-  norm_fwd_warp_kernel<R, NV><<<grid, wpb * 32, 0, s>>>((const bf*)x, (const bf*)g1, (const bf*)b1, (bf*)y1, (const bf*)g2, \
-                                                  (const bf*)b2, (bf*)y2, (float*)mean, (float*)rstd, rows, H, eps)
+  NX_CUDA_CHECK(launch_dependent(norm_fwd_warp_kernel<R, NV>, dim3(grid), dim3(wpb * 32), 0, s, 0, (const bf*)x,        \
+                                 (const bf*)g1, (const bf*)b1, (bf*)y1, (const bf*)g2, (const bf*)b2, (bf*)y2,          \
+                                 (float*)mean, (float*)rstd, rows, H, eps))
 #define NX_NORM_WARP_NV(R)                \
   do {                                    \
     if (nvl <= 2) NX_NORM_WARP(R, 2);     \

@@ -172,6 +172,20 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* er
 }
 
 // ---------------------------------------------------------------------------
+// programmatic dependent launch: a kernel launched by launch_dependent (common.h) may begin while the one before it in its
+// stream is still running.  What it does before grid_dependency_wait must touch no memory that a kernel could write (setting up
+// barriers and tensor memory, prefetching into L2); every block passes the wait, so that the completion of a kernel
+// implies that of all before it, whatever the next one waits for.  allow_dependents lets the next one begin.
+// Inputs of such a kernel are not `const __restrict__` (nor read by ld.global.nc): they may still be written when it begins.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* m, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y)
+               : "memory");
+}
+
+// ---------------------------------------------------------------------------
 // TMA (tiled bulk tensor copies, this GPU's memory -> this CTA's shared memory)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {

@@ -134,6 +134,8 @@ __global__ void __launch_bounds__(256) rope_qk_kernel(const RopeQKArgs a) {
   const unsigned n_q = a.NQ * a.G, n_k = a.NK * a.G, n_u = a.NQ * a.QT, n_t = a.NK * a.KT,
                  per = n_q + n_k + n_u + n_t + a.NK * a.VT;
   const unsigned i = blockIdx.x * 256u + threadIdx.x, tok = i / per;
+  allow_dependents();
+  grid_dependency_wait();
   if (tok >= a.tokens) return;
   unsigned r = i - tok * per;
   const unsigned s = tok / a.B, b = tok - s * a.B;
@@ -267,8 +269,8 @@ NX_API int NX_SYM(nx_rope_qk)(const void* q, const void* k, const void* v, void*
   const long long total = static_cast<long long>(S) * B * per;
   if (total == 0) return NX_OK;
   NX_REQUIRE(total < (1ll << 31), "rope_qk: too many elements");
-  rope_qk_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream_>>>(a);
-  NX_LAUNCH_CHECK();
+  NX_CUDA_CHECK(launch_dependent(rope_qk_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, (cudaStream_t)stream_, 0,
+                                 a));
   return NX_OK;
 }
 NX_API int NX_SYM(nx_embedding_fwd)(const void* ids, const void* table, void* out, long long n, int H,

@@ -816,3 +816,57 @@ def test_branch_sum_of_other_types_shapes_and_alignments():
     assert rel(branch_sum(x, a, b, none, None), want - m.float()) < 1e-2
     cpu = branch_sum(*(t.cpu() for t in (x, a, b, m)), None)
     assert rel(cpu.to(DEV), want) < 2e-2
+
+
+@pytest.mark.parametrize("captured", [False, True], ids=["eager", "graph"])
+@pytest.mark.parametrize("rows,h,f", [(1, 512, 256), (4, 1024, 2816), (64, 768, 1024)])
+def test_dependent_launches_see_what_the_kernel_before_wrote(rows, h, f, captured):
+    """Kernels that may begin while the one before them runs (few-rows GEMM, gated activation, norm): every input, the weights
+    too, is written by the kernel right before.  The same chain with a synchronisation after every launch gives the same bits."""
+    from gpt_neox_b200.ops.elementwise import gated_act
+    from gpt_neox_b200.ops.gemm import gemm
+    from gpt_neox_b200.ops.norm import layer_norm
+    torch.manual_seed(5)
+    x, w1, w2, g, b = bf(rows, h), bf(2 * f, h, scale=0.05), bf(h, f, scale=0.05), bf(h), bf(h)
+    step = torch.zeros((), device=DEV, dtype=DT)
+
+    def chain(pause):
+        step.add_(0.25)
+        outs = []
+        y = x * step
+        for _ in range(3):
+            pause()
+            a, c = w1 * step, w2 * step
+            pause()
+            u = gemm(y, a)
+            pause()
+            u = gated_act(u, "swiglu")
+            pause()
+            u = gemm(u, c)
+            pause()
+            y = layer_norm(u, g, b)
+            pause()
+            outs += [u, y]
+        return outs
+
+    with torch.no_grad():
+        want = []
+        for _ in range(6):
+            want.append([t.clone() for t in chain(torch.cuda.synchronize)])
+        step.zero_()
+        if captured:
+            graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                chain(lambda: None)
+            torch.cuda.current_stream().wait_stream(side)
+            with torch.cuda.graph(graph):
+                outs = chain(lambda: None)
+            step.zero_()
+        for ref in want:
+            if captured:
+                graph.replay()
+            else:
+                outs = chain(lambda: None)
+            for got, r in zip(outs, ref):
+                assert torch.equal(got, r)
