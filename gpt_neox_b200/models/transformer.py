@@ -472,22 +472,23 @@ class ParallelTransformerLayer(nn.Module):
                 and mpu.get_model_parallel_world_size() == 1 and m._fusable(x)):
             return None
         hn = a.hidden_size_per_attention_head
-        linears = (a.query_key_value, a.dense, m.linear1, m.linear2)
+        linears = (_sub(a, "query_key_value"), _sub(a, "dense"), _sub(m, "linear1"), _sub(m, "linear2"))
+        n1, n2, rotary = self.input_layernorm, self.post_attention_layernorm, _sub(a, "rotary_emb")
         if hn % 8 or hn > 128 or a.rotary_dim % 16 \
                 or not (_plain(linears[0], mpu.ColumnParallelLinear) and _plain(linears[2], mpu.ColumnParallelLinear)
                         and _plain(linears[1], mpu.RowParallelLinear) and _plain(linears[3], mpu.RowParallelLinear)
-                        and _plain(a.rotary_emb, RotaryEmbedding) and _plain(self.input_layernorm, LayerNorm)
-                        and _plain(self.post_attention_layernorm, LayerNorm)) \
+                        and _plain(rotary, RotaryEmbedding) and _plain(n1, LayerNorm) and _plain(n2, LayerNorm)) \
                 or any(l.use_mup or l.use_fp8 or getattr(l, "gather_output", False) for l in linears) \
                 or linears[0].skip_bias_add or torch.nn.modules.module._has_any_global_hook():
             return None
-        n1, n2, up = self.input_layernorm, self.post_attention_layernorm, m.linear1.weight
-        ptrs = pointers(x, n1.weight, n1.bias, n2.weight, n2.bias, *(t for l in linears for t in (l.weight, l.bias)))
+        weights = [t for l in (n1, n2) + linears for t in (_param(l, "weight"), _param(l, "bias"))]
+        up = weights[8]
+        ptrs = pointers(x, *weights)
         if ptrs is None or n1.eps != n2.eps:
             return None
         has_past = layer_past is not None and (not torch.is_tensor(layer_past) or layer_past.numel() > 0)
         past = layer_past[0].shape[0] if has_past else 0
-        cos, sin = a.rotary_emb(seq_len=x.shape[0] + past)
+        cos, sin = rotary(seq_len=x.shape[0] + past)
         if (cos.data_ptr() | sin.data_ptr()) & 15:
             return None
         kvp = a.num_kv_heads_per_partition
@@ -609,6 +610,21 @@ def _plain(m, cls):
     d = m.__dict__
     return type(m) is cls and cls.forward is _FORWARD[cls] and "forward" not in d and not d["_forward_hooks"] \
         and not d["_forward_pre_hooks"]
+
+
+def _sub(m, name):
+    """``getattr(m, name)`` for a submodule of a module that is plain (its class has no attribute of that name), without the
+    module's ``__getattr__`` where nothing in the instance stands before it."""
+    d = m.__dict__
+    found = None if name in d else d["_modules"].get(name)
+    return found if found is not None else getattr(m, name)
+
+
+def _param(m, name):
+    """``getattr(m, name)`` for a parameter (or None), likewise."""
+    d = m.__dict__
+    params = d["_parameters"]
+    return params[name] if name in params and name not in d else getattr(m, name)
 
 
 def _sum_bias(a, b):

@@ -113,7 +113,8 @@ class SequentialWrapper(nn.Module):
             def exec_func(*inputs):
                 if len(inputs) == 1:
                     inputs = inputs[0]
-                for layer in self.sequential[start:end]:
+                # (a slice of an nn.Sequential is a new one with every layer registered again)
+                for layer in list(self.sequential._modules.values())[start:end]:
                     inputs = layer(inputs)
                 return inputs
             return exec_func

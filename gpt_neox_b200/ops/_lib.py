@@ -180,7 +180,8 @@ def untracked() -> bool:
 
 
 def stream():
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    # (torch.cuda.current_stream() builds a Stream object around this number)
+    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def read_device_error(clear: bool = True) -> int:
