@@ -20,12 +20,15 @@
 //              Q_t[i] = sum_j G_t[i][j] S_t[i][j] one has Q_{t-1} - Q_t = r_t gr_t - k_t gk_t and
 //              dL/d(ew_t) = Q_t - k_t (gk_t - r_t u s_t),  s_t = <gy_t, v_t>,  ew = -exp(w)
 // Step by step the shared-memory loads and exchanges of the steps are the bound (32 x 512 tokens, 12 heads of 64, forward +
-// backward 788 us); 581 us with the products of
-// a block in their place (125 us for each sweep, 190 for gk with the decay gradient).
+// backward 788 us); 570 us with the products of
+// a block in their place (125 us for each sweep, 175 for gk with the decay gradient).  Those are bound by latency at 2.6 warps per
+// scheduler (issue slots 46 % busy, tensor pipe 25 %).
 //
 // The sequence is cut into chunks only when batch x heads leaves the chip idle (wkv_chunk_count): the recurrence is
 // linear, so a chunk's end state is  P (.) S_start + S_local  with P[i] = prod_t d_t[i]; local passes start every chunk
 // from zero, a fold gives the chunks' start states, and Q at a chunk's end is <G, S> there.
+#include <stddef.h>
+
 #include "common.h"
 #include "ptx.cuh"
 
@@ -436,13 +439,22 @@ __device__ __forceinline__ int wm_time(int t_lo, int t_hi, int q, int s) {
 }
 
 struct WmColSmem {
-  WmIn a, b, c;
+  WmIn a, b;
   float d[WM][WN];
-  uint16_t ap[3][WM][WP], bp[3][WM][WP];     // parts of a Pre, b Suf
-  uint16_t A[3][WM][24];
-  float tot[WN];
-  uint16_t out[WM][WP];
+  struct alignas(16) Block {                 // what the products of block q read and give, in slot q & 1
+    WmIn c;
+    uint16_t ap[3][WM][WP], bp[3][WM][WP];   // parts of a Pre, b Suf
+    uint16_t A[3][WM][24];
+    uint16_t out[WM][WP];
+    float tot[WN];
+    bool finite;
+  } blk[2];
 };
+static_assert(offsetof(WmColSmem, d) % 16 == 0 && offsetof(WmColSmem, blk) % 16 == 0 && sizeof(WmColSmem::Block) % 16 == 0 &&
+                  offsetof(WmColSmem::Block, ap) % 16 == 0 && offsetof(WmColSmem::Block, bp) % 16 == 0 &&
+                  offsetof(WmColSmem::Block, A) % 16 == 0 && offsetof(WmColSmem::Block, out) % 16 == 0 &&
+                  offsetof(WmColSmem::Block, tot) % 16 == 0,
+              "ldmatrix and 16-byte accesses");
 
 // Column sums (y, or gv in reverse), or (LOCAL) only the end state of a chunk from a zero state and the sums of ew.
 template <bool REV, bool LOCAL, bool VEC>
@@ -465,7 +477,7 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
       if (!LOCAL && p.start != nullptr) S[n][e] = p.start[(base * WN + 8 * n + i0 + (e & 1)) * WN + j0 + (e >> 1) * 8];
     }
   // the zeros of A (its upper triangle is never written)
-  for (int x = tid; x < 3 * WM * 24; x += WM_THREADS) (&s.A[0][0][0])[x] = 0;
+  for (int x = tid; x < 3 * WM * 24; x += WM_THREADS) (&s.blk[0].A[0][0][0])[x] = (&s.blk[1].A[0][0][0])[x] = 0;
   const int trow = tid >> 3, ch8 = (tid & 7) * 8;
   float sew[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const int nblk = (t_hi - t_lo + WM - 1) / WM;
@@ -481,11 +493,15 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
     rw = wk_load8<VEC>(p.w + o, live);
   };
   fetch(0);
-  for (int q = 0; q < nblk; ++q) {
-    if (!LOCAL) s.a.put(trow, ch8, ra);
-    s.b.put(trow, ch8, rb);
-    s.c.put(trow, ch8, rc);
-    {
+  // Round q: block q is staged, then its vectors (a Pre, b Suf, A) and the products of block q - 1 come between the same two
+  // barriers, so that the warps' unequal vector work and the latencies of the two overlap.
+  for (int q = 0; q <= nblk; ++q) {
+    auto& now = s.blk[q & 1];
+    auto& former = s.blk[(q & 1) ^ 1];
+    if (q < nblk) {
+      if (!LOCAL) s.a.put(trow, ch8, ra);
+      s.b.put(trow, ch8, rb);
+      now.c.put(trow, ch8, rc);
       float w8[8], d8[8];
       wk_unpack8(rw, w8);
 #pragma unroll
@@ -497,9 +513,16 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
       *reinterpret_cast<float4*>(&s.d[trow][ch8]) = make_float4(d8[0], d8[1], d8[2], d8[3]);
       *reinterpret_cast<float4*>(&s.d[trow][ch8 + 4]) = make_float4(d8[4], d8[5], d8[6], d8[7]);
     }
-    const bool finite = !__syncthreads_or(!LOCAL && !wm_all_finite(rc));
-    if (q + 1 < nblk) fetch(q + 1);      // in flight during this block
-    if (warp == 0) {
+    const bool all_finite = !__syncthreads_or(!LOCAL && q < nblk && !wm_all_finite(rc));
+    if (tid == 0) now.finite = all_finite;
+    if (q + 1 < nblk) fetch(q + 1);      // in flight during this round
+    if (!LOCAL && q > 1) {               // (the sums of block q - 2, laid out in the last round)
+      const int t = wm_time<REV>(t_lo, t_hi, q - 2, trow);
+      if (t >= t_lo && t < t_hi)
+        *reinterpret_cast<uint4*>((REV ? p.o_gv : p.y) + bi * p.osb + (long long)t * p.ost + h * WN + ch8) =
+            *reinterpret_cast<const uint4*>(&now.out[trow][ch8]);
+    }
+    if (q < nblk && warp == 0) {
       // a Pre, and Tot; two channels per thread
       const int c = lane * 2;
       float2 pre = make_float2(1.f, 1.f);
@@ -510,12 +533,12 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
           uint32_t x[3];
           wm_split(fmul2(s.a.pair(t, c), pre), x);
 #pragma unroll
-          for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&s.ap[k][t][c]) = x[k];
+          for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&now.ap[k][t][c]) = x[k];
         }
         pre = fmul2(pre, d);
       }
-      *reinterpret_cast<float2*>(&s.tot[c]) = pre;
-    } else if (warp == 1) {
+      *reinterpret_cast<float2*>(&now.tot[c]) = pre;
+    } else if (q < nblk && warp == 1) {
       const int c = lane * 2;
       float2 suf = make_float2(1.f, 1.f);
 #pragma unroll 4
@@ -524,10 +547,10 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
         uint32_t x[3];
         wm_split(fmul2(s.b.pair(t, c), suf), x);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&s.bp[k][t][c]) = x[k];
+        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(&now.bp[k][t][c]) = x[k];
         suf = fmul2(suf, d);
       }
-    } else if (!LOCAL) {
+    } else if (!LOCAL && q < nblk) {
       // A: eight groups of eight lanes (8 channels each); group g takes columns s = g and s = 15 - g, 15 entries together
       const int g = (tid - 64) >> 3, c = (tid & 7) * 8, turn = WM - 1 - g;
       float2 qv[4];
@@ -583,7 +606,7 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
         uint32_t y[3];
         wm_split(make_float2(x, 0.f), y);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) s.A[k][t][col] = static_cast<uint16_t>(y[k]);
+        for (int k = 0; k < 3; ++k) now.A[k][t][col] = static_cast<uint16_t>(y[k]);
       };
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
@@ -594,13 +617,14 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
       }
       if ((lane & 7) == 0) put_A(turn, turn, diag);
     }
-    __syncthreads();
-    // ---- products
+    if (q > 0) {
+    // ---- products of block q - 1
     uint32_t cv[WM_IN][4];               // c^T: 16 rows j of this warp x 16 steps
 #pragma unroll
-    for (int k = 0; k < WM_IN; ++k) wm_ld4<true>(cv[k], s.c.parts(k), 0, warp * 16, WP, false);
+    for (int k = 0; k < WM_IN; ++k) wm_ld4<true>(cv[k], former.c.parts(k), 0, warp * 16, WP, false);
     if (!LOCAL) {
       float y[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      float z[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};      // (two chains of dependent products)
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
         uint32_t sp[3][4];               // S^T[16 j][16 i]
@@ -614,19 +638,24 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
           uint32_t b[4];
-          wm_ld4<false>(b, &s.ap[k][0][0], 0, 16 * ks, WP, false);
+          wm_ld4<false>(b, &former.ap[k][0][0], 0, 16 * ks, WP, false);
 #pragma unroll
           for (int m = 2 - k; m >= 0; --m) {
-            wm_mma(y[0], sp[m], b[0], b[1]);
-            wm_mma(y[1], sp[m], b[2], b[3]);
+            wm_mma(m & 1 ? z[0] : y[0], sp[m], b[0], b[1]);
+            wm_mma(m & 1 ? z[1] : y[1], sp[m], b[2], b[3]);
           }
         }
       }
-      if (finite) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        y[0][e] += z[0][e];
+        y[1][e] += z[1][e];
+      }
+      if (former.finite) {
 #pragma unroll
         for (int k = 2; k >= 0; --k) {
           uint32_t b[4];
-          wm_ld4<false>(b, &s.A[k][0][0], 0, 0, 24, false);
+          wm_ld4<false>(b, &former.A[k][0][0], 0, 0, 24, false);
 #pragma unroll
           for (int m = 0; m < WM_IN; ++m) {
             wm_mma(y[0], cv[m], b[0], b[1]);
@@ -641,8 +670,8 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
             const int t = 8 * n + i0 + (e & 1), j = j0 + (e >> 1) * 8;
             for (int x = 0; x <= t; ++x) {
               float a = 0.f;
-              for (int k = 2; k >= 0; --k) a += __uint_as_float(static_cast<uint32_t>(s.A[k][t][x]) << 16);
-              y[n][e] += a * s.c.at(x, j);
+              for (int k = 2; k >= 0; --k) a += __uint_as_float(static_cast<uint32_t>(former.A[k][t][x]) << 16);
+              y[n][e] += a * former.c.at(x, j);
             }
           }
       }
@@ -651,12 +680,12 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const h16 o = float_to_h16(y[n][e]);
-          s.out[8 * n + i0 + (e & 1)][j0 + (e >> 1) * 8] = reinterpret_cast<const uint16_t&>(o);
+          former.out[8 * n + i0 + (e & 1)][j0 + (e >> 1) * 8] = reinterpret_cast<const uint16_t&>(o);
         }
     }
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
-      const float2 d = *reinterpret_cast<const float2*>(&s.tot[8 * n + i0]);
+      const float2 d = *reinterpret_cast<const float2*>(&former.tot[8 * n + i0]);
       S[n][0] *= d.x; S[n][1] *= d.y; S[n][2] *= d.x; S[n][3] *= d.y;
     }
 #pragma unroll
@@ -664,21 +693,21 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
 #pragma unroll
       for (int k = 2; k >= 0; --k) {
         uint32_t b[4];
-        wm_ld4<true>(b, &s.bp[k][0][0], 0, 8 * n, WP, true);
+        wm_ld4<true>(b, &former.bp[k][0][0], 0, 8 * n, WP, true);
 #pragma unroll
         for (int m = 0; m < WM_IN; ++m) {
           wm_mma(S[n], cv[m], b[0], b[1]);
           wm_mma(S[n + 1], cv[m], b[2], b[3]);
         }
       }
-    __syncthreads();
-    if (!LOCAL) {
-      const int t = wm_time<REV>(t_lo, t_hi, q, trow);
-      if (t >= t_lo && t < t_hi)
-        *reinterpret_cast<uint4*>((REV ? p.o_gv : p.y) + bi * p.osb + (long long)t * p.ost + h * WN + ch8) =
-            *reinterpret_cast<const uint4*>(&s.out[trow][ch8]);
-      // (`out` is written again after the next block's two barriers)
     }
+    __syncthreads();
+  }
+  if (!LOCAL) {
+    const int t = wm_time<REV>(t_lo, t_hi, nblk - 1, trow);
+    if (t >= t_lo && t < t_hi)
+      *reinterpret_cast<uint4*>((REV ? p.o_gv : p.y) + bi * p.osb + (long long)t * p.ost + h * WN + ch8) =
+          *reinterpret_cast<const uint4*>(&s.blk[(nblk - 1) & 1].out[trow][ch8]);
   }
   if (LOCAL) {
 #pragma unroll
@@ -699,16 +728,22 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
 }
 
 struct WmRowSmem {
-  WmIn b, c, e;
-  uint16_t k[WM][WP];                        // gk: the other factor of the decay gradient
-  float d[WM][WN], ew[WM][WN];
-  uint16_t bp[3][WM][WP];
+  float d[WM][WN];
   float M[2][WM][8];                         // <e_t, c_s>: s even | odd
-  float st[WM];
-  float part[2][WM][WN];                     // what a block's own steps add, by the parity of s
-  float pre[WM][WN], tot[WN];
   float inter[WM][WN + 4];
+  struct alignas(16) Block {                 // of block q, in slot q & 1
+    WmIn b, c, e;
+    uint16_t k[WM][WP];                      // gk: the other factor of the decay gradient
+    float ew[WM][WN];
+    uint16_t bp[3][WM][WP];
+    float st[WM];
+    float part[2][WM][WN];                   // what a block's own steps add, by the parity of s
+    float pre[WM][WN], tot[WN];
+  } blk[2];
 };
+static_assert(offsetof(WmRowSmem, M) % 16 == 0 && offsetof(WmRowSmem, blk) % 16 == 0 && sizeof(WmRowSmem::Block) % 16 == 0 &&
+                  offsetof(WmRowSmem::Block, k) % 16 == 0 && offsetof(WmRowSmem::Block, bp) % 16 == 0,
+              "ldmatrix and 16-byte accesses");
 
 // Row sums: gr (fp32 and rounded), or in reverse gk with the decay gradient and the sums for the gradient of u.
 template <bool REV, bool VEC>
@@ -751,43 +786,50 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_row_kernel(const WkvParams 
     if (REV) rk = wk_load8<VEC>(p.k + o, live);
   };
   fetch(0);
-  for (int q = 0; q < nblk; ++q) {
-    const int steps = min(WM, t_hi - t_lo - q * WM);
-    s.b.put(trow, ch8, rb);
-    s.c.put(trow, ch8, rc);
-    s.e.put(trow, ch8, re);
-    if (REV) *reinterpret_cast<uint4*>(&s.k[trow][ch8]) = rk;
+  // Round q: block q is staged; M of block q and the products of block q - 1; the results of block q - 1 and what block q's own
+  // steps add.  Three barriers a round.
+  const long long oo = bi * p.osb + h * WN + me;
+  for (int q = 0; q <= nblk; ++q) {
+    auto& now = s.blk[q & 1];
+    auto& former = s.blk[(q & 1) ^ 1];
+    const int steps = min(WM, t_hi - t_lo - (q - 1) * WM);      // of block q - 1
+    if (q < nblk) {
+    now.b.put(trow, ch8, rb);
+    now.c.put(trow, ch8, rc);
+    now.e.put(trow, ch8, re);
+    if (REV) *reinterpret_cast<uint4*>(&now.k[trow][ch8]) = rk;
     {
       float w8[8];
       wk_unpack8(rw, w8);
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const float ew = live ? -__expf(w8[e]) : 0.f;
-        s.ew[trow][ch8 + e] = ew;
+        now.ew[trow][ch8 + e] = ew;
         s.d[trow][ch8 + e] = __expf(ew);
       }
     }
+    }
     __syncthreads();
-    if (q + 1 < nblk) fetch(q + 1);      // in flight during this block
-    const long long oo = bi * p.osb + h * WN + me;
+    if (q + 1 < nblk) fetch(q + 1);      // in flight during this round
     float gr[REV ? WM : 1];
-    if (REV && half == 0) {
+    if (REV && half == 0 && q > 0) {
 #pragma unroll
-      for (int t = 0; t < WM; ++t) gr[REV ? t : 0] = t < steps ? p.gr32[oo + (long long)(t_hi - 1 - q * WM - t) * p.ost] : 0.f;
+      for (int t = 0; t < WM; ++t)
+        gr[REV ? t : 0] = t < steps ? p.gr32[oo + (long long)(t_hi - 1 - (q - 1) * WM - t) * p.ost] : 0.f;
     }
     // ---- M: warp 0 the first eight s, warp 1 the others
-    if (warp < 2) {
+    if (q < nblk && warp < 2) {
       float m4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks)
 #pragma unroll
         for (int x = 0; x < WM_IN; ++x) {
           uint32_t a[4];
-          wm_ld4<false>(a, s.e.parts(x), 0, 16 * ks, WP, true);
+          wm_ld4<false>(a, now.e.parts(x), 0, 16 * ks, WP, true);
 #pragma unroll
           for (int z = 0; z < WM_IN; ++z) {
             uint32_t b[4];
-            wm_ld4<false>(b, s.c.parts(z), 0, 16 * ks, WP, false);
+            wm_ld4<false>(b, now.c.parts(z), 0, 16 * ks, WP, false);
             wm_mma(m4, a, warp == 0 ? b[0] : b[2], warp == 0 ? b[1] : b[3]);
           }
         }
@@ -795,10 +837,90 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_row_kernel(const WkvParams 
       for (int e = 0; e < 4; ++e) {
         const int t = (lane >> 2) + (e >> 1) * 8, x = warp * 8 + n0 + (e & 1);
         s.M[x & 1][t][x >> 1] = m4[e];
-        if (t == x) s.st[t] = m4[e];
+        if (t == x) now.st[t] = m4[e];
       }
     }
+    if (q > 0) {
+    // ---- products
+    {
+      float y[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) {
+        uint32_t sp[3][4];               // S[16 i][16 j]
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          uint32_t x[3];
+          const float* src = S[2 * ks + (e >> 1)] + (e & 1) * 2;
+          wm_split(make_float2(src[0], src[1]), x);
+          sp[0][e] = x[0]; sp[1][e] = x[1]; sp[2][e] = x[2];
+        }
+#pragma unroll
+        for (int z = 0; z < WM_IN; ++z) {
+          uint32_t b[4];
+          wm_ld4<false>(b, former.e.parts(z), 0, 16 * ks, WP, false);
+#pragma unroll
+          for (int m = 2; m >= 0; --m) {
+            wm_mma(y[0], sp[m], b[0], b[1]);
+            wm_mma(y[1], sp[m], b[2], b[3]);
+          }
+        }
+      }
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s.inter[8 * n + n0 + (e & 1)][r0 + (e >> 1) * 8] = y[n][e];
+      const float t0 = former.tot[r0], t1 = former.tot[r0 + 8];
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        S[n][0] *= t0; S[n][1] *= t0; S[n][2] *= t1; S[n][3] *= t1;
+      }
+      uint32_t bt[3][4];                 // (b Suf)^T: 16 rows i x 16 steps
+#pragma unroll
+      for (int k = 0; k < 3; ++k) wm_ld4<true>(bt[k], &former.bp[k][0][0], 0, warp * 16, WP, false);
+#pragma unroll
+      for (int n = 0; n < 8; n += 2)
+#pragma unroll
+        for (int z = 0; z < WM_IN; ++z) {
+          uint32_t b[4];
+          wm_ld4<true>(b, former.c.parts(z), 0, 8 * n, WP, true);
+#pragma unroll
+          for (int k = 2; k >= 0; --k) {
+            wm_mma(S[n], bt[k], b[0], b[1]);
+            wm_mma(S[n + 1], bt[k], b[2], b[3]);
+          }
+        }
+    }
+    }
     __syncthreads();
+    if (q > 0) {
+    // ---- results
+    if (!REV) {
+#pragma unroll
+      for (int x = 0; x < WM / 2; ++x) {
+        const int t = half * (WM / 2) + x;
+        if (t >= steps) continue;
+        const float row = former.pre[t][me] * s.inter[t][me] + (former.part[0][t][me] + former.part[1][t][me]);
+        const float gr = row + u_me * former.b.at(t, me) * former.st[t];
+        const long long o = oo + (long long)(t_lo + (q - 1) * WM + t) * p.ost;
+        p.gr32[o] = gr;
+        p.o_gr[o] = float_to_h16(gr);
+      }
+    } else if (half == 0) {
+#pragma unroll
+      for (int t = 0; t < WM; ++t) {
+        if (t >= steps) continue;
+        const float row = former.pre[t][me] * s.inter[t][me] + (former.part[0][t][me] + former.part[1][t][me]);
+        const float r_ = former.b.at(t, me), k_ = h16_to_float(reinterpret_cast<const h16&>(former.k[t][me])), st = former.st[t];
+        const float gk = row + u_me * r_ * st;
+        const long long o = oo + (long long)(t_hi - 1 - (q - 1) * WM - t) * p.ost;
+        p.o_gk[o] = float_to_h16(gk);
+        p.o_gw[o] = float_to_h16((Q - k_ * row) * former.ew[t][me]);
+        Q += r_ * gr[REV ? t : 0] - k_ * gk;
+        gu += r_ * k_ * st;
+      }
+    }
+    }
+    if (q < nblk) {
     // ---- a block's own steps, for one channel and every second s
     {
       float qv[8], pre = 1.f;
@@ -819,98 +941,22 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_row_kernel(const WkvParams 
             qv[x] *= d;
           }
         }
-        if ((t & 1) == half) qv[t >> 1] = s.b.at(t, me);
-        s.part[half][t][me] = acc;
+        if ((t & 1) == half) qv[t >> 1] = now.b.at(t, me);
+        now.part[half][t][me] = acc;
         if (half == 0) {
-          s.pre[t][me] = pre;
+          now.pre[t][me] = pre;
           pre *= d;
         }
       }
-      if (half == 0) s.tot[me] = pre;
+      if (half == 0) now.tot[me] = pre;
 #pragma unroll
       for (int x = 0; x < 8; ++x) {
         uint32_t y[3];
         wm_split(make_float2(qv[x], 0.f), y);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) s.bp[k][2 * x + half][me] = static_cast<uint16_t>(y[k]);
+        for (int k = 0; k < 3; ++k) now.bp[k][2 * x + half][me] = static_cast<uint16_t>(y[k]);
       }
     }
-    __syncthreads();
-    // ---- products
-    {
-      float y[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-        uint32_t sp[3][4];               // S[16 i][16 j]
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          uint32_t x[3];
-          const float* src = S[2 * ks + (e >> 1)] + (e & 1) * 2;
-          wm_split(make_float2(src[0], src[1]), x);
-          sp[0][e] = x[0]; sp[1][e] = x[1]; sp[2][e] = x[2];
-        }
-#pragma unroll
-        for (int z = 0; z < WM_IN; ++z) {
-          uint32_t b[4];
-          wm_ld4<false>(b, s.e.parts(z), 0, 16 * ks, WP, false);
-#pragma unroll
-          for (int m = 2; m >= 0; --m) {
-            wm_mma(y[0], sp[m], b[0], b[1]);
-            wm_mma(y[1], sp[m], b[2], b[3]);
-          }
-        }
-      }
-#pragma unroll
-      for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) s.inter[8 * n + n0 + (e & 1)][r0 + (e >> 1) * 8] = y[n][e];
-      const float t0 = s.tot[r0], t1 = s.tot[r0 + 8];
-#pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        S[n][0] *= t0; S[n][1] *= t0; S[n][2] *= t1; S[n][3] *= t1;
-      }
-      uint32_t bt[3][4];                 // (b Suf)^T: 16 rows i x 16 steps
-#pragma unroll
-      for (int k = 0; k < 3; ++k) wm_ld4<true>(bt[k], &s.bp[k][0][0], 0, warp * 16, WP, false);
-#pragma unroll
-      for (int n = 0; n < 8; n += 2)
-#pragma unroll
-        for (int z = 0; z < WM_IN; ++z) {
-          uint32_t b[4];
-          wm_ld4<true>(b, s.c.parts(z), 0, 8 * n, WP, true);
-#pragma unroll
-          for (int k = 2; k >= 0; --k) {
-            wm_mma(S[n], bt[k], b[0], b[1]);
-            wm_mma(S[n + 1], bt[k], b[2], b[3]);
-          }
-        }
-    }
-    __syncthreads();
-    // ---- results
-    if (!REV) {
-#pragma unroll
-      for (int x = 0; x < WM / 2; ++x) {
-        const int t = half * (WM / 2) + x;
-        if (t >= steps) continue;
-        const float row = s.pre[t][me] * s.inter[t][me] + (s.part[0][t][me] + s.part[1][t][me]);
-        const float gr = row + u_me * s.b.at(t, me) * s.st[t];
-        const long long o = oo + (long long)(t_lo + q * WM + t) * p.ost;
-        p.gr32[o] = gr;
-        p.o_gr[o] = float_to_h16(gr);
-      }
-    } else if (half == 0) {
-#pragma unroll
-      for (int t = 0; t < WM; ++t) {
-        if (t >= steps) continue;
-        const float row = s.pre[t][me] * s.inter[t][me] + (s.part[0][t][me] + s.part[1][t][me]);
-        const float r_ = s.b.at(t, me), k_ = h16_to_float(reinterpret_cast<const h16&>(s.k[t][me])), st = s.st[t];
-        const float gk = row + u_me * r_ * st;
-        const long long o = oo + (long long)(t_hi - 1 - q * WM - t) * p.ost;
-        p.o_gk[o] = float_to_h16(gk);
-        p.o_gw[o] = float_to_h16((Q - k_ * row) * s.ew[t][me]);
-        Q += r_ * gr[REV ? t : 0] - k_ * gk;
-        gu += r_ * k_ * st;
-      }
     }
     __syncthreads();
   }
