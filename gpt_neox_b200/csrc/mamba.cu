@@ -414,16 +414,24 @@ __device__ __forceinline__ void load_coef(const float* p, const RowOf8& r, float
 }
 
 // B or C of a block: 32 steps x 16 states, one column of 4 steps per thread.
-__device__ __forceinline__ void load_bc(const h16* p, long long st, int t0, int t_end, float (&v)[4]) {
+// They stay 16-bit in shared memory, so a step reads 4 states of each in 8 bytes and not 16: the pipe of shared memory and
+// exchanges is the bound of the scans (70 - 80 % busy), issue slots are half free for the widening.  4 x 2048 x 1536, fp16,
+// us: final forward pass 131 -> 119, its light pass 72.5 -> 70.1, backward light pass 95.9 -> 86.7, backward 413 -> 406.
+__device__ __forceinline__ void load_bc(const h16* p, long long st, int t0, int t_end, uint16_t (&v)[4]) {
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int t = (threadIdx.x >> 4) + 8 * k;
-    v[k] = t0 + t < t_end ? ldbf(p + (t0 + t) * st + (threadIdx.x & 15)) : 0.f;
+    v[k] = t0 + t < t_end ? reinterpret_cast<const uint16_t*>(p)[(t0 + t) * st + (threadIdx.x & 15)] : 0;
   }
 }
-__device__ __forceinline__ void put_bc(float (*s)[16], const float (&v)[4]) {
+__device__ __forceinline__ void put_bc(uint16_t (*s)[16], const uint16_t (&v)[4]) {
 #pragma unroll
   for (int k = 0; k < 4; ++k) s[(threadIdx.x >> 4) + 8 * k][threadIdx.x & 15] = v[k];
+}
+__device__ __forceinline__ float4 bc4(const uint16_t* p) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  const float2 a = unpack_h16x2(u.x), b = unpack_h16x2(u.y);
+  return make_float4(a.x, a.y, b.x, b.y);
 }
 
 __device__ __forceinline__ void exp4(float2 a01, float2 a23, float dl, float2 (&a)[2]) {
@@ -439,7 +447,7 @@ template <bool FINAL, bool VEC>
 __global__ void __launch_bounds__(SC_THREADS, SC_FWD_CTAS)
 scan_fwd_kernel(const ScanParams p) {
   __shared__ __align__(16) float2 dd[SC_T][SC_CH];        // (delta, delta * x)
-  __shared__ __align__(16) float Bs[SC_T][16], Cs[FINAL ? SC_T : 1][16];
+  __shared__ __align__(16) uint16_t Bs[SC_T][16], Cs[FINAL ? SC_T : 1][16];
   __shared__ __align__(16) float ys[FINAL ? SC_T : 1][SC_LD];
   const int ch = threadIdx.x >> 2, q = threadIdx.x & 3;
   const int d0 = blockIdx.x * SC_CH, d = d0 + ch;
@@ -468,7 +476,7 @@ scan_fwd_kernel(const ScanParams p) {
   load_coef(p.dt_bias, row, bias8);
   float sdt = 0.f;
   uint4 xu, du, zu = make_uint4(0u, 0u, 0u, 0u);
-  float bv[4], cv[4];
+  uint16_t bv[4], cv[4];
   auto fetch = [&](int t0) {
     const int n = t0 + row.t < t_end ? row.n : 0;
     xu = load8<VEC>(xp + (t0 + row.t) * p.xst, n);
@@ -504,14 +512,14 @@ scan_fwd_kernel(const ScanParams p) {
       for (int u = 0; u < 4; ++u) {
         const int t = g + u;
         const float2 dv2 = dd[t][ch];
-        const float4 B4 = *reinterpret_cast<const float4*>(&Bs[t][q * 4]);
+        const float4 B4 = bc4(&Bs[t][q * 4]);
         const float2 dx2 = make_float2(dv2.y, dv2.y);
         float2 a[2];
         exp4(A01, A23, dv2.x, a);
         h[0] = ffma2(a[0], h[0], fmul2(dx2, make_float2(B4.x, B4.y)));
         h[1] = ffma2(a[1], h[1], fmul2(dx2, make_float2(B4.z, B4.w)));
         if (FINAL) {
-          const float4 C4 = *reinterpret_cast<const float4*>(&Cs[t][q * 4]);
+          const float4 C4 = bc4(&Cs[t][q * 4]);
           const float2 y2 = ffma2(h[1], make_float2(C4.z, C4.w), fmul2(h[0], make_float2(C4.x, C4.y)));
           yp[u] = y2.x + y2.y;
         } else {
@@ -547,7 +555,7 @@ template <bool VEC>
 __global__ void __launch_bounds__(SC_THREADS)
 scan_bwd_local_kernel(const ScanParams p) {
   __shared__ __align__(16) float2 dd[SC_T][SC_CH];        // (delta, gradient of the ungated output)
-  __shared__ __align__(16) float Cs[SC_T][16];
+  __shared__ __align__(16) uint16_t Cs[SC_T][16];
   const int ch = threadIdx.x >> 2, q = threadIdx.x & 3;
   const int d0 = blockIdx.x * SC_CH, d = d0 + ch;
   const int c = blockIdx.y + 1, b = blockIdx.z;
@@ -566,7 +574,8 @@ scan_bwd_local_kernel(const ScanParams p) {
     const int n = in ? row.n : 0;
     const uint4 du = load8<VEC>(p.dt + b * p.dsb + tt * p.dst + row.d, n);
     const uint4 gu = load8<VEC>(p.dout + b * p.gsb + tt * p.gst + row.d, n);
-    float dv[8], gv[8], zv[8], cv[4];
+    float dv[8], gv[8], zv[8];
+    uint16_t cv[4];
     unpack8f(du, dv);
     unpack8f(gu, gv);
     if (p.z != nullptr) unpack8f(load8<VEC>(p.z + b * p.zsb + tt * p.zst + row.d, n), zv);
@@ -581,7 +590,7 @@ scan_bwd_local_kernel(const ScanParams p) {
 #pragma unroll
     for (int t = SC_T - 1; t >= 0; --t) {
       const float2 v = dd[t][ch];
-      const float4 C4 = *reinterpret_cast<const float4*>(&Cs[t][q * 4]);
+      const float4 C4 = bc4(&Cs[t][q * 4]);
       const float2 g2 = make_float2(v.y, v.y);
       float2 a[2];
       exp4(A01, A23, v.x, a);
@@ -599,7 +608,7 @@ scan_bwd_local_kernel(const ScanParams p) {
 
 struct ScanBwdSmem {
   float4 dd[SC_T][SC_CH];                     // delta, delta * x, gradient of the ungated output, sigmoid(dt)
-  float Bs[SC_T][16], Cs[SC_T][16];
+  uint16_t Bs[SC_T][16], Cs[SC_T][16];
   float dzf[SC_T][SC_LD];                     // d out / d z without the scan value
   float s_gb[SC_T][SC_LD], s_da[SC_T][SC_LD], s_hc[SC_T][SC_LD];   // sums over the 16 states
   float4 ck[SC_T / SC_REG][SC_THREADS];       // states at the starts of the block's quarters
@@ -638,7 +647,7 @@ scan_bwd_kernel(const ScanParams p) {
   const int idx = (b2 ? 4 : 0) + (b3 ? 2 : 0) + (b4 ? 1 : 0);
   const int col = idx < 4 ? q * 4 + idx : 16 + q * 4 + (idx - 4);
   uint4 xu, du, gu, zu = make_uint4(0u, 0u, 0u, 0u);
-  float bv[4], cv[4];
+  uint16_t bv[4], cv[4];
   float4 hc;                                  // state at the start of the block
   auto fetch = [&](int t0) {
     const int tt = t0 + row.t, n = tt < t_end ? row.n : 0;
@@ -693,7 +702,7 @@ scan_bwd_kernel(const ScanParams p) {
         for (int k = 0; k < SC_REG; ++k) {
           const int t = (quarter - 1) * SC_REG + k;
           const float4 v = s.dd[t][ch];
-          const float4 B4 = *reinterpret_cast<const float4*>(&s.Bs[t][q * 4]);
+          const float4 B4 = bc4(&s.Bs[t][q * 4]);
           const float2 dx2 = make_float2(v.y, v.y);
           float2 a[2];
           exp4(A01, A23, v.x, a);
@@ -714,7 +723,7 @@ scan_bwd_kernel(const ScanParams p) {
 #pragma unroll
       for (int t = 0; t < SC_REG; ++t) {
         const float4 v = s.dd[tb + t][ch];
-        const float4 B4 = *reinterpret_cast<const float4*>(&s.Bs[tb + t][q * 4]);
+        const float4 B4 = bc4(&s.Bs[tb + t][q * 4]);
         const float2 dx2 = make_float2(v.y, v.y);
         exp4(A01, A23, v.x, as[t]);
         hs[t + 1][0] = ffma2(as[t][0], hs[t][0], fmul2(dx2, make_float2(B4.x, B4.y)));
@@ -727,8 +736,8 @@ scan_bwd_kernel(const ScanParams p) {
         for (int u = 3; u >= 0; --u) {
           const int t = g + u;
           const float4 v = s.dd[tb + t][ch];
-          const float4 B4 = *reinterpret_cast<const float4*>(&s.Bs[tb + t][q * 4]);
-          const float4 C4 = *reinterpret_cast<const float4*>(&s.Cs[tb + t][q * 4]);
+          const float4 B4 = bc4(&s.Bs[tb + t][q * 4]);
+          const float4 C4 = bc4(&s.Cs[tb + t][q * 4]);
           const float2 dl2 = make_float2(v.x, v.x), dx2 = make_float2(v.y, v.y), dy2 = make_float2(v.z, v.z);
           const float2 g0 = ffma2(make_float2(C4.x, C4.y), dy2, r[0]), g1 = ffma2(make_float2(C4.z, C4.w), dy2, r[1]);
           r[0] = fmul2(as[t][0], g0);
