@@ -21,7 +21,9 @@
 //              dL/d(ew_t) = Q_t - k_t (gk_t - r_t u s_t),  s_t = <gy_t, v_t>,  ew = -exp(w)
 // Step by step the shared-memory loads and exchanges of the steps are the bound (32 x 512 tokens, 12 heads of 64, forward +
 // backward 788 us).  With the products of a block in their place 581 us, and 570 with a block's vectors beside the former
-// block's products (125 us for each sweep, 175 for gk with the decay gradient).
+// block's products (125 us for each sweep, 175 for gk with the decay gradient).  No pipe is the bound then but latency, at 2.6
+// warps per scheduler: issue slots 46 / 43 / 38 % busy (column sums, row sums, gk with the decay gradient), tensor pipe
+// 25 / 16 / 11 %.
 //
 // The sequence is cut into chunks only when batch x heads leaves the chip idle (wkv_chunk_count): the recurrence is
 // linear, so a chunk's end state is  P (.) S_start + S_local  with P[i] = prod_t d_t[i]; local passes start every chunk
