@@ -415,7 +415,8 @@ __device__ __forceinline__ void load_coef(const float* p, const RowOf8& r, float
 
 // B or C of a block: 32 steps x 16 states, one column of 4 steps per thread.
 // They stay 16-bit in shared memory, so a step reads 4 states of each in 8 bytes and not 16: the pipe of shared memory and
-// exchanges is the bound of the scans (70 - 80 % busy), issue slots are half free for the widening.  4 x 2048 x 1536, fp16,
+// exchanges bounded the scans (70 - 80 % busy with floats here; its wavefronts are at 49 - 73 % of their rate now, issue
+// slots at 48 - 63 %).  4 x 2048 x 1536, fp16,
 // us: final forward pass 131 -> 119, its light pass 72.5 -> 70.1, backward light pass 95.9 -> 86.7, backward 413 -> 406.
 __device__ __forceinline__ void load_bc(const h16* p, long long st, int t0, int t_end, uint16_t (&v)[4]) {
 #pragma unroll
