@@ -413,10 +413,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             const uint4 u = *reinterpret_cast<const uint4*>(aux_box + epi_chunk(lane, k));
             x[4 * k] = u.x; x[4 * k + 1] = u.y; x[4 * k + 2] = u.z; x[4 * k + 3] = u.w;
           }
-          // Every lane has its values before the next piece comes in: this vote needs one word of each of their loads (never
-          // true, since M is positive).  A barrier alone lets the copy overtake loads that are still queued: 1 % of a
-          // gradient was wrong.
-          if (__any_sync(0xffffffffu, (x[3] ^ x[7] ^ x[11] ^ x[15]) == 0u && p.M < 0)) aborted = true;
+          // The next piece comes in over this one: every lane's fence orders its loads before the copy, which belongs to another
+          // proxy, and the barrier hands that order to the lane that issues it.  (The barrier alone orders ordinary
+          // accesses; the copy then overtook loads that were still queued, and 1 % of a gradient was wrong.)
+          fence_proxy_async_smem();
+          __syncwarp();
           // the next piece: of this tile, or the first of the next
           const bool here = c + 1 < c_end && col0 + 32 < p.N;
           fetched = here || (tile_nx < num_tiles && tn_nx * BN + c_begin * 32 < p.N);

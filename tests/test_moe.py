@@ -188,3 +188,33 @@ def test_grouped_rows_epilogues(T, n, K, kind, dtype):
     assert (deriv[rows] - wd).abs().sub(eps * wd.abs()).max() <= slack
     ref = z.detach() * deriv[rows].double()
     assert (prod[rows] - ref).abs().sub(eps * ref.abs()).max() <= 2 ** -18
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["mul", "erf", "tanh"])
+@pytest.mark.parametrize("T,n,K", [(9000, 3072, 64), (20000, 520, 192)])
+def test_grouped_rows_read_their_side_operand_before_the_next_piece(T, n, K, kind):
+    """The side operand's pieces follow each other through one box of shared memory: short reductions, where the epilogue
+    waits for nothing else, many pieces per CTA, run over and over.  Every run has the bits of the first, and those are the
+    fp32 product rounded once (sums and erf are 2 ** -20 off, tanh.approx 2 ** -11, the derivative up to 16 times that)."""
+    from gpt_neox_b200.ops import moe as M
+    torch.manual_seed(5)
+    E, dtype = 4, torch.bfloat16
+    plan = M.Plan(torch.randint(0, E, (T, 2), device="cuda"), E)
+    rows = (plan.src_copy >= 0).nonzero().flatten()
+    xp = M.gather_rows(torch.randn(T, K, device="cuda").to(dtype), plan)
+    w = (torch.randn(E * n, K, device="cuda") * K ** -0.5).to(dtype)
+    side = torch.randn(plan.max_rows, n, device="cuda").to(dtype)
+    run = lambda: M.grouped_gemm_rows(xp, w, plan, n, trans_b=False, dgelu_aux=side, dgelu=kind)
+    first = run()
+    for _ in range(20):
+        assert torch.equal(run()[rows], first[rows])
+    expert = plan.tile_expert.long()[rows // 128]
+    for e in range(E):
+        r = rows[expert == e]
+        x = side[r].double().requires_grad_()
+        d = x.detach() if kind == "mul" else torch.autograd.grad(
+            torch.nn.functional.gelu(x, approximate="tanh" if kind == "tanh" else "none").sum(), x)[0]
+        z = xp[r].double() @ w.view(E, n, K)[e].double().t()
+        err = (first[r] - z * d).abs() - 2 ** -8 * (z * d).abs()
+        assert err.max() <= (2 ** -7 if kind == "tanh" else 2 ** -16) * z.abs().max()
