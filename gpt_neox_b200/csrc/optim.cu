@@ -188,9 +188,13 @@ __global__ void __launch_bounds__(256) adam8_kernel(float* __restrict__ p, uint8
   }
 }
 
-// acc[0] += sum(x^2) ; acc[1] = max(acc[1], any non-finite ? 1 : 0)   (acc: float[2])
+// acc[0] += sum(x^2) ; acc[1] = max(acc[1], any non-finite ? 1 : 0)   (acc: float[2]), the same bits on every run: block b
+// writes its sum and its flag to part[b], and a second launch adds the sums in the order of the blocks, in 64 bits.  (The
+// clip coefficient multiplies every gradient, so a last bit of the norm reaches the whole state: with block sums that met
+// in atomic adds, in the order in which blocks ended, two runs differed by a step of single 16-bit weights.)
+constexpr int SUMSQ_BLOCKS_PER_SM = 8, FOLD_THREADS = 256;
 template <typename G>
-__global__ void sumsq_kernel(const G* __restrict__ x, long long n, float* __restrict__ acc) {
+__global__ void sumsq_kernel(const G* __restrict__ x, long long n, float2* __restrict__ part) {
   __shared__ float sh[64];
   float s = 0.f;
   float bad = 0.f;
@@ -210,9 +214,28 @@ __global__ void sumsq_kernel(const G* __restrict__ x, long long n, float* __rest
   }
   if (!isfinite(s)) bad = 1.f;
   const float2 r = block_sum2(s, bad, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = make_float2(r.x, r.y > 0.f || !isfinite(r.x) ? 1.f : 0.f);
+}
+
+__global__ void __launch_bounds__(FOLD_THREADS) sumsq_fold_kernel(const float2* part, int parts, float* acc) {
+  __shared__ double sh[FOLD_THREADS / 32];
+  grid_dependency_wait();
+  double s = 0.;
+  bool bad = false;
+  for (int i = threadIdx.x; i < parts; i += FOLD_THREADS) {
+    const float2 v = part[i];
+    s += v.x;
+    bad = bad || v.y != 0.f;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  bad = __syncthreads_or(bad);
   if (threadIdx.x == 0) {
-    atomicAdd(acc, r.x);
-    if (r.y > 0.f || !isfinite(r.x)) atomicExch(acc + 1, 1.f);
+    s = acc[0];
+    for (int w = 0; w < FOLD_THREADS / 32; ++w) s += sh[w];
+    acc[0] = static_cast<float>(s);
+    if (bad) acc[1] = 1.f;
   }
 }
 
@@ -282,17 +305,19 @@ NX_API int NX_SYM(nx_adamw8bit_step)(void* p, void* m8, void* v8, void* scale_m,
   NX_LAUNCH_CHECK();
   return NX_OK;
 }
-NX_API int NX_SYM(nx_sumsq)(const void* x, long long n, void* acc, int dtype, void* stream_) {
+// part: float scratch [max_parts, 2] of this call.
+NX_API int NX_SYM(nx_sumsq)(const void* x, long long n, void* acc, void* part, int max_parts, int dtype, void* stream_) {
   using namespace nx;
   if (n == 0) return NX_OK;
-  const long long nvec = (n + 3) / 4;
-  long long g_ = (nvec + 255) / 256;
-  const long long cap = static_cast<long long>(sm_count()) * 8;
-  const int grid = static_cast<int>(g_ < cap ? g_ : cap);
+  NX_REQUIRE(part != nullptr && max_parts > 0, "sumsq: scratch for the blocks' sums is missing");
+  const long long blocks = ((n + 3) / 4 + 255) / 256;
+  const int grid = static_cast<int>(min(blocks, static_cast<long long>(min(sm_count() * SUMSQ_BLOCKS_PER_SM, max_parts))));
   auto s = (cudaStream_t)stream_;
-  if (dtype == 0) sumsq_kernel<h16><<<grid, 256, 0, s>>>((const h16*)x, n, (float*)acc);
-  else sumsq_kernel<float><<<grid, 256, 0, s>>>((const float*)x, n, (float*)acc);
+  if (dtype == 0) sumsq_kernel<h16><<<grid, 256, 0, s>>>((const h16*)x, n, (float2*)part);
+  else sumsq_kernel<float><<<grid, 256, 0, s>>>((const float*)x, n, (float2*)part);
   NX_LAUNCH_CHECK();
+  NX_CUDA_CHECK(launch_dependent(sumsq_fold_kernel, dim3(1), dim3(FOLD_THREADS), 0, s, 0, (const float2*)part, grid,
+                                 (float*)acc));
   return NX_OK;
 }
 NX_API int NX_SYM(nx_clip_coef)(const void* acc, float max_norm, float inv_scale, void* out, void* skip,

@@ -98,7 +98,7 @@ def _declare(lib):
     sig("nx_ce_bwd", [P, P, P, P, P, L, I, L, L, I, I, P])
     sig("nx_adamw_step", [P, P, P, P, P, L, F, F, F, F, F, F, F, I, P, P, I, P])
     sig("nx_adamw8bit_step", [P, P, P, P, P, P, P, L, F, F, F, F, F, F, F, I, P, P, I, P])
-    sig("nx_sumsq", [P, L, P, I, P])
+    sig("nx_sumsq", [P, L, P, P, I, I, P])
     sig("nx_clip_coef", [P, F, F, P, P, P])
     sig("nx_conv1d_silu_fwd", [P, L, L, P, P, P, L, L, I, I, I, I, P])
     sig("nx_conv1d_silu_bwd", [P, L, L, P, P, P, L, L, P, L, L, P, P, I, I, I, I, P])

@@ -9,15 +9,19 @@ from . import _lib
 from .gemm import LAUNCHES
 
 
+_SUMSQ_PARTS = 2048      # block sums of one call: more than the kernel has blocks
+
+
 def sumsq_(x: torch.Tensor, acc: torch.Tensor):
-    """acc[0] += sum(x^2); acc[1] = 1 if a non-finite value was seen. acc: float32[2]."""
+    """acc[0] += sum(x^2); acc[1] = 1 if a non-finite value was seen. acc: float32[2].  The same bits on every run."""
     if x.numel() == 0:
         return
     if x.is_cuda:
         assert x.is_contiguous() and x.dtype in (torch.bfloat16, torch.float16, torch.float32)
-        LAUNCHES["n"] += 1
-        _lib.check(_lib.lib(x).nx_sumsq(_lib.ptr(x), x.numel(), _lib.ptr(acc), 1 if x.dtype == torch.float32 else 0,
-                                       _lib.stream()), "nx_sumsq")
+        LAUNCHES["n"] += 2
+        part = torch.empty((_SUMSQ_PARTS, 2), device=x.device, dtype=torch.float32)
+        _lib.check(_lib.lib(x).nx_sumsq(_lib.ptr(x), x.numel(), _lib.ptr(acc), _lib.ptr(part), _SUMSQ_PARTS,
+                                       1 if x.dtype == torch.float32 else 0, _lib.stream()), "nx_sumsq")
     else:
         s = x.float().pow(2).sum()
         acc[0] += s

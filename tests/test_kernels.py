@@ -273,6 +273,57 @@ def test_adamw_sumsq_clip():
     assert torch.equal(before, p)
 
 
+@pytest.mark.parametrize("wide", [False, True], ids=["16bit", "fp32"])
+@pytest.mark.parametrize("n", [1, 3, 1024, 1025, 1_212_421, 30_000_003])
+def test_optimizer_step_repeats_bit_for_bit(n, wide):
+    """Gradient norm, clip coefficient and AdamW from the same state give the same bits on every run, on two streams at
+    once too, and the norm is that of 64 bits: a thread adds up to 100 squares in fp32, a block 256 threads in a tree."""
+    from gpt_neox_b200.ops.optim import adamw_step_, clip_coef_, sumsq_
+    torch.manual_seed(26)
+    g, p0 = torch.randn(n, device=DEV) * 1e-2, torch.randn(n, device=DEV) * 0.02
+    g = g if wide else g.to(DT)
+    m0, v0 = torch.randn(n, device=DEV) * 1e-4, torch.rand(n, device=DEV) * 1e-8
+
+    def step():
+        p, m, v, lp = p0.clone(), m0.clone(), v0.clone(), torch.empty(n, device=DEV, dtype=DT)
+        acc, out, skip = torch.full((2,), 0.0, device=DEV), torch.zeros(2, device=DEV), torch.ones(1, dtype=torch.int32, device=DEV)
+        sumsq_(g, acc)
+        one = acc.clone()
+        sumsq_(g, acc)                     # a second buffer adds to the first
+        clip_coef_(acc, 1e-3, 1.0, out, skip)
+        adamw_step_(p, m, v, g, lp, lr=1e-4, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1, step=100, grad_scale=out,
+                    skip=skip)
+        return one, acc, out, skip, p, m, v, lp
+
+    want = step()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    for _ in range(4 if n > 10_000_000 else 20):
+        with torch.cuda.stream(side):
+            other = step()
+        here = step()
+        torch.cuda.current_stream().wait_stream(side)
+        for a, b, c in zip(want, here, other):
+            assert torch.equal(a, b) and torch.equal(a, c)
+        side.wait_stream(torch.cuda.current_stream())
+    total = g.double().square().sum()
+    assert want[1][1] == 0 and want[3] == 0
+    assert abs(want[0][0].double() - total) <= 2 ** -20 * total
+    assert abs(want[1][0].double() - 2 * total) <= 2 ** -20 * 2 * total
+
+
+@pytest.mark.parametrize("bad", [math.nan, math.inf, -math.inf])
+@pytest.mark.parametrize("n,at", [(1, 0), (1025, 1024), (5_000_001, 3_333_333)])
+def test_gradient_norm_marks_what_is_not_finite(n, at, bad):
+    from gpt_neox_b200.ops.optim import sumsq_
+    g, acc = torch.ones(n, device=DEV, dtype=DT), torch.zeros(2, device=DEV)
+    sumsq_(g, acc)
+    assert acc.tolist() == [n, 0.0]        # (below 2^24 ones add up exactly)
+    g[at] = bad
+    sumsq_(g, acc)
+    assert acc[1] == 1 and not acc[0].isfinite()
+
+
 def test_adamw_8bit_state_kernel_matches_the_pytorch_statement():
     """csrc/optim.cu adam8_kernel against ops/optim.py's PyTorch statement of the same update and the same 8-bit
     block-wise codes: the master weights agree to fp32 rounding, the codes agree except where a value sits on a
