@@ -1,4 +1,5 @@
-// Flash attention backward on tcgen05 (causal / sliding window / ALiBi / GQA).
+// Flash attention backward on tcgen05 (causal / sliding window / ALiBi / GQA; dropout, block-sparse layouts and small calls:
+// attention_bwd_tile.cu).
 //
 // Three launches, no atomics, no fp32 scratch for dQ, deterministic:
 //   1. attn_delta_kernel    delta[b,h,q] = sum_d O * dO
@@ -28,37 +29,13 @@
 // 331 -> 232 us and 438 -> 322 us (before: a CTA per item, one issuing thread, all eight element-wise warps on the same 64
 // columns).  What was slower: two groups of four warps that write their results over their scores (260 / 333 us), dQ by 16
 // warps with 32 columns each (215 us), dQ with two K stages (258 us), one V stage (212 us).
-#include "common.h"
+#include "attention_bwd.h"
 #include "ptx.cuh"
 #include "reduce.cuh"
 
 namespace nx {
 
-constexpr int AB = 128;  // rows per resident tile and per key block of the dQ kernel
-constexpr int ABS = 64;  // query rows per block of the dK / dV kernel
 constexpr int DQ_THREADS = 32 * 12, DKV_THREADS = 32 * 20;
-constexpr float LOG2E = 1.4426950408889634f;
-
-struct AttnBwdParams {
-  const float* lse;    // [B,H,Sq_pad] base-2 log-sum-exp, +inf in the padding
-  const float* delta;  // [B,H,Sq_pad], 0 in the padding
-  const float* alibi;
-  h16 *dq, *dk, *dv;
-  long long dq_sb, dq_sh, dq_ss, dk_sb, dk_sh, dk_ss, dv_sb, dv_sh, dv_ss;
-  int B, H, Hk, Sq, Sk, D, Sq_pad;
-  float scale, scale_log2;
-  int causal, window;
-  int* err;
-  // dropout as in the forward (same seed and threshold): dP is masked and scaled before delta is subtracted,
-  // and the P^T that feeds dV is the dropped one
-  uint32_t drop_thr, seed_lo, seed_hi;
-  float drop_rp;
-  // block-sparse layout tables of the forward (null = dense): blk_rows[q * blk_nkt + kt] bit j = row q attends to
-  // key sub-block j of key tile kt; blk_any[qt * blk_nkt + kt] != 0 = tile (qt, kt) has any live block
-  const uint8_t* blk_rows;
-  const uint8_t* blk_any;
-  int blk_shift, blk_nkt;
-};
 
 // delta = rowsum(O * dO), 0 in the padding rows [Sq, Sq_pad).  A group of LPR lanes (D / 8 rounded up to a power of two)
 // takes a row with one 16-byte load per lane and tensor, and four rows at a time so that eight loads per lane are in
@@ -208,8 +185,6 @@ struct BwdOrder {
   }
 };
 
-// GEN: block-sparse layouts skip the 128 x 128 tiles without a live block, in every role alike.
-template <bool GEN>
 struct DqWork {
   const AttnBwdParams& p;
   BwdOrder order;
@@ -233,11 +208,7 @@ struct DqWork {
     it.j1 = max((kv_end + AB - 1) / AB, it.j0);
     return true;
   }
-  __device__ __forceinline__ bool live(const BwdItem& it, int j) const {
-    return !GEN || p.blk_any == nullptr || p.blk_any[static_cast<long long>(it.tile) * p.blk_nkt + j] != 0;
-  }
 };
-template <bool GEN>
 struct DkvWork {
   const AttnBwdParams& p;
   BwdOrder order;
@@ -263,10 +234,6 @@ struct DkvWork {
     it.j0 = 0;
     it.j1 = it.n_i * group;
     return true;
-  }
-  __device__ __forceinline__ bool live(const BwdItem& it, int j) const {
-    return !GEN || p.blk_any == nullptr ||
-           p.blk_any[static_cast<long long>((it.i0 + j % it.n_i) >> 1) * p.blk_nkt + it.tile] != 0;
   }
 };
 
@@ -328,20 +295,13 @@ __device__ __forceinline__ void bwd_store(h16* base, long long row_stride, const
   __syncwarp();
 }
 
-// The first live block from j on (j1: none).
-template <class Work>
-__device__ __forceinline__ int next_live(const Work& work, const BwdItem& it, int j) {
-  while (j < it.j1 && !work.live(it, j)) ++j;
-  return j;
-}
 // ------------------------------------------------------------------------------------------------
 // dQ kernel.  Resident: Q, dO (128 rows).  Streamed: K, V (128 rows).  An element-wise warp has 64 of a block's key columns, in
 // two chunks of 32; dS goes over the first half of the score columns the warp itself has read.
 // TMEM: S of block n at [128 (n & 1), ...), dP [256, 384), dQ [384, 384 + DP).
-// GEN (this kernel and the next): ALiBi and block-sparse layouts; without them a block that needs a mask differs from one
-// that does not by one select per element.
+// Without ALIBI (this kernel and the next) a block that needs a mask differs from one that does not by one select per element.
 // ------------------------------------------------------------------------------------------------
-template <int DP, bool DROP, bool GEN>
+template <int DP, bool ALIBI>
 __global__ void __launch_bounds__(DQ_THREADS, 1)
     attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -361,7 +321,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int off = p.Sk - p.Sq;
-  const DqWork<GEN> work(p);
+  const DqWork work(p);
   if (threadIdx.x == 0) bwd_init_barriers(bar0);
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
@@ -382,7 +342,6 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
         const int kv_head = it.head / (p.H / p.Hk);
         bool any = false;
         for (int j = it.j0; j < it.j1; ++j) {
-          if (!work.live(it, j)) continue;
           const int vs = n & 1;
           if (!mbar_wait(bar(STR_EMPTY, ks), kph ^ 1, p.err, 32)) { aborted = true; break; }
           mbar_expect_tx(bar(STR_FULL, ks), 2 * L::T64);
@@ -416,8 +375,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
     while (!aborted && work.next(round, it)) {
       bool any = false;
       for (int j = it.j0; j < it.j1; ++j) {
-        if (!work.live(it, j)) continue;
-        const bool last = next_live(work, it, j + 1) >= it.j1;
+        const bool last = j + 1 == it.j1;
         const int st = n & 1;
         const uint32_t ph = (n >> 1) & 1;
         // (S buffer n & 1 is free when dQ has taken dS of block n - 2: its stage is two back in the ring of three)
@@ -457,7 +415,6 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
     while (!aborted && work.next(round, it)) {
       bool any = false;
       for (int j = it.j0; j < it.j1; ++j) {
-        if (!work.live(it, j)) continue;
         if ((!any && !warp_wait(bar(ACC_EMPTY, 0), (t & 1) ^ 1, p.err, 33)) ||
             !warp_wait(bar(P_FULL, n & 1), (n >> 1) & 1, p.err, 41)) {
           aborted = true;
@@ -529,9 +486,9 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
         delta_nx = p.delta[stat_of(nx)];
       }
       const int q0 = it.tile * AB, qi = q0 + r, qpos = qi + off;
-      const float slope2 = GEN && p.alibi != nullptr ? p.alibi[it.head] * LOG2E : 0.f;
+      const float slope2 = ALIBI ? p.alibi[it.head] * LOG2E : 0.f;
       // scores of the 32 keys from k0 on -> probabilities, in place
-      auto probs = [&](uint32_t (&sv)[32], int k0, uint32_t bits) {
+      auto probs = [&](uint32_t (&sv)[32], int k0) {
         const bool need_mask = (k0 + 32 > p.Sk) || (p.causal && k0 + 31 > q0 + quad * 32 + off) ||
                                (p.window >= 0 && k0 < q0 + quad * 32 + 31 + off - p.window);
         // columns e (0..31) are alive for lo <= e <= hi
@@ -539,7 +496,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
         int hi = p.Sk - k0 - 1;
         if (p.causal) hi = min(hi, -rel0);
         const int lo = p.window >= 0 ? -rel0 - p.window : -(1 << 30);
-        if (!GEN) {
+        if (!ALIBI) {
           if (need_mask) {      // masked scores: -inf, probability 0
 #pragma unroll
             for (int e = 0; e < 32; ++e)
@@ -558,25 +515,13 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
           for (int e = 0; e < 32; ++e) {
             const float x = fmaf(__uint_as_float(sv[e]), p.scale_log2, fmaf(slope2, static_cast<float>(e), bias0));
             float pr = exp2f(x);
-            if (e < lo || e > hi || !((bits >> ((k0 % AB + e) >> p.blk_shift)) & 1u)) pr = 0.f;
+            if (e < lo || e > hi) pr = 0.f;
             sv[e] = __float_as_uint(pr);
           }
         }
       };
       // probabilities, dP -> dS (16 bit); the softmax scale is applied once, to dQ, when it is stored
-      auto grads = [&](const uint32_t (&pr)[32], uint32_t (&dv)[32], int k0, uint32_t (&pk)[16]) {
-        if (DROP) {
-          // dP of a dropped probability is zero, of a kept one it carries the 1 / (1 - p) factor
-#pragma unroll
-          for (int e = 0; e < 32; e += 2) {
-            const int kk = k0 + e;
-            const uint32_t patch = dropout_patch(p.seed_lo, p.seed_hi, static_cast<uint32_t>(it.batch * p.H + it.head),
-                                                 static_cast<uint32_t>(qi) >> 1, static_cast<uint32_t>(kk) >> 1);
-            dv[e] = dropout_keep(patch, qi, kk, p.drop_thr) ? __float_as_uint(__uint_as_float(dv[e]) * p.drop_rp) : 0u;
-            dv[e + 1] = dropout_keep(patch, qi, kk + 1, p.drop_thr)
-                            ? __float_as_uint(__uint_as_float(dv[e + 1]) * p.drop_rp) : 0u;
-          }
-        }
+      auto grads = [&](const uint32_t (&pr)[32], const uint32_t (&dv)[32], uint32_t (&pk)[16]) {
         const float2 nd2 = make_float2(-delta, -delta);
 #pragma unroll
         for (int e = 0; e < 32; e += 2) {
@@ -585,7 +530,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
         }
       };
       uint32_t sa[32], sb[32], dv[32], pk[16];
-      int j = next_live(work, it, it.j0);
+      int j = it.j0;
       const bool live = j < it.j1;
       if (live) {
         if (!wait(S_FULL, n & 1, (n >> 1) & 1, 38)) { aborted = true; break; }
@@ -594,18 +539,16 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
       }
       bool first = true;
       while (j < it.j1) {
-        const int jn = next_live(work, it, j + 1), k0 = j * AB + c0;
+        const int jn = j + 1, k0 = j * AB + c0;
         const uint32_t t_sn = t_s + (n & 1) * AB;
-        uint32_t bits = 0xffffffffu;
-        if (GEN && p.blk_rows != nullptr) bits = qi < p.Sq ? p.blk_rows[static_cast<long long>(qi) * p.blk_nkt + j] : 0u;
         tmem_ld_32x32b_x32(t_sn + 32, sb);      // in flight during the first chunk's exponentials
-        probs(sa, k0, bits);
+        probs(sa, k0);
         tmem_ld_wait_for(sb);
         if (!wait(DP_FULL, 0, n & 1, 44)) { aborted = true; break; }
         tmem_ld_32x32b_x32(t_dp, dv);           // ... the second chunk's
-        probs(sb, k0 + 32, bits);
+        probs(sb, k0 + 32);
         tmem_ld_wait_for(dv);
-        grads(sa, dv, k0, pk);
+        grads(sa, dv, pk);
         tmem_ld_32x32b_x32(t_dp + 32, dv);
         tmem_st_32x32b_x16(t_sn, pk);
         tmem_ld_wait_for(dv);
@@ -616,7 +559,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
           if (!wait(S_FULL, (n + 1) & 1, ((n + 1) >> 1) & 1, 38)) { aborted = true; break; }
           tmem_ld_32x32b_x32(t_s + ((n + 1) & 1) * AB, sa);
         }
-        grads(sb, dv, k0 + 32, pk);
+        grads(sb, dv, pk);
         tmem_st_32x32b_x16(t_sn + 16, pk);
         tmem_st_wait();
         tc_fence_before_sync();
@@ -662,7 +605,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
 // TMEM: S^T of block n at [64 (n & 1), ...), dP^T [128, 192), P^T [192, 224), dS^T [224, 256), dK [256, 256 + DP), dV [384, 384 +
 // DP).
 // ------------------------------------------------------------------------------------------------
-template <int DP, bool DROP, bool GEN>
+template <int DP, bool ALIBI>
 __global__ void __launch_bounds__(DKV_THREADS, 1)
     attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                         const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -681,7 +624,7 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int off = p.Sk - p.Sq;
-  const DkvWork<GEN> work(p);
+  const DkvWork work(p);
   if (threadIdx.x == 0) bwd_init_barriers(bar0);
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
@@ -706,7 +649,6 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
             ib = it.i0;
             ++g;
           }
-          if (!work.live(it, j)) continue;
           const int q0 = ib * ABS, head = it.head * work.group + g;
           if (!mbar_wait(bar(STR_EMPTY, st), ph ^ 1, p.err, 52)) { aborted = true; break; }
           mbar_expect_tx(bar(STR_FULL, st), 2 * L::T64 + 2 * ABS * 4);
@@ -742,8 +684,7 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
     while (!aborted && work.next(round, it)) {
       bool any = false;
       for (int j = 0; j < it.j1; ++j) {
-        if (!work.live(it, j)) continue;
-        const bool last = next_live(work, it, j + 1) >= it.j1;
+        const bool last = j + 1 == it.j1;
         if ((!any && !warp_wait(bar(RES_FULL, 0), t & 1, p.err, 53)) || !warp_wait(bar(STR_FULL, st), ph, p.err, 54) ||
             !warp_wait(bar(S_EMPTY, n & 1), ((n >> 1) & 1) ^ 1, p.err, 60)) {
           aborted = true;
@@ -779,7 +720,6 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
     while (!aborted && work.next(round, it)) {
       bool any = false;
       for (int j = 0; j < it.j1; ++j) {
-        if (!work.live(it, j)) continue;
         const int h = n & 1;
         if ((!any && !warp_wait(bar(ACC_EMPTY, 0), (t & 1) ^ 1, p.err, 55)) ||
             !warp_wait(bar(P_FULL, h), (n >> 1) & 1, p.err, 56)) {
@@ -845,7 +785,6 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
     while (!aborted && work.next(round, it)) {
       const int kcol = it.tile * AB + r;
       const bool key_ok = kcol < p.Sk;
-      const uint32_t kbit = 1u << (r >> p.blk_shift);      // this key row's sub-block within the key tile
       bool first = true;
       int g = 0, ib = it.i0 - 1;
       for (int j = 0; j < it.j1; ++j) {
@@ -853,7 +792,6 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
           ib = it.i0;
           ++g;
         }
-        if (!work.live(it, j)) continue;
         const int i = n++, cur = st;
         const uint32_t cur_ph = ph;
         if (++st == BWD_STAGES) {
@@ -868,13 +806,13 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
           continue;
         }
         const int q0 = ib * ABS + c0, head = it.head * work.group + g;      // this warp's first query row
-        const float slope2 = GEN && p.alibi != nullptr ? p.alibi[head] * LOG2E : 0.f;
+        const float slope2 = ALIBI ? p.alibi[head] * LOG2E : 0.f;
         // this warp's query columns e (0..31) are alive for lo <= e <= hi
         const int rel0 = kcol - q0 - off;  // key position minus position of query column 0
         const int lo = p.causal ? rel0 : -(1 << 30);
         int hi = p.window >= 0 ? rel0 + p.window : (1 << 30);
         if (!key_ok) hi = -(1 << 30);
-        const bool need_mask = __any_sync(0xffffffffu, lo > 0 || hi < 31) || (GEN && p.blk_rows != nullptr);
+        const bool need_mask = __any_sync(0xffffffffu, lo > 0 || hi < 31);
         const uint32_t par = (i >> 1) & 1;
         // (lse / delta of a query block were bulk-copied next to the Q / dO tiles)
         const float4* v_lse = reinterpret_cast<const float4*>(sgen + L::VEC_OFF + cur * (2 * ABS * 4)) + c0 / 4;
@@ -886,14 +824,14 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(S_EMPTY, h));
-        // probabilities, in place; dV takes them rounded (and dropped)
-        if (!GEN && need_mask) {      // masked scores: -inf, probability 0
+        // probabilities, in place; dV takes them rounded
+        if (!ALIBI && need_mask) {      // masked scores: -inf, probability 0
 #pragma unroll
           for (int e = 0; e < 32; ++e)
             if (e < lo || e > hi) sv[e] = __float_as_uint(p.scale_log2 < 0.f ? INFINITY : -INFINITY);
         }
         auto probs = [&](int first_e) {
-          if (!GEN) {
+          if (!ALIBI) {
             const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
 #pragma unroll
             for (int z = 0; z < 16; z += 4) {
@@ -917,22 +855,13 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
               float kept[4];
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
-                const int idx = e0 + e, qq = q0 + idx;
-                float x = fmaf(__uint_as_float(sv[idx]), p.scale_log2, -lq[e]);
-                if (p.alibi != nullptr) x += fmaf(-slope2, static_cast<float>(idx), bias0);
+                const int idx = e0 + e;
+                const float x = fmaf(__uint_as_float(sv[idx]), p.scale_log2, -lq[e]) +
+                                fmaf(-slope2, static_cast<float>(idx), bias0);
                 float pr = exp2f(x);
-                if (need_mask) {
-                  if (idx < lo || idx > hi) pr = 0.f;
-                  if (p.blk_rows != nullptr &&       // the layout byte of query row qq (the same for the whole warp)
-                      !(p.blk_rows[static_cast<long long>(min(qq, p.Sq - 1)) * p.blk_nkt + it.tile] & kbit)) pr = 0.f;
-                }
+                if (need_mask && (idx < lo || idx > hi)) pr = 0.f;
                 sv[idx] = __float_as_uint(pr);
                 kept[e] = pr;
-                if (DROP) {
-                  const uint32_t patch = dropout_patch(p.seed_lo, p.seed_hi, static_cast<uint32_t>(it.batch * p.H + head),
-                                                       static_cast<uint32_t>(qq) >> 1, static_cast<uint32_t>(kcol) >> 1);
-                  kept[e] *= dropout_keep(patch, qq, kcol, p.drop_thr) ? p.drop_rp : 0.f;
-                }
               }
               pk[e0 >> 1] = pack_h16x2(kept[0], kept[1]);
               pk[(e0 >> 1) + 1] = pack_h16x2(kept[2], kept[3]);
@@ -947,15 +876,6 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(DP_EMPTY, 0));
-        if (DROP) {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            const int qq = q0 + e;
-            const uint32_t patch = dropout_patch(p.seed_lo, p.seed_hi, static_cast<uint32_t>(it.batch * p.H + head),
-                                                 static_cast<uint32_t>(qq) >> 1, static_cast<uint32_t>(kcol) >> 1);
-            dv[e] = __float_as_uint(__uint_as_float(dv[e]) * (dropout_keep(patch, qq, kcol, p.drop_thr) ? p.drop_rp : 0.f));
-          }
-        }
         uint32_t pd[16];
         const float2 m1 = make_float2(-1.f, -1.f);
 #pragma unroll
@@ -1010,38 +930,50 @@ static bool bwd_map(CUtensorMap* m, const void* base, int B, int Hh, int S, int 
   return make_tma_4d(m, base, dims, strides, box, 2, true);
 }
 
-struct BwdMaps {
-  CUtensorMap q, k, v, d_o;
+// Which kernels a call takes: persistent ones or one CTA per tile (attention_bwd_tile.cu).  Persistent CTAs overlap one item
+// with the next, so they need more items than SMs; a single item costs them 1 - 4 us more (more roles, barriers and
+// threads to set up).  Measured over 64 .. 2048 tokens x 4 .. 256 heads, time per tile / persistent:
+//   dropout     0.5 (registers spill);  block-sparse layouts 0.7 - 1 (a CTA's share is fixed, and tiles are of any length)
+//   dQ, ALiBi   0.96 - 2.7: always persistent
+//   dQ, 128     more items than SMs 1.13 - 1.66; fewer, 256 keys and more 0.98 - 1.15, fewer keys 0.86 - 1.17
+//   dQ, 64      causal, more items than SMs and more than one key block 1.02 - 1.63, one block 0.92 - 0.97; not causal 0.88 - 1.02
+//               up to 512 items, 1.08 - 1.18 from 768 on (blocks are short, the SMs' last round counts); fewer items 0.77 - 1.01
+//   dK / dV     more items than SMs: 128 1.0 - 1.38; 64, causal from 384 queries on (ALiBi 200) 0.98 - 1.40, below 0.86 - 1.0,
+//               not causal 0.8 - 1.0; fewer items than SMs 0.66 - 1.05
+struct BwdRoute {
+  long long dq_items, dkv_items;
+  bool dq, dkv;      // persistent
 };
+static BwdRoute attn_bwd_route(const AttnBwdParams& p) {
+  BwdRoute r;
+  r.dq_items = static_cast<long long>((p.Sq + AB - 1) / AB) * p.H * p.B;
+  r.dkv_items = static_cast<long long>((p.Sk + AB - 1) / AB) * p.Hk * p.B;
+  r.dq = r.dkv = false;
+  if (p.drop_thr > 0u || p.blk_rows != nullptr || p.scale == 0.f) return r;
+  const bool alibi = p.alibi != nullptr;
+  const int sms = sm_count();
+  if (alibi) r.dq = true;
+  else if (p.D > 64) r.dq = r.dq_items > sms || p.Sk >= 256;
+  else r.dq = p.causal ? r.dq_items > sms && p.Sk > AB : r.dq_items > 4 * sms;
+  r.dkv = r.dkv_items > sms && (p.D > 64 || (p.causal && p.Sq >= (alibi ? 200 : 384)));
+  return r;
+}
 
-template <int DP, bool DROP, bool GEN>
-static int launch_bwd_as(const BwdMaps& m, const AttnBwdParams& p, cudaStream_t s) {
-  auto dq = attn_bwd_dq_kernel<DP, DROP, GEN>;
-  auto dkv = attn_bwd_dkv_kernel<DP, DROP, GEN>;
-  static bool cfg = false;
-  if (!cfg) {
-    NX_CUDA_CHECK(cudaFuncSetAttribute(dq, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<DP>::DYN));
-    NX_CUDA_CHECK(cudaFuncSetAttribute(dkv, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem<DP>::DYN));
-    cfg = true;
-  }
-  const long long nq = static_cast<long long>((p.Sq + AB - 1) / AB) * p.H * p.B;
-  const long long nk = static_cast<long long>((p.Sk + AB - 1) / AB) * p.Hk * p.B;
-  NX_REQUIRE(nq < (1ll << 30) && nk < (1ll << 30), "flash_attn_bwd: too many tiles");
-  dq<<<static_cast<unsigned>(min(nq, static_cast<long long>(sm_count()))), DQ_THREADS, BwdSmem<DP>::DYN, s>>>(m.q, m.k, m.v, m.d_o, p);
-  NX_LAUNCH_CHECK();
-  dkv<<<static_cast<unsigned>(min(nk, static_cast<long long>(sm_count()))), DKV_THREADS, BwdSmem<DP>::DYN, s>>>(m.q, m.k, m.v, m.d_o, p);
+template <typename Smem, typename K>
+static int persistent_launch(K kern, int threads, long long items, const BwdMaps& m, const AttnBwdParams& p, cudaStream_t s) {
+  NX_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::DYN));
+  kern<<<static_cast<unsigned>(min(items, static_cast<long long>(sm_count()))), threads, Smem::DYN, s>>>(m.q, m.k, m.v, m.d_o, p);
   NX_LAUNCH_CHECK();
   return NX_OK;
 }
 
-template <int DP, bool DROP>
-static int launch_bwd(const BwdMaps& m, const AttnBwdParams& p, cudaStream_t s) {
-  // (a zero scale would turn a masked score into NaN)
-  if constexpr (!DROP) {
-    if (p.alibi == nullptr && p.blk_rows == nullptr && p.scale != 0.f)
-      return launch_bwd_as<DP, false, false>(m, p, s);
-  }
-  return launch_bwd_as<DP, DROP, true>(m, p, s);
+template <int DP, bool ALIBI>
+static int launch_bwd(const BwdMaps& m, const AttnBwdParams& p, const BwdRoute& r, cudaStream_t s) {
+  const int rc = r.dq ? persistent_launch<BwdSmem<DP>>(attn_bwd_dq_kernel<DP, ALIBI>, DQ_THREADS, r.dq_items, m, p, s)
+                      : attn_bwd_tile_dq(m, p, s);
+  if (rc != NX_OK) return rc;
+  return r.dkv ? persistent_launch<BwdSmem<DP>>(attn_bwd_dkv_kernel<DP, ALIBI>, DKV_THREADS, r.dkv_items, m, p, s)
+               : attn_bwd_tile_dkv(m, p, s);
 }
 
 }  // namespace nx
@@ -1113,7 +1045,8 @@ NX_API int NX_SYM(nx_flash_attn_bwd)(const void* q, const void* k, const void* v
   p.blk_any = static_cast<const uint8_t*>(blk_any);
   p.blk_nkt = (Sk + AB - 1) / AB;
   p.blk_shift = blk_size == 16 ? 4 : blk_size == 32 ? 5 : blk_size == 64 ? 6 : 7;
-  if (p.drop_thr > 0u) return D <= 64 ? launch_bwd<64, true>(m, p, s) : launch_bwd<128, true>(m, p, s);
-  if (D <= 64) return launch_bwd<64, false>(m, p, s);
-  return launch_bwd<128, false>(m, p, s);
+  const BwdRoute route = attn_bwd_route(p);
+  NX_REQUIRE(route.dq_items < (1ll << 30) && route.dkv_items < (1ll << 30), "flash_attn_bwd: too many tiles");
+  if (alibi != nullptr) return D <= 64 ? launch_bwd<64, true>(m, p, route, s) : launch_bwd<128, true>(m, p, route, s);
+  return D <= 64 ? launch_bwd<64, false>(m, p, route, s) : launch_bwd<128, false>(m, p, route, s);
 }

@@ -502,6 +502,35 @@ def test_flash_attention_backward_tiles(b, sq, sk, h, hk, causal, window, d):
         assert (x.double() - y).norm() <= 3 * eps * (y.norm() + d ** 0.5 * x.numel() ** 0.5 * (sk == 1))
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("form", ["causal", "full", "window", "alibi", "alibi_full", "dropout", "sparse", "scale0"])
+@pytest.mark.parametrize("b,s,h,hk", [
+    (1, 190, 3, 3),             # fewer tiles than SMs
+    (3, 400, 40, 40),           # several items per SM
+    (5, 400, 40, 20),           # more than four, two query heads per key head
+    (128, 72, 3, 1)])           # several single-block items per SM
+def test_flash_attention_backward_routes(b, s, h, hk, form, d):
+    """Every form at sizes on both sides of the choice between persistent kernels and one CTA per tile, against the fp32
+    oracle's autograd: three roundings of unit eps, as above."""
+    from gpt_neox_b200.models.sparse_attention import block_layout
+    from gpt_neox_b200.ops.attention import BlockLayout, alibi_slopes, attention_reference, flash_attention
+    torch.manual_seed(30)
+    kw = {"full": dict(causal=False), "window": dict(window=130), "alibi": dict(alibi=alibi_slopes(h).to(DEV)),
+          "alibi_full": dict(alibi=alibi_slopes(h).to(DEV), causal=False), "dropout": dict(dropout_p=0.1, seed=5),
+          "scale0": dict(scale=0.0)}.get(form, {})
+    if form == "sparse":
+        kw = dict(block_layout=BlockLayout(block_layout("bigbird", (s + 31) // 32, {
+            "num_sliding_window_blocks": 3, "num_global_blocks": 1, "num_random_blocks": 1, "block": 32}, seed=3), 32))
+    ts = [bf(b, s, n, d, grad=True) for n in (h, hk, hk)]
+    g = bf(b, s, h, d)
+    got = torch.autograd.grad(flash_attention(*ts, **kw), ts, g)
+    ref = [t.detach().float().requires_grad_() for t in ts]
+    want = torch.autograd.grad(attention_reference(*ref, **kw)[0], ref, g.float())
+    eps = 2 ** -8 if DT == torch.bfloat16 else 2 ** -11
+    for x, y in zip(got, want):
+        assert (x.float() - y).norm() <= 3 * eps * y.norm() + 1e-6
+
+
 @pytest.mark.parametrize("env", [{"NEOX_ATTN_FWD_SHAPE": "1"}, {"NEOX_ATTN_FWD_SHAPE": "3"},
                                  {"NEOX_ATTN_BWD_WARPS": "4"}, {"NEOX_ATTN_DKV_PIPE": "0", "NEOX_ATTN_DQ_PIPE": "0"}],
                          ids=["fwd_shape1", "fwd_shape3", "bwd_4warps", "bwd_unpipelined"])
