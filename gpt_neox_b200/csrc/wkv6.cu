@@ -7,8 +7,8 @@
 // kernel_backward_111 / _222), which walks the whole sequence in one thread per channel and needs
 // the sequence length as a compile-time constant for a per-thread array.
 //
-// Heads of 64 (every configuration here) go in blocks of 16 steps as matrix products (second half of this file).  Heads of 32
-// go step by step: one CTA of 2 N threads walks one head's piece of the sequence with the N x N state in registers: warp w owns
+// Heads of 64 in bf16 go in blocks of 16 steps as matrix products (second half of this file; wkv_in_blocks).  Heads of 32,
+// fp16 and a few short sequences go step by step: one CTA of 2 N threads walks one head's piece of the sequence with the N x N state in registers: warp w owns
 // 16 columns j, a lane N / 8 rows i by 4 columns.  Per step a lane reads N / 8 values of each row vector and 4 of each column
 // vector from shared memory (column vectors are stored twice side by side, so that the packed fp32 pairs, which run
 // over neighbouring rows, need no register moves) and does 3 packed operations per 2 state elements: one for the output
@@ -16,7 +16,7 @@
 // one value.  Sums over rows / columns leave a lane by transposing exchanges.
 //   forward  : one sweep: y (sum over i)
 //   backward : a forward sweep: gr (sum over j), then a reverse sweep of the gradient state G = dL/dS with gk (sum over j)
-//              and gv (sum over i; a sweep of its own for heads of 64), which also forms the decay gradient: with
+//              and gv (sum over i; a sweep of its own in blocks), which also forms the decay gradient: with
 //              Q_t[i] = sum_j G_t[i][j] S_t[i][j] one has Q_{t-1} - Q_t = r_t gr_t - k_t gk_t and
 //              dL/d(ew_t) = Q_t - k_t (gk_t - r_t u s_t),  s_t = <gy_t, v_t>,  ew = -exp(w)
 // Step by step the shared-memory loads and exchanges of the steps are the bound (32 x 512 tokens, 12 heads of 64, forward +
@@ -332,9 +332,8 @@ __global__ void __launch_bounds__(2 * N) wkv_kernel(const WkvParams p) {
 //
 // Four warps; the state is the accumulators of mma.m16n8k16 (warp w: 16 of its rows, a thread 32 values), fp32 throughout.
 // What is not a 16-bit input is split into three bf16 parts (24 bits: the products of parts of weight 2^-16 and above are
-// all formed; the rest is below fp32's last bit), fp16 inputs into two, which is exact: the sums are those of fp32
-// arithmetic in another order.  These products are far too small for tcgen05 (M = 16 rows of steps, operands made in
-// registers between every two of them), hence mma.sync.
+// all formed; the rest is below fp32's last bit): the sums are those of fp32 arithmetic in another order.  These products
+// are far too small for tcgen05 (M = 16 rows of steps, operands made in registers between every two of them), hence mma.sync.
 // Infinite states or inputs give NaN where step-by-step arithmetic may give infinities (a part of zero times infinity); a
 // product over a block's steps is formed value by value where an input of the block is not finite, so that what is not finite
 // does not reach earlier steps.
@@ -344,9 +343,9 @@ constexpr int WN = 64;              // head size
 constexpr int WP = WN + 8;          // row pitch of the 16-bit arrays: ldmatrix without bank conflicts
 constexpr int WM_THREADS = 128;
 #ifdef NX_HALF
-constexpr int WM_IN = 2;            // bf16 parts of an input
+constexpr bool WM_BLOCKS = false;
 #else
-constexpr int WM_IN = 1;
+constexpr bool WM_BLOCKS = true;
 #endif
 
 __device__ __forceinline__ uint32_t wm_bf16x2(float lo, float hi) {
@@ -387,34 +386,12 @@ __device__ __forceinline__ void wm_ld4(uint32_t (&r)[4], const uint16_t* base, i
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 
-// An input block: as it lies in memory (for the scalar uses), and as bf16 parts (for the products).
+// An input block.
 struct WmIn {
   uint16_t raw[WM][WP];
-#ifdef NX_HALF
-  uint16_t part[WM_IN][WM][WP];
-  __device__ __forceinline__ const uint16_t* parts(int p) const { return &part[p][0][0]; }
-#else
-  __device__ __forceinline__ const uint16_t* parts(int) const { return &raw[0][0]; }
-#endif
-  __device__ __forceinline__ void put(int t, int c8, const uint4& u) {
-    *reinterpret_cast<uint4*>(&raw[t][c8]) = u;
-#ifdef NX_HALF
-    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-    uint32_t hi[4], lo[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float2 x = unpack_h16x2(w[k]), m1 = make_float2(-1.f, -1.f);
-      hi[k] = wm_bf16x2(x.x, x.y);
-      const float2 rest = ffma2(wm_floats(hi[k]), m1, x);
-      lo[k] = wm_bf16x2(rest.x, rest.y);
-    }
-    *reinterpret_cast<uint4*>(&part[0][t][c8]) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-    *reinterpret_cast<uint4*>(&part[1][t][c8]) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-#endif
-  }
-  __device__ __forceinline__ float at(int t, int c) const {
-    return h16_to_float(reinterpret_cast<const h16&>(raw[t][c]));
-  }
+  __device__ __forceinline__ const uint16_t* data() const { return &raw[0][0]; }
+  __device__ __forceinline__ void put(int t, int c8, const uint4& u) { *reinterpret_cast<uint4*>(&raw[t][c8]) = u; }
+  __device__ __forceinline__ float at(int t, int c) const { return h16_to_float(reinterpret_cast<const h16&>(raw[t][c])); }
   __device__ __forceinline__ float2 pair(int t, int c) const {
     return unpack_h16x2(*reinterpret_cast<const uint32_t*>(&raw[t][c]));
   }
@@ -422,11 +399,7 @@ struct WmIn {
 
 __device__ __forceinline__ bool wm_all_finite(const uint4& u) {
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#ifdef NX_HALF
-  constexpr uint32_t E = 0x7c00u;
-#else
   constexpr uint32_t E = 0x7f80u;
-#endif
   bool ok = true;
 #pragma unroll
   for (int k = 0; k < 4; ++k) ok = ok && (w[k] & E) != E && ((w[k] >> 16) & E) != E;
@@ -506,10 +479,15 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
       float w8[8], d8[8];
       wk_unpack8(rw, w8);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float ew = live ? -__expf(w8[e]) : 0.f;
-        d8[e] = __expf(ew);
-        if (LOCAL) sew[e] += ew;
+      for (int e = 0; e < 8; e += 2) {
+        const float2 ew = live ? make_float2(-__expf(w8[e]), -__expf(w8[e + 1])) : make_float2(0.f, 0.f);
+        const float2 d = make_float2(__expf(ew.x), __expf(ew.y));
+        d8[e] = d.x;
+        d8[e + 1] = d.y;
+        if (LOCAL) {
+          sew[e] += ew.x;
+          sew[e + 1] += ew.y;
+        }
       }
       *reinterpret_cast<float4*>(&s.d[trow][ch8]) = make_float4(d8[0], d8[1], d8[2], d8[3]);
       *reinterpret_cast<float4*>(&s.d[trow][ch8 + 4]) = make_float4(d8[4], d8[5], d8[6], d8[7]);
@@ -620,9 +598,8 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
     }
     if (q > 0) {
     // ---- products of block q - 1
-    uint32_t cv[WM_IN][4];               // c^T: 16 rows j of this warp x 16 steps
-#pragma unroll
-    for (int k = 0; k < WM_IN; ++k) wm_ld4<true>(cv[k], former.c.parts(k), 0, warp * 16, WP, false);
+    uint32_t cv[4];                      // c^T: 16 rows j of this warp x 16 steps
+    wm_ld4<true>(cv, former.c.data(), 0, warp * 16, WP, false);
     if (!LOCAL) {
       float y[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
       float z[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};      // (two chains of dependent products)
@@ -657,11 +634,8 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
         for (int k = 2; k >= 0; --k) {
           uint32_t b[4];
           wm_ld4<false>(b, &former.A[k][0][0], 0, 0, 24, false);
-#pragma unroll
-          for (int m = 0; m < WM_IN; ++m) {
-            wm_mma(y[0], cv[m], b[0], b[1]);
-            wm_mma(y[1], cv[m], b[2], b[3]);
-          }
+          wm_mma(y[0], cv, b[0], b[1]);
+          wm_mma(y[1], cv, b[2], b[3]);
         }
       } else {
 #pragma unroll
@@ -695,11 +669,8 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
       for (int k = 2; k >= 0; --k) {
         uint32_t b[4];
         wm_ld4<true>(b, &former.bp[k][0][0], 0, 8 * n, WP, true);
-#pragma unroll
-        for (int m = 0; m < WM_IN; ++m) {
-          wm_mma(S[n], cv[m], b[0], b[1]);
-          wm_mma(S[n + 1], cv[m], b[2], b[3]);
-        }
+        wm_mma(S[n], cv, b[0], b[1]);
+        wm_mma(S[n + 1], cv, b[2], b[3]);
       }
     }
     __syncthreads();
@@ -803,10 +774,10 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_row_kernel(const WkvParams 
       float w8[8];
       wk_unpack8(rw, w8);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float ew = live ? -__expf(w8[e]) : 0.f;
-        now.ew[trow][ch8 + e] = ew;
-        s.d[trow][ch8 + e] = __expf(ew);
+      for (int e = 0; e < 8; e += 2) {
+        const float2 ew = live ? make_float2(-__expf(w8[e]), -__expf(w8[e + 1])) : make_float2(0.f, 0.f);
+        *reinterpret_cast<float2*>(&now.ew[trow][ch8 + e]) = ew;
+        *reinterpret_cast<float2*>(&s.d[trow][ch8 + e]) = make_float2(__expf(ew.x), __expf(ew.y));
       }
     }
     }
@@ -822,18 +793,12 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_row_kernel(const WkvParams 
     if (q < nblk && warp < 2) {
       float m4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-        for (int x = 0; x < WM_IN; ++x) {
-          uint32_t a[4];
-          wm_ld4<false>(a, now.e.parts(x), 0, 16 * ks, WP, true);
-#pragma unroll
-          for (int z = 0; z < WM_IN; ++z) {
-            uint32_t b[4];
-            wm_ld4<false>(b, now.c.parts(z), 0, 16 * ks, WP, false);
-            wm_mma(m4, a, warp == 0 ? b[0] : b[2], warp == 0 ? b[1] : b[3]);
-          }
-        }
+      for (int ks = 0; ks < 4; ++ks) {
+        uint32_t a[4], b[4];
+        wm_ld4<false>(a, now.e.data(), 0, 16 * ks, WP, true);
+        wm_ld4<false>(b, now.c.data(), 0, 16 * ks, WP, false);
+        wm_mma(m4, a, warp == 0 ? b[0] : b[2], warp == 0 ? b[1] : b[3]);
+      }
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int t = (lane >> 2) + (e >> 1) * 8, x = warp * 8 + n0 + (e & 1);
@@ -855,15 +820,12 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_row_kernel(const WkvParams 
           wm_split(make_float2(src[0], src[1]), x);
           sp[0][e] = x[0]; sp[1][e] = x[1]; sp[2][e] = x[2];
         }
+        uint32_t b[4];
+        wm_ld4<false>(b, former.e.data(), 0, 16 * ks, WP, false);
 #pragma unroll
-        for (int z = 0; z < WM_IN; ++z) {
-          uint32_t b[4];
-          wm_ld4<false>(b, former.e.parts(z), 0, 16 * ks, WP, false);
-#pragma unroll
-          for (int m = 2; m >= 0; --m) {
-            wm_mma(y[0], sp[m], b[0], b[1]);
-            wm_mma(y[1], sp[m], b[2], b[3]);
-          }
+        for (int m = 2; m >= 0; --m) {
+          wm_mma(y[0], sp[m], b[0], b[1]);
+          wm_mma(y[1], sp[m], b[2], b[3]);
         }
       }
 #pragma unroll
@@ -879,17 +841,15 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_row_kernel(const WkvParams 
 #pragma unroll
       for (int k = 0; k < 3; ++k) wm_ld4<true>(bt[k], &former.bp[k][0][0], 0, warp * 16, WP, false);
 #pragma unroll
-      for (int n = 0; n < 8; n += 2)
+      for (int n = 0; n < 8; n += 2) {
+        uint32_t b[4];
+        wm_ld4<true>(b, former.c.data(), 0, 8 * n, WP, true);
 #pragma unroll
-        for (int z = 0; z < WM_IN; ++z) {
-          uint32_t b[4];
-          wm_ld4<true>(b, former.c.parts(z), 0, 8 * n, WP, true);
-#pragma unroll
-          for (int k = 2; k >= 0; --k) {
-            wm_mma(S[n], bt[k], b[0], b[1]);
-            wm_mma(S[n + 1], bt[k], b[2], b[3]);
-          }
+        for (int k = 2; k >= 0; --k) {
+          wm_mma(S[n], bt[k], b[0], b[1]);
+          wm_mma(S[n + 1], bt[k], b[2], b[3]);
         }
+      }
     }
     }
     __syncthreads();
@@ -1059,46 +1019,61 @@ static int wkv_row(const WkvParams& p, bool vec, cudaStream_t stream) {
   return wkv64_launch<WmRowSmem>(wkv_row_kernel<REV, true>, wkv_row_kernel<REV, false>, p, vec, p.NC, stream);
 }
 
+// Which calls go in blocks: bf16 (an fp16 input would take two parts, and its products twice to four times as many: 32 x 512, 12
+// heads 997 us, step by step 780; 8 x 2048, 16 heads 1,508 against 1,363), and not a few short sequences, where the fourth
+// sweep's launch and a block's latency count (forward + backward, step by step / in blocks: 1 x 16, 12 heads 0.89, 8 x 16
+// 0.87, 4 x 32 0.95, 1 x 128, 8 heads 0.97; 16 x 16 0.99, 32 x 16 1.11, 8 x 64, 8 heads 1.07, 1 x 200, 16 heads 1.05).
+static bool wkv_in_blocks(int B, int T, int H, int N) {
+  return WM_BLOCKS && N == WN && (T > 128 || static_cast<long long>(B) * H * T >= 3072);
+}
+
+// One sweep, in blocks or step by step.
+template <int N, int MODE>
+static int wkv_sweep(const WkvParams& p, bool vec, int chunks, cudaStream_t stream) {
+  if constexpr (N == WN && WM_BLOCKS) {
+    if (wkv_in_blocks(p.B, p.T, p.H, N)) {
+      if constexpr (MODE == WK_LOCAL_FWD) return wkv_col<false, true>(p, vec, chunks, stream);
+      if constexpr (MODE == WK_LOCAL_REV) return wkv_col<true, true>(p, vec, chunks, stream);
+      if constexpr (MODE == WK_Y) return wkv_col<false, false>(p, vec, chunks, stream);
+      if constexpr (MODE == WK_GR) return wkv_row<false>(p, vec, stream);
+      if constexpr (MODE == WK_G) {
+        const int rc = wkv_row<true>(p, vec, stream);
+        return rc != NX_OK ? rc : wkv_col<true, false>(p, vec, chunks, stream);
+      }
+    }
+  }
+  return wkv_launch<N, MODE>(p, vec, chunks, stream);
+}
+
 template <int N>
 static int wkv_forward(WkvParams p, float* start, cudaStream_t stream) {
   const bool vec = wkv_vec_ok(p);
   if (p.NC > 1) {
-    int rc;
-    if constexpr (N == WN) rc = wkv_col<false, true>(p, vec, p.NC - 1, stream);
-    else rc = wkv_launch<N, WK_LOCAL_FWD>(p, vec, p.NC - 1, stream);
+    const int rc = wkv_sweep<N, WK_LOCAL_FWD>(p, vec, p.NC - 1, stream);
     if (rc != NX_OK) return rc;
     wkv_fold_kernel<N, false><<<dim3(N, p.H, p.B), N, 0, stream>>>(p.local, p.sumew, start, p.NC);
     NX_LAUNCH_CHECK();
     p.start = start;
   }
-  if constexpr (N == WN) return wkv_col<false, false>(p, vec, p.NC, stream);
-  else return wkv_launch<N, WK_Y>(p, vec, p.NC, stream);
+  return wkv_sweep<N, WK_Y>(p, vec, p.NC, stream);
 }
 
 template <int N>
 static int wkv_backward(WkvParams p, const float* fstart, float* rstart, float* gu, cudaStream_t stream) {
   const bool vec = wkv_vec_ok(p);
   p.start = p.NC > 1 ? fstart : nullptr;
-  int rc;
-  if constexpr (N == WN) rc = wkv_row<false>(p, vec, stream);
-  else rc = wkv_launch<N, WK_GR>(p, vec, p.NC, stream);
+  int rc = wkv_sweep<N, WK_GR>(p, vec, p.NC, stream);
   if (rc != NX_OK) return rc;
   p.start = nullptr;
   if (p.NC > 1) {
-    if constexpr (N == WN) rc = wkv_col<true, true>(p, vec, p.NC - 1, stream);
-    else rc = wkv_launch<N, WK_LOCAL_REV>(p, vec, p.NC - 1, stream);
+    rc = wkv_sweep<N, WK_LOCAL_REV>(p, vec, p.NC - 1, stream);
     if (rc != NX_OK) return rc;
     wkv_fold_kernel<N, true><<<dim3(N, p.H, p.B), N, 0, stream>>>(p.local, p.sumew, rstart, p.NC);
     NX_LAUNCH_CHECK();
     p.start = rstart;
     p.fstart = fstart;
   }
-  if constexpr (N == WN) {
-    rc = wkv_row<true>(p, vec, stream);
-    if (rc == NX_OK) rc = wkv_col<true, false>(p, vec, p.NC, stream);
-  } else {
-    rc = wkv_launch<N, WK_G>(p, vec, p.NC, stream);
-  }
+  rc = wkv_sweep<N, WK_G>(p, vec, p.NC, stream);
   if (rc != NX_OK) return rc;
   wkv_sum_kernel<<<(p.H * N + WK_SUM_X - 1) / WK_SUM_X, dim3(WK_SUM_X, WK_SUM_Y), 0, stream>>>(p.gu_part, gu, p.B * p.NC,
                                                                                           p.H * N);
@@ -1107,6 +1082,8 @@ static int wkv_backward(WkvParams p, const float* fstart, float* rstart, float* 
 }
 
 NX_API int NX_SYM(nx_wkv6_chunks)(int B, int T, int H) { return wkv_chunk_count(B, T, H); }
+// Kernels a backward launches (two more where there are several chunks).
+NX_API int NX_SYM(nx_wkv6_bwd_launches)(int B, int T, int H, int N) { return wkv_in_blocks(B, T, H, N) ? 4 : 3; }
 
 // r, k, v, w: bf16 [B, T, H*N] addressed by (sb, st); u fp32 [H, N]; y bf16 by (osb, ost).  With NC =
 // nx_wkv6_chunks(B, T, H) > 1: local / start fp32 [B, H, NC, N, N] and sumew fp32 [B, H, NC, N] are scratch, and

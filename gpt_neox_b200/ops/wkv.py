@@ -103,8 +103,9 @@ class _WkvFn(torch.autograd.Function):
         if start is not None:
             local, rstart = torch.empty_like(start), torch.empty_like(start)
             sumew = torch.empty(start.shape[:4], device=dev, dtype=torch.float32)
-        LAUNCHES["n"] += (4 if N == 64 else 3) + (0 if start is None else 2)
-        _lib.check(_lib.lib(r).nx_wkv6_bwd(
+        lib = _lib.lib(r)
+        LAUNCHES["n"] += lib.nx_wkv6_bwd_launches(B, T, H, N) + (0 if start is None else 2)
+        _lib.check(lib.nx_wkv6_bwd(
             _lib.ptr(r), _lib.ptr(k), _lib.ptr(v), _lib.ptr(w), _lib.ptr(gy), r.stride(0), r.stride(1), _lib.ptr(u32),
             _lib.ptr(gr), _lib.ptr(gk), _lib.ptr(gv), _lib.ptr(gw), _lib.ptr(gr32), _lib.ptr(gu), _lib.ptr(gu_part),
             gr.stride(0), gr.stride(1), _lib.ptr(local), _lib.ptr(start), _lib.ptr(rstart), _lib.ptr(sumew), B, T, H, N,

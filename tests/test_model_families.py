@@ -132,7 +132,8 @@ def test_wkv6_gradients_repeat_bit_for_bit(B, T, H, N):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("B,T,H", [(1, 15, 1), (2, 16, 3), (1, 33, 2), (45, 50, 10), (1, 600, 2)])
+@pytest.mark.parametrize("B,T,H", [(1, 15, 1), (2, 16, 3), (1, 33, 2), (45, 50, 10), (1, 600, 2), (64, 15, 4), (24, 33, 4),
+                                   (3, 129, 1)])
 @pytest.mark.parametrize("w", [-12.0, -1.0, 2.0, 6.0])
 def test_wkv6_blocks_of_steps(B, T, H, w, dtype):
     """Heads of 64 in blocks of 16 steps: short blocks, one chunk and many, decays from 1 - 6e-6 to an underflowing one, against
