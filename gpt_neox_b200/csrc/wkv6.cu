@@ -334,9 +334,8 @@ __global__ void __launch_bounds__(2 * N) wkv_kernel(const WkvParams p) {
 // What is not a 16-bit input is split into three bf16 parts (24 bits: the products of parts of weight 2^-16 and above are
 // all formed; the rest is below fp32's last bit): the sums are those of fp32 arithmetic in another order.  These products
 // are far too small for tcgen05 (M = 16 rows of steps, operands made in registers between every two of them), hence mma.sync.
-// Infinite states or inputs give NaN where step-by-step arithmetic may give infinities (a part of zero times infinity); a
-// product over a block's steps is formed value by value where an input of the block is not finite, so that what is not finite
-// does not reach earlier steps.
+// Infinity and what bf16 rounds to it have no parts, and a product of two vectors may leave fp32's range where the steps' own
+// products do not: a block with such an input or state is done step by step, with the results of the step-by-step kernel.
 // ------------------------------------------------------------------------------------------------
 constexpr int WM = 16;              // steps per block
 constexpr int WN = 64;              // head size
@@ -397,13 +396,30 @@ struct WmIn {
   }
 };
 
-__device__ __forceinline__ bool wm_all_finite(const uint4& u) {
+// Whether all of eight bf16 inputs are below 2^20 (infinity and NaN are not).  Then no product over a block's vectors
+// overflows, and what one loses when it underflows is below 2^-100.
+__device__ __forceinline__ bool wm_ordinary(const uint4& u) {
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-  constexpr uint32_t E = 0x7f80u;
+  constexpr uint32_t E = (127u + 20u) << 7;
   bool ok = true;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) ok = ok && (w[k] & E) != E && ((w[k] >> 16) & E) != E;
+  for (int k = 0; k < 4; ++k) ok = ok && (w[k] & 0x7f80u) < E && ((w[k] >> 16) & 0x7f80u) < E;
   return ok;
+}
+
+// Whether this warp's states hold something that three parts do not: infinity, NaN, or a value that bf16 rounds to infinity
+// (squares overflow long before; a state above 1e19 is as right step by step).
+constexpr float WM_PART_MAX = 3.0e38f;
+__device__ __forceinline__ bool wm_odd_state(const float (&S)[8][4]) {
+  float2 z[2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll
+  for (int n = 0; n < 8; ++n)
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const float2 x = make_float2(S[n][2 * k], S[n][2 * k + 1]);
+      z[k] = ffma2(x, x, z[k]);
+    }
+  return __any_sync(0xffffffffu, !(z[0].x + z[0].y + (z[1].x + z[1].y) < INFINITY));
 }
 
 // Step s of block q in a sweep's order -> time.  Blocks start at the sweep's first step, so that a short one is the last.
@@ -421,7 +437,7 @@ struct WmColSmem {
     uint16_t A[3][WM][24];
     uint16_t out[WM][WP];
     float tot[WN];
-    bool finite;
+    int odd_input, odd_A[2];                 // an input / an entry of A (by warp; u is in it) out of the products' range
   } blk[2];
 };
 static_assert(offsetof(WmColSmem, d) % 16 == 0 && offsetof(WmColSmem, blk) % 16 == 0 && sizeof(WmColSmem::Block) % 16 == 0 &&
@@ -432,7 +448,7 @@ static_assert(offsetof(WmColSmem, d) % 16 == 0 && offsetof(WmColSmem, blk) % 16 
 
 // Column sums (y, or gv in reverse), or (LOCAL) only the end state of a chunk from a zero state and the sums of ew.
 template <bool REV, bool LOCAL, bool VEC>
-__global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams p) {
+__global__ void __launch_bounds__(WM_THREADS, 3) wkv_col_kernel(const WkvParams p) {
   extern __shared__ __align__(16) unsigned char wk_raw[];
   WmColSmem& s = *reinterpret_cast<WmColSmem*>(wk_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -492,8 +508,8 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
       *reinterpret_cast<float4*>(&s.d[trow][ch8]) = make_float4(d8[0], d8[1], d8[2], d8[3]);
       *reinterpret_cast<float4*>(&s.d[trow][ch8 + 4]) = make_float4(d8[4], d8[5], d8[6], d8[7]);
     }
-    const bool all_finite = !__syncthreads_or(!LOCAL && q < nblk && !wm_all_finite(rc));
-    if (tid == 0) now.finite = all_finite;
+    const int odd_input = __syncthreads_or(q < nblk && !(wm_ordinary(rb) && wm_ordinary(rc) && (LOCAL || wm_ordinary(ra))));
+    if (tid == 0) now.odd_input = odd_input;
     if (q + 1 < nblk) fetch(q + 1);      // in flight during this round
     if (!LOCAL && q > 1) {               // (the sums of block q - 2, laid out in the last round)
       const int t = wm_time<REV>(t_lo, t_hi, q - 2, trow);
@@ -581,7 +597,9 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
 #pragma unroll
       for (int k = 0; k < 2; ++k)
         v2[k] = (h1 ? v4[2 + k] : v4[k]) + __shfl_xor_sync(0xffffffffu, h1 ? v4[k] : v4[2 + k], 1);
+      bool odd_A = false;
       auto put_A = [&](int t, int col, float x) {
+        odd_A = odd_A || !(fabsf(x) < WM_PART_MAX);
         uint32_t y[3];
         wm_split(make_float2(x, 0.f), y);
 #pragma unroll
@@ -595,8 +613,48 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
         else put_A(turn + 1 + (it - turn), turn, v2[k]);
       }
       if ((lane & 7) == 0) put_A(turn, turn, diag);
+      odd_A = __any_sync(0xffffffffu, odd_A);
+      if (lane == 0) now.odd_A[warp - 2] = odd_A;
     }
-    if (q > 0) {
+    if (q > 0 && (former.odd_input || (!LOCAL && (former.odd_A[0] || former.odd_A[1])) || wm_odd_state(S))) {
+      // ---- block q - 1 step by step
+#pragma unroll 1
+      for (int x = 0; x < WM; ++x) {
+        const int t = wm_time<REV>(t_lo, t_hi, q - 1, x);
+        if (t < t_lo || t >= t_hi) break;
+        const long long o = bi * p.sb + (long long)t * p.st + h * WN;
+        const float c0 = former.c.at(x, j0), c1 = former.c.at(x, j0 + 8);
+        float y0 = 0.f, y1 = 0.f, dot = 0.f;
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int i = 8 * n + i0 + e;
+            const float b = h16_to_float(gb[o + i]), d = __expf(-__expf(h16_to_float(p.w[o + i])));
+            if (!LOCAL) {
+              const float a = h16_to_float(ga[o + i]);
+              y0 += a * S[n][e];
+              y1 += a * S[n][2 + e];
+              dot += a * p.u[h * WN + i] * b;
+            }
+            S[n][e] = S[n][e] * d + b * c0;
+            S[n][2 + e] = S[n][2 + e] * d + b * c1;
+          }
+        if (!LOCAL) {
+#pragma unroll
+          for (int m = 2; m > 0; m >>= 1) {
+            y0 += __shfl_xor_sync(0xffffffffu, y0, m);
+            y1 += __shfl_xor_sync(0xffffffffu, y1, m);
+            dot += __shfl_xor_sync(0xffffffffu, dot, m);
+          }
+          if ((lane & 3) == 0) {
+            const h16 o0 = float_to_h16(y0 + c0 * dot), o1 = float_to_h16(y1 + c1 * dot);
+            former.out[x][j0] = reinterpret_cast<const uint16_t&>(o0);
+            former.out[x][j0 + 8] = reinterpret_cast<const uint16_t&>(o1);
+          }
+        }
+      }
+    } else if (q > 0) {
     // ---- products of block q - 1
     uint32_t cv[4];                      // c^T: 16 rows j of this warp x 16 steps
     wm_ld4<true>(cv, former.c.data(), 0, warp * 16, WP, false);
@@ -629,26 +687,12 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_col_kernel(const WkvParams 
         y[0][e] += z[0][e];
         y[1][e] += z[1][e];
       }
-      if (former.finite) {
 #pragma unroll
-        for (int k = 2; k >= 0; --k) {
-          uint32_t b[4];
-          wm_ld4<false>(b, &former.A[k][0][0], 0, 0, 24, false);
-          wm_mma(y[0], cv, b[0], b[1]);
-          wm_mma(y[1], cv, b[2], b[3]);
-        }
-      } else {
-#pragma unroll
-        for (int n = 0; n < 2; ++n)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int t = 8 * n + i0 + (e & 1), j = j0 + (e >> 1) * 8;
-            for (int x = 0; x <= t; ++x) {
-              float a = 0.f;
-              for (int k = 2; k >= 0; --k) a += __uint_as_float(static_cast<uint32_t>(former.A[k][t][x]) << 16);
-              y[n][e] += a * former.c.at(x, j);
-            }
-          }
+      for (int k = 2; k >= 0; --k) {
+        uint32_t b[4];
+        wm_ld4<false>(b, &former.A[k][0][0], 0, 0, 24, false);
+        wm_mma(y[0], cv, b[0], b[1]);
+        wm_mma(y[1], cv, b[2], b[3]);
       }
 #pragma unroll
       for (int n = 0; n < 2; ++n)
@@ -711,6 +755,7 @@ struct WmRowSmem {
     float st[WM];
     float part[2][WM][WN];                   // what a block's own steps add, by the parity of s
     float pre[WM][WN], tot[WN];
+    int odd_input;                           // an input out of the products' range
   } blk[2];
 };
 static_assert(offsetof(WmRowSmem, M) % 16 == 0 && offsetof(WmRowSmem, blk) % 16 == 0 && sizeof(WmRowSmem::Block) % 16 == 0 &&
@@ -719,7 +764,7 @@ static_assert(offsetof(WmRowSmem, M) % 16 == 0 && offsetof(WmRowSmem, blk) % 16 
 
 // Row sums: gr (fp32 and rounded), or in reverse gk with the decay gradient and the sums for the gradient of u.
 template <bool REV, bool VEC>
-__global__ void __launch_bounds__(WM_THREADS, 4) wkv_row_kernel(const WkvParams p) {
+__global__ void __launch_bounds__(WM_THREADS, 3) wkv_row_kernel(const WkvParams p) {
   extern __shared__ __align__(16) unsigned char wk_raw[];
   WmRowSmem& s = *reinterpret_cast<WmRowSmem*>(wk_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -781,7 +826,8 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_row_kernel(const WkvParams 
       }
     }
     }
-    __syncthreads();
+    const int odd_input = __syncthreads_or(q < nblk && !(wm_ordinary(rb) && wm_ordinary(rc) && wm_ordinary(re)));
+    if (tid == 0) now.odd_input = odd_input;
     if (q + 1 < nblk) fetch(q + 1);      // in flight during this round
     float gr[REV ? WM : 1];
     if (REV && half == 0 && q > 0) {
@@ -806,7 +852,41 @@ __global__ void __launch_bounds__(WM_THREADS, 4) wkv_row_kernel(const WkvParams 
         if (t == x) now.st[t] = m4[e];
       }
     }
-    if (q > 0) {
+    if (q > 0 && (former.odd_input || wm_odd_state(S))) {
+      // ---- block q - 1 step by step: whole row sums, in the place of the state's part of them
+#pragma unroll 1
+      for (int x = 0; x < steps; ++x) {
+        const float b0 = former.b.at(x, r0), b1 = former.b.at(x, r0 + 8);
+        const float2 d = make_float2(__expf(former.ew[x][r0]), __expf(former.ew[x][r0 + 8]));
+        float y0 = 0.f, y1 = 0.f, st = 0.f;
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const float c = former.c.at(x, 8 * n + n0 + k), e = former.e.at(x, 8 * n + n0 + k);
+            y0 += e * S[n][k];
+            y1 += e * S[n][2 + k];
+            st += e * c;
+            S[n][k] = S[n][k] * d.x + b0 * c;
+            S[n][2 + k] = S[n][2 + k] * d.y + b1 * c;
+          }
+#pragma unroll
+        for (int m = 2; m > 0; m >>= 1) {
+          y0 += __shfl_xor_sync(0xffffffffu, y0, m);
+          y1 += __shfl_xor_sync(0xffffffffu, y1, m);
+          st += __shfl_xor_sync(0xffffffffu, st, m);
+        }
+        if ((lane & 3) == 0) {
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            s.inter[x][r0 + 8 * k] = k == 0 ? y0 : y1;
+            former.pre[x][r0 + 8 * k] = 1.f;
+            former.part[0][x][r0 + 8 * k] = former.part[1][x][r0 + 8 * k] = 0.f;
+          }
+        }
+        if (former.odd_input && tid == 0) former.st[x] = st;
+      }
+    } else if (q > 0) {
     // ---- products
     {
       float y[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};

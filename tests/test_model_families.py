@@ -1,5 +1,7 @@
 """RWKV-6, gMLP / aMLP and mixed stacks build and train through the public training entry on CPU;
 kernel numerics of the WKV recurrence on the GPU."""
+import math
+
 import pytest
 import torch
 
@@ -181,3 +183,83 @@ def test_wkv6_passes_nan_and_inf_on(what, value, at):
     got, want = wkv6(*ts, u), wkv6_reference(*(t.float() for t in ts), u.float())
     assert torch.equal(got.isfinite(), want.isfinite())
     assert got.isfinite().all() == want.isfinite().all()
+
+
+def _wkv6_sweeps(r, k, v, w, u, gy):
+    """y and the gradients of r, k, v, w, u as two sweeps form them, one step after the other, in fp32 (64 bits for 64-bit inputs)."""
+    B, T, _ = r.shape
+    H, N = u.shape
+    wide = lambda t: t if t.dtype == torch.float64 else t.float()
+    r, k, v, w, gy = (wide(t).reshape(B, T, H, N) for t in (r, k, v, w, gy))
+    u, ew = wide(u), -torch.exp(w)
+    S, out = r.new_zeros(B, H, N, N), [[] for _ in range(5)]
+    dot = lambda a, b: (a * b).sum(-1, keepdim=True)
+    for t in range(T):
+        st = dot(gy[:, t], v[:, t])
+        out[0].append((r[:, t, :, :, None] * S).sum(-2) + dot(r[:, t] * u, k[:, t]) * v[:, t])
+        out[1].append((S * gy[:, t, :, None]).sum(-1) + u * k[:, t] * st)
+        S = torch.exp(ew[:, t])[..., None] * S + k[:, t, :, :, None] * v[:, t, :, None]
+    G, Q, gu = torch.zeros_like(S), torch.zeros_like(r[:, 0]), torch.zeros_like(r[:, 0])
+    for t in reversed(range(T)):
+        st = dot(gy[:, t], v[:, t])
+        row = (G * v[:, t, :, None]).sum(-1)
+        gk = row + u * r[:, t] * st
+        out[2].append(gk)
+        out[3].append((k[:, t, :, :, None] * G).sum(-2) + dot(k[:, t] * u, r[:, t]) * gy[:, t])
+        out[4].append((Q - k[:, t] * row) * ew[:, t])
+        Q = Q + r[:, t] * out[1][t] - k[:, t] * gk
+        gu = gu + r[:, t] * k[:, t] * st
+        G = torch.exp(ew[:, t])[..., None] * G + r[:, t, :, :, None] * gy[:, t, :, None]
+    y, gr = (torch.stack(x, 1).flatten(2) for x in out[:2])
+    gk, gv, gw = (torch.stack(x[::-1], 1).flatten(2) for x in out[2:])
+    return y, gr, gk, gv, gw, gu.sum(0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,T,H", [(1, 100, 2), (1, 200, 2), (45, 50, 10)])       # step by step; many chunks and one
+@pytest.mark.parametrize("positive", [True, False])
+@pytest.mark.parametrize("what", [0, 1, 2, 4])                           # r, k, v, the gradient of y
+def test_wkv6_infinities_are_those_of_single_steps(what, positive, B, T, H, dtype):
+    """An infinite value gives infinities and NaN where sums of one step after the other give them, no more."""
+    from gpt_neox_b200.ops.wkv import wkv6
+    torch.manual_seed(12)
+    N = 64
+    ts = [(torch.randn(B, T, H * N, device="cuda") * 0.5 - (3.0 if i == 3 else 0.0)).to(dtype) for i in range(5)]
+    u = (torch.randn(H, N, device="cuda") * 0.3).to(dtype)
+    if positive:
+        u, ts = u.abs(), [t if i == 3 else t.abs() for i, t in enumerate(ts)]
+    ts[what][0, 21, 70] = math.inf
+    leaves = [t.requires_grad_() for t in (*ts[:4], u)]
+    y = wkv6(*leaves)
+    got = (y.detach(),) + torch.autograd.grad(y, leaves, ts[4])
+    gr, gk, gv, gw, gu = got[1:]
+    want = _wkv6_sweeps(*(t.detach() for t in ts[:4]), u.detach(), ts[4])
+    for n, (a, b) in enumerate(zip((y, gr, gk, gv, gw, gu), want)):
+        if n == 4 and B == 1:
+            continue                    # (the running difference starts anew in every chunk)
+        b = b.to(dtype)
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isposinf(), b.isposinf()) \
+            and torch.equal(a.isneginf(), b.isneginf()), n
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,T", [(1, 24), (64, 48), (1, 150)])
+@pytest.mark.parametrize("scales", [(2.0 ** 100, 2.0 ** 100, 2.0 ** -100, 2.0 ** -90),      # r k and gy v overflow, k v does not
+                                    (2.0 ** -100, 2.0 ** 100, 2.0 ** 27, 2.0 ** -20)])       # a state above bf16's largest value
+def test_wkv6_finite_extremes(scales, B, T):
+    """Steps whose own products stay in fp32's range give finite results."""
+    from gpt_neox_b200.ops.wkv import wkv6
+    torch.manual_seed(13)
+    H, N = 1, 64
+    r, k, v, gy = (torch.full((B, T, N), c, device="cuda").bfloat16() for c in scales)
+    if scales[2] > 1:
+        k[:, 2:], v[:, 0], v[:, 1] = 0, 1.9921875 * 2.0 ** 27, 1.5 * 2.0 ** 19        # the state: 1.998 * 2 ** 127
+    w, u = torch.full_like(r, -30.0), torch.zeros(H, N, device="cuda").bfloat16()
+    leaves = [t.requires_grad_() for t in (r, k, v, w, u)]
+    y = wkv6(*leaves)
+    gr, gk, gv, gw, gu = torch.autograd.grad(y, leaves, gy)
+    want = _wkv6_sweeps(*(t.detach() for t in (r, k, v, w, u)), gy)
+    for n, (a, b) in enumerate(zip((y, gr, gk, gv), want)):
+        assert b.isfinite().all()
+        assert (a.float() - b).abs().max() <= 2 ** -7 * b.abs().max(), n
