@@ -332,8 +332,13 @@ __global__ void __launch_bounds__(2 * N) wkv_kernel(const WkvParams p) {
 //
 // Four warps; the state is the accumulators of mma.m16n8k16 (warp w: 16 of its rows, a thread 32 values), fp32 throughout.
 // What is not a 16-bit input is split into three bf16 parts (24 bits: the products of parts of weight 2^-16 and above are
-// all formed; the rest is below fp32's last bit): the sums are those of fp32 arithmetic in another order.  These products
-// are far too small for tcgen05 (M = 16 rows of steps, operands made in registers between every two of them), hence mma.sync.
+// all formed; the rest is below fp32's last bit).  The tensor core cuts off what is below the last bit of a sum, always towards
+// zero, so a sum that lives long is not its accumulator: a block's products start from zero and are added to the state, and
+// to the sums over the state, by rounded additions.  Row sums of 512 steps, error against 64 bits over their norm, decays
+// of 1 - 6e-6 | the configured ones | 0.69: 3.4e-7 | 2.8e-7 | 8.3e-8; step by step 1.5e-6 | 1.6e-6 | 9.1e-8, with the
+// state as accumulator and the decays of the step-by-step kernel 2.5e-6 | 2.2e-6 | 1.3e-7.
+// These products are far too small for tcgen05 (M = 16 rows of steps, operands made in registers between every two of them),
+// hence mma.sync.
 // Infinity and what bf16 rounds to it have no parts, and a product of two vectors may leave fp32's range where the steps' own
 // products do not: a block with such an input or state is done step by step, with the results of the step-by-step kernel.
 // ------------------------------------------------------------------------------------------------
@@ -369,6 +374,20 @@ __device__ __forceinline__ void wm_mma(float (&c)[4], const uint32_t (&a)[4], ui
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// The same on top of zero.
+__device__ __forceinline__ void wm_mma0(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// y += A B, with the addition to y rounded (the tensor core drops what is below a sum's last bit).
+__device__ __forceinline__ void wm_add(float (&y)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  float d[4];
+  wm_mma0(d, a, b0, b1);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) y[e] += d[e];
+}
 // Four 8 x 8 matrices: (rows r0 .. r0 + 7 | r0 + 8 ..) x (columns c0 .. | c0 + 8 ..) of a 16-bit array.  Plain: registers 0, 1 =
 // the first rows' two column groups, 2, 3 = the second rows'; TRANS: each matrix transposed.
 template <bool TRANS>
@@ -383,6 +402,19 @@ __device__ __forceinline__ void wm_ld4(uint32_t (&r)[4], const uint16_t* base, i
   else
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+
+// exp(x) of x <= 0.  A weak decay stays in the state for many steps, so a bias of its approximation adds up (ex2.approx: an
+// error of 1e-6 after 500 steps); near zero the series, whose last addition rounds.
+__device__ __forceinline__ float2 wm_decay(float2 x) {
+  auto c2 = [](float c) { return make_float2(c, c); };
+  float2 p = ffma2(x, c2(1.f / 720), c2(1.f / 120));
+  p = ffma2(p, x, c2(1.f / 24));
+  p = ffma2(p, x, c2(1.f / 6));
+  p = ffma2(p, x, c2(0.5f));
+  p = ffma2(p, x, c2(1.f));
+  p = ffma2(p, x, c2(1.f));
+  return make_float2(x.x > -0.25f ? p.x : __expf(x.x), x.y > -0.25f ? p.y : __expf(x.y));
 }
 
 // An input block.
@@ -497,7 +529,7 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_col_kernel(const WkvParams 
 #pragma unroll
       for (int e = 0; e < 8; e += 2) {
         const float2 ew = live ? make_float2(-__expf(w8[e]), -__expf(w8[e + 1])) : make_float2(0.f, 0.f);
-        const float2 d = make_float2(__expf(ew.x), __expf(ew.y));
+        const float2 d = wm_decay(ew);
         d8[e] = d.x;
         d8[e + 1] = d.y;
         if (LOCAL) {
@@ -630,7 +662,7 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_col_kernel(const WkvParams 
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const int i = 8 * n + i0 + e;
-            const float b = h16_to_float(gb[o + i]), d = __expf(-__expf(h16_to_float(p.w[o + i])));
+            const float ew = -__expf(h16_to_float(p.w[o + i])), b = h16_to_float(gb[o + i]), d = wm_decay(make_float2(ew, ew)).x;
             if (!LOCAL) {
               const float a = h16_to_float(ga[o + i]);
               y0 += a * S[n][e];
@@ -660,7 +692,7 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_col_kernel(const WkvParams 
     wm_ld4<true>(cv, former.c.data(), 0, warp * 16, WP, false);
     if (!LOCAL) {
       float y[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-      float z[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};      // (two chains of dependent products)
+      float z[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};      // the products of lower parts
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
         uint32_t sp[3][4];               // S^T[16 j][16 i]
@@ -677,22 +709,32 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_col_kernel(const WkvParams 
           wm_ld4<false>(b, &former.ap[k][0][0], 0, 16 * ks, WP, false);
 #pragma unroll
           for (int m = 2 - k; m >= 0; --m) {
-            wm_mma(m & 1 ? z[0] : y[0], sp[m], b[0], b[1]);
-            wm_mma(m & 1 ? z[1] : y[1], sp[m], b[2], b[3]);
+            if (m + k == 0) {
+              wm_add(y[0], sp[m], b[0], b[1]);
+              wm_add(y[1], sp[m], b[2], b[3]);
+            } else {
+              wm_mma(z[0], sp[m], b[0], b[1]);
+              wm_mma(z[1], sp[m], b[2], b[3]);
+            }
           }
+        }
+      }
+#pragma unroll
+      for (int k = 2; k >= 0; --k) {
+        uint32_t b[4];
+        wm_ld4<false>(b, &former.A[k][0][0], 0, 0, 24, false);
+        if (k > 0) {
+          wm_mma(z[0], cv, b[0], b[1]);
+          wm_mma(z[1], cv, b[2], b[3]);
+        } else {
+          wm_add(y[0], cv, b[0], b[1]);
+          wm_add(y[1], cv, b[2], b[3]);
         }
       }
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         y[0][e] += z[0][e];
         y[1][e] += z[1][e];
-      }
-#pragma unroll
-      for (int k = 2; k >= 0; --k) {
-        uint32_t b[4];
-        wm_ld4<false>(b, &former.A[k][0][0], 0, 0, 24, false);
-        wm_mma(y[0], cv, b[0], b[1]);
-        wm_mma(y[1], cv, b[2], b[3]);
       }
 #pragma unroll
       for (int n = 0; n < 2; ++n)
@@ -703,19 +745,27 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_col_kernel(const WkvParams 
         }
     }
 #pragma unroll
-    for (int n = 0; n < 8; ++n) {
-      const float2 d = *reinterpret_cast<const float2*>(&former.tot[8 * n + i0]);
-      S[n][0] *= d.x; S[n][1] *= d.y; S[n][2] *= d.x; S[n][3] *= d.y;
-    }
-#pragma unroll
-    for (int n = 0; n < 8; n += 2)
+    for (int n = 0; n < 8; n += 2) {
+      float add[2][4];
 #pragma unroll
       for (int k = 2; k >= 0; --k) {
         uint32_t b[4];
         wm_ld4<true>(b, &former.bp[k][0][0], 0, 8 * n, WP, true);
-        wm_mma(S[n], cv, b[0], b[1]);
-        wm_mma(S[n + 1], cv, b[2], b[3]);
+        if (k == 2) {
+          wm_mma0(add[0], cv, b[0], b[1]);
+          wm_mma0(add[1], cv, b[2], b[3]);
+        } else {
+          wm_mma(add[0], cv, b[0], b[1]);
+          wm_mma(add[1], cv, b[2], b[3]);
+        }
       }
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        const float2 d = *reinterpret_cast<const float2*>(&former.tot[8 * (n + x) + i0]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S[n + x][e] = fmaf(S[n + x][e], e & 1 ? d.y : d.x, add[x][e]);
+      }
+    }
     }
     __syncthreads();
   }
@@ -822,7 +872,7 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_row_kernel(const WkvParams 
       for (int e = 0; e < 8; e += 2) {
         const float2 ew = live ? make_float2(-__expf(w8[e]), -__expf(w8[e + 1])) : make_float2(0.f, 0.f);
         *reinterpret_cast<float2*>(&now.ew[trow][ch8 + e]) = ew;
-        *reinterpret_cast<float2*>(&s.d[trow][ch8 + e]) = make_float2(__expf(ew.x), __expf(ew.y));
+        *reinterpret_cast<float2*>(&s.d[trow][ch8 + e]) = wm_decay(ew);
       }
     }
     }
@@ -843,7 +893,7 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_row_kernel(const WkvParams 
         uint32_t a[4], b[4];
         wm_ld4<false>(a, now.e.data(), 0, 16 * ks, WP, true);
         wm_ld4<false>(b, now.c.data(), 0, 16 * ks, WP, false);
-        wm_mma(m4, a, warp == 0 ? b[0] : b[2], warp == 0 ? b[1] : b[3]);
+        wm_add(m4, a, warp == 0 ? b[0] : b[2], warp == 0 ? b[1] : b[3]);
       }
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -857,7 +907,7 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_row_kernel(const WkvParams 
 #pragma unroll 1
       for (int x = 0; x < steps; ++x) {
         const float b0 = former.b.at(x, r0), b1 = former.b.at(x, r0 + 8);
-        const float2 d = make_float2(__expf(former.ew[x][r0]), __expf(former.ew[x][r0 + 8]));
+        const float2 d = wm_decay(make_float2(former.ew[x][r0], former.ew[x][r0 + 8]));
         float y0 = 0.f, y1 = 0.f, st = 0.f;
 #pragma unroll
         for (int n = 0; n < 8; ++n)
@@ -890,6 +940,7 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_row_kernel(const WkvParams 
     // ---- products
     {
       float y[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      float z[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};      // the products of lower parts
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
         uint32_t sp[3][4];               // S[16 i][16 j]
@@ -903,20 +954,18 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_row_kernel(const WkvParams 
         uint32_t b[4];
         wm_ld4<false>(b, former.e.data(), 0, 16 * ks, WP, false);
 #pragma unroll
-        for (int m = 2; m >= 0; --m) {
-          wm_mma(y[0], sp[m], b[0], b[1]);
-          wm_mma(y[1], sp[m], b[2], b[3]);
+        for (int m = 2; m > 0; --m) {
+          wm_mma(z[0], sp[m], b[0], b[1]);
+          wm_mma(z[1], sp[m], b[2], b[3]);
         }
+        wm_add(y[0], sp[0], b[0], b[1]);
+        wm_add(y[1], sp[0], b[2], b[3]);
       }
 #pragma unroll
       for (int n = 0; n < 2; ++n)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) s.inter[8 * n + n0 + (e & 1)][r0 + (e >> 1) * 8] = y[n][e];
+        for (int e = 0; e < 4; ++e) s.inter[8 * n + n0 + (e & 1)][r0 + (e >> 1) * 8] = y[n][e] + z[n][e];
       const float t0 = former.tot[r0], t1 = former.tot[r0 + 8];
-#pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        S[n][0] *= t0; S[n][1] *= t0; S[n][2] *= t1; S[n][3] *= t1;
-      }
       uint32_t bt[3][4];                 // (b Suf)^T: 16 rows i x 16 steps
 #pragma unroll
       for (int k = 0; k < 3; ++k) wm_ld4<true>(bt[k], &former.bp[k][0][0], 0, warp * 16, WP, false);
@@ -924,11 +973,18 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_row_kernel(const WkvParams 
       for (int n = 0; n < 8; n += 2) {
         uint32_t b[4];
         wm_ld4<true>(b, former.c.data(), 0, 8 * n, WP, true);
+        float add[2][4];
+        wm_mma0(add[0], bt[2], b[0], b[1]);
+        wm_mma0(add[1], bt[2], b[2], b[3]);
 #pragma unroll
-        for (int k = 2; k >= 0; --k) {
-          wm_mma(S[n], bt[k], b[0], b[1]);
-          wm_mma(S[n + 1], bt[k], b[2], b[3]);
+        for (int k = 1; k >= 0; --k) {
+          wm_mma(add[0], bt[k], b[0], b[1]);
+          wm_mma(add[1], bt[k], b[2], b[3]);
         }
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) S[n + x][e] = fmaf(S[n + x][e], e < 2 ? t0 : t1, add[x][e]);
       }
     }
     }

@@ -185,6 +185,35 @@ def test_wkv6_passes_nan_and_inf_on(what, value, at):
     assert got.isfinite().all() == want.isfinite().all()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,T,H", [(32, 512, 12), (8, 2048, 16)])        # chunks of 512 and of 688 steps
+@pytest.mark.parametrize("w", [-12.0, -6.0, -1.0])
+def test_wkv6_row_sums_have_fp32_precision(B, T, H, w):
+    """The gradient of r before it is rounded, which the decay gradient is made of: an error of a last bit per step that adds
+    up like noise, and no drift that grows with the steps."""
+    from gpt_neox_b200.ops import _lib
+    torch.manual_seed(15)
+    N, C = 64, H * 64
+    r, k, v, gy = ((torch.randn(B, T, C, device="cuda") * 0.5).bfloat16() for _ in range(4))
+    w = (torch.randn(B, T, C, device="cuda") * 0.5 + w).bfloat16()
+    u = torch.randn(H, N, device="cuda") * 0.3
+    lib, P = _lib.lib(r), _lib.ptr
+    nc = lib.nx_wkv6_chunks(B, T, H)
+    f32 = lambda *s: torch.empty(s, device="cuda")
+    local, start, rstart, sumew = f32(B, H, nc, N, N), f32(B, H, nc, N, N), f32(B, H, nc, N, N), f32(B, H, nc, N)
+    y, gr, gk, gv, gw = (torch.empty_like(r) for _ in range(5))
+    gr32, gu, gu_part = f32(B, T, C), f32(H, N), f32(B, nc, H, N)
+    lay = (r.stride(0), r.stride(1))
+    _lib.check(lib.nx_wkv6_fwd(P(r), P(k), P(v), P(w), *lay, P(u), P(y), *lay, P(local), P(start), P(sumew), B, T, H, N,
+                               _lib.stream()), "nx_wkv6_fwd")
+    _lib.check(lib.nx_wkv6_bwd(P(r), P(k), P(v), P(w), P(gy), *lay, P(u), P(gr), P(gk), P(gv), P(gw), P(gr32), P(gu), P(gu_part),
+                               *lay, P(local), P(start), P(rstart), P(sumew), B, T, H, N, _lib.stream()), "nx_wkv6_bwd")
+    part = [t[:1, :, :2 * N].double() for t in (r, k, v, w)]
+    want = _wkv6_sweeps(*part, u[:2].double(), gy[:1, :, :2 * N].double())[1]
+    err = gr32[:1, :, :2 * N].double() - want
+    assert err.norm() <= 2 ** -24 * (min(T, 700) ** 0.5 / 2 + 1) * want.norm()
+
+
 def _wkv6_sweeps(r, k, v, w, u, gy):
     """y and the gradients of r, k, v, w, u as two sweeps form them, one step after the other, in fp32 (64 bits for 64-bit inputs)."""
     B, T, _ = r.shape
