@@ -163,8 +163,14 @@ def test_wkv6_blocks_of_steps(B, T, H, w, dtype):
         # (fp16: results below 2^-14 are subnormal, rounded to 2^-25)
         lim = eps * b.norm() + (2 ** -20 * b.abs().max() + 2 ** -25) * b.numel() ** 0.5
         if n == 4:
-            # the decay gradient is ew times a running difference of r gr and k gk: T terms of fp32 precision, which cancel
-            lim += T * 2 ** -20 * (ref[0].abs().max() * want[1].abs().max()) * ref[3].exp().max() * b.numel() ** 0.5
+            # The decay gradient is ew times a running difference of r gr and k gk, which cancel: what fp32 leaves of it is a
+            # last bit of the sizes of all terms behind a step.  (Plain fp32 sums stay below 0.1 of that; at w = 6, where the
+            # gradient itself is 0, it is the whole bound.)
+            size = _wkv6_sweeps(*(t.detach().abs() for t in leaves[:3]), leaves[3].detach(), leaves[4].detach().abs(), gy.abs())
+            terms = leaves[0].detach().abs() * size[1] + leaves[1].detach().abs() * size[2]
+            fp32 = 2 ** -24 * (ref[3].detach().exp() * terms.double().flip(1).cumsum(1).flip(1)).norm()
+            assert fp32 <= (0.05 * b.norm() if w < 6 else 5e-2 * b.numel() ** 0.5)
+            lim = eps * b.norm() + 2 ** -25 * b.numel() ** 0.5 + fp32
         assert (a.double() - b).norm() <= lim, n
 
 
@@ -183,6 +189,35 @@ def test_wkv6_passes_nan_and_inf_on(what, value, at):
     got, want = wkv6(*ts, u), wkv6_reference(*(t.float() for t in ts), u.float())
     assert torch.equal(got.isfinite(), want.isfinite())
     assert got.isfinite().all() == want.isfinite().all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,T,H", [(32, 512, 12), (8, 2048, 16)])        # chunks of 512 and of 688 steps
+@pytest.mark.parametrize("w", [-12.0, -1.0])
+def test_wkv6_long_sweeps(B, T, H, w, dtype):
+    """Many blocks of steps in one CTA, with decays that keep the state and that forget it, against 64 bits: all results, and the
+    steps at the far ends of both sweeps, where what every block leaves out would have added up."""
+    from gpt_neox_b200.ops.wkv import wkv6
+    torch.manual_seed(14)
+    N, n = 64, 2                                   # (sequences and heads that are checked)
+    mk = lambda m=0.0: (torch.randn(B, T, H * N, device="cuda") * 0.5 + m).to(dtype)
+    leaves = [t.requires_grad_() for t in (mk(), mk(), mk(), mk(w), (torch.randn(H, N, device="cuda") * 0.3).to(dtype))]
+    gy = mk()
+    y = wkv6(*leaves)
+    got = (y.detach(),) + torch.autograd.grad(y, leaves, gy)
+    part = [t.detach()[:n, :, :n * N].double() for t in leaves[:4]] + [leaves[4].detach()[:n].double(), gy[:n, :, :n * N].double()]
+    want = _wkv6_sweeps(*part)
+    size = _wkv6_sweeps(*(t if i == 3 else t.abs() for i, t in enumerate(part)))
+    terms = part[0].abs() * size[1] + part[1].abs() * size[2]
+    size = (*size[:4], part[3].exp() * terms.flip(1).cumsum(1).flip(1))
+    eps = 2 ** -9 if dtype == torch.bfloat16 else 2 ** -12
+    for i, (a, b, c) in enumerate(zip(got, want, size)):
+        a = a[:n, :, :n * N].double()
+        for t in (slice(None), slice(0, 16), slice(T - 16, T)):
+            # one rounding; in front of it fp32, and the decays' own error times the steps that remember it
+            lim = eps * b[:, t].norm() + 2 ** -24 * c[:, t].norm() + 2 ** -25 * b[:, t].numel() ** 0.5
+            assert (a[:, t] - b[:, t]).norm() <= lim, (i, t)
 
 
 @pytest.mark.gpu
