@@ -531,9 +531,7 @@ def test_flash_attention_backward_routes(b, s, h, hk, form, d):
         assert (x.float() - y).norm() <= 3 * eps * y.norm() + 1e-6
 
 
-@pytest.mark.parametrize("env", [{"NEOX_ATTN_FWD_SHAPE": "1"}, {"NEOX_ATTN_FWD_SHAPE": "3"},
-                                 {"NEOX_ATTN_BWD_WARPS": "4"}, {"NEOX_ATTN_DKV_PIPE": "0", "NEOX_ATTN_DQ_PIPE": "0"}],
-                         ids=["fwd_shape1", "fwd_shape3", "bwd_4warps", "bwd_unpipelined"])
+@pytest.mark.parametrize("env", [{"NEOX_ATTN_FWD_SHAPE": "1"}, {"NEOX_ATTN_FWD_SHAPE": "3"}], ids=["fwd_shape1", "fwd_shape3"])
 def test_flash_attention_selectable_kernel_shapes(env):
     """The kernel shapes that an environment variable selects instead of the defaults (read once per process, hence a
     child process): the dense, dropout and block-sparse cases of this file under each of them."""
@@ -543,7 +541,7 @@ def test_flash_attention_selectable_kernel_shapes(env):
     if "_dtype" in globals() and DT != torch.bfloat16:
         pytest.skip("one operand type is enough for the shape selection")
     cmd = [sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", os.path.abspath(__file__), "-k",
-           "(test_flash_attention or test_block_sparse_flash_attention) and not selectable and not varlen"]
+           "(test_flash_attention or test_block_sparse_flash_attention) and not selectable and not varlen and not backward"]
     r = subprocess.run(cmd, capture_output=True, text=True, timeout=900, env=dict(os.environ, **env))
     assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]
     assert " passed" in r.stdout
