@@ -25,16 +25,17 @@
 // buffers is all that the accumulators leave).  Hence everything that lets blocks overlap: issuers apart from each other (one
 // thread issuing all was the bound at 1,700 cycles per 64 rows), scores two blocks ahead, score buffers given back as soon as
 // they are in registers, the next item's tiles and stores in the shadow of the running one.
-// Batch 4, 32 heads, 2048 x 128 causal: dQ 293 -> 197 us, dK / dV 330 -> 290 us; 5003 tokens, 32 heads on 8, window of 4096:
-// 331 -> 232 us and 438 -> 322 us (before: a CTA per item, one issuing thread, all eight element-wise warps on the same 64
-// columns).  What was slower: two groups of four warps that write their results over their scores (260 / 333 us), dQ by 16
-// warps with 32 columns each (215 us), dQ with two K stages (258 us), one V stage (212 us).
+// Batch 4, 32 heads, 2048 x 128 causal: dQ 290 -> 202 us, dK / dV 324 -> 293 us; 5003 tokens, 32 heads on 8, window of 4096:
+// 326 -> 238 us and 435 -> 325 us (before: one CTA per tile).  What was slower: two groups of four warps that write their
+// results over their scores (260 / 333 us), dQ by 16 warps with 32 columns each (215 us), dQ with two K stages (258 us), one V
+// stage (212 us).
 #include "attention_bwd.h"
 #include "ptx.cuh"
 #include "reduce.cuh"
 
 namespace nx {
 
+constexpr int ABS = 64;     // query rows per block of the dK / dV kernel
 constexpr int DQ_THREADS = 32 * 12, DKV_THREADS = 32 * 20;
 
 // delta = rowsum(O * dO), 0 in the padding rows [Sq, Sq_pad).  A group of LPR lanes (D / 8 rounded up to a power of two)
@@ -923,23 +924,28 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
 }
 
 static bool bwd_map(CUtensorMap* m, const void* base, int B, int Hh, int S, int D, long long sb,
-                    long long sh, long long ss) {
+                    long long sh, long long ss, int rows) {
   const uint64_t dims[4] = {(uint64_t)D, (uint64_t)S, (uint64_t)Hh, (uint64_t)B};
   const uint64_t strides[3] = {(uint64_t)ss * 2, (uint64_t)sh * 2, (uint64_t)sb * 2};
-  const uint32_t box[4] = {64, ABS, 1, 1};
+  const uint32_t box[4] = {64, (uint32_t)rows, 1, 1};
   return make_tma_4d(m, base, dims, strides, box, 2, true);
 }
 
 // Which kernels a call takes: persistent ones or one CTA per tile (attention_bwd_tile.cu).  Persistent CTAs overlap one item
 // with the next, so they need more items than SMs; a single item costs them 1 - 4 us more (more roles, barriers and
-// threads to set up).  Measured over 64 .. 2048 tokens x 4 .. 256 heads, time per tile / persistent:
-//   dropout     0.5 (registers spill);  block-sparse layouts 0.7 - 1 (a CTA's share is fixed, and tiles are of any length)
-//   dQ, ALiBi   0.96 - 2.7: always persistent
-//   dQ, 128     more items than SMs 1.13 - 1.66; fewer, 256 keys and more 0.98 - 1.15, fewer keys 0.86 - 1.17
-//   dQ, 64      causal, more items than SMs and more than one key block 1.02 - 1.63, one block 0.92 - 0.97; not causal 0.88 - 1.02
-//               up to 512 items, 1.08 - 1.18 from 768 on (blocks are short, the SMs' last round counts); fewer items 0.77 - 1.01
-//   dK / dV     more items than SMs: 128 1.0 - 1.38; 64, causal from 384 queries on (ALiBi 200) 0.98 - 1.40, below 0.86 - 1.0,
-//               not causal 0.8 - 1.0; fewer items than SMs 0.66 - 1.05
+// threads to set up).  Measured over 64 .. 2048 tokens x 4 .. 1536 heads, time per tile / persistent:
+//   dropout      0.5 (registers spill);  block-sparse layouts 0.7 - 1 (a CTA's share is fixed, and tiles are of any length)
+//   dQ, ALiBi    0.93 - 2.7: always persistent
+//   dQ, 128      more items than SMs 1.13 - 1.66; fewer, 256 keys and more 0.98 - 1.15, fewer keys 0.86 - 1.17
+//   dQ, 64       causal, more items than SMs 1.01 - 1.63; rows of 65 .. 128 keys 0.98 below 2 items per SM, 1.05 - 1.19 above,
+//                of 64 keys 0.91 - 0.98 and 1.05 from 9 on; not causal 0.88 - 1.02 up to 4 items per SM, then 0.97 - 1.25
+//   dK / dV, 128 more items than SMs 0.95 - 1.38; fewer 0.76 - 1.03 up to 2048 queries, with more 0.98 - 1.16 (blocks of 64
+//                queries waste less of a ragged end than tiles of 128)
+//   dK / dV, 64  fewer items than SMs 0.64 - 1.05; more:
+//                ALiBi from 256 queries on 0.96 - 1.4, fewer queries with up to 5 items per SM 0.89 - 1.1, with more 0.99 - 1.3;
+//                causal 384 .. 1535 queries 0.98 - 1.17, fewer 0.86 - 1.0 and 0.99 - 1.24, 2048 queries 1.0 - 1.08 and 0.93 - 0.96;
+//                not causal up to 512 queries 0.83 - 1.0 below 9 items per SM, 1.04 - 1.24 above, longer 0.8 - 0.98
+//                (queries times the query heads of a key head)
 struct BwdRoute {
   long long dq_items, dkv_items;
   bool dq, dkv;      // persistent
@@ -954,8 +960,14 @@ static BwdRoute attn_bwd_route(const AttnBwdParams& p) {
   const int sms = sm_count();
   if (alibi) r.dq = true;
   else if (p.D > 64) r.dq = r.dq_items > sms || p.Sk >= 256;
-  else r.dq = p.causal ? r.dq_items > sms && p.Sk > AB : r.dq_items > 4 * sms;
-  r.dkv = r.dkv_items > sms && (p.D > 64 || (p.causal && p.Sq >= (alibi ? 200 : 384)));
+  else r.dq = r.dq_items > (!p.causal ? 4 : p.Sk > AB ? 1 : p.Sk > ABS ? 2 : 9) * sms;
+  const bool many = r.dkv_items > 5 * sms;
+  const long long rows = static_cast<long long>(p.Sq) * (p.H / p.Hk);      // an item's queries
+  if (p.D > 64) r.dkv = r.dkv_items > sms || rows > 2048;
+  else if (r.dkv_items <= sms) r.dkv = false;
+  else if (alibi) r.dkv = rows >= 256 || many;
+  else if (p.causal) r.dkv = rows < 384 ? many : rows < 2048 || !many;
+  else r.dkv = rows <= 512 && r.dkv_items > 9 * sms;
   return r;
 }
 
@@ -968,12 +980,12 @@ static int persistent_launch(K kern, int threads, long long items, const BwdMaps
 }
 
 template <int DP, bool ALIBI>
-static int launch_bwd(const BwdMaps& m, const AttnBwdParams& p, const BwdRoute& r, cudaStream_t s) {
-  const int rc = r.dq ? persistent_launch<BwdSmem<DP>>(attn_bwd_dq_kernel<DP, ALIBI>, DQ_THREADS, r.dq_items, m, p, s)
-                      : attn_bwd_tile_dq(m, p, s);
+static int launch_bwd(const BwdMaps (&m)[2], const AttnBwdParams& p, const BwdRoute& r, cudaStream_t s) {
+  const int rc = r.dq ? persistent_launch<BwdSmem<DP>>(attn_bwd_dq_kernel<DP, ALIBI>, DQ_THREADS, r.dq_items, m[0], p, s)
+                      : attn_bwd_tile_dq(m[1], p, s);
   if (rc != NX_OK) return rc;
-  return r.dkv ? persistent_launch<BwdSmem<DP>>(attn_bwd_dkv_kernel<DP, ALIBI>, DKV_THREADS, r.dkv_items, m, p, s)
-               : attn_bwd_tile_dkv(m, p, s);
+  return r.dkv ? persistent_launch<BwdSmem<DP>>(attn_bwd_dkv_kernel<DP, ALIBI>, DKV_THREADS, r.dkv_items, m[0], p, s)
+               : attn_bwd_tile_dkv(m[1], p, s);
 }
 
 }  // namespace nx
@@ -1021,10 +1033,6 @@ NX_API int NX_SYM(nx_flash_attn_bwd)(const void* q, const void* k, const void* v
     else run(attn_delta_kernel<16>, 16 * DELTA_ROWS);
     NX_LAUNCH_CHECK();
   }
-  BwdMaps m;
-  if (!bwd_map(&m.q, q, B, H, Sq, D, q_sb, q_sh, q_ss) || !bwd_map(&m.k, k, B, Hk, Sk, D, k_sb, k_sh, k_ss) ||
-      !bwd_map(&m.v, v, B, Hk, Sk, D, v_sb, v_sh, v_ss) || !bwd_map(&m.d_o, dO, B, H, Sq, D, do_sb, do_sh, do_ss))
-    return NX_ERR_ARG;
   AttnBwdParams p;
   p.lse = (const float*)lse; p.delta = (const float*)delta; p.alibi = (const float*)alibi;
   p.dq = (h16*)dq; p.dk = (h16*)dk; p.dv = (h16*)dv;
@@ -1046,6 +1054,15 @@ NX_API int NX_SYM(nx_flash_attn_bwd)(const void* q, const void* k, const void* v
   p.blk_nkt = (Sk + AB - 1) / AB;
   p.blk_shift = blk_size == 16 ? 4 : blk_size == 32 ? 5 : blk_size == 64 ? 6 : 7;
   const BwdRoute route = attn_bwd_route(p);
+  BwdMaps m[2];      // for persistent kernels and for one CTA per tile
+  for (int t = 0; t < 2; ++t) {
+    if (t == 0 ? !route.dq && !route.dkv : route.dq && route.dkv) continue;
+    const int rows = t == 0 ? ABS : AB;
+    if (!bwd_map(&m[t].q, q, B, H, Sq, D, q_sb, q_sh, q_ss, rows) || !bwd_map(&m[t].k, k, B, Hk, Sk, D, k_sb, k_sh, k_ss, rows) ||
+        !bwd_map(&m[t].v, v, B, Hk, Sk, D, v_sb, v_sh, v_ss, rows) ||
+        !bwd_map(&m[t].d_o, dO, B, H, Sq, D, do_sb, do_sh, do_ss, rows))
+      return NX_ERR_ARG;
+  }
   NX_REQUIRE(route.dq_items < (1ll << 30) && route.dkv_items < (1ll << 30), "flash_attn_bwd: too many tiles");
   if (alibi != nullptr) return D <= 64 ? launch_bwd<64, true>(m, p, route, s) : launch_bwd<128, true>(m, p, route, s);
   return D <= 64 ? launch_bwd<64, false>(m, p, route, s) : launch_bwd<128, false>(m, p, route, s);

@@ -7,7 +7,6 @@
 namespace nx {
 
 constexpr int AB = 128;     // rows per resident tile
-constexpr int ABS = 64;     // rows per box of the tensor maps
 constexpr float LOG2E = 1.4426950408889634f;
 
 struct AttnBwdParams {
@@ -32,7 +31,7 @@ struct AttnBwdParams {
 };
 
 struct BwdMaps {
-  CUtensorMap q, k, v, d_o;      // boxes of ABS rows x 64 columns, swizzled
+  CUtensorMap q, k, v, d_o;      // swizzled boxes of 64 columns and 64 rows, or 128 for the kernels of one CTA per tile
 };
 
 // Kernels of one CTA per tile: dQ (dropout, block-sparse layouts and scale 0 included), dK / dV.

@@ -27,13 +27,11 @@ struct TileSmem {
   static constexpr int DYN = TOTAL + 1024;
 };
 
-// Loads one [128 x DP] tile (rows contiguous in d) as swizzled boxes of ABS rows x 64 columns.
+// Loads one [128 x DP] tile (rows contiguous in d) as swizzled boxes of 128 rows x 64 columns.
 template <int DP>
 __device__ __forceinline__ void tile_load(uint32_t dst, const CUtensorMap* m, uint32_t bar, int row0, int head, int batch) {
 #pragma unroll
-  for (int c = 0; c < DP / 64; ++c)
-#pragma unroll
-    for (int r = 0; r < AB; r += ABS) tma_load_4d(dst + c * (AB * 128) + r * 128, m, bar, c * 64, row0 + r, head, batch);
+  for (int c = 0; c < DP / 64; ++c) tma_load_4d(dst + c * (AB * 128), m, bar, c * 64, row0, head, batch);
 }
 // D[128 x 64] = A[128 x DP] * B[64 x DP]^T, both K-major (head dim contiguous); b points at the first of the 64 rows of a
 // 128-row tile.
