@@ -20,10 +20,9 @@
 //              Q_t[i] = sum_j G_t[i][j] S_t[i][j] one has Q_{t-1} - Q_t = r_t gr_t - k_t gk_t and
 //              dL/d(ew_t) = Q_t - k_t (gk_t - r_t u s_t),  s_t = <gy_t, v_t>,  ew = -exp(w)
 // Step by step the shared-memory loads and exchanges of the steps are the bound (32 x 512 tokens, 12 heads of 64, forward +
-// backward 788 us).  With the products of a block in their place 581 us, and 570 with a block's vectors beside the former
-// block's products (125 us for each sweep, 175 for gk with the decay gradient).  No pipe is the bound then but latency, at 2.6
-// warps per scheduler: issue slots 46 / 43 / 38 % busy (column sums, row sums, gk with the decay gradient), tensor pipe
-// 25 / 16 / 11 %.
+// backward 788 us).  With the products of a block in their place, and a block's vectors beside the former block's products, 570
+// (134 us for column sums, 123 for row sums, 159 for gk with the decay gradient).  No pipe is the bound then but latency, at 2.6
+// warps per scheduler: issue slots 48 / 51 / 47 % busy, tensor pipe 23 / 16 / 12 %.
 //
 // The sequence is cut into chunks only when batch x heads leaves the chip idle (wkv_chunk_count): the recurrence is
 // linear, so a chunk's end state is  P (.) S_start + S_local  with P[i] = prod_t d_t[i]; local passes start every chunk
@@ -1111,8 +1110,11 @@ static int wkv_launch(const WkvParams& p, bool vec, int chunks, cudaStream_t str
 }
 
 // Chunks the sequence is cut into.  The sweeps are bound by latency until an SM holds WK_CTAS CTAs, so time goes with the
-// chunk length times the number of rounds the CTAs take; more than one chunk adds the local pass (2 of the sweep's 3
-// operations) over all chunks but one, and the fold.  The count depends on the batch, and the chunks' states are folded in
+// chunk length times the number of rounds the CTAs take; more than one chunk adds the local passes over all chunks but one, and
+// the fold.  The weights come from the step-by-step sweeps; in blocks, every count from 1 to 32 tried, the rule's is the best or
+// within 10 % of it for 1 - 64 sequences of 50 - 8192 steps (1 x 512, 12 heads: 32 chunks 83 us, 16 76; 4 x 2048 9 chunks 364, 4
+// 570; 8 x 2048, 16 heads 3 chunks 920, 10 909; 32 x 512, 12 heads 1 chunk 556, 2 674) but for 40 x 512, 12 heads, whose CTAs just
+// exceed a round: 8 chunks 1010, 1 887.  The count depends on the batch, and the chunks' states are folded in
 // fp32: a sequence's last bits are not those it has in another batch.
 constexpr int WK_CTAS = 3;
 static int wkv_chunk_count(int B, int T, int H) {
