@@ -6,9 +6,9 @@
 //
 // Warp 0 loads (TMA), one thread of warp 1 issues the MMAs, eight element-wise warps take 32 columns of each half of a block.
 // Against the persistent kernels a CTA pays its prologue, pipeline fill and stores alone, but its threads have twice the
-// registers (dropout there spilled 500 bytes: batch 4, 32 heads, 2048 x 128 causal with dropout 1826 us for the whole
-// backward, 956 here), the hardware hands the tiles out as SMs become free (block-sparse tiles are of any length: 1 x 8192, 8
-// heads of 128, 746 us persistent, 506 here), and starting takes less (12 heads of 64, 8 x 128 tokens: 19.6 us, 16.3 here).
+// registers (dropout there spilled 500 bytes: batch 4, 32 heads, 2048 x 128 causal with dropout 1833 us for the whole
+// backward, 953 here), the hardware hands the tiles out as SMs become free (block-sparse tiles are of any length: 1 x 8192, 8
+// heads of 128, 731 us persistent, 499 here), and starting takes less (12 heads of 64, 8 x 128 tokens: 19.5 us, 16.3 here).
 // Counterpart of the flash-attn 2 backward the reference calls through autograd (megatron/model/transformer.py:573-690).
 #include "attention_bwd.h"
 #include "ptx.cuh"
