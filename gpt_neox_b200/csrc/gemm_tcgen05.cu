@@ -180,11 +180,11 @@ __device__ __forceinline__ void epi_put(uint8_t* box, int lane, const float (&v)
 }
 
 // TMA_EPI (grouped rows with more than 128 columns): a warp's 32 x 32 pieces of the result and of the stored derivative
-// leave through shared memory as TMA boxes, and a stored derivative comes in the same way, one piece ahead.  The GEMMs of a
+// leave through shared memory as TMA boxes, and a stored derivative comes in the same way, behind the piece before.  The GEMMs of a
 // short reduction are bound by their epilogue warps, which are bound by latency: what counts is that the 32 values of a lane
 // go through GeLU and derivative side by side, so the activation is chosen once per piece (chosen per value, the values' chains ran
 // one after the other: 3,400 cycles per piece).  Dropless MoE, 32,768 rows, 768 -> 3072: the GEMM with GeLU and derivative
-// 275 -> 179 us, the one that multiplies by the derivative 275 -> 151 us; with the chains one after the other 216 / 203, with
+// 275 -> 176 us, the one that multiplies by the derivative 275 -> 156 us; with the chains one after the other 216 / 203, with
 // pieces transposed in registers instead of boxes 184 / 168; without any epilogue work 110.
 template <int BN, int STAGES, bool A_MN, bool B_MN, bool TMA_EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
@@ -399,6 +399,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+        bool next_here = false;
         if (aux_in) {
           if (!fetched) fetch_aux(tm, tn, c);
           ok = mbar_wait(aux_bar, aux_phase, p.err, 9);
@@ -413,15 +414,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             const uint4 u = *reinterpret_cast<const uint4*>(aux_box + epi_chunk(lane, k));
             x[4 * k] = u.x; x[4 * k + 1] = u.y; x[4 * k + 2] = u.z; x[4 * k + 3] = u.w;
           }
-          // The next piece comes in over this one: every lane's fence orders its loads before the copy, which belongs to another
-          // proxy, and the barrier hands that order to the lane that issues it.  (The barrier alone orders ordinary
-          // accesses; the copy then overtook loads that were still queued, and 1 % of a gradient was wrong.)
-          fence_proxy_async_smem();
-          __syncwarp();
           // the next piece: of this tile, or the first of the next
           const bool here = c + 1 < c_end && col0 + 32 < p.N;
           fetched = here || (tile_nx < num_tiles && tn_nx * BN + c_begin * 32 < p.N);
-          if (fetched) fetch_aux(here ? tm : tm_nx, here ? tn : tn_nx, here ? c + 1 : c_begin);
+          next_here = here;
           auto times = [&](auto f) {
 #pragma unroll
             for (int k = 0; k < 16; ++k) {
@@ -479,6 +475,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         epi_put(out_box, lane, v);
         fence_proxy_async_smem();
         __syncwarp();
+        // The side operand's next piece comes in over this one: the results made of this one are laid down, and the fence above
+        // orders the loads, too, before the copy, which belongs to another proxy.  (A barrier alone, of the warp or an mbarrier
+        // that every lane arrives on, orders ordinary accesses; a copy behind one overtook loads that were still queued behind
+        // the other warps', and 1 % of a gradient was wrong.)
+        if (aux_in && fetched) fetch_aux(next_here ? tm : tm_nx, next_here ? tn : tn_nx, next_here ? c + 1 : c_begin);
         if (lane == 0) {
           tma_store_2d(&em.out, smem_u32(out_box), col0, m0 + quad * 32);
           tma_store_commit();
