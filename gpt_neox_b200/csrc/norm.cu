@@ -512,7 +512,11 @@ norm_bwd_ring_kernel(const h16* __restrict__ dy1, const h16* __restrict__ dy2, c
         s2 += w[j];
       }
     }
-    const float2 r = block_sum2(s1, s2, sh);   // every thread has read its part of the stage once this returns
+    // Every thread has read its part of the stage once the sum returns.  What the sum is made of has arrived by then; what is
+    // only kept (the gradient of the residual stream) may still be queued, and the next copy into the stage, which belongs to
+    // another proxy, does not wait for it without a fence.
+    if (dx_in != nullptr) fence_proxy_async_smem();
+    const float2 r = block_sum2(s1, s2, sh);
     if (threadIdx.x == 0) {
       const long long nr = row + static_cast<long long>(nst) * gridDim.x;
       if (nr < rows) fill(st, nr);

@@ -97,6 +97,28 @@ def test_dual_layernorm_with_residual_carry_one_backward_pass(rows, H):
         assert rel(bs[i].grad, br[i].grad) < 2e-2
 
 
+@pytest.mark.parametrize("rows,H", [(20000, 2048), (4096, 4096)])
+def test_norm_gradients_with_residual_carry_repeat_bit_for_bit(rows, H):
+    """Rows follow each other through one ring of shared memory; the residual stream's gradient is the value of a row that is
+    only used after the next row may have been asked for."""
+    from gpt_neox_b200.ops.norm import dual_layer_norm
+    torch.manual_seed(31)
+    x, ws = bf(rows, H, grad=True), [bf(H, grad=True) for _ in range(4)]
+    gs = [bf(rows, H) for _ in range(3)]
+    run = lambda: torch.autograd.grad(dual_layer_norm(x, *ws, carry=True), [x, *ws], gs)
+    first = run()
+    r = [t.detach().double().requires_grad_() for t in (x, *ws)]
+    ys = [r[0]] + [F.layer_norm(r[0], (H,), r[i], r[i + 1], 1e-5) for i in (1, 3)]
+    (want,) = torch.autograd.grad(ys, r[:1], [t.double() for t in gs])
+    # a sum of three gradients in fp32, rounded once: half a unit in the last of 8 bits (11) is up to 2^-8 (2^-11) of the value
+    eps = 2 ** -8 if DT == torch.bfloat16 else 2 ** -11
+    err = (first[0] - want).abs()
+    assert (err <= 1.01 * eps * want.abs() + 1e-5 * want.abs().max()).all()
+    for _ in range(20):
+        assert all(torch.equal(a, b) for a, b in zip(first, run()))
+
+
+
 def test_rmsnorm_carry_adds_residual_gradient():
     from gpt_neox_b200.ops.norm import rms_norm
     torch.manual_seed(5)
