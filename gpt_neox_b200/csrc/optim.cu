@@ -11,6 +11,8 @@
 #include "ptx.cuh"
 #include "reduce.cuh"
 
+#include <type_traits>
+
 namespace nx {
 
 struct AdamArgs {
@@ -18,17 +20,17 @@ struct AdamArgs {
   int adam_w_mode;  // 1 = decoupled weight decay (AdamW), 0 = L2 added to the gradient
 };
 
+// four gradients as they lie in memory, and as floats
 template <typename G>
-__device__ __forceinline__ float4 load_grad4(const G* g, long long i);
-template <>
-__device__ __forceinline__ float4 load_grad4<float>(const float* g, long long i) {
-  return *reinterpret_cast<const float4*>(g + i);
-}
-template <>
-__device__ __forceinline__ float4 load_grad4<h16>(const h16* g, long long i) {
-  const uint2 u = *reinterpret_cast<const uint2*>(g + i);
+using Grad4 = std::conditional_t<sizeof(G) == 4, float4, uint2>;
+__device__ __forceinline__ float4 grad4(const float4& v) { return v; }
+__device__ __forceinline__ float4 grad4(const uint2& u) {
   const float2 a = unpack_h16x2(u.x), b = unpack_h16x2(u.y);
   return make_float4(a.x, a.y, b.x, b.y);
+}
+template <typename G>
+__device__ __forceinline__ float4 load_grad4(const G* g, long long i) {
+  return grad4(*reinterpret_cast<const Grad4<G>*>(g + i));
 }
 
 template <typename G>
@@ -193,16 +195,31 @@ __global__ void __launch_bounds__(256) adam8_kernel(float* __restrict__ p, uint8
 // clip coefficient multiplies every gradient, so a last bit of the norm reaches the whole state: with block sums that met
 // in atomic adds, in the order in which blocks ended, two runs differed by a step of single 16-bit weights.)
 constexpr int SUMSQ_BLOCKS_PER_SM = 8, FOLD_THREADS = 256;
+__device__ __forceinline__ void add_squares(float& s, const float4& v) {
+  s += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+}
+// Bound by memory latency times the loads in flight: 64 bytes a thread are asked for before the first is used.  The squares
+// are added in the order in which a loop of single loads adds them, so the sum's bits do not depend on how many are in flight.
+// 176.8 M 16-bit values: 164 us with one load in flight (2.2 TB/s), 70 us now (5.1 TB/s of 6.54 measured).
 template <typename G>
-__global__ void sumsq_kernel(const G* __restrict__ x, long long n, float2* __restrict__ part) {
+__global__ void __launch_bounds__(256, SUMSQ_BLOCKS_PER_SM)
+sumsq_kernel(const G* __restrict__ x, long long n, float2* __restrict__ part) {
+  constexpr int AHEAD = 16 / sizeof(G);
   __shared__ float sh[64];
   float s = 0.f;
   float bad = 0.f;
-  for (long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * 4; i < n;
-       i += (long long)gridDim.x * blockDim.x * 4) {
+  const long long stride = (long long)gridDim.x * blockDim.x * 4;
+  long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * 4;
+  for (; i + (AHEAD - 1) * stride + 4 <= n; i += AHEAD * stride) {
+    Grad4<G> v[AHEAD];
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k) v[k] = *reinterpret_cast<const Grad4<G>*>(x + i + k * stride);
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k) add_squares(s, grad4(v[k]));
+  }
+  for (; i < n; i += stride) {
     if (i + 4 <= n) {
-      const float4 v = load_grad4<G>(x, i);
-      s += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+      add_squares(s, load_grad4<G>(x, i));
     } else {
       for (long long j = i; j < n; ++j) {
         float f;
