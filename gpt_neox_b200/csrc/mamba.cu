@@ -6,20 +6,26 @@
 // the external causal_conv1d / mamba_ssm packages, called at megatron/model/mamba/mamba.py:220-247
 // and :264-320 (which run on [batch, channel, seq] and need two rearranges per block).
 //
-// Scan parallelisation: a thread owns 4 of the 16 states of one channel (a quad of lanes per channel), 32 channels per
-// CTA, and walks its piece of the sequence in blocks of 32 steps.  The sequence is cut into as few chunks as keep the
-// chip busy (scan_chunk_count): one chunk needs one pass; with more, a light pass first runs every chunk from a zero
-// state and records its end state and its sum of delta (the chunk's decay is exp(A * sum delta)), and the main pass
-// folds the earlier chunks into its start state.  The reverse recurrence of dL/dh is cut the same way.
-// The forward keeps the state at the start of every 32-step block for the backward, which recomputes 8 steps at a
-// time into registers and walks them in reverse.  Those states take 2 bytes per token and channel from the forward to the
-// backward (25 MB for 4 x 2048 x 1536, as much as one more 16-bit activation; 6 MB when a state per 128 steps was kept),
-// and the tiles' partial sums of dB and dC 4 bytes during the backward.
-// Bound by the shared-memory pipe (78-80 % busy in the main passes: a step's inputs, and the exchanges that sum dB, dC and
-// the channel sums over lanes); issue slots 42-50 %, DRAM 6-9 %.  Convolution + scan, forward + backward, 4 x
-// 2048 steps of 1536 channels: 1.78 ms with chunks of 128 steps in two passes each way, the states recomputed in three of
-// them and scalar staging; 0.98 ms with two (forward three) CTAs an SM; 0.86 ms with the exchanges of dB / dC step by
-// step; 0.82 ms now (backward sweep 418 us, 466 before).
+// Scan parallelisation: a lane owns 4 of the 16 states of two neighbouring channels (a quad of lanes per pair), a warp 16
+// channels, and walks its piece of the sequence in blocks of 32 steps, cut into segments of four: lane q of a quad reads,
+// prepares and finishes step q of a segment, so the forward sweeps and the light reverse sweep need no barrier but the
+// warp's.  The sequence is cut into as few chunks as keep the chip busy (scan_chunk_count): one chunk needs one pass; with
+// more, a light pass first runs every chunk from a zero state and records its end state and its sum of delta (the chunk's
+// decay is exp(A * sum delta)), and the main pass folds the other chunks into its start state.  The reverse recurrence of
+// dL/dh is cut the same way.
+// The forward keeps the state at the start of every 32-step block for the backward, which recomputes the states at the
+// starts of the segments, then four steps at a time into registers, and walks them in reverse; dB and dC are added over a
+// lane's two channels before lanes and warps exchange them, and the next block's segment is staged where the walked one
+// was.  Those states take 2 bytes per token and channel from the forward to the backward (25 MB for 4 x 2048 x 1536, as
+// much as one more 16-bit activation), and the tiles' partial sums of dB and dC 2 bytes during the backward.
+// Bound by: light sweeps, the unit of exponentials (16 per step and channel; 82 and 72 % busy); forward, that unit 68 %, shared
+// memory 69 % and issue slots 62 % together; backward, issue slots (59 % with 3 warps per scheduler; shared memory 55 %),
+// where a step and channel costs 500 lane operations for 16 states.  DRAM 6-10 %.
+// Convolution + scan, forward + backward, 4 x 2048 steps of 1536 channels, fp16: 785 us with one channel per quad, inputs staged by the
+// whole CTA and dB / dC exchanged per channel (final forward sweep 119, light ones 70 and 86, backward 407 us); 605 us now (95,
+// 63 and 78, 283).  Whole calls of few channels and one block are latency: 2 x 31 x 768 takes 46 us of kernels, 43 before.
+// Tried for the backward: states packed per channel pair instead of per state pair (B and C twice in shared memory, no copies
+// of a step's scalars): shared memory 62 % busy, 305 - 330 us; inputs staged per block with its loads waited for: 290 - 320.
 #include "common.h"
 #include "ptx.cuh"
 
@@ -330,14 +336,13 @@ NX_API int NX_SYM(nx_conv1d_silu_bwd)(const void* x, long long xsb, long long xs
 // ---------------------------------------------------------------------------------------------
 // selective scan
 // ---------------------------------------------------------------------------------------------
-constexpr int SC_CH = 32;       // channels per CTA
-constexpr int SC_T = 32;        // timesteps per block (staged together; the forward keeps a state per block)
-constexpr int SC_REG = 8;       // steps whose states the backward holds in registers
-constexpr int SC_THREADS = SC_CH * 4;
-constexpr int SC_LD = 40;       // row length of the [step][channel] result arrays: four steps land on distinct banks
-constexpr int SC_MAX_CHUNKS = 32;
-constexpr int SC_FWD_CTAS = 5, SC_BWD_CTAS = 3;   // CTAs per SM: latency (exponentials, shared memory, exchanges) is hidden
-                                                  // by other warps, so registers are bounded for more of them
+constexpr int SC_T = 32;        // steps per block (the forward keeps a state per block for the backward)
+constexpr int SC_SEG = 4;       // steps per segment: lane q of a quad reads, and writes the results of, step q of it
+constexpr int SC_SEGS = SC_T / SC_SEG;
+constexpr int SC_WCH = 16;      // channels per warp, two neighbouring ones per quad of lanes
+constexpr int SC_WARPS = 4, SC_THREADS = SC_WARPS * 32, SC_CH = SC_WARPS * SC_WCH;    // channels per CTA
+constexpr int SC_MAX_CHUNKS = 64;
+constexpr int SC_FWD_CTAS = 5, SC_BWD_CTAS = 3;   // CTAs per SM: registers are bounded for so many of them
 constexpr float LOG2E = 1.44269504088896340736f, LN2 = 0.69314718055994530942f;
 
 struct ScanParams {
@@ -348,487 +353,546 @@ struct ScanParams {
   long long osb, ost;
   float *chunk_state, *chunk_sumdt;   // [B, NC, D, 16] / [B, NC, D]: end state (or reverse carry) and sum of delta
   float *ckpt;                        // [B, ceil(L / 32), D, 16]: state at the start of every block; null = not kept
-  float *partBC;                      // [ceil(D / 32), B, L, 32]
+  float *partBC;                      // [ceil(D / 64), B, L, 32]
   float *dA, *dD, *dbias;
   int B, L, D, NC, clen;              // clen: steps per chunk, a multiple of SC_T
+  bool bc_vec;                        // four neighbouring values of B (and of C) can be read as 8 bytes
 };
 
-__device__ __forceinline__ float softplus_f(float v) { return v > 20.f ? v : log1pf(__expf(v)); }
-__device__ __forceinline__ float sigmoid_f(float v) { return 1.f / (1.f + __expf(-v)); }
+__device__ __forceinline__ float sigmoid_f(float v) { return __fdividef(1.f, 1.f + __expf(-v)); }
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+// log(1 + exp(v)) = max(v, 0) + log(1 + e) with e = exp(-|v|) <= 1, and log(1 + e) = 2 artanh(s) with s = e / (2 + e) <= 1/3,
+// whose series is cut off below 2e-8 of the value; no branch, and right for small e, infinities and NaN.  `e` goes out too.
+__device__ __forceinline__ float2 softplus2(float2 v, float2& e) {
+  e = make_float2(exp2f(-fabsf(v.x) * LOG2E), exp2f(-fabsf(v.y) * LOG2E));
+  const float2 n = fadd2(e, both(2.f)), s = make_float2(__fdividef(e.x, n.x), __fdividef(e.y, n.y)), u = fmul2(s, s);
+  float2 c = ffma2(u, both(1.f / 13.f), both(1.f / 11.f));
+  c = ffma2(u, c, both(1.f / 9.f));
+  c = ffma2(u, c, both(1.f / 7.f));
+  c = ffma2(u, c, both(1.f / 5.f));
+  c = ffma2(u, c, both(1.f / 3.f));
+  c = ffma2(u, c, both(1.f));
+  return ffma2(fadd2(s, s), c, make_float2(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f)));
+}
 
 // Sums four values per lane over the quad: lane q returns the total of v[q] (three exchanges instead of eight).
-__device__ __forceinline__ float quad_transpose_sum(const float (&v)[4], int q) {
+__device__ __forceinline__ float quad_transpose_sum(float v0, float v1, float v2, float v3, int q) {
   const bool hi = q & 2, odd = q & 1;
-  float a = hi ? v[2] : v[0], b = hi ? v[3] : v[1];
-  a += __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], 2);
-  b += __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], 2);
+  float a = hi ? v2 : v0, b = hi ? v3 : v1;
+  a += __shfl_xor_sync(0xffffffffu, hi ? v0 : v2, 2);
+  b += __shfl_xor_sync(0xffffffffu, hi ? v1 : v3, 2);
   const float keep = odd ? b : a;
   return keep + __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
 }
+__device__ __forceinline__ float quad_transpose_sum(const float (&v)[SC_SEG], int q) {
+  return quad_transpose_sum(v[0], v[1], v[2], v[3], q);
+}
+__device__ __forceinline__ float quad_sum(float v) {
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
 
-// The staging role of a thread: step tid / 4 of the block, 8 channels from (tid % 4) * 8.
-struct RowOf8 {
-  int t, c8, d;     // step in block, first channel in tile, first channel
-  int n;            // live channels (0..8)
+// A lane's place: states 4 q .. 4 q + 3 of the channels d and d + 1.
+struct ScanLane {
+  int lane, warp, j, q, d, n;       // n: live channels of the two
 };
-__device__ __forceinline__ RowOf8 row_of8(int d0, int D) {
-  RowOf8 r;
-  r.t = threadIdx.x >> 2;
-  r.c8 = (threadIdx.x & 3) * 8;
-  r.d = d0 + r.c8;
-  r.n = min(8, max(0, D - r.d));
-  return r;
+__device__ __forceinline__ ScanLane scan_lane(int D) {
+  ScanLane s;
+  s.lane = threadIdx.x & 31;
+  s.warp = threadIdx.x >> 5;
+  s.j = s.lane >> 2;
+  s.q = s.lane & 3;
+  s.d = blockIdx.x * SC_CH + s.warp * SC_WCH + 2 * s.j;
+  s.n = min(2, max(0, D - s.d));
+  return s;
 }
-// 8 consecutive 16-bit elements (zero where dead): one 16-byte load when VEC, single elements otherwise.
+// Two neighbouring 16-bit elements (zero where dead): one 4-byte access when VEC, single elements otherwise.
 template <bool VEC>
-__device__ __forceinline__ uint4 load8(const h16* p, int n) {
-  uint4 u = make_uint4(0u, 0u, 0u, 0u);
-  if (VEC) {
-    if (n > 0) u = *reinterpret_cast<const uint4*>(p);
-    return u;
-  }
-  uint16_t e[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) e[j] = j < n ? reinterpret_cast<const uint16_t*>(p)[j] : 0;
-  u.x = e[0] | (uint32_t)e[1] << 16; u.y = e[2] | (uint32_t)e[3] << 16;
-  u.z = e[4] | (uint32_t)e[5] << 16; u.w = e[6] | (uint32_t)e[7] << 16;
-  return u;
+__device__ __forceinline__ uint32_t load2(const h16* p, int n) {
+  if (VEC) return n > 0 ? *reinterpret_cast<const uint32_t*>(p) : 0u;
+  const uint16_t* e = reinterpret_cast<const uint16_t*>(p);
+  return (n > 0 ? e[0] : 0u) | (n > 1 ? static_cast<uint32_t>(e[1]) << 16 : 0u);
 }
 template <bool VEC>
-__device__ __forceinline__ void store8(h16* p, const float (&f)[8], int n) {
+__device__ __forceinline__ void store2(h16* p, float2 v, int n) {
   if (VEC) {
-    if (n > 0) store_vec<8>(p, f);
+    if (n > 0) *reinterpret_cast<uint32_t*>(p) = pack_h16x2(v.x, v.y);
     return;
   }
-#pragma unroll
-  for (int j = 0; j < 8; ++j)
-    if (j < n) p[j] = float_to_h16(f[j]);
+  if (n > 0) p[0] = float_to_h16(v.x);
+  if (n > 1) p[1] = float_to_h16(v.y);
 }
-__device__ __forceinline__ void unpack8f(const uint4& u, float (&f)[8]) {
-  const float2 a = unpack_h16x2(u.x), b = unpack_h16x2(u.y), c = unpack_h16x2(u.z), d = unpack_h16x2(u.w);
-  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+__device__ __forceinline__ float2 coef2(const float* p, const ScanLane& s) {
+  return make_float2(p != nullptr && s.n > 0 ? p[s.d] : 0.f, p != nullptr && s.n > 1 ? p[s.d + 1] : 0.f);
 }
-__device__ __forceinline__ void load_coef(const float* p, const RowOf8& r, float (&f)[8]) {
-#pragma unroll
-  for (int j = 0; j < 8; ++j) f[j] = (p != nullptr && j < r.n) ? p[r.d + j] : 0.f;
+// A lane's states: [channel of the two][pair of states].  In memory [channel][16] floats from the channel d on; zero where dead.
+__device__ __forceinline__ void get4(const float4& v, float2 (&h)[2]) {
+  h[0] = make_float2(v.x, v.y);
+  h[1] = make_float2(v.z, v.w);
 }
-
-// B or C of a block: 32 steps x 16 states, one column of 4 steps per thread.
-// They stay 16-bit in shared memory, so a step reads 4 states of each in 8 bytes and not 16: the pipe of shared memory and
-// exchanges bounded the scans (70 - 80 % busy with floats here; its wavefronts are at 49 - 73 % of their rate now, issue
-// slots at 48 - 63 %).  4 x 2048 x 1536, fp16,
-// us: final forward pass 131 -> 119, its light pass 72.5 -> 70.1, backward light pass 95.9 -> 86.7, backward 413 -> 406.
-__device__ __forceinline__ void load_bc(const h16* p, long long st, int t0, int t_end, uint16_t (&v)[4]) {
+__device__ __forceinline__ float4 put4(const float2 (&h)[2]) { return make_float4(h[0].x, h[0].y, h[1].x, h[1].y); }
+__device__ __forceinline__ void load_states(const float* p, const ScanLane& s, float2 (&h)[2][2]) {
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int t = (threadIdx.x >> 4) + 8 * k;
-    v[k] = t0 + t < t_end ? reinterpret_cast<const uint16_t*>(p)[(t0 + t) * st + (threadIdx.x & 15)] : 0;
+  for (int i = 0; i < 2; ++i) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < s.n) v = *reinterpret_cast<const float4*>(p + i * 16 + s.q * 4);
+    get4(v, h[i]);
   }
 }
-__device__ __forceinline__ void put_bc(uint16_t (*s)[16], const uint16_t (&v)[4]) {
+__device__ __forceinline__ void store_states(float* p, const ScanLane& s, const float2 (&h)[2][2]) {
 #pragma unroll
-  for (int k = 0; k < 4; ++k) s[(threadIdx.x >> 4) + 8 * k][threadIdx.x & 15] = v[k];
+  for (int i = 0; i < 2; ++i)
+    if (i < s.n) *reinterpret_cast<float4*>(p + i * 16 + s.q * 4) = put4(h[i]);
 }
-__device__ __forceinline__ float4 bc4(const uint16_t* p) {
-  const uint2 u = *reinterpret_cast<const uint2*>(p);
+// The states' decay rates times log2(e).
+__device__ __forceinline__ void load_A(const float* A, const ScanLane& s, float2 (&a)[2][2]) {
+  load_states(A + static_cast<long long>(s.d) * 16, s, a);
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int k = 0; k < 2; ++k) a[i][k] = fmul2(a[i][k], both(LOG2E));
+}
+// Four neighbouring values of a row of B or C.
+__device__ __forceinline__ uint2 load_bc4(const h16* p, bool vec) {
+  if (vec) return *reinterpret_cast<const uint2*>(p);
+  const uint16_t* e = reinterpret_cast<const uint16_t*>(p);
+  return make_uint2(e[0] | static_cast<uint32_t>(e[1]) << 16, e[2] | static_cast<uint32_t>(e[3]) << 16);
+}
+__device__ __forceinline__ float4 bc4(const uint2& u) {
   const float2 a = unpack_h16x2(u.x), b = unpack_h16x2(u.y);
   return make_float4(a.x, a.y, b.x, b.y);
 }
 
-__device__ __forceinline__ void exp4(float2 a01, float2 a23, float dl, float2 (&a)[2]) {
-  const float2 d2 = make_float2(dl, dl);
-  const float2 u = fmul2(d2, a01), v = fmul2(d2, a23);
-  a[0] = make_float2(exp2f(u.x), exp2f(u.y));
-  a[1] = make_float2(exp2f(v.x), exp2f(v.y));
+__device__ __forceinline__ float2 exp2_2(float2 v) { return make_float2(exp2f(v.x), exp2f(v.y)); }
+__device__ __forceinline__ void decay(const float2 (&A)[2], float dl, float2 (&a)[2]) {
+  a[0] = exp2_2(fmul2(both(dl), A[0]));
+  a[1] = exp2_2(fmul2(both(dl), A[1]));
 }
-__device__ __forceinline__ float4 f4(const float2 (&h)[2]) { return make_float4(h[0].x, h[0].y, h[1].x, h[1].y); }
+// One step of a channel's four states: h1 = a h0 + dx B, with a = exp(delta A).
+__device__ __forceinline__ void scan_step(const float2 (&A)[2], float dl, float dx, const float4& B, float2 (&a)[2],
+                                          const float2 (&h0)[2], float2 (&h1)[2]) {
+  decay(A, dl, a);
+  h1[0] = ffma2(a[0], h0[0], fmul2(both(dx), make_float2(B.x, B.y)));
+  h1[1] = ffma2(a[1], h0[1], fmul2(both(dx), make_float2(B.z, B.w)));
+}
+__device__ __forceinline__ float dot4(const float2 (&a)[2], const float4& b) {
+  const float2 v = ffma2(a[1], make_float2(b.z, b.w), fmul2(a[0], make_float2(b.x, b.y)));
+  return v.x + v.y;
+}
+// The state after the chunk c, whose walk from a zero state ended in chunk_state.
+__device__ __forceinline__ void fold_chunk(const ScanParams& p, const ScanLane& s, const float2 (&A)[2][2], int b, int c,
+                                           float2 (&h)[2][2]) {
+  const long long o = (static_cast<long long>(b) * p.NC + c) * p.D + s.d;
+  float2 e[2][2];
+  load_states(p.chunk_state + o * 16, s, e);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    float2 a[2];
+    decay(A[i], i < s.n ? p.chunk_sumdt[o + i] : 0.f, a);
+    h[i][0] = ffma2(a[0], h[i][0], e[i][0]);
+    h[i][1] = ffma2(a[1], h[i][1], e[i][1]);
+  }
+}
+__device__ __forceinline__ void put_chunk(const ScanParams& p, const ScanLane& s, int b, int c, const float2 (&h)[2][2],
+                                          float2 sdt) {
+  const long long o = (static_cast<long long>(b) * p.NC + c) * p.D + s.d;
+  store_states(p.chunk_state + o * 16, s, h);
+  sdt = make_float2(quad_sum(sdt.x), quad_sum(sdt.y));
+  if (s.q < s.n) p.chunk_sumdt[o + s.q] = s.q == 0 ? sdt.x : sdt.y;
+}
 
 // FINAL = false: chunks 0 .. NC - 2 from a zero state -> end state and sum of delta.
 template <bool FINAL, bool VEC>
 __global__ void __launch_bounds__(SC_THREADS, SC_FWD_CTAS)
 scan_fwd_kernel(const ScanParams p) {
-  __shared__ __align__(16) float2 dd[SC_T][SC_CH];        // (delta, delta * x)
-  __shared__ __align__(16) uint16_t Bs[SC_T][16], Cs[FINAL ? SC_T : 1][16];
-  __shared__ __align__(16) float ys[FINAL ? SC_T : 1][SC_LD];
-  const int ch = threadIdx.x >> 2, q = threadIdx.x & 3;
-  const int d0 = blockIdx.x * SC_CH, d = d0 + ch;
-  const int c = blockIdx.y, b = blockIdx.z;
-  const bool dv_ok = d < p.D;
-  const int dd_ = dv_ok ? d : 0;
-  const RowOf8 row = row_of8(d0, p.D);
-  const float4 Av = *reinterpret_cast<const float4*>(p.A + dd_ * 16 + q * 4);
-  const float2 A01 = make_float2(Av.x * LOG2E, Av.y * LOG2E), A23 = make_float2(Av.z * LOG2E, Av.w * LOG2E);
-  float2 h[2] = {{0.f, 0.f}, {0.f, 0.f}};
+  // per warp and for two segments in turn: delta and delta * x of a quad's two channels; B and C of the segment's steps
+  __shared__ float4 dd[SC_WARPS][2][SC_SEG][8], bc[SC_WARPS][2][SC_SEG][FINAL ? 8 : 4];
+  const ScanLane s = scan_lane(p.D);
+  const int c = blockIdx.y, b = blockIdx.z, q = s.q;
+  float2 A[2][2], h[2][2] = {};
+  load_A(p.A, s, A);
   if (FINAL) {
-    for (int cp = 0; cp < c; ++cp) {
-      const long long o = ((long long)b * p.NC + cp) * p.D + dd_;
-      float2 a[2];
-      exp4(A01, A23, p.chunk_sumdt[o], a);
-      const float4 e = *reinterpret_cast<const float4*>(p.chunk_state + o * 16 + q * 4);
-      h[0] = ffma2(h[0], a[0], make_float2(e.x, e.y));
-      h[1] = ffma2(h[1], a[1], make_float2(e.z, e.w));
-    }
+#pragma unroll 4
+    for (int cp = 0; cp < c; ++cp) fold_chunk(p, s, A, b, cp, h);     // (four chunks' loads in flight)
   }
   const int tc0 = c * p.clen, t_end = min(tc0 + p.clen, p.L);
-  const h16 *xp = p.x + b * p.xsb + row.d, *dp = p.dt + b * p.dsb + row.d;
-  const h16* zp = p.z != nullptr ? p.z + b * p.zsb + row.d : nullptr;
-  const h16 *bp = p.Bm + b * p.bsb, *cp_ = p.Cm + b * p.csb;
-  float bias8[8];
-  load_coef(p.dt_bias, row, bias8);
-  float sdt = 0.f;
-  uint4 xu, du, zu = make_uint4(0u, 0u, 0u, 0u);
-  uint16_t bv[4], cv[4];
-  auto fetch = [&](int t0) {
-    const int n = t0 + row.t < t_end ? row.n : 0;
-    xu = load8<VEC>(xp + (t0 + row.t) * p.xst, n);
-    du = load8<VEC>(dp + (t0 + row.t) * p.dst, n);
-    if (FINAL && zp != nullptr) zu = load8<VEC>(zp + (t0 + row.t) * p.zst, n);
-    load_bc(bp, p.bst, t0, t_end, bv);
-    if (FINAL) load_bc(cp_, p.cst, t0, t_end, cv);
+  // the lane's next segment: step q of it of x, dt and z, and four values of B or C of step lane / 8
+  const int bt = s.lane >> 3, bn = (s.lane & 7) * 4;
+  const bool isC = bn >= 16;
+  const h16 *xp = p.x + b * p.xsb + (tc0 + q) * p.xst + s.d, *dp = p.dt + b * p.dsb + (tc0 + q) * p.dst + s.d;
+  const h16* zp = FINAL && p.z != nullptr ? p.z + b * p.zsb + (tc0 + q) * p.zst + s.d : nullptr;
+  const h16* bcp = isC ? p.Cm + b * p.csb + (tc0 + bt) * p.cst + bn - 16 : p.Bm + b * p.bsb + (tc0 + bt) * p.bst + bn;
+  h16* op = FINAL ? p.out + b * p.osb + (tc0 + q) * p.ost + s.d : nullptr;
+  const float2 bias = coef2(p.dt_bias, s), Dv = FINAL ? coef2(p.Dv, s) : both(0.f);
+  float2 sdt = both(0.f);
+  struct Raw { uint32_t x, d, z; uint2 bc; } raw[2];
+  auto fetch = [&](int t0, Raw& r) {              // called for the segments one after the other
+    const int n = t0 + q < t_end ? s.n : 0;
+    r.x = load2<VEC>(xp, n);
+    r.d = load2<VEC>(dp, n);
+    xp += SC_SEG * p.xst;
+    dp += SC_SEG * p.dst;
+    r.z = 0u;
+    if (FINAL && zp != nullptr) {
+      r.z = load2<VEC>(zp, n);
+      zp += SC_SEG * p.zst;
+    }
+    r.bc = make_uint2(0u, 0u);
+    if (t0 + bt < t_end && (FINAL || !isC)) r.bc = load_bc4(bcp, p.bc_vec);
+    bcp += SC_SEG * (isC ? p.cst : p.bst);
   };
-  fetch(tc0);
-  for (int t0 = tc0; t0 < t_end; t0 += SC_T) {
-    const bool in = t0 + row.t < t_end;
-    float xv[8], dv[8];
-    unpack8f(xu, xv);
-    unpack8f(du, dv);
+  fetch(tc0, raw[0]);
+  fetch(tc0 + SC_SEG, raw[1]);
+  for (int tb = tc0; tb < t_end; tb += 2 * SC_SEG) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float dl = in && j < row.n ? softplus_f(dv[j] + bias8[j]) : 0.f;
-      dd[row.t][row.c8 + j] = make_float2(dl, dl * xv[j]);
-    }
-    put_bc(Bs, bv);
-    if (FINAL) put_bc(Cs, cv);
-    const uint4 zc = zu;
-    if (t0 + SC_T < t_end) fetch(t0 + SC_T);      // in flight during the 32 steps
-    if (FINAL && p.ckpt != nullptr && dv_ok)
-      *reinterpret_cast<float4*>(p.ckpt + (((long long)b * ((p.L + SC_T - 1) / SC_T) + t0 / SC_T) * p.D + d) * 16 + q * 4) =
-          f4(h);
-    __syncthreads();
-    const int live = t_end - t0;                  // (padded steps of the last group of four leave the state as it is)
-#pragma unroll 2
-    for (int g = 0; g < SC_T && g < live; g += 4) {
-      float yp[4];
+    for (int k = 0; k < 2; ++k) {
+      const int t0 = tb + k * SC_SEG;
+      if (t0 >= t_end) break;
+      const bool in = t0 + q < t_end;
+      const float2 xv = unpack_h16x2(raw[k].x), zv = unpack_h16x2(raw[k].z);
+      float2 e, dl = softplus2(fadd2(unpack_h16x2(raw[k].d), bias), e);
+      if (!in) dl = both(0.f);                    // (a step beyond the end leaves the state as it is)
+      const float2 dx = fmul2(dl, xv);
+      dd[s.warp][k][q][s.j ^ (2 * q)] = make_float4(dl.x, dx.x, dl.y, dx.y);   // (neither writers nor readers collide)
+      if (!FINAL) sdt = fadd2(sdt, dl);
+      if (FINAL || !isC) bc[s.warp][k][bt][s.lane & 7] = bc4(raw[k].bc);
+      fetch(t0 + 2 * SC_SEG, raw[k]);             // in flight during two segments
+      if (FINAL && p.ckpt != nullptr && (t0 & (SC_T - 1)) == 0)
+        store_states(p.ckpt + ((static_cast<long long>(b) * ((p.L + SC_T - 1) / SC_T) + t0 / SC_T) * p.D + s.d) * 16, s, h);
+      __syncwarp();        // (this buffer's last readers have passed the other one's)
+      float yp[2][SC_SEG];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int t = g + u;
-        const float2 dv2 = dd[t][ch];
-        const float4 B4 = bc4(&Bs[t][q * 4]);
-        const float2 dx2 = make_float2(dv2.y, dv2.y);
+      for (int t = 0; t < SC_SEG; ++t) {
+        const float4 v = dd[s.warp][k][t][s.j ^ (2 * t)], B4 = bc[s.warp][k][t][q];
         float2 a[2];
-        exp4(A01, A23, dv2.x, a);
-        h[0] = ffma2(a[0], h[0], fmul2(dx2, make_float2(B4.x, B4.y)));
-        h[1] = ffma2(a[1], h[1], fmul2(dx2, make_float2(B4.z, B4.w)));
+        scan_step(A[0], v.x, v.y, B4, a, h[0], h[0]);
+        scan_step(A[1], v.z, v.w, B4, a, h[1], h[1]);
         if (FINAL) {
-          const float4 C4 = bc4(&Cs[t][q * 4]);
-          const float2 y2 = ffma2(h[1], make_float2(C4.z, C4.w), fmul2(h[0], make_float2(C4.x, C4.y)));
-          yp[u] = y2.x + y2.y;
-        } else {
-          sdt += dv2.x;
+          const float4 C4 = bc[s.warp][k][t][4 + q];
+          yp[0][t] = dot4(h[0], C4);
+          yp[1][t] = dot4(h[1], C4);
         }
       }
-      if (FINAL) ys[g + q][ch] = quad_transpose_sum(yp, q);
-    }
-    __syncthreads();
-    if (FINAL) {
-      if (in) {
-        float y8[8], z8[8];
-        unpack8f(zc, z8);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float Dj = p.Dv != nullptr && j < row.n ? p.Dv[row.d + j] : 0.f;
-          y8[j] = ys[row.t][row.c8 + j] + Dj * xv[j];
-          if (zp != nullptr) y8[j] *= silu(z8[j]);
-        }
-        store8<VEC>(p.out + b * p.osb + (t0 + row.t) * p.ost + row.d, y8, row.n);
+      if (FINAL) {
+        float2 y = ffma2(Dv, xv, make_float2(quad_transpose_sum(yp[0], q), quad_transpose_sum(yp[1], q)));
+        if (p.z != nullptr) y = make_float2(y.x * silu(zv.x), y.y * silu(zv.y));
+        if (in) store2<VEC>(op, y, s.n);
+        op += SC_SEG * p.ost;
       }
     }
   }
-  if (!FINAL && dv_ok) {
-    const long long o = ((long long)b * p.NC + c) * p.D + d;
-    *reinterpret_cast<float4*>(p.chunk_state + o * 16 + q * 4) = f4(h);
-    if (q == 0) p.chunk_sumdt[o] = sdt;
-  }
+  if (!FINAL) put_chunk(p, s, b, c, h, sdt);
 }
 
 // Reverse recurrence of chunks 1 .. NC - 1 from a zero carry: chunk_state[c] = what chunk c hands to chunk c - 1.
 template <bool VEC>
-__global__ void __launch_bounds__(SC_THREADS)
+__global__ void __launch_bounds__(SC_THREADS, SC_FWD_CTAS)
 scan_bwd_local_kernel(const ScanParams p) {
-  __shared__ __align__(16) float2 dd[SC_T][SC_CH];        // (delta, gradient of the ungated output)
-  __shared__ __align__(16) uint16_t Cs[SC_T][16];
-  const int ch = threadIdx.x >> 2, q = threadIdx.x & 3;
-  const int d0 = blockIdx.x * SC_CH, d = d0 + ch;
-  const int c = blockIdx.y + 1, b = blockIdx.z;
-  const bool dv_ok = d < p.D;
-  const RowOf8 row = row_of8(d0, p.D);
-  const float4 Av = *reinterpret_cast<const float4*>(p.A + (dv_ok ? d : 0) * 16 + q * 4);
-  const float2 A01 = make_float2(Av.x * LOG2E, Av.y * LOG2E), A23 = make_float2(Av.z * LOG2E, Av.w * LOG2E);
-  float2 r[2] = {{0.f, 0.f}, {0.f, 0.f}};
+  // as in the forward: delta and the gradient of the ungated output of a quad's two channels; C
+  __shared__ float4 dd[SC_WARPS][2][SC_SEG][8], cs[SC_WARPS][2][SC_SEG][4];
+  const ScanLane s = scan_lane(p.D);
+  const int c = blockIdx.y + 1, b = blockIdx.z, q = s.q;
+  float2 A[2][2], r[2][2] = {};
+  load_A(p.A, s, A);
   const int tc0 = c * p.clen, t_end = min(tc0 + p.clen, p.L);
-  float bias8[8];
-  load_coef(p.dt_bias, row, bias8);
-  float sdt = 0.f;
-  for (int t0 = tc0 + (t_end - 1 - tc0) / SC_T * SC_T; t0 >= tc0; t0 -= SC_T) {
-    const int tt = t0 + row.t;
-    const bool in = tt < t_end;
-    const int n = in ? row.n : 0;
-    const uint4 du = load8<VEC>(p.dt + b * p.dsb + tt * p.dst + row.d, n);
-    const uint4 gu = load8<VEC>(p.dout + b * p.gsb + tt * p.gst + row.d, n);
-    float dv[8], gv[8], zv[8];
-    uint16_t cv[4];
-    unpack8f(du, dv);
-    unpack8f(gu, gv);
-    if (p.z != nullptr) unpack8f(load8<VEC>(p.z + b * p.zsb + tt * p.zst + row.d, n), zv);
-    load_bc(p.Cm + b * p.csb, p.cst, t0, t_end, cv);
-    __syncthreads();
+  const int last = tc0 + (t_end - 1 - tc0) / SC_SEG * SC_SEG, bt = s.j & 3;
+  const h16 *dp = p.dt + b * p.dsb + (last + q) * p.dst + s.d, *gp = p.dout + b * p.gsb + (last + q) * p.gst + s.d;
+  const h16* zp = p.z != nullptr ? p.z + b * p.zsb + (last + q) * p.zst + s.d : nullptr;
+  const h16* cp = p.Cm + b * p.csb + (last + bt) * p.cst + q * 4;
+  const float2 bias = coef2(p.dt_bias, s);
+  float2 sdt = both(0.f);
+  struct Raw { uint32_t d, g, z; uint2 c; } raw[2];
+  auto fetch = [&](int t0, Raw& u) {              // called for the segments one before the other
+    const int n = t0 >= tc0 && t0 + q < t_end ? s.n : 0;
+    u.d = load2<VEC>(dp, n);
+    u.g = load2<VEC>(gp, n);
+    dp -= SC_SEG * p.dst;
+    gp -= SC_SEG * p.gst;
+    u.z = 0u;
+    if (zp != nullptr) {
+      u.z = load2<VEC>(zp, n);
+      zp -= SC_SEG * p.zst;
+    }
+    u.c = make_uint2(0u, 0u);
+    if (t0 >= tc0 && t0 + bt < t_end) u.c = load_bc4(cp, p.bc_vec);
+    cp -= SC_SEG * p.cst;
+  };
+  fetch(last, raw[0]);
+  fetch(last - SC_SEG, raw[1]);
+  for (int tb = last; tb >= tc0; tb -= 2 * SC_SEG) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-      dd[row.t][row.c8 + j] = make_float2(in && j < row.n ? softplus_f(dv[j] + bias8[j]) : 0.f,
-                                          p.z != nullptr ? gv[j] * silu(zv[j]) : gv[j]);
-    put_bc(Cs, cv);
-    __syncthreads();
+    for (int k = 0; k < 2; ++k) {
+      const int t0 = tb - k * SC_SEG;
+      if (t0 < tc0) break;
+      float2 e, dl = softplus2(fadd2(unpack_h16x2(raw[k].d), bias), e), g = unpack_h16x2(raw[k].g);
+      if (t0 + q >= t_end) dl = both(0.f);
+      if (p.z != nullptr) {
+        const float2 zv = unpack_h16x2(raw[k].z);
+        g = fmul2(g, make_float2(silu(zv.x), silu(zv.y)));
+      }
+      dd[s.warp][k][q][s.j ^ (2 * q)] = make_float4(dl.x, g.x, dl.y, g.y);
+      sdt = fadd2(sdt, dl);
+      if (s.j < SC_SEG) cs[s.warp][k][bt][q] = bc4(raw[k].c);
+      fetch(t0 - 2 * SC_SEG, raw[k]);
+      __syncwarp();
 #pragma unroll
-    for (int t = SC_T - 1; t >= 0; --t) {
-      const float2 v = dd[t][ch];
-      const float4 C4 = bc4(&Cs[t][q * 4]);
-      const float2 g2 = make_float2(v.y, v.y);
-      float2 a[2];
-      exp4(A01, A23, v.x, a);
-      r[0] = fmul2(a[0], ffma2(make_float2(C4.x, C4.y), g2, r[0]));
-      r[1] = fmul2(a[1], ffma2(make_float2(C4.z, C4.w), g2, r[1]));
-      sdt += v.x;
+      for (int t = SC_SEG - 1; t >= 0; --t) {
+        const float4 v = dd[s.warp][k][t][s.j ^ (2 * t)], C4 = cs[s.warp][k][t][q];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float2 g2 = both(i == 0 ? v.y : v.w);
+          float2 a[2];
+          decay(A[i], i == 0 ? v.x : v.z, a);
+          r[i][0] = fmul2(a[0], ffma2(make_float2(C4.x, C4.y), g2, r[i][0]));
+          r[i][1] = fmul2(a[1], ffma2(make_float2(C4.z, C4.w), g2, r[i][1]));
+        }
+      }
     }
   }
-  if (dv_ok) {
-    const long long o = ((long long)b * p.NC + c) * p.D + d;
-    *reinterpret_cast<float4*>(p.chunk_state + o * 16 + q * 4) = f4(r);
-    if (q == 0) p.chunk_sumdt[o] = sdt;
-  }
+  put_chunk(p, s, b, c, r, sdt);
 }
 
-struct ScanBwdSmem {
-  float4 dd[SC_T][SC_CH];                     // delta, delta * x, gradient of the ungated output, sigmoid(dt)
-  uint16_t Bs[SC_T][16], Cs[SC_T][16];
-  float dzf[SC_T][SC_LD];                     // d out / d z without the scan value
-  float s_gb[SC_T][SC_LD], s_da[SC_T][SC_LD], s_hc[SC_T][SC_LD];   // sums over the 16 states
-  float4 ck[SC_T / SC_REG][SC_THREADS];       // states at the starts of the block's quarters
-  float acc[SC_THREADS][17];                  // dD and dbias of a staging thread's 8 channels
-  float bc[SC_THREADS / 32][SC_T][32];
+struct ScanBwdWarp {
+  float4 dd[SC_T][SC_WCH];            // delta, x, gradient of the ungated output, sigmoid(dt) of the warp's channels
+  float4 ck[SC_SEGS - 1][2][32];      // a lane's states at the starts of the segments 1 .., per channel
+  float2 dzf[SC_SEGS][32];            // d out / d z without the scan value, of the lane that writes it
+  // A segment's states make room, once used: the first half for the sums over the warp's channels, dB and dC as [step][32]
+  // (segment 0 has no states here, its sums go to the second half of segment 5), the second halves of the last two for the
+  // state at the block's start, and of segments 3 and 4 for that of the next block to be walked.
+  __device__ __forceinline__ float* sums(int sg) { return reinterpret_cast<float*>(sg > 0 ? ck[sg - 1][0] : ck[4][1]); }
+  __device__ __forceinline__ float4* start(int i, int lane) { return &ck[5 + i][1][lane]; }
+  __device__ __forceinline__ float4* next_start(int i, int lane) { return &ck[2 + i][1][lane]; }
+  // a step's 16 channels, placed so that neither a segment's writers (a step per lane of a quad) nor a step's readers collide
+  static __device__ __forceinline__ int slot(int t, int j, int i) { return i * 8 + (j ^ (2 * (t & 3))); }
 };
+struct ScanBwdSmem {
+  ScanBwdWarp w[SC_WARPS];
+  float bc[SC_T][32];                 // B | C
+};
+// 16 bytes to shared memory behind the thread's back (zeros where dead); waited for by the thread that asked.
+__device__ __forceinline__ void copy16_async(float4* dst, const float* src, bool live) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src), "r"(live ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 template <bool VEC>
 __global__ void __launch_bounds__(SC_THREADS, SC_BWD_CTAS)
 scan_bwd_kernel(const ScanParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  ScanBwdSmem& s = *reinterpret_cast<ScanBwdSmem*>(smem_raw);
-  const int ch = threadIdx.x >> 2, q = threadIdx.x & 3;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int d0 = blockIdx.x * SC_CH, d = d0 + ch;
-  const int c = blockIdx.y, b = blockIdx.z;
-  const bool dv_ok = d < p.D;
-  const int dd_ = dv_ok ? d : 0;
-  const RowOf8 row = row_of8(d0, p.D);
-  const float4 Av = *reinterpret_cast<const float4*>(p.A + dd_ * 16 + q * 4);
-  const float2 A01 = make_float2(Av.x * LOG2E, Av.y * LOG2E), A23 = make_float2(Av.z * LOG2E, Av.w * LOG2E);
-  float2 r[2] = {{0.f, 0.f}, {0.f, 0.f}}, dA[2] = {{0.f, 0.f}, {0.f, 0.f}};
-  for (int cp = p.NC - 1; cp > c; --cp) {
-    const long long o = ((long long)b * p.NC + cp) * p.D + dd_;
-    float2 a[2];
-    exp4(A01, A23, p.chunk_sumdt[o], a);
-    const float4 e = *reinterpret_cast<const float4*>(p.chunk_state + o * 16 + q * 4);
-    r[0] = ffma2(a[0], r[0], make_float2(e.x, e.y));
-    r[1] = ffma2(a[1], r[1], make_float2(e.z, e.w));
-  }
-#pragma unroll
-  for (int j = 0; j < 16; ++j) s.acc[threadIdx.x][j] = 0.f;
+  ScanBwdSmem& sm = *reinterpret_cast<ScanBwdSmem*>(smem_raw);
+  const ScanLane s = scan_lane(p.D);
+  ScanBwdWarp& w = sm.w[s.warp];
+  const int c = blockIdx.y, b = blockIdx.z, q = s.q, lane = s.lane;
+  float2 A[2][2], r[2][2] = {}, dA[2][2] = {};
+  load_A(p.A, s, A);
+#pragma unroll 4
+  for (int cp = p.NC - 1; cp > c; --cp) fold_chunk(p, s, A, b, cp, r);
   const int tc0 = c * p.clen, t_end = min(tc0 + p.clen, p.L);
   // which of the quad's 8 values (dB of 4 states, dC of 4 states) this lane ends up with after the exchange over channels
   const bool b2 = lane & 4, b3 = lane & 8, b4 = lane & 16;
   const int idx = (b2 ? 4 : 0) + (b3 ? 2 : 0) + (b4 ? 1 : 0);
   const int col = idx < 4 ? q * 4 + idx : 16 + q * 4 + (idx - 4);
-  uint4 xu, du, gu, zu = make_uint4(0u, 0u, 0u, 0u);
-  uint16_t bv[4], cv[4];
-  float4 hc;                                  // state at the start of the block
-  auto fetch = [&](int t0) {
-    const int tt = t0 + row.t, n = tt < t_end ? row.n : 0;
-    xu = load8<VEC>(p.x + b * p.xsb + tt * p.xst + row.d, n);
-    du = load8<VEC>(p.dt + b * p.dsb + tt * p.dst + row.d, n);
-    gu = load8<VEC>(p.dout + b * p.gsb + tt * p.gst + row.d, n);
-    if (p.z != nullptr) zu = load8<VEC>(p.z + b * p.zsb + tt * p.zst + row.d, n);
-    load_bc(p.Bm + b * p.bsb, p.bst, t0, t_end, bv);
-    load_bc(p.Cm + b * p.csb, p.cst, t0, t_end, cv);
-    hc = *reinterpret_cast<const float4*>(
-        p.ckpt + (((long long)b * ((p.L + SC_T - 1) / SC_T) + t0 / SC_T) * p.D + dd_) * 16 + q * 4);
+  const float2 bias = coef2(p.dt_bias, s), Dv = coef2(p.Dv, s);
+  float2 sumD = both(0.f), sumb = both(0.f);
+  const float* ckpt = p.ckpt + (static_cast<long long>(b) * ((p.L + SC_T - 1) / SC_T) * p.D + s.d) * 16 + q * 4;
+  const int last = tc0 + (t_end - 1 - tc0) / SC_T * SC_T;
+  struct Raw { uint32_t x, d, g, z; };
+  auto fetch = [&](int t, Raw& u) {               // the lane's two channels of step t
+    const int n = t < t_end ? s.n : 0;
+    u.x = load2<VEC>(p.x + b * p.xsb + t * p.xst + s.d, n);
+    u.d = load2<VEC>(p.dt + b * p.dsb + t * p.dst + s.d, n);
+    u.g = load2<VEC>(p.dout + b * p.gsb + t * p.gst + s.d, n);
+    u.z = p.z != nullptr ? load2<VEC>(p.z + b * p.zsb + t * p.zst + s.d, n) : 0u;
   };
-  int t0 = tc0 + (t_end - 1 - tc0) / SC_T * SC_T;
-  fetch(t0);
-  for (; t0 >= tc0; t0 -= SC_T) {
-    const bool in = t0 + row.t < t_end;
-    const uint4 xc = xu;
-    {
-      float xv[8], dv[8], gv[8], zv[8];
-      unpack8f(xu, xv);
-      unpack8f(du, dv);
-      unpack8f(gu, gv);
-      unpack8f(zu, zv);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float dl = 0.f, sg = 0.f, dys = gv[j], dzf = 0.f;
-        if (in && j < row.n) {
-          const float raw = dv[j] + p.dt_bias[row.d + j], e = __expf(raw);
-          dl = raw > 20.f ? raw : log1pf(e);
-          sg = raw > 20.f ? 1.f : e / (1.f + e);
-        }
-        if (p.z != nullptr) {
-          const float sz = sigmoid_f(zv[j]);
-          dys = gv[j] * (zv[j] * sz);
-          dzf = gv[j] * (sz * (1.f + zv[j] * (1.f - sz)));
-        }
-        s.dd[row.t][row.c8 + j] = make_float4(dl, dl * xv[j], dys, sg);
-        s.dzf[row.t][row.c8 + j] = dzf;
-      }
+  auto stage = [&](int sg, const Raw& u, bool in) {
+    const float2 xv = unpack_h16x2(u.x), v = fadd2(unpack_h16x2(u.d), bias);
+    float2 e, dl = softplus2(v, e), sd, dys = unpack_h16x2(u.g), dzf = both(0.f);
+    sd = make_float2(__fdividef(v.x >= 0.f ? 1.f : e.x, 1.f + e.x), __fdividef(v.y >= 0.f ? 1.f : e.y, 1.f + e.y));
+    if (!in) dl = sd = both(0.f);
+    if (p.z != nullptr) {
+      const float2 z = unpack_h16x2(u.z), sz = make_float2(sigmoid_f(z.x), sigmoid_f(z.y)), zs = fmul2(z, sz);
+      // silu' = sz (1 + z (1 - sz)) = sz + z sz (1 - sz)
+      dzf = fmul2(dys, ffma2(zs, fadd2(both(1.f), make_float2(-sz.x, -sz.y)), sz));
+      dys = fmul2(dys, zs);
     }
-    put_bc(s.Bs, bv);
-    put_bc(s.Cs, cv);
-    __syncthreads();
-    // the states at the starts of the quarters (read back by the thread that wrote them)
-    const int quarters = min(SC_T / SC_REG, (t_end - t0 + SC_REG - 1) / SC_REG);
-    {
-      float2 h[2] = {{hc.x, hc.y}, {hc.z, hc.w}};
-      s.ck[0][threadIdx.x] = f4(h);
-#pragma unroll 1
-      for (int quarter = 1; quarter < quarters; ++quarter) {
-#pragma unroll
-        for (int k = 0; k < SC_REG; ++k) {
-          const int t = (quarter - 1) * SC_REG + k;
-          const float4 v = s.dd[t][ch];
-          const float4 B4 = bc4(&s.Bs[t][q * 4]);
-          const float2 dx2 = make_float2(v.y, v.y);
-          float2 a[2];
-          exp4(A01, A23, v.x, a);
-          h[0] = ffma2(a[0], h[0], fmul2(dx2, make_float2(B4.x, B4.y)));
-          h[1] = ffma2(a[1], h[1], fmul2(dx2, make_float2(B4.z, B4.w)));
-        }
-        s.ck[quarter][threadIdx.x] = f4(h);
-      }
+    w.dd[sg * SC_SEG + q][w.slot(q, s.j, 0)] = make_float4(dl.x, xv.x, dys.x, sd.x);
+    w.dd[sg * SC_SEG + q][w.slot(q, s.j, 1)] = make_float4(dl.y, xv.y, dys.y, sd.y);
+    w.dzf[sg][lane] = dzf;
+  };
+  auto fetch_start = [&](int t0, float4* a, float4* b, bool any) {        // the state at the start of a block
+    if (any) {
+      const float* src = ckpt + static_cast<long long>(t0 / SC_T) * p.D * 16;
+      copy16_async(a, s.n > 0 ? src : p.ckpt, s.n > 0);
+      copy16_async(b, s.n > 1 ? src + 16 : p.ckpt, s.n > 1);
     }
-    if (t0 - SC_T >= tc0) fetch(t0 - SC_T);       // in flight during this block
+    copy_async_commit();
+  };
+  // Blocks from the last one back, before it a turn that only brings it in: while a block's segment is walked, the same
+  // segment of the block to be walked next is on its way from memory, and takes its place afterwards.
+  for (int t0 = last + SC_T;; t0 -= SC_T) {
+    const bool more = t0 > tc0;
+    const int segs = t0 <= last ? min(SC_SEGS, (t_end - t0 + SC_SEG - 1) / SC_SEG) : 0, tn = t0 - SC_T;
+    if (segs == 0) {
+      Raw u[SC_SEGS];
+#pragma unroll
+      for (int sg = 0; sg < SC_SEGS; ++sg) fetch(tn + sg * SC_SEG + q, u[sg]);
+      fetch_start(tn, w.next_start(0, lane), w.next_start(1, lane), true);
+#pragma unroll
+      for (int sg = 0; sg < SC_SEGS; ++sg) stage(sg, u[sg], tn + sg * SC_SEG + q < t_end);
+    }
 #pragma unroll 1
-    for (int quarter = quarters - 1; quarter >= 0; --quarter) {
-      const int tb = quarter * SC_REG;
-      float2 hs[SC_REG + 1][2], as[SC_REG][2];    // hs[t + 1]: state after step t
-      const float4 h0 = s.ck[quarter][threadIdx.x];
-      hs[0][0] = make_float2(h0.x, h0.y);
-      hs[0][1] = make_float2(h0.z, h0.w);
-#pragma unroll
-      for (int t = 0; t < SC_REG; ++t) {
-        const float4 v = s.dd[tb + t][ch];
-        const float4 B4 = bc4(&s.Bs[tb + t][q * 4]);
-        const float2 dx2 = make_float2(v.y, v.y);
-        exp4(A01, A23, v.x, as[t]);
-        hs[t + 1][0] = ffma2(as[t][0], hs[t][0], fmul2(dx2, make_float2(B4.x, B4.y)));
-        hs[t + 1][1] = ffma2(as[t][1], hs[t][1], fmul2(dx2, make_float2(B4.z, B4.w)));
+    for (int sg = segs > 0 ? SC_SEGS - 1 : -1; sg >= 0; --sg) {
+      const int tb = sg * SC_SEG;
+      Raw raw = {};
+      if (more) fetch(tn + tb + q, raw);          // (a full block: only the last one walked first may be short)
+      if (sg == 1) fetch_start(t0, w.start(0, lane), w.start(1, lane), true);
+      if (sg == 0) {
+        fetch_start(tn, w.next_start(0, lane), w.next_start(1, lane), more);
+        copy_async_wait<1>();
       }
+      if (sg < segs) {
+        float2 aB[SC_SEG][2], aC[SC_SEG][2];        // dB and dC of the quad's two channels
+        float ox[2], ot[2], oz[2];
+        const bool in = t0 + tb + q < t_end;
+        const float2 dzf = w.dzf[sg][lane];
 #pragma unroll
-      for (int g = SC_REG - 4; g >= 0; g -= 4) {
-        float v_gb[4], v_da[4], v_hc[4], vB[4][4], vC[4][4];
+        for (int i = 0; i < 2; ++i) {
+          float2 hs[SC_SEG + 1][2], as[SC_SEG][2];  // hs[t + 1]: state after step t
+          float4 v[SC_SEG];
+          float dx[SC_SEG];
+          get4(sg > 0 ? w.ck[sg - 1][i][lane] : *w.start(i, lane), hs[0]);
 #pragma unroll
-        for (int u = 3; u >= 0; --u) {
-          const int t = g + u;
-          const float4 v = s.dd[tb + t][ch];
-          const float4 B4 = bc4(&s.Bs[tb + t][q * 4]);
-          const float4 C4 = bc4(&s.Cs[tb + t][q * 4]);
-          const float2 dl2 = make_float2(v.x, v.x), dx2 = make_float2(v.y, v.y), dy2 = make_float2(v.z, v.z);
-          const float2 g0 = ffma2(make_float2(C4.x, C4.y), dy2, r[0]), g1 = ffma2(make_float2(C4.z, C4.w), dy2, r[1]);
-          r[0] = fmul2(as[t][0], g0);
-          r[1] = fmul2(as[t][1], g1);
-          const float2 e0 = fmul2(r[0], hs[t][0]), e1 = fmul2(r[1], hs[t][1]);     // g * a * h_{t-1}
-          dA[0] = ffma2(e0, dl2, dA[0]);
-          dA[1] = ffma2(e1, dl2, dA[1]);
-          const float2 da = ffma2(e1, A23, fmul2(e0, A01));
-          const float2 gb = ffma2(g1, make_float2(B4.z, B4.w), fmul2(g0, make_float2(B4.x, B4.y)));
-          const float2 hcv = ffma2(hs[t + 1][1], make_float2(C4.z, C4.w), fmul2(hs[t + 1][0], make_float2(C4.x, C4.y)));
-          v_da[u] = da.x + da.y;
-          v_gb[u] = gb.x + gb.y;
-          v_hc[u] = hcv.x + hcv.y;
-          const float2 b0 = fmul2(g0, dx2), b1 = fmul2(g1, dx2);                   // dB
-          const float2 c0 = fmul2(hs[t + 1][0], dy2), c1 = fmul2(hs[t + 1][1], dy2);   // dC
-          vB[u][0] = b0.x; vB[u][1] = b0.y; vB[u][2] = b1.x; vB[u][3] = b1.y;
-          vC[u][0] = c0.x; vC[u][1] = c0.y; vC[u][2] = c1.x; vC[u][3] = c1.y;
+          for (int t = 0; t < SC_SEG; ++t) {
+            v[t] = w.dd[tb + t][w.slot(t, s.j, i)];
+            dx[t] = v[t].x * v[t].y;
+            scan_step(A[i], v[t].x, dx[t], *reinterpret_cast<const float4*>(&sm.bc[tb + t][q * 4]), as[t], hs[t], hs[t + 1]);
+          }
+          float v_gb[SC_SEG], v_da[SC_SEG], v_hc[SC_SEG];
+#pragma unroll
+          for (int t = SC_SEG - 1; t >= 0; --t) {
+            const float4 B4 = *reinterpret_cast<const float4*>(&sm.bc[tb + t][q * 4]);
+            const float4 C4 = *reinterpret_cast<const float4*>(&sm.bc[tb + t][16 + q * 4]);
+            const float2 dl2 = both(v[t].x), dx2 = both(dx[t]), dy2 = both(v[t].z);
+            const float2 g[2] = {ffma2(make_float2(C4.x, C4.y), dy2, r[i][0]), ffma2(make_float2(C4.z, C4.w), dy2, r[i][1])};
+            r[i][0] = fmul2(as[t][0], g[0]);
+            r[i][1] = fmul2(as[t][1], g[1]);
+            const float2 e0 = fmul2(r[i][0], hs[t][0]), e1 = fmul2(r[i][1], hs[t][1]);     // g * a * h_{t-1}
+            dA[i][0] = ffma2(e0, dl2, dA[i][0]);
+            dA[i][1] = ffma2(e1, dl2, dA[i][1]);
+            const float2 da = ffma2(e1, A[i][1], fmul2(e0, A[i][0]));
+            v_da[t] = da.x + da.y;
+            v_gb[t] = dot4(g, B4);
+            v_hc[t] = dot4(hs[t + 1], C4);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              aB[t][k] = i == 0 ? fmul2(g[k], dx2) : ffma2(g[k], dx2, aB[t][k]);
+              aC[t][k] = i == 0 ? fmul2(hs[t + 1][k], dy2) : ffma2(hs[t + 1][k], dy2, aC[t][k]);
+            }
+          }
+          const float da = quad_transpose_sum(v_da, q), gb = quad_transpose_sum(v_gb, q), hc = quad_transpose_sum(v_hc, q);
+          const float4 m = w.dd[tb + q][w.slot(q, s.j, i)];
+          const float Di = i == 0 ? Dv.x : Dv.y;
+          ox[i] = m.x * gb + Di * m.z;
+          ot[i] = (LN2 * da + m.y * gb) * m.w;                                             // A was scaled by log2(e)
+          oz[i] = (i == 0 ? dzf.x : dzf.y) * (hc + Di * m.y);
+          if (in) {
+            (i == 0 ? sumD.x : sumD.y) += m.z * m.y;
+            (i == 0 ? sumb.x : sumb.y) += ot[i];
+          }
         }
-        // sum dB / dC over the 8 channels of the warp, halving the value set at every exchange; four steps together, so
+        if (in) {
+          const long long o = b * p.osb + (t0 + tb + q) * p.ost + s.d;
+          store2<VEC>(p.dx + o, make_float2(ox[0], ox[1]), s.n);
+          store2<VEC>(p.ddt + o, make_float2(ot[0], ot[1]), s.n);
+          if (p.dz != nullptr) store2<VEC>(p.dz + o, make_float2(oz[0], oz[1]), s.n);
+        }
+        // sum dB / dC over the 8 quads of the warp, halving the value set at every exchange; four steps together, so
         // that their exchanges overlap
-        float w4[4][4], w2[4][2];
+        float w4[SC_SEG][4], w2[SC_SEG][2];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int t = 0; t < SC_SEG; ++t) {
+          const float vB[4] = {aB[t][0].x, aB[t][0].y, aB[t][1].x, aB[t][1].y};
+          const float vC[4] = {aC[t][0].x, aC[t][0].y, aC[t][1].x, aC[t][1].y};
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            w4[u][j] = (b2 ? vC[u][j] : vB[u][j]) + __shfl_xor_sync(0xffffffffu, b2 ? vB[u][j] : vC[u][j], 4);
+          for (int k = 0; k < 4; ++k) w4[t][k] = (b2 ? vC[k] : vB[k]) + __shfl_xor_sync(0xffffffffu, b2 ? vB[k] : vC[k], 4);
+        }
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int t = 0; t < SC_SEG; ++t)
 #pragma unroll
-          for (int j = 0; j < 2; ++j)
-            w2[u][j] = (b3 ? w4[u][2 + j] : w4[u][j]) + __shfl_xor_sync(0xffffffffu, b3 ? w4[u][j] : w4[u][2 + j], 8);
+          for (int k = 0; k < 2; ++k)
+            w2[t][k] = (b3 ? w4[t][2 + k] : w4[t][k]) + __shfl_xor_sync(0xffffffffu, b3 ? w4[t][k] : w4[t][2 + k], 8);
+        __syncwarp();                   // every lane has read its states of this segment, and the segment's inputs
+        float* sums = w.sums(sg);
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          s.bc[warp][tb + g + u][col] =
-              (b4 ? w2[u][1] : w2[u][0]) + __shfl_xor_sync(0xffffffffu, b4 ? w2[u][0] : w2[u][1], 16);
-        s.s_da[tb + g + q][ch] = quad_transpose_sum(v_da, q);
-        s.s_gb[tb + g + q][ch] = quad_transpose_sum(v_gb, q);
-        s.s_hc[tb + g + q][ch] = quad_transpose_sum(v_hc, q);
+        for (int t = 0; t < SC_SEG; ++t)
+          sums[t * 32 + col] = (b4 ? w2[t][1] : w2[t][0]) + __shfl_xor_sync(0xffffffffu, b4 ? w2[t][0] : w2[t][1], 16);
       }
+      if (more) stage(sg, raw, true);
     }
-    __syncthreads();
-    if (in && row.n > 0) {
-      float xv[8], ox[8], ot[8], oz[8];
-      unpack8f(xc, xv);
+    uint2 bcu[2];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float4 v = s.dd[row.t][row.c8 + j];
-        const float Dj = p.Dv != nullptr && j < row.n ? p.Dv[row.d + j] : 0.f;
-        const float gb = s.s_gb[row.t][row.c8 + j];
-        ox[j] = v.x * gb + Dj * v.z;
-        ot[j] = (LN2 * s.s_da[row.t][row.c8 + j] + xv[j] * gb) * v.w;              // A was scaled by log2(e)
-        oz[j] = s.dzf[row.t][row.c8 + j] * (s.s_hc[row.t][row.c8 + j] + Dj * xv[j]);
-        s.acc[threadIdx.x][j] += v.z * xv[j];
-        s.acc[threadIdx.x][8 + j] += ot[j];
-      }
-      const long long o = b * p.osb + (t0 + row.t) * p.ost + row.d;
-      store8<VEC>(p.dx + o, ox, row.n);
-      store8<VEC>(p.ddt + o, ot, row.n);
-      if (p.dz != nullptr) store8<VEC>(p.dz + o, oz, row.n);
+    for (int k = 0; k < 2; ++k) {
+      const int t = tn + (threadIdx.x >> 3) + 16 * k, n4 = (threadIdx.x & 7) * 4;
+      bcu[k] = make_uint2(0u, 0u);
+      if (more && t < t_end)
+        bcu[k] = load_bc4(n4 < 16 ? p.Bm + b * p.bsb + t * p.bst + n4 : p.Cm + b * p.csb + t * p.cst + n4 - 16, p.bc_vec);
     }
-    for (int i = threadIdx.x; i < SC_T * 8; i += SC_THREADS) {
-      const int t = i >> 3, c4 = (i & 7) * 4;
-      if (t0 + t < t_end) {
+    __syncthreads();                  // the warps' sums of the block are there, and B and C have been used
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int t = (threadIdx.x >> 3) + 16 * k, c4 = (threadIdx.x & 7) * 4;
+      if (segs > 0 && t0 + t < t_end) {
         float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int w = 0; w < SC_THREADS / 32; ++w) {
-          const float4 v = *reinterpret_cast<const float4*>(&s.bc[w][t][c4]);
-          a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+        for (int ww = 0; ww < SC_WARPS; ++ww) {
+          const float4 u = *reinterpret_cast<const float4*>(sm.w[ww].sums(t / SC_SEG) + (t & (SC_SEG - 1)) * 32 + c4);
+          a.x += u.x; a.y += u.y; a.z += u.z; a.w += u.w;
         }
-        *reinterpret_cast<float4*>(p.partBC + (((long long)blockIdx.x * p.B + b) * p.L + t0 + t) * 32 + c4) = a;
+        *reinterpret_cast<float4*>(p.partBC + ((static_cast<long long>(blockIdx.x) * p.B + b) * p.L + t0 + t) * 32 + c4) = a;
       }
+      *reinterpret_cast<float4*>(&sm.bc[t][c4]) = bc4(bcu[k]);
     }
-    __syncthreads();
-  }
-  if (dv_ok) {
-    float* o = p.dA + d * 16 + q * 4;
-    atomicAdd(o, dA[0].x);
-    atomicAdd(o + 1, dA[0].y);
-    atomicAdd(o + 2, dA[1].x);
-    atomicAdd(o + 3, dA[1].y);
-  }
-  if (threadIdx.x < 2 * SC_CH) {                  // 32 steps' staging threads -> one value per channel
-    const int cc = threadIdx.x % SC_CH, which = threadIdx.x / SC_CH;
-    float a = 0.f;
-    for (int t = 0; t < SC_T; ++t) a += s.acc[t * 4 + cc / 8][which * 8 + cc % 8];
-    if (d0 + cc < p.D) {
-      if (which == 1) atomicAdd(p.dbias + d0 + cc, a);
-      else if (p.dD != nullptr) atomicAdd(p.dD + d0 + cc, a);
+    if (!more) break;
+    copy_async_wait<0>();
+    float2 h[2][2];
+    get4(*w.next_start(0, lane), h[0]);
+    get4(*w.next_start(1, lane), h[1]);
+    __syncthreads();                  // B and C of the next block are there, and the sums have been read
+    // the states at the starts of its segments (read back by the lane that wrote them)
+    const int next_segs = min(SC_SEGS, (t_end - tn + SC_SEG - 1) / SC_SEG);
+#pragma unroll 1
+    for (int sg = 0; sg < next_segs - 1; ++sg) {
+#pragma unroll
+      for (int t = 0; t < SC_SEG; ++t) {
+        const float4 B4 = *reinterpret_cast<const float4*>(&sm.bc[sg * SC_SEG + t][q * 4]);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float2 v = *reinterpret_cast<const float2*>(&w.dd[sg * SC_SEG + t][w.slot(t, s.j, i)]);
+          float2 a[2];
+          scan_step(A[i], v.x, v.x * v.y, B4, a, h[i], h[i]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) w.ck[sg][i][lane] = put4(h[i]);
     }
   }
+  sumD = make_float2(quad_sum(sumD.x), quad_sum(sumD.y));
+  sumb = make_float2(quad_sum(sumb.x), quad_sum(sumb.y));
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    if (i < s.n) {
+      float* o = p.dA + (s.d + i) * 16 + q * 4;
+      atomicAdd(o, dA[i][0].x);
+      atomicAdd(o + 1, dA[i][0].y);
+      atomicAdd(o + 2, dA[i][1].x);
+      atomicAdd(o + 3, dA[i][1].y);
+      if (q == 0) atomicAdd(p.dbias + s.d + i, i == 0 ? sumb.x : sumb.y);
+      if (q == 1 && p.dD != nullptr) atomicAdd(p.dD + s.d + i, i == 0 ? sumD.x : sumD.y);
+    }
 }
 
 // dB and dC of every (batch, step): the channel tiles' partial sums, rounded once.
@@ -848,19 +912,30 @@ scan_bc_reduce_kernel(const float* __restrict__ part, int ntiles, long long rows
   *reinterpret_cast<uint2*>(o) = make_uint2(pack_h16x2(a.x, a.y), pack_h16x2(a.z, a.w));
 }
 
-// Chunks the sequence is cut into.  The kernels are bound by latency until an SM holds its `ctas` CTAs, so time goes with
-// the chunk length times the number of rounds the CTAs take; more than one chunk adds the light pass over all chunks but
-// one (about `light` of the main pass).  The count depends on the batch and the channels, and the chunks' states are folded
-// in fp32: a sequence's last bits are not those it has in another batch.
+// Chunks the sequence is cut into.  Time goes with the blocks of a chunk times the rounds that the CTAs take; a last round
+// that leaves an SM only some of its CTAs is shorter (measured, time of a block with 1, 2, 3 CTAs on every SM: backward 0.57,
+// 0.77, 1; forward, 1 .. 5: 0.48, 0.54, 0.66, 0.85, 1).  More than one chunk adds the light pass over all chunks but one, whose
+// block takes `light` of the main pass's (forward 7.2 of 10 us, backward 9 of 18.5, with every SM full).  us, forward + backward,
+// fp16, with 1, 4, 8, 16, 22 and 32 chunks: 4 x 2048 x 1536: 983, 586, 552, 511, 506, 525 (the rule: 22 and 32);
+// 16 x 512 x 1536: 416, 485, 486, 531 (1 and 1); 1 x 4096 x 1536: 1871, 779, 473, 312, 315, 311 (26 and 16).  The count depends
+// on the batch and the channels, and the chunks' states are folded in fp32: a sequence's last bits are not those it has in
+// another batch.
+static float scan_rounds(long long ctas, int per_sm) {
+  const int sms = sm_count();
+  const long long slots = static_cast<long long>(per_sm) * sms, rest = ctas % slots;
+  return static_cast<float>(ctas / slots) + (rest > 0 ? 0.35f + 0.65f * static_cast<float>((rest + sms - 1) / sms) / per_sm : 0.f);
+}
 static int scan_chunk_count(int B, int L, int D, int ctas, float light) {
-  const int tiles = (D + SC_CH - 1) / SC_CH * B, blocks = (L + SC_T - 1) / SC_T, slots = ctas * sm_count();
+  const long long tiles = static_cast<long long>((D + SC_CH - 1) / SC_CH) * B;
+  const int blocks = (L + SC_T - 1) / SC_T;
   int best = 1;
   float best_cost = 1e30f;
   for (int nc = 1; nc <= SC_MAX_CHUNKS && nc <= blocks; ++nc) {
     const int len = (blocks + nc - 1) / nc, real = (blocks + len - 1) / len;
     if (real != nc) continue;
-    const int rounds = static_cast<int>((static_cast<long long>(tiles) * nc + slots - 1) / slots);
-    const float cost = len * rounds * (1.f + light * (nc - 1) / nc) + 0.02f * blocks * (nc > 1);
+    // (a tenth of a block to begin a chunk, and its fold of the other chunks' states)
+    float cost = (len + 0.1f + 0.002f * nc) * scan_rounds(tiles * nc, ctas);
+    if (nc > 1) cost += light * (len + 0.1f) * scan_rounds(tiles * (nc - 1), SC_FWD_CTAS);
     if (cost < best_cost) {
       best_cost = cost;
       best = nc;
@@ -868,7 +943,7 @@ static int scan_chunk_count(int B, int L, int D, int ctas, float light) {
   }
   return best;
 }
-constexpr float LIGHT_FWD = 0.6f, LIGHT_BWD = 0.25f;
+constexpr float LIGHT_FWD = 0.7f, LIGHT_BWD = 0.48f;
 
 NX_API int NX_SYM(nx_scan_chunks)(int B, int L, int D, int backward) {
   return scan_chunk_count(B, L, D, backward ? SC_BWD_CTAS : SC_FWD_CTAS, backward ? LIGHT_BWD : LIGHT_FWD);
@@ -880,6 +955,7 @@ static void scan_common(ScanParams& p, int B, int L, int D, int ctas, float ligh
   p.B = B; p.L = L; p.D = D;
   p.NC = scan_chunk_count(B, L, D, ctas, light);
   p.clen = ((L + SC_T - 1) / SC_T + p.NC - 1) / p.NC * SC_T;
+  p.bc_vec = vec_ok(p.Bm, p.bsb, p.bst, 4) && vec_ok(p.Cm, p.csb, p.cst, 4);
 }
 
 // A [D,16] fp32 (negative), Dv [D] fp32 or null, dt_bias [D] fp32; x/dt/z/out bf16 addressed by
@@ -903,8 +979,8 @@ NX_API int NX_SYM(nx_selective_scan_fwd)(const void* x, long long xsb, long long
   p.chunk_state = (float*)chunk_state; p.chunk_sumdt = (float*)chunk_sumdt; p.ckpt = (float*)ckpt;
   if (B <= 0 || L <= 0 || D <= 0) return NX_OK;
   scan_common(p, B, L, D, SC_FWD_CTAS, LIGHT_FWD);
-  const bool vec = D % 8 == 0 && vec_ok(x, xsb, xst, 8) && vec_ok(dt, dsb, dst, 8) && vec_ok(z, zsb, zst, 8) &&
-                   vec_ok(out, osb, ost, 8);
+  const bool vec = D % 2 == 0 && vec_ok(x, xsb, xst, 2) && vec_ok(dt, dsb, dst, 2) && vec_ok(z, zsb, zst, 2) &&
+                   vec_ok(out, osb, ost, 2);
   const dim3 grid((D + SC_CH - 1) / SC_CH, p.NC, B);
   if (p.NC > 1) {
     const dim3 light(grid.x, p.NC - 1, B);
@@ -942,9 +1018,9 @@ NX_API int NX_SYM(nx_selective_scan_bwd)(const void* x, long long xsb, long long
   p.ckpt = (float*)ckpt; p.chunk_state = (float*)chunk_state; p.chunk_sumdt = (float*)chunk_sumdt;
   if (B <= 0 || L <= 0 || D <= 0) return NX_OK;
   scan_common(p, B, L, D, SC_BWD_CTAS, LIGHT_BWD);
-  const bool vec = D % 8 == 0 && vec_ok(x, xsb, xst, 8) && vec_ok(dt, dsb, dst, 8) && vec_ok(z, zsb, zst, 8) &&
-                   vec_ok(dout, gsb, gst, 8) && vec_ok(dx, osb, ost, 8) && vec_ok(ddt, osb, ost, 8) &&
-                   vec_ok(dz, osb, ost, 8);
+  const bool vec = D % 2 == 0 && vec_ok(x, xsb, xst, 2) && vec_ok(dt, dsb, dst, 2) && vec_ok(z, zsb, zst, 2) &&
+                   vec_ok(dout, gsb, gst, 2) && vec_ok(dx, osb, ost, 2) && vec_ok(ddt, osb, ost, 2) &&
+                   vec_ok(dz, osb, ost, 2);
   const dim3 grid((D + SC_CH - 1) / SC_CH, p.NC, B);
   const int smem = (int)sizeof(ScanBwdSmem);
   static bool attr_set = false;
@@ -954,7 +1030,7 @@ NX_API int NX_SYM(nx_selective_scan_bwd)(const void* x, long long xsb, long long
     attr_set = true;
   }
   if (p.NC > 1) {
-    const dim3 light(grid.x, p.NC - 1, B);
+    const dim3 light((D + SC_CH - 1) / SC_CH, p.NC - 1, B);
     if (vec) scan_bwd_local_kernel<true><<<light, SC_THREADS, 0, stream>>>(p);
     else scan_bwd_local_kernel<false><<<light, SC_THREADS, 0, stream>>>(p);
     NX_LAUNCH_CHECK();

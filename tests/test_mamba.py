@@ -154,6 +154,34 @@ def test_selective_scan_blocks_and_chunks(B, L, D, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,L,D,off,use_z", [(1, 1, 1, 0, True), (2, 3, 2, 0, False), (1, 5, 15, 0, True), (2, 32, 17, 1, True),
+                                             (1, 36, 63, 0, False), (3, 65, 66, 1, True), (1, 130, 64, 0, False),
+                                             (1, 997, 129, 0, True)])
+def test_selective_scan_pairs_and_segments(B, L, D, off, use_z, dtype):
+    """Odd channel counts and bases (a quad's second channel dead or read by itself), warps and CTAs with few live channels,
+    segments of four and blocks of 32 that the length cuts, B and C on 8-byte boundaries, one chunk and many, no gate, no D."""
+    from gpt_neox_b200.ops.mamba import selective_scan, selective_scan_reference
+    torch.manual_seed(7)
+    mk = lambda *s: (torch.randn(*s, device="cuda") * 0.5).to(dtype)
+    xz, bc = mk(L, B, 2 * D + off), mk(L, B, 32)
+    x, z, dt = xz[..., off:off + D].transpose(0, 1), xz[..., off + D:].transpose(0, 1), mk(L, B, D).transpose(0, 1)
+    dt = (dt.float() * 8 - 2).to(dtype)          # both branches of the softplus, and steps that forget everything
+    A, dtb = -(torch.rand(D, 16, device="cuda") * 4 + 0.5), torch.randn(D, device="cuda") * 0.5 - 2.0
+    Dp = torch.randn(D, device="cuda") if use_z else None
+    args = [x, dt, A, bc[..., :16].transpose(0, 1), bc[..., 16:].transpose(0, 1), Dp, z if use_z else None, dtb]
+    leaves = [None if t is None else t.detach().requires_grad_(True) for t in args]
+    ref = [None if t is None else t.detach().float().clone().requires_grad_(True) for t in leaves]
+    g = mk(B, L, D)
+    y, yr = selective_scan(*leaves), selective_scan_reference(*ref)
+    got = torch.autograd.grad(y, [t for t in leaves if t is not None], g)
+    want = torch.autograd.grad(yr, [t for t in ref if t is not None], g.float())
+    eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -11
+    for a, r in zip((y,) + got, (yr,) + want):                  # one rounding to 16 bits; fp32 sums on both sides
+        assert (a.float() - r).abs().max().item() <= 2 * eps * r.abs().max().item() + 1e-4
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("what,value", [("x", float("nan")), ("dt", float("nan")), ("B", float("nan")), ("C", float("inf")),
                                         ("z", float("nan")), ("x", float("inf"))])
 @pytest.mark.parametrize("at", [0, 37, 255, 299])
