@@ -63,18 +63,8 @@ struct GemmParams {
   long long ld_aux;
   int flags;
   float alpha;
-  int tiles_m, tiles_n;
+  int tiles_m, tiles_n, total_tiles;
   int* err;
-  // ---- grouped (mixture-of-experts) modes; group_mode == GROUP_NONE leaves them unused
-  //  GROUP_ROWS: the rows of A / C are expert segments aligned to BM; grp_tile_expert[tm] names the expert of
-  //              row tile tm (-1: tile unused); B holds the experts' matrices stacked, grp_b_rows apart.
-  //  GROUP_K   : one output matrix per expert (grp_c_stride apart), reduction over the expert's row segment
-  //              [grp_row_offsets[e], grp_row_offsets[e+1]) of MN-major A and B (weight gradients).
-  int group_mode, total_tiles;
-  const int* grp_tile_expert;
-  const int* grp_row_offsets;
-  int grp_b_rows;
-  long long grp_c_stride;
   // ---- fused collective (tensor-parallel group of `ws` ranks, this rank = `rank`); comm == COMM_NONE
   //      leaves everything below unused
   int comm, rank, ws;
@@ -93,7 +83,6 @@ struct GemmParams {
 };
 
 enum CommMode : int { COMM_NONE = 0, COMM_RS = 1, COMM_AG = 2 };
-enum GroupMode : int { GROUP_NONE = 0, GROUP_ROWS = 1, GROUP_K = 2 };
 
 template <int BN, int STAGES>
 struct SmemLayout {
@@ -103,13 +92,10 @@ struct SmemLayout {
   static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
   // full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2], tmem base word
   static constexpr int RS_OFFSET = BAR_OFFSET + (2 * STAGES + 4) * 8 + 16 + 8 * 8;   // + 8 chunk-ready barriers
-  // the epilogue that stores by TMA: a barrier per epilogue warp, then 2 x 2 KB per warp
-  static constexpr int AUX_BAR_OFFSET = RS_OFFSET;
-  static constexpr int EPI_OFFSET = (AUX_BAR_OFFSET + 8 * 8 + 1023) / 1024 * 1024;
-  static constexpr int TOTAL = RS_OFFSET + RS_STAGE_BYTES, TMA_EPI_TOTAL = EPI_OFFSET + 8 * 4096;
-  static constexpr int dyn_bytes(bool tma_epi) { return (tma_epi ? TMA_EPI_TOTAL : TOTAL) + 1024; }  // slack for manual 1024-byte alignment
+  static constexpr int TOTAL = RS_OFFSET + RS_STAGE_BYTES;
+  static constexpr int DYN_BYTES = TOTAL + 1024;  // slack for manual 1024-byte alignment
 };
-static_assert(SmemLayout<256, 4>::dyn_bytes(true) <= 232448, "shared memory of one SM");
+static_assert(SmemLayout<256, 4>::DYN_BYTES <= 232448, "shared memory of one SM");
 
 __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int& tm, int& tn) {
   // Group 8 row-tiles together so that concurrently running CTAs share B panels in L2.
@@ -140,56 +126,10 @@ __device__ __forceinline__ void tile_coords_p(int tile, const GemmParams& p, int
   tm = chunk * p.tiles_m_chunk + tl;
 }
 
-
-// Grouped modes: expert of the tile and the range of K blocks it reduces over.  Returns false for a tile
-// that has no work (unused row tile / expert without rows); every warp role skips it the same way.
-__device__ __forceinline__ bool group_tile(int tile, const GemmParams& p, int num_kb, int& tm, int& tn, int& chunk,
-                                           int& e, int& kb0, int& kb1) {
-  e = 0;
-  kb0 = 0;
-  kb1 = num_kb;
-  if (p.group_mode == GROUP_K) {
-    const int per = p.tiles_m * p.tiles_n;
-    e = tile / per;
-    chunk = 0;
-    tile_coords(tile - e * per, p.tiles_m, p.tiles_n, tm, tn);
-    kb0 = p.grp_row_offsets[e] / BK;
-    kb1 = p.grp_row_offsets[e + 1] / BK;
-    return kb1 > kb0;
-  }
-  tile_coords_p(tile, p, tm, tn, chunk);
-  if (p.group_mode == GROUP_ROWS) {
-    e = p.grp_tile_expert[tm];
-    return e >= 0;
-  }
-  return true;
-}
-
-// The tensor maps of the epilogue that stores by TMA: the result, aux_out, aux_in (32 x 32 boxes, rows of 64 bytes).
-struct EpiMaps {
-  CUtensorMap out, aux_out, aux_in;
-};
-// Chunk c (16 bytes) of row r of such a box (a swizzle, which would take the bank conflicts away, measured the same).
-__device__ __forceinline__ uint32_t epi_chunk(int r, int c) { return r * 64 + c * 16; }
-__device__ __forceinline__ void epi_put(uint8_t* box, int lane, const float (&v)[32]) {
-#pragma unroll
-  for (int c = 0; c < 4; ++c)
-    *reinterpret_cast<uint4*>(box + epi_chunk(lane, c)) =
-        make_uint4(pack_h16x2(v[8 * c], v[8 * c + 1]), pack_h16x2(v[8 * c + 2], v[8 * c + 3]),
-                   pack_h16x2(v[8 * c + 4], v[8 * c + 5]), pack_h16x2(v[8 * c + 6], v[8 * c + 7]));
-}
-
-// TMA_EPI (grouped rows with more than 128 columns): a warp's 32 x 32 pieces of the result and of the stored derivative
-// leave through shared memory as TMA boxes, and a stored derivative comes in the same way, behind the piece before.  The GEMMs of a
-// short reduction are bound by their epilogue warps, which are bound by latency: what counts is that the 32 values of a lane
-// go through GeLU and derivative side by side, so the activation is chosen once per piece (chosen per value, the values' chains ran
-// one after the other: 3,400 cycles per piece).  Dropless MoE, 32,768 rows, 768 -> 3072: the GEMM with GeLU and derivative
-// 275 -> 176 us, the one that multiplies by the derivative 275 -> 156 us; with the chains one after the other 216 / 203, with
-// pieces transposed in registers instead of boxes 184 / 168; without any epilogue work 110.
-template <int BN, int STAGES, bool A_MN, bool B_MN, bool TMA_EPI>
+template <int BN, int STAGES, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                     const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ EpiMaps em, const GemmParams p) {
+                     const __grid_constant__ CUtensorMap tmA2, const GemmParams p) {
   using L = SmemLayout<BN, STAGES>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -221,8 +161,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       mbar_init(tmem_empty_bar(a), p.comm == COMM_NONE ? 8 : 4);  // one arrival per epilogue warp
     }
     for (int k = 0; k < 8; ++k) mbar_init(ag_bar(k), 4);  // one arrival per push warp
-    if (TMA_EPI)
-      for (int k = 0; k < 8; ++k) mbar_init(smem_base + L::AUX_BAR_OFFSET + 8 * k, 1);
     *ag_abort = 0;
     fence_barrier_init();
   }
@@ -250,11 +188,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       uint32_t phase = 0;
       int ag_ready_chunk = -1;
       for (int tile = blockIdx.x; tile < num_tiles && !aborted; tile += gridDim.x) {
-        int tm, tn, chunk, ge, kb0, kb1;
-        if (!group_tile(tile, p, num_kb, tm, tn, chunk, ge, kb0, kb1)) continue;
+        int tm, tn, chunk;
+        tile_coords_p(tile, p, tm, tn, chunk);
         int m0 = tm * BM;
         const int n0 = tn * BN;
-        const int b_off = p.group_mode == GROUP_ROWS ? ge * p.grp_b_rows : 0;   // expert's block of stacked B
         const CUtensorMap* mapA = &tmA;
         if (p.comm == COMM_AG) {
           if (chunk == p.rank) {
@@ -273,7 +210,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             ag_ready_chunk = chunk;
           }
         }
-        for (int kb = kb0; kb < kb1; ++kb) {
+        for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1, p.err, 1)) {
             aborted = true;
             break;
@@ -290,11 +227,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
               tma_load_2d(a_dst + j * (BK * 128), &tmA, full_bar(stage), m0 + j * 64, k0);
           }
           if constexpr (!B_MN) {
-            tma_load_2d(b_dst, &tmB, full_bar(stage), k0, n0 + b_off);
+            tma_load_2d(b_dst, &tmB, full_bar(stage), k0, n0);
           } else {
 #pragma unroll
             for (int j = 0; j < BN / 64; ++j)
-              tma_load_2d(b_dst + j * (BK * 128), &tmB, full_bar(stage), n0 + j * 64, k0 + b_off);
+              tma_load_2d(b_dst + j * (BK * 128), &tmB, full_bar(stage), n0 + j * 64, k0);
           }
           if (++stage == STAGES) {
             stage = 0;
@@ -318,15 +255,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       int acc = 0;
       uint32_t acc_phase = 0;
       for (int tile = blockIdx.x; tile < num_tiles && !aborted; tile += gridDim.x) {
-        int tm_, tn_, chunk_, ge_, kb0, kb1;
-        if (!group_tile(tile, p, num_kb, tm_, tn_, chunk_, ge_, kb0, kb1)) continue;
         if (!mbar_wait(tmem_empty_bar(acc), acc_phase ^ 1, p.err, 2)) {
           aborted = true;
           break;
         }
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = kb0; kb < kb1; ++kb) {
+        for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(full_bar(stage), phase, p.err, 3)) {
             aborted = true;
             break;
@@ -338,7 +273,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
           for (int k = 0; k < BK / UMMA_K; ++k) {
             const uint64_t adesc = umma_smem_desc_sw128(a_addr + k * A_KADV, A_LBO, 1024);
             const uint64_t bdesc = umma_smem_desc_sw128(b_addr + k * B_KADV, B_LBO, 1024);
-            umma_bf16_ss(d_tmem, adesc, bdesc, idesc, ((kb - kb0) | k) != 0 ? 1u : 0u);
+            umma_bf16_ss(d_tmem, adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u);
           }
           umma_commit(empty_bar(stage));  // frees the smem slot once these MMAs retire
           if (++stage == STAGES) {
@@ -354,155 +289,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         }
       }
     }
-  } else if constexpr (TMA_EPI) {
-    const int w = warp - 2, quad = warp & 3;
-    const int c_begin = w < 4 ? 0 : BN / 64, c_end = w < 4 ? BN / 64 : BN / 32;
-    const uint32_t aux_bar = smem_base + L::AUX_BAR_OFFSET + 8 * w;
-    uint8_t* out_box = smem_gen + L::EPI_OFFSET + w * 4096;
-    uint8_t* aux_box = out_box + 2048;
-    const int flags = p.flags;
-    const bool aux_in = flags & (EPI_DGELU_ERF | EPI_DGELU_TANH | EPI_MUL_AUX);
-    int acc = 0, tm = 0, tn = 0, chunk, ge, kb0_, kb1_;
-    uint32_t acc_phase = 0, aux_phase = 0;
-    int tile = static_cast<int>(blockIdx.x) - static_cast<int>(gridDim.x);
-    auto next_tile = [&](int t, int& m, int& n) {      // the next tile with work after t
-      do {
-        t += gridDim.x;
-      } while (t < num_tiles && !group_tile(t, p, num_kb, m, n, chunk, ge, kb0_, kb1_));
-      return t;
-    };
-    auto fetch_aux = [&](int m, int n, int c) {
-      if (lane == 0) {
-        mbar_expect_tx(aux_bar, 2048);
-        tma_load_2d(smem_u32(aux_box), &em.aux_in, aux_bar, n * BN + c * 32, m * BM + quad * 32);
-      }
-    };
-    tile = next_tile(tile, tm, tn);
-    bool fetched = false;      // the piece that comes next is on its way
-    while (tile < num_tiles && !aborted) {
-      const int m0 = tm * BM, n0 = tn * BN;
-      int tm_nx = 0, tn_nx = 0;
-      const int tile_nx = next_tile(tile, tm_nx, tn_nx);
-      bool ok = mbar_wait(tmem_full_bar(acc), acc_phase, p.err, 4);
-      if (!__all_sync(0xffffffffu, ok)) {
-        aborted = true;
-        break;
-      }
-      tc_fence_after_sync();
-#pragma unroll 1
-      for (int c = c_begin; c < c_end; ++c) {
-        const int col0 = n0 + c * 32;
-        if (col0 >= p.N) break;  // warp-uniform
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(tmem_base + acc * BN + c * 32 + (static_cast<uint32_t>(quad * 32) << 16), r);
-        tmem_ld_wait();
-        float v[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-        bool next_here = false;
-        if (aux_in) {
-          if (!fetched) fetch_aux(tm, tn, c);
-          ok = mbar_wait(aux_bar, aux_phase, p.err, 9);
-          if (!__all_sync(0xffffffffu, ok)) {
-            aborted = true;
-            break;
-          }
-          aux_phase ^= 1;
-          uint32_t x[16];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const uint4 u = *reinterpret_cast<const uint4*>(aux_box + epi_chunk(lane, k));
-            x[4 * k] = u.x; x[4 * k + 1] = u.y; x[4 * k + 2] = u.z; x[4 * k + 3] = u.w;
-          }
-          // the next piece: of this tile, or the first of the next
-          const bool here = c + 1 < c_end && col0 + 32 < p.N;
-          fetched = here || (tile_nx < num_tiles && tn_nx * BN + c_begin * 32 < p.N);
-          next_here = here;
-          auto times = [&](auto f) {
-#pragma unroll
-            for (int k = 0; k < 16; ++k) {
-              const float2 a = unpack_h16x2(x[k]);
-              v[2 * k] *= f(a.x);
-              v[2 * k + 1] *= f(a.y);
-            }
-          };
-          if (flags & EPI_MUL_AUX) times([](float a) { return a; });
-          else if (flags & EPI_DGELU_ERF) times([](float a) { return gelu_erf_grad(a); });
-          else times([](float a) { return gelu_tanh_grad(a); });
-        }
-        const bool aux_out = flags & EPI_AUX_OUT;
-        if (flags & EPI_AUX_DERIV) {
-          float d[32];
-          if (flags & EPI_GELU_TANH) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) gelu_tanh_both(v[j], v[j], d[j]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; j += 2) gelu_erf_both2(v[j], v[j + 1], d[j], d[j + 1]);
-          }
-          if (aux_out) {
-            if (lane == 0) tma_store_wait_read<1>();      // (all but the last store have left their boxes)
-            __syncwarp();
-            epi_put(aux_box, lane, d);
-          }
-        } else if (aux_out) {
-          if (lane == 0) tma_store_wait_read<1>();
-          __syncwarp();
-          epi_put(aux_box, lane, v);
-        }
-        if (aux_out) {
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            tma_store_2d(&em.aux_out, smem_u32(aux_box), col0, m0 + quad * 32);
-            tma_store_commit();
-          }
-        }
-        if (!(flags & EPI_AUX_DERIV)) {
-          if (flags & EPI_GELU_ERF) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = gelu_erf(v[j]);
-          } else if (flags & EPI_GELU_TANH) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = gelu_tanh(v[j]);
-          }
-        }
-        if (lane == 0) {
-          if (aux_out) tma_store_wait_read<1>();
-          else tma_store_wait_read<0>();
-        }
-        __syncwarp();
-        epi_put(out_box, lane, v);
-        fence_proxy_async_smem();
-        __syncwarp();
-        // The side operand's next piece comes in over this one: the results made of this one are laid down, and the fence above
-        // orders the loads, too, before the copy, which belongs to another proxy.  (A barrier alone, of the warp or an mbarrier
-        // that every lane arrives on, orders ordinary accesses; a copy behind one overtook loads that were still queued behind
-        // the other warps', and 1 % of a gradient was wrong.)
-        if (aux_in && fetched) fetch_aux(next_here ? tm : tm_nx, next_here ? tn : tn_nx, next_here ? c + 1 : c_begin);
-        if (lane == 0) {
-          tma_store_2d(&em.out, smem_u32(out_box), col0, m0 + quad * 32);
-          tma_store_commit();
-        }
-      }
-      // This warp is done reading the accumulator: hand it back to the MMA issuer.
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(tmem_empty_bar(acc));
-      if (++acc == 2) {
-        acc = 0;
-        acc_phase ^= 1;
-      }
-      tile = tile_nx;
-      tm = tm_nx;
-      tn = tn_nx;
-    }
-    if (lane == 0) tma_store_wait_read<0>();      // shared memory outlives its last reader
   } else if (warp < 6 || p.comm == COMM_NONE) {
     // ------------------------------------------------------------------ epilogue (warps 2..5; without a collective
     // warps 6..9 too, each pair of warps of a lane quadrant taking half of the tile's columns: with four warps the
-    // GeLU and its derivative, or the loads of a stored derivative, took longer than the MMAs of a short reduction:
-    // dropless-MoE layer of 16384 tokens, 768 -> 3072, forward + backward 1454 -> 1341 us)
+    // GeLU and its derivative, or the loads of a stored derivative, took longer than the MMAs of a short reduction)
     const int quad = warp & 3;  // TMEM lane quadrant this warp may access
     const int c_begin = p.comm == COMM_NONE && warp >= 6 ? BN / 64 : 0;
     const int c_end = p.comm == COMM_NONE && warp < 6 ? BN / 64 : BN / 32;
@@ -512,10 +302,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     const int flags = p.flags;
     const long long chunk_rows = static_cast<long long>(p.tiles_m_chunk) * BM;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-      int tm, tn, chunk, ge, kb0_, kb1_;
-      if (!group_tile(tile, p, num_kb, tm, tn, chunk, ge, kb0_, kb1_)) continue;
+      int tm, tn, chunk;
+      tile_coords_p(tile, p, tm, tn, chunk);
       const int m0 = tm * BM, n0 = tn * BN;
-      const long long c_off = p.group_mode == GROUP_K ? ge * p.grp_c_stride : 0;
       if (!mbar_wait(tmem_full_bar(acc), acc_phase, p.err, 4)) {
         aborted = true;
         break;
@@ -705,7 +494,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
               }
             }
           } else if (flags & EPI_OUT_F32) {
-            float* cp = reinterpret_cast<float*>(p.C) + c_off + row * p.ldc + col0;
+            float* cp = reinterpret_cast<float*>(p.C) + row * p.ldc + col0;
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
               if (col0 + j < p.N) {
@@ -718,7 +507,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
               }
             }
           } else {
-            h16* cp = reinterpret_cast<h16*>(p.C) + c_off + row * p.ldc + col0;
+            h16* cp = reinterpret_cast<h16*>(p.C) + row * p.ldc + col0;
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
               if (col0 + j < p.N) {
@@ -824,38 +613,30 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   }
 }
 
-template <int BN, int STAGES, bool A_MN, bool B_MN, bool TMA_EPI = false>
-static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmA2, const EpiMaps& em,
-                       const GemmParams& p, cudaStream_t stream) {
+template <int BN, int STAGES, bool A_MN, bool B_MN>
+static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmA2, const GemmParams& p,
+                       cudaStream_t stream) {
   using L = SmemLayout<BN, STAGES>;
-  auto kern = gemm_bf16_kernel<BN, STAGES, A_MN, B_MN, TMA_EPI>;
+  auto kern = gemm_bf16_kernel<BN, STAGES, A_MN, B_MN>;
   static bool configured = false;
   if (!configured) {
-    NX_CUDA_CHECK(
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::dyn_bytes(TMA_EPI)));
+    NX_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::DYN_BYTES));
     configured = true;
   }
   const int tiles = p.total_tiles;
   const int grid = tiles < sm_count() ? tiles : sm_count();
-  kern<<<grid, GEMM_THREADS, L::dyn_bytes(TMA_EPI), stream>>>(tmA, tmB, tmA2, em, p);
+  kern<<<grid, GEMM_THREADS, L::DYN_BYTES, stream>>>(tmA, tmB, tmA2, p);
   NX_LAUNCH_CHECK();
   return NX_OK;
 }
 
 template <int BN, int STAGES>
 static int dispatch_layout(int transA, int transB, const CUtensorMap& tmA, const CUtensorMap& tmB,
-                           const CUtensorMap& tmA2, const EpiMaps& em, bool tma_epi, const GemmParams& p,
-                           cudaStream_t stream) {
-  if constexpr (BN == 256) {
-    if (tma_epi) {
-      if (!transB) return launch_gemm<BN, STAGES, false, false, true>(tmA, tmB, tmA2, em, p, stream);
-      return launch_gemm<BN, STAGES, false, true, true>(tmA, tmB, tmA2, em, p, stream);
-    }
-  }
-  if (!transA && !transB) return launch_gemm<BN, STAGES, false, false>(tmA, tmB, tmA2, em, p, stream);
-  if (!transA && transB) return launch_gemm<BN, STAGES, false, true>(tmA, tmB, tmA2, em, p, stream);
-  if (transA && !transB) return launch_gemm<BN, STAGES, true, false>(tmA, tmB, tmA2, em, p, stream);
-  return launch_gemm<BN, STAGES, true, true>(tmA, tmB, tmA2, em, p, stream);
+                           const CUtensorMap& tmA2, const GemmParams& p, cudaStream_t stream) {
+  if (!transA && !transB) return launch_gemm<BN, STAGES, false, false>(tmA, tmB, tmA2, p, stream);
+  if (!transA && transB) return launch_gemm<BN, STAGES, false, true>(tmA, tmB, tmA2, p, stream);
+  if (transA && !transB) return launch_gemm<BN, STAGES, true, false>(tmA, tmB, tmA2, p, stream);
+  return launch_gemm<BN, STAGES, true, true>(tmA, tmB, tmA2, p, stream);
 }
 
 }  // namespace nx
@@ -869,11 +650,6 @@ struct CommArgs {
   long long ld_res2 = 0;
   const void* ag_src = nullptr;
   long long ag_ld = 0;
-  // grouped (mixture-of-experts) modes
-  int group_mode = 0, experts = 1;
-  const int* tile_expert = nullptr;
-  const int* row_offsets = nullptr;
-  long long c_stride = 0;
   bool skinny = false;   // few rows: gemm_skinny_tcgen05.cu
 };
 
@@ -966,9 +742,8 @@ static int gemm_common(const void* A, const void* B, void* C, int M, int N, int 
   if (!transA) ok = make_tma_2d(&tmA, A, M, K, lda * 2, BM, BK, 2);
   else         ok = make_tma_2d(&tmA, A, K, M, lda * 2, BK, 64, 2);
   if (!ok) return NX_ERR_ARG;
-  const long long eb = ca.group_mode == GROUP_ROWS ? ca.experts : 1;    // stacked expert matrices
-  if (!transB) ok = make_tma_2d(&tmB, B, eb * N, K, ldb * 2, BN, BK, 2);
-  else         ok = make_tma_2d(&tmB, B, eb * K, N, ldb * 2, BK, 64, 2);
+  if (!transB) ok = make_tma_2d(&tmB, B, N, K, ldb * 2, BN, BK, 2);
+  else         ok = make_tma_2d(&tmB, B, K, N, ldb * 2, BK, 64, 2);
   if (!ok) return NX_ERR_ARG;
   tmA2 = tmA;
   if (ca.mode == COMM_AG) {
@@ -986,35 +761,9 @@ static int gemm_common(const void* A, const void* B, void* C, int M, int N, int 
   p.tiles_m = (M + BM - 1) / BM;
   p.tiles_n = (N + BN - 1) / BN;
   p.total_tiles = p.tiles_m * p.tiles_n;
-  p.group_mode = ca.group_mode;
-  if (ca.group_mode == GROUP_ROWS) {
-    NX_REQUIRE(!transA && ca.mode == COMM_NONE && ca.tile_expert != nullptr && M % BM == 0,
-               "gemm_grouped: row mode needs row-major A, a tile->expert table and M %% %d == 0", BM);
-    p.grp_tile_expert = ca.tile_expert;
-    p.grp_b_rows = transB ? K : N;
-  } else if (ca.group_mode == GROUP_K) {
-    NX_REQUIRE(transA && transB && ca.mode == COMM_NONE && ca.row_offsets != nullptr,
-               "gemm_grouped: reduction mode needs MN-major A and B and the experts' row offsets");
-    p.grp_row_offsets = ca.row_offsets;
-    p.grp_c_stride = ca.c_stride;
-    p.total_tiles = p.tiles_m * p.tiles_n * ca.experts;
-  }
   p.err = device_error_word();
-  // (the other epilogues of grouped rows, which nothing here asks for, stay with the general kernel)
-  constexpr int aux_in_flags = EPI_DGELU_ERF | EPI_DGELU_TANH | EPI_MUL_AUX;
-  constexpr int tma_flags = EPI_GELU_ERF | EPI_GELU_TANH | EPI_AUX_OUT | EPI_AUX_DERIV | aux_in_flags;
-  const bool tma_epi = BN == 256 && ca.group_mode == GROUP_ROWS && (flags & ~tma_flags) == 0 &&
-                       !((flags & EPI_AUX_OUT) && (flags & aux_in_flags));
-  EpiMaps em;
-  memset(&em, 0, sizeof(em));
-  if (tma_epi) {
-    ok = make_tma_2d(&em.out, C, M, N, ldc * 2, 32, 32, 2, false);
-    if (flags & EPI_AUX_OUT) ok = ok && make_tma_2d(&em.aux_out, aux_out, M, N, ld_aux * 2, 32, 32, 2, false);
-    if (flags & aux_in_flags) ok = ok && make_tma_2d(&em.aux_in, aux_in, M, N, ld_aux * 2, 32, 32, 2, false);
-    if (!ok) return NX_ERR_ARG;
-  }
-  if (BN == 128) return dispatch_layout<128, 6>(transA, transB, tmA, tmB, tmA2, em, tma_epi, p, stream);
-  return dispatch_layout<256, 4>(transA, transB, tmA, tmB, tmA2, em, tma_epi, p, stream);
+  if (BN == 128) return dispatch_layout<128, 6>(transA, transB, tmA, tmB, tmA2, p, stream);
+  return dispatch_layout<256, 4>(transA, transB, tmA, tmB, tmA2, p, stream);
 }
 
 // C[M,N] = epilogue(op(A) * op(B)).  Leading dimensions in elements.  bias/aux/residual may be
@@ -1028,25 +777,6 @@ NX_API int NX_SYM(nx_gemm_bf16)(const void* A, const void* B, void* C, int M, in
   ca.skinny = skinny_better(M, N, K, transA, transB, flags);
   return gemm_common(A, B, C, M, N, K, lda, ldb, ldc, transA, transB, bias, aux_in, aux_out, residual, ld_aux,
                      flags, alpha, ca, static_cast<cudaStream_t>(stream_));
-}
-
-// Grouped GEMMs over expert row segments that are aligned to 128 rows (the layout the MoE permute kernel
-// writes).  mode 1: C[rows, N] = A[rows, K] * op(B_e) with B the experts' matrices stacked ([E*N, K] for
-// transB = 0, [E*K, N] for transB = 1) and tile_expert[row tile] -> expert (or -1).  mode 2: per-expert
-// weight gradient C_e[M, N] (+)= A[rows_e, M]^T * B[rows_e, N], rows_e = [row_offsets[e], row_offsets[e+1]);
-// C_e = C + e * c_stride; experts without rows are left untouched.  All tables live on the device: no host
-// synchronisation on the routing result.
-NX_API int NX_SYM(nx_gemm_bf16_grouped)(int mode, const void* A, const void* B, void* C, int M, int N, int K, long long lda,
-                                long long ldb, long long ldc, int transB, int experts, const void* tile_expert,
-                                const void* row_offsets, long long c_stride, const void* aux_in, void* aux_out,
-                                long long ld_aux, int flags, void* stream_) {
-  CommArgs ca;
-  ca.group_mode = mode; ca.experts = experts;
-  ca.tile_expert = static_cast<const int*>(tile_expert);
-  ca.row_offsets = static_cast<const int*>(row_offsets);
-  ca.c_stride = c_stride;
-  return gemm_common(A, B, C, M, N, K, lda, ldb, ldc, mode == 2 ? 1 : 0, mode == 2 ? 1 : transB, nullptr, aux_in,
-                     aux_out, nullptr, ld_aux, flags, 1.0f, ca, static_cast<cudaStream_t>(stream_));
 }
 
 // Number of CTAs the GEMM of this shape launches (the all-gather mode's flag count per source rank).

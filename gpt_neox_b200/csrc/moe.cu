@@ -3,10 +3,12 @@
 //
 // Given the top-k expert ids of T tokens (C = T*k routed copies) the plan kernels produce a *padded
 // permuted layout*: the copies of expert e occupy rows [offsets[e], offsets[e] + counts[e]) of a matrix
-// whose expert segments start at multiples of 128 rows, in the original (token, slot) order (a stable
-// counting sort).  Segment alignment means a 128-row GEMM tile never straddles two experts, so the
-// grouped GEMM (csrc/gemm_tcgen05.cu, GROUP_ROWS / GROUP_K) needs only a tile -> expert table, and the
-// padding rows are zero so weight-gradient reductions over a segment are exact.
+// whose expert segments start at multiples of 256 rows, in the original (token, slot) order (a stable
+// counting sort).  Segment alignment means a 256-row GEMM tile never straddles two experts, so the grouped
+// GEMM (csrc/gemm2_grouped_tcgen05.cu) needs only a table of the expert of every 128 rows, and the padding
+// rows are zero so weight-gradient reductions over a segment are exact.  (Segments of 128-row multiples, with
+// GEMMs of 128-row tiles, hold half the padding, at most 127 rows per expert; their GEMMs were slower at every
+// size, see there.)
 //
 // Counterparts in the reference: megablocks ops.sort / histogram / inclusive_cumsum / gather / scatter
 // called at megatron/model/moe.py:62-83,128,153.
@@ -17,7 +19,7 @@ namespace nx {
 
 constexpr int MOE_BLOCK = 1024;
 constexpr int MOE_MAX_E = 256;
-constexpr int MOE_ALIGN = 128;
+constexpr int MOE_ALIGN = 256, MOE_TILE = 128;         // MOE_TILE: rows per entry of tile_expert
 
 // hist[b][e] = number of copies of expert e among copies [b*1024, (b+1)*1024)
 __global__ void __launch_bounds__(MOE_BLOCK)
@@ -32,7 +34,7 @@ moe_hist_kernel(const long long* __restrict__ expert, int C, int E, int* __restr
 }
 
 // One block.  base[b][e] = copies of expert e in earlier blocks; counts[e]; offsets[e] (segment starts,
-// multiples of 128, offsets[E] = padded total); tile_expert[t] for every 128-row tile (-1 past the end).
+// multiples of 256, offsets[E] = padded total); tile_expert[t] for every 128 rows (-1 past the end).
 __global__ void __launch_bounds__(MOE_MAX_E)
 moe_plan_kernel(const int* __restrict__ hist, int nblk, int E, int* __restrict__ base, int* __restrict__ counts,
                 int* __restrict__ offsets, int* __restrict__ tile_expert, int max_tiles) {
@@ -59,8 +61,8 @@ moe_plan_kernel(const int* __restrict__ hist, int nblk, int E, int* __restrict__
   __syncthreads();
   for (int i = threadIdx.x; i <= E; i += MOE_MAX_E) offsets[i] = off[i];
   if (e < E)
-    for (int t = off[e] / MOE_ALIGN; t < off[e + 1] / MOE_ALIGN; ++t) tile_expert[t] = e;
-  for (int t = off[E] / MOE_ALIGN + threadIdx.x; t < max_tiles; t += MOE_MAX_E) tile_expert[t] = -1;
+    for (int t = off[e] / MOE_TILE; t < off[e + 1] / MOE_TILE; ++t) tile_expert[t] = e;
+  for (int t = off[E] / MOE_TILE + threadIdx.x; t < max_tiles; t += MOE_MAX_E) tile_expert[t] = -1;
 }
 
 // dest_row[c] = offsets[e] + base[block][e] + (copies of e earlier in this block); src_copy[dest] = c.
@@ -197,7 +199,7 @@ NX_API int NX_SYM(nx_moe_plan)(const void* expert, int C, int E, void* hist, voi
   moe_hist_kernel<<<nblk, MOE_BLOCK, 0, stream>>>((const long long*)expert, C, E, (int*)hist);
   NX_LAUNCH_CHECK();
   moe_plan_kernel<<<1, MOE_MAX_E, 0, stream>>>((const int*)hist, nblk, E, (int*)base, (int*)counts, (int*)offsets,
-                                               (int*)tile_expert, max_rows / MOE_ALIGN);
+                                               (int*)tile_expert, max_rows / MOE_TILE);
   NX_LAUNCH_CHECK();
   moe_rank_kernel<<<nblk, MOE_BLOCK, sizeof(int) * 32 * E, stream>>>((const long long*)expert, C, E, (const int*)base,
                                                                      (const int*)offsets, (int*)dest_row, (int*)src_copy);

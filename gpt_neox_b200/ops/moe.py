@@ -1,8 +1,8 @@
 """Dropless MoE expert computation on the device: routing plan -> padded permutation -> grouped tcgen05
-GEMMs -> weighted combine (csrc/moe.cu, csrc/gemm_tcgen05.cu grouped modes).
+GEMMs -> weighted combine (csrc/moe.cu, csrc/gemm2_grouped_tcgen05.cu).
 
 Nothing in the layer reads the routing result on the host: buffer sizes are the static worst case
-(``tokens * k + experts * 127`` rows, rounded to 128) and the kernels skip the unused tail by consulting
+(``tokens * k + experts * 255`` rows, rounded to 256) and the kernels skip the unused tail by consulting
 device-side tables.  Reference path: megatron/model/moe.py:62-160 (megablocks sort / gather / scatter) and
 megatron/model/moe_mlp.py:212-223 (grouped_gemm, which needs the per-expert batch sizes on the CPU).
 """
@@ -100,7 +100,7 @@ def grouped_wgrad(a, b, plan: Plan, weight):
     if mg is not None and mg.dtype == torch.float32:
         out, flags, ret = mg, EPI_ACCUM | EPI_OUT_F32, None
     else:
-        out = torch.zeros((plan.E * M, N), device=a.device, dtype=a.dtype)
+        out = torch.empty((plan.E * M, N), device=a.device, dtype=a.dtype)      # (zeros for an expert without rows)
         flags, ret = 0, out
     LAUNCHES["n"] += 1
     _lib.check(_lib.lib(a).nx_gemm_bf16_grouped(2, _lib.ptr(a), _lib.ptr(b), _lib.ptr(out), M, N, a.shape[0], a.stride(0),

@@ -218,3 +218,48 @@ def test_grouped_rows_read_their_side_operand_before_the_next_piece(T, n, K, kin
         z = xp[r].double() @ w.view(E, n, K)[e].double().t()
         err = (first[r] - z * d).abs() - 2 ** -8 * (z * d).abs()
         assert err.max() <= (2 ** -7 if kind == "tanh" else 2 ** -16) * z.abs().max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,E,M,N", [(40, 5, 8, 8), (300, 3, 264, 520), (700, 4, 40, 24), (1500, 2, 512, 256), (260, 9, 1000, 136)])
+def test_grouped_gemms_at_tile_edges(T, E, M, N, dtype):
+    """Row and reduction form against 64 bits at sizes that tiles of 256, pieces of 64 and 32 and 32-byte stores cut, with an
+    expert that gets no token: the operand sums are fp32 and rounded once.  Weight gradients: zeros for that expert, and with
+    an fp32 main_grad the sum with what was there."""
+    from gpt_neox_b200.ops import moe as MO
+    torch.manual_seed(7)
+    idx = torch.randint(0, E - 1, (T, 2), device="cuda")                 # the last expert has no rows
+    idx[idx == 0] = 0 if E < 4 else 1                                    # and with four or more the first one, too
+    plan = MO.Plan(idx, E)
+    rows = (plan.src_copy >= 0).nonzero().flatten()
+    expert = plan.tile_expert.long()[rows // 128]
+    mk = lambda *s: torch.randn(*s, device="cuda").to(dtype)
+    a, b = MO.gather_rows(mk(T, M), plan), MO.gather_rows(mk(T, N), plan)
+    eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -11
+
+    def slack(terms):
+        # the tensor core adds 16 products at a time to an fp32 sum, which it cuts off: terms / 16 steps of at most 2^-22 of a
+        # partial sum, which stays below 8 sqrt(terms) for products of order 1 (a bound of terms * 2^-22, as if partial sums
+        # were of order 1, was too small for 3000 terms: 8e-4 at a sum of 122)
+        return (terms / 16 + 1) * 8 * terms ** 0.5 * 2 ** -22
+
+    def close(got, want, terms):
+        assert ((got.double() - want).abs() <= eps * want.abs() + slack(terms)).all()       # one rounding to 16 bits
+
+    w, wt = mk(E * N, M), mk(E * M, N)
+    got = MO.grouped_gemm_rows(a, w, plan, N, trans_b=False)
+    close(got[rows], torch.einsum("rk,rnk->rn", a[rows].double(), w.view(E, N, M).double()[expert]), M)
+    got = MO.grouped_gemm_rows(a, wt, plan, N, trans_b=True)
+    close(got[rows], torch.einsum("rk,rkn->rn", a[rows].double(), wt.view(E, M, N).double()[expert]), M)
+    want = torch.stack([a[rows][expert == e].double().t() @ b[rows][expert == e].double() for e in range(E)])
+    weight = torch.nn.Parameter(torch.empty(E * M, N, device="cuda", dtype=dtype))
+    got = MO.grouped_wgrad(a, b, plan, weight).view(E, M, N)
+    close(got, want, 2 * T)
+    assert bool((got[E - 1] == 0).all())
+    before = torch.randn(E, M, N, device="cuda")
+    weight.main_grad = before.clone().view(E * M, N)
+    assert MO.grouped_wgrad(a, b, plan, weight) is None
+    got = weight.main_grad.view(E, M, N)
+    assert ((got.double() - before.double() - want).abs() <= slack(2 * T) + 2 ** -23 * got.abs()).all()
+    assert torch.equal(got[E - 1], before[E - 1])
