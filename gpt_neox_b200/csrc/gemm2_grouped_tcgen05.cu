@@ -72,35 +72,6 @@ struct Tile {
 
 // Chunk c (16 bytes) of row r of a box, in the 128-byte swizzle of its tensor map: a warp's 16-byte stores do not collide.
 __device__ __forceinline__ uint32_t box_chunk(int r, int c) { return r * 128 + ((c ^ (r & 7)) * 16); }
-__device__ __forceinline__ uint4 pack8(const float* v) {
-  return make_uint4(pack_h16x2(v[0], v[1]), pack_h16x2(v[2], v[3]), pack_h16x2(v[4], v[5]), pack_h16x2(v[6], v[7]));
-}
-
-// 16 neighbouring values of a row, of which the first `left` (a multiple of 8) are the matrix's: one access of a whole
-// 32-byte sector where `wide`.
-__device__ __forceinline__ void store16(h16* p, const uint4& a, const uint4& b, int left, bool wide) {
-  if (wide && left >= 16) {
-    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
-                 "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
-                 : "memory");
-    return;
-  }
-  if (left >= 8) *reinterpret_cast<uint4*>(p) = a;
-  if (left >= 16) *reinterpret_cast<uint4*>(p + 8) = b;
-}
-__device__ __forceinline__ void load16(const h16* p, uint4& a, uint4& b, int left, bool wide) {
-  if (wide && left >= 16) {
-    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
-                 : "l"(p)
-                 : "memory");
-    return;
-  }
-  a = b = make_uint4(0u, 0u, 0u, 0u);
-  if (left >= 8) a = *reinterpret_cast<const uint4*>(p);
-  if (left >= 16) b = *reinterpret_cast<const uint4*>(p + 8);
-}
-
 // The pair's tile of round r; false past the last one.  REDUCE: the experts in `order`, the longest reductions first, and every
 // other round backwards, so that the pairs' sums of different lengths come out nearly the same.
 template <bool REDUCE>
@@ -341,17 +312,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         }
         const long long at = (REDUCE ? t.e * p.c_stride : 0) + row * p.ldc + col0 + 32 * h;
         if (REDUCE && (flags & OUT_F32)) {
-          float* cp = static_cast<float*>(p.C) + at;
-#pragma unroll
-          for (int j = 0; j < 32; j += 4)
-            if (j < rest) {
-              float4 o = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-              if (flags & ACCUM) {
-                const float4 old = *reinterpret_cast<const float4*>(cp + j);
-                o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-              }
-              *reinterpret_cast<float4*>(cp + j) = o;
-            }
+          put_f32(static_cast<float*>(p.C) + at, v, rest, flags & ACCUM, p.wide);
         } else {
           h16* cp = static_cast<h16*>(p.C) + at;
 #pragma unroll
@@ -622,7 +583,8 @@ NX_API int NX_SYM(nx_gemm_bf16_grouped)(int mode, const void* A, const void* B, 
   p.M = M; p.N = N; p.K = K;
   p.C = C; p.ldc = ldc; p.c_stride = c_stride;
   p.flags = flags;
-  p.wide = (reinterpret_cast<uintptr_t>(C) & 31) == 0 && ldc % 16 == 0 && c_stride % 16 == 0;
+  p.wide = (reinterpret_cast<uintptr_t>(C) & 31) == 0 && ldc % (flags & OUT_F32 ? 8 : 16) == 0 &&
+           c_stride % (flags & OUT_F32 ? 8 : 16) == 0;
   p.tiles_m = (M + 2 * BM - 1) / (2 * BM);
   p.tiles_n = (N + BN - 1) / BN;
   p.experts = experts;

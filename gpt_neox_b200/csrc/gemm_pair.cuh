@@ -19,11 +19,8 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// The same for an accumulator that has been read (after tcgen05.wait::ld and tc_fence_before_sync): no memory that the warp
-// wrote is handed over, so nothing waits for its stores, which a release to the cluster does.
+// Arrival for an accumulator that has been read (after tcgen05.wait::ld and tc_fence_before_sync): no memory that the warp
+// wrote is handed over, so nothing waits for its stores, as a release to the cluster would.
 __device__ __forceinline__ void mbar_arrive_cluster_read(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -75,6 +72,26 @@ __device__ __forceinline__ void tile_coords2(int tile, int tiles_m, int tiles_n,
   const int r = tile - g * per_group;
   tm = first_m + (r % gsize);
   tn = r / gsize;
+}
+
+// 32 columns of an fp32 row (N is a multiple of 8), set or added to.
+__device__ __forceinline__ void put_f32(float* p, const float (&v)[32], int left, bool add, bool wide) {
+#pragma unroll
+  for (int j = 0; j < 32; j += 8)
+    if (j < left) {
+      h16* at = reinterpret_cast<h16*>(p + j);
+      float o[8] = {v[j], v[j + 1], v[j + 2], v[j + 3], v[j + 4], v[j + 5], v[j + 6], v[j + 7]};
+      uint4 a, b;
+      if (add) {
+        load16(at, a, b, 16, wide);
+        const uint32_t old[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int k = 0; k < 8; ++k) o[k] += __uint_as_float(old[k]);
+      }
+      a = make_uint4(__float_as_uint(o[0]), __float_as_uint(o[1]), __float_as_uint(o[2]), __float_as_uint(o[3]));
+      b = make_uint4(__float_as_uint(o[4]), __float_as_uint(o[5]), __float_as_uint(o[6]), __float_as_uint(o[7]));
+      store16(at, a, b, 16, wide);
+    }
 }
 
 }  // namespace g2

@@ -611,4 +611,33 @@ __device__ __forceinline__ float h16_to_float(h16 x) { return __bfloat162float(x
 __device__ __forceinline__ h16 float_to_h16(float x) { return __float2bfloat16(x); }
 #endif
 
+__device__ __forceinline__ uint4 pack8(const float* v) {
+  return make_uint4(pack_h16x2(v[0], v[1]), pack_h16x2(v[2], v[3]), pack_h16x2(v[4], v[5]), pack_h16x2(v[6], v[7]));
+}
+
+// 16 neighbouring values of a row, of which the first `left` (a multiple of 8) are the matrix's: one access of a whole
+// 32-byte sector where `wide`.
+__device__ __forceinline__ void store16(h16* p, const uint4& a, const uint4& b, int left, bool wide) {
+  if (wide && left >= 16) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
+                 "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
+    return;
+  }
+  if (left >= 8) *reinterpret_cast<uint4*>(p) = a;
+  if (left >= 16) *reinterpret_cast<uint4*>(p + 8) = b;
+}
+__device__ __forceinline__ void load16(const h16* p, uint4& a, uint4& b, int left, bool wide) {
+  if (wide && left >= 16) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                 : "l"(p)
+                 : "memory");
+    return;
+  }
+  a = b = make_uint4(0u, 0u, 0u, 0u);
+  if (left >= 8) a = *reinterpret_cast<const uint4*>(p);
+  if (left >= 16) b = *reinterpret_cast<const uint4*>(p + 8);
+}
+
 }  // namespace nx

@@ -970,3 +970,43 @@ def test_dependent_launches_see_what_the_kernel_before_wrote(rows, h, f, capture
                 outs = chain(lambda: None)
             for got, r in zip(outs, ref):
                 assert torch.equal(got, r)
+
+
+@pytest.mark.parametrize("wide", [False, True], ids=["16bit", "fp32"])
+@pytest.mark.parametrize("M,N,off,pad", [(256, 256, 0, 0), (300, 264, 0, 8), (513, 520, 8, 0), (700, 272, 8, 16), (260, 776, 0, 4)])
+def test_pair_gemm_rows_on_16_and_32_byte_boundaries(M, N, off, pad, wide):
+    """Result, side operands and sums whose rows start on 32-byte boundaries and on 16-byte ones only (a base or a leading
+    dimension that is no multiple of 32 bytes), at column counts that cut tiles of 256 and pieces of 32 and 16: the fp32
+    product of 64 terms of order 1 (sums 2 ** -18 off at most), rounded once per 16-bit step."""
+    from gpt_neox_b200.ops.gemm import gemm
+    if pad == 4 and not wide:
+        pytest.skip("16-bit rows are multiples of 16 bytes")
+    torch.manual_seed(31)
+    K, eps = 64, 2.0 ** -8 if DT == torch.bfloat16 else 2.0 ** -11
+    mk = lambda *s: torch.randn(*s, device=DEV).to(DT)
+
+    def place(dtype, like=None):           # [M, N] inside rows of N + pad, `off` elements behind a 32-byte boundary
+        t = torch.zeros(off + M * (N + pad) + 32, device=DEV, dtype=dtype)[off:off + M * (N + pad)].view(M, N + pad)[:, :N]
+        return t if like is None else t.copy_(like)
+
+    a, b = mk(M, K), mk(N, K)
+    z = a.double() @ b.double().t()
+    if wide:
+        out = place(torch.float32, torch.randn(M, N, device=DEV))
+        want = out.double() + z
+        got = gemm(a, b, out=out, accumulate=True)
+        assert (got.double() - want).abs().max() <= 2 ** -18 * 64
+        assert (gemm(a, b, out=place(torch.float32)).double() - z).abs().max() <= 2 ** -18 * 64
+        return
+    near = lambda got, want, steps=1: (got.double() - want).abs().sub(steps * eps * want.abs()).max() <= 2 ** -12
+    assert near(gemm(a, b, out=place(DT)), z)
+    res = place(DT, mk(M, N))
+    assert near(gemm(a, b, out=place(DT), residual=res), z + res.double())
+    assert near(gemm(a, b, out=place(DT), dgelu_aux=res, dgelu="mul"), z * res.double())
+    out = place(DT, res)
+    assert near(gemm(a, b, out=out, accumulate=True), z + res.double())
+    deriv, act = place(DT), place(DT)
+    gemm(a, b, out=act, gelu="erf", aux_out=deriv, aux_deriv=True)
+    x = z.detach().requires_grad_()
+    y = torch.nn.functional.gelu(x)
+    assert near(act, y) and near(deriv, torch.autograd.grad(y.sum(), x)[0])
