@@ -5,6 +5,7 @@
   ``gpt_neox_b200.ops`` binds with ctypes.
 * ``lib/libneox_data.so`` – the CPU dataset-index builders (g++), the counterpart of the
   reference's ``megatron/data/helpers.cpp`` built by ``megatron/data/Makefile``.
+* ``lib/neox_host_calls.so`` – native calls from Python into the kernel library (g++, csrc/host_calls.cpp).
 * ``lib/libneox_host.so`` – host AdamW for optimizer-state offload (g++, csrc/cpu_adam.cpp).
 
 Objects are cached under ``build/`` and rebuilt when a source or any header is newer.
@@ -17,6 +18,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -116,6 +118,21 @@ def build_host_ops(force: bool = False) -> Path:
     return out
 
 
+def build_host_calls(force: bool = False) -> Path:
+    """``lib/neox_host_calls.so``: native calls from Python into the kernel library (csrc/host_calls.cpp, an extension module
+    of this interpreter)."""
+    LIB.mkdir(parents=True, exist_ok=True)
+    src = CSRC / "host_calls.cpp"
+    out = LIB / "neox_host_calls.so"
+    if force or _stale(out, [src]):
+        cmd = [os.environ.get("CXX", "g++"), *CXX_FLAGS, "-fvisibility=hidden", "-I", sysconfig.get_paths()["include"], str(src),
+               "-o", str(out)]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"g++ failed:\n{r.stdout}\n{r.stderr}")
+    return out
+
+
 def build_data_helpers_sanitized(out_dir, cxx=None) -> Path:
     """The dataset-index builders compiled with AddressSanitizer + UBSan (host code only; the GPU pool offers
     no compute-sanitizer).  The library must be loaded into a process that preloads the ASan runtime:
@@ -133,6 +150,7 @@ def build_data_helpers_sanitized(out_dir, cxx=None) -> Path:
 def build_all(force: bool = False, verbose: bool = False):
     a = build_data_helpers(force)
     build_host_ops(force)
+    build_host_calls(force)
     b = build_cuda(force, verbose)
     return a, b
 

@@ -22,7 +22,7 @@ import weakref
 import torch
 
 _LOCK = threading.Lock()
-#: layer -> (weak reference to the cache it returned last, stream); the cache itself is held by whoever uses it
+#: layer -> [weak reference to the cache it returned last or None, stream]; the cache itself is held by whoever uses it
 _LAST: "weakref.WeakKeyDictionary" = weakref.WeakKeyDictionary()
 _MIN_ROOM = 256
 
@@ -31,15 +31,23 @@ def _stream(t):
     return torch._C._cuda_getCurrentRawStream(t.get_device()) if t.is_cuda else 0
 
 
-def _claim(layer, past, stream) -> bool:
-    """Whether ``past`` is the cache ``layer`` returned last; the answer is yes once per returned cache."""
+def _slot(layer):
     with _LOCK:
-        ref, st = _LAST.get(layer, (None, None))
+        slot = _LAST.get(layer)
+        if slot is None:
+            slot = _LAST[layer] = [None, None]
+        return slot
+
+
+def _claim(slot, past, stream) -> bool:
+    """Whether ``past`` is the cache the layer returned last; the answer is yes once per returned cache."""
+    with _LOCK:
+        ref, st = slot
         if ref is None or ref() is not past or st != stream:
             return False
         if past.is_inference() and not torch.is_inference_mode_enabled():
             return False                # its buffer may not be written outside inference mode
-        del _LAST[layer]
+        slot[0] = None
         return True
 
 
@@ -50,14 +58,14 @@ def extend(layer, past, rows: int, like: torch.Tensor, shape=None) -> torch.Tens
     n = 0 if past is None else past.shape[1] if torch.is_tensor(past) else past[0].shape[0]
     shape = tuple(like.shape[1:]) if shape is None else shape
     stream, total = _stream(like), n + rows
-    buf = None
+    present, slot = None, _slot(layer)
     capturing = like.is_cuda and torch.cuda.is_current_stream_capturing()
     if torch.is_tensor(past) and past.dtype == like.dtype and past.device == like.device and not capturing \
-            and past.shape[2:] == shape and _claim(layer, past, stream):
-        room = past.stride(0) // past.stride(1)
-        if total <= room:
-            buf = past.as_strided((2, room) + shape, past.stride())
-    if buf is None:
+            and past.shape[2:] == shape and _claim(slot, past, stream):
+        stride = past.stride()
+        if total <= stride[0] // stride[1]:
+            present = past.as_strided((2, total) + shape, stride)
+    if present is None:
         if n and not (past[0].shape == past[1].shape == (n,) + shape):
             # (the copies would broadcast the cache of another batch or head count)
             raise RuntimeError("kv_cache: the cache holds keys %s and values %s, this step appends rows of %s"
@@ -66,8 +74,8 @@ def extend(layer, past, rows: int, like: torch.Tensor, shape=None) -> torch.Tens
         if n:
             buf[0, :n].copy_(past[0])
             buf[1, :n].copy_(past[1])
-    present = buf[:, :total]
+        present = buf[:, :total]
     if not capturing:
         with _LOCK:
-            _LAST[layer] = (weakref.ref(present), stream)
+            slot[0], slot[1] = weakref.ref(present), stream
     return present

@@ -463,42 +463,55 @@ class ParallelTransformerLayer(nn.Module):
         """The whole layer in one native call, or None where it has to run op by op: generation without autograd, dense
         parallel-residual layer with two LayerNorms, rotary flash attention and a GeLU MLP on one tensor-parallel rank,
         plain modules whose calls nobody hooks into or replaces."""
-        a, m = self.attention, self.mlp
         if not (self.use_cache and x.is_cuda and x.is_contiguous() and x.shape[0] > 0 and x.shape[1] > 0
-                and kernel_lib.untracked() and self._dual_norm_ok(x)
-                and _plain(a, ParallelSelfAttention) and _plain(m, ParallelMLP) and a.use_cache and a.use_flash_attention
-                and not a.use_qk_layernorm and a.rpe is None and a.rotary_emb is not None
+                and kernel_lib.untracked() and not self.gpt_j_tied):
+            return None
+        calls = kernel_lib.calls()
+        sub = calls.sub
+        get = sub if type(self) in (ParallelTransformerLayer, ParallelTransformerLayerPipe) else getattr
+        a, m, n1, n2 = get(self, "attention"), get(self, "mlp"), get(self, "input_layernorm"), get(self, "post_attention_layernorm")
+        if not (calls.plain(a, ParallelSelfAttention, _FORWARD[ParallelSelfAttention], m, ParallelMLP, _FORWARD[ParallelMLP],
+                            n1, LayerNorm, _FORWARD[LayerNorm], n2, LayerNorm, _FORWARD[LayerNorm])
+                and len(n1.normalized_shape) == 1 and a.use_cache and a.use_flash_attention
+                and not a.use_qk_layernorm and a.rpe is None and not m.is_gated and m.activation_type == "gelu"
                 and not (self.training and (self.hidden_dropout > 0 or a.dropout_p > 0))
-                and mpu.get_model_parallel_world_size() == 1 and m._fusable(x)):
+                and mpu.get_model_parallel_world_size() == 1 and not torch.nn.modules.module._has_any_global_hook()):
             return None
-        hn = a.hidden_size_per_attention_head
-        linears = (_sub(a, "query_key_value"), _sub(a, "dense"), _sub(m, "linear1"), _sub(m, "linear2"))
-        n1, n2, rotary = self.input_layernorm, self.post_attention_layernorm, _sub(a, "rotary_emb")
-        if hn % 8 or hn > 128 or a.rotary_dim % 16 \
-                or not (_plain(linears[0], mpu.ColumnParallelLinear) and _plain(linears[2], mpu.ColumnParallelLinear)
-                        and _plain(linears[1], mpu.RowParallelLinear) and _plain(linears[3], mpu.RowParallelLinear)
-                        and _plain(rotary, RotaryEmbedding) and _plain(n1, LayerNorm) and _plain(n2, LayerNorm)) \
-                or any(l.use_mup or l.use_fp8 or getattr(l, "gather_output", False) for l in linears) \
-                or linears[0].skip_bias_add or torch.nn.modules.module._has_any_global_hook():
+        hn, rotary = a.hidden_size_per_attention_head, sub(a, "rotary_emb")
+        qkv, dense, up, down = sub(a, "query_key_value"), sub(a, "dense"), sub(m, "linear1"), sub(m, "linear2")
+        if rotary is None or hn % 8 or hn > 128 or a.rotary_dim % 16 or n1.eps != n2.eps \
+                or not calls.plain(rotary, RotaryEmbedding, _FORWARD[RotaryEmbedding],
+                                   qkv, mpu.ColumnParallelLinear, _FORWARD[mpu.ColumnParallelLinear],
+                                   up, mpu.ColumnParallelLinear, _FORWARD[mpu.ColumnParallelLinear],
+                                   dense, mpu.RowParallelLinear, _FORWARD[mpu.RowParallelLinear],
+                                   down, mpu.RowParallelLinear, _FORWARD[mpu.RowParallelLinear]):
             return None
-        weights = [t for l in (n1, n2) + linears for t in (_param(l, "weight"), _param(l, "bias"))]
-        up = weights[8]
-        ptrs = pointers(x, *weights)
-        if ptrs is None or n1.eps != n2.eps:
+        for l in (qkv, dense, up, down):       # (of known classes: an attribute that is not there costs more than a look)
+            d = l.__dict__
+            if l.use_mup or l.use_fp8 or d.get("gather_output", False):
+                return None
+        if qkv.skip_bias_add:
+            return None
+        ptrs = pointers(x, n1, n2, qkv, dense, up, down)
+        if ptrs is None:
             return None
         has_past = layer_past is not None and (not torch.is_tensor(layer_past) or layer_past.numel() > 0)
         past = layer_past[0].shape[0] if has_past else 0
-        cos, sin = rotary(seq_len=x.shape[0] + past)
+        assert x.shape[0] + past <= rotary.max_seq_len
+        cos, sin = sub(rotary, "cos_table"), sub(rotary, "sin_table")
         if (cos.data_ptr() | sin.data_ptr()) & 15:
             return None
         kvp = a.num_kv_heads_per_partition
         present = kv_cache.extend(a, layer_past if has_past else None, x.shape[0], x, (x.shape[1], kvp, hn))
         out = layer_infer(
             x, ptrs, cos, sin, present, past,
-            heads=a.num_attention_heads_per_partition, kv_heads=kvp, head_dim=hn, ffn=up.shape[0], rot=a.rotary_dim,
+            heads=a.num_attention_heads_per_partition, kv_heads=kvp, head_dim=hn, ffn=up.output_size_per_partition, rot=a.rotary_dim,
             window=a.sliding_window_width if a.sliding_window_width is not None else -1, scale=a.attn_scale, eps=n1.eps,
             act=("tanh" if m.bias_gelu_fusion else "erf", not m.recompute_act))
-        self.layer_past = present
+        if get is sub and "layer_past" in self.__dict__:
+            self.__dict__["layer_past"] = present      # (what the module's __setattr__ comes to for a plain attribute)
+        else:
+            self.layer_past = present
         return out
 
     def _dual_norm_ok(self, x):
@@ -507,12 +520,13 @@ class ParallelTransformerLayer(nn.Module):
 
     def forward(self, x, attention_mask=None, layer_past=None):
         layer_past = layer_past if layer_past is not None else self.layer_past
+        if self.gpt_j_residual and self.use_cache:
+            out = self._infer(x, layer_past)
+            if out is not None:
+                return out
         p = self.hidden_dropout if self.training else 0.0
         ws = mpu.get_model_parallel_world_size()
         if self.gpt_j_residual:
-            out = self._infer(x, layer_past) if self.use_cache else None
-            if out is not None:
-                return out
             residual = x
             if self.gpt_j_tied:
                 x1 = x2 = self.input_layernorm(x)
@@ -599,32 +613,11 @@ class ParallelTransformerLayer(nn.Module):
         return bias_dropout_add(mlp_output, mlp_bias, attention_output, p, self.training)
 
 
-#: the forwards whose work the native layer call does itself
+#: the forwards whose work the native layer call does itself.  A module is plain (``plain`` of csrc/host_calls.cpp) if calling it
+#: runs its class's forward as it was defined and nothing else: no subclass (a parametrized module is one), no hook, no
+#: forward replaced on the instance or on the class.
 _FORWARD = {c: c.forward for c in (ParallelSelfAttention, ParallelMLP, LayerNorm, RotaryEmbedding, mpu.ColumnParallelLinear,
                                    mpu.RowParallelLinear)}
-
-
-def _plain(m, cls):
-    """Whether calling ``m`` runs ``cls.forward`` as it was defined and nothing else: no subclass (a parametrized module is
-    one), no hook, no forward replaced on the instance or on the class."""
-    d = m.__dict__
-    return type(m) is cls and cls.forward is _FORWARD[cls] and "forward" not in d and not d["_forward_hooks"] \
-        and not d["_forward_pre_hooks"]
-
-
-def _sub(m, name):
-    """``getattr(m, name)`` for a submodule of a module that is plain (its class has no attribute of that name), without the
-    module's ``__getattr__`` where nothing in the instance stands before it."""
-    d = m.__dict__
-    found = None if name in d else d["_modules"].get(name)
-    return found if found is not None else getattr(m, name)
-
-
-def _param(m, name):
-    """``getattr(m, name)`` for a parameter (or None), likewise."""
-    d = m.__dict__
-    params = d["_parameters"]
-    return params[name] if name in params and name not in d else getattr(m, name)
 
 
 def _sum_bias(a, b):

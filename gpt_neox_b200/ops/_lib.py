@@ -1,4 +1,5 @@
-"""ctypes binding of ``lib/libneox_b200.so`` (the sm_100a kernel library).
+"""ctypes binding of ``lib/libneox_b200.so`` (the sm_100a kernel library), with native calls in its place for the entry
+points that csrc/host_calls.cpp knows.
 
 The library is loaded lazily on first use.  On a machine with a CUDA device a missing
 or unloadable library is a hard error: the CUDA ops never fall back silently to
@@ -7,6 +8,8 @@ PyTorch kernels.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 from pathlib import Path
 
@@ -14,6 +17,7 @@ import torch
 
 _LIB = None
 _HALF = None
+_CALLS = None
 # NEOX_KERNEL_LIB=debug loads the range-checking build (python -m gpt_neox_b200.build --debug-bounds)
 _LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / (
     "libneox_b200_dbg.so" if os.environ.get("NEOX_KERNEL_LIB") == "debug" else "libneox_b200.so")
@@ -53,7 +57,19 @@ class _HalfView:
         return fn
 
 
-def _declare(lib):
+def _load_calls():
+    """The native module built from csrc/host_calls.cpp."""
+    path = _LIB_PATH.parent / "neox_host_calls.so"
+    if not path.exists():
+        raise KernelError(f"{path} is missing: build it with `python -m gpt_neox_b200.build`")
+    spec = importlib.util.spec_from_loader("neox_host_calls", importlib.machinery.ExtensionFileLoader("neox_host_calls", str(path)))
+    calls = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(calls)
+    calls.set_host_tensor_error(ptr)
+    return calls
+
+
+def _declare(lib, calls):
     def sig(name, argtypes, restype=c_int):
         for nm in (name, name + "_f16"):
             try:
@@ -62,6 +78,9 @@ def _declare(lib):
                 continue
             fn.argtypes = argtypes
             fn.restype = restype
+            native = calls.bind(nm, C.cast(fn, c_void_p).value)
+            if native is not None:       # takes tensors and addresses alike
+                setattr(lib, nm, native)
 
     P, I, L, F, U = c_void_p, c_int, c_ll, c_float, C.c_ulonglong
     sig("nx_last_error", [], C.c_char_p)
@@ -141,7 +160,7 @@ def available() -> bool:
 def lib(like=None):
     """The kernel library.  ``like``: a tensor or dtype; for ``torch.float16`` the returned object resolves
     every entry point to its fp16 build."""
-    global _LIB, _HALF
+    global _LIB, _HALF, _CALLS
     if _LIB is not None:
         dt = getattr(like, "dtype", like)
         return _HALF if dt == torch.float16 else _LIB
@@ -151,9 +170,17 @@ def lib(like=None):
                 f"{_LIB_PATH} is missing: build it with `python -m gpt_neox_b200.build` "
                 "(the CUDA ops have no PyTorch fallback on a GPU)"
             )
-        _LIB = _declare(C.CDLL(str(_LIB_PATH), mode=os.RTLD_GLOBAL if hasattr(os, "RTLD_GLOBAL") else 0))
+        _CALLS = _load_calls()
+        _LIB = _declare(C.CDLL(str(_LIB_PATH), mode=os.RTLD_GLOBAL if hasattr(os, "RTLD_GLOBAL") else 0), _CALLS)
         _HALF = _HalfView(_LIB)
     return lib(like)
+
+
+def calls():
+    """The native module (csrc/host_calls.cpp): ``sub``, ``plain`` and ``pointers`` beside the bound entry points."""
+    if _CALLS is None:
+        lib()
+    return _CALLS
 
 
 def check(status: int, what: str = "kernel"):
@@ -163,14 +190,14 @@ def check(status: int, what: str = "kernel"):
 
 
 def ptr(t):
-    """Device pointer of a tensor (or None) as a ctypes void pointer."""
+    """Device pointer of a tensor (or None)."""
     if t is None:
         return None
     if not t.is_cuda:
         # every kernel dereferences its pointers on the device: refuse a host tensor here instead
         # of letting the GPU fault on it
         raise KernelError(f"host tensor (shape {tuple(t.shape)}, {t.dtype}) passed to a CUDA kernel")
-    return c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def untracked() -> bool:
@@ -182,7 +209,7 @@ def untracked() -> bool:
 
 def stream():
     # (torch.cuda.current_stream() builds a Stream object around this number)
-    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def read_device_error(clear: bool = True) -> int:

@@ -114,18 +114,23 @@ def bias_act(x: torch.Tensor, bias: torch.Tensor | None, act: str) -> torch.Tens
     return _torch_act(act, x if bias is None else x + bias)
 
 
+def _gated_act_forward(x, act_id):
+    """-> (output, x as contiguous rows)."""
+    F2 = x.shape[-1]
+    x2 = x.reshape(-1, F2).contiguous()
+    y = torch.empty((x2.shape[0], F2 // 2), device=x.device, dtype=x.dtype)
+    LAUNCHES["n"] += 1
+    _lib.check(_lib.lib(x2).nx_gated_act_fwd(x2, y, x2.shape[0], F2 // 2, act_id, _lib.stream()), "nx_gated_act_fwd")
+    return y.view(*x.shape[:-1], F2 // 2), x2
+
+
 class _GatedActFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, act_id):
-        F2 = x.shape[-1]
-        x2 = x.reshape(-1, F2).contiguous()
-        y = torch.empty((x2.shape[0], F2 // 2), device=x.device, dtype=x.dtype)
-        LAUNCHES["n"] += 1
-        _lib.check(_lib.lib(x2).nx_gated_act_fwd(_lib.ptr(x2), _lib.ptr(y), x2.shape[0], F2 // 2, act_id,
-                                               _lib.stream()), "nx_gated_act_fwd")
+        y, x2 = _gated_act_forward(x, act_id)
         ctx.save_for_backward(x2)
         ctx.act_id, ctx.shape = act_id, x.shape
-        return y.view(*x.shape[:-1], F2 // 2)
+        return y
 
     @staticmethod
     def backward(ctx, gy):
@@ -144,6 +149,8 @@ def gated_act(x: torch.Tensor, kind: str) -> torch.Tensor:
     (chunk order of megatron/model/transformer.py:189-198)."""
     act = GATED[kind]
     if _cuda_ok(x) and (x.shape[-1] // 2) % 8 == 0:
+        if _lib.untracked():
+            return _gated_act_forward(x, ACT_IDS[act])[0]
         return _GatedActFn.apply(x, ACT_IDS[act])
     if x.is_cuda:
         raise _lib.KernelError("gated_act: CUDA path needs bf16 and F % 8 == 0")

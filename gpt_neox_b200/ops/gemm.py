@@ -117,9 +117,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
     if PAIR_GEMM["on"] and M >= 256 and N >= 256:
         fn, name = L.nx_gemm2_bf16, "nx_gemm2_bf16"      # CTA-pair kernel (cta_group::2, 256 x 256 tiles)
     _lib.check(fn(
-        _lib.ptr(a), _lib.ptr(b), _lib.ptr(out), M, N, K, a.stride(0), b.stride(0), out.stride(0),
-        int(trans_a), int(trans_b), _lib.ptr(bias), _lib.ptr(dgelu_aux), _lib.ptr(aux_out),
-        _lib.ptr(residual), ld_aux, flags, float(alpha if alpha is not None else 1.0),
+        a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0),
+        int(trans_a), int(trans_b), bias, dgelu_aux, aux_out,
+        residual, ld_aux, flags, float(alpha if alpha is not None else 1.0),
         _lib.stream()), name)
     return out
 

@@ -41,8 +41,8 @@ def _forward(kind, x, gamma, beta, eps, gamma2, beta2):
     rstd = torch.empty(rows, device=x.device, dtype=torch.float32)
     LAUNCHES["n"] += 1
     _lib.check(_lib.lib(x2).nx_norm_fwd(
-        kind, _lib.ptr(x2), _lib.ptr(gamma), _lib.ptr(beta), _lib.ptr(y1), _lib.ptr(gamma2),
-        _lib.ptr(beta2), _lib.ptr(y2), _lib.ptr(mean), _lib.ptr(rstd), rows, H, float(eps),
+        kind, x2, gamma, beta, y1, gamma2,
+        beta2, y2, mean, rstd, rows, H, float(eps),
         _lib.stream()), "nx_norm_fwd")
     return x2, y1, y2, mean, rstd
 
@@ -115,9 +115,9 @@ class _NormFn(torch.autograd.Function):
                 out[i] = m if direct else torch.empty(H, device=x2.device, dtype=x2.dtype if out16 else torch.float32)
             LAUNCHES["n"] += 2
             _lib.check(L.nx_norm_bwd(
-                ctx.kind, _lib.ptr(ga), _lib.ptr(g2 if both else None), _lib.ptr(x2), _lib.ptr(mean), _lib.ptr(rstd),
-                _lib.ptr(gma), _lib.ptr(gmb), _lib.ptr(gres), _lib.ptr(dx), _lib.ptr(out[ia]), _lib.ptr(out[ia + 1]),
-                _lib.ptr(out[2] if both else None), _lib.ptr(out[3] if both else None), _lib.ptr(ws), rows, H,
+                ctx.kind, ga, g2 if both else None, x2, mean, rstd,
+                gma, gmb, gres, dx, out[ia], out[ia + 1],
+                out[2] if both else None, out[3] if both else None, ws, rows, H,
                 1 if direct else 0, 1 if out16 else 0, _lib.stream()), "nx_norm_bwd")
             if not direct:
                 for i in want:
