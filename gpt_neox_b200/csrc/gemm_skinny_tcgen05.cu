@@ -14,6 +14,8 @@
 
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 namespace cg = cooperative_groups;
 
 namespace nx {
@@ -85,9 +87,17 @@ __device__ __forceinline__ void skinny_store4(const SkinnyParams& p, int m, int 
   *reinterpret_cast<uint2*>(p.C + m * p.ldc + n) = make_uint2(pack_h16x2(v[0], v[1]), pack_h16x2(v[2], v[3]));
 }
 
-template <int NX, int STAGES>
-__global__ void __launch_bounds__(SK_THREADS)
-gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const SkinnyParams p) {
+// One product, or two side by side: the tiles from first_tiles on are the second one's.  Clusters are as large as the larger
+// number of splits; a CTA beyond its product's splits has no part in it.
+template <int COUNT>
+struct SkinnyArgs {
+  CUtensorMap w[COUNT], x[COUNT];
+  SkinnyParams p[COUNT];
+  int splits[COUNT], first_tiles;
+};
+
+template <int NX, int STAGES, int COUNT>
+__global__ void __launch_bounds__(SK_THREADS) gemm_skinny_kernel(const __grid_constant__ SkinnyArgs<COUNT> args) {
   using L = SkinnySmem<NX, STAGES>;
   constexpr uint32_t TMEM_COLS = NX < 32 ? 32 : NX;
   extern __shared__ uint8_t smem_raw[];
@@ -101,8 +111,13 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   cg::cluster_group cluster = cg::this_cluster();
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nsplit = gridDim.x, split = blockIdx.x;         // the cluster spans the x dimension
-  const int n0 = blockIdx.y * SK_BW;
+  const int which = COUNT > 1 && static_cast<int>(blockIdx.y) >= args.first_tiles;
+  // (one product's parameters are read where they are: copied, 40 - 60 rows took 1 - 3 % longer)
+  const std::conditional_t<COUNT == 1, const SkinnyParams&, SkinnyParams> p = args.p[which];
+  const CUtensorMap &tmW = args.w[which], &tmX = args.x[which];
+  const int nsplit = COUNT > 1 ? args.splits[which] : gridDim.x, split = blockIdx.x;      // the cluster spans the x dimension
+  const bool part_of = COUNT == 1 || split < nsplit;
+  const int n0 = (blockIdx.y - (which ? args.first_tiles : 0)) * SK_BW;
   const int num_kb = (p.K + SK_BK - 1) / SK_BK;
   const int kb0 = static_cast<int>(static_cast<long long>(num_kb) * split / nsplit);
   const int kb1 = static_cast<int>(static_cast<long long>(num_kb) * (split + 1) / nsplit);
@@ -120,7 +135,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   if (warp == 1) {
     tmem_alloc(tmem_slot, TMEM_COLS);
     tmem_relinquish();
-  } else if (warp == 0 && elect_one()) {
+  } else if (warp == 0 && part_of && elect_one()) {
     // the first weights on their way into L2 while the kernel before this one ends (which may even be writing them: what is
     // read later is what L2 has then)
     for (int kb = kb0; kb < kb1 && kb < kb0 + STAGES; ++kb) tma_prefetch_l2_2d(&tmW, kb * SK_BK, n0);
@@ -132,7 +147,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   bool aborted = false;
   grid_dependency_wait();
 
-  if (warp == 0) {
+  if (!part_of) {
+    // nothing but the barriers below
+  } else if (warp == 0) {
     if (elect_one()) {
       for (int kb = kb0; kb < kb1; ++kb) {
         const int i = kb - kb0, st = i % STAGES;
@@ -161,7 +178,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   }
   // ---- epilogue warps: the accumulator to shared memory as [row of A][row of W], then 4 columns of C per thread
   float* part = reinterpret_cast<float*>(sgen);             // [NX][SK_BW], over the drained ring
-  if (warp >= 2) {
+  if (warp >= 2 && part_of) {
     const int col = (warp & 3) * 32 + lane;                 // row of W in the tile == TMEM lane
     aborted = !__all_sync(0xffffffffu, mbar_wait(done_bar, 0, p.err, 72));
     tc_fence_after_sync();
@@ -184,9 +201,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   // one SM and none on another, and their own prefetches part of the bandwidth (1 row, 4096 -> 22016, one call after the
   // other: 33.3 us when they might come at the start, 29.2 so, 30.5 without overlap; 768 -> 768 3.70, 3.58, 4.69).
   allow_dependents();
-  if (nsplit > 1) cluster.sync();
+  if (gridDim.x > 1) cluster.sync();
   else __syncthreads();
-  if (warp >= 2 && !aborted) {
+  if (warp >= 2 && part_of && !aborted) {
     const int t = threadIdx.x - 64, n = n0 + (t & 31) * 4;
     if (n < p.N) {
       float bias[4] = {0.f, 0.f, 0.f, 0.f};
@@ -216,7 +233,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       }
     }
   }
-  if (nsplit > 1) cluster.sync();                           // nobody leaves while its partial tile may still be read
+  if (gridDim.x > 1) cluster.sync();                        // nobody leaves while its partial tile may still be read
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) {
@@ -225,36 +242,57 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   }
 }
 
-template <int NX, int STAGES>
-static int launch_skinny(const void* A, const void* B, long long lda, long long ldb, const SkinnyParams& p,
-                         cudaStream_t stream) {
+// splits: until two CTAs per SM are in flight, with at least four 64-wide steps each
+static int skinny_splits(int N, int K) {
+  const int tiles = (N + SK_BW - 1) / SK_BW, num_kb = (K + SK_BK - 1) / SK_BK;
+  int splits = 1;
+  while (splits < SK_MAX_SPLITS && tiles * splits * 2 <= 2 * sm_count() && num_kb >= splits * 2 * 4) splits *= 2;
+  return splits;
+}
+
+template <int NX, int STAGES, int COUNT>
+static int launch_skinny(const SkinnyProduct* q, cudaStream_t stream) {
   using L = SkinnySmem<NX, STAGES>;
-  auto kern = gemm_skinny_kernel<NX, STAGES>;
+  auto kern = gemm_skinny_kernel<NX, STAGES, COUNT>;
   static bool configured = false;
   if (!configured) {
     NX_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::DYN));
     configured = true;
   }
-  CUtensorMap tmW, tmX;
-  if (!make_tma_2d(&tmW, B, p.N, p.K, ldb * 2, SK_BW, SK_BK, 2)) return NX_ERR_ARG;
-  if (!make_tma_2d(&tmX, A, p.M, p.K, lda * 2, NX, SK_BK, 2)) return NX_ERR_ARG;
-  const int tiles = (p.N + SK_BW - 1) / SK_BW, num_kb = (p.K + SK_BK - 1) / SK_BK;
-  // splits: until two CTAs per SM are in flight, with at least four 64-wide steps each
-  int splits = 1;
-  while (splits < SK_MAX_SPLITS && tiles * splits * 2 <= 2 * sm_count() && num_kb >= splits * 2 * 4) splits *= 2;
+  SkinnyArgs<COUNT> a;
+  int tiles = 0, splits = 1;
+  for (int i = 0; i < COUNT; ++i) {
+    const SkinnyParams& p = q[i].p;
+    if (!make_tma_2d(&a.w[i], q[i].B, p.N, p.K, q[i].ldb * 2, SK_BW, SK_BK, 2)) return NX_ERR_ARG;
+    if (!make_tma_2d(&a.x[i], q[i].A, p.M, p.K, q[i].lda * 2, NX, SK_BK, 2)) return NX_ERR_ARG;
+    a.p[i] = p;
+    a.splits[i] = skinny_splits(p.N, p.K);
+    splits = a.splits[i] > splits ? a.splits[i] : splits;
+    tiles += (p.N + SK_BW - 1) / SK_BW;
+    if (i == 0) a.first_tiles = tiles;
+  }
   // The launch, the set-up and the first weights' way into L2 lie under the kernel before (7B gated MLP, 4 rows, three launches:
   // 74.6 -> 70.5 us; one query row against 1543 keys, whose kernel is launched the same way, 38.7 -> 37.2 us).
-  NX_CUDA_CHECK(launch_dependent(kern, dim3(splits, tiles), dim3(SK_THREADS), L::DYN, stream, splits, tmW, tmX, p));
+  NX_CUDA_CHECK(launch_dependent(kern, dim3(splits, tiles), dim3(SK_THREADS), L::DYN, stream, splits, a));
   return NX_OK;
+}
+
+template <int COUNT>
+static int launch_skinny_rows(const SkinnyProduct* q, cudaStream_t stream) {
+  // ring depths: two CTAs fit an SM's shared memory
+  const int M = q[0].p.M;
+  if (M <= 16) return launch_skinny<16, 6, COUNT>(q, stream);
+  if (M <= 32) return launch_skinny<32, 5, COUNT>(q, stream);
+  if (M <= 64) return launch_skinny<64, 4, COUNT>(q, stream);
+  return launch_skinny<128, 3, COUNT>(q, stream);
 }
 
 int gemm_skinny_launch(const void* A, const void* B, long long lda, long long ldb, const SkinnyParams& p,
                        cudaStream_t stream) {
-  // ring depths: two CTAs fit an SM's shared memory
-  if (p.M <= 16) return launch_skinny<16, 6>(A, B, lda, ldb, p, stream);
-  if (p.M <= 32) return launch_skinny<32, 5>(A, B, lda, ldb, p, stream);
-  if (p.M <= 64) return launch_skinny<64, 4>(A, B, lda, ldb, p, stream);
-  return launch_skinny<128, 3>(A, B, lda, ldb, p, stream);
+  const SkinnyProduct q{A, B, lda, ldb, p};
+  return launch_skinny_rows<1>(&q, stream);
 }
+
+int gemm_skinny_launch_pair(const SkinnyProduct (&q)[2], cudaStream_t stream) { return launch_skinny_rows<2>(q, stream); }
 
 }  // namespace nx

@@ -653,6 +653,8 @@ struct CommArgs {
   bool skinny = false;   // few rows: gemm_skinny_tcgen05.cu
 };
 
+namespace nx {
+
 // Whether a product goes to the few-rows kernel: its layouts and epilogues, and up to 64 rows (a generation step; 4 rows of
 // the 7B gated MLP: 164 -> 54 us for its two GEMMs), up to 128 where the tiles here would leave half the SMs without one
 // and the reduction is long enough to be split in four (us, here / there, 128 rows: 4096 x 4096 30.9 / 15.2, 4096 x 16384
@@ -662,8 +664,7 @@ struct CommArgs {
 //   6.4 / 8.3; 136 x 64, 96 rows 6.4 / 7.0; 64 x 1024, 128 rows 7.0 / 7.5);
 // - with more tiles than SMs the chip is full here too, and the rows of a short reduction cost the few-rows kernel's
 //   epilogue more (50304 x 768, 48 rows 22.2 / 21.9, 64 rows 22.2 / 23.1; 65536 x 640, 64 rows 0.92 of the rate).
-static bool skinny_better(int M, int N, int K, int transA, int transB, int flags) {
-  using namespace nx;
+bool skinny_better(int M, int N, int K, int transA, int transB, int flags) {
   constexpr int known = EPI_BIAS | EPI_GELU_ERF | EPI_GELU_TANH | EPI_AUX_OUT | EPI_AUX_DERIV | EPI_RESIDUAL | EPI_SCALE;
   if (transA || transB || (flags & ~known) != 0 || M > SKINNY_MAX_M) return false;
   const int BN = N <= 128 ? 128 : 256;
@@ -675,6 +676,8 @@ static bool skinny_better(int M, int N, int K, int transA, int transB, int flags
   if (tiles > sm_count() && K > 256 && K <= 1024 && M > 48) return false;
   return M <= 64 || (2 * tiles <= sm_count() && (M <= 96 || deep));
 }
+
+}  // namespace nx
 
 static int gemm_common(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                        long long ldc, int transA, int transB, const void* bias, const void* aux_in, void* aux_out,
@@ -774,7 +777,7 @@ NX_API int NX_SYM(nx_gemm_bf16)(const void* A, const void* B, void* C, int M, in
                         const void* aux_in, void* aux_out, const void* residual, long long ld_aux,
                         int flags, float alpha, void* stream_) {
   CommArgs ca;
-  ca.skinny = skinny_better(M, N, K, transA, transB, flags);
+  ca.skinny = nx::skinny_better(M, N, K, transA, transB, flags);
   return gemm_common(A, B, C, M, N, K, lda, ldb, ldc, transA, transB, bias, aux_in, aux_out, residual, ld_aux,
                      flags, alpha, ca, static_cast<cudaStream_t>(stream_));
 }

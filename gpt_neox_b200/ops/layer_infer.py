@@ -40,6 +40,8 @@ def layer_infer(x, ptrs, cos, sin, present, past, *, heads, kv_heads, head_dim, 
         heads, kv_heads, head_dim, ffn, past, rot, window,
         (EPI_GELU_TANH if act[0] == "tanh" else EPI_GELU_ERF) | (EPI_AUX_DERIV if act[1] else 0), int(PAIR_GEMM["on"]),
         eps, scale)
-    LAUNCHES["n"] += 8
-    _lib.check(lib.nx_layer_infer(args, _lib.stream()), "nx_layer_infer")
+    status = lib.nx_layer_infer(args, _lib.stream())
+    if status > 0:
+        _lib.check(status, "nx_layer_infer")
+    LAUNCHES["n"] -= status        # (minus the number of launches)
     return out

@@ -377,6 +377,40 @@ def test_a_layer_in_one_call_gives_the_bits_of_the_op_by_op_path(over, precision
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("hidden,heads", [(768, 12), (1024, 8)])
+def test_products_in_one_launch_give_the_bits_of_two(hidden, heads):
+    """Few rows: query / key / value with the MLP's first product, and dense with its second one, in one launch each, with
+    different numbers of splits (dense 2, down 8) - at both sides of every row count the kernel is built for, and of the
+    128 from which they are launched by themselves."""
+    from test_model_gpu import _build
+    _, model = _build(tiny_config(num_layers=1, hidden_size=hidden, num_attention_heads=heads, seq_length=512,
+                                  max_position_embeddings=512, synthetic_vocab_size=1000, pipe_parallel_size=0,
+                                  attention_config=[[["flash"], 1]], distributed_backend="nccl", precision="bfloat16"))
+    model.inference_mode(use_cache=True)
+    mlp = next(m for m in model.modules() if type(m).__name__ == "ParallelMLP")
+    tokens = torch.randint(0, 1000, (1, 512), device="cuda")
+    pos = torch.arange(512, device="cuda")[None]
+
+    def steps():
+        model.clear_cache()
+        out, at = [], 0
+        with torch.no_grad():
+            for n in (1, 15, 16, 17, 32, 33, 64, 65, 96, 128):
+                out.append(model((tokens[:, at:at + n].contiguous(), pos[:, at:at + n].contiguous(), None)))
+                at += n
+                if at > 300:
+                    model.clear_cache()
+                    at = 0
+        return out
+
+    one = steps()
+    handle = mlp.register_forward_hook(lambda *a: None)
+    ops = steps()
+    handle.remove()
+    assert all(torch.equal(a, b) for a, b in zip(one, ops)) and all(t.isfinite().all() for t in one)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("precision,x,branch,want", [("bfloat16", 1024.0, 3.0, 1032.0), ("fp16", 16384.0, 6.0, 16400.0)])
 @pytest.mark.parametrize("hook", [False, True])
 @pytest.mark.parametrize("rows", [1, 130, 300])
