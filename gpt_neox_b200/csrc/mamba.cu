@@ -22,8 +22,8 @@
 // memory 69 % and issue slots 62 % together; backward, issue slots (59 % with 3 warps per scheduler; shared memory 55 %),
 // where a step and channel costs 500 lane operations for 16 states.  DRAM 6-10 %.
 // Convolution + scan, forward + backward, 4 x 2048 steps of 1536 channels, fp16: 785 us with one channel per quad, inputs staged by the
-// whole CTA and dB / dC exchanged per channel (final forward sweep 119, light ones 70 and 86, backward 407 us); 605 us now (95,
-// 63 and 78, 283).  Whole calls of few channels and one block are latency: 2 x 31 x 768 takes 46 us of kernels, 43 before.
+// whole CTA and dB / dC exchanged per channel (final forward sweep 119, light ones 70 and 86, backward 407 us); 605 us with
+// the present scan (95, 63 and 78, 283), 594 with the present convolution, too.  Whole calls of few channels and one block are latency: 2 x 31 x 768 takes 46 us of kernels, 43 before.
 // Tried for the backward: states packed per channel pair instead of per state pair (B and C twice in shared memory, no copies
 // of a step's scalars): shared memory 62 % busy, 305 - 330 us; inputs staged per block with its loads waited for: 290 - 320.
 #include "common.h"
@@ -113,167 +113,151 @@ conv1d_silu_bwd_kernel(const h16* __restrict__ x, long long xsb, long long xst,
   if (dbias) atomicAdd(dbias + d, ab);
 }
 
-// Vector forms: a thread owns V neighbouring channels (one V * 2-byte load per step) and CV_T steps; the steps' loads
-// are issued before the first use.  The one-channel kernels above keep one 2-byte load in flight per thread and are
-// bound by its latency; they remain for channel counts, strides or bases that are not multiples of V elements.
+// Vector forms: a thread owns four neighbouring channels (an 8-byte load per step, packed pairs) and CV_FWD_T / CV_BWD_T steps, in
+// groups whose loads are asked for together, in the forward one group ahead (the backward has no registers left for that: 54
+// us).  The one-channel kernels above keep one 2-byte load in flight per thread and are bound by its latency; they remain for
+// channel counts, strides or bases that are not multiples of four elements.  The backward walks three steps more than it owns,
+// whose gradient reaches back into its tile; 21 + 3 are whole groups and leave enough blocks (29: 30.4 / 42.2 us).
+// Bound by latency at 28 and 16 warps an SM and by issue slots.  4 x 2048 x 1536 / 16 x 512 x 2048, fp16, us: forward 19.8 / 26.5 with
+// eight channels a thread and no pairs (142 registers), 13.5 / 15.8 now; backward 37.3 / 47.2 with 16 steps a thread, 32.1 / 39.1.
 constexpr int CV_X = 32;    // channel groups per block
 constexpr int CV_Y = 4;     // time tiles per block
-constexpr int CV_T = 16;    // steps per thread
-constexpr int CV_FWD_V = 8, CV_BWD_V = 4;
-
-template <int V>
-__device__ __forceinline__ void load_vec(const h16* p, float (&f)[V]) {
-  uint32_t w[V / 2];
-  if constexpr (V == 8) {
-    const uint4 u = *reinterpret_cast<const uint4*>(p);
-    w[0] = u.x; w[1] = u.y; w[2] = u.z; w[3] = u.w;
-  } else {
-    const uint2 u = *reinterpret_cast<const uint2*>(p);
-    w[0] = u.x; w[1] = u.y;
-  }
-#pragma unroll
-  for (int i = 0; i < V / 2; ++i) {
-    const float2 a = unpack_h16x2(w[i]);
-    f[2 * i] = a.x;
-    f[2 * i + 1] = a.y;
-  }
+constexpr int CV_V = 4;     // channels per thread
+constexpr int CV_FWD_T = 32, CV_BWD_T = 21, CV_G = 4;
+struct Conv4 { float2 a, b; };      // four channels
+__device__ __forceinline__ Conv4 conv_unpack(const uint2& u) { return {unpack_h16x2(u.x), unpack_h16x2(u.y)}; }
+__device__ __forceinline__ uint2 conv_pack(const Conv4& v) { return make_uint2(pack_h16x2(v.a.x, v.a.y), pack_h16x2(v.b.x, v.b.y)); }
+__device__ __forceinline__ Conv4 conv_fma(const Conv4& x, const Conv4& y, const Conv4& z) { return {ffma2(x.a, y.a, z.a), ffma2(x.b, y.b, z.b)}; }
+__device__ __forceinline__ Conv4 conv_mul(const Conv4& x, const Conv4& y) { return {fmul2(x.a, y.a), fmul2(x.b, y.b)}; }
+__device__ __forceinline__ Conv4 conv_sigmoid(const Conv4& x) {
+  auto f = [](float v) { return __fdividef(1.f, 1.f + __expf(-v)); };
+  return {make_float2(f(x.a.x), f(x.a.y)), make_float2(f(x.b.x), f(x.b.y))};
 }
-template <int V>
-__device__ __forceinline__ void store_vec(h16* p, const float (&f)[V]) {
-  if constexpr (V == 8)
-    *reinterpret_cast<uint4*>(p) = make_uint4(pack_h16x2(f[0], f[1]), pack_h16x2(f[2], f[3]), pack_h16x2(f[4], f[5]),
-                                              pack_h16x2(f[6], f[7]));
-  else
-    *reinterpret_cast<uint2*>(p) = make_uint2(pack_h16x2(f[0], f[1]), pack_h16x2(f[2], f[3]));
+// wk[k]: the tap on step t - 3 + k (zeros in front of a shorter kernel), and the bias
+__device__ __forceinline__ void conv_taps(const h16* w, const h16* bias, int d, int W, Conv4 (&wk)[4], Conv4& bv) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    float t[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) t[c] = k >= 4 - W ? ldbf(w + (long long)(d + c) * W + k - (4 - W)) : 0.f;
+    wk[k] = {make_float2(t[0], t[1]), make_float2(t[2], t[3])};
+  }
+  bv = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+  if (bias != nullptr) bv = {make_float2(ldbf(bias + d), ldbf(bias + d + 1)), make_float2(ldbf(bias + d + 2), ldbf(bias + d + 3))};
 }
-template <int V>
-__device__ __forceinline__ void load_taps(const h16* w, int d, int W, float (&wk)[V][4]) {
-#pragma unroll
-  for (int c = 0; c < V; ++c)
-#pragma unroll
-    for (int k = 0; k < 4; ++k) wk[c][k] = k >= 4 - W ? ldbf(w + (long long)(d + c) * W + k - (4 - W)) : 0.f;
+__device__ __forceinline__ Conv4 conv_pre(const Conv4 (&wk)[4], const Conv4& bv, const Conv4 (&win)[3], const Conv4& cur) {
+  return conv_fma(wk[3], cur, conv_fma(wk[2], win[2], conv_fma(wk[1], win[1], conv_fma(wk[0], win[0], bv))));
 }
 
 __global__ void __launch_bounds__(CV_X * CV_Y)
 conv1d_silu_fwd_vec_kernel(const h16* __restrict__ x, long long xsb, long long xst, const h16* __restrict__ w,
                            const h16* __restrict__ bias, h16* __restrict__ y, long long ysb, long long yst, int L,
                            int D, int W) {
-  constexpr int V = CV_FWD_V;
-  const int d = (blockIdx.x * CV_X + threadIdx.x) * V;
-  const int t0 = (blockIdx.y * CV_Y + threadIdx.y) * CV_T, b = blockIdx.z;
+  const int d = (blockIdx.x * CV_X + threadIdx.x) * CV_V;
+  const int t0 = (blockIdx.y * CV_Y + threadIdx.y) * CV_FWD_T, b = blockIdx.z;
   if (d >= D || t0 >= L) return;
-  float wk[V][4], bv[V], win[3][V];
-  load_taps<V>(w, d, W, wk);
+  const int t1 = min(t0 + CV_FWD_T, L);
   const h16* xp = x + b * xsb + d;
+  uint2 now[CV_G], next[CV_G];
+  auto fetch = [&](int t, uint2 (&u)[CV_G]) {
 #pragma unroll
-  for (int c = 0; c < V; ++c) bv[c] = bias ? ldbf(bias + d + c) : 0.f;
+    for (int k = 0; k < CV_G; ++k) {
+      u[k] = make_uint2(0u, 0u);
+      if (t + k < t1) u[k] = *reinterpret_cast<const uint2*>(xp + (t + k) * xst);
+    }
+  };
+  fetch(t0, now);
+  Conv4 wk[4], bv, win[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-#pragma unroll
-    for (int c = 0; c < V; ++c) win[k][c] = 0.f;
-    if (t0 - 3 + k >= 0) load_vec<V>(xp + (t0 - 3 + k) * xst, win[k]);
+    uint2 u = make_uint2(0u, 0u);
+    if (t0 - 3 + k >= 0) u = *reinterpret_cast<const uint2*>(xp + (t0 - 3 + k) * xst);
+    win[k] = conv_unpack(u);
   }
+  conv_taps(w, bias, d, W, wk, bv);
+  h16* yp = y + b * ysb + t0 * yst + d;
 #pragma unroll 1
-  for (int s = 0; s < CV_T; s += 8) {
-    uint4 raw[8];
+  for (int t = t0; t < t1; t += CV_G) {
+    fetch(t + CV_G, next);
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (t0 + s + u < L) raw[u] = *reinterpret_cast<const uint4*>(xp + (t0 + s + u) * xst);
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int t = t0 + s + u;
-      if (t < L) {
-        const uint32_t ww[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
-        float o[V];
-#pragma unroll
-        for (int c = 0; c < V; ++c) {
-          const float2 p2 = unpack_h16x2(ww[c / 2]);
-          const float cur = (c & 1) ? p2.y : p2.x;
-          o[c] = silu(bv[c] + wk[c][0] * win[0][c] + wk[c][1] * win[1][c] + wk[c][2] * win[2][c] + wk[c][3] * cur);
-          win[0][c] = win[1][c]; win[1][c] = win[2][c]; win[2][c] = cur;
-        }
-        store_vec<V>(y + b * ysb + t * yst + d, o);
-      }
+    for (int k = 0; k < CV_G; ++k) {
+      const Conv4 cur = conv_unpack(now[k]), pre = conv_pre(wk, bv, win, cur);
+      if (t + k < t1) *reinterpret_cast<uint2*>(yp) = conv_pack(conv_mul(pre, conv_sigmoid(pre)));
+      yp += yst;
+      win[0] = win[1]; win[1] = win[2]; win[2] = cur;
     }
+#pragma unroll
+    for (int k = 0; k < CV_G; ++k) now[k] = next[k];
   }
 }
 
-__global__ void __launch_bounds__(CV_X * CV_Y)
+__global__ void __launch_bounds__(CV_X * CV_Y, 4)
 conv1d_silu_bwd_vec_kernel(const h16* __restrict__ x, long long xsb, long long xst, const h16* __restrict__ w,
                            const h16* __restrict__ bias, const h16* __restrict__ dy, long long dsb, long long dst,
                            h16* __restrict__ dx, long long gsb, long long gst, float* __restrict__ dw,
                            float* __restrict__ dbias, int L, int D, int W) {
-  constexpr int V = CV_BWD_V;
-  __shared__ float red[CV_Y][CV_X][V * 5 + 1];
-  const int d = (blockIdx.x * CV_X + threadIdx.x) * V;
-  const int t0 = (blockIdx.y * CV_Y + threadIdx.y) * CV_T, b = blockIdx.z;
-  float aw[V][5];
-#pragma unroll
-  for (int c = 0; c < V; ++c)
-#pragma unroll
-    for (int k = 0; k < 5; ++k) aw[c][k] = 0.f;
+  __shared__ float red[CV_Y][CV_X][CV_V * 5 + 1];
+  const int d = (blockIdx.x * CV_X + threadIdx.x) * CV_V;
+  const int t0 = (blockIdx.y * CV_Y + threadIdx.y) * CV_BWD_T, b = blockIdx.z;
+  Conv4 aw[5] = {};                       // gradients of the four taps and the bias
   if (d < D && t0 < L) {
-    float wk[V][4], bv[V], win[3][V], dp[3][V];
-    load_taps<V>(w, d, W, wk);
     const h16* xp = x + b * xsb + d;
     const h16* gp = dy + b * dsb + d;
+    const int t_own = min(t0 + CV_BWD_T, L), t_end = min(t0 + CV_BWD_T + 3, L);
+    uint2 rx[CV_G], rg[CV_G];
+    auto fetch = [&](int t, uint2 (&u)[CV_G], uint2 (&g)[CV_G]) {
 #pragma unroll
-    for (int c = 0; c < V; ++c) {
-      bv[c] = bias ? ldbf(bias + d + c) : 0.f;
-      dp[0][c] = dp[1][c] = dp[2][c] = 0.f;
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-#pragma unroll
-      for (int c = 0; c < V; ++c) win[k][c] = 0.f;
-      if (t0 - 3 + k >= 0) load_vec<V>(xp + (t0 - 3 + k) * xst, win[k]);
-    }
-    const int t_own = min(t0 + CV_T, L);
-    // three steps beyond the tile: their dpre reaches back into it
-#pragma unroll 1
-    for (int s = 0; s < CV_T + 3; s += 4) {
-      uint2 rx[4], rg[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        rx[u] = rg[u] = make_uint2(0u, 0u);
-        const int t = t0 + s + u;
-        if (t < L && s + u < CV_T + 3) {
-          rx[u] = *reinterpret_cast<const uint2*>(xp + t * xst);
-          rg[u] = *reinterpret_cast<const uint2*>(gp + t * dst);
+      for (int k = 0; k < CV_G; ++k) {
+        u[k] = g[k] = make_uint2(0u, 0u);
+        if (t + k < t_end) {
+          u[k] = *reinterpret_cast<const uint2*>(xp + (t + k) * xst);
+          g[k] = *reinterpret_cast<const uint2*>(gp + (t + k) * dst);
         }
       }
+    };
+    Conv4 wk[4], bv, win[3], dp[3] = {};
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int t = t0 + s + u, to = t - 3;
-        const float2 x0 = unpack_h16x2(rx[u].x), x1 = unpack_h16x2(rx[u].y);
-        const float2 g0 = unpack_h16x2(rg[u].x), g1 = unpack_h16x2(rg[u].y);
-        const float xc[4] = {x0.x, x0.y, x1.x, x1.y}, gc[4] = {g0.x, g0.y, g1.x, g1.y};
-        float o[V];
+    for (int k = 0; k < 3; ++k) {
+      uint2 u = make_uint2(0u, 0u);
+      if (t0 - 3 + k >= 0) u = *reinterpret_cast<const uint2*>(xp + (t0 - 3 + k) * xst);
+      win[k] = conv_unpack(u);
+    }
+    conv_taps(w, bias, d, W, wk, bv);
+#pragma unroll 1
+    for (int s = 0; s < CV_BWD_T + 3; s += CV_G) {
+      fetch(t0 + s, rx, rg);
 #pragma unroll
-        for (int c = 0; c < V; ++c) {
-          const float pre = bv[c] + wk[c][0] * win[0][c] + wk[c][1] * win[1][c] + wk[c][2] * win[2][c] + wk[c][3] * xc[c];
-          const float dpre = gc[c] * silu_grad(pre);      // 0 beyond the sequence: dy was read as 0 there
-          if (t < t_own) {
-            aw[c][0] += dpre * win[0][c]; aw[c][1] += dpre * win[1][c]; aw[c][2] += dpre * win[2][c];
-            aw[c][3] += dpre * xc[c];
-            aw[c][4] += dpre;
-          }
-          o[c] = wk[c][3] * dp[0][c] + wk[c][2] * dp[1][c] + wk[c][1] * dp[2][c] + wk[c][0] * dpre;
-          win[0][c] = win[1][c]; win[1][c] = win[2][c]; win[2][c] = xc[c];
-          dp[0][c] = dp[1][c]; dp[1][c] = dp[2][c]; dp[2][c] = dpre;
+      for (int k = 0; k < CV_G; ++k) {
+        const int t = t0 + s + k, to = t - 3;
+        const Conv4 cur = conv_unpack(rx[k]), pre = conv_pre(wk, bv, win, cur), sg = conv_sigmoid(pre);
+        // silu' = s (1 + x (1 - s)); 0 beyond the sequence: dy was read as 0 there
+        auto grad = [](float2 xx, float2 ss) {
+          return fmul2(ss, ffma2(xx, ffma2(ss, make_float2(-1.f, -1.f), make_float2(1.f, 1.f)), make_float2(1.f, 1.f)));
+        };
+        const Conv4 dpre = conv_mul(conv_unpack(rg[k]), {grad(pre.a, sg.a), grad(pre.b, sg.b)});
+        if (t < t_own) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) aw[c] = conv_fma(dpre, win[c], aw[c]);
+          aw[3] = conv_fma(dpre, cur, aw[3]);
+          aw[4] = {fadd2(aw[4].a, dpre.a), fadd2(aw[4].b, dpre.b)};
         }
-        if (to >= t0 && to < t_own) store_vec<V>(dx + b * gsb + to * gst + d, o);
+        if (to >= t0 && to < t_own)
+          *reinterpret_cast<uint2*>(dx + b * gsb + to * gst + d) =
+              conv_pack(conv_fma(wk[0], dpre, conv_fma(wk[1], dp[2], conv_fma(wk[2], dp[1], conv_mul(wk[3], dp[0])))));
+        win[0] = win[1]; win[1] = win[2]; win[2] = cur;
+        dp[0] = dp[1]; dp[1] = dp[2]; dp[2] = dpre;
       }
     }
   }
   // one atomic per block and parameter: the block's time tiles are summed in shared memory first
 #pragma unroll
-  for (int c = 0; c < V; ++c)
-#pragma unroll
-    for (int k = 0; k < 5; ++k) red[threadIdx.y][threadIdx.x][c * 5 + k] = aw[c][k];
+  for (int k = 0; k < 5; ++k) {
+    float* r = red[threadIdx.y][threadIdx.x] + k;
+    r[0] = aw[k].a.x; r[5] = aw[k].a.y; r[10] = aw[k].b.x; r[15] = aw[k].b.y;
+  }
   __syncthreads();
-  for (int i = threadIdx.y * CV_X + threadIdx.x; i < CV_X * V * 5; i += CV_X * CV_Y) {
-    const int gx = i / (V * 5), r = i % (V * 5), ch = (blockIdx.x * CV_X + gx) * V + r / 5, k = r % 5;
+  for (int i = threadIdx.y * CV_X + threadIdx.x; i < CV_X * CV_V * 5; i += CV_X * CV_Y) {
+    const int gx = i / (CV_V * 5), r = i % (CV_V * 5), ch = (blockIdx.x * CV_X + gx) * CV_V + r / 5, k = r % 5;
     if (ch >= D) continue;
     float a = 0.f;
 #pragma unroll
@@ -289,16 +273,16 @@ conv1d_silu_bwd_vec_kernel(const h16* __restrict__ x, long long xsb, long long x
 static bool vec_ok(const void* p, long long sb, long long st, int V) {
   return (reinterpret_cast<uintptr_t>(p) & (V * 2 - 1)) == 0 && sb % V == 0 && st % V == 0;
 }
-static dim3 conv_vec_grid(int B, int L, int D, int V) {
-  return dim3((D / V + CV_X - 1) / CV_X, (L + CV_T * CV_Y - 1) / (CV_T * CV_Y), B);
+static dim3 conv_vec_grid(int B, int L, int D, int steps) {
+  return dim3((D / CV_V + CV_X - 1) / CV_X, (L + steps * CV_Y - 1) / (steps * CV_Y), B);
 }
 
 NX_API int NX_SYM(nx_conv1d_silu_fwd)(const void* x, long long xsb, long long xst, const void* w, const void* bias,
                               void* y, long long ysb, long long yst, int B, int L, int D, int W,
                               cudaStream_t stream) {
   NX_REQUIRE(W >= 1 && W <= 4, "conv1d: kernel width %d not in [1, 4]", W);
-  if (D % CV_FWD_V == 0 && vec_ok(x, xsb, xst, CV_FWD_V) && vec_ok(y, ysb, yst, CV_FWD_V)) {
-    conv1d_silu_fwd_vec_kernel<<<conv_vec_grid(B, L, D, CV_FWD_V), dim3(CV_X, CV_Y), 0, stream>>>(
+  if (D % CV_V == 0 && vec_ok(x, xsb, xst, CV_V) && vec_ok(y, ysb, yst, CV_V)) {
+    conv1d_silu_fwd_vec_kernel<<<conv_vec_grid(B, L, D, CV_FWD_T), dim3(CV_X, CV_Y), 0, stream>>>(
         (const h16*)x, xsb, xst, (const h16*)w, (const h16*)bias, (h16*)y, ysb, yst, L, D, W);
     NX_LAUNCH_CHECK();
     return NX_OK;
@@ -316,9 +300,8 @@ NX_API int NX_SYM(nx_conv1d_silu_bwd)(const void* x, long long xsb, long long xs
                               long long gst, void* dw, void* dbias, int B, int L, int D, int W,
                               cudaStream_t stream) {
   NX_REQUIRE(W >= 1 && W <= 4, "conv1d: kernel width %d not in [1, 4]", W);
-  if (D % CV_BWD_V == 0 && vec_ok(x, xsb, xst, CV_BWD_V) && vec_ok(dy, dsb, dst, CV_BWD_V) &&
-      vec_ok(dx, gsb, gst, CV_BWD_V)) {
-    conv1d_silu_bwd_vec_kernel<<<conv_vec_grid(B, L, D, CV_BWD_V), dim3(CV_X, CV_Y), 0, stream>>>(
+  if (D % CV_V == 0 && vec_ok(x, xsb, xst, CV_V) && vec_ok(dy, dsb, dst, CV_V) && vec_ok(dx, gsb, gst, CV_V)) {
+    conv1d_silu_bwd_vec_kernel<<<conv_vec_grid(B, L, D, CV_BWD_T), dim3(CV_X, CV_Y), 0, stream>>>(
         (const h16*)x, xsb, xst, (const h16*)w, (const h16*)bias, (const h16*)dy, dsb, dst, (h16*)dx, gsb, gst,
         (float*)dw, (float*)dbias, L, D, W);
     NX_LAUNCH_CHECK();
