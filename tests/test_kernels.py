@@ -553,6 +553,25 @@ def test_flash_attention_backward_routes(b, s, h, hk, form, d):
         assert (x.float() - y).norm() <= 3 * eps * y.norm() + 1e-6
 
 
+@pytest.mark.parametrize("d", [8, 56, 64, 72, 128])
+@pytest.mark.parametrize("b,s,h", [(1, 1, 1), (2, 63, 3), (3, 129, 5), (1, 700, 40)])
+def test_flash_attention_backward_output_gradient_layouts(b, s, h, d):
+    """The layouts of the output's gradient (heads together, each head's rows together, rows on 16-byte boundaries only, one
+    broadcast row) take different forms of the kernel that sums O * dO over a row; all add in the same order."""
+    from gpt_neox_b200.ops.attention import flash_attention
+    torch.manual_seed(31)
+    ts = [bf(b, s, h, d, grad=True) for _ in range(3)]
+    grads = lambda g: torch.autograd.grad(flash_attention(*ts), ts, g)
+    g = bf(b, s, h, d)
+    by_head = g.transpose(1, 2).contiguous().transpose(1, 2)
+    room = torch.full((b, s, h, d + 8 if d % 16 == 0 else d), float("nan"), device=DEV, dtype=DT)
+    room[..., :d] = g
+    row = g[:1, :1, :1].expand(b, s, h, d)
+    for one, other in ((g, by_head), (g, room[..., :d]), (row.contiguous(), row)):
+        for x, y in zip(grads(one), grads(other)):
+            assert torch.equal(x, y)
+
+
 @pytest.mark.parametrize("env", [{"NEOX_ATTN_FWD_SHAPE": "1"}, {"NEOX_ATTN_FWD_SHAPE": "3"}], ids=["fwd_shape1", "fwd_shape3"])
 def test_flash_attention_selectable_kernel_shapes(env):
     """The kernel shapes that an environment variable selects instead of the defaults (read once per process, hence a
