@@ -21,8 +21,10 @@
 //              dL/d(ew_t) = Q_t - k_t (gk_t - r_t u s_t),  s_t = <gy_t, v_t>,  ew = -exp(w)
 // Step by step the shared-memory loads and exchanges of the steps are the bound (32 x 512 tokens, 12 heads of 64, forward +
 // backward 788 us).  With the products of a block in their place, and a block's vectors beside the former block's products, 570
-// (134 us for column sums, 123 for row sums, 159 for gk with the decay gradient).  No pipe is the bound then but latency, at 2.6
-// warps per scheduler: issue slots 48 / 51 / 47 % busy, tensor pipe 23 / 16 / 12 %.
+// (134 us for column sums, 123 for row sums, 159 for gk with the decay gradient); without bank conflicts on the decays 554 (129, 120,
+// 153).  The bound is latency between a block's steps, at 2.6 warps per scheduler (issue slots 48 - 51 % busy, tensor pipe 12 - 23 %)
+// but with shared memory about 70 % busy on an SM with three CTAs: twice the warps, a group for the vectors beside one for
+// the products, took 573 us (80 registers a thread; the same wavefronts, most warps at a barrier).
 //
 // The sequence is cut into chunks only when batch x heads leaves the chip idle (wkv_chunk_count): the recurrence is
 // linear, so a chunk's end state is  P (.) S_start + S_local  with P[i] = prod_t d_t[i]; local passes start every chunk
@@ -427,6 +429,10 @@ struct WmIn {
   }
 };
 
+// Where channel c stands in a row of 64 fp32 values that is written and read as halves of eight channels: with the halves of the
+// upper eights swapped, eight threads' halves lie in different banks.
+__device__ __forceinline__ int wm_at(int c) { return c ^ ((c >> 3) & 4); }
+
 // Whether all of eight bf16 inputs are below 2^20 (infinity and NaN are not).  Then no product over a block's vectors
 // overflows, and what one loses when it underflows is below 2^-100.
 __device__ __forceinline__ bool wm_ordinary(const uint4& u) {
@@ -536,8 +542,8 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_col_kernel(const WkvParams 
           sew[e + 1] += ew.y;
         }
       }
-      *reinterpret_cast<float4*>(&s.d[trow][ch8]) = make_float4(d8[0], d8[1], d8[2], d8[3]);
-      *reinterpret_cast<float4*>(&s.d[trow][ch8 + 4]) = make_float4(d8[4], d8[5], d8[6], d8[7]);
+      *reinterpret_cast<float4*>(&s.d[trow][wm_at(ch8)]) = make_float4(d8[0], d8[1], d8[2], d8[3]);
+      *reinterpret_cast<float4*>(&s.d[trow][wm_at(ch8 + 4)]) = make_float4(d8[4], d8[5], d8[6], d8[7]);
     }
     const int odd_input = __syncthreads_or(q < nblk && !(wm_ordinary(rb) && wm_ordinary(rc) && (LOCAL || wm_ordinary(ra))));
     if (tid == 0) now.odd_input = odd_input;
@@ -554,7 +560,7 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_col_kernel(const WkvParams 
       float2 pre = make_float2(1.f, 1.f);
 #pragma unroll 4
       for (int t = 0; t < WM; ++t) {
-        const float2 d = *reinterpret_cast<const float2*>(&s.d[t][c]);
+        const float2 d = *reinterpret_cast<const float2*>(&s.d[t][wm_at(c)]);
         if (!LOCAL) {
           uint32_t x[3];
           wm_split(fmul2(s.a.pair(t, c), pre), x);
@@ -569,7 +575,7 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_col_kernel(const WkvParams 
       float2 suf = make_float2(1.f, 1.f);
 #pragma unroll 4
       for (int t = WM - 1; t >= 0; --t) {
-        const float2 d = *reinterpret_cast<const float2*>(&s.d[t][c]);
+        const float2 d = *reinterpret_cast<const float2*>(&s.d[t][wm_at(c)]);
         uint32_t x[3];
         wm_split(fmul2(s.b.pair(t, c), suf), x);
 #pragma unroll
@@ -591,7 +597,8 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_col_kernel(const WkvParams 
         if (it == turn) load_b(turn);
         const int t = it < turn ? g + 1 + it : turn + 1 + (it - turn);
         float2 acc = make_float2(0.f, 0.f);
-        const float4 d0 = *reinterpret_cast<const float4*>(&s.d[t][c]), d1 = *reinterpret_cast<const float4*>(&s.d[t][c + 4]);
+        const float4 d0 = *reinterpret_cast<const float4*>(&s.d[t][wm_at(c)]),
+                     d1 = *reinterpret_cast<const float4*>(&s.d[t][wm_at(c + 4)]);
         const float2 dd[4] = {{d0.x, d0.y}, {d0.z, d0.w}, {d1.x, d1.y}, {d1.z, d1.w}};
         const uint4 u = *reinterpret_cast<const uint4*>(&s.a.raw[t][c]);
         const uint32_t aw[4] = {u.x, u.y, u.z, u.w};
@@ -868,10 +875,15 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_row_kernel(const WkvParams 
       float w8[8];
       wk_unpack8(rw, w8);
 #pragma unroll
-      for (int e = 0; e < 8; e += 2) {
-        const float2 ew = live ? make_float2(-__expf(w8[e]), -__expf(w8[e + 1])) : make_float2(0.f, 0.f);
-        *reinterpret_cast<float2*>(&now.ew[trow][ch8 + e]) = ew;
-        *reinterpret_cast<float2*>(&s.d[trow][ch8 + e]) = wm_decay(ew);
+      for (int e = 0; e < 8; e += 4) {
+        float2 ew[2], d[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          ew[k] = live ? make_float2(-__expf(w8[e + 2 * k]), -__expf(w8[e + 2 * k + 1])) : make_float2(0.f, 0.f);
+          d[k] = wm_decay(ew[k]);
+        }
+        *reinterpret_cast<float4*>(&now.ew[trow][wm_at(ch8 + e)]) = make_float4(ew[0].x, ew[0].y, ew[1].x, ew[1].y);
+        *reinterpret_cast<float4*>(&s.d[trow][wm_at(ch8 + e)]) = make_float4(d[0].x, d[0].y, d[1].x, d[1].y);
       }
     }
     }
@@ -906,7 +918,7 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_row_kernel(const WkvParams 
 #pragma unroll 1
       for (int x = 0; x < steps; ++x) {
         const float b0 = former.b.at(x, r0), b1 = former.b.at(x, r0 + 8);
-        const float2 d = wm_decay(make_float2(former.ew[x][r0], former.ew[x][r0 + 8]));
+        const float2 d = wm_decay(make_float2(former.ew[x][wm_at(r0)], former.ew[x][wm_at(r0 + 8)]));
         float y0 = 0.f, y1 = 0.f, st = 0.f;
 #pragma unroll
         for (int n = 0; n < 8; ++n)
@@ -1010,7 +1022,7 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_row_kernel(const WkvParams 
         const float gk = row + u_me * r_ * st;
         const long long o = oo + (long long)(t_hi - 1 - (q - 1) * WM - t) * p.ost;
         p.o_gk[o] = float_to_h16(gk);
-        p.o_gw[o] = float_to_h16((Q - k_ * row) * former.ew[t][me]);
+        p.o_gw[o] = float_to_h16((Q - k_ * row) * former.ew[t][wm_at(me)]);
         Q += r_ * gr[REV ? t : 0] - k_ * gk;
         gu += r_ * k_ * st;
       }
@@ -1022,7 +1034,7 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_row_kernel(const WkvParams 
       float qv[8], pre = 1.f;
 #pragma unroll
       for (int t = 0; t < WM; ++t) {
-        const float d = s.d[t][me];
+        const float d = s.d[t][wm_at(me)];
         float acc = 0.f;
         const float4 m0 = *reinterpret_cast<const float4*>(&s.M[half][t][0]), m1 = *reinterpret_cast<const float4*>(&s.M[half][t][4]);
         const float m[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
