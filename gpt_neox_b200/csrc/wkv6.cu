@@ -33,6 +33,7 @@
 
 #include "common.h"
 #include "ptx.cuh"
+#include "reduce.cuh"
 
 namespace nx {
 
@@ -72,6 +73,21 @@ __device__ __forceinline__ uint4 wk_load8(const h16* p, bool ok) {
 __device__ __forceinline__ void wk_unpack8(const uint4& u, float (&f)[8]) {
   const float2 a = unpack_h16x2(u.x), b = unpack_h16x2(u.y), c = unpack_h16x2(u.z), d = unpack_h16x2(u.w);
   f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+}
+
+// out[i] = <g[i], f[i]> of two states, N / 16 warps: each takes its rows one after the other, a row's values side by side (a thread
+// per row, as it was, reads N lines at a time: 16 us of the 25 us of a reverse sweep of one block of steps).
+template <int N>
+__device__ __forceinline__ void wk_state_dots(const float* g, const float* f, float* out, int warp, int lane) {
+#pragma unroll 8
+  for (int x = 0; x < 16; ++x) {
+    const int i = warp * 16 + x;
+    float v = 0.f;
+#pragma unroll
+    for (int j = lane; j < N; j += 32) v += g[i * N + j] * f[i * N + j];
+    v = warp_sum(v);
+    if (lane == 0) out[i] = v;
+  }
 }
 
 template <int N, int MODE>
@@ -120,10 +136,10 @@ __global__ void __launch_bounds__(2 * N) wkv_kernel(const WkvParams p) {
   const int me = threadIdx.x % N, second = threadIdx.x / N;
   float Q = 0.f, gu = 0.f;
   const float u_me = p.u[h * N + me];
-  if (MODE == WK_G && !second && p.fstart != nullptr && c + 1 < p.NC) {
-    const float* g = p.start + (base * N + me) * N;
-    const float* f = p.fstart + ((base + 1) * N + me) * N;
-    for (int j = 0; j < N; ++j) Q += g[j] * f[j];
+  if (MODE == WK_G && p.fstart != nullptr && c + 1 < p.NC) {
+    wk_state_dots<N>(p.start + base * N * N, p.fstart + (base + 1) * N * N, &s.colsum[0][0], warp, lane);
+    __syncthreads();
+    Q = s.colsum[0][me];
   }
   // ---- staging role: step trow, 8 channels from ch8
   const int trow = threadIdx.x / TPR, ch8 = (threadIdx.x % TPR) * 8;
@@ -839,10 +855,10 @@ __global__ void __launch_bounds__(WM_THREADS, 3) wkv_row_kernel(const WkvParams 
   const int me = tid & (WN - 1), half = tid >> 6;
   const float u_me = p.u[h * WN + me];
   float Q = 0.f, gu = 0.f;
-  if (REV && half == 0 && p.fstart != nullptr && ch + 1 < p.NC) {
-    const float* g = p.start + (base * WN + me) * WN;
-    const float* f = p.fstart + ((base + 1) * WN + me) * WN;
-    for (int j = 0; j < WN; ++j) Q += g[j] * f[j];
+  if (REV && p.fstart != nullptr && ch + 1 < p.NC) {
+    wk_state_dots<WN>(p.start + base * WN * WN, p.fstart + (base + 1) * WN * WN, &s.inter[0][0], warp, lane);
+    __syncthreads();
+    Q = s.inter[0][me];
   }
   const int trow = tid >> 3, ch8 = (tid & 7) * 8;
   const int nblk = (t_hi - t_lo + WM - 1) / WM;
