@@ -1137,13 +1137,23 @@ static int wkv_launch(const WkvParams& p, bool vec, int chunks, cudaStream_t str
   return NX_OK;
 }
 
-// Chunks the sequence is cut into.  The sweeps are bound by latency until an SM holds WK_CTAS CTAs, so time goes with the
-// chunk length times the number of rounds the CTAs take; more than one chunk adds the local passes over all chunks but one, and
-// the fold.  The weights come from the step-by-step sweeps; in blocks, every count from 1 to 32 tried, the rule's is the best or
-// within 10 % of it for 1 - 64 sequences of 50 - 8192 steps (1 x 512, 12 heads: 32 chunks 83 us, 16 76; 4 x 2048 9 chunks 364, 4
-// 570; 8 x 2048, 16 heads 3 chunks 920, 10 909; 32 x 512, 12 heads 1 chunk 556, 2 674) but for 40 x 512, 12 heads, whose CTAs just
-// exceed a round: 8 chunks 1010, 1 887.  The count depends on the batch, and the chunks' states are folded in
-// fp32: a sequence's last bits are not those it has in another batch.
+// Which calls go in blocks: bf16 (an fp16 input would take two parts, and its products twice to four times as many: 32 x 512, 12
+// heads 997 us, step by step 780; 8 x 2048, 16 heads 1,508 against 1,363), and not a few short sequences, where the fourth
+// sweep's launch and a block's latency count (forward + backward, step by step / in blocks: 1 x 16, 12 heads 0.89, 8 x 16
+// 0.87, 4 x 32 0.95, 1 x 128, 8 heads 0.97; 16 x 16 0.99, 32 x 16 1.11, 8 x 64, 8 heads 1.07, 1 x 200, 16 heads 1.05).
+static bool wkv_in_blocks(int B, int T, int H, int N) {
+  return WM_BLOCKS && N == WN && (T > 128 || static_cast<long long>(B) * H * T >= 3072);
+}
+
+// Chunks the sequence is cut into.  A block of steps of the sweeps takes as long as the SM's CTAs need: latency until it holds
+// WK_CTAS, so with one or two CTAs 2/3 and 5/6 of the time with three, which also holds for the CTAs left over by full rounds
+// (40 x 512, 12 heads: 480 CTAs on 444 places take 1.62 rounds).  More than one chunk adds the local passes over all chunks but one,
+// the fold's launches and chain, and the states' traffic.  In units of a round of a block, 16.6 us.  Times of forward + backward
+// by the number of chunks, this rule's first: 1 x 512, 12 heads 16: 67 us, 32: 67, 8: 78; 4 x 2048 9: 337, 8: 355, 16: 373, 1: 1387;
+// 8 x 2048, 16 heads 10: 850, 3: 877, 1: 1437; 40 x 300, 12 heads 1: 515, 3: 542, 19: 908 (the choice when only rounds and steps
+// were counted); 40 x 512 4: 823, 1: 860, 8: 900; 16 x 1000, 16 heads 5: 844, 1: 871; 10 x 400, 12 heads 3: 207, 1: 267.  Step by
+// step (LOCAL is as long as the others there) whole rounds and more for the local passes.  The count depends on the batch,
+// and the chunks' states are folded in fp32: a sequence's last bits are not those it has in another batch.
 constexpr int WK_CTAS = 3;
 static int wkv_chunk_count(int B, int T, int H) {
   const int subs = (T + WK_SUB - 1) / WK_SUB, slots = WK_CTAS * sm_count();
@@ -1152,8 +1162,14 @@ static int wkv_chunk_count(int B, int T, int H) {
   for (int nc = 1; nc <= WK_MAX_CHUNKS && nc <= subs; ++nc) {
     const int len = (subs + nc - 1) / nc;
     if ((subs + len - 1) / len != nc) continue;
-    const long long rounds = (static_cast<long long>(B) * H * nc + slots - 1) / slots;
-    const float cost = len * rounds * (1.f + 0.67f * (nc - 1) / nc) + (nc > 1 ? 0.5f + 0.1f * nc : 0.f);
+    const long long ctas = static_cast<long long>(B) * H * nc, full = ctas / slots, rest = ctas - full * slots;
+    const int per_sm = static_cast<int>((rest + sm_count() - 1) / sm_count());
+    float cost;
+    if (wkv_in_blocks(B, T, H, WN))
+      cost = len * (full + (rest > 0 ? 0.5f + per_sm / 6.f : 0.f)) * (1.f + 0.3f * (nc - 1) / nc) +
+             (nc > 1 ? 1.5f + 0.05f * nc + 0.0015f * ctas : 0.f);
+    else
+      cost = len * (full + (rest > 0)) * (1.f + 0.67f * (nc - 1) / nc) + (nc > 1 ? 0.5f + 0.1f * nc : 0.f);
     if (cost < best_cost) {
       best_cost = cost;
       best = nc;
@@ -1183,14 +1199,6 @@ static int wkv_col(const WkvParams& p, bool vec, int chunks, cudaStream_t stream
 template <bool REV>
 static int wkv_row(const WkvParams& p, bool vec, cudaStream_t stream) {
   return wkv64_launch<WmRowSmem>(wkv_row_kernel<REV, true>, wkv_row_kernel<REV, false>, p, vec, p.NC, stream);
-}
-
-// Which calls go in blocks: bf16 (an fp16 input would take two parts, and its products twice to four times as many: 32 x 512, 12
-// heads 997 us, step by step 780; 8 x 2048, 16 heads 1,508 against 1,363), and not a few short sequences, where the fourth
-// sweep's launch and a block's latency count (forward + backward, step by step / in blocks: 1 x 16, 12 heads 0.89, 8 x 16
-// 0.87, 4 x 32 0.95, 1 x 128, 8 heads 0.97; 16 x 16 0.99, 32 x 16 1.11, 8 x 64, 8 heads 1.07, 1 x 200, 16 heads 1.05).
-static bool wkv_in_blocks(int B, int T, int H, int N) {
-  return WM_BLOCKS && N == WN && (T > 128 || static_cast<long long>(B) * H * T >= 3072);
 }
 
 // One sweep, in blocks or step by step.

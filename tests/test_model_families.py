@@ -193,7 +193,7 @@ def test_wkv6_passes_nan_and_inf_on(what, value, at):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("B,T,H", [(32, 512, 12), (8, 2048, 16)])        # chunks of 512 and of 688 steps
+@pytest.mark.parametrize("B,T,H", [(32, 512, 12), (8, 2048, 16)])        # chunks of 512 and of 208 steps
 @pytest.mark.parametrize("w", [-12.0, -1.0])
 def test_wkv6_long_sweeps(B, T, H, w, dtype):
     """Many blocks of steps in one CTA, with decays that keep the state and that forget it, against 64 bits: all results, and the
@@ -221,7 +221,7 @@ def test_wkv6_long_sweeps(B, T, H, w, dtype):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("B,T,H", [(32, 512, 12), (8, 2048, 16)])        # chunks of 512 and of 688 steps
+@pytest.mark.parametrize("B,T,H", [(32, 512, 12), (8, 2048, 16)])        # chunks of 512 and of 208 steps
 @pytest.mark.parametrize("w", [-12.0, -6.0, -1.0])
 def test_wkv6_row_sums_have_fp32_precision(B, T, H, w):
     """The gradient of r before it is rounded, which the decay gradient is made of: an error of a last bit per step that adds
@@ -247,6 +247,15 @@ def test_wkv6_row_sums_have_fp32_precision(B, T, H, w):
     want = _wkv6_sweeps(*part, u[:2].double(), gy[:1, :, :2 * N].double())[1]
     err = gr32[:1, :, :2 * N].double() - want
     assert err.norm() <= 2 ** -24 * (min(T, 700) ** 0.5 / 2 + 1) * want.norm()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,T,H", [(27, 2048, 16), (16, 700, 12), (40, 512, 12), (8, 333, 16)])
+@pytest.mark.parametrize("w", [-12.0, -1.0])
+def test_wkv6_chunks_of_all_lengths(B, T, H, w):
+    """On 148 SMs one chunk of 2048 steps, two of 352, four of 128 and three of 112, ragged ones among them: what
+    test_wkv6_long_sweeps asks for, of sequences whose reverse sweeps begin with the products of two states."""
+    test_wkv6_long_sweeps(B, T, H, w, torch.bfloat16)
 
 
 def _wkv6_sweeps(r, k, v, w, u, gy):
