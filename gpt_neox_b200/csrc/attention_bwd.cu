@@ -18,15 +18,14 @@
 //   warps 1, 2  tcgen05.mma issuers, one for the scores (which runs ahead, across items), one for the products
 //   warps 4 ..  element-wise: dQ eight warps, 64 of a block's key columns each; dK / dV two sets of eight warps (32 query
 //               columns each) that take the blocks in turn, so that one set's waits lie under the other's arithmetic.  They also
-//               store a finished item's accumulators, after the next item's first block.
+//               store a finished item's accumulators (a set dK, the other dV), beside the next item's first block.
 // What bounds them (cycle counts of the roles): neither the tensor cores nor the exponentials but the chain scores -> registers
 // -> 16-bit results -> products, with about 500 cycles from a commit or an arrival to the warp that waits for it, so a block
-// costs dQ 2,300 cycles (MMAs 1,536, exponentials 1,024) and dK / dV 1,750 per 64 queries (MMAs 1,024: one pair of result
-// buffers is all that the accumulators leave).  Hence everything that lets blocks overlap: issuers apart from each other (one
+// costs dQ 2,300 cycles (MMAs 1,536, exponentials 1,024) and dK / dV 1,650 per 64 queries (MMAs 1,024).  Hence everything that lets blocks overlap: issuers apart from each other (one
 // thread issuing all was the bound at 1,700 cycles per 64 rows), scores two blocks ahead, score buffers given back as soon as
 // they are in registers, the next item's tiles and stores in the shadow of the running one.
-// Batch 4, 32 heads, 2048 x 128 causal: dQ 290 -> 202 us, dK / dV 324 -> 293 us; 5003 tokens, 32 heads on 8, window of 4096:
-// 326 -> 238 us and 435 -> 325 us (before: one CTA per tile).  What was slower: two groups of four warps that write their
+// Batch 4, 32 heads, 2048 x 128 causal: dQ 290 -> 202 us, dK / dV 324 -> 275 us; 5003 tokens, 32 heads on 8, window of 4096:
+// 326 -> 238 us and 435 -> 299 us (before: one CTA per tile).  What was slower: two groups of four warps that write their
 // results over their scores (260 / 333 us), dQ by 16 warps with 32 columns each (215 us), dQ with two K stages (258 us), one V
 // stage (212 us).
 #include "attention_bwd.h"
@@ -110,14 +109,15 @@ static_assert(BWD_STAGES * 2 * 64 * 4 <= 2 * BwdSmem<64>::T64, "lse / delta fit 
 
 // Barriers.  RES: the two resident tiles; STR / STR2: rings of streamed tiles (STR2: V of the dQ kernel); S: scores of block n
 // in buffer n & 1 written by the tensor core (FULL), in the element-wise warps' registers (EMPTY: dK / dV); DP: the same of the
-// one dP buffer (dK / dV: FULL per set); P_FULL: the 16-bit results of block n written.  That these are consumed STR_EMPTY
+// dP buffer (dK / dV: buffer n & 1, FULL only); P_FULL: the 16-bit results of block n written.  That these are consumed STR_EMPTY
 // tells: the products of a block are its stage's last readers.  ACC: an item's accumulators complete / read.
 enum { RES_FULL = 0, RES_EMPTY = 2, STR_FULL = 4, STR_EMPTY = 8, STR2_FULL = 12, STR2_EMPTY = 14, S_FULL = 16, S_EMPTY = 18,
        DP_FULL = 20, DP_EMPTY = 22, P_FULL = 23, ACC_FULL = 25, ACC_EMPTY = 26, BWD_NBAR = 27 };
-__device__ __forceinline__ void bwd_init_barriers(uint32_t bar0) {
+__device__ __forceinline__ void bwd_init_barriers(uint32_t bar0, int element_warps) {
   for (int i = 0; i < BWD_NBAR; ++i) {
-    const bool by_warps = i == S_EMPTY || i == S_EMPTY + 1 || i == DP_EMPTY || i == P_FULL || i == P_FULL + 1 || i == ACC_EMPTY;
-    mbar_init(bar0 + 8u * i, by_warps ? 8 : 1);     // one arrival per element-wise warp that shares a block
+    const bool by_warps = i == S_EMPTY || i == S_EMPTY + 1 || i == DP_EMPTY || i == P_FULL || i == P_FULL + 1;
+    // one arrival per element-wise warp that shares a block; of all of them
+    mbar_init(bar0 + 8u * i, by_warps ? 8 : i == ACC_EMPTY ? element_warps : 1);
   }
   fence_barrier_init();
 }
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int off = p.Sk - p.Sq;
   const DqWork work(p);
-  if (threadIdx.x == 0) bwd_init_barriers(bar0);
+  if (threadIdx.x == 0) bwd_init_barriers(bar0, 8);
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
@@ -598,8 +598,11 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
 // ------------------------------------------------------------------------------------------------
 // dK / dV kernel.  Resident: K, V (128 rows).  Streamed: Q, dO (64 rows) with their lse / delta.  Two sets of eight element-wise
 // warps (32 query columns each) take the blocks in turn, so that one set's waits lie under the other's arithmetic.
-// TMEM: S^T of block n at [64 (n & 1), ...), dP^T [128, 192), P^T [192, 224), dS^T [224, 256), dK [256, 256 + DP), dV [384, 384 +
-// DP).
+// TMEM: S^T of block n at [64 (n & 1), ...), dP^T [128 + 64 (n & 1), ...), dK [256, 256 + DP), dV [384, 384 + DP).  A warp's P^T and
+// dS^T (16 columns each) take the place of its own 32 columns of dP^T, which thus has two buffers as the scores have: with one, and
+// one pair for the results, two chains of two handoffs each held a block (294 us, batch 4, 32 heads, 2048 x 128 causal; now 275;
+// results in the place of the scores, three buffers of them and one of dP^T 287).  What bounds a block now is the element-wise
+// warps: a set is busy for 2,600 cycles of a block of its own, 1,300 per block, at 8 cycles an instruction.
 // ------------------------------------------------------------------------------------------------
 template <int DP, bool ALIBI>
 __global__ void __launch_bounds__(DKV_THREADS, 1)
@@ -616,12 +619,12 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
   volatile uint32_t* tmem_slot_gen = reinterpret_cast<volatile uint32_t*>(sgen + L::BAR_OFF + 8 * BWD_NBAR);
   auto res = [&](int which) { return sbase + which * (2 * L::T64); };
   auto str = [&](int stage, int which) { return sbase + L::STR_OFF + (stage * 2 + which) * L::T64; };
-  constexpr uint32_t T_DP = 128, T_P = 192, T_DS = 224, T_DK = 256, T_DV = 384;
+  constexpr uint32_t T_DP = 128, T_DK = 256, T_DV = 384;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int off = p.Sk - p.Sq;
   const DkvWork work(p);
-  if (threadIdx.x == 0) bwd_init_barriers(bar0);
+  if (threadIdx.x == 0) bwd_init_barriers(bar0, 16);
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
@@ -690,13 +693,14 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
         mma_nt<DP, ABS>(leader, tmem + (n & 1) * ABS, res(0), str(st, 0));
         umma_commit_by(leader, bar(S_FULL, n & 1));
         if (last) umma_commit_by(leader, bar(RES_EMPTY, 0));
+        // (the products of block n - 2: its stage, two back in the ring, and the phase of that use)
         if ((!any && !warp_wait(bar(RES_FULL, 1), t & 1, p.err, 64)) ||
-            !warp_wait(bar(DP_EMPTY, 0), (n & 1) ^ 1, p.err, 62)) {
+            (n >= 2 && !warp_wait(bar(STR_EMPTY, (n - 2) % BWD_STAGES), ((n - 2) / BWD_STAGES) & 1, p.err, 62))) {
           aborted = true;
           break;
         }
         tc_fence_after_sync();
-        mma_nt<DP, ABS>(leader, tmem + T_DP, res(1), str(st, 1));
+        mma_nt<DP, ABS>(leader, tmem + T_DP + (n & 1) * ABS, res(1), str(st, 1));
         umma_commit_by(leader, bar(DP_FULL, n & 1));
         if (last) umma_commit_by(leader, bar(RES_EMPTY, 1));
         any = true;
@@ -716,15 +720,15 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
     while (!aborted && work.next(round, it)) {
       bool any = false;
       for (int j = 0; j < it.j1; ++j) {
-        const int h = n & 1;
+        const uint32_t t_p = tmem + T_DP + (n & 1) * ABS;
         if ((!any && !warp_wait(bar(ACC_EMPTY, 0), (t & 1) ^ 1, p.err, 55)) ||
-            !warp_wait(bar(P_FULL, h), (n >> 1) & 1, p.err, 56)) {
+            !warp_wait(bar(P_FULL, n & 1), (n >> 1) & 1, p.err, 56)) {
           aborted = true;
           break;
         }
         tc_fence_after_sync();
-        mma_ts<DP, ABS>(leader, tmem + T_DV, tmem + T_P, 16, str(st, 1), any);
-        mma_ts<DP, ABS>(leader, tmem + T_DK, tmem + T_DS, 16, str(st, 0), any);
+        mma_ts<DP, ABS>(leader, tmem + T_DV, t_p, 32, str(st, 1), any);
+        mma_ts<DP, ABS>(leader, tmem + T_DK, t_p + 16, 32, str(st, 0), any);
         umma_commit_by(leader, bar(STR_EMPTY, st));
         any = true;
         ++n;
@@ -740,14 +744,15 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
     const int quad = warp & 3, h = (warp - 4) >> 3, half = (warp >> 2) & 1;
     const int r = quad * 32 + lane, c0 = half * 32;      // key row in tile; first of this warp's 32 query columns of a block
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t t_s = tmem + h * ABS + c0 + lane_off, t_dp = tmem + T_DP + c0 + lane_off,
-                   t_p = tmem + T_P + c0 / 2 + lane_off, t_ds = t_p + (T_DS - T_P);
+    const uint32_t t_s = tmem + h * ABS + c0 + lane_off, t_dp = t_s + T_DP;
     int n = 0, round = -1, t = 0, st = 0;
     uint32_t ph = 0;
     BwdItem it;
-    bool pending = false;      // `done`: an item whose gradients this warp has still to store (set 0 stores)
+    bool pending = false;      // `done`: an item whose gradients this warp has still to store
     BwdItem done;
-    const bool stores = half * 64 < DP;      // (64 columns of dK and of dV per warp; dK carries the softmax scale of dS)
+    // 64 columns per warp, of dK (set 0; it carries the softmax scale of dS) or of dV (set 1: one set that stored both was the later
+    // one, at 11 % of its time)
+    const bool stores = half * 64 < DP;
     auto finish = [&](const BwdItem& i, bool live) -> bool {
       uint32_t lo[32], hi[32];
 #pragma unroll
@@ -756,20 +761,16 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
         const bool ok = mbar_wait(bar(ACC_FULL, 0), t & 1, p.err, 59);
         if (!__all_sync(0xffffffffu, ok)) return false;
         tc_fence_after_sync();
-        if (stores) bwd_acc_load(tmem + T_DK + half * 64 + lane_off, lo, hi);
-      }
-      const int row = i.tile * AB + quad * 32;
-      if (stores)
-        bwd_store(p.dk + i.batch * p.dk_sb + i.head * p.dk_sh, p.dk_ss, lo, hi, p.scale, half * 64, row, p.Sk, p.D);
-      if (live) {
-        if (stores) bwd_acc_load(tmem + T_DV + half * 64 + lane_off, lo, hi);
+        if (stores) bwd_acc_load(tmem + (h == 0 ? T_DK : T_DV) + half * 64 + lane_off, lo, hi);
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(ACC_EMPTY, 0));
         ++t;
       }
-      if (stores)
-        bwd_store(p.dv + i.batch * p.dv_sb + i.head * p.dv_sh, p.dv_ss, lo, hi, 1.f, half * 64, row, p.Sk, p.D);
+      if (stores) {
+        h16* out = h == 0 ? p.dk + i.batch * p.dk_sb + i.head * p.dk_sh : p.dv + i.batch * p.dv_sb + i.head * p.dv_sh;
+        bwd_store(out, h == 0 ? p.dk_ss : p.dv_ss, lo, hi, h == 0 ? p.scale : 1.f, half * 64, i.tile * AB + quad * 32, p.Sk, p.D);
+      }
       return true;
     };
     auto wait = [&](int which, int idx, uint32_t parity, int where) -> bool {
@@ -869,9 +870,6 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
         tmem_ld_32x32b_x32(t_dp, dv);           // in flight during the second half's exponentials
         probs(16);
         tmem_ld_wait_for(dv);
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(DP_EMPTY, 0));
         uint32_t pd[16];
         const float2 m1 = make_float2(-1.f, -1.f);
 #pragma unroll
@@ -882,20 +880,15 @@ __global__ void __launch_bounds__(DKV_THREADS, 1)
           pd[e >> 1] = pack_h16x2(s0.x, s0.y);
           pd[(e >> 1) + 1] = pack_h16x2(s1.x, s1.y);
         }
-        // the products have taken block i - 1's results (its stage, one back in the ring, and the phase of that use)
-        if (i > 0 && !wait(STR_EMPTY, cur == 0 ? BWD_STAGES - 1 : cur - 1, cur == 0 ? cur_ph ^ 1 : cur_ph, 61)) {
-          aborted = true;
-          break;
-        }
-        tmem_st_32x32b_x16(t_p, pk);
-        tmem_st_32x32b_x16(t_ds, pd);
+        tmem_st_32x32b_x16(t_dp, pk);
+        tmem_st_32x32b_x16(t_dp + 16, pd);
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(P_FULL, h));
         if (store_former && !finish(done, true)) { aborted = true; break; }
       }
-      if (!aborted && h == 0) {
+      if (!aborted) {
         if (!first) {
           done = it;
           pending = true;
