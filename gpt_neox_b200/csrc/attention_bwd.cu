@@ -21,9 +21,10 @@
 //               store a finished item's accumulators (a set dK, the other dV), beside the next item's first block.
 // What bounds them (cycle counts of the roles): neither the tensor cores nor the exponentials but the chain scores -> registers
 // -> 16-bit results -> products, with about 500 cycles from a commit or an arrival to the warp that waits for it, so a block
-// costs dQ 2,300 cycles (MMAs 1,536, exponentials 1,024) and dK / dV 1,650 per 64 queries (MMAs 1,024).  Hence everything that lets blocks overlap: issuers apart from each other (one
-// thread issuing all was the bound at 1,700 cycles per 64 rows), scores two blocks ahead, score buffers given back as soon as
-// they are in registers, the next item's tiles and stores in the shadow of the running one.
+// costs dQ 2,300 cycles (MMAs 1,536, exponentials 1,024) and dK / dV 1,650 per 64 queries (MMAs 1,024).  Hence everything that
+// lets blocks overlap: issuers apart from each other (one thread issuing all was the bound at 1,700 cycles per 64 rows), scores
+// two blocks ahead, score buffers given back as soon as they are in registers, the next item's tiles and stores in the shadow of
+// the running one.
 // Batch 4, 32 heads, 2048 x 128 causal: dQ 290 -> 202 us, dK / dV 324 -> 275 us; 5003 tokens, 32 heads on 8, window of 4096:
 // 326 -> 238 us and 435 -> 299 us (before: one CTA per tile).  What was slower: two groups of four warps that write their
 // results over their scores (260 / 333 us), dQ by 16 warps with 32 columns each (215 us), dQ with two K stages (258 us), one V
@@ -927,13 +928,10 @@ static bool bwd_map(CUtensorMap* m, const void* base, int B, int Hh, int S, int 
 //   dQ, 128      more items than SMs 1.13 - 1.66; fewer, 256 keys and more 0.98 - 1.15, fewer keys 0.86 - 1.17
 //   dQ, 64       causal, more items than SMs 1.01 - 1.63; rows of 65 .. 128 keys 0.98 below 2 items per SM, 1.05 - 1.19 above,
 //                of 64 keys 0.91 - 0.98 and 1.05 from 9 on; not causal 0.88 - 1.02 up to 4 items per SM, then 0.97 - 1.25
-//   dK / dV, 128 more items than SMs 0.95 - 1.38; fewer 0.76 - 1.03 up to 2048 queries, with more 0.98 - 1.16 (blocks of 64
-//                queries waste less of a ragged end than tiles of 128)
-//   dK / dV, 64  fewer items than SMs 0.64 - 1.05; more:
-//                ALiBi from 256 queries on 0.96 - 1.4, fewer queries with up to 5 items per SM 0.89 - 1.1, with more 0.99 - 1.3;
-//                causal 384 .. 1535 queries 0.98 - 1.17, fewer 0.86 - 1.0 and 0.99 - 1.24, 2048 queries 1.0 - 1.08 and 0.93 - 0.96;
-//                not causal up to 512 queries 0.83 - 1.0 below 9 items per SM, 1.04 - 1.24 above, longer 0.8 - 0.98
-//                (queries times the query heads of a key head)
+//   dK / dV, 128 and ALiBi  more items than SMs 1.15 - 1.9, fewer 0.98 - 1.2: always persistent
+//   dK / dV, 64  fewer items than SMs 0.91 - 1.02, but 1.08 - 1.17 with 300 queries (blocks of 64 queries waste less of a ragged
+//                end than tiles of 128); more: causal 1.11 - 1.65; not causal up to 1023 queries 1.06 - 1.41, with more 1.05 -
+//                1.11 above 5 items per SM and 0.94 - 1.0 below, 4096 queries 0.98 (queries times the query heads of a key head)
 struct BwdRoute {
   long long dq_items, dkv_items;
   bool dq, dkv;      // persistent
@@ -951,11 +949,7 @@ static BwdRoute attn_bwd_route(const AttnBwdParams& p) {
   else r.dq = r.dq_items > (!p.causal ? 4 : p.Sk > AB ? 1 : p.Sk > ABS ? 2 : 9) * sms;
   const bool many = r.dkv_items > 5 * sms;
   const long long rows = static_cast<long long>(p.Sq) * (p.H / p.Hk);      // an item's queries
-  if (p.D > 64) r.dkv = r.dkv_items > sms || rows > 2048;
-  else if (r.dkv_items <= sms) r.dkv = false;
-  else if (alibi) r.dkv = rows >= 256 || many;
-  else if (p.causal) r.dkv = rows < 384 ? many : rows < 2048 || !many;
-  else r.dkv = rows <= 512 && r.dkv_items > 9 * sms;
+  r.dkv = p.D > 64 || alibi || (r.dkv_items > sms && (p.causal || rows < 1024 || (many && rows < 4096)));
   return r;
 }
 
