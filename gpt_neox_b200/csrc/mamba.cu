@@ -21,9 +21,10 @@
 // Bound by: light sweeps, the unit of exponentials (16 per step and channel; 82 and 72 % busy); forward, that unit 68 %, shared
 // memory 69 % and issue slots 62 % together; backward, issue slots (59 % with 3 warps per scheduler; shared memory 55 %),
 // where a step and channel costs 500 lane operations for 16 states.  DRAM 6-10 %.
-// Convolution + scan, forward + backward, 4 x 2048 steps of 1536 channels, fp16: 785 us with one channel per quad, inputs staged by the
-// whole CTA and dB / dC exchanged per channel (final forward sweep 119, light ones 70 and 86, backward 407 us); 605 us with
-// the present scan (95, 63 and 78, 283), 594 with the present convolution, too.  Whole calls of few channels and one block are latency: 2 x 31 x 768 takes 46 us of kernels, 43 before.
+// Convolution + scan, forward + backward, 4 x 2048 steps of 1536 channels, fp16: 785 us with one channel per quad, inputs staged
+// by the whole CTA and dB / dC exchanged per channel (final forward sweep 119, light ones 70 and 86, backward 407 us); 605 us
+// with the present scan (95, 63 and 78, 283), 594 with the present convolution, too.  Whole calls of few channels and one block
+// are latency: 2 x 31 x 768 takes 46 us of kernels, 43 before.
 // Tried for the backward: states packed per channel pair instead of per state pair (B and C twice in shared memory, no copies
 // of a step's scalars): shared memory 62 % busy, 305 - 330 us; inputs staged per block with its loads waited for: 290 - 320.
 #include "common.h"

@@ -8,9 +8,9 @@
 // the sequence length as a compile-time constant for a per-thread array.
 //
 // Heads of 64 in bf16 go in blocks of 16 steps as matrix products (second half of this file; wkv_in_blocks).  Heads of 32,
-// fp16 and a few short sequences go step by step: one CTA of 2 N threads walks one head's piece of the sequence with the N x N state in registers: warp w owns
-// 16 columns j, a lane N / 8 rows i by 4 columns.  Per step a lane reads N / 8 values of each row vector and 4 of each column
-// vector from shared memory (column vectors are stored twice side by side, so that the packed fp32 pairs, which run
+// fp16 and a few short sequences go step by step: one CTA of 2 N threads walks one head's piece of the sequence with the N x N
+// state in registers: warp w owns 16 columns j, a lane N / 8 rows i by 4 columns.  Per step a lane reads N / 8 values of each row
+// vector and 4 of each column vector from shared memory (column vectors are stored twice side by side, so that the packed fp32 pairs, which run
 // over neighbouring rows, need no register moves) and does 3 packed operations per 2 state elements: one for the output
 // sum, two for the update.  The u term is taken out of the sums: it is a dot product per step (formed while staging) times
 // one value.  Sums over rows / columns leave a lane by transposing exchanges.
@@ -22,12 +22,12 @@
 // Step by step the shared-memory loads and exchanges of the steps are the bound (32 x 512 tokens, 12 heads of 64, forward +
 // backward 788 us).  With the products of a block in their place, and a block's vectors beside the former block's products, 570
 // (134 us for column sums, 123 for row sums, 159 for gk with the decay gradient); without bank conflicts on the decays 554 (129, 120,
-// 153).  The bound is latency between a block's steps, at 2.6 warps per scheduler (issue slots 48 - 51 % busy, tensor pipe 12 - 23 %)
-// but with shared memory about 70 % busy on an SM with three CTAs: twice the warps, a group for the vectors beside one for
-// the products, took 573 us (80 registers a thread; the same wavefronts, most warps at a barrier).
+// 153).  The bound is latency between a block's steps, at 2.6 warps per scheduler (issue slots 48 - 52 % busy, tensor pipe 13 - 24 %,
+// shared memory 40 - 49 %, on average over SMs with two and with three CTAs): twice the warps, a group for the vectors beside one
+// for the products, took 573 us (80 registers a thread, most warps at a barrier).
 //
-// The sequence is cut into chunks only when batch x heads leaves the chip idle (wkv_chunk_count): the recurrence is
-// linear, so a chunk's end state is  P (.) S_start + S_local  with P[i] = prod_t d_t[i]; local passes start every chunk
+// The sequence is cut into chunks where that is faster, as a rule when batch x heads leaves the chip idle (wkv_chunk_count): the
+// recurrence is linear, so a chunk's end state is  P (.) S_start + S_local  with P[i] = prod_t d_t[i]; local passes start every chunk
 // from zero, a fold gives the chunks' start states, and Q at a chunk's end is <G, S> there.
 #include <stddef.h>
 
