@@ -21,14 +21,14 @@
 //               store a finished item's accumulators (a set dK, the other dV), beside the next item's first block.
 // What bounds them (cycle counts of the roles): neither the tensor cores nor the exponentials but the chain scores -> registers
 // -> 16-bit results -> products, with about 500 cycles from a commit or an arrival to the warp that waits for it, so a block
-// costs dQ 2,300 cycles (MMAs 1,536, exponentials 1,024) and dK / dV 1,650 per 64 queries (MMAs 1,024).  Hence everything that
+// costs dQ 2,250 cycles (MMAs 1,536, exponentials 1,024) and dK / dV 1,650 per 64 queries (MMAs 1,024).  Hence everything that
 // lets blocks overlap: issuers apart from each other (one thread issuing all was the bound at 1,700 cycles per 64 rows), scores
-// two blocks ahead, score buffers given back as soon as they are in registers, the next item's tiles and stores in the shadow of
+// and dP ahead, score buffers given back as soon as they are in registers, the next item's tiles and stores in the shadow of
 // the running one.
 // Batch 4, 32 heads, 2048 x 128 causal: dQ 290 -> 202 us, dK / dV 324 -> 275 us; 5003 tokens, 32 heads on 8, window of 4096:
-// 326 -> 238 us and 435 -> 299 us (before: one CTA per tile).  What was slower: two groups of four warps that write their
-// results over their scores (260 / 333 us), dQ by 16 warps with 32 columns each (215 us), dQ with two K stages (258 us), one V
-// stage (212 us).
+// 326 -> 229 us and 435 -> 299 us (before: one CTA per tile).  What was slower: two groups of four warps that write their
+// results over their scores (260 / 333 us); before dP had two buffers, dQ by 16 warps with 32 columns each (215 us), dQ with two
+// K stages (258 us), one V stage (212 us).
 #include "attention_bwd.h"
 #include "ptx.cuh"
 #include "reduce.cuh"
@@ -101,7 +101,7 @@ struct BwdSmem {
   static constexpr int V_OFF = STR_OFF + 6 * T64;              // dQ
   static constexpr int VEC_OFF = STR_OFF + 8 * T64;            // dK / dV: [BWD_STAGES][lse, delta][64]
   static constexpr int BAR_OFF = STR_OFF + 10 * T64;
-  static constexpr int TOTAL = BAR_OFF + 28 * 8;               // 27 barriers and the TMEM base word
+  static constexpr int TOTAL = BAR_OFF + 27 * 8;               // 26 barriers and the TMEM base word
   static constexpr int DYN = TOTAL + 1024;
 };
 constexpr int BWD_STAGES = 4;
@@ -109,14 +109,14 @@ static_assert(BwdSmem<128>::DYN <= 232448, "shared memory of one SM");
 static_assert(BWD_STAGES * 2 * 64 * 4 <= 2 * BwdSmem<64>::T64, "lse / delta fit behind the ring");
 
 // Barriers.  RES: the two resident tiles; STR / STR2: rings of streamed tiles (STR2: V of the dQ kernel); S: scores of block n
-// in buffer n & 1 written by the tensor core (FULL), in the element-wise warps' registers (EMPTY: dK / dV); DP: the same of the
-// dP buffer (dK / dV: buffer n & 1, FULL only); P_FULL: the 16-bit results of block n written.  That these are consumed STR_EMPTY
+// in buffer n & 1 (dQ: one buffer) written by the tensor core (FULL), in the element-wise warps' registers (EMPTY); DP: dP in
+// buffer n & 1 written; P_FULL: the 16-bit results of block n written, in dP's place.  That these are consumed STR_EMPTY
 // tells: the products of a block are its stage's last readers.  ACC: an item's accumulators complete / read.
 enum { RES_FULL = 0, RES_EMPTY = 2, STR_FULL = 4, STR_EMPTY = 8, STR2_FULL = 12, STR2_EMPTY = 14, S_FULL = 16, S_EMPTY = 18,
-       DP_FULL = 20, DP_EMPTY = 22, P_FULL = 23, ACC_FULL = 25, ACC_EMPTY = 26, BWD_NBAR = 27 };
+       DP_FULL = 20, P_FULL = 22, ACC_FULL = 24, ACC_EMPTY = 25, BWD_NBAR = 26 };
 __device__ __forceinline__ void bwd_init_barriers(uint32_t bar0, int element_warps) {
   for (int i = 0; i < BWD_NBAR; ++i) {
-    const bool by_warps = i == S_EMPTY || i == S_EMPTY + 1 || i == DP_EMPTY || i == P_FULL || i == P_FULL + 1;
+    const bool by_warps = i == S_EMPTY || i == S_EMPTY + 1 || i == P_FULL || i == P_FULL + 1;
     // one arrival per element-wise warp that shares a block; of all of them
     mbar_init(bar0 + 8u * i, by_warps ? 8 : i == ACC_EMPTY ? element_warps : 1);
   }
@@ -294,8 +294,10 @@ __device__ __forceinline__ void bwd_store(h16* base, long long row_stride, const
 
 // ------------------------------------------------------------------------------------------------
 // dQ kernel.  Resident: Q, dO (128 rows).  Streamed: K, V (128 rows).  An element-wise warp has 64 of a block's key columns, in
-// two chunks of 32; dS goes over the first half of the score columns the warp itself has read.
-// TMEM: S of block n at [128 (n & 1), ...), dP [256, 384), dQ [384, 384 + DP).
+// two chunks of 32; dS goes over the first half of the dP columns the warp itself has read.
+// TMEM: S [0, 128), dP of block n at [128 + 128 (n & 1), ...), dQ [384, 384 + DP).  The single buffer is the scores', which
+// are read as soon as they are there: a single one of dP, held from the first chunk's read to the second's, took 206 us (now
+// 202; 243 -> 229 with a window, 131 -> 121 with heads of 64; ALiBi 0.97 - 1.04 of the rate).
 // Without ALIBI (this kernel and the next) a block that needs a mask differs from one that does not by one select per element.
 // ------------------------------------------------------------------------------------------------
 template <int DP, bool ALIBI>
@@ -314,7 +316,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
   auto res = [&](int which) { return sbase + which * (2 * L::T64); };
   auto kst = [&](int stage) { return sbase + L::STR_OFF + stage * (2 * L::T64); };
   auto vst = [&](int stage) { return sbase + L::V_OFF + stage * (2 * L::T64); };
-  constexpr uint32_t T_DP = 256, T_DQ = 384;
+  constexpr uint32_t T_DP = 128, T_DQ = 384;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int off = p.Sk - p.Sq;
@@ -375,24 +377,24 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
         const bool last = j + 1 == it.j1;
         const int st = n & 1;
         const uint32_t ph = (n >> 1) & 1;
-        // (S buffer n & 1 is free when dQ has taken dS of block n - 2: its stage is two back in the ring of three)
         if ((!any && !warp_wait(bar(RES_FULL, 0), t & 1, p.err, 34)) || !warp_wait(bar(STR_FULL, ks), kph, p.err, 35) ||
+            !warp_wait(bar(S_EMPTY, 0), (n & 1) ^ 1, p.err, 43)) {
+          aborted = true;
+          break;
+        }
+        tc_fence_after_sync();
+        mma_nt<DP, AB>(leader, tmem, res(0), kst(ks));
+        umma_commit_by(leader, bar(S_FULL, 0));
+        if (last) umma_commit_by(leader, bar(RES_EMPTY, 0));
+        // (dP buffer n & 1 is free when dQ has taken dS of block n - 2: its stage is two back in the ring of three)
+        if ((!any && !warp_wait(bar(RES_FULL, 1), t & 1, p.err, 45)) || !warp_wait(bar(STR2_FULL, st), ph, p.err, 36) ||
             (n >= 2 && !warp_wait(bar(STR_EMPTY, ks < 2 ? ks + 1 : 0), ks < 2 ? kph ^ 1 : kph, p.err, 39))) {
           aborted = true;
           break;
         }
         tc_fence_after_sync();
-        mma_nt<DP, AB>(leader, tmem + st * AB, res(0), kst(ks));
-        umma_commit_by(leader, bar(S_FULL, st));
-        if (last) umma_commit_by(leader, bar(RES_EMPTY, 0));
-        if ((!any && !warp_wait(bar(RES_FULL, 1), t & 1, p.err, 45)) || !warp_wait(bar(STR2_FULL, st), ph, p.err, 36) ||
-            !warp_wait(bar(DP_EMPTY, 0), (n & 1) ^ 1, p.err, 43)) {
-          aborted = true;
-          break;
-        }
-        tc_fence_after_sync();
-        mma_nt<DP, AB>(leader, tmem + T_DP, res(1), vst(st));
-        umma_commit_by(leader, bar(DP_FULL, 0));
+        mma_nt<DP, AB>(leader, tmem + T_DP + st * AB, res(1), vst(st));
+        umma_commit_by(leader, bar(DP_FULL, st));
         umma_commit_by(leader, bar(STR2_EMPTY, st));
         if (last) umma_commit_by(leader, bar(RES_EMPTY, 1));
         any = true;
@@ -418,7 +420,7 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
           break;
         }
         tc_fence_after_sync();
-        mma_ts<DP, AB>(leader, tmem + T_DQ, tmem + (n & 1) * AB, 64, kst(ks), any);
+        mma_ts<DP, AB>(leader, tmem + T_DQ, tmem + T_DP + (n & 1) * AB, 64, kst(ks), any);
         umma_commit_by(leader, bar(STR_EMPTY, ks));
         any = true;
         ++n;
@@ -529,42 +531,35 @@ __global__ void __launch_bounds__(DQ_THREADS, 1)
       uint32_t sa[32], sb[32], dv[32], pk[16];
       int j = it.j0;
       const bool live = j < it.j1;
-      if (live) {
-        if (!wait(S_FULL, n & 1, (n >> 1) & 1, 38)) { aborted = true; break; }
-        tmem_ld_32x32b_x32(t_s + (n & 1) * AB, sa);
-        tmem_ld_wait_for(sa);
-      }
       bool first = true;
       while (j < it.j1) {
-        const int jn = j + 1, k0 = j * AB + c0;
-        const uint32_t t_sn = t_s + (n & 1) * AB;
-        tmem_ld_32x32b_x32(t_sn + 32, sb);      // in flight during the first chunk's exponentials
-        probs(sa, k0);
+        const int k0 = j * AB + c0;
+        const uint32_t t_dn = t_dp + (n & 1) * AB;
+        if (!wait(S_FULL, 0, n & 1, 38)) { aborted = true; break; }
+        tmem_ld_32x32b_x32(t_s, sa);
+        tmem_ld_32x32b_x32(t_s + 32, sb);
+        tmem_ld_wait_for(sa);
         tmem_ld_wait_for(sb);
-        if (!wait(DP_FULL, 0, n & 1, 44)) { aborted = true; break; }
-        tmem_ld_32x32b_x32(t_dp, dv);           // ... the second chunk's
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(S_EMPTY, 0));
+        probs(sa, k0);
+        if (!wait(DP_FULL, n & 1, (n >> 1) & 1, 44)) { aborted = true; break; }
+        tmem_ld_32x32b_x32(t_dn, dv);           // in flight during the second chunk's exponentials
         probs(sb, k0 + 32);
         tmem_ld_wait_for(dv);
         grads(sa, dv, pk);
-        tmem_ld_32x32b_x32(t_dp + 32, dv);
-        tmem_st_32x32b_x16(t_sn, pk);
+        tmem_ld_32x32b_x32(t_dn + 32, dv);
+        tmem_st_32x32b_x16(t_dn, pk);
         tmem_ld_wait_for(dv);
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(DP_EMPTY, 0));
-        if (jn < it.j1) {                       // the next block's first chunk
-          if (!wait(S_FULL, (n + 1) & 1, ((n + 1) >> 1) & 1, 38)) { aborted = true; break; }
-          tmem_ld_32x32b_x32(t_s + ((n + 1) & 1) * AB, sa);
-        }
         grads(sb, dv, pk);
-        tmem_st_32x32b_x16(t_sn + 16, pk);
+        tmem_st_32x32b_x16(t_dn + 16, pk);
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(P_FULL, n & 1));
-        tmem_ld_wait_for(sa);
         ++n;
-        j = jn;
+        ++j;
         // the former item's dQ
         if (first && pending && !finish(done, true)) { aborted = true; break; }
         first = false;
