@@ -16,7 +16,7 @@
 namespace {
 
 PyObject *s_is_cuda, *s_data_ptr, *s_dtype, *s_is_contiguous, *s_forward, *s_forward_hooks, *s_forward_pre_hooks, *s_parameters,
-    *s_modules, *s_buffers, *s_weight, *s_bias, *s_dict;
+    *s_modules, *s_buffers, *s_weight, *s_bias, *s_dict, *s_shape;
 PyObject* host_tensor = nullptr;      // called with a tensor that is not on the GPU: raises
 
 struct Ref {      // an owned reference
@@ -251,6 +251,49 @@ PyObject* pointers(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return PyBytes_FromStringAndSize(reinterpret_cast<const char*>(out), count * sizeof(out[0]));
 }
 
+// A tensor's extents; their number, or -1 with an exception.  (More than two count, but are not read.)
+Py_ssize_t extents(PyObject* tensor, long long (&out)[2]) {
+  Ref shape(PyObject_GetAttr(tensor, s_shape));
+  if (!shape) return -1;
+  if (!PyTuple_Check(shape.o)) {
+    PyErr_SetString(PyExc_TypeError, "a tensor's shape is no tuple");
+    return -1;
+  }
+  const Py_ssize_t n = PyTuple_GET_SIZE(shape.o);
+  for (Py_ssize_t i = 0; i < n && i < 2; ++i)
+    if (!convert(PyTuple_GET_ITEM(shape.o, i), out[i])) return -1;
+  return n;
+}
+
+// rows(module): the rows of its weight.
+PyObject* rows(PyObject*, PyObject* m) {
+  Ref w(parameter(m, s_weight));
+  if (!w) return nullptr;
+  long long at[2];
+  const Py_ssize_t n = w.o == Py_None ? 0 : extents(w.o, at);
+  if (n < 0) return nullptr;
+  return PyLong_FromLongLong(n > 0 ? at[0] : 0);
+}
+
+// sized(module, rows, columns, ...): whether every module's weight is [rows, columns], or [rows] where columns is 0, and its bias
+// None or [rows].
+PyObject* sized(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  for (Py_ssize_t i = 0; i + 2 < n; i += 3) {
+    long long want[2], at[2];
+    if (!convert(args[i + 1], want[0]) || !convert(args[i + 2], want[1])) return nullptr;
+    for (PyObject* name : {s_weight, s_bias}) {
+      Ref t(parameter(args[i], name));
+      if (!t) return nullptr;
+      if (t.o == Py_None && name == s_bias) continue;
+      if (t.o == Py_None) Py_RETURN_FALSE;
+      const Py_ssize_t dims = extents(t.o, at), expected = name == s_weight && want[1] != 0 ? 2 : 1;
+      if (dims < 0) return nullptr;
+      if (dims != expected || at[0] != want[0] || (expected == 2 && at[1] != want[1])) Py_RETURN_FALSE;
+    }
+  }
+  Py_RETURN_TRUE;
+}
+
 PyObject* set_host_tensor_error(PyObject*, PyObject* f) {
   Py_XSETREF(host_tensor, Py_NewRef(f));
   Py_RETURN_NONE;
@@ -262,7 +305,8 @@ constexpr PyMethodDef fast(const char* name) {
 }
 PyMethodDef methods[] = {{"bind", bind, METH_VARARGS, nullptr},
                          {"set_host_tensor_error", set_host_tensor_error, METH_O, nullptr},
-                         fast<sub>("sub"), fast<plain>("plain"), fast<pointers>("pointers"),
+                         {"rows", rows, METH_O, nullptr},
+                         fast<sub>("sub"), fast<plain>("plain"), fast<pointers>("pointers"), fast<sized>("sized"),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "neox_host_calls", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
@@ -275,7 +319,7 @@ PyMODINIT_FUNC PyInit_neox_host_calls(void) {
   } names[] = {{&s_is_cuda, "is_cuda"}, {&s_data_ptr, "data_ptr"}, {&s_dtype, "dtype"}, {&s_is_contiguous, "is_contiguous"},
                {&s_forward, "forward"}, {&s_forward_hooks, "_forward_hooks"}, {&s_forward_pre_hooks, "_forward_pre_hooks"},
                {&s_parameters, "_parameters"}, {&s_modules, "_modules"}, {&s_buffers, "_buffers"}, {&s_weight, "weight"}, {&s_bias, "bias"},
-               {&s_dict, "__dict__"}};
+               {&s_dict, "__dict__"}, {&s_shape, "shape"}};
   for (auto& n : names)
     if ((*n.at = PyUnicode_InternFromString(n.name)) == nullptr) return nullptr;
   return PyModule_Create(&module_def);

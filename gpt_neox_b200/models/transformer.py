@@ -495,17 +495,20 @@ class ParallelTransformerLayer(nn.Module):
         ptrs = pointers(x, n1, n2, qkv, dense, up, down)
         if ptrs is None:
             return None
+        # the kernels walk the weights by the sizes that they are told: those of the tensors, whatever the modules were built with
+        h, heads, kvp, ffn = x.shape[2], a.num_attention_heads_per_partition, a.num_kv_heads_per_partition, calls.rows(up)
+        if not calls.sized(n1, h, 0, n2, h, 0, qkv, (heads + 2 * kvp) * hn, h, dense, h, heads * hn, up, ffn, h, down, h, ffn):
+            return None
         has_past = layer_past is not None and (not torch.is_tensor(layer_past) or layer_past.numel() > 0)
         past = layer_past[0].shape[0] if has_past else 0
         assert x.shape[0] + past <= rotary.max_seq_len
         cos, sin = sub(rotary, "cos_table"), sub(rotary, "sin_table")
         if (cos.data_ptr() | sin.data_ptr()) & 15:
             return None
-        kvp = a.num_kv_heads_per_partition
         present = kv_cache.extend(a, layer_past if has_past else None, x.shape[0], x, (x.shape[1], kvp, hn))
         out = layer_infer(
             x, ptrs, cos, sin, present, past,
-            heads=a.num_attention_heads_per_partition, kv_heads=kvp, head_dim=hn, ffn=up.output_size_per_partition, rot=a.rotary_dim,
+            heads=heads, kv_heads=kvp, head_dim=hn, ffn=ffn, rot=a.rotary_dim,
             window=a.sliding_window_width if a.sliding_window_width is not None else -1, scale=a.attn_scale, eps=n1.eps,
             act=("tanh" if m.bias_gelu_fusion else "erf", not m.recompute_act))
         if get is sub and "layer_past" in self.__dict__:

@@ -177,7 +177,8 @@ def lib(like=None):
 
 
 def calls():
-    """The native module (csrc/host_calls.cpp): ``sub``, ``plain`` and ``pointers`` beside the bound entry points."""
+    """The native module (csrc/host_calls.cpp): ``sub``, ``plain``, ``pointers``, ``rows`` and ``sized`` beside the bound entry
+    points."""
     if _CALLS is None:
         lib()
     return _CALLS

@@ -123,3 +123,117 @@ def test_pointers(calls):
     del real._parameters["weight"]
     with pytest.raises(AttributeError):
         calls.pointers(_lib.H16, x, real)
+
+
+def test_weight_sizes(calls):
+    """Weights and biases are compared with the sizes that a caller expects, wherever a module holds them."""
+    lin = lambda n, k, bias=True: torch.nn.Linear(k, n, bias=bias)
+    a, b, norm = lin(6, 4), lin(4, 6, bias=False), torch.nn.LayerNorm(4)
+    assert calls.rows(a) == 6 and calls.rows(norm) == 4
+    assert calls.sized(norm, 4, 0, a, 6, 4, b, 4, 6)
+    for m, n, k in ((a, 5, 4), (a, 6, 5), (a, 6, 0), (norm, 4, 1), (norm, 3, 0)):
+        assert not calls.sized(b, 4, 6, m, n, k)
+    a.bias = torch.nn.Parameter(torch.zeros(5))
+    assert not calls.sized(a, 6, 4)
+    a.bias = torch.nn.Parameter(torch.zeros(6, 1))
+    assert not calls.sized(a, 6, 4)
+    a.bias = None
+    a.weight = torch.nn.Parameter(torch.zeros(8, 4))
+    assert calls.rows(a) == 8 and calls.sized(a, 8, 4) and not calls.sized(a, 6, 4)
+    a.weight = torch.nn.Parameter(torch.zeros(8, 4, 1))
+    assert not calls.sized(a, 8, 4)
+    with pytest.raises(AttributeError):
+        calls.sized(torch.nn.Identity(), 1, 1)
+
+
+def _resized_mlp(layer, up, down):
+    """Parameters of other widths in a layer's MLP: a pruned or grown one."""
+    m, h = layer.mlp, layer.mlp.linear2.weight.shape[0]
+    like = m.linear1.weight
+    new = lambda *s: torch.nn.Parameter(torch.randn(s, device=like.device, dtype=like.dtype) * 0.05)
+    m.linear1.weight, m.linear1.bias, m.linear2.weight = new(up, h), new(up), new(h, down)
+
+
+@pytest.mark.parametrize("up,down", [(None, None), (40, 40), (512, 512), (40, 64), (512, 40)])
+def test_a_layer_in_one_call_goes_by_the_weights_it_is_given(calls, up, down, monkeypatch):
+    """What the native layer call is told, with weights that stand in for ones on the GPU: the MLP's width is its weights', and
+    weights that do not fit one another send the layer down the op-by-op path, which refuses them."""
+    import types
+
+    from common import tiny_config
+    from test_generation import _model
+    from gpt_neox_b200.models import transformer
+    _, model = _model(hidden_size=256, num_attention_heads=4)
+    model.eval()
+    model.inference_mode(use_cache=True)
+    layer = next(m for m in model.modules() if isinstance(m, transformer.ParallelTransformerLayer))
+    if up is not None:
+        _resized_mlp(layer, up, down)
+    a, m = layer.attention, layer.mlp
+    a.use_flash_attention = True
+    width = m.linear1.weight.shape[0]
+    for module in (layer.input_layernorm, layer.post_attention_layernorm, a.query_key_value, a.dense, m.linear1, m.linear2):
+        for name in ("weight", "bias"):
+            t = getattr(module, name)
+            if t is not None:
+                fake = _OnGpu(4096)
+                fake.shape = t.shape
+                module.__dict__[name] = fake
+    h = a.hidden_size_per_attention_head * a.num_attention_heads_per_partition
+    x = _OnGpu(4096)
+    x.shape = torch.Size((2, 1, h))
+    got = []
+    monkeypatch.setattr(transformer.kernel_lib, "_CALLS", calls)
+    monkeypatch.setattr(transformer, "layer_infer", lambda *args, **kw: got.append(kw["ffn"]) or "out")
+    monkeypatch.setattr(transformer.kv_cache, "extend", lambda *args: types.SimpleNamespace())
+    with torch.no_grad():
+        out = layer._infer(x, None)
+    assert (out, got) == (("out", [width]) if up == down else (None, []))
+    # any other weight or bias that does not fit
+    for module, name in ((layer.input_layernorm, "weight"), (a.query_key_value, "weight"), (a.dense, "weight"),
+                         (m.linear1, "bias"), (m.linear2, "bias")):
+        fake = module.__dict__[name]
+        fit, fake.shape = fake.shape, torch.Size((fake.shape[0] + 8,) + tuple(fake.shape[1:]))
+        with torch.no_grad():
+            assert layer._infer(x, None) is None
+        fake.shape = fit
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("up,down", [(520, 520), (1536, 1536), (520, 1024)])
+def test_a_generation_step_with_an_mlp_of_another_width(up, down, monkeypatch):
+    """The same on the GPU: the bits of the op-by-op path, and its refusal of weights that do not fit one another."""
+    from common import tiny_config
+    from test_model_gpu import _build
+    from gpt_neox_b200.models import transformer
+    _, model = _build(tiny_config(num_layers=2, hidden_size=256, num_attention_heads=4, seq_length=512, pipe_parallel_size=0,
+                                  max_position_embeddings=512, synthetic_vocab_size=1000, attention_config=[[["flash"], 2]],
+                                  distributed_backend="nccl", precision="bfloat16"))
+    model.eval()
+    model.inference_mode(use_cache=True)
+    layers = [m for m in model.modules() if isinstance(m, transformer.ParallelTransformerLayer)]
+    _resized_mlp(layers[1], up, down)
+    native, call = [], transformer.layer_infer
+    monkeypatch.setattr(transformer, "layer_infer", lambda *a, **k: (native.append(k["ffn"]), call(*a, **k))[1])
+    tokens, pos = torch.randint(0, 1000, (3, 300), device="cuda"), torch.arange(300, device="cuda")[None].expand(3, -1)
+
+    def steps():
+        model.clear_cache()
+        out, at = [], 0
+        with torch.no_grad():
+            for n in (5, 1, 290, 1):
+                out.append(model((tokens[:, at:at + n].contiguous(), pos[:, at:at + n].contiguous(), None)))
+                at += n
+        return out
+
+    if up != down:
+        with pytest.raises(AssertionError, match="inner dimensions differ"):
+            steps()
+        return
+    one = steps()
+    assert native == [1024, up] * 4
+    handles = [l.mlp.register_forward_hook(lambda *a: None) for l in layers]
+    ops = steps()
+    for handle in handles:
+        handle.remove()
+    assert len(native) == 8 and all(torch.equal(a, b) for a, b in zip(one, ops))
