@@ -1163,18 +1163,26 @@ static bool wkv_in_blocks(int B, int T, int H, int N) {
   return WM_BLOCKS && N == WN && (T > 128 || static_cast<long long>(B) * H * T >= 3072);
 }
 
-// Chunks the sequence is cut into.  A block of steps of the sweeps takes as long as the SM's CTAs need: latency until it holds
-// WK_CTAS, so with one or two CTAs 2/3 and 5/6 of the time with three, which also holds for the CTAs left over by full rounds
-// (40 x 512, 12 heads: 480 CTAs on 444 places take 1.62 rounds).  More than one chunk adds the local passes over all chunks but one,
-// the fold's launches and chain, and the states' traffic.  In units of a round of a block, 16.6 us.  Times of forward + backward
-// by the number of chunks, this rule's first: 1 x 512, 12 heads 16: 67 us, 32: 67, 8: 78; 4 x 2048 9: 337, 8: 355, 16: 373, 1: 1387;
-// 8 x 2048, 16 heads 10: 850, 3: 877, 1: 1437; 40 x 300, 12 heads 1: 515, 3: 542, 19: 908 (the choice when only rounds and steps
-// were counted); 40 x 512 4: 823, 1: 860, 8: 900; 16 x 1000, 16 heads 5: 844, 1: 871; 10 x 400, 12 heads 3: 207, 1: 267.  Step by
-// step (LOCAL is as long as the others there) whole rounds and more for the local passes.  The count depends on the batch,
-// and the chunks' states are folded in fp32: a sequence's last bits are not those it has in another batch.
-constexpr int WK_CTAS = 3;
-static int wkv_chunk_count(int B, int T, int H) {
-  const int subs = (T + WK_SUB - 1) / WK_SUB, slots = WK_CTAS * sm_count();
+// Chunks the sequence is cut into.  More than one chunk adds the local passes over all chunks but one, the fold's launches and
+// chain, and the states' traffic.  In units of a round of 16 steps; `per_sm`: CTAs on an SM in a last round that is not full.
+// In blocks: a block of steps takes as long as the SM's CTAs need: latency until it holds WK_CTAS, so with one or two CTAs 2/3 and
+// 5/6 of the time with three, which also holds for the CTAs left over by full rounds (40 x 512, 12 heads: 480 CTAs on 444 places
+// take 1.62 rounds).  A round: 16.6 us.  Times of forward + backward by the number of chunks, this rule's first: 1 x 512, 12 heads
+// 16: 67 us, 32: 67, 8: 78; 4 x 2048 9: 337, 8: 355, 16: 373, 1: 1387; 8 x 2048, 16 heads 10: 850, 3: 877, 1: 1437; 40 x 300, 12
+// heads 1: 515, 3: 542, 19: 908 (the choice when only rounds and steps were counted); 40 x 512 4: 823, 1: 860, 8: 900; 16 x 1000, 16
+// heads 5: 844, 1: 871; 10 x 400, 12 heads 3: 207, 1: 267.
+// Heads of 32: CTAs of two warps, eight on an SM; the local passes are nearly as long as the others.  us, this rule's first, then
+// that of the next line, then that of blocks: 8 x 2048, 16 heads 8: 515, 3: 692, 10: 582; 4 x 2048, 24 heads 12: 394, 4: 520, 9: 411; 2 x
+// 4096, 32 heads 16: 517, 20: 587, 13: 540; 40 x 512, 12 heads 1: 440, 8: 487, 4: 473; 4 x 300, 24 heads 10: 84, 4: 98; 10 x 400, 24 heads
+// 3: 225, 5: 228, 1: 239; 1 x 8192, 24 heads 29: 466, 18: 498, 32: 438; 32 x 512, 24 heads 1: 597.  Of 19 such calls none is more than
+// 7 % above its best count's time, and none slower than with the next line's count.
+// Heads of 64 step by step (the local passes are as long as the others): whole rounds.
+// The count depends on the batch, and the chunks' states are folded in fp32: a sequence's last bits are not those it has in
+// another batch.
+constexpr int WK_CTAS = 3, WK_CTAS_32 = 8;
+static int wkv_chunk_count(int B, int T, int H, int N) {
+  const bool blocks = wkv_in_blocks(B, T, H, N);
+  const int subs = (T + WK_SUB - 1) / WK_SUB, slots = (N == 32 ? WK_CTAS_32 : WK_CTAS) * sm_count();
   int best = 1;
   float best_cost = 1e30f;
   for (int nc = 1; nc <= WK_MAX_CHUNKS && nc <= subs; ++nc) {
@@ -1183,9 +1191,12 @@ static int wkv_chunk_count(int B, int T, int H) {
     const long long ctas = static_cast<long long>(B) * H * nc, full = ctas / slots, rest = ctas - full * slots;
     const int per_sm = static_cast<int>((rest + sm_count() - 1) / sm_count());
     float cost;
-    if (wkv_in_blocks(B, T, H, WN))
+    if (blocks)
       cost = len * (full + (rest > 0 ? 0.5f + per_sm / 6.f : 0.f)) * (1.f + 0.3f * (nc - 1) / nc) +
              (nc > 1 ? 1.5f + 0.05f * nc + 0.0015f * ctas : 0.f);
+    else if (N == 32)
+      cost = len * (full + (rest > 0 ? 0.25f + 0.75f * per_sm / WK_CTAS_32 : 0.f)) * (1.f + 0.7f * (nc - 1) / nc) +
+             (nc > 1 ? 0.5f + 0.0005f * ctas : 0.f);
     else
       cost = len * (full + (rest > 0)) * (1.f + 0.67f * (nc - 1) / nc) + (nc > 1 ? 0.5f + 0.1f * nc : 0.f);
     if (cost < best_cost) {
@@ -1273,12 +1284,14 @@ static int wkv_backward(WkvParams p, const float* fstart, float* rstart, float* 
   return NX_OK;
 }
 
-NX_API int NX_SYM(nx_wkv6_chunks)(int B, int T, int H) { return wkv_chunk_count(B, T, H); }
+// Chunks for heads of N, and of 64.
+NX_API int NX_SYM(nx_wkv6_head_chunks)(int B, int T, int H, int N) { return wkv_chunk_count(B, T, H, N); }
+NX_API int NX_SYM(nx_wkv6_chunks)(int B, int T, int H) { return wkv_chunk_count(B, T, H, WN); }
 // Kernels a backward launches (two more where there are several chunks).
 NX_API int NX_SYM(nx_wkv6_bwd_launches)(int B, int T, int H, int N) { return wkv_in_blocks(B, T, H, N) ? 4 : 3; }
 
 // r, k, v, w: bf16 [B, T, H*N] addressed by (sb, st); u fp32 [H, N]; y bf16 by (osb, ost).  With NC =
-// nx_wkv6_chunks(B, T, H) > 1: local / start fp32 [B, H, NC, N, N] and sumew fp32 [B, H, NC, N] are scratch, and
+// nx_wkv6_head_chunks(B, T, H, N) > 1: local / start fp32 [B, H, NC, N, N] and sumew fp32 [B, H, NC, N] are scratch, and
 // `start` is kept for the backward; they may be null for NC = 1.
 NX_API int NX_SYM(nx_wkv6_fwd)(const void* r, const void* k, const void* v, const void* w, long long sb, long long st,
                        const void* u, void* y, long long osb, long long ost, void* local, void* start, void* sumew,
@@ -1290,7 +1303,7 @@ NX_API int NX_SYM(nx_wkv6_fwd)(const void* r, const void* k, const void* v, cons
   p.sb = sb; p.st = st; p.u = (const float*)u;
   p.y = (h16*)y; p.osb = osb; p.ost = ost;
   p.local = (float*)local; p.sumew = (float*)sumew;
-  p.B = B; p.T = T; p.H = H; p.NC = wkv_chunk_count(B, T, H); p.clen = wkv_chunk_len(T, p.NC);
+  p.B = B; p.T = T; p.H = H; p.NC = wkv_chunk_count(B, T, H, N); p.clen = wkv_chunk_len(T, p.NC);
   return N == 64 ? wkv_forward<64>(p, (float*)start, stream) : wkv_forward<32>(p, (float*)start, stream);
 }
 
@@ -1309,7 +1322,7 @@ NX_API int NX_SYM(nx_wkv6_bwd)(const void* r, const void* k, const void* v, cons
   p.o_gr = (h16*)gr; p.o_gk = (h16*)gk; p.o_gv = (h16*)gv; p.o_gw = (h16*)gw;
   p.gr32 = (float*)gr32; p.gu_part = (float*)gu_part; p.osb = osb; p.ost = ost;
   p.local = (float*)local; p.sumew = (float*)sumew;
-  p.B = B; p.T = T; p.H = H; p.NC = wkv_chunk_count(B, T, H); p.clen = wkv_chunk_len(T, p.NC);
+  p.B = B; p.T = T; p.H = H; p.NC = wkv_chunk_count(B, T, H, N); p.clen = wkv_chunk_len(T, p.NC);
   return N == 64 ? wkv_backward<64>(p, (const float*)fstart, (float*)rstart, (float*)gu, stream)
                  : wkv_backward<32>(p, (const float*)fstart, (float*)rstart, (float*)gu, stream);
 }

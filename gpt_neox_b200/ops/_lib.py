@@ -128,6 +128,7 @@ def _declare(lib, calls):
     sig("nx_selective_scan_bwd", [P, L, L, P, L, L, P, L, L, P, L, L, P, L, L, P, P, P, P, L, L, P, P, P, L, L, P, P,
                                   P, P, P, P, P, P, P, I, I, I, P])
     sig("nx_wkv6_chunks", [I, I, I])
+    sig("nx_wkv6_head_chunks", [I, I, I, I])
     sig("nx_wkv6_bwd_launches", [I, I, I, I])
     sig("nx_wkv6_fwd", [P, P, P, P, L, L, P, P, L, L, P, P, P, I, I, I, I, P])
     sig("nx_wkv6_bwd", [P, P, P, P, P, L, L, P, P, P, P, P, P, P, P, L, L, P, P, P, P, I, I, I, I, P])

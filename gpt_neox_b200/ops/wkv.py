@@ -68,7 +68,7 @@ class _WkvFn(torch.autograd.Function):
         r, k, v, w = _same_layout(r, k, v, w)
         u32 = u.float().contiguous()
         lib = _lib.lib(r)
-        nc = lib.nx_wkv6_chunks(B, T, H)
+        nc = lib.nx_wkv6_head_chunks(B, T, H, N)
         dev = r.device
         local = start = sumew = None
         if nc > 1:

@@ -112,6 +112,28 @@ def test_wkv6_chunks_and_layouts(B, T, H, N, pad, dtype):
         assert (a.float() - r).abs().max().item() <= 2 * eps * r.abs().max().item() + 1e-3
 
 
+@pytest.mark.parametrize("B,T,H,counts", [(4, 2048, 24, (12, 9)), (8, 2048, 16, (8, 10)), (2, 4096, 32, (16, 13)),
+                                          (40, 512, 12, (1, 4)), (4, 300, 24, (10, 4)), (10, 400, 24, (3, 1)), (1, 10, 4, (1, 1))])
+def test_wkv6_chunks_go_by_the_head_size(B, T, H, counts):
+    """Heads of 32 go step by step, with CTAs of half the size: on 148 SMs the counts that were measured to be the best ones or
+    within 7 % of them, not those of heads of 64 in blocks."""
+    from gpt_neox_b200.ops import _lib
+    lib = _lib.lib(torch.bfloat16)
+    if lib.nx_sm_count() != 148:
+        pytest.skip("the counts are those of 148 SMs")
+    assert (lib.nx_wkv6_head_chunks(B, T, H, 32), lib.nx_wkv6_head_chunks(B, T, H, 64)) == counts
+    assert lib.nx_wkv6_chunks(B, T, H) == counts[1]
+    assert _lib.lib(torch.float16).nx_wkv6_head_chunks(B, T, H, 32) == counts[0]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,T,H", [(1, 517, 5), (4, 300, 24), (2, 1000, 3)])
+def test_wkv6_heads_of_32_in_many_chunks(B, T, H, dtype):
+    """32, 10 and 32 chunks on 148 SMs, the last one ragged."""
+    test_wkv6_chunks_and_layouts(B, T, H, 32, 0, dtype)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("B,T,H,N", [(96, 40, 2, 64), (1, 900, 2, 64), (3, 400, 1, 32)])
 def test_wkv6_gradients_repeat_bit_for_bit(B, T, H, N):
