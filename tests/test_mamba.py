@@ -182,6 +182,40 @@ def test_selective_scan_pairs_and_segments(B, L, D, off, use_z, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("lo,hi,units", [(-40.0, -10.0, 16), (-10.0, -5.0, 4), (-5.0, -3.0, 1.8), (-3.0, -1.0, 1.25), (-1.0, 0.0, 1),
+                                         (0.0, 1.0, 1), (1.0, 20.0, 0.5), (20.0, 60.0, 0.25)])
+def test_selective_scan_softplus_has_fp32_precision(lo, hi, units):
+    """The step that the scan forms from dt + dt_bias, in fp32: without decay the state behind one step of input 1 is that step.
+    Root mean square of the relative error against 64 bits, in units of 2 ** -24: below one where the roundings of log(1 + e) are
+    all there is, more where the argument's rounding before the exponential (|v| units at most, a third on average) counts, less
+    where v itself is nearly all of the result.  (2 artanh(e / (2 + e)) with a division had 1.22 and 1.4 in (-1, 0) and (-3, -1).)"""
+    from gpt_neox_b200.ops import mamba
+    torch.manual_seed(5)
+    D, L = 1 << 16, 33
+    v = torch.empty(D, device="cuda").uniform_(lo, hi)
+    zeros = lambda *s: torch.zeros(s, device="cuda", dtype=torch.float16)
+    x, B = zeros(1, L, D), zeros(1, L, 16)
+    x[:, 0], B[..., 0] = 1, 1
+    _, states = mamba._scan_forward(x, zeros(1, L, D), torch.zeros(D, 16, device="cuda"), B, zeros(1, L, 16), None, None, v, True)
+    want = torch.log1p(torch.exp(-v.double().abs())) + v.double().clamp(min=0)
+    err = states[0, 1, :, 0].double() / want - 1
+    assert err.square().mean().sqrt() <= units * 2 ** -24
+
+
+@pytest.mark.gpu
+def test_selective_scan_softplus_at_the_ends():
+    from gpt_neox_b200.ops import mamba
+    v = torch.tensor([float("inf"), float("-inf"), float("nan"), 0.0, -200.0, 3e38, -3e38, 88.0], device="cuda")
+    zeros = lambda *s: torch.zeros(s, device="cuda", dtype=torch.float16)
+    x, B = zeros(1, 33, 8), zeros(1, 33, 16) + 1
+    x[:, 0] = 1
+    out, states = mamba._scan_forward(x, zeros(1, 33, 8), torch.full((8, 16), -1.0, device="cuda"), B, B / 16, None, None, v, True)
+    y = out[0, 0].float()                          # the step itself, rounded to fp16 (16 states with a sixteenth each)
+    assert y[0].isposinf() and y[1] == 0 and y[2].isnan() and abs(y[3] - 0.6931) < 5e-4
+    assert y[4] == 0 and y[5].isposinf() and y[6] == 0 and y[7] == 88
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("what,value", [("x", float("nan")), ("dt", float("nan")), ("B", float("nan")), ("C", float("inf")),
                                         ("z", float("nan")), ("x", float("inf"))])
 @pytest.mark.parametrize("at", [0, 37, 255, 299])
