@@ -2,7 +2,8 @@
 // entries in place of ctypes, and the look over a generation layer's modules.
 //
 // Generation with 12 layers of 768, batch 4, a prompt of 100 tokens and 16 steps: 17.4 ms when ctypes and Python did this, 12.4 ms
-// now (a step's kernels, captured as a graph, take 0.4 ms; a layer's host work 87 us before, 59 now, 22 of it its 8 launches).
+// with these calls (11.4 with the layer's launches made fewer, csrc/layer_infer.cu; a step's kernels, captured as a graph, take
+// 0.33 ms).
 // The module looks everything up on each call and keeps nothing but the functions' addresses.  Plain CPython, no torch headers:
 // tensors are asked through their attributes, so whatever answers to is_cuda and data_ptr() passes as before.
 #define PY_SSIZE_T_CLEAN
@@ -11,6 +12,7 @@
 #include <cstdint>
 #include <cstring>
 #include <tuple>
+#include <type_traits>
 #include <utility>
 
 namespace {
@@ -111,12 +113,25 @@ using P = void*;
 using L = long long;
 using I = int;
 using F = float;
-template <class E>
-constexpr PyMethodDef def(const char* name) {
-  return {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&E::entry)), METH_FASTCALL, nullptr};
+template <class T>
+constexpr char letter = std::is_same_v<T, P> ? 'P' : std::is_same_v<T, L> ? 'L' : std::is_same_v<T, I> ? 'I' : 'F';
+template <class... A>
+struct Signature {
+  static constexpr char text[] = {letter<A>..., 0};
+};
+struct Bound {
+  PyMethodDef def;
+  const char* types;
+};
+template <class... A>
+constexpr Bound bound(const char* name, Entry<A...>*) {
+  return {{name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&Entry<A...>::entry)), METH_FASTCALL, nullptr},
+          Signature<A...>::text};
 }
+template <class E>
+constexpr Bound def(const char* name) { return bound(name, static_cast<E*>(nullptr)); }
 // The signatures of the entry points (csrc/*.cu); `name` or `name_f16`.
-PyMethodDef entries[] = {
+Bound entries[] = {
     def<Entry<I, P, P, P, P, P, P, P, P, P, L, I, F, P>>("nx_norm_fwd"),
     def<Entry<I, P, P, P, P, P, P, P, P, P, P, P, P, P, P, L, I, I, I, P>>("nx_norm_bwd"),
     def<Entry<P, P, P, I, I, I, L, L, L, I, I, P, P, P, P, L, I, F, P>>("nx_gemm_bf16"),
@@ -125,16 +140,21 @@ PyMethodDef entries[] = {
     def<Entry<P, P>>("nx_layer_infer"),
 };
 
-// bind(name, address) -> the entry point as a callable, or None if its signature is not known here.
+// bind(name, address[, types]) -> the entry point as a callable, or None if its signature is not known here.  `types`: a letter of
+// "PILF" (pointer, int, long long, float) per parameter as the caller declares them; a difference is an error.
 PyObject* bind(PyObject*, PyObject* args) {
-  const char* name;
+  const char *name, *types = nullptr;
   unsigned long long at;
-  if (!PyArg_ParseTuple(args, "sK", &name, &at)) return nullptr;
-  for (PyMethodDef& d : entries) {
-    const std::size_t n = std::strlen(d.ml_name);
-    if (std::strncmp(name, d.ml_name, n) != 0 || (name[n] != 0 && std::strcmp(name + n, "_f16") != 0)) continue;
+  if (!PyArg_ParseTuple(args, "sK|z", &name, &at, &types)) return nullptr;
+  for (Bound& e : entries) {
+    const std::size_t n = std::strlen(e.def.ml_name);
+    if (std::strncmp(name, e.def.ml_name, n) != 0 || (name[n] != 0 && std::strcmp(name + n, "_f16") != 0)) continue;
+    if (types != nullptr && std::strcmp(types, e.types) != 0) {
+      PyErr_Format(PyExc_TypeError, "%s takes (%s) here and is declared as (%s)", name, e.types, types);
+      return nullptr;
+    }
     Ref capsule(PyCapsule_New(reinterpret_cast<void*>(static_cast<std::uintptr_t>(at)), nullptr, nullptr));
-    return capsule ? PyCFunction_New(&d, capsule.o) : nullptr;
+    return capsule ? PyCFunction_New(&e.def, capsule.o) : nullptr;
   }
   Py_RETURN_NONE;
 }

@@ -8,6 +8,8 @@
 // With few rows the two branches' first products go in one launch, and their second ones: a step is a chain of short kernels,
 // which it makes shorter by two (a captured step of 12 layers of 768, batch 4: 400 us with eight launches per layer, 327 with
 // six).
+#include <cstddef>
+
 #include "common.h"
 #include "gemm_skinny.h"
 
@@ -37,6 +39,7 @@ extern "C" {
 // rows [past, past + s) written here.
 struct nx_layer_infer_args {
   const void *x, *ln1_w, *ln1_b, *ln2_w, *ln2_b, *w_qkv, *b_qkv, *w_dense, *b_dense, *w1, *b1, *w2, *b2;
+  long long bytes;                      // of this block, as the caller packs it
   const void *cos, *sin;
   // scratch: work, 16-bit: x1, x2, the attention branch (rows x h each), qkv, context, the MLP's hidden
   // layer; stats, fp32: mean and rstd of every row, the log-sum-exp of the attention [b, np, s rounded up to 128]
@@ -46,11 +49,15 @@ struct nx_layer_infer_args {
   float eps, scale;
 };
 }
+// (packed by ops/layer_infer.py: 13 addresses, the size, and behind it no gap)
+static_assert(offsetof(nx_layer_infer_args, bytes) == 13 * 8 && offsetof(nx_layer_infer_args, cache_kv_stride) == 20 * 8 &&
+              offsetof(nx_layer_infer_args, eps) == 21 * 8 + 12 * 4 && sizeof(nx_layer_infer_args) == 22 * 8 + 12 * 4);
 
 // An error, or minus the number of launches.
 NX_API int NX_SYM(nx_layer_infer)(const nx_layer_infer_args* a, void* stream) {
   using namespace nx;
   enum { BIAS = 1 };
+  NX_REQUIRE(a->bytes == sizeof(*a), "layer_infer: a block of %lld bytes, not %zu", a->bytes, sizeof(*a));
   const long long rows = static_cast<long long>(a->s) * a->b;
   if (rows == 0) return NX_OK;
   NX_REQUIRE(rows < (1ll << 31), "layer_infer: too many rows");

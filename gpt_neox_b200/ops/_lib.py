@@ -23,6 +23,8 @@ _LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / (
     "libneox_b200_dbg.so" if os.environ.get("NEOX_KERNEL_LIB") == "debug" else "libneox_b200.so")
 
 c_void_p, c_int, c_ll, c_float = C.c_void_p, C.c_int, C.c_longlong, C.c_float
+#: the letters by which csrc/host_calls.cpp compares a declaration with its own
+_LETTERS = {c_void_p: "P", c_int: "I", c_ll: "L", c_float: "F"}
 
 
 class KernelError(RuntimeError):
@@ -78,7 +80,7 @@ def _declare(lib, calls):
                 continue
             fn.argtypes = argtypes
             fn.restype = restype
-            native = calls.bind(nm, C.cast(fn, c_void_p).value)
+            native = calls.bind(nm, C.cast(fn, c_void_p).value, "".join(_LETTERS.get(t, "?") for t in argtypes))
             if native is not None:       # takes tensors and addresses alike
                 setattr(lib, nm, native)
 

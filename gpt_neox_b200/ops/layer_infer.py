@@ -12,9 +12,10 @@ import torch
 from . import _lib
 from .gemm import LAUNCHES, PAIR_GEMM, EPI_AUX_DERIV, EPI_GELU_ERF, EPI_GELU_TANH
 
-#: ``nx_layer_infer_args`` of csrc/layer_infer.cu behind its first 13 pointers: cos, sin, cache, work, stats, out,
-#: cache_kv_stride; s, b, h, np, kvp, hn, ffn, past, rot, window, act, pair_gemm; eps, scale
-_TAIL = struct.Struct("@6Pq12i2f")
+#: ``nx_layer_infer_args`` of csrc/layer_infer.cu behind its first 13 pointers: the size of the whole; cos, sin, cache, work,
+#: stats, out, cache_kv_stride; s, b, h, np, kvp, hn, ffn, past, rot, window, act, pair_gemm; eps, scale
+_TAIL = struct.Struct("@q6Pq12i2f")
+_BYTES = 13 * 8 + _TAIL.size
 
 
 def pointers(x, *modules):
@@ -36,7 +37,7 @@ def layer_infer(x, ptrs, cos, sin, present, past, *, heads, kv_heads, head_dim, 
     work = torch.empty(2 * stats + rows * (3 * h + 2 * width + 2 * kv_heads * head_dim + ffn), device=x.device, dtype=x.dtype)
     w = work.data_ptr()
     args = ptrs + _TAIL.pack(
-        cos.data_ptr(), sin.data_ptr(), present.data_ptr(), w + 4 * stats, w, out.data_ptr(), present.stride(0), s, b, h,
+        _BYTES, cos.data_ptr(), sin.data_ptr(), present.data_ptr(), w + 4 * stats, w, out.data_ptr(), present.stride(0), s, b, h,
         heads, kv_heads, head_dim, ffn, past, rot, window,
         (EPI_GELU_TANH if act[0] == "tanh" else EPI_GELU_ERF) | (EPI_AUX_DERIV if act[1] else 0), int(PAIR_GEMM["on"]),
         eps, scale)

@@ -57,6 +57,32 @@ def test_bound_entry_gets_its_arguments(calls, name, types):
     assert got == [] and calls.bind("nx_gemm_bf16_grouped", 16) is None
 
 
+def test_declarations_are_compared(calls):
+    """A declaration that is not the native module's is refused; the library's own are taken when it is loaded."""
+    assert calls.bind("nx_layer_infer", 16, "PP") is not None and calls.bind("nx_gated_act_fwd_f16", 16, "PPLIIP") is not None
+    for name, types in (("nx_layer_infer", "PL"), ("nx_layer_infer", "PPP"), ("nx_gated_act_fwd", "PPIIIP"), ("nx_gated_act_fwd", "")):
+        with pytest.raises(TypeError, match="declared"):
+            calls.bind(name, 16, types)
+    assert _lib._declare(C.CDLL(str(_lib._LIB_PATH)), calls) is not None
+    moved = C.CDLL(str(_lib._LIB_PATH))
+
+    class Other:
+        bind = staticmethod(lambda name, at, types: calls.bind(name, at, types.replace("L", "I")))
+    with pytest.raises(TypeError, match="declared"):
+        _lib._declare(moved, Other)
+
+
+def test_layer_arguments_say_their_size():
+    """A block of another layout is refused before anything of it is used (without a GPU: no row to work on)."""
+    from gpt_neox_b200.ops import layer_infer
+    lib = _lib.lib(torch.bfloat16)
+    block = lambda size: bytes(13 * 8) + layer_infer._TAIL.pack(size, *([0] * 19), 0.0, 0.0)
+    assert len(block(0)) == layer_infer._BYTES
+    assert lib.nx_layer_infer(block(layer_infer._BYTES), None) == 0
+    for size in (0, layer_infer._BYTES - 8, layer_infer._BYTES + 8):
+        assert lib.nx_layer_infer(block(size), None) > 0 and b"layer_infer" in lib.nx_last_error()
+
+
 def test_bound_entry_takes_bytes(calls):
     seen = []
     target = C.CFUNCTYPE(I, P, P)(lambda a, b: (seen.append(C.string_at(a, 4)), 0)[1])
