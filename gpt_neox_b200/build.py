@@ -5,7 +5,8 @@
   ``gpt_neox_b200.ops`` binds with ctypes.
 * ``lib/libneox_data.so`` – the CPU dataset-index builders (g++), the counterpart of the
   reference's ``megatron/data/helpers.cpp`` built by ``megatron/data/Makefile``.
-* ``lib/neox_host_calls.so`` – native calls from Python into the kernel library (g++, csrc/host_calls.cpp).
+* ``lib/neox_host_calls.<tag>.so`` – native calls from Python into the kernel library (g++ and this interpreter's headers,
+  csrc/host_calls.cpp); ``<tag>`` names the interpreter (``cpython-312-x86_64-linux-gnu``), each has its own.
 * ``lib/libneox_host.so`` – host AdamW for optimizer-state offload (g++, csrc/cpu_adam.cpp).
 
 Objects are cached under ``build/`` and rebuilt when a source or any header is newer.
@@ -118,15 +119,21 @@ def build_host_ops(force: bool = False) -> Path:
     return out
 
 
+def host_calls_path() -> Path:
+    """Where this interpreter's native calls are: a tree built under one interpreter is not loaded under another."""
+    return LIB / ("neox_host_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
 def build_host_calls(force: bool = False) -> Path:
-    """``lib/neox_host_calls.so``: native calls from Python into the kernel library (csrc/host_calls.cpp, an extension module
-    of this interpreter)."""
+    """Native calls from Python into the kernel library (csrc/host_calls.cpp, an extension module of this interpreter)."""
     LIB.mkdir(parents=True, exist_ok=True)
-    src = CSRC / "host_calls.cpp"
-    out = LIB / "neox_host_calls.so"
+    src, out = CSRC / "host_calls.cpp", host_calls_path()
     if force or _stale(out, [src]):
-        cmd = [os.environ.get("CXX", "g++"), *CXX_FLAGS, "-fvisibility=hidden", "-I", sysconfig.get_paths()["include"], str(src),
-               "-o", str(out)]
+        include = sysconfig.get_paths()["include"]
+        if not os.path.exists(os.path.join(include, "Python.h")):
+            raise RuntimeError(f"{include}/Python.h is missing: the native calls need the interpreter's headers "
+                               "(the python3-dev package of the system's Python)")
+        cmd = [os.environ.get("CXX", "g++"), *CXX_FLAGS, "-fvisibility=hidden", "-I", include, str(src), "-o", str(out)]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"g++ failed:\n{r.stdout}\n{r.stderr}")

@@ -15,6 +15,8 @@ from pathlib import Path
 
 import torch
 
+from .. import build
+
 _LIB = None
 _HALF = None
 _CALLS = None
@@ -61,9 +63,9 @@ class _HalfView:
 
 def _load_calls():
     """The native module built from csrc/host_calls.cpp."""
-    path = _LIB_PATH.parent / "neox_host_calls.so"
+    path = build.host_calls_path()
     if not path.exists():
-        raise KernelError(f"{path} is missing: build it with `python -m gpt_neox_b200.build`")
+        raise KernelError(f"{path} is missing: build it under this interpreter with `python -m gpt_neox_b200.build`")
     spec = importlib.util.spec_from_loader("neox_host_calls", importlib.machinery.ExtensionFileLoader("neox_host_calls", str(path)))
     calls = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(calls)

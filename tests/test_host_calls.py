@@ -1,5 +1,6 @@
 """Native calls into the kernel library (csrc/host_calls.cpp): arguments, and what a layer's modules are asked, on the CPU."""
 import ctypes as C
+import sys
 
 import pytest
 import torch
@@ -12,6 +13,18 @@ from gpt_neox_b200.ops import _lib
 def calls():
     build.build_host_calls()
     return _lib._load_calls()
+
+
+def test_the_module_is_this_interpreters(calls, monkeypatch, tmp_path):
+    """The file names the interpreter that it was built under; another one does not load it, and is told what to do."""
+    name = build.host_calls_path().name
+    assert sys.implementation.cache_tag in name and calls.__spec__.origin.endswith(name)
+    monkeypatch.setattr(build.sysconfig, "get_config_var", lambda key: ".cpython-399-x86_64-linux-gnu.so")
+    with pytest.raises(_lib.KernelError, match="cpython-399.*this interpreter"):
+        _lib._load_calls()
+    monkeypatch.setattr(build.sysconfig, "get_paths", lambda: {"include": str(tmp_path)})
+    with pytest.raises(RuntimeError, match="headers"):
+        build.build_host_calls()
 
 
 class _OnGpu:
