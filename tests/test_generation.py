@@ -378,11 +378,21 @@ def test_a_layer_in_one_call_gives_the_bits_of_the_op_by_op_path(over, precision
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("hidden,heads", [(768, 12), (1024, 8)])
-def test_products_in_one_launch_give_the_bits_of_two(hidden, heads):
+def test_products_in_one_launch_give_the_bits_of_two(hidden, heads, monkeypatch):
     """Few rows: query / key / value with the MLP's first product, and dense with its second one, in one launch each, with
     different numbers of splits (dense 2, down 8) - at both sides of every row count the kernel is built for, and of the
-    128 from which they are launched by themselves."""
+    128 from which they are launched by themselves: six launches a layer with both pairs, eight with none."""
     from test_model_gpu import _build
+    from gpt_neox_b200.models import transformer
+    from gpt_neox_b200.ops.gemm import LAUNCHES
+    launches, call = [], transformer.layer_infer
+
+    def counted(*a, **k):
+        before = LAUNCHES["n"]
+        out = call(*a, **k)
+        launches.append(LAUNCHES["n"] - before)
+        return out
+    monkeypatch.setattr(transformer, "layer_infer", counted)
     _, model = _build(tiny_config(num_layers=1, hidden_size=hidden, num_attention_heads=heads, seq_length=512,
                                   max_position_embeddings=512, synthetic_vocab_size=1000, pipe_parallel_size=0,
                                   attention_config=[[["flash"], 1]], distributed_backend="nccl", precision="bfloat16"))
@@ -391,11 +401,13 @@ def test_products_in_one_launch_give_the_bits_of_two(hidden, heads):
     tokens = torch.randint(0, 1000, (1, 512), device="cuda")
     pos = torch.arange(512, device="cuda")[None]
 
+    rows = (1, 15, 16, 17, 32, 33, 64, 65, 96, 128, 130)
+
     def steps():
         model.clear_cache()
         out, at = [], 0
         with torch.no_grad():
-            for n in (1, 15, 16, 17, 32, 33, 64, 65, 96, 128):
+            for n in rows:
                 out.append(model((tokens[:, at:at + n].contiguous(), pos[:, at:at + n].contiguous(), None)))
                 at += n
                 if at > 300:
@@ -404,9 +416,12 @@ def test_products_in_one_launch_give_the_bits_of_two(hidden, heads):
         return out
 
     one = steps()
+    # (128 rows of 768 -> 768 go to the other kernel, whose tiles are enough there)
+    assert launches == [6] * 9 + [8 if hidden == 768 else 6, 8]
     handle = mlp.register_forward_hook(lambda *a: None)
     ops = steps()
     handle.remove()
+    assert len(launches) == len(rows)                   # (the second run went op by op)
     assert all(torch.equal(a, b) for a, b in zip(one, ops)) and all(t.isfinite().all() for t in one)
 
 
