@@ -114,17 +114,18 @@ conv1d_silu_bwd_kernel(const h16* __restrict__ x, long long xsb, long long xst,
   if (dbias) atomicAdd(dbias + d, ab);
 }
 
-// Vector forms: a thread owns four neighbouring channels (an 8-byte load per step, packed pairs) and CV_FWD_T / CV_BWD_T steps, in
+// Vector forms: a thread owns four neighbouring channels (an 8-byte load per step, packed pairs) and `steps` steps (conv_steps), in
 // groups whose loads are asked for together, in the forward one group ahead (the backward has no registers left for that: 54
 // us).  The one-channel kernels above keep one 2-byte load in flight per thread and are bound by its latency; they remain for
 // channel counts, strides or bases that are not multiples of four elements.  The backward walks three steps more than it owns,
-// whose gradient reaches back into its tile; 21 + 3 are whole groups and leave enough blocks (29: 30.4 / 42.2 us).
-// Bound by latency at 28 and 16 warps an SM and by issue slots.  4 x 2048 x 1536 / 16 x 512 x 2048, fp16, us: forward 19.8 / 26.5 with
-// eight channels a thread and no pairs (142 registers), 13.5 / 15.8 now; backward 37.3 / 47.2 with 16 steps a thread, 32.1 / 39.1.
+// whose gradient reaches back into its tile: 5, 13 and 21 + 3 are whole groups.
+// Bound by latency at 28 and 16 warps an SM and by issue slots; calls that leave the chip idle by the chain of a thread's steps.
+// 4 x 2048 x 1536 / 16 x 512 x 2048, fp16, us: forward 19.8 / 26.5 with eight channels a thread and no pairs (142 registers), 12.8 /
+// 15.2 now; backward 37.3 / 47.2 with 16 steps a thread, 32.1 / 39.1.  bf16 the same since conv_loaded: its backward took 56.
 constexpr int CV_X = 32;    // channel groups per block
 constexpr int CV_Y = 4;     // time tiles per block
 constexpr int CV_V = 4;     // channels per thread
-constexpr int CV_FWD_T = 32, CV_BWD_T = 21, CV_G = 4;
+constexpr int CV_G = 4;     // steps per group
 struct Conv4 { float2 a, b; };      // four channels
 __device__ __forceinline__ Conv4 conv_unpack(const uint2& u) { return {unpack_h16x2(u.x), unpack_h16x2(u.y)}; }
 __device__ __forceinline__ uint2 conv_pack(const Conv4& v) { return make_uint2(pack_h16x2(v.a.x, v.a.y), pack_h16x2(v.b.x, v.b.y)); }
@@ -133,6 +134,12 @@ __device__ __forceinline__ Conv4 conv_mul(const Conv4& x, const Conv4& y) { retu
 __device__ __forceinline__ Conv4 conv_sigmoid(const Conv4& x) {
   auto f = [](float v) { return __fdividef(1.f, 1.f + __expf(-v)); };
   return {make_float2(f(x.a.x), f(x.a.y)), make_float2(f(x.b.x), f(x.b.y))};
+}
+// The loads of a group stay together in front of their first use: without this the bf16 build, whose conversions are plain
+// integer operations, moves them into the branches of the single loads, which then wait for one another.
+__device__ __forceinline__ void conv_loaded(uint2 (&u)[CV_G]) {
+#pragma unroll
+  for (int k = 0; k < CV_G; ++k) asm volatile("" : "+r"(u[k].x), "+r"(u[k].y));
 }
 // wk[k]: the tap on step t - 3 + k (zeros in front of a shorter kernel), and the bias
 __device__ __forceinline__ void conv_taps(const h16* w, const h16* bias, int d, int W, Conv4 (&wk)[4], Conv4& bv) {
@@ -153,11 +160,11 @@ __device__ __forceinline__ Conv4 conv_pre(const Conv4 (&wk)[4], const Conv4& bv,
 __global__ void __launch_bounds__(CV_X * CV_Y)
 conv1d_silu_fwd_vec_kernel(const h16* __restrict__ x, long long xsb, long long xst, const h16* __restrict__ w,
                            const h16* __restrict__ bias, h16* __restrict__ y, long long ysb, long long yst, int L,
-                           int D, int W) {
+                           int D, int W, int steps) {
   const int d = (blockIdx.x * CV_X + threadIdx.x) * CV_V;
-  const int t0 = (blockIdx.y * CV_Y + threadIdx.y) * CV_FWD_T, b = blockIdx.z;
+  const int t0 = (blockIdx.y * CV_Y + threadIdx.y) * steps, b = blockIdx.z;
   if (d >= D || t0 >= L) return;
-  const int t1 = min(t0 + CV_FWD_T, L);
+  const int t1 = min(t0 + steps, L);
   const h16* xp = x + b * xsb + d;
   uint2 now[CV_G], next[CV_G];
   auto fetch = [&](int t, uint2 (&u)[CV_G]) {
@@ -179,6 +186,9 @@ conv1d_silu_fwd_vec_kernel(const h16* __restrict__ x, long long xsb, long long x
   h16* yp = y + b * ysb + t0 * yst + d;
 #pragma unroll 1
   for (int t = t0; t < t1; t += CV_G) {
+#ifndef NX_HALF
+    conv_loaded(now);      // (fp16: 0.7 us more)
+#endif
     fetch(t + CV_G, next);
 #pragma unroll
     for (int k = 0; k < CV_G; ++k) {
@@ -192,6 +202,7 @@ conv1d_silu_fwd_vec_kernel(const h16* __restrict__ x, long long xsb, long long x
   }
 }
 
+template <int STEPS>      // (a number that the kernel is called with takes 4 - 7 % longer)
 __global__ void __launch_bounds__(CV_X * CV_Y, 4)
 conv1d_silu_bwd_vec_kernel(const h16* __restrict__ x, long long xsb, long long xst, const h16* __restrict__ w,
                            const h16* __restrict__ bias, const h16* __restrict__ dy, long long dsb, long long dst,
@@ -199,12 +210,12 @@ conv1d_silu_bwd_vec_kernel(const h16* __restrict__ x, long long xsb, long long x
                            float* __restrict__ dbias, int L, int D, int W) {
   __shared__ float red[CV_Y][CV_X][CV_V * 5 + 1];
   const int d = (blockIdx.x * CV_X + threadIdx.x) * CV_V;
-  const int t0 = (blockIdx.y * CV_Y + threadIdx.y) * CV_BWD_T, b = blockIdx.z;
+  const int t0 = (blockIdx.y * CV_Y + threadIdx.y) * STEPS, b = blockIdx.z;
   Conv4 aw[5] = {};                       // gradients of the four taps and the bias
   if (d < D && t0 < L) {
     const h16* xp = x + b * xsb + d;
     const h16* gp = dy + b * dsb + d;
-    const int t_own = min(t0 + CV_BWD_T, L), t_end = min(t0 + CV_BWD_T + 3, L);
+    const int t_own = min(t0 + STEPS, L), t_end = min(t0 + STEPS + 3, L);
     uint2 rx[CV_G], rg[CV_G];
     auto fetch = [&](int t, uint2 (&u)[CV_G], uint2 (&g)[CV_G]) {
 #pragma unroll
@@ -215,6 +226,8 @@ conv1d_silu_bwd_vec_kernel(const h16* __restrict__ x, long long xsb, long long x
           g[k] = *reinterpret_cast<const uint2*>(gp + (t + k) * dst);
         }
       }
+      conv_loaded(u);
+      conv_loaded(g);
     };
     Conv4 wk[4], bv, win[3], dp[3] = {};
 #pragma unroll
@@ -225,7 +238,7 @@ conv1d_silu_bwd_vec_kernel(const h16* __restrict__ x, long long xsb, long long x
     }
     conv_taps(w, bias, d, W, wk, bv);
 #pragma unroll 1
-    for (int s = 0; s < CV_BWD_T + 3; s += CV_G) {
+    for (int s = 0; s < STEPS + 3; s += CV_G) {
       fetch(t0 + s, rx, rg);
 #pragma unroll
       for (int k = 0; k < CV_G; ++k) {
@@ -274,6 +287,16 @@ conv1d_silu_bwd_vec_kernel(const h16* __restrict__ x, long long xsb, long long x
 static bool vec_ok(const void* p, long long sb, long long st, int V) {
   return (reinterpret_cast<uintptr_t>(p) & (V * 2 - 1)) == 0 && sb % V == 0 && st % V == 0;
 }
+// Steps per thread, by the work per SM (in steps of four channels): as few as still leave every SM enough threads, since a thread's
+// steps are a chain; more where the three steps in front of a tile (backward: behind it), which are read again, count.  us,
+// forward, 4 / 8 / 16 / 32 steps: 1 x 128 x 1536 (330 per SM) 2.3, 2.7, 3.5, 5.2; 4 x 128 x 1536 (1,330) 3.3, 3.3, 3.6, 5.2; 4 x 512 x
+// 1536 (5,300) 7.1, 5.9, 5.6, 6.3; 4 x 2048 x 1536 (21,000) 19.5, 14.2, 12.8, 13.5; 16 x 512 x 2048 (28,000) 25.4, 17.8, 15.5, 15.2.
+// Backward with its forward, 5 / 13 / 21 steps: 14.8, 16.4, 18.1; 16.4, 16.5, 18.1; 25.2, 21.7, 22.6; 66, 51, 52; 83, 65, 62.
+static int conv_steps(int B, int L, int D, bool backward) {
+  const long long per_sm = static_cast<long long>(B) * L * (D / CV_V) / sm_count();
+  if (backward) return per_sm <= 1800 ? 5 : per_sm <= 6800 ? 13 : 21;
+  return per_sm <= 450 ? 4 : per_sm <= 1800 ? 8 : per_sm <= 24000 ? 16 : 32;
+}
 static dim3 conv_vec_grid(int B, int L, int D, int steps) {
   return dim3((D / CV_V + CV_X - 1) / CV_X, (L + steps * CV_Y - 1) / (steps * CV_Y), B);
 }
@@ -283,8 +306,9 @@ NX_API int NX_SYM(nx_conv1d_silu_fwd)(const void* x, long long xsb, long long xs
                               cudaStream_t stream) {
   NX_REQUIRE(W >= 1 && W <= 4, "conv1d: kernel width %d not in [1, 4]", W);
   if (D % CV_V == 0 && vec_ok(x, xsb, xst, CV_V) && vec_ok(y, ysb, yst, CV_V)) {
-    conv1d_silu_fwd_vec_kernel<<<conv_vec_grid(B, L, D, CV_FWD_T), dim3(CV_X, CV_Y), 0, stream>>>(
-        (const h16*)x, xsb, xst, (const h16*)w, (const h16*)bias, (h16*)y, ysb, yst, L, D, W);
+    const int steps = conv_steps(B, L, D, false);
+    conv1d_silu_fwd_vec_kernel<<<conv_vec_grid(B, L, D, steps), dim3(CV_X, CV_Y), 0, stream>>>(
+        (const h16*)x, xsb, xst, (const h16*)w, (const h16*)bias, (h16*)y, ysb, yst, L, D, W, steps);
     NX_LAUNCH_CHECK();
     return NX_OK;
   }
@@ -302,9 +326,15 @@ NX_API int NX_SYM(nx_conv1d_silu_bwd)(const void* x, long long xsb, long long xs
                               cudaStream_t stream) {
   NX_REQUIRE(W >= 1 && W <= 4, "conv1d: kernel width %d not in [1, 4]", W);
   if (D % CV_V == 0 && vec_ok(x, xsb, xst, CV_V) && vec_ok(dy, dsb, dst, CV_V) && vec_ok(dx, gsb, gst, CV_V)) {
-    conv1d_silu_bwd_vec_kernel<<<conv_vec_grid(B, L, D, CV_BWD_T), dim3(CV_X, CV_Y), 0, stream>>>(
-        (const h16*)x, xsb, xst, (const h16*)w, (const h16*)bias, (const h16*)dy, dsb, dst, (h16*)dx, gsb, gst,
-        (float*)dw, (float*)dbias, L, D, W);
+    const int steps = conv_steps(B, L, D, true);
+    auto run = [&](auto kern) {
+      kern<<<conv_vec_grid(B, L, D, steps), dim3(CV_X, CV_Y), 0, stream>>>(
+          (const h16*)x, xsb, xst, (const h16*)w, (const h16*)bias, (const h16*)dy, dsb, dst, (h16*)dx, gsb, gst,
+          (float*)dw, (float*)dbias, L, D, W);
+    };
+    if (steps == 5) run(conv1d_silu_bwd_vec_kernel<5>);
+    else if (steps == 13) run(conv1d_silu_bwd_vec_kernel<13>);
+    else run(conv1d_silu_bwd_vec_kernel<21>);
     NX_LAUNCH_CHECK();
     return NX_OK;
   }

@@ -216,6 +216,25 @@ def test_selective_scan_softplus_at_the_ends():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,L,D", [(1, 22, 8), (3, 129, 2052), (2, 707, 1536), (4, 2501, 1544)])
+def test_conv1d_silu_steps_per_thread(B, L, D, dtype):
+    """4, 8, 16 and 32 steps a thread forward, and 5, 5, 13 and 21 backward (on 148 SMs), with ragged ends."""
+    from gpt_neox_b200.ops.mamba import causal_conv1d_silu, causal_conv1d_silu_reference
+    torch.manual_seed(8)
+    mk = lambda *s: (torch.randn(*s, device="cuda") * 0.5).to(dtype).requires_grad_()
+    x, w, b, g = mk(B, L, D), mk(D, 4), mk(D), mk(B, L, D).detach()
+    ref = [t.detach().double().requires_grad_() for t in (x, w, b)]
+    y = causal_conv1d_silu(x, w, b)
+    yr = torch.nn.functional.silu(torch.nn.functional.conv1d(ref[0].transpose(1, 2), ref[1][:, None], ref[2], padding=3,
+                                                             groups=D)[..., :L].transpose(1, 2))
+    eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -11
+    for a, r in zip((y,) + torch.autograd.grad(y, [x, w, b], g), (yr,) + torch.autograd.grad(yr, ref, g.double())):
+        # one rounding to 16 bits; fp32 sums over B L steps for the taps and the bias
+        assert ((a.double() - r).abs() <= eps * r.abs() + 2 ** -20 * (B * L) ** 0.5).all()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("what,value", [("x", float("nan")), ("dt", float("nan")), ("B", float("nan")), ("C", float("inf")),
                                         ("z", float("nan")), ("x", float("inf"))])
 @pytest.mark.parametrize("at", [0, 37, 255, 299])
