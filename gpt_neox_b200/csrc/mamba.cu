@@ -6,27 +6,29 @@
 // the external causal_conv1d / mamba_ssm packages, called at megatron/model/mamba/mamba.py:220-247
 // and :264-320 (which run on [batch, channel, seq] and need two rearranges per block).
 //
-// Scan parallelisation: a lane owns 4 of the 16 states of two neighbouring channels (a quad of lanes per pair), a warp 16
-// channels, and walks its piece of the sequence in blocks of 32 steps, cut into segments of four: lane q of a quad reads,
-// prepares and finishes step q of a segment, so the forward sweeps and the light reverse sweep need no barrier but the
-// warp's.  The sequence is cut into as few chunks as keep the chip busy (scan_chunk_count): one chunk needs one pass; with
-// more, a light pass first runs every chunk from a zero state and records its end state and its sum of delta (the chunk's
-// decay is exp(A * sum delta)), and the main pass folds the other chunks into its start state.  The reverse recurrence of
-// dL/dh is cut the same way.
+// Scan parallelisation: a lane owns 4 of the 16 states of two neighbouring channels (a quad of lanes per pair; of one channel where
+// there are so few that the chip would be idle), a warp 16 (8) channels, and walks its piece of the sequence in blocks of 32
+// steps, cut into segments of four: lane q of a quad reads, prepares and finishes step q of a segment, so the forward sweeps and the
+// light reverse sweep need no barrier but the warp's.  The sequence is cut into as few chunks as keep the chip busy (scan_plan): one
+// chunk needs one pass; with more, a light pass first runs every chunk from a zero state and records its end state and its sum
+// of delta (the chunk's decay is exp(A * sum delta)), and the main pass folds the other chunks into its start state.  The reverse
+// recurrence of dL/dh is cut the same way.
 // The forward keeps the state at the start of every 32-step block for the backward, which recomputes the states at the
 // starts of the segments, then four steps at a time into registers, and walks them in reverse; dB and dC are added over a
-// lane's two channels before lanes and warps exchange them, and the next block's segment is staged where the walked one
+// lane's channels before lanes and warps exchange them, and the next block's segment is staged where the walked one
 // was.  Those states take 2 bytes per token and channel from the forward to the backward (25 MB for 4 x 2048 x 1536, as
 // much as one more 16-bit activation), and the tiles' partial sums of dB and dC 2 bytes during the backward.
 // Bound by: light sweeps, the unit of exponentials (16 per step and channel; 82 and 72 % busy); forward, that unit 68 %, shared
 // memory 69 % and issue slots 62 % together; backward, issue slots (59 % with 3 warps per scheduler; shared memory 55 %),
 // where a step and channel costs 500 lane operations for 16 states.  DRAM 6-10 %.
 // Convolution + scan, forward + backward, 4 x 2048 steps of 1536 channels, fp16: 785 us with one channel per quad, inputs staged
-// by the whole CTA and dB / dC exchanged per channel (final forward sweep 119, light ones 70 and 86, backward 407 us); 605 us
-// with the present scan (95, 63 and 78, 283), 594 with the present convolution, too.  Whole calls of few channels and one block
-// are latency: 2 x 31 x 768 takes 46 us of kernels, 43 before.
+// by the whole CTA and dB / dC exchanged per channel (final forward sweep 119, light ones 70 and 86, backward 407 us); 583 us
+// now (91, 60 and 74, 277).  Calls of few channels and steps are latency, us, forward / forward + backward, that kernel and this
+// one: 2 x 31 x 768 4.9 / 20.0, 5.2 / 18.1; 1 x 64 x 768 8.7 / 27.1, 8.1 / 25.6; 1 x 128 x 768 9.0 / 28.6, 10.1 / 29.1; 1 x 128 x 1536 9.9 / 37.7,
+// 10.9 / 32.3; 1 x 256 x 1536 13.1 / 45.7, 13.4 / 39.6; 4 x 128 x 1536 18.5 / 66.3, 14.9 / 48.3.
 // Tried for the backward: states packed per channel pair instead of per state pair (B and C twice in shared memory, no copies
-// of a step's scalars): shared memory 62 % busy, 305 - 330 us; inputs staged per block with its loads waited for: 290 - 320.
+// of a step's scalars): shared memory 62 % busy, 305 - 330 us; inputs staged per block with its loads waited for: 290 - 320.  For the
+// forward: the next segment prepared beside the walk of this one: 3 - 5 % more time, with one channel or two.
 #include "common.h"
 #include "ptx.cuh"
 
@@ -353,8 +355,9 @@ NX_API int NX_SYM(nx_conv1d_silu_bwd)(const void* x, long long xsb, long long xs
 constexpr int SC_T = 32;        // steps per block (the forward keeps a state per block for the backward)
 constexpr int SC_SEG = 4;       // steps per segment: lane q of a quad reads, and writes the results of, step q of it
 constexpr int SC_SEGS = SC_T / SC_SEG;
-constexpr int SC_WCH = 16;      // channels per warp, two neighbouring ones per quad of lanes
-constexpr int SC_WARPS = 4, SC_THREADS = SC_WARPS * 32, SC_CH = SC_WARPS * SC_WCH;    // channels per CTA
+constexpr int SC_WARPS = 4, SC_THREADS = SC_WARPS * 32;
+// C, the channels of a quad of lanes: two neighbouring ones, or one where that leaves the chip idle (scan_plan)
+constexpr int scan_channels(int C) { return SC_WARPS * 8 * C; }      // of a CTA
 constexpr int SC_MAX_CHUNKS = 64;
 constexpr int SC_FWD_CTAS = 5, SC_BWD_CTAS = 3;   // CTAs per SM: registers are bounded for so many of them
 constexpr float LOG2E = 1.44269504088896340736f, LN2 = 0.69314718055994530942f;
@@ -406,18 +409,19 @@ __device__ __forceinline__ float quad_sum(float v) {
   return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
-// A lane's place: states 4 q .. 4 q + 3 of the channels d and d + 1.
+// A lane's place: states 4 q .. 4 q + 3 of the channels d .. d + C - 1.
 struct ScanLane {
-  int lane, warp, j, q, d, n;       // n: live channels of the two
+  int lane, warp, j, q, d, n;       // n: live channels of the quad's
 };
+template <int C>
 __device__ __forceinline__ ScanLane scan_lane(int D) {
   ScanLane s;
   s.lane = threadIdx.x & 31;
   s.warp = threadIdx.x >> 5;
   s.j = s.lane >> 2;
   s.q = s.lane & 3;
-  s.d = blockIdx.x * SC_CH + s.warp * SC_WCH + 2 * s.j;
-  s.n = min(2, max(0, D - s.d));
+  s.d = blockIdx.x * scan_channels(C) + (s.warp * 8 + s.j) * C;
+  s.n = min(C, max(0, D - s.d));
   return s;
 }
 // Two neighbouring 16-bit elements (zero where dead): one 4-byte access when VEC, single elements otherwise.
@@ -439,30 +443,33 @@ __device__ __forceinline__ void store2(h16* p, float2 v, int n) {
 __device__ __forceinline__ float2 coef2(const float* p, const ScanLane& s) {
   return make_float2(p != nullptr && s.n > 0 ? p[s.d] : 0.f, p != nullptr && s.n > 1 ? p[s.d + 1] : 0.f);
 }
-// A lane's states: [channel of the two][pair of states].  In memory [channel][16] floats from the channel d on; zero where dead.
+// A lane's states: [channel of the quad][pair of states].  In memory [channel][16] floats from the channel d on; zero where dead.
 __device__ __forceinline__ void get4(const float4& v, float2 (&h)[2]) {
   h[0] = make_float2(v.x, v.y);
   h[1] = make_float2(v.z, v.w);
 }
 __device__ __forceinline__ float4 put4(const float2 (&h)[2]) { return make_float4(h[0].x, h[0].y, h[1].x, h[1].y); }
-__device__ __forceinline__ void load_states(const float* p, const ScanLane& s, float2 (&h)[2][2]) {
+template <int C>
+__device__ __forceinline__ void load_states(const float* p, const ScanLane& s, float2 (&h)[C][2]) {
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
+  for (int i = 0; i < C; ++i) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i < s.n) v = *reinterpret_cast<const float4*>(p + i * 16 + s.q * 4);
     get4(v, h[i]);
   }
 }
-__device__ __forceinline__ void store_states(float* p, const ScanLane& s, const float2 (&h)[2][2]) {
+template <int C>
+__device__ __forceinline__ void store_states(float* p, const ScanLane& s, const float2 (&h)[C][2]) {
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < C; ++i)
     if (i < s.n) *reinterpret_cast<float4*>(p + i * 16 + s.q * 4) = put4(h[i]);
 }
 // The states' decay rates times log2(e).
-__device__ __forceinline__ void load_A(const float* A, const ScanLane& s, float2 (&a)[2][2]) {
+template <int C>
+__device__ __forceinline__ void load_A(const float* A, const ScanLane& s, float2 (&a)[C][2]) {
   load_states(A + static_cast<long long>(s.d) * 16, s, a);
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < C; ++i)
 #pragma unroll
     for (int k = 0; k < 2; ++k) a[i][k] = fmul2(a[i][k], both(LOG2E));
 }
@@ -494,20 +501,22 @@ __device__ __forceinline__ float dot4(const float2 (&a)[2], const float4& b) {
   return v.x + v.y;
 }
 // The state after the chunk c, whose walk from a zero state ended in chunk_state.
-__device__ __forceinline__ void fold_chunk(const ScanParams& p, const ScanLane& s, const float2 (&A)[2][2], int b, int c,
-                                           float2 (&h)[2][2]) {
+template <int C>
+__device__ __forceinline__ void fold_chunk(const ScanParams& p, const ScanLane& s, const float2 (&A)[C][2], int b, int c,
+                                           float2 (&h)[C][2]) {
   const long long o = (static_cast<long long>(b) * p.NC + c) * p.D + s.d;
-  float2 e[2][2];
+  float2 e[C][2];
   load_states(p.chunk_state + o * 16, s, e);
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
+  for (int i = 0; i < C; ++i) {
     float2 a[2];
     decay(A[i], i < s.n ? p.chunk_sumdt[o + i] : 0.f, a);
     h[i][0] = ffma2(a[0], h[i][0], e[i][0]);
     h[i][1] = ffma2(a[1], h[i][1], e[i][1]);
   }
 }
-__device__ __forceinline__ void put_chunk(const ScanParams& p, const ScanLane& s, int b, int c, const float2 (&h)[2][2],
+template <int C>
+__device__ __forceinline__ void put_chunk(const ScanParams& p, const ScanLane& s, int b, int c, const float2 (&h)[C][2],
                                           float2 sdt) {
   const long long o = (static_cast<long long>(b) * p.NC + c) * p.D + s.d;
   store_states(p.chunk_state + o * 16, s, h);
@@ -516,14 +525,14 @@ __device__ __forceinline__ void put_chunk(const ScanParams& p, const ScanLane& s
 }
 
 // FINAL = false: chunks 0 .. NC - 2 from a zero state -> end state and sum of delta.
-template <bool FINAL, bool VEC>
+template <bool FINAL, int C, bool VEC>
 __global__ void __launch_bounds__(SC_THREADS, SC_FWD_CTAS)
 scan_fwd_kernel(const ScanParams p) {
-  // per warp and for two segments in turn: delta and delta * x of a quad's two channels; B and C of the segment's steps
+  // per warp and for two segments in turn: delta and delta * x of a quad's channels; B and C of the segment's steps
   __shared__ float4 dd[SC_WARPS][2][SC_SEG][8], bc[SC_WARPS][2][SC_SEG][FINAL ? 8 : 4];
-  const ScanLane s = scan_lane(p.D);
+  const ScanLane s = scan_lane<C>(p.D);
   const int c = blockIdx.y, b = blockIdx.z, q = s.q;
-  float2 A[2][2], h[2][2] = {};
+  float2 A[C][2], h[C][2] = {};
   load_A(p.A, s, A);
   if (FINAL) {
 #pragma unroll 4
@@ -574,21 +583,21 @@ scan_fwd_kernel(const ScanParams p) {
       if (FINAL && p.ckpt != nullptr && (t0 & (SC_T - 1)) == 0)
         store_states(p.ckpt + ((static_cast<long long>(b) * ((p.L + SC_T - 1) / SC_T) + t0 / SC_T) * p.D + s.d) * 16, s, h);
       __syncwarp();        // (this buffer's last readers have passed the other one's)
-      float yp[2][SC_SEG];
+      float yp[C][SC_SEG];
 #pragma unroll
       for (int t = 0; t < SC_SEG; ++t) {
         const float4 v = dd[s.warp][k][t][s.j ^ (2 * t)], B4 = bc[s.warp][k][t][q];
         float2 a[2];
-        scan_step(A[0], v.x, v.y, B4, a, h[0], h[0]);
-        scan_step(A[1], v.z, v.w, B4, a, h[1], h[1]);
+#pragma unroll
+        for (int i = 0; i < C; ++i) scan_step(A[i], i == 0 ? v.x : v.z, i == 0 ? v.y : v.w, B4, a, h[i], h[i]);
         if (FINAL) {
           const float4 C4 = bc[s.warp][k][t][4 + q];
-          yp[0][t] = dot4(h[0], C4);
-          yp[1][t] = dot4(h[1], C4);
+#pragma unroll
+          for (int i = 0; i < C; ++i) yp[i][t] = dot4(h[i], C4);
         }
       }
       if (FINAL) {
-        float2 y = ffma2(Dv, xv, make_float2(quad_transpose_sum(yp[0], q), quad_transpose_sum(yp[1], q)));
+        float2 y = ffma2(Dv, xv, make_float2(quad_transpose_sum(yp[0], q), C > 1 ? quad_transpose_sum(yp[C - 1], q) : 0.f));
         if (p.z != nullptr) y = make_float2(y.x * silu(zv.x), y.y * silu(zv.y));
         if (in) store2<VEC>(op, y, s.n);
         op += SC_SEG * p.ost;
@@ -599,14 +608,14 @@ scan_fwd_kernel(const ScanParams p) {
 }
 
 // Reverse recurrence of chunks 1 .. NC - 1 from a zero carry: chunk_state[c] = what chunk c hands to chunk c - 1.
-template <bool VEC>
+template <int C, bool VEC>
 __global__ void __launch_bounds__(SC_THREADS, SC_FWD_CTAS)
 scan_bwd_local_kernel(const ScanParams p) {
-  // as in the forward: delta and the gradient of the ungated output of a quad's two channels; C
+  // as in the forward: delta and the gradient of the ungated output of a quad's channels; C
   __shared__ float4 dd[SC_WARPS][2][SC_SEG][8], cs[SC_WARPS][2][SC_SEG][4];
-  const ScanLane s = scan_lane(p.D);
+  const ScanLane s = scan_lane<C>(p.D);
   const int c = blockIdx.y + 1, b = blockIdx.z, q = s.q;
-  float2 A[2][2], r[2][2] = {};
+  float2 A[C][2], r[C][2] = {};
   load_A(p.A, s, A);
   const int tc0 = c * p.clen, t_end = min(tc0 + p.clen, p.L);
   const int last = tc0 + (t_end - 1 - tc0) / SC_SEG * SC_SEG, bt = s.j & 3;
@@ -653,7 +662,7 @@ scan_bwd_local_kernel(const ScanParams p) {
       for (int t = SC_SEG - 1; t >= 0; --t) {
         const float4 v = dd[s.warp][k][t][s.j ^ (2 * t)], C4 = cs[s.warp][k][t][q];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < C; ++i) {
           const float2 g2 = both(i == 0 ? v.y : v.w);
           float2 a[2];
           decay(A[i], i == 0 ? v.x : v.z, a);
@@ -666,21 +675,38 @@ scan_bwd_local_kernel(const ScanParams p) {
   put_chunk(p, s, b, c, r, sdt);
 }
 
-struct ScanBwdWarp {
-  float4 dd[SC_T][SC_WCH];            // delta, x, gradient of the ungated output, sigmoid(dt) of the warp's channels
-  float4 ck[SC_SEGS - 1][2][32];      // a lane's states at the starts of the segments 1 .., per channel
+// With one channel there are no second halves of a segment's states (see ScanBwdWarp): room of its own.
+template <int C>
+struct ScanBwdRoom { float4 own[3][32]; };
+template <>
+struct ScanBwdRoom<2> {};
+template <int C>
+struct ScanBwdWarp : ScanBwdRoom<C> {
+  float4 dd[SC_T][8 * C];             // delta, x, gradient of the ungated output, sigmoid(dt) of the warp's channels
+  float4 ck[SC_SEGS - 1][C][32];      // a lane's states at the starts of the segments 1 .., per channel
   float2 dzf[SC_SEGS][32];            // d out / d z without the scan value, of the lane that writes it
   // A segment's states make room, once used: the first half for the sums over the warp's channels, dB and dC as [step][32]
   // (segment 0 has no states here, its sums go to the second half of segment 5), the second halves of the last two for the
   // state at the block's start, and of segments 3 and 4 for that of the next block to be walked.
-  __device__ __forceinline__ float* sums(int sg) { return reinterpret_cast<float*>(sg > 0 ? ck[sg - 1][0] : ck[4][1]); }
-  __device__ __forceinline__ float4* start(int i, int lane) { return &ck[5 + i][1][lane]; }
-  __device__ __forceinline__ float4* next_start(int i, int lane) { return &ck[2 + i][1][lane]; }
-  // a step's 16 channels, placed so that neither a segment's writers (a step per lane of a quad) nor a step's readers collide
+  __device__ __forceinline__ float* sums(int sg) {
+    if (sg > 0) return reinterpret_cast<float*>(ck[sg - 1][0]);
+    if constexpr (C > 1) return reinterpret_cast<float*>(ck[4][1]);
+    else return reinterpret_cast<float*>(this->own[0]);
+  }
+  __device__ __forceinline__ float4* start(int i, int lane) {
+    if constexpr (C > 1) return &ck[5 + i][1][lane];
+    else return &this->own[1][lane];
+  }
+  __device__ __forceinline__ float4* next_start(int i, int lane) {
+    if constexpr (C > 1) return &ck[2 + i][1][lane];
+    else return &this->own[2][lane];
+  }
+  // a step's channels, placed so that neither a segment's writers (a step per lane of a quad) nor a step's readers collide
   static __device__ __forceinline__ int slot(int t, int j, int i) { return i * 8 + (j ^ (2 * (t & 3))); }
 };
+template <int C>
 struct ScanBwdSmem {
-  ScanBwdWarp w[SC_WARPS];
+  ScanBwdWarp<C> w[SC_WARPS];
   float bc[SC_T][32];                 // B | C
 };
 // 16 bytes to shared memory behind the thread's back (zeros where dead); waited for by the thread that asked.
@@ -693,15 +719,15 @@ __device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.com
 template <int N>
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <bool VEC>
+template <int C, bool VEC>
 __global__ void __launch_bounds__(SC_THREADS, SC_BWD_CTAS)
 scan_bwd_kernel(const ScanParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  ScanBwdSmem& sm = *reinterpret_cast<ScanBwdSmem*>(smem_raw);
-  const ScanLane s = scan_lane(p.D);
-  ScanBwdWarp& w = sm.w[s.warp];
+  ScanBwdSmem<C>& sm = *reinterpret_cast<ScanBwdSmem<C>*>(smem_raw);
+  const ScanLane s = scan_lane<C>(p.D);
+  ScanBwdWarp<C>& w = sm.w[s.warp];
   const int c = blockIdx.y, b = blockIdx.z, q = s.q, lane = s.lane;
-  float2 A[2][2], r[2][2] = {}, dA[2][2] = {};
+  float2 A[C][2], r[C][2] = {}, dA[C][2] = {};
   load_A(p.A, s, A);
 #pragma unroll 4
   for (int cp = p.NC - 1; cp > c; --cp) fold_chunk(p, s, A, b, cp, r);
@@ -715,7 +741,7 @@ scan_bwd_kernel(const ScanParams p) {
   const float* ckpt = p.ckpt + (static_cast<long long>(b) * ((p.L + SC_T - 1) / SC_T) * p.D + s.d) * 16 + q * 4;
   const int last = tc0 + (t_end - 1 - tc0) / SC_T * SC_T;
   struct Raw { uint32_t x, d, g, z; };
-  auto fetch = [&](int t, Raw& u) {               // the lane's two channels of step t
+  auto fetch = [&](int t, Raw& u) {               // the lane's channels of step t
     const int n = t < t_end ? s.n : 0;
     u.x = load2<VEC>(p.x + b * p.xsb + t * p.xst + s.d, n);
     u.d = load2<VEC>(p.dt + b * p.dsb + t * p.dst + s.d, n);
@@ -734,14 +760,14 @@ scan_bwd_kernel(const ScanParams p) {
       dys = fmul2(dys, zs);
     }
     w.dd[sg * SC_SEG + q][w.slot(q, s.j, 0)] = make_float4(dl.x, xv.x, dys.x, sd.x);
-    w.dd[sg * SC_SEG + q][w.slot(q, s.j, 1)] = make_float4(dl.y, xv.y, dys.y, sd.y);
+    if (C > 1) w.dd[sg * SC_SEG + q][w.slot(q, s.j, C - 1)] = make_float4(dl.y, xv.y, dys.y, sd.y);
     w.dzf[sg][lane] = dzf;
   };
   auto fetch_start = [&](int t0, float4* a, float4* b, bool any) {        // the state at the start of a block
     if (any) {
       const float* src = ckpt + static_cast<long long>(t0 / SC_T) * p.D * 16;
       copy16_async(a, s.n > 0 ? src : p.ckpt, s.n > 0);
-      copy16_async(b, s.n > 1 ? src + 16 : p.ckpt, s.n > 1);
+      if (C > 1) copy16_async(b, s.n > 1 ? src + 16 : p.ckpt, s.n > 1);
     }
     copy_async_commit();
   };
@@ -769,12 +795,12 @@ scan_bwd_kernel(const ScanParams p) {
         copy_async_wait<1>();
       }
       if (sg < segs) {
-        float2 aB[SC_SEG][2], aC[SC_SEG][2];        // dB and dC of the quad's two channels
-        float ox[2], ot[2], oz[2];
+        float2 aB[SC_SEG][2], aC[SC_SEG][2];        // dB and dC of the quad's channels
+        float ox[2] = {}, ot[2] = {}, oz[2] = {};
         const bool in = t0 + tb + q < t_end;
         const float2 dzf = w.dzf[sg][lane];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < C; ++i) {
           float2 hs[SC_SEG + 1][2], as[SC_SEG][2];  // hs[t + 1]: state after step t
           float4 v[SC_SEG];
           float dx[SC_SEG];
@@ -872,9 +898,9 @@ scan_bwd_kernel(const ScanParams p) {
     }
     if (!more) break;
     copy_async_wait<0>();
-    float2 h[2][2];
-    get4(*w.next_start(0, lane), h[0]);
-    get4(*w.next_start(1, lane), h[1]);
+    float2 h[C][2];
+#pragma unroll
+    for (int i = 0; i < C; ++i) get4(*w.next_start(i, lane), h[i]);
     __syncthreads();                  // B and C of the next block are there, and the sums have been read
     // the states at the starts of its segments (read back by the lane that wrote them)
     const int next_segs = min(SC_SEGS, (t_end - tn + SC_SEG - 1) / SC_SEG);
@@ -884,20 +910,20 @@ scan_bwd_kernel(const ScanParams p) {
       for (int t = 0; t < SC_SEG; ++t) {
         const float4 B4 = *reinterpret_cast<const float4*>(&sm.bc[sg * SC_SEG + t][q * 4]);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < C; ++i) {
           const float2 v = *reinterpret_cast<const float2*>(&w.dd[sg * SC_SEG + t][w.slot(t, s.j, i)]);
           float2 a[2];
           scan_step(A[i], v.x, v.x * v.y, B4, a, h[i], h[i]);
         }
       }
 #pragma unroll
-      for (int i = 0; i < 2; ++i) w.ck[sg][i][lane] = put4(h[i]);
+      for (int i = 0; i < C; ++i) w.ck[sg][i][lane] = put4(h[i]);
     }
   }
   sumD = make_float2(quad_sum(sumD.x), quad_sum(sumD.y));
   sumb = make_float2(quad_sum(sumb.x), quad_sum(sumb.y));
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < C; ++i)
     if (i < s.n) {
       float* o = p.dA + (s.d + i) * 16 + q * 4;
       atomicAdd(o, dA[i][0].x);
@@ -909,67 +935,87 @@ scan_bwd_kernel(const ScanParams p) {
     }
 }
 
-// dB and dC of every (batch, step): the channel tiles' partial sums, rounded once.
+// dB and dC of every (batch, step): the channel tiles' partial sums, rounded once.  Four groups of eight lanes share a row's tiles,
+// so that few rows with many tiles are a short chain of loads.
 __global__ void __launch_bounds__(256)
 scan_bc_reduce_kernel(const float* __restrict__ part, int ntiles, long long rows, h16* __restrict__ dB,
                       h16* __restrict__ dC) {
-  const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;    // 4 of a row's 32 values
-  if (i >= rows * 8) return;
+  const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);    // a warp per row
+  if (row >= rows) return;
+  const int c4 = (threadIdx.x & 7) * 4;                                                 // 4 of its 32 values
+  part += row * 32 + c4;
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-  for (int k = 0; k < ntiles; ++k) {
-    const float4 v = *reinterpret_cast<const float4*>(part + (k * rows * 8 + i) * 4);
+#pragma unroll 4
+  for (int k = (threadIdx.x >> 3) & 3; k < ntiles; k += 4) {
+    const float4 v = *reinterpret_cast<const float4*>(part + k * rows * 32);
     a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
   }
-  const int c4 = static_cast<int>(i & 7) * 4;
-  h16* o = (c4 < 16 ? dB : dC) + (i >> 3) * 16 + (c4 & 15);
+#pragma unroll
+  for (int m = 8; m < 32; m *= 2) {
+    a.x += __shfl_xor_sync(0xffffffffu, a.x, m);
+    a.y += __shfl_xor_sync(0xffffffffu, a.y, m);
+    a.z += __shfl_xor_sync(0xffffffffu, a.z, m);
+    a.w += __shfl_xor_sync(0xffffffffu, a.w, m);
+  }
+  if (threadIdx.x & 24) return;
+  h16* o = (c4 < 16 ? dB : dC) + row * 16 + (c4 & 15);
   *reinterpret_cast<uint2*>(o) = make_uint2(pack_h16x2(a.x, a.y), pack_h16x2(a.z, a.w));
 }
 
-// Chunks the sequence is cut into.  Time goes with the blocks of a chunk times the rounds that the CTAs take; a last round
-// that leaves an SM only some of its CTAs is shorter (measured, time of a block with 1, 2, 3 CTAs on every SM: backward 0.57,
-// 0.77, 1; forward, 1 .. 5: 0.48, 0.54, 0.66, 0.85, 1).  More than one chunk adds the light pass over all chunks but one, whose
-// block takes `light` of the main pass's (forward 7.2 of 10 us, backward 9 of 18.5, with every SM full).  us, forward + backward,
-// fp16, with 1, 4, 8, 16, 22 and 32 chunks: 4 x 2048 x 1536: 983, 586, 552, 511, 506, 525 (the rule: 22 and 32);
-// 16 x 512 x 1536: 416, 485, 486, 531 (1 and 1); 1 x 4096 x 1536: 1871, 779, 473, 312, 315, 311 (26 and 16).  The count depends
-// on the batch and the channels, and the chunks' states are folded in fp32: a sequence's last bits are not those it has in
-// another batch.
+static int scan_tiles(int D, int C) { return (D + scan_channels(C) - 1) / scan_channels(C); }
+// Channels of a quad and chunks the sequence is cut into.  Time goes with the blocks of a chunk times the rounds that the CTAs take; a
+// last round that leaves an SM only some of its CTAs is shorter (measured, time of a block with 1, 2, 3 CTAs on every SM: backward
+// 0.57, 0.77, 1; forward, 1 .. 5: 0.48, 0.54, 0.66, 0.85, 1).  More than one chunk adds the light pass over all chunks but one, whose
+// block takes `light` of the main pass's (forward 7.2 of 10 us, backward 9 of 18.5, with every SM full), and its launch.  us, forward +
+// backward, fp16, with 1, 4, 8, 16, 22 and 32 chunks: 4 x 2048 x 1536: 980, 568, 530, 506, 502, 514 (the rule: 22 and 16);
+// 16 x 512 x 1536: 413, 446, 444, 473 (1 and 1); 1 x 4096 x 1536: 1808, 683, 466, 312, 315, 311 (43 and 43).
+// With one channel a quad a block takes `one` of the time with two, and there are twice the CTAs: shorter where CTAs are few.  us,
+// forward / backward, two channels and one, at the better count of chunks: 2 x 31 x 768 6.2, 5.3 / 16.0, 12.8; 1 x 64 x 768 10.1, 7.9 /
+// 21.4, 17.9; 1 x 128 x 1536 11.5, 10.9 / 22.7, 21.5; 1 x 512 x 768 15.1, 13.9 / 27.8, 26.2; 4 x 128 x 1536 14.8, 17.5 / 32.9, 40.0; 4 x
+// 2048 x 1536 144, 186 / 356, 465.
+// Both depend on the batch and the channels, and the chunks' states are folded in fp32: a sequence's last bits are not those it has
+// in another batch.
 static float scan_rounds(long long ctas, int per_sm) {
   const int sms = sm_count();
   const long long slots = static_cast<long long>(per_sm) * sms, rest = ctas % slots;
   return static_cast<float>(ctas / slots) + (rest > 0 ? 0.35f + 0.65f * static_cast<float>((rest + sms - 1) / sms) / per_sm : 0.f);
 }
-static int scan_chunk_count(int B, int L, int D, int ctas, float light) {
-  const long long tiles = static_cast<long long>((D + SC_CH - 1) / SC_CH) * B;
-  const int blocks = (L + SC_T - 1) / SC_T;
-  int best = 1;
+struct ScanPlan { int C, NC; };      // channels of a quad, chunks
+static ScanPlan scan_plan(int B, int L, int D, bool backward) {
+  const int ctas = backward ? SC_BWD_CTAS : SC_FWD_CTAS, blocks = (L + SC_T - 1) / SC_T;
+  const float light = backward ? 0.48f : 0.7f, one = backward ? 0.67f : 0.74f, launch = backward ? 0.11f : 0.2f;
+  ScanPlan best{2, 1};
   float best_cost = 1e30f;
-  for (int nc = 1; nc <= SC_MAX_CHUNKS && nc <= blocks; ++nc) {
-    const int len = (blocks + nc - 1) / nc, real = (blocks + len - 1) / len;
-    if (real != nc) continue;
-    // (a tenth of a block to begin a chunk, and its fold of the other chunks' states)
-    float cost = (len + 0.1f + 0.002f * nc) * scan_rounds(tiles * nc, ctas);
-    if (nc > 1) cost += light * (len + 0.1f) * scan_rounds(tiles * (nc - 1), SC_FWD_CTAS);
-    if (cost < best_cost) {
-      best_cost = cost;
-      best = nc;
+  for (int C = 2; C >= 1; --C) {
+    const long long tiles = static_cast<long long>(scan_tiles(D, C)) * B;
+    const float unit = C == 1 ? one : 1.f;
+    for (int nc = 1; nc <= SC_MAX_CHUNKS && nc <= blocks; ++nc) {
+      const int len = (blocks + nc - 1) / nc, real = (blocks + len - 1) / len;
+      if (real != nc) continue;
+      // (a tenth of a block to begin a chunk, and its fold of the other chunks' states)
+      float cost = unit * (len + 0.1f + 0.002f * nc) * scan_rounds(tiles * nc, ctas);
+      if (nc > 1) cost += unit * light * (len + 0.1f) * scan_rounds(tiles * (nc - 1), SC_FWD_CTAS) + launch;
+      if (cost < best_cost) {
+        best_cost = cost;
+        best = {C, nc};
+      }
     }
   }
   return best;
 }
-constexpr float LIGHT_FWD = 0.7f, LIGHT_BWD = 0.48f;
 
-NX_API int NX_SYM(nx_scan_chunks)(int B, int L, int D, int backward) {
-  return scan_chunk_count(B, L, D, backward ? SC_BWD_CTAS : SC_FWD_CTAS, backward ? LIGHT_BWD : LIGHT_FWD);
-}
-NX_API int NX_SYM(nx_scan_channel_blocks)(int D) { return (D + SC_CH - 1) / SC_CH; }
+NX_API int NX_SYM(nx_scan_chunks)(int B, int L, int D, int backward) { return scan_plan(B, L, D, backward != 0).NC; }
+NX_API int NX_SYM(nx_scan_tiles)(int B, int L, int D) { return scan_tiles(D, scan_plan(B, L, D, true).C); }
 NX_API int NX_SYM(nx_scan_blocks)(int L) { return (L + SC_T - 1) / SC_T; }
 
-static void scan_common(ScanParams& p, int B, int L, int D, int ctas, float light) {
+// -> channels of a quad
+static int scan_common(ScanParams& p, int B, int L, int D, bool backward) {
+  const ScanPlan plan = scan_plan(B, L, D, backward);
   p.B = B; p.L = L; p.D = D;
-  p.NC = scan_chunk_count(B, L, D, ctas, light);
+  p.NC = plan.NC;
   p.clen = ((L + SC_T - 1) / SC_T + p.NC - 1) / p.NC * SC_T;
   p.bc_vec = vec_ok(p.Bm, p.bsb, p.bst, 4) && vec_ok(p.Cm, p.csb, p.cst, 4);
+  return plan.C;
 }
 
 // A [D,16] fp32 (negative), Dv [D] fp32 or null, dt_bias [D] fp32; x/dt/z/out bf16 addressed by
@@ -992,24 +1038,26 @@ NX_API int NX_SYM(nx_selective_scan_fwd)(const void* x, long long xsb, long long
   p.out = (h16*)out; p.osb = osb; p.ost = ost;
   p.chunk_state = (float*)chunk_state; p.chunk_sumdt = (float*)chunk_sumdt; p.ckpt = (float*)ckpt;
   if (B <= 0 || L <= 0 || D <= 0) return NX_OK;
-  scan_common(p, B, L, D, SC_FWD_CTAS, LIGHT_FWD);
+  const int C = scan_common(p, B, L, D, false);
   const bool vec = D % 2 == 0 && vec_ok(x, xsb, xst, 2) && vec_ok(dt, dsb, dst, 2) && vec_ok(z, zsb, zst, 2) &&
                    vec_ok(out, osb, ost, 2);
-  const dim3 grid((D + SC_CH - 1) / SC_CH, p.NC, B);
-  if (p.NC > 1) {
-    const dim3 light(grid.x, p.NC - 1, B);
-    if (vec) scan_fwd_kernel<false, true><<<light, SC_THREADS, 0, stream>>>(p);
-    else scan_fwd_kernel<false, false><<<light, SC_THREADS, 0, stream>>>(p);
+  const dim3 grid(scan_tiles(D, C), p.NC, B), light(grid.x, p.NC - 1, B);
+  auto run = [&](auto local, auto final) {
+    if (p.NC > 1) {
+      local<<<light, SC_THREADS, 0, stream>>>(p);
+      NX_LAUNCH_CHECK();
+    }
+    final<<<grid, SC_THREADS, 0, stream>>>(p);
     NX_LAUNCH_CHECK();
-  }
-  if (vec) scan_fwd_kernel<true, true><<<grid, SC_THREADS, 0, stream>>>(p);
-  else scan_fwd_kernel<true, false><<<grid, SC_THREADS, 0, stream>>>(p);
-  NX_LAUNCH_CHECK();
-  return NX_OK;
+    return NX_OK;
+  };
+  if (C == 1) return run(scan_fwd_kernel<false, 1, false>, scan_fwd_kernel<true, 1, false>);
+  if (vec) return run(scan_fwd_kernel<false, 2, true>, scan_fwd_kernel<true, 2, true>);
+  return run(scan_fwd_kernel<false, 2, false>, scan_fwd_kernel<true, 2, false>);
 }
 
 // dx / ddt / dz: bf16 with strides (osb, ost). dB / dC: bf16 [B, L, 16] contiguous.  dA [D,16], dD [D], dbias [D] fp32,
-// zeroed by the caller.  ckpt from the forward.  Scratch (fp32): partBC [nx_scan_channel_blocks(D), B, L, 32],
+// zeroed by the caller.  ckpt from the forward.  Scratch (fp32): partBC [nx_scan_tiles(B, L, D), B, L, 32],
 // chunk_state / chunk_sumdt as in the forward with NC = nx_scan_chunks(B, L, D, 1).
 NX_API int NX_SYM(nx_selective_scan_bwd)(const void* x, long long xsb, long long xst, const void* dt, long long dsb,
                                  long long dst, const void* z, long long zsb, long long zst, const void* Bm,
@@ -1031,29 +1079,34 @@ NX_API int NX_SYM(nx_selective_scan_bwd)(const void* x, long long xsb, long long
   p.partBC = (float*)partBC; p.dA = (float*)dA; p.dD = (float*)dD; p.dbias = (float*)dbias;
   p.ckpt = (float*)ckpt; p.chunk_state = (float*)chunk_state; p.chunk_sumdt = (float*)chunk_sumdt;
   if (B <= 0 || L <= 0 || D <= 0) return NX_OK;
-  scan_common(p, B, L, D, SC_BWD_CTAS, LIGHT_BWD);
+  const int C = scan_common(p, B, L, D, true);
   const bool vec = D % 2 == 0 && vec_ok(x, xsb, xst, 2) && vec_ok(dt, dsb, dst, 2) && vec_ok(z, zsb, zst, 2) &&
                    vec_ok(dout, gsb, gst, 2) && vec_ok(dx, osb, ost, 2) && vec_ok(ddt, osb, ost, 2) &&
                    vec_ok(dz, osb, ost, 2);
-  const dim3 grid((D + SC_CH - 1) / SC_CH, p.NC, B);
-  const int smem = (int)sizeof(ScanBwdSmem);
+  const dim3 grid(scan_tiles(D, C), p.NC, B), light(grid.x, p.NC - 1, B);
+  constexpr int smem1 = sizeof(ScanBwdSmem<1>), smem2 = sizeof(ScanBwdSmem<2>);
   static bool attr_set = false;
   if (!attr_set) {
-    NX_CUDA_CHECK(cudaFuncSetAttribute(scan_bwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    NX_CUDA_CHECK(cudaFuncSetAttribute(scan_bwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    NX_CUDA_CHECK(cudaFuncSetAttribute(scan_bwd_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem1));
+    NX_CUDA_CHECK(cudaFuncSetAttribute(scan_bwd_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2));
+    NX_CUDA_CHECK(cudaFuncSetAttribute(scan_bwd_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2));
     attr_set = true;
   }
-  if (p.NC > 1) {
-    const dim3 light((D + SC_CH - 1) / SC_CH, p.NC - 1, B);
-    if (vec) scan_bwd_local_kernel<true><<<light, SC_THREADS, 0, stream>>>(p);
-    else scan_bwd_local_kernel<false><<<light, SC_THREADS, 0, stream>>>(p);
+  auto run = [&](auto local, auto kern, int smem) {
+    if (p.NC > 1) {
+      local<<<light, SC_THREADS, 0, stream>>>(p);
+      NX_LAUNCH_CHECK();
+    }
+    kern<<<grid, SC_THREADS, smem, stream>>>(p);
     NX_LAUNCH_CHECK();
-  }
-  if (vec) scan_bwd_kernel<true><<<grid, SC_THREADS, smem, stream>>>(p);
-  else scan_bwd_kernel<false><<<grid, SC_THREADS, smem, stream>>>(p);
-  NX_LAUNCH_CHECK();
+    return NX_OK;
+  };
+  const int rc = C == 1 ? run(scan_bwd_local_kernel<1, false>, scan_bwd_kernel<1, false>, smem1)
+                 : vec  ? run(scan_bwd_local_kernel<2, true>, scan_bwd_kernel<2, true>, smem2)
+                        : run(scan_bwd_local_kernel<2, false>, scan_bwd_kernel<2, false>, smem2);
+  if (rc != NX_OK) return rc;
   const long long rows = static_cast<long long>(B) * L;
-  scan_bc_reduce_kernel<<<static_cast<unsigned>((rows * 8 + 255) / 256), 256, 0, stream>>>(
+  scan_bc_reduce_kernel<<<static_cast<unsigned>((rows + 7) / 8), 256, 0, stream>>>(
       (const float*)partBC, (int)grid.x, rows, (h16*)dB, (h16*)dC);
   NX_LAUNCH_CHECK();
   return NX_OK;

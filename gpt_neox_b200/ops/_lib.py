@@ -126,7 +126,7 @@ def _declare(lib, calls):
     sig("nx_conv1d_silu_fwd", [P, L, L, P, P, P, L, L, I, I, I, I, P])
     sig("nx_conv1d_silu_bwd", [P, L, L, P, P, P, L, L, P, L, L, P, P, I, I, I, I, P])
     sig("nx_scan_chunks", [I, I, I, I])
-    sig("nx_scan_channel_blocks", [I])
+    sig("nx_scan_tiles", [I, I, I])
     sig("nx_scan_blocks", [I])
     sig("nx_selective_scan_fwd", [P, L, L, P, L, L, P, L, L, P, L, L, P, L, L, P, P, P, P, L, L, P, P, P, I, I, I, P])
     sig("nx_selective_scan_bwd", [P, L, L, P, L, L, P, L, L, P, L, L, P, L, L, P, P, P, P, L, L, P, P, P, L, L, P, P,

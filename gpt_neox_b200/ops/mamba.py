@@ -135,7 +135,7 @@ class _ScanFn(torch.autograd.Function):
         ddt = torch.empty((L, B, Dm), device=dev, dtype=x.dtype).transpose(0, 1)
         dz = torch.empty((L, B, Dm), device=dev, dtype=x.dtype).transpose(0, 1) if z is not None else None
         dB, dC = (torch.empty((B, L, 16), device=dev, dtype=x.dtype) for _ in range(2))
-        part = torch.empty((L_.nx_scan_channel_blocks(Dm), B, L, 32), device=dev, dtype=torch.float32)
+        part = torch.empty((L_.nx_scan_tiles(B, L, Dm), B, L, 32), device=dev, dtype=torch.float32)
         sums = torch.zeros(Dm * 18, device=dev, dtype=torch.float32)           # dA [Dm, 16], dD [Dm], d dt_bias [Dm]
         dA, dD, dbias = sums[:16 * Dm].view(Dm, 16), sums[16 * Dm:17 * Dm], sums[17 * Dm:]
         dD = dD if D is not None else None

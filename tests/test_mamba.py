@@ -235,6 +235,17 @@ def test_conv1d_silu_steps_per_thread(B, L, D, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,L,D,off,use_z", [(500, 1, 33, 0, True), (480, 3, 34, 0, False), (480, 5, 47, 0, True), (460, 37, 49, 1, True),
+                                             (480, 36, 63, 0, True), (250, 97, 129, 0, False), (460, 40, 64, 1, False)])
+def test_selective_scan_two_channels_a_quad(B, L, D, off, use_z, dtype):
+    """The same with so many sequences that a quad has two channels, the second one dead or read by itself."""
+    from gpt_neox_b200.ops import _lib
+    assert _lib.lib(dtype).nx_scan_tiles(B, L, D) == -(-D // 64)
+    test_selective_scan_pairs_and_segments(B, L, D, off, use_z, dtype)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("what,value", [("x", float("nan")), ("dt", float("nan")), ("B", float("nan")), ("C", float("inf")),
                                         ("z", float("nan")), ("x", float("inf"))])
 @pytest.mark.parametrize("at", [0, 37, 255, 299])
