@@ -18,7 +18,7 @@
 namespace {
 
 PyObject *s_is_cuda, *s_data_ptr, *s_dtype, *s_is_contiguous, *s_forward, *s_forward_hooks, *s_forward_pre_hooks, *s_parameters,
-    *s_modules, *s_buffers, *s_weight, *s_bias, *s_dict, *s_shape;
+    *s_modules, *s_buffers, *s_weight, *s_bias, *s_dict, *s_shape, *s_numel;
 PyObject* host_tensor = nullptr;      // called with a tensor that is not on the GPU: raises
 
 struct Ref {      // an owned reference
@@ -184,12 +184,11 @@ int is_plain(PyObject* m, PyObject* cls, PyObject* forward) {
   return 1;
 }
 
-// A module's parameter (or None): getattr, without the module's __getattr__ where nothing in the instance stands before it.
-PyObject* parameter(PyObject* m, PyObject* name) {
-  Ref d(PyObject_GetAttr(m, s_dict));
-  if (!d) return nullptr;
-  PyObject* params = item(d.o, s_parameters);
-  if (params != nullptr && PyDict_Check(params) && item(d.o, name) == nullptr) {
+// A module's parameter (or None): getattr, without the module's __getattr__ where nothing in the instance, whose __dict__ is `d`,
+// stands before it.
+PyObject* parameter(PyObject* m, PyObject* d, PyObject* name) {
+  PyObject* params = item(d, s_parameters);
+  if (params != nullptr && PyDict_Check(params) && item(d, name) == nullptr) {
     PyObject* p = item(params, name);
     if (p != nullptr) return Py_NewRef(p);
   }
@@ -223,95 +222,133 @@ PyObject* plain(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Py_RETURN_TRUE;
 }
 
-// pointers(dtypes, x, module, ...): the addresses of x and of every module's weight and bias (0 for None) as bytes, if the
-// kernels read them where they are: on the GPU, contiguous, 16-byte aligned, of x's type, which is one of `dtypes`; else None.
-PyObject* pointers(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  constexpr int MAX = 64;
-  std::uintptr_t out[MAX], bits = 0;
-  int count = 0;
-  if (n < 2 || 2 * (n - 2) + 1 > MAX || !PyTuple_Check(args[0])) {
-    PyErr_SetString(PyExc_TypeError, "pointers(dtypes, x, module, ...)");
-    return nullptr;
-  }
-  Ref dtype(PyObject_GetAttr(args[1], s_dtype));
-  if (!dtype) return nullptr;
-  bool known = false;
-  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(args[0]); ++i) known = known || PyTuple_GET_ITEM(args[0], i) == dtype.o;
-  if (!known) Py_RETURN_NONE;
+// The addresses of x and of modules' weights and biases (0 for None), if the kernels read them where they are: on the GPU,
+// contiguous, 16-byte aligned, of x's type, which is one of `dtypes`.
+class Addresses {
+ public:
   // 1: taken, 0: not where the kernels read it, -1: exception
-  auto take = [&](PyObject* t) {
+  int begin(PyObject* dtypes, PyObject* x) {
+    if (!PyTuple_Check(dtypes)) {
+      PyErr_SetString(PyExc_TypeError, "the first argument is a tuple of types");
+      return -1;
+    }
+    dtype_ = PyObject_GetAttr(x, s_dtype);
+    if (dtype_ == nullptr) return -1;
+    for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(dtypes); ++i)
+      if (PyTuple_GET_ITEM(dtypes, i) == dtype_) return take(x);
+    return 0;
+  }
+  // [rows, columns]: the extents the weight has to have ([rows] for no columns), and the bias [rows]; null: any.  A negative extent is
+  // the width that all weights with one share.
+  int module(PyObject* m, const long long* size) {
+    Ref d(PyObject_GetAttr(m, s_dict));
+    if (!d) return -1;
+    long long rows = 0;
+    for (PyObject* name : {s_weight, s_bias}) {
+      Ref t(parameter(m, d.o, name));
+      if (!t) return -1;
+      int ok = take(t.o);
+      if (ok == 1 && size != nullptr) {
+        if (name == s_bias) ok = t.o == Py_None ? 1 : has_elements(t.o, rows);
+        else ok = t.o == Py_None ? 0 : has_size(t.o, size, rows);
+      }
+      if (ok != 1) return ok;
+    }
+    return 1;
+  }
+  PyObject* bytes() const {
+    if ((bits_ & 15) != 0) Py_RETURN_NONE;
+    return PyBytes_FromStringAndSize(reinterpret_cast<const char*>(out_), count_ * sizeof(out_[0]));
+  }
+  long long width() const { return width_; }
+  static constexpr int MAX = 64;
+  Addresses() = default;
+  Addresses(const Addresses&) = delete;
+  ~Addresses() { Py_XDECREF(dtype_); }
+
+ private:
+  int take(PyObject* t) {
     if (t == Py_None) {
-      out[count++] = 0;
+      out_[count_++] = 0;
       return 1;
     }
     int ok = truth(t, s_is_cuda);
     if (ok <= 0) return ok;
     Ref dt(PyObject_GetAttr(t, s_dtype));
     if (!dt) return -1;
-    if (dt.o != dtype.o) return 0;
+    if (dt.o != dtype_) return 0;
     Ref c(PyObject_CallMethodNoArgs(t, s_is_contiguous));
     if (!c) return -1;
     ok = PyObject_IsTrue(c.o);
     if (ok <= 0) return ok;
     void* p;
     if (!address(t, p)) return -1;
-    out[count] = reinterpret_cast<std::uintptr_t>(p);
-    bits |= out[count++];
+    out_[count_] = reinterpret_cast<std::uintptr_t>(p);
+    bits_ |= out_[count_++];
     return 1;
-  };
-  int ok = take(args[1]);
-  for (Py_ssize_t i = 2; i < n && ok == 1; ++i)
-    for (PyObject* name : {s_weight, s_bias}) {
-      Ref t(parameter(args[i], name));
-      ok = t ? take(t.o) : -1;
-      if (ok != 1) break;
+  }
+  static int has_elements(PyObject* t, long long n) {
+    Ref v(PyObject_CallMethodNoArgs(t, s_numel));
+    long long at;
+    if (!v || !convert(v.o, at)) return -1;
+    return at == n;
+  }
+  int is_extent(long long at, long long want) {
+    if (want >= 0) return at == want;
+    if (width_ < 0) width_ = at;
+    return at == width_;
+  }
+  int has_size(PyObject* t, const long long* size, long long& rows) {
+    rows = size[0];
+    if (size[1] == 0) return has_elements(t, rows);
+    Ref shape(PyObject_GetAttr(t, s_shape));
+    if (!shape) return -1;
+    if (!PyTuple_Check(shape.o) || PyTuple_GET_SIZE(shape.o) != 2) return 0;
+    long long at[2];
+    for (int i = 0; i < 2; ++i) {
+      if (!convert(PyTuple_GET_ITEM(shape.o, i), at[i])) return -1;
+      if (!is_extent(at[i], size[i])) return 0;
     }
+    rows = at[0];
+    return 1;
+  }
+  std::uintptr_t out_[MAX], bits_ = 0;
+  int count_ = 0;
+  long long width_ = -1;
+  PyObject* dtype_ = nullptr;
+};
+
+// pointers(dtypes, x, module, ...): the addresses as bytes, or None.
+PyObject* pointers(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n < 2 || 2 * (n - 2) + 1 > Addresses::MAX) {
+    PyErr_SetString(PyExc_TypeError, "pointers(dtypes, x, module, ...)");
+    return nullptr;
+  }
+  Addresses a;
+  int ok = a.begin(args[0], args[1]);
+  for (Py_ssize_t i = 2; i < n && ok == 1; ++i) ok = a.module(args[i], nullptr);
   if (ok < 0) return nullptr;
-  if (ok == 0 || (bits & 15) != 0) Py_RETURN_NONE;
-  return PyBytes_FromStringAndSize(reinterpret_cast<const char*>(out), count * sizeof(out[0]));
+  if (ok == 0) Py_RETURN_NONE;
+  return a.bytes();
 }
 
-// A tensor's extents; their number, or -1 with an exception.  (More than two count, but are not read.)
-Py_ssize_t extents(PyObject* tensor, long long (&out)[2]) {
-  Ref shape(PyObject_GetAttr(tensor, s_shape));
-  if (!shape) return -1;
-  if (!PyTuple_Check(shape.o)) {
-    PyErr_SetString(PyExc_TypeError, "a tensor's shape is no tuple");
-    return -1;
+// weights(dtypes, x, module, rows, columns, ...): (the addresses as bytes, the width that the negative extents stand for), if every
+// weight has the size beside its module; else (None, that width or a negative number).
+PyObject* weights(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n < 2 || (n - 2) % 3 != 0 || (n - 2) / 3 * 2 + 1 > Addresses::MAX) {
+    PyErr_SetString(PyExc_TypeError, "weights(dtypes, x, module, rows, columns, ...)");
+    return nullptr;
   }
-  const Py_ssize_t n = PyTuple_GET_SIZE(shape.o);
-  for (Py_ssize_t i = 0; i < n && i < 2; ++i)
-    if (!convert(PyTuple_GET_ITEM(shape.o, i), out[i])) return -1;
-  return n;
-}
-
-// rows(module): the rows of its weight.
-PyObject* rows(PyObject*, PyObject* m) {
-  Ref w(parameter(m, s_weight));
-  if (!w) return nullptr;
-  long long at[2];
-  const Py_ssize_t n = w.o == Py_None ? 0 : extents(w.o, at);
-  if (n < 0) return nullptr;
-  return PyLong_FromLongLong(n > 0 ? at[0] : 0);
-}
-
-// sized(module, rows, columns, ...): whether every module's weight is [rows, columns], or [rows] where columns is 0, and its bias
-// None or [rows].
-PyObject* sized(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  for (Py_ssize_t i = 0; i + 2 < n; i += 3) {
-    long long want[2], at[2];
-    if (!convert(args[i + 1], want[0]) || !convert(args[i + 2], want[1])) return nullptr;
-    for (PyObject* name : {s_weight, s_bias}) {
-      Ref t(parameter(args[i], name));
-      if (!t) return nullptr;
-      if (t.o == Py_None && name == s_bias) continue;
-      if (t.o == Py_None) Py_RETURN_FALSE;
-      const Py_ssize_t dims = extents(t.o, at), expected = name == s_weight && want[1] != 0 ? 2 : 1;
-      if (dims < 0) return nullptr;
-      if (dims != expected || at[0] != want[0] || (expected == 2 && at[1] != want[1])) Py_RETURN_FALSE;
-    }
+  Addresses a;
+  int ok = a.begin(args[0], args[1]);
+  for (Py_ssize_t i = 2; i < n && ok == 1; i += 3) {
+    long long size[2];
+    if (!convert(args[i + 1], size[0]) || !convert(args[i + 2], size[1])) return nullptr;
+    ok = a.module(args[i], size);
   }
-  Py_RETURN_TRUE;
+  if (ok < 0) return nullptr;
+  Ref bytes(ok == 1 ? a.bytes() : Py_NewRef(Py_None));
+  return bytes ? Py_BuildValue("(OL)", bytes.o, a.width()) : nullptr;
 }
 
 PyObject* set_host_tensor_error(PyObject*, PyObject* f) {
@@ -325,8 +362,7 @@ constexpr PyMethodDef fast(const char* name) {
 }
 PyMethodDef methods[] = {{"bind", bind, METH_VARARGS, nullptr},
                          {"set_host_tensor_error", set_host_tensor_error, METH_O, nullptr},
-                         {"rows", rows, METH_O, nullptr},
-                         fast<sub>("sub"), fast<plain>("plain"), fast<pointers>("pointers"), fast<sized>("sized"),
+                         fast<sub>("sub"), fast<plain>("plain"), fast<pointers>("pointers"), fast<weights>("weights"),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "neox_host_calls", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
@@ -339,7 +375,7 @@ PyMODINIT_FUNC PyInit_neox_host_calls(void) {
   } names[] = {{&s_is_cuda, "is_cuda"}, {&s_data_ptr, "data_ptr"}, {&s_dtype, "dtype"}, {&s_is_contiguous, "is_contiguous"},
                {&s_forward, "forward"}, {&s_forward_hooks, "_forward_hooks"}, {&s_forward_pre_hooks, "_forward_pre_hooks"},
                {&s_parameters, "_parameters"}, {&s_modules, "_modules"}, {&s_buffers, "_buffers"}, {&s_weight, "weight"}, {&s_bias, "bias"},
-               {&s_dict, "__dict__"}, {&s_shape, "shape"}};
+               {&s_dict, "__dict__"}, {&s_shape, "shape"}, {&s_numel, "numel"}};
   for (auto& n : names)
     if ((*n.at = PyUnicode_InternFromString(n.name)) == nullptr) return nullptr;
   return PyModule_Create(&module_def);

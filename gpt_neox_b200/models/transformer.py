@@ -23,7 +23,7 @@ from ..ops.attention import flash_attention, next_dropout_seed
 from ..ops.elementwise import bias_dropout_add, branch_sum
 from ..ops.gemm import gemm as gemm_op
 from ..ops.gemm import linear as linear_op
-from ..ops.layer_infer import layer_infer, pointers
+from ..ops.layer_infer import layer_infer
 from ..ops.norm import dual_layer_norm
 from ..ops import _lib as kernel_lib
 from ..ops import rope as rope_ops
@@ -492,12 +492,11 @@ class ParallelTransformerLayer(nn.Module):
                 return None
         if qkv.skip_bias_add:
             return None
-        ptrs = pointers(x, n1, n2, qkv, dense, up, down)
-        if ptrs is None:
-            return None
         # the kernels walk the weights by the sizes that they are told: those of the tensors, whatever the modules were built with
-        h, heads, kvp, ffn = x.shape[2], a.num_attention_heads_per_partition, a.num_kv_heads_per_partition, calls.rows(up)
-        if not calls.sized(n1, h, 0, n2, h, 0, qkv, (heads + 2 * kvp) * hn, h, dense, h, heads * hn, up, ffn, h, down, h, ffn):
+        h, heads, kvp = x.shape[2], a.num_attention_heads_per_partition, a.num_kv_heads_per_partition
+        ptrs, ffn = calls.weights(kernel_lib.H16, x, n1, h, 0, n2, h, 0, qkv, (heads + 2 * kvp) * hn, h, dense, h, heads * hn,
+                                  up, -1, h, down, h, -1)
+        if ptrs is None:
             return None
         has_past = layer_past is not None and (not torch.is_tensor(layer_past) or layer_past.numel() > 0)
         past = layer_past[0].shape[0] if has_past else 0

@@ -182,8 +182,7 @@ def lib(like=None):
 
 
 def calls():
-    """The native module (csrc/host_calls.cpp): ``sub``, ``plain``, ``pointers``, ``rows`` and ``sized`` beside the bound entry
-    points."""
+    """The native module (csrc/host_calls.cpp): ``sub``, ``plain``, ``pointers`` and ``weights`` beside the bound entry points."""
     if _CALLS is None:
         lib()
     return _CALLS

@@ -18,17 +18,11 @@ _TAIL = struct.Struct("@q6Pq12i2f")
 _BYTES = 13 * 8 + _TAIL.size
 
 
-def pointers(x, *modules):
-    """The addresses of x and of every module's weight and bias, if the kernels read them where they are: on the GPU,
-    contiguous, 16-byte aligned, of one 16-bit type.  None otherwise."""
-    return _lib.calls().pointers(_lib.H16, x, *modules)
-
-
 def layer_infer(x, ptrs, cos, sin, present, past, *, heads, kv_heads, head_dim, ffn, rot, window, scale, eps, act):
-    """x [s, b, h] -> x + attention + MLP [s, b, h].  ``ptrs``: ``pointers`` of x, the two norms, qkv, dense, up and down;
-    ``present`` [2, past + s, b, kv_heads, head_dim]: the cache, whose last s rows are written.  ``act``: ("tanh" or "erf",
-    whether a recorded pass would store the GeLU's derivative).  One scratch allocation holds what csrc/layer_infer.cu
-    names."""
+    """x [s, b, h] -> x + attention + MLP [s, b, h].  ``ptrs``: the addresses that ``weights`` of csrc/host_calls.cpp gives for x, the
+    two norms, qkv, dense, up and down; ``present`` [2, past + s, b, kv_heads, head_dim]: the cache, whose last s rows are
+    written.  ``act``: ("tanh" or "erf", whether a recorded pass would store the GeLU's derivative).  One scratch allocation
+    holds what csrc/layer_infer.cu names."""
     s, b, h = x.shape
     lib = _lib.lib(x)
     out = torch.empty_like(x)

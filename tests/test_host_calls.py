@@ -164,25 +164,43 @@ def test_pointers(calls):
         calls.pointers(_lib.H16, x, real)
 
 
+class _Shaped(_OnGpu):
+    def __init__(self, at, *shape):
+        super().__init__(at)
+        self.shape = torch.Size(shape)
+
+    def numel(self):
+        return self.shape.numel()
+
+
 def test_weight_sizes(calls):
-    """Weights and biases are compared with the sizes that a caller expects, wherever a module holds them."""
-    lin = lambda n, k, bias=True: torch.nn.Linear(k, n, bias=bias)
-    a, b, norm = lin(6, 4), lin(4, 6, bias=False), torch.nn.LayerNorm(4)
-    assert calls.rows(a) == 6 and calls.rows(norm) == 4
-    assert calls.sized(norm, 4, 0, a, 6, 4, b, 4, 6)
-    for m, n, k in ((a, 5, 4), (a, 6, 5), (a, 6, 0), (norm, 4, 1), (norm, 3, 0)):
-        assert not calls.sized(b, 4, 6, m, n, k)
-    a.bias = torch.nn.Parameter(torch.zeros(5))
-    assert not calls.sized(a, 6, 4)
-    a.bias = torch.nn.Parameter(torch.zeros(6, 1))
-    assert not calls.sized(a, 6, 4)
-    a.bias = None
-    a.weight = torch.nn.Parameter(torch.zeros(8, 4))
-    assert calls.rows(a) == 8 and calls.sized(a, 8, 4) and not calls.sized(a, 6, 4)
-    a.weight = torch.nn.Parameter(torch.zeros(8, 4, 1))
-    assert not calls.sized(a, 8, 4)
+    """Addresses are given where every weight has the size beside its module, and its bias as many elements as it has rows."""
+    x = _OnGpu(16)
+
+    def held(weight, bias=None):
+        m = _Plain()
+        m.__dict__.update(weight=weight, bias=bias)
+        return m
+
+    def given(*modules_and_sizes):
+        got, width = calls.weights(_lib.H16, x, *modules_and_sizes)
+        return (None if got is None else [int.from_bytes(got[i:i + 8], "little") for i in range(0, len(got), 8)]), width
+
+    a, b, norm = held(_Shaped(32, 6, 4), _Shaped(48, 6)), held(_Shaped(64, 4, 6)), held(_Shaped(80, 4), _Shaped(96, 4))
+    where = [16, 80, 96, 32, 48, 64, 0]
+    assert given(norm, 4, 0, a, 6, 4, b, 4, 6) == (where, -1)
+    assert given(norm, 4, 0, a, -1, 4, b, 4, -1) == (where, 6)
+    for m, n, k in ((a, 5, 4), (a, 6, 5), (a, 4, 6), (a, 6, 0), (norm, 4, 1), (norm, 3, 0)):
+        assert given(b, 4, 6, m, n, k)[0] is None
+    assert given(a, -1, 4, b, -1, 6)[0] is None and given(a, -1, 4, held(_Shaped(64, 4, 5)), 4, -1)[0] is None
+    for bias in (_Shaped(48, 5), _Shaped(48, 0), _OnGpu(48, is_cuda=False), _Shaped(56, 6)):
+        assert given(held(_Shaped(32, 6, 4), bias), 6, 4)[0] is None
+    assert given(held(_Shaped(32, 6, 4, 1)), 6, 4)[0] is None and given(held(None), 6, 4)[0] is None
+    for args in ((), (_lib.H16,), (_lib.H16, x, a, 6), (list(_lib.H16), x)):
+        with pytest.raises(TypeError):
+            calls.weights(*args)
     with pytest.raises(AttributeError):
-        calls.sized(torch.nn.Identity(), 1, 1)
+        calls.weights(_lib.H16, x, torch.nn.Identity(), 1, 1)
 
 
 def _resized_mlp(layer, up, down):
@@ -215,9 +233,7 @@ def test_a_layer_in_one_call_goes_by_the_weights_it_is_given(calls, up, down, mo
         for name in ("weight", "bias"):
             t = getattr(module, name)
             if t is not None:
-                fake = _OnGpu(4096)
-                fake.shape = t.shape
-                module.__dict__[name] = fake
+                module.__dict__[name] = _Shaped(4096, *t.shape)
     h = a.hidden_size_per_attention_head * a.num_attention_heads_per_partition
     x = _OnGpu(4096)
     x.shape = torch.Size((2, 1, h))
