@@ -918,7 +918,8 @@ static bool bwd_map(CUtensorMap* m, const void* base, int B, int Hh, int S, int 
 // Which kernels a call takes: persistent ones or one CTA per tile (attention_bwd_tile.cu).  Persistent CTAs overlap one item
 // with the next, so they need more items than SMs; a single item costs them 1 - 4 us more (more roles, barriers and
 // threads to set up).  Measured over 64 .. 2048 tokens x 4 .. 1536 heads, time per tile / persistent:
-//   dropout      0.5 (registers spill);  block-sparse layouts 0.7 - 1 (a CTA's share is fixed, and tiles are of any length)
+//   dropout      0.5 (registers spill);  block-sparse layouts 0.7 - 1 (a CTA's share is fixed, and tiles are of any length).  A
+//                softmax scale of 0, which makes a masked score NaN in the other forms, goes with them
 //   dQ, ALiBi    0.93 - 2.7: always persistent
 //   dQ, 128      more items than SMs 1.13 - 1.66; fewer, 256 keys and more 0.98 - 1.15, fewer keys 0.86 - 1.17
 //   dQ, 64       causal, more items than SMs 1.01 - 1.63; rows of 65 .. 128 keys 0.98 below 2 items per SM, 1.05 - 1.19 above,

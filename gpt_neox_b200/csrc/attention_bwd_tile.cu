@@ -1,5 +1,6 @@
-// Flash attention backward, one CTA per tile: the kernels for dropout, for block-sparse layouts and for calls whose tiles do
-// not fill the SMs more than once (attn_bwd_route in attention_bwd.cu says which call takes which and why).
+// Flash attention backward, one CTA per tile: the kernels for dropout and for block-sparse layouts, and otherwise for heads of up to
+// 64 (dQ: also for larger ones) in calls whose tiles do not fill the SMs often enough (attn_bwd_route in attention_bwd.cu says
+// which call takes which and why).  A softmax scale of 0 comes here, too, to the general forms.
 //
 //   dQ       a CTA per 128 query rows: loops over blocks of 128 keys (longest tiles first)
 //   dK / dV  a CTA per 128 keys of a kv head: loops over the query heads of its group and over blocks of 128 query rows
@@ -603,8 +604,10 @@ static int tile_dkv(const BwdMaps& m, const AttnBwdParams& p, cudaStream_t s) {
   const dim3 grid((p.Sk + AB - 1) / AB, p.Hk, p.B);
   constexpr int dyn = TileSmem<DP>::DYN;
   if (p.drop_thr > 0u) return tile_launch(attn_bwd_tile_dkv_kernel<DP, true, true>, dyn, grid, m, p, s);
-  if (tile_general(p)) return tile_launch(attn_bwd_tile_dkv_kernel<DP, false, true>, dyn, grid, m, p, s);
-  return tile_launch(attn_bwd_tile_dkv_kernel<DP, false, false>, dyn, grid, m, p, s);
+  if constexpr (DP <= 64) {      // (larger heads without dropout, layout and a scale of 0 are persistent)
+    if (!tile_general(p)) return tile_launch(attn_bwd_tile_dkv_kernel<DP, false, false>, dyn, grid, m, p, s);
+  }
+  return tile_launch(attn_bwd_tile_dkv_kernel<DP, false, true>, dyn, grid, m, p, s);
 }
 
 int attn_bwd_tile_dq(const BwdMaps& m, const AttnBwdParams& p, cudaStream_t s) {

@@ -71,7 +71,7 @@ def combine_bwd(g, y, plan: Plan, weights):
 
 def grouped_gemm_rows(a, w, plan: Plan, n_out, *, trans_b, gelu=None, aux_out=None, dgelu_aux=None, dgelu=None,
                       aux_deriv=False):
-    """C[rows, n_out] = A[rows, K] x op(W_e) per 128-row tile; ``w`` stacks the experts' matrices
+    """C[rows, n_out] = A[rows, K] x op(W_e), e the expert of a tile of 256 rows; ``w`` stacks the experts' matrices
     ([E * n_out, K] for trans_b False, [E * K, n_out] for trans_b True)."""
     rows, K = a.shape
     out = torch.empty((rows, n_out), device=a.device, dtype=a.dtype)
