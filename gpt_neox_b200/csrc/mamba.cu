@@ -18,9 +18,9 @@
 // lane's channels before lanes and warps exchange them, and the next block's segment is staged where the walked one
 // was.  Those states take 2 bytes per token and channel from the forward to the backward (25 MB for 4 x 2048 x 1536, as
 // much as one more 16-bit activation), and the tiles' partial sums of dB and dC 2 bytes during the backward.
-// Bound by: light sweeps, the unit of exponentials (16 per step and channel; 82 and 72 % busy); forward, that unit 68 %, shared
-// memory 69 % and issue slots 62 % together; backward, issue slots (59 % with 3 warps per scheduler; shared memory 55 %),
-// where a step and channel costs 500 lane operations for 16 states.  DRAM 6-10 %.
+// Bound by: light sweeps, the unit of exponentials (16 per step and channel; 81 and 70 % busy); forward, that unit 66 %, shared
+// memory 68 % and issue slots 63 % together; backward, issue slots (60 % with 3 warps per scheduler; shared memory 52 %),
+// where a step and channel costs 500 lane operations for 16 states.  DRAM 8-14 %.
 // Convolution + scan, forward + backward, 4 x 2048 steps of 1536 channels, fp16: 785 us with one channel per quad, inputs staged
 // by the whole CTA and dB / dC exchanged per channel (final forward sweep 119, light ones 70 and 86, backward 407 us); 583 us
 // now (91, 60 and 74, 277).  Calls of few channels and steps are latency, us, forward / forward + backward, that kernel and this
